@@ -151,6 +151,25 @@ def test_attention_bwd_rising_scores():
         assert rel_err(dqkv[:, i * HD:(i + 1) * HD], x.grad[:, i * HD:(i + 1) * HD]) < 2e-2
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("nw,N,H", [(2, 15, 2), (3, 64, 1), (40, 64, 8), (2, 65, 2), (1, 127, 2), (2, 129, 3), (5, 225, 30)])
+def test_attention_bwd_tile_edges(nw, N, H, d):
+    """Windows around the 64-row streamed and the 128-row resident tile, single-tile windows (an item shorter than the
+    number of chains), and more items than SMs (the persistent CTAs carry their rings over item boundaries). P, dS and
+    the result are rounded to bf16 (2^-9 each, at most), the products are accumulated in fp32: three roundings, 6e-3."""
+    from aeris_gb_b200.ops import attention as A
+    qkv = torch.randn(nw * N, 3 * H * d, device=DEV).bfloat16()
+    go = torch.randn(nw * N, H * d, device=DEV).bfloat16()
+    o, lse = A.attn_fwd(qkv, nw, N, H, d)
+    dqkv = torch.full_like(qkv, float("nan"))
+    A.attn_bwd(qkv, o, go, lse, nw, N, H, d, dqkv=dqkv)
+    x = qkv.float().requires_grad_(True)
+    A.attn_reference(x, nw, N, H, d).backward(go.float())
+    HD = H * d
+    for i in range(3):
+        assert rel_err(dqkv[:, i * HD:(i + 1) * HD], x.grad[:, i * HD:(i + 1) * HD]) < 6e-3
+
+
 @pytest.mark.parametrize("D", [128, 1536])
 @pytest.mark.parametrize("mode", [0, 1])
 def test_modnorm_fwd_bwd(D, mode):
