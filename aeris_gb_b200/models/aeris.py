@@ -348,11 +348,12 @@ class SwinLayer(nn.Module):
         return m
 
     def forward(self, x: torch.Tensor, dt: torch.Tensor, ctx: StreamContext, regroup=None,
-                publish_out: bool = False) -> torch.Tensor:
+                publish_out: bool = False, keep_from: int | None = None) -> torch.Tensor:
         """``regroup = (src_shift, dst_shift)``: the stream arrives in the ``src`` window layout and this layer works
         in ``dst``. On the CUDA path the re-partition (with its halo exchange under WP) is fused into the first
         block's modulate+norm kernel; the oracle path applies it as a separate gather. ``publish_out``: the caller
-        re-partitions this layer's output next, so under WP the last block writes it into a peer-readable buffer."""
+        re-partitions this layer's output next, so under WP the last block writes it into a peer-readable buffer.
+        ``keep_from``: blocks from this index on keep their internals for the backward pass (CUDA path)."""
         cfg = self.cfg
         eps = cfg.eps(x.dtype)
         if regroup is not None and regroup[0] == regroup[1]:
@@ -371,7 +372,8 @@ class SwinLayer(nn.Module):
                 meta = fused.BlockMeta(ctx.grid.windows_per_rank, ctx.grid.n_local, cfg.heads, cfg.head_dim,
                                        E.MODE_MOD_THEN_NORM if after_mod_norm else E.MODE_NORM_THEN_MOD,
                                        eps, cfg.chunk_windows, sp=ctx.sp_exchange if ctx.grid.sp > 1 else None,
-                                       rope=ctx.rope(x.device), tp=ctx.tp_exchange if cfg.tp > 1 else None)
+                                       rope=ctx.rope(x.device), tp=ctx.tp_exchange if cfg.tp > 1 else None,
+                                       keep=keep_from is not None and j >= keep_from)
                 if cfg.tp > 1 and ctx.tp_exchange is None:
                     raise RuntimeError("tensor parallelism on CUDA needs StreamContext.tp_exchange (tensor.TPExchange)")
                 rg = None
@@ -515,13 +517,26 @@ class AerisModel(nn.Module):
         self.layers = nn.ModuleList([SwinLayer(cfg) for _ in range(cfg.n_layers)]).to(cfg.model_dtype)
         self.output_stage = OutputStage(cfg)
 
+    def _first_kept_block(self, x: torch.Tensor, ctx: StreamContext) -> int:
+        """Index of the first block that keeps its internals for the backward pass (the number of blocks: none does).
+        The last blocks keep theirs: the backward pass gives that memory back first."""
+        cfg = self.cfg
+        n_blocks = len(self.layers) * cfg.sublayers
+        if not (torch.is_grad_enabled() and use_fused(x)) or ctx.grid.sp > 1 or cfg.tp > 1:
+            return n_blocks
+        from . import fused
+        return n_blocks - fused.plan_kept_blocks(x.shape[0], cfg.dim, cfg.heads * cfg.head_dim, cfg.heads, cfg.mlp_dim,
+                                                 n_blocks, cfg.chunk_windows * ctx.grid.n_local, x.device)
+
     def trunk(self, x: torch.Tensor, dt: torch.Tensor, ctx: StreamContext) -> torch.Tensor:
         cur = (0, 0)
         n = len(self.layers)
+        first_kept = self._first_kept_block(x, ctx)
         for i, layer in enumerate(self.layers):
             nxt = self.cfg.layer_shift(i)
             after = self.cfg.layer_shift(i + 1) if i + 1 < n else (0, 0)     # layout of whoever consumes the output
-            x = layer(x, dt, ctx, regroup=(cur, nxt), publish_out=(after != nxt))
+            x = layer(x, dt, ctx, regroup=(cur, nxt), publish_out=(after != nxt),
+                      keep_from=max(0, first_kept - i * self.cfg.sublayers))
             cur = nxt
         return ctx.regroup_unfused(x, cur, (0, 0))
 

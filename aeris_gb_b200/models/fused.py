@@ -3,14 +3,16 @@
 The block is processed in *chunks of whole windows* of one sample: inside a block every token only interacts with its
 own window, so a chunk runs modulate+RMSNorm -> QKV GEMM -> window attention -> (wo GEMM + gated residual) ->
 modulate+RMSNorm -> (w1 GEMM + SwiGLU) -> (w2 GEMM + gated residual) with a working set of a few GB no matter how
-large the image is. Training keeps only the block input (activation checkpointing, absent from the reference and
-mandatory for one million tokens per sample); the backward pass recomputes a chunk's internals and immediately
-back-propagates through them, accumulating weight gradients in fp32 directly from the GEMM epilogue.
+large the image is. Training keeps a block's internals where memory allows (:func:`plan_kept_blocks`) and only the block
+input elsewhere (activation checkpointing, absent from the reference and mandatory for one million tokens per sample);
+the backward pass then recomputes a chunk's internals and immediately back-propagates through them, accumulating weight
+gradients in fp32 directly from the GEMM epilogue.
 
 Math restated from src/aeris/models/parallel_swin.py:453-472 (block), :82-104 (SwiGLU), :261-308 (attention).
 """
 from __future__ import annotations
 
+import math
 from dataclasses import dataclass
 
 import torch
@@ -32,6 +34,7 @@ class BlockMeta:
     sp: "SPExchange | None" = None     # Ulysses sequence parallelism: L is then the LOCAL token count of a window
     rope: tuple | None = None          # (cos, sin) [L, head_dim / 2]: optional 2-D rotary embedding of q and k
     tp: object | None = None           # parallel.tensor.TPExchange: w1 / w2 are this rank's shards of the MLP weights
+    keep: bool = False                 # forward keeps its internals for the backward pass (see plan_kept_blocks)
 
 
 class Workspace:
@@ -117,8 +120,61 @@ def _rope_qk_(qkv: torch.Tensor, meta: BlockMeta, nw: int, inverse: bool = False
     E.rope_qk_(qkv, cos.float().contiguous(), sin.float().contiguous(), meta.L, meta.heads, meta.head_dim, inverse)
 
 
-def _chunks(meta: BlockMeta):
-    step = min(meta.chunk_windows, meta.n_win_per_sample)
+KEPT = ("h1", "qkv", "o", "lse", "x1", "h2", "act", "u")
+
+
+def _kept_shapes(T: int, D: int, HD: int, heads: int, F: int) -> dict[str, tuple[tuple[int, ...], torch.dtype]]:
+    """What a block keeps for its backward pass: every internal the recompute would produce again."""
+    bf = torch.bfloat16
+    return {"h1": ((T, D), bf), "qkv": ((T, 3 * HD), bf), "o": ((T, HD), bf), "lse": ((T * heads,), torch.float32),
+            "x1": ((T, D), bf), "h2": ((T, D), bf), "act": ((T, F), bf), "u": ((T, 2 * F), bf)}
+
+
+def kept_bytes(T: int, D: int, HD: int, heads: int, F: int) -> int:
+    return sum(math.prod(shape) * dt.itemsize for shape, dt in _kept_shapes(T, D, HD, heads, F).values())
+
+
+def n_kept(n_blocks: int, per_block: int, base: int, free: int) -> int:
+    """How many of ``n_blocks`` blocks may keep their internals: these take at most half of what is left of ``free``
+    after the ``base`` bytes that the step needs in any case."""
+    return max(0, min(n_blocks, (free - base) // 2 // per_block))
+
+
+def plan_kept_blocks(T: int, D: int, HD: int, heads: int, F: int, n_blocks: int, chunk_rows: int, device) -> int:
+    """How many blocks of a training forward keep their internals instead of recomputing them in the backward pass.
+
+    The recompute is a quarter of a step's tensor-core work (one more QKV, wo and w1 product and attention forward per
+    block) and under the power cap time follows work, so it is only worth its price where memory is short: a full-size
+    image (1 M tokens x 40 blocks) needs it, one with a few GB of internals on a 180 GB GPU does not. What counts is the
+    memory that is free now (unused allocator cache included), less the block inputs and the chunk workspaces that the
+    step will also allocate. The driver is asked only when the allocator's own cache does not cover the need (the question
+    costs up to milliseconds on a busy host), and not at all for needs below 1/256 of the device."""
+    per_block = kept_bytes(T, D, HD, heads, F)
+    if per_block * n_blocks <= torch.cuda.get_device_properties(device).total_memory // 256:
+        return n_blocks
+    # block inputs (a shifted layer holds its source too), stream gradients, two chunk working sets
+    base = (n_blocks + 4) * T * D * 2 + 2 * kept_bytes(min(T, chunk_rows), D, HD, heads, F)
+    stats = torch.cuda.memory_stats_as_nested_dict(device)
+    held = [stats.get(k, {}).get("all", {}).get("current", 0) for k in ("reserved_bytes", "allocated_bytes")]
+    cached = max(0, held[0] - held[1])
+    if n_blocks * per_block + base <= cached:      # nothing new to ask the driver for (any step after the first)
+        return n_blocks
+    free = cached + torch.cuda.mem_get_info(device)[0]
+    return n_kept(n_blocks, per_block, base, free)
+
+
+MIN_CHUNK_BYTES = 512 << 20
+
+
+def chunk_step(meta: BlockMeta, D: int, F: int) -> int:
+    """Windows per chunk: ``meta.chunk_windows`` bounds the working set, but a chunk whose internals take less than half a
+    gigabyte saves no memory worth having and costs launches that the GPU finishes faster than they are issued (32
+    windows of 64 tokens at dim 128 in chunks of 8: 1,582 launches per step for 7 ms of device time)."""
+    floor = MIN_CHUNK_BYTES // (kept_bytes(1, D, meta.heads * meta.head_dim, meta.heads, F) * meta.L)
+    return min(max(meta.chunk_windows, floor), meta.n_win_per_sample)
+
+
+def _chunks(meta: BlockMeta, step: int):
     for w0 in range(0, meta.n_win_per_sample, step):
         yield w0, min(step, meta.n_win_per_sample - w0)
 
@@ -189,13 +245,22 @@ def _tp_mlp_fwd(tp, x1, sc2, sh2, wn2, meta: BlockMeta, w1, w2, g2, act, y_out):
     TP.gemm_reduce_scatter(tp, act[:M], w2, resid=x1, gate=g2, out=y_out)
 
 
+def _chunk_views(bufs: dict[str, torch.Tensor], r0: int, n: int, heads: int):
+    """Rows ``[r0, r0 + n)`` of h1, qkv, o, x1, h2, act and the matching slice of lse (whole windows: rows x heads)."""
+    return (*(bufs[k][r0:r0 + n] for k in ("h1", "qkv", "o", "x1", "h2", "act")), bufs["lse"][r0 * heads:(r0 + n) * heads])
+
+
 def block_forward(x: torch.Tensor, mod: torch.Tensor, meta: BlockMeta, wn1, wqkv, wo, wn2, w1, w2,
-                  out: torch.Tensor | None = None, gather=None) -> torch.Tensor:
+                  out: torch.Tensor | None = None, gather=None,
+                  kept: dict[str, torch.Tensor] | None = None) -> torch.Tensor:
     """x: [B * n_win * L, D] bf16 window-major; mod: [B, 6D] fp32 (shift1, scale1, gate1, shift2, scale2, gate2).
 
     ``gather = (table, peer_ptrs, src)``: ``x`` is then an EMPTY buffer in this block's window layout; the first
     modulate+norm kernel of every chunk pulls its rows through the table from ``src`` on this or a peer GPU (the
-    re-partition / halo exchange of a shifted layer) and writes them into ``x`` on the way."""
+    re-partition / halo exchange of a shifted layer) and writes them into ``x`` on the way.
+
+    ``kept``: full-size buffers (:func:`_kept_shapes`) that receive the block's internals; without it they live in chunk
+    workspaces and are gone afterwards."""
     T, D = x.shape
     B = mod.shape[0]
     F = w2.shape[1]
@@ -204,50 +269,56 @@ def block_forward(x: torch.Tensor, mod: torch.Tensor, meta: BlockMeta, wn1, wqkv
     assert T == B * rows_per_sample
     y = out if out is not None else torch.empty_like(x)
     ws, dev, bf = _WS, x.device, torch.bfloat16
-    cmax = min(meta.chunk_windows, meta.n_win_per_sample) * meta.L
-    h = ws.get("h", (cmax, D), bf, dev)
-    qkv = ws.get("qkv", (cmax, 3 * HD), bf, dev)
-    o = ws.get("o", (cmax, HD), bf, dev)
-    x1 = ws.get("x1", (cmax, D), bf, dev)
-    tpn = meta.tp.tp if meta.tp is not None else 1       # gathered rows x local features: the same element count
-    act = ws.get("act", (cmax * tpn, F), bf, dev)
-    lse = ws.get("lse", (cmax * meta.heads,), torch.float32, dev)
+    step = chunk_step(meta, D, F)
+    if kept is None:
+        cmax = step * meta.L
+        h = ws.get("h", (cmax, D), bf, dev)
+        tpn = meta.tp.tp if meta.tp is not None else 1   # gathered rows x local features: the same element count
+        chunk_bufs = {"h1": h, "qkv": ws.get("qkv", (cmax, 3 * HD), bf, dev), "o": ws.get("o", (cmax, HD), bf, dev),
+                      "lse": ws.get("lse", (cmax * meta.heads,), torch.float32, dev),
+                      "x1": ws.get("x1", (cmax, D), bf, dev), "h2": h, "act": ws.get("act", (cmax * tpn, F), bf, dev)}
     mod = mod.contiguous()
     for b in range(B):
         sh1, sc1, g1, sh2, sc2, g2 = [mod[b, i * D:(i + 1) * D] for i in range(6)]
-        for w0, nw in _chunks(meta):
+        for w0, nw in _chunks(meta, step):
             r0 = b * rows_per_sample + w0 * meta.L
             n = nw * meta.L
             xc = x[r0:r0 + n]
+            h1, qkv, o, x1, h2, act, lse = _chunk_views(kept, r0, n, meta.heads) if kept is not None else \
+                _chunk_views(chunk_bufs, 0, n, meta.heads)
             if gather is not None:
                 table, peers, src = gather
-                E.modnorm_fwd(None, sc1, sh1, wn1, mode=meta.mode, eps=meta.eps, out=h[:n],
+                E.modnorm_fwd(None, sc1, sh1, wn1, mode=meta.mode, eps=meta.eps, out=h1,
                               gather_idx=table[r0:r0 + n], peer_ptrs=peers, x_out=xc, rows=n,
                               src_rows=src.shape[0])
             else:
-                E.modnorm_fwd(xc, sc1, sh1, wn1, mode=meta.mode, eps=meta.eps, out=h[:n])
+                E.modnorm_fwd(xc, sc1, sh1, wn1, mode=meta.mode, eps=meta.eps, out=h1)
             if meta.sp is None:
-                G.gemm(h[:n], wqkv, out=qkv[:n])
+                G.gemm(h1, wqkv, out=qkv)
                 if meta.rope is not None:
-                    _rope_qk_(qkv[:n], meta, nw)
-                A.attn_fwd(qkv[:n], nw, meta.L, meta.heads, meta.head_dim, out=o[:n],
-                           lse=lse[:n * meta.heads].view(nw, meta.heads, meta.L))
-                oc = o[:n]
+                    _rope_qk_(qkv, meta, nw)
+                A.attn_fwd(qkv, nw, meta.L, meta.heads, meta.head_dim, out=o, lse=lse.view(nw, meta.heads, meta.L))
+                oc = o
             else:
-                oc = _sp_attention_fwd(meta, h[:n], wqkv, nw, keep_local=False)[0]
-            G.gemm(oc, wo, out=x1[:n], epi=G.EPI_GATE_RESID, resid=xc, gate=g1)
+                oc = _sp_attention_fwd(meta, h1, wqkv, nw, keep_local=False)[0]
+            G.gemm(oc, wo, out=x1, epi=G.EPI_GATE_RESID, resid=xc, gate=g1)
             if meta.tp is not None:
-                _tp_mlp_fwd(meta.tp, x1[:n], sc2, sh2, wn2, meta, w1, w2, g2, act, y[r0:r0 + n])
+                _tp_mlp_fwd(meta.tp, x1, sc2, sh2, wn2, meta, w1, w2, g2, chunk_bufs["act"], y[r0:r0 + n])
                 continue
-            E.modnorm_fwd(x1[:n], sc2, sh2, wn2, mode=meta.mode, eps=meta.eps, out=h[:n])
-            G.gemm(h[:n], w1, out=act[:n], epi=G.EPI_SWIGLU)
-            G.gemm(act[:n], w2, out=y[r0:r0 + n], epi=G.EPI_GATE_RESID, resid=x1[:n], gate=g2)
+            E.modnorm_fwd(x1, sc2, sh2, wn2, mode=meta.mode, eps=meta.eps, out=h2)
+            if kept is not None:
+                G.gemm(h2, w1, out=act, epi=G.EPI_SWIGLU_BOTH, aux=kept["u"][r0:r0 + n])
+            else:
+                G.gemm(h2, w1, out=act, epi=G.EPI_SWIGLU)
+            G.gemm(act, w2, out=y[r0:r0 + n], epi=G.EPI_GATE_RESID, resid=x1, gate=g2)
     return y
 
 
 def block_backward(x: torch.Tensor, mod: torch.Tensor, dy: torch.Tensor, meta: BlockMeta, wn1, wqkv, wo, wn2, w1, w2,
-                   grads: dict[str, torch.Tensor], dx: torch.Tensor | None = None):
-    """Recompute-and-backpropagate. ``grads`` maps n1, to_qkv, wo, n2, w1, w2 to fp32 accumulators (+=).
+                   grads: dict[str, torch.Tensor], dx: torch.Tensor | None = None,
+                   kept: dict[str, torch.Tensor] | None = None):
+    """Recompute-and-backpropagate; with ``kept`` (what :func:`block_forward` stored) nothing is recomputed and ``kept`` is
+    only read. ``grads`` maps n1, to_qkv, wo, n2, w1, w2 to fp32 accumulators (+=).
     Returns (dx bf16, dmod [B, 6D] fp32). ``dx`` may alias ``dy``."""
     T, D = x.shape
     B = mod.shape[0]
@@ -255,17 +326,16 @@ def block_backward(x: torch.Tensor, mod: torch.Tensor, dy: torch.Tensor, meta: B
     HD = meta.heads * meta.head_dim
     rows_per_sample = meta.n_win_per_sample * meta.L
     ws, dev, bf, f32 = _WS, x.device, torch.bfloat16, torch.float32
-    cmax = min(meta.chunk_windows, meta.n_win_per_sample) * meta.L
-    h1 = ws.get("h", (cmax, D), bf, dev)
-    qkv = ws.get("qkv", (cmax, 3 * HD), bf, dev)
-    o = ws.get("o", (cmax, HD), bf, dev)
-    x1 = ws.get("x1", (cmax, D), bf, dev)
+    step = chunk_step(meta, D, F)
+    cmax = step * meta.L
     tp = meta.tp
     tpn = tp.tp if tp is not None else 1
-    act = ws.get("act", (cmax * tpn, F), bf, dev)
-    lse = ws.get("lse", (cmax * meta.heads,), f32, dev)
-    h2 = ws.get("h2", (cmax, D), bf, dev)
-    u = ws.get("u", (cmax * tpn, 2 * F), bf, dev)
+    if kept is None:
+        act_b = ws.get("act", (cmax * tpn, F), bf, dev)
+        chunk_bufs = {"h1": ws.get("h", (cmax, D), bf, dev), "qkv": ws.get("qkv", (cmax, 3 * HD), bf, dev),
+                      "o": ws.get("o", (cmax, HD), bf, dev), "lse": ws.get("lse", (cmax * meta.heads,), f32, dev),
+                      "x1": ws.get("x1", (cmax, D), bf, dev), "h2": ws.get("h2", (cmax, D), bf, dev), "act": act_b}
+    du_b = ws.get("u", (cmax * tpn, 2 * F), bf, dev)
     dh = ws.get("dh", (cmax, D), bf, dev)
     dx1 = ws.get("dx1", (cmax, D), bf, dev)
     d_o = ws.get("d_o", (cmax, HD), bf, dev)
@@ -285,22 +355,26 @@ def block_backward(x: torch.Tensor, mod: torch.Tensor, dy: torch.Tensor, meta: B
         dsh1, dsc1, dg1, dsh2, dsc2, dg2 = [dmod[b, i * D:(i + 1) * D] for i in range(6)]
         E.scale_rows(w2, g2, out=w2g)
         E.scale_rows(wo, g1, out=wog)
-        for w0, nw in _chunks(meta):
+        for w0, nw in _chunks(meta, step):
             r0 = b * rows_per_sample + w0 * meta.L
             n = nw * meta.L
             xc, dyc = x[r0:r0 + n], dy[r0:r0 + n]
-            lse_c = lse[:n * meta.heads].view(nw, meta.heads, meta.L)
-            # ---- recompute the chunk's forward internals
-            E.modnorm_fwd(xc, sc1, sh1, wn1, mode=meta.mode, eps=meta.eps, out=h1[:n])
-            if meta.sp is None:
-                G.gemm(h1[:n], wqkv, out=qkv[:n])
-                if meta.rope is not None:
-                    _rope_qk_(qkv[:n], meta, nw)
-                A.attn_fwd(qkv[:n], nw, meta.L, meta.heads, meta.head_dim, out=o[:n], lse=lse_c)
-                oc = o[:n]
-            else:
-                oc, sp_state = _sp_attention_fwd(meta, h1[:n], wqkv, nw, keep_local=True)
-            G.gemm(oc, wo, out=x1[:n], epi=G.EPI_GATE_RESID, resid=xc, gate=g1)
+            h1, qkv, o, x1, h2, act, lse = _chunk_views(kept, r0, n, meta.heads) if kept is not None else \
+                _chunk_views(chunk_bufs, 0, n, meta.heads)
+            lse_c = lse.view(nw, meta.heads, meta.L)
+            oc, du = o, du_b[:n]
+            u = kept["u"][r0:r0 + n] if kept is not None else du
+            if kept is None:
+                # ---- recompute the chunk's forward internals
+                E.modnorm_fwd(xc, sc1, sh1, wn1, mode=meta.mode, eps=meta.eps, out=h1)
+                if meta.sp is None:
+                    G.gemm(h1, wqkv, out=qkv)
+                    if meta.rope is not None:
+                        _rope_qk_(qkv, meta, nw)
+                    A.attn_fwd(qkv, nw, meta.L, meta.heads, meta.head_dim, out=o, lse=lse_c)
+                else:
+                    oc, sp_state = _sp_attention_fwd(meta, h1, wqkv, nw, keep_local=True)
+                G.gemm(oc, wo, out=x1, epi=G.EPI_GATE_RESID, resid=xc, gate=g1)
             if tp is not None:
                 # tensor-parallel MLP half: h2 and dy are gathered over the group inside the two GEMMs that consume
                 # them, the partial dh2 is reduced and scattered by the epilogue of the GEMM that produces it
@@ -309,30 +383,31 @@ def block_backward(x: torch.Tensor, mod: torch.Tensor, dy: torch.Tensor, meta: B
                 sl = slice(tp.rank * n, (tp.rank + 1) * n)
                 x_buf, x_peers = tp.buffer("ag_x", (Mg, D))
                 g_buf, g_peers = tp.buffer("ag_dy", (Mg, D))
-                E.modnorm_fwd(x1[:n], sc2, sh2, wn2, mode=meta.mode, eps=meta.eps, out=x_buf[sl])
+                E.modnorm_fwd(x1, sc2, sh2, wn2, mode=meta.mode, eps=meta.eps, out=x_buf[sl])
                 g_buf[sl].copy_(dyc)
                 tp.barrier()
-                TP.gemm_allgather_a(tp, x_buf, x_peers, w1, out=act[:Mg], epi=G.EPI_SWIGLU_BOTH, aux=u[:Mg])
-                TP.gemm_allgather_a(tp, g_buf, g_peers, w2g, b_t=True, out=u[:Mg], epi=G.EPI_SWIGLU_BWD, resid=u[:Mg])
-                G.gemm(g_buf, act[:Mg], a_t=True, b_t=True, out=G2, epi=G.EPI_ACC_F32, k_splits=ksplit_tok)
-                G.gemm(u[:Mg], x_buf, a_t=True, b_t=True, out=grads["w1"], epi=G.EPI_ACC_F32, k_splits=ksplit_tok)
-                TP.gemm_reduce_scatter(tp, u[:Mg], w1, b_t=True, name="rs_dx", out=dh[:n])
+                TP.gemm_allgather_a(tp, x_buf, x_peers, w1, out=act_b[:Mg], epi=G.EPI_SWIGLU_BOTH, aux=du_b[:Mg])
+                TP.gemm_allgather_a(tp, g_buf, g_peers, w2g, b_t=True, out=du_b[:Mg], epi=G.EPI_SWIGLU_BWD, resid=du_b[:Mg])
+                G.gemm(g_buf, act_b[:Mg], a_t=True, b_t=True, out=G2, epi=G.EPI_ACC_F32, k_splits=ksplit_tok)
+                G.gemm(du_b[:Mg], x_buf, a_t=True, b_t=True, out=grads["w1"], epi=G.EPI_ACC_F32, k_splits=ksplit_tok)
+                TP.gemm_reduce_scatter(tp, du_b[:Mg], w1, b_t=True, name="rs_dx", out=dh[:n])
             else:
-                E.modnorm_fwd(x1[:n], sc2, sh2, wn2, mode=meta.mode, eps=meta.eps, out=h2[:n])
-                G.gemm(h2[:n], w1, out=act[:n], epi=G.EPI_SWIGLU_BOTH, aux=u[:n])     # act and the raw [gate | up]
+                if kept is None:
+                    E.modnorm_fwd(x1, sc2, sh2, wn2, mode=meta.mode, eps=meta.eps, out=h2)
+                    G.gemm(h2, w1, out=act, epi=G.EPI_SWIGLU_BOTH, aux=u)     # act and the raw [gate | up]
                 # ---- MLP half: y = x1 + g2 * (act @ w2^T)
-                G.gemm(dyc, act[:n], a_t=True, b_t=True, out=G2, epi=G.EPI_ACC_F32, k_splits=ksplit_tok)
-                # dact = (dy * g2) @ w2 never reaches memory: the epilogue turns it into du, overwriting u
-                G.gemm(dyc, w2g, b_t=True, out=u[:n], epi=G.EPI_SWIGLU_BWD, resid=u[:n])
-                G.gemm(u[:n], w1, b_t=True, out=dh[:n])                                # dh2 = du @ w1
-                G.gemm(u[:n], h2[:n], a_t=True, b_t=True, out=grads["w1"], epi=G.EPI_ACC_F32, k_splits=ksplit_tok)
-            E.modnorm_bwd(x1[:n], dh[:n], dyc, sc2, sh2, wn2, mode=meta.mode, eps=meta.eps, dx=dx1[:n],
+                G.gemm(dyc, act, a_t=True, b_t=True, out=G2, epi=G.EPI_ACC_F32, k_splits=ksplit_tok)
+                # dact = (dy * g2) @ w2 never reaches memory: the epilogue turns it into du (over u unless that is kept)
+                G.gemm(dyc, w2g, b_t=True, out=du, epi=G.EPI_SWIGLU_BWD, resid=u)
+                G.gemm(du, w1, b_t=True, out=dh[:n])                                # dh2 = du @ w1
+                G.gemm(du, h2, a_t=True, b_t=True, out=grads["w1"], epi=G.EPI_ACC_F32, k_splits=ksplit_tok)
+            E.modnorm_bwd(x1, dh[:n], dyc, sc2, sh2, wn2, mode=meta.mode, eps=meta.eps, dx=dx1[:n],
                           dscale=dsc2, dshift=dsh2, dw=grads["n2"])
             # ---- attention half: x1 = x + g1 * (o @ wo^T)
             G.gemm(dx1[:n], oc, a_t=True, b_t=True, out=Go, epi=G.EPI_ACC_F32, k_splits=ksplit_tok)
             if meta.sp is None:
                 G.gemm(dx1[:n], wog, b_t=True, out=d_o[:n])                            # do = (dx1 * g1) @ wo
-                A.attn_bwd(qkv[:n], o[:n], d_o[:n], lse_c, nw, meta.L, meta.heads, meta.head_dim, dqkv=dqkv[:n],
+                A.attn_bwd(qkv, o, d_o[:n], lse_c, nw, meta.L, meta.heads, meta.head_dim, dqkv=dqkv[:n],
                            delta=delta[:n * meta.heads].view(nw, meta.heads, meta.L))
                 if meta.rope is not None:
                     _rope_qk_(dqkv[:n], meta, nw, inverse=True)
@@ -340,7 +415,7 @@ def block_backward(x: torch.Tensor, mod: torch.Tensor, dy: torch.Tensor, meta: B
             else:
                 dq_c = _sp_attention_bwd(meta, dx1[:n], wog, nw, sp_state)
             G.gemm(dq_c, wqkv, b_t=True, out=dh[:n])                                   # dh1 = dqkv @ wqkv
-            G.gemm(dq_c, h1[:n], a_t=True, b_t=True, out=grads["to_qkv"], epi=G.EPI_ACC_F32, k_splits=ksplit_tok)
+            G.gemm(dq_c, h1, a_t=True, b_t=True, out=grads["to_qkv"], epi=G.EPI_ACC_F32, k_splits=ksplit_tok)
             E.modnorm_bwd(xc, dh[:n], dx1[:n], sc1, sh1, wn1, mode=meta.mode, eps=meta.eps, dx=dx[r0:r0 + n],
                           dscale=dsc1, dshift=dsh1, dw=grads["n1"])
         # per-sample gate handling: dW += g * G ; dg = rowsum(W * G) ; G <- 0
@@ -355,7 +430,7 @@ def _pool_alloc(peer_fn, gradient: bool = False):
 
 
 class FusedBlock(torch.autograd.Function):
-    """Autograd wrapper: saves only the block input; weight gradients go to ``param.main_grad`` (fp32) when the
+    """Autograd wrapper: saves the block input and, with ``meta.keep``, the block's internals; weight gradients go to ``param.main_grad`` (fp32) when the
     engine provides one, otherwise they are returned to autograd."""
 
     @staticmethod
@@ -367,21 +442,27 @@ class FusedBlock(torch.autograd.Function):
         ctx.meta = meta
         ctx.regroup = regroup
         out = out_alloc(x.shape[0], x.shape[1], x.dtype) if out_alloc is not None else None
+        kept = None
+        if meta.keep:
+            shapes = _kept_shapes(regroup[0].numel() if regroup is not None else x.shape[0], x.shape[1],
+                                  meta.heads * meta.head_dim, meta.heads, w2.shape[1])
+            kept = {k: torch.empty(shape, dtype=dt, device=x.device) for k, (shape, dt) in shapes.items()}
         if regroup is not None:
             table_fwd, _, peer_fn = regroup
             peers = peer_fn(x, "fwd") if peer_fn is not None else [x.data_ptr()]
             xg = torch.empty((table_fwd.numel(), x.shape[1]), dtype=x.dtype, device=x.device)
             y = block_forward(xg, mod.float(), meta, wn1, wqkv, wo, wn2, w1, w2, out=out,
-                              gather=(table_fwd, peers, x))
+                              gather=(table_fwd, peers, x), kept=kept)
             x = xg
         else:
-            y = block_forward(x, mod.float(), meta, wn1, wqkv, wo, wn2, w1, w2, out=out)
-        ctx.save_for_backward(x, mod, wn1, wqkv, wo, wn2, w1, w2)
+            y = block_forward(x, mod.float(), meta, wn1, wqkv, wo, wn2, w1, w2, out=out, kept=kept)
+        ctx.save_for_backward(x, mod, wn1, wqkv, wo, wn2, w1, w2, *([kept[k] for k in KEPT] if kept is not None else ()))
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x, mod, wn1, wqkv, wo, wn2, w1, w2 = ctx.saved_tensors
+        x, mod, wn1, wqkv, wo, wn2, w1, w2, *rest = ctx.saved_tensors
+        kept = dict(zip(KEPT, rest)) if rest else None
         params = {"n1": wn1, "to_qkv": wqkv, "wo": wo, "n2": wn2, "w1": w1, "w2": w2}
         grads, ret = {}, {}
         for k, p in params.items():
@@ -393,7 +474,7 @@ class FusedBlock(torch.autograd.Function):
                 grads[k] = torch.zeros(p.shape, dtype=torch.float32, device=p.device)
                 ret[k] = grads[k]
         dy = dy.contiguous()
-        dx, dmod = block_backward(x, mod.float(), dy, ctx.meta, wn1, wqkv, wo, wn2, w1, w2, grads, dx=dy)
+        dx, dmod = block_backward(x, mod.float(), dy, ctx.meta, wn1, wqkv, wo, wn2, w1, w2, grads, dx=dy, kept=kept)
         if ctx.regroup is not None:
             _, table_bwd, peer_fn = ctx.regroup
             peers = peer_fn(dx, "bwd") if peer_fn is not None else [dx.data_ptr()]

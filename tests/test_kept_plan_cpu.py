@@ -1,0 +1,31 @@
+"""How many blocks keep their internals for the backward pass, and how small a chunk may get."""
+import pytest
+
+from aeris_gb_b200.models import fused
+from aeris_gb_b200.ops import elementwise as E
+
+
+@pytest.mark.parametrize("free,want", [(100 << 30, 10), (30 << 30, 5), (11 << 30, 0), (5 << 30, 0), (12 << 30, 0)])
+def test_kept_blocks_take_at_most_half_of_the_free_memory(free, want):
+    # 10 blocks of 2 GiB next to 10 GiB that the step needs anyway
+    n = fused.n_kept(10, 2 << 30, 10 << 30, free)
+    assert n == want and n * (2 << 30) <= max(0, free - (10 << 30)) / 2
+
+
+def test_a_block_keeps_every_recomputed_internal():
+    per_row = 3 * 1536 * 2 + 4 * 1536 * 2 + 3 * 4096 * 2 + 24 * 4        # h1, x1, h2 | qkv, o | act, u | lse
+    assert fused.kept_bytes(1000, 1536, 1536, 24, 4096) == 1000 * per_row
+    assert set(fused._kept_shapes(8, 16, 16, 2, 32)) == set(fused.KEPT)
+
+
+@pytest.mark.parametrize("dim,heads,mlp,L,chunk,n_win,want", [
+    (1536, 24, 4096, 900, 72, 288, 72),       # the caller's bound holds where a chunk is large
+    (1536, 24, 4096, 900, 4, 288, 12),        # 512 MiB of internals: 12 windows
+    (128, 4, 256, 64, 8, 32, 32),             # a toy sample is one chunk
+    (5120, 40, 13696, 900, 72, 32, 32)])
+def test_chunks_below_half_a_gigabyte_are_merged(dim, heads, mlp, L, chunk, n_win, want):
+    meta = fused.BlockMeta(n_win, L, heads, dim // heads, E.MODE_MOD_THEN_NORM, 1e-6, chunk)
+    step = fused.chunk_step(meta, dim, mlp)
+    assert step == want
+    spans = list(fused._chunks(meta, step))
+    assert sum(n for _, n in spans) == n_win and [w for w, _ in spans] == list(range(0, n_win, step))

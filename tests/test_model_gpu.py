@@ -148,3 +148,38 @@ def test_train_step_raises_on_a_device_timeout_instead_of_stepping():
     assert all(float(g.abs().max()) == 0.0 for g in tr.opt.grad_buffers())
     loss = tr.train_step(x, c)              # status cleared, gradients dropped: the next step runs normally
     assert loss == loss and tr.opt.step_count == steps + 1
+
+
+@pytest.mark.parametrize("mod_first", [True, False])
+def test_kept_internals_give_the_gradients_of_the_recompute(mod_first, monkeypatch):
+    """A block that keeps its internals and one that recomputes them launch the same kernels on the same values: equal
+    outputs, and gradients equal up to the order of the fp32 atomic sums. What is kept must survive a backward pass (the
+    gated product is written beside it, not over it): a second one over the retained graph gives the same."""
+    from aeris_gb_b200.models import fused
+    from aeris_gb_b200.models.aeris import AerisConfig, AerisModel
+    cfg = AerisConfig(img=(30, 60), window=(15, 15), in_channels=20, out_channels=8, dim=256, heads=4, head_dim=64,
+                      mlp_dim=512, n_layers=2, sublayers=2, after_mod_norm=mod_first, chunk_windows=3)
+    monkeypatch.setattr(fused, "MIN_CHUNK_BYTES", 1)          # three-window chunks: 8 windows leave a remainder
+    torch.manual_seed(3)
+    model = AerisModel(cfg).cuda()
+    for p in model.parameters():
+        torch.nn.init.normal_(p, std=0.05)
+    x = torch.randn(2, 30, 60, 20, device="cuda")
+    t = torch.tensor([0.4, 1.1], device="cuda")
+    n_blocks, runs = 4, {}
+    for keep in (0, 3, n_blocks):
+        monkeypatch.setattr(fused, "plan_kept_blocks", lambda *a, keep=keep: keep)
+        model.zero_grad(set_to_none=True)
+        y = model(x, t)
+        loss = (y * torch.linspace(-1, 1, y.numel(), device="cuda").view_as(y)).sum()
+        loss.backward(retain_graph=True)
+        first = {n: p.grad.float().clone() for n, p in model.named_parameters() if p.grad is not None}
+        model.zero_grad(set_to_none=True)
+        loss.backward()
+        runs[keep] = (y.detach(), first, {n: p.grad.float().clone() for n, p in model.named_parameters() if p.grad is not None})
+    for keep in (3, n_blocks):
+        assert torch.equal(runs[keep][0], runs[0][0])
+        for got in runs[keep][1:]:
+            for n, g in runs[0][1].items():
+                # bf16 gradients of bf16 weights: an atomic sum in another order may round to the neighbouring value
+                assert rel_err(got[n], g) < 2.0 ** -9, n
