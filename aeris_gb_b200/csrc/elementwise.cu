@@ -100,12 +100,14 @@ __device__ __forceinline__ void block_sum(float (&v)[NRED], float* red, int pari
   }
 }
 
-// Block-wide sums of FOUR values per thread for CTAs of at most eight warps, built for few instructions: inside a warp
-// the four values are folded by halving (lanes that differ in bit 4 split the values two and two, lanes that differ in
-// bit 3 one and one: 6 shuffles instead of 20), the four lane groups write value k of warp w to slot k * 8 + w, and
-// after one __syncthreads every lane sums one slot row with three more shuffles and fetches the four totals.
-// `red`: [2][32] floats zeroed at kernel start (slots of absent warps stay zero), double buffered by `parity`.
-__device__ __forceinline__ void block_sum4_shfl(float (&s)[4], float (*red)[32], int parity, int lane, int warp) {
+// Sums of FOUR values per thread over a GROUP of `nt` threads (at most 8 * W8 whole warps; a CTA may hold several groups),
+// built for few instructions: inside a warp the four values are folded by halving (lanes that differ in bit 4 split the
+// values two and two, lanes that differ in bit 3 one and one: 6 shuffles instead of 20), the four lane groups write value
+// k of warp w to slot 8 W8 k + w, and after one barrier every lane adds W8 slots and fetches the totals with seven
+// shuffles. `bar` is the group's named barrier (0: the whole CTA), `red` its 32 * W8 floats of this parity, zeroed at kernel
+// start (slots of absent warps stay zero) and double buffered by the caller.
+template <int W8>
+__device__ __forceinline__ void group_sum4(float (&s)[4], float* red, int lane, int warp, int bar, int nt) {
   const bool b4 = lane & 16, b3 = lane & 8;
   float a0 = b4 ? s[2] : s[0], a1 = b4 ? s[3] : s[1];
   const float g0 = b4 ? s[0] : s[2], g1 = b4 ? s[1] : s[3];
@@ -117,14 +119,19 @@ __device__ __forceinline__ void block_sum4_shfl(float (&s)[4], float (*red)[32],
   c += __shfl_xor_sync(0xffffffffu, c, 4);
   c += __shfl_xor_sync(0xffffffffu, c, 2);
   c += __shfl_xor_sync(0xffffffffu, c, 1);
-  if ((lane & 7) == 0) red[parity][(lane >> 3) * 8 + warp] = c;      // value index = 2 * bit4 + bit3 = lane >> 3
-  __syncthreads();
-  float t = red[parity][lane];
-  t += __shfl_xor_sync(0xffffffffu, t, 4);
-  t += __shfl_xor_sync(0xffffffffu, t, 2);
-  t += __shfl_xor_sync(0xffffffffu, t, 1);
+  if (nt > 32) {
+    float* slot = red + (lane >> 3) * 8 * W8;                   // value index = 2 * bit4 + bit3 = lane >> 3
+    if ((lane & 7) == 0) slot[warp] = c;
+    asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(nt) : "memory");
+    c = slot[lane & 7];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) s[j] = __shfl_sync(0xffffffffu, t, j * 8);
+    for (int i = 1; i < W8; ++i) c += slot[8 * i + (lane & 7)];
+    c += __shfl_xor_sync(0xffffffffu, c, 4);
+    c += __shfl_xor_sync(0xffffffffu, c, 2);
+    c += __shfl_xor_sync(0xffffffffu, c, 1);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) s[j] = __shfl_sync(0xffffffffu, c, j * 8);
 }
 
 // ------------------------------------------------------------------------------------------------ modulate + RMSNorm
@@ -231,20 +238,23 @@ __global__ void modnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const ui
   }
 }
 
-// The same forward for rows of up to 1536 columns (at most six warps), written for the instruction issue rate: the kernel
-// above executes 20.6 warp instructions per element and keeps the schedulers 64 % busy with no memory stall to speak
-// of. Here every per-element operation works on a column pair (`*.f32x2`), 1 + scale is formed once, the row mean uses
-// a multiplication, and the four rows' sums go through block_sum4_shfl.
-__global__ void __launch_bounds__(192, 3)
+// The same forward for rows of up to 5120 columns, written for the instruction issue rate: the kernel above executes 20.6
+// warp instructions per element and keeps the schedulers 64 % busy with no memory stall to speak of. Here every
+// per-element operation works on a column pair (`*.f32x2`), 1 + scale is formed once, the row mean uses a multiplication,
+// and the four rows' sums go through group_sum4. Rows of up to 1536 columns: three CTAs of at most six warps per SM
+// at their widest; up to 2560 two CTAs of at most ten; wider ones: one
+// CTA of up to twenty warps (28800 x 5120: 165 -> 98 us, 6.0 TB/s).
+template <int MAXT, int MINB, int W8>
+__global__ void __launch_bounds__(MAXT, MINB)
 modnorm_fwd_pair_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __restrict__ gidx, PeerPtrs peers,
                         __nv_bfloat16* __restrict__ x_out, const float* __restrict__ scale,
                         const float* __restrict__ shift, const __nv_bfloat16* __restrict__ w,
                         __nv_bfloat16* __restrict__ h, int rows, int D, int mode, float eps,
                         const float* __restrict__ wf, __nv_bfloat16* __restrict__ h_lo) {
-  static_assert(FWD_RPI == 4, "block_sum4_shfl reduces four values");
-  __shared__ float red[2][32];
+  static_assert(FWD_RPI == 4 && MAXT <= 256 * W8, "group_sum4 adds four values of at most 8 * W8 warps");
+  __shared__ float red[2][32 * W8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < 64; i += blockDim.x) (&red[0][0])[i] = 0.f;
+  for (int i = threadIdx.x; i < 64 * W8; i += blockDim.x) (&red[0][0])[i] = 0.f;
   const int c0 = threadIdx.x * 8;
   const bool active = c0 < D;
   uint64_t sc1[4], sh[4], wv[4];
@@ -315,7 +325,7 @@ modnorm_fwd_pair_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __r
       f2_unpack(p, p0, p1);
       ss[k] = live ? p0 + p1 : 0.f;
     }
-    block_sum4_shfl(ss, red, parity, lane, warp);
+    group_sum4<W8>(ss, red[parity], lane, warp, 0, blockDim.x);
 #pragma unroll
     for (int k = 0; k < FWD_RPI; ++k) {
       const int rr = r + k;
@@ -344,19 +354,15 @@ modnorm_fwd_pair_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __r
 
 // Backward of the above. dx = dres + d(norm path). Column sums are kept in registers over the CTA's rows and
 // flushed with atomics at the end: dscale, dshift (fp32 [D], one modulation vector per launch) and dw (fp32 [D]).
-// MAXT / MINB: launch bounds by row width: up to 1536 columns 192 threads and two CTAs per SM (three were measured slower: spills), up to 5120 columns
-// 640 threads, wider rows 1024 threads (register cap 64: spills, but it launches).
-template <int MAXT, int MINB, int RPI>
-__global__ void __launch_bounds__(MAXT, MINB)
+// Serves rows wider than 5120 columns (1024 threads, register cap 64: spills, but it launches).
+__global__ void __launch_bounds__(1024, 1)
 modnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dh,
                                    const __nv_bfloat16* __restrict__ dres, const float* __restrict__ scale,
                                    const float* __restrict__ shift, const __nv_bfloat16* __restrict__ w,
                                    __nv_bfloat16* __restrict__ dx, float* __restrict__ dscale,
                                    float* __restrict__ dshift, float* __restrict__ dw, int rows, int D, int mode,
-                                   float eps, int rows_per_cta, const float* __restrict__ wf) {
-  // RPI rows per iteration share one block-wide reduction, and the next RPI rows are requested before it: with
-  // RPI = 2 every thread keeps 12 sixteen-byte loads in flight (one row at a time left the memory system idle
-  // during the reduction)
+                                   float eps, const float* __restrict__ wf) {
+  constexpr int RPI = 1;
   __shared__ float red[2 * 2 * RPI * 32];
   const int c0 = threadIdx.x * 8;
   const bool active = c0 < D;
@@ -368,7 +374,6 @@ modnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
     if (shift) loadf8(shift + c0, sh);
     if (wf) loadf8(wf + c0, wv); else load8(w + c0, wv);
   }
-  (void)rows_per_cta;
   const int r1 = rows;
   const int stride = gridDim.x * RPI;
   int parity = 0;
@@ -477,174 +482,222 @@ modnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   }
 }
 
-// The same backward for rows of up to 1536 columns (at most six warps per row), cut down to what the instruction
-// issue rate allows: the one-row-at-a-time kernel above executed about 42 warp instructions per element and kept the
-// schedulers 53 % busy with three resident warps each, i.e. it was bound by instruction issue, not by memory.
-//   * every per-element operation works on a pair of columns (`*.f32x2`, half the issue slots);
-//   * two rows share one block-wide reduction, whose cross-warp part is one shared-memory load and seven shuffles per
-//     thread (lane k * 8 + w holds value k of warp w) instead of 24 loads and adds;
-//   * 1 + scale is formed once per thread.
-template <int RPI, int MINB>
-__global__ void __launch_bounds__(192, MINB)
-modnorm_bwd_pair_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dh,
-                        const __nv_bfloat16* __restrict__ dres, const float* __restrict__ scale,
-                        const float* __restrict__ shift, const __nv_bfloat16* __restrict__ w,
-                        __nv_bfloat16* __restrict__ dx, float* __restrict__ dscale, float* __restrict__ dshift,
-                        float* __restrict__ dw, int rows, int D, int mode, float eps, const float* __restrict__ wf) {
-  constexpr int NV = 2 * RPI;                    // values to reduce per iteration
-  constexpr int NL = (NV * 8 + 31) / 32;         // slot k * 8 + w holds value k of warp w; a lane sums NL of them
-  __shared__ float red[2][NL * 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < 2 * NL * 32; i += blockDim.x) (&red[0][0])[i] = 0.f;   // slots of absent warps stay zero
-  const int c0 = threadIdx.x * 8;
-  const bool active = c0 < D;
-  uint64_t sc1[4], sh[4], wv[4], a_sc[4], a_sh[4], a_w[4];
-  {
+// The same backward for rows of up to 5120 columns, built for few instructions and few atomics.
+//   * Every per-element operation works on a pair of columns (`*.f32x2`, half the issue slots); a thread owns VPT vectors of
+//     eight columns, RPI rows share one reduction, and the next RPI rows are requested before it.
+//   * A row is worked on by a GROUP of nt threads (D / (8 VPT), whole warps) with a named barrier of its own; a CTA holds as
+//     many groups as fit MAXT threads and there is one CTA per SM. The column sums of all groups meet in shared memory
+//     once, at the end, so every column gets 148 vector reductions per launch instead of one scalar atomic from each of
+//     1,184 single-group CTAs, which took most of the time on narrow rows.
+//   * VPT = 2 (rows wider than 1536) halves the threads that a row's sum has to cross and reads scale, shift and weight
+//     from shared memory; one row per reduction is what the registers hold then (two spilled).
+// Before and now: 28800 x 512 columns 110 -> 26 us, 28800 x 768 117 -> 37 us, 64800 x 1536 203 -> 142 us (5.6 TB/s),
+// 28800 x 5120 500 -> 330 us.
+template <int VPT, int RPI, int MAXT>
+__global__ void __launch_bounds__(MAXT, 1)
+modnorm_bwd_group_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dh,
+                         const __nv_bfloat16* __restrict__ dres, const float* __restrict__ scale,
+                         const float* __restrict__ shift, const __nv_bfloat16* __restrict__ w,
+                         __nv_bfloat16* __restrict__ dx, float* __restrict__ dscale, float* __restrict__ dshift,
+                         float* __restrict__ dw, int rows, int D, int mode, float eps, const float* __restrict__ wf, int nt,
+                         int vec_atomics) {
+  static_assert(RPI <= 2, "group_sum4 adds two values of two rows");
+  constexpr bool PSMEM = VPT > 1;
+  extern __shared__ __align__(16) float sm[];    // [groups][3][D] column sums; with PSMEM first [3][D]: 1 + scale, shift, weight
+  __shared__ float red[MAXT / 32][2][64];
+  const int groups = blockDim.x / nt;
+  const int grp = threadIdx.x / nt, tid = threadIdx.x - grp * nt;
+  const int lane = threadIdx.x & 31, warp = tid >> 5;
+  for (int i = threadIdx.x; i < (MAXT / 32) * 2 * 64; i += blockDim.x) (&red[0][0][0])[i] = 0.f;   // absent warps stay zero
+  int col[VPT];
+  bool act[VPT];
+  uint64_t p_sc[VPT][4], p_sh[VPT][4], p_w[VPT][4], a_sc[VPT][4], a_sh[VPT][4], a_w[VPT][4];
+#pragma unroll
+  for (int q = 0; q < VPT; ++q) {
+    col[q] = (q * nt + tid) * 8;
+    act[q] = col[q] < D;
     float t_sc[8], t_sh[8], t_w[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) { t_sc[i] = 0.f; t_sh[i] = 0.f; t_w[i] = 0.f; }
-    if (active) {
-      if (scale) loadf8(scale + c0, t_sc);
-      if (shift) loadf8(shift + c0, t_sh);
-      if (wf) loadf8(wf + c0, t_w); else load8(w + c0, t_w);
+    if (act[q] && (!PSMEM || grp == 0)) {
+      if (scale) loadf8(scale + col[q], t_sc);
+      if (shift) loadf8(shift + col[q], t_sh);
+      if (wf) loadf8(wf + col[q], t_w); else load8(w + col[q], t_w);
+    }
+    if (PSMEM) {
+      if (act[q] && grp == 0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          sm[col[q] + i] = 1.f + t_sc[i];
+          sm[D + col[q] + i] = t_sh[i];
+          sm[2 * D + col[q] + i] = t_w[i];
+        }
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        p_sc[q][i] = f2_pack(1.f + t_sc[2 * i], 1.f + t_sc[2 * i + 1]);
+        p_sh[q][i] = f2_pack(t_sh[2 * i], t_sh[2 * i + 1]);
+        p_w[q][i] = f2_pack(t_w[2 * i], t_w[2 * i + 1]);
+      }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      sc1[i] = f2_pack(1.f + t_sc[2 * i], 1.f + t_sc[2 * i + 1]);
-      sh[i] = f2_pack(t_sh[2 * i], t_sh[2 * i + 1]);
-      wv[i] = f2_pack(t_w[2 * i], t_w[2 * i + 1]);
-      a_sc[i] = a_sh[i] = a_w[i] = 0ull;
-    }
+    for (int i = 0; i < 4; ++i) a_sc[q][i] = a_sh[q][i] = a_w[q][i] = 0ull;
   }
   __syncthreads();
-  const int r1 = rows;
-  const int gstep = gridDim.x;
+  // the three parameter vectors of column vector q: from shared memory (VPT > 1) or the registers filled above
+  auto params = [&](int q) {
+    if constexpr (PSMEM) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int c = act[q] ? col[q] + 4 * h : 0;
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(sm + c);
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(sm + D + c);
+        const ulonglong2 e = *reinterpret_cast<const ulonglong2*>(sm + 2 * D + c);
+        p_sc[q][2 * h] = a.x; p_sc[q][2 * h + 1] = a.y;
+        p_sh[q][2 * h] = b.x; p_sh[q][2 * h + 1] = b.y;
+        p_w[q][2 * h] = e.x; p_w[q][2 * h + 1] = e.y;
+      }
+    }
+  };
+  const int gstep = gridDim.x * groups;            // groups of the whole grid; each takes every gstep-th row
   const int stride = gstep * RPI;
   const float inv_d = 1.f / D;
   int parity = 0;
-  uint4 nx[RPI], ng[RPI], nr[RPI];
+  uint4 nx[RPI][VPT], ng[RPI][VPT], nr[RPI][VPT];
 #pragma unroll
-  for (int k = 0; k < RPI; ++k) nx[k] = ng[k] = nr[k] = make_uint4(0u, 0u, 0u, 0u);
+  for (int k = 0; k < RPI; ++k)
+#pragma unroll
+    for (int q = 0; q < VPT; ++q) nx[k][q] = ng[k][q] = nr[k][q] = make_uint4(0u, 0u, 0u, 0u);
   auto fetch = [&](int base) {
 #pragma unroll
     for (int k = 0; k < RPI; ++k) {
       const int r = base + k * gstep;
-      if (active && r < r1) {
-        const size_t off = static_cast<size_t>(r) * D + c0;
-        nx[k] = *reinterpret_cast<const uint4*>(x + off);
-        ng[k] = *reinterpret_cast<const uint4*>(dh + off);
-        if (dres) nr[k] = *reinterpret_cast<const uint4*>(dres + off);
+#pragma unroll
+      for (int q = 0; q < VPT; ++q) {
+        if (act[q] && r < rows) {
+          const size_t off = static_cast<size_t>(r) * D + col[q];
+          nx[k][q] = *reinterpret_cast<const uint4*>(x + off);
+          ng[k][q] = *reinterpret_cast<const uint4*>(dh + off);
+          if (dres) nr[k][q] = *reinterpret_cast<const uint4*>(dres + off);
+        }
       }
     }
   };
-  fetch(blockIdx.x);
-  for (int base = blockIdx.x; base < r1; base += stride, parity ^= 1) {
-    uint64_t v[RPI][4], g[RPI][4];
-    uint4 dr[RPI];
+  const int first = blockIdx.x * groups + grp;
+  if (first < rows) fetch(first);
+  for (int base = first; base < rows; base += stride, parity ^= 1) {
+    uint4 cx[RPI][VPT], cg[RPI][VPT], cr[RPI][VPT];
 #pragma unroll
-    for (int k = 0; k < RPI; ++k) {
-      const uint32_t xw[4] = {nx[k].x, nx[k].y, nx[k].z, nx[k].w}, gw[4] = {ng[k].x, ng[k].y, ng[k].z, ng[k].w};
+    for (int k = 0; k < RPI; ++k)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        v[k][i] = f2_from_bf16x2(xw[i]);
-        g[k][i] = f2_from_bf16x2(gw[i]);
-      }
-      dr[k] = nr[k];
-    }
-    if (base + stride < r1) fetch(base + stride);
+      for (int q = 0; q < VPT; ++q) { cx[k][q] = nx[k][q]; cg[k][q] = ng[k][q]; cr[k][q] = nr[k][q]; }
+    if (base + stride < rows) fetch(base + stride);
     // ---- the two row sums of each row: mode 0  sum y^2, sum y (g w);  mode 1  sum x^2, sum x (g (1 + sc) w)
-    float s[2 * RPI];
+    uint64_t p0[RPI], p1[RPI];
+#pragma unroll
+    for (int k = 0; k < RPI; ++k) p0[k] = p1[k] = 0ull;
+#pragma unroll
+    for (int q = 0; q < VPT; ++q) {
+      params(q);
+#pragma unroll
+      for (int k = 0; k < RPI; ++k) {
+        const uint32_t xw[4] = {cx[k][q].x, cx[k][q].y, cx[k][q].z, cx[k][q].w};
+        const uint32_t gw[4] = {cg[k][q].x, cg[k][q].y, cg[k][q].z, cg[k][q].w};
+        const bool live = act[q] && base + k * gstep < rows;
+        uint64_t s0 = 0ull, s1 = 0ull;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint64_t v = f2_from_bf16x2(xw[i]), g = f2_from_bf16x2(gw[i]);
+          if (mode == 0) {
+            const uint64_t y = f2_fma(v, p_sc[q][i], p_sh[q][i]);
+            s0 = f2_fma(y, y, s0);
+            s1 = f2_fma(y, f2_mul(g, p_w[q][i]), s1);
+          } else {
+            s0 = f2_fma(v, v, s0);
+            s1 = f2_fma(v, f2_mul(f2_mul(g, p_sc[q][i]), p_w[q][i]), s1);
+          }
+        }
+        if (live) { p0[k] = f2_add(p0[k], s0); p1[k] = f2_add(p1[k], s1); }
+      }
+    }
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int k = 0; k < RPI; ++k) {
-      uint64_t p0 = 0ull, p1 = 0ull;
-      if (mode == 0) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint64_t y = f2_fma(v[k][i], sc1[i], sh[i]);
-          p0 = f2_fma(y, y, p0);
-          p1 = f2_fma(y, f2_mul(g[k][i], wv[i]), p1);
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          p0 = f2_fma(v[k][i], v[k][i], p0);
-          p1 = f2_fma(v[k][i], f2_mul(f2_mul(g[k][i], sc1[i]), wv[i]), p1);
-        }
-      }
-      float a0, a1, b0, b1;
-      f2_unpack(p0, a0, a1);
-      f2_unpack(p1, b0, b1);
-      const bool live = active && base + k * gstep < r1;
-      s[2 * k] = live ? a0 + a1 : 0.f;
-      s[2 * k + 1] = live ? b0 + b1 : 0.f;
+      float lo, hi;
+      f2_unpack(p0[k], lo, hi);
+      s[2 * k] = lo + hi;
+      f2_unpack(p1[k], lo, hi);
+      s[2 * k + 1] = lo + hi;
     }
-    // ---- block-wide sums
-    if constexpr (RPI == 2) {
-      block_sum4_shfl(s, red, parity, lane, warp);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 2 * RPI; ++j) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
-      }
-      if (lane == 0) {
-#pragma unroll
-        for (int j = 0; j < 2 * RPI; ++j) red[parity][j * 8 + warp] = s[j];
-      }
-      __syncthreads();
-      float t[NL];
-#pragma unroll
-      for (int q = 0; q < NL; ++q) {
-        t[q] = red[parity][q * 32 + lane];
-        t[q] += __shfl_xor_sync(0xffffffffu, t[q], 4);
-        t[q] += __shfl_xor_sync(0xffffffffu, t[q], 2);
-        t[q] += __shfl_xor_sync(0xffffffffu, t[q], 1);
-      }
-#pragma unroll
-      for (int j = 0; j < NV; ++j) s[j] = __shfl_sync(0xffffffffu, t[j / 4], (j % 4) * 8);
-    }
+    group_sum4<2>(s, red[grp][parity], lane, warp, grp + 1, nt);
     // ---- gradients
 #pragma unroll
-    for (int k = 0; k < RPI; ++k) {
-      const int r = base + k * gstep;
-      if (!active || r >= r1) continue;
-      const float rinv = rsqrtf(s[2 * k] * inv_d + eps);
-      const float ncoef = -rinv * rinv * rinv * (s[2 * k + 1] * inv_d);
-      const uint64_t rinv2 = f2_pack(rinv, rinv), ncoef2 = f2_pack(ncoef, ncoef);
-      const uint32_t dw4[4] = {dr[k].x, dr[k].y, dr[k].z, dr[k].w};
-      uint32_t ow[4];
-      if (mode == 0) {
+    for (int q = 0; q < VPT; ++q) {
+      params(q);
+#pragma unroll
+      for (int k = 0; k < RPI; ++k) {
+        const int r = base + k * gstep;
+        if (!act[q] || r >= rows) continue;
+        const float rinv = rsqrtf(s[2 * k] * inv_d + eps);
+        const float ncoef = -rinv * rinv * rinv * (s[2 * k + 1] * inv_d);
+        const uint64_t rinv2 = f2_pack(rinv, rinv), ncoef2 = f2_pack(ncoef, ncoef);
+        const uint32_t xw[4] = {cx[k][q].x, cx[k][q].y, cx[k][q].z, cx[k][q].w};
+        const uint32_t gw[4] = {cg[k][q].x, cg[k][q].y, cg[k][q].z, cg[k][q].w};
+        const uint32_t dw4[4] = {cr[k][q].x, cr[k][q].y, cr[k][q].z, cr[k][q].w};
+        uint32_t ow[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const uint64_t y = f2_fma(v[k][i], sc1[i], sh[i]);
-          const uint64_t dy = f2_fma(ncoef2, y, f2_mul(rinv2, f2_mul(g[k][i], wv[i])));
-          a_w[i] = f2_fma(f2_mul(g[k][i], y), rinv2, a_w[i]);
-          a_sc[i] = f2_fma(dy, v[k][i], a_sc[i]);
-          a_sh[i] = f2_add(a_sh[i], dy);
-          ow[i] = f2_to_bf16x2(f2_fma(dy, sc1[i], f2_from_bf16x2(dw4[i])));
+          const uint64_t v = f2_from_bf16x2(xw[i]), g = f2_from_bf16x2(gw[i]);
+          if (mode == 0) {
+            const uint64_t y = f2_fma(v, p_sc[q][i], p_sh[q][i]);
+            const uint64_t dy = f2_fma(ncoef2, y, f2_mul(rinv2, f2_mul(g, p_w[q][i])));
+            a_w[q][i] = f2_fma(f2_mul(g, y), rinv2, a_w[q][i]);
+            a_sc[q][i] = f2_fma(dy, v, a_sc[q][i]);
+            a_sh[q][i] = f2_add(a_sh[q][i], dy);
+            ow[i] = f2_to_bf16x2(f2_fma(dy, p_sc[q][i], f2_from_bf16x2(dw4[i])));
+          } else {
+            const uint64_t n = f2_mul(v, rinv2);
+            const uint64_t dhn = f2_mul(g, p_sc[q][i]);
+            a_sc[q][i] = f2_fma(f2_mul(g, n), p_w[q][i], a_sc[q][i]);
+            a_sh[q][i] = f2_add(a_sh[q][i], g);
+            a_w[q][i] = f2_fma(dhn, n, a_w[q][i]);
+            const uint64_t t2 = f2_fma(rinv2, f2_mul(dhn, p_w[q][i]), f2_from_bf16x2(dw4[i]));
+            ow[i] = f2_to_bf16x2(f2_fma(ncoef2, v, t2));
+          }
         }
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint64_t n = f2_mul(v[k][i], rinv2);
-          const uint64_t dhn = f2_mul(g[k][i], sc1[i]);
-          a_sc[i] = f2_fma(f2_mul(g[k][i], n), wv[i], a_sc[i]);
-          a_sh[i] = f2_add(a_sh[i], g[k][i]);
-          a_w[i] = f2_fma(dhn, n, a_w[i]);
-          const uint64_t t2 = f2_fma(rinv2, f2_mul(dhn, wv[i]), f2_from_bf16x2(dw4[i]));
-          ow[i] = f2_to_bf16x2(f2_fma(ncoef2, v[k][i], t2));
-        }
+        *reinterpret_cast<uint4*>(dx + static_cast<size_t>(r) * D + col[q]) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
       }
-      *reinterpret_cast<uint4*>(dx + static_cast<size_t>(r) * D + c0) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
     }
   }
-  if (active) {
+  // ---- column sums: [group][3][D] in shared memory, added up and handed to memory by the whole CTA
+  float* part = sm + (PSMEM ? 3 * D : 0);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float lo, hi;
-      if (dscale) { f2_unpack(a_sc[i], lo, hi); atomicAdd(dscale + c0 + 2 * i, lo); atomicAdd(dscale + c0 + 2 * i + 1, hi); }
-      if (dshift) { f2_unpack(a_sh[i], lo, hi); atomicAdd(dshift + c0 + 2 * i, lo); atomicAdd(dshift + c0 + 2 * i + 1, hi); }
-      if (dw) { f2_unpack(a_w[i], lo, hi); atomicAdd(dw + c0 + 2 * i, lo); atomicAdd(dw + c0 + 2 * i + 1, hi); }
+  for (int q = 0; q < VPT; ++q) {
+    if (!act[q]) continue;
+    float* t = part + static_cast<size_t>(grp) * 3 * D + col[q];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      *reinterpret_cast<ulonglong2*>(t + 4 * h) = make_ulonglong2(a_sc[q][2 * h], a_sc[q][2 * h + 1]);
+      *reinterpret_cast<ulonglong2*>(t + D + 4 * h) = make_ulonglong2(a_sh[q][2 * h], a_sh[q][2 * h + 1]);
+      *reinterpret_cast<ulonglong2*>(t + 2 * D + 4 * h) = make_ulonglong2(a_w[q][2 * h], a_w[q][2 * h + 1]);
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x * 4; i < 3 * D; i += blockDim.x * 4) {
+    float4 v = *reinterpret_cast<const float4*>(part + i);
+    for (int g = 1; g < groups; ++g) {
+      const float4 u = *reinterpret_cast<const float4*>(part + static_cast<size_t>(g) * 3 * D + i);
+      v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+    }
+    const int which = i / D, c = i - which * D;          // D is a multiple of 8: the four columns share one target
+    float* dst = which == 0 ? dscale : which == 1 ? dshift : dw;
+    if (!dst) continue;
+    dst += c;
+    if (vec_atomics) {
+      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+    } else {
+      atomicAdd(dst, v.x); atomicAdd(dst + 1, v.y); atomicAdd(dst + 2, v.z); atomicAdd(dst + 3, v.w);
     }
   }
 }
@@ -942,14 +995,19 @@ extern "C" int aeris_modnorm_fwd(const void* x, const void* gidx, const void* co
   AERIS_FILL_CHECK(pp, n_peers);
   const int rpc = pick_rows_per_cta(rows);
   int grid = (rows + FWD_RPI - 1) / FWD_RPI;
-  if (grid > aeris_num_sms() * 8) grid = aeris_num_sms() * 8;
-  if (row_threads(D) <= 192) {
-    modnorm_fwd_pair_kernel<<<grid, row_threads(D), 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  if (D <= 5120) {
+    // as many CTAs as the registers of an SM hold at once, each sweeping over the rows
+    const int nt = row_threads(D), per_sm = nt > 320 ? 1 : nt > 192 ? 2 : 576 / nt;
+    if (grid > aeris_num_sms() * per_sm) grid = aeris_num_sms() * per_sm;
+    auto kern = nt <= 192 ? modnorm_fwd_pair_kernel<192, 3, 1>
+              : nt <= 320 ? modnorm_fwd_pair_kernel<320, 2, 2> : modnorm_fwd_pair_kernel<640, 1, 3>;
+    kern<<<grid, nt, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
         reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const uint32_t*>(gidx), pp,
         reinterpret_cast<__nv_bfloat16*>(x_out), scale, shift, reinterpret_cast<const __nv_bfloat16*>(w),
         reinterpret_cast<__nv_bfloat16*>(h), rows, D, mode, eps, w_f32, reinterpret_cast<__nv_bfloat16*>(h_lo));
     return cudaGetLastError() == cudaSuccess ? 0 : -21;
   }
+  if (grid > aeris_num_sms() * 8) grid = aeris_num_sms() * 8;
   modnorm_fwd_kernel<<<grid, row_threads(D), 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const uint32_t*>(gidx), pp,
       reinterpret_cast<__nv_bfloat16*>(x_out), scale, shift, reinterpret_cast<const __nv_bfloat16*>(w),
@@ -961,24 +1019,31 @@ extern "C" int aeris_modnorm_bwd(const void* x, const void* dh, const void* dres
                                  const float* shift, const void* w, void* dx, float* dscale, float* dshift,
                                  float* dw, int rows, int D, int mode, float eps, const float* w_f32, void* stream) {
   if (D % 8 || D > 8192 || rows <= 0 || (!w && !w_f32)) return -1;
+  if (D <= 5120) {
+    // one group of nt threads per row; CTAs of at most 384 (320) threads, one per SM
+    const int vpt = D <= 1536 ? 1 : 2, maxt = vpt == 1 ? 384 : 320;
+    const int nt = (D / 8 + vpt * 32 - 1) / (vpt * 32) * 32;
+    const int groups = maxt / nt;
+    const int smem = (groups + (vpt > 1 ? 1 : 0)) * 3 * D * 4;
+    const int need = (rows + groups - 1) / groups;
+    const int grid = need < aeris_num_sms() ? need : aeris_num_sms();
+    const int vec = ((reinterpret_cast<uintptr_t>(dscale) | reinterpret_cast<uintptr_t>(dshift) | reinterpret_cast<uintptr_t>(dw)) & 15) == 0;
+    auto kern = vpt == 1 ? modnorm_bwd_group_kernel<1, 2, 384> : modnorm_bwd_group_kernel<2, 1, 320>;
+    if (smem > 32 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess)
+      return -20;
+    kern<<<grid, groups * nt, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
+        reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(dh),
+        reinterpret_cast<const __nv_bfloat16*>(dres), scale, shift, reinterpret_cast<const __nv_bfloat16*>(w),
+        reinterpret_cast<__nv_bfloat16*>(dx), dscale, dshift, dw, rows, D, mode, eps, w_f32, nt, vec);
+    return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  }
   int rpc = pick_rows_per_cta(rows);
   if (rpc < 16) rpc = rows < 16 ? rows : 16;  // amortise the atomic flush of the column sums
   const int grid = (rows + rpc - 1) / rpc;    // every CTA takes about rpc rows, interleaved with the others
-  const int nt = row_threads(D);
-  if (nt <= 192) {
-    // two rows per reduction and two CTAs per SM measured best (0.381 ms for 129600 x 1536; one row and three CTAs
-    // 0.430 ms, four rows and one CTA 0.398 ms, two rows under a 112-register cap spill: 0.822 ms)
-    modnorm_bwd_pair_kernel<2, 2><<<grid, nt, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(dh),
-        reinterpret_cast<const __nv_bfloat16*>(dres), scale, shift, reinterpret_cast<const __nv_bfloat16*>(w),
-        reinterpret_cast<__nv_bfloat16*>(dx), dscale, dshift, dw, rows, D, mode, eps, w_f32);
-    return cudaGetLastError() == cudaSuccess ? 0 : -21;
-  }
-  auto kern = (nt <= 640) ? modnorm_bwd_kernel<640, 1, 1> : modnorm_bwd_kernel<1024, 1, 1>;
-  kern<<<grid, row_threads(D), 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  modnorm_bwd_kernel<<<grid, row_threads(D), 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(dh),
       reinterpret_cast<const __nv_bfloat16*>(dres), scale, shift, reinterpret_cast<const __nv_bfloat16*>(w),
-      reinterpret_cast<__nv_bfloat16*>(dx), dscale, dshift, dw, rows, D, mode, eps, rpc, w_f32);
+      reinterpret_cast<__nv_bfloat16*>(dx), dscale, dshift, dw, rows, D, mode, eps, w_f32);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 

@@ -170,6 +170,36 @@ def test_attention_bwd_tile_edges(nw, N, H, d):
         assert rel_err(dqkv[:, i * HD:(i + 1) * HD], x.grad[:, i * HD:(i + 1) * HD]) < 6e-3
 
 
+@pytest.mark.parametrize("rows,D", [(1, 8), (5, 128), (3601, 256), (30, 264), (999, 768), (301, 1536), (7, 1544),
+                                    (300, 2048), (40, 2568), (151, 5120)])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_modnorm_row_widths(rows, D, mode):
+    """One row group per CTA, several, one vector per thread and two, widths that leave threads idle, rows that leave
+    groups idle, and the edges of the variants (1536, 5120). fp32 sums over the rows and columns of bf16 inputs:
+    2^-24 relative per addition; the outputs are rounded to bf16 (2^-9 at most). Targets of the column sums may start
+    at any 4-byte address."""
+    from aeris_gb_b200.ops import elementwise as E
+    eps = 1e-3
+    x, g, r = (torch.randn(rows, D, device=DEV).bfloat16() for _ in range(3))
+    w = torch.randn(D, device=DEV).bfloat16()
+    sc, sh = torch.randn(D, device=DEV) * 0.3, torch.randn(D, device=DEV) * 0.3
+    xr = x.double().requires_grad_(True)
+    a, b, c = (v.double().requires_grad_(True) for v in (sc, sh, w))
+    norm = lambda v: v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + eps)
+    h = norm(xr * (1 + a) + b) * c if mode == 0 else norm(xr) * c * (1 + a) + b
+    h.backward(g.double())
+    lo = torch.empty_like(x)
+    y = E.modnorm_fwd(x, sc, sh, w, mode=mode, eps=eps, out_lo=lo)
+    assert rel_err(y, h) < 2.0 ** -9 and rel_err(y.float() + lo.float(), h) < 2.0 ** -15
+    for shift in (0, 1):           # 16-byte aligned and unaligned column sums
+        ds, dh, dw = (torch.ones(D + shift, device=DEV)[shift:] for _ in range(3))
+        dx = torch.empty_like(x)
+        E.modnorm_bwd(x, g, r, sc, sh, w, mode=mode, eps=eps, dx=dx, dscale=ds, dshift=dh, dw=dw)
+        assert rel_err(dx, xr.grad + r.double()) < 2.0 ** -8
+        for got, want in ((ds, a.grad), (dh, b.grad), (dw, c.grad)):
+            assert rel_err(got, want + 1) < 1e-5
+
+
 @pytest.mark.parametrize("D", [128, 1536])
 @pytest.mark.parametrize("mode", [0, 1])
 def test_modnorm_fwd_bwd(D, mode):
