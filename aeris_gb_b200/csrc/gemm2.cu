@@ -119,12 +119,28 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   const int n_clusters = gridDim.x >> 1;
 
   const int m_tiles = (p.M + 2 * G2_BM - 1) / (2 * G2_BM);
-  const int n_tiles = p.N / G2_BN;
+  const int n_tiles = (p.N + G2_BN - 1) / G2_BN;     // the last tile may be half empty (N a multiple of 128)
   const int kb_total = (p.K + G2_BK - 1) / G2_BK;
   const int kb_per_split = (kb_total + p.k_splits - 1) / p.k_splits;
   const int total_tiles = m_tiles * n_tiles * p.k_splits;
   const int tm_rot = AG ? (p.ag_rank * p.ag_rows) / (2 * G2_BM) : p.tm_rot;
-  auto phys_tm = [&](int tm) { return (tm + tm_rot) % m_tiles; };
+  // Order of the tiles of one K split. The CTA pairs at work together cover `group_m` m-tiles by about 74 / group_m
+  // n-tiles instead of one or two m-tiles by all n-tiles: with a wide B (w1 of dim 5120 is 280 MB, more than L2) the
+  // pairs would otherwise stream all of B from HBM once per wave. group_m = 1 keeps n fastest, which the peer-memory
+  // variants rely on (rows in order of arrival). 28800 x 27392 x 5120 with the SwiGLU
+  // epilogue: 7.60 -> 6.34 ms; its data gradient 7.28 -> 5.40 ms; no change where B fits L2.
+  auto tile_mn = [&](int mn, int& tm, int& tn) {
+    if (p.group_m <= 1) {
+      tm = mn / n_tiles;
+      tn = mn - tm * n_tiles;
+      tm = (tm + tm_rot) % m_tiles;
+    } else {
+      const int g = mn / (p.group_m * n_tiles), in = mn - g * p.group_m * n_tiles;
+      const int gm = min(p.group_m, m_tiles - g * p.group_m);
+      tn = in / gm;
+      tm = g * p.group_m + in - tn * gm;
+    }
+  };
 
   if (threadIdx.x == 0) {
     prefetch_tmap(&tmap_a);
@@ -160,7 +176,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       for (int tile = cluster_id; tile < total_tiles && ok; tile += n_clusters) {
         const int split = tile / (m_tiles * n_tiles);
         const int mn = tile - split * (m_tiles * n_tiles);
-        const int tm = phys_tm(mn / n_tiles), tn = mn - (mn / n_tiles) * n_tiles;
+        int tm, tn;
+        tile_mn(mn, tm, tn);
         const int kb0 = split * kb_per_split;
         const int kb1 = min(kb_total, kb0 + kb_per_split);
         const int m0 = tm * 2 * G2_BM + crank * G2_BM;
@@ -249,7 +266,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     for (int tile = cluster_id; tile < total_tiles && ok; tile += n_clusters) {
       const int split = tile / (m_tiles * n_tiles);
       const int mn = tile - split * (m_tiles * n_tiles);
-      const int tm = phys_tm(mn / n_tiles), tn = mn - (mn / n_tiles) * n_tiles;
+      int tm, tn;
+      tile_mn(mn, tm, tn);
       if (!mbar_wait_poll(&tfull_bar[acc], acc_phase, p.status, ERR_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       const int row = tm * 2 * G2_BM + crank * G2_BM + q * 32 + lane;
@@ -276,6 +294,23 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   if (warp == 1) tmem_dealloc2(tmem_base, 2 * G2_BN);
 }
 
+// Split of the reduction dimension of an accumulating product (weight gradients: few output tiles, a reduction over all
+// tokens): the number of slices that minimises rounds x (k-blocks per slice + fixed cost of a slice), a round being one
+// slice per CTA pair. Constant four left the last round of many shapes nearly empty and small weights (dim 256: 4 slices
+// on 74 pairs) on a handful of SMs. The fixed cost, filling the ring and adding 256 x 256 fp32 values to memory, is
+// taken as 10 k-blocks of 64; slices of fewer than 8 are not made. Four slices
+// and now: 512 x 512 x 28800: 43.6 -> 22.6 us, 768 x 2048 x 28800: 83.6 -> 69.6 us, 1536 x 4096 x 64800: 716 -> 621 us.
+static int auto_k_splits(int mn_tiles, int kb_total, int pairs) {
+  int best = 1;
+  long long best_cost = 0x7fffffffffffll;
+  for (int s = 1; s <= 64 && (s == 1 || kb_total / s >= 8); ++s) {
+    const long long rounds = (static_cast<long long>(mn_tiles) * s + pairs - 1) / pairs;
+    const long long cost = rounds * ((kb_total + s - 1) / s + 10);
+    if (cost < best_cost) { best_cost = cost; best = s; }
+  }
+  return best;
+}
+
 template <int A_MN, int B_MN, bool AG = false>
 static int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p_in, cudaStream_t stream) {
   static bool configured = false;
@@ -287,7 +322,7 @@ static int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
     configured = true;
   }
   const int m_tiles = (p.M + 2 * G2_BM - 1) / (2 * G2_BM);
-  const int tiles = m_tiles * (p.N / G2_BN) * p.k_splits;
+  const int mn_tiles = m_tiles * ((p.N + G2_BN - 1) / G2_BN);
   // persistent grid = the number of CTA pairs the device can actually hold at once
   static int max_clusters = 0;
   if (max_clusters == 0) {
@@ -305,6 +340,8 @@ static int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
     if (getenv("AERIS_DEBUG")) fprintf(stderr, "gemm2: max active clusters %d\n", n);
   }
   int clusters = max_clusters;
+  if (p.k_splits == 0) p.k_splits = auto_k_splits(mn_tiles, (p.K + G2_BK - 1) / G2_BK, clusters);
+  const int tiles = mn_tiles * p.k_splits;
   if (tiles < clusters && !AG) clusters = tiles;
   if (AG) p.ag_expect *= static_cast<unsigned>(2 * clusters);   // came in as the call index
   kern<<<2 * clusters, THREADS, G2_SMEM, stream>>>(ta, tb, p);
@@ -315,24 +352,25 @@ static int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
 
 using namespace aeris;
 
-// Same contract as aeris_gemm_bf16 (api.h); N must be a multiple of 256.
+// Same contract as aeris_gemm_bf16 (api.h); N must be a multiple of 128 (of 256 for the SwiGLU forward epilogues, whose
+// tiles pair gate and up columns). k_splits = 0 with EPI_ACC_F32: chosen by auto_k_splits.
 extern "C" int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb,
                                     int ldc, int a_mn, int b_mn, int epi, const void* resid, int ldr,
                                     const float* gate, int rows_per_gate, void* aux, int ld_aux, int swiglu_f,
                                     int k_splits, int* status, void* stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   if (M <= 0 || N <= 0 || K <= 0) return -1;
-  if (N % G2_BN != 0) return -2;
   const bool swiglu_fwd = (epi == EPI_SWIGLU || epi == EPI_SWIGLU_BOTH);
+  if (N % (swiglu_fwd ? G2_BN : G2_BN / 2) != 0) return -2;
   if (swiglu_fwd && b_mn) return -3;
-  if (k_splits < 1) k_splits = 1;
+  if (k_splits < 0 || (k_splits == 0 && epi != EPI_ACC_F32)) k_splits = 1;
   if (k_splits > 1 && epi != EPI_ACC_F32) return -4;
   GemmParams p{};
   p.M = M; p.N = N; p.K = K; p.epi = epi; p.C = C; p.ldc = ldc;
   p.resid = reinterpret_cast<const __nv_bfloat16*>(resid); p.ldr = ldr;
   p.gate = gate; p.rows_per_gate = rows_per_gate > 0 ? rows_per_gate : M;
   p.aux = reinterpret_cast<__nv_bfloat16*>(aux); p.ld_aux = ld_aux;
-  p.k_splits = k_splits; p.status = status; p.swiglu_f = swiglu_f;
+  p.k_splits = k_splits; p.status = status; p.swiglu_f = swiglu_f; p.group_m = 8;
   {
     // bf16-output epilogues write through the shared-memory stage as 256-byte row segments (measured 1-13 % faster
     // than one 16-byte piece per row and instruction); AERIS_GEMM_STAGED_OUT=0 selects the direct stores

@@ -47,6 +47,7 @@ struct GemmParams {
   int tm_rot;       // first m-tile (of 256 rows) visited by the two-CTA kernel; the others follow cyclically. The
                     // reduce-scatter GEMM starts at the rows of rank + 1 and ends with its own, so that at any moment
                     // every rank pushes to a different owner and no GPU's ingress carries all the traffic
+  int group_m;      // two-CTA kernel: m-tiles per group of the tile order (<= 1: n fastest)
   int staged_out;   // bf16-output epilogues: move rows through the warp's shared-memory stage (coalesced global stores)
   int staged_red;   // split-K fp32 accumulation: stage 32 rows x 64 columns and issue the reductions row-contiguously
   int* status;
@@ -158,6 +159,7 @@ template <int BN>
 __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t taddr, int row, bool row_ok, int tn,
                                                   bool kempty, uint8_t* stage = nullptr) {
   const int lane = threadIdx.x & 31;
+  const int ncols = min(BN, p.N - tn * BN);      // 128 in a half-empty last tile of the two-CTA kernel
 
   if (p.epi == EPI_SCATTER_HEADS) {
     const int w = row / p.scat_n_local;
@@ -228,7 +230,7 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
     const __nv_bfloat16* usrc = p.resid + static_cast<size_t>(row) * p.ldr + tn * BN;
     __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(row) * p.ldc + tn * BN;
 #pragma unroll 1
-    for (int c = 0; c < BN; c += 32) {
+    for (int c = 0; c < ncols; c += 32) {
       uint32_t v[32];
       tmem_ld32(taddr + c, v);
       tmem_wait_ld();
@@ -345,7 +347,7 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
     float* out = reinterpret_cast<float*>(p.C) + static_cast<size_t>(row) * p.ldc + tn * BN;
     const bool live = row_ok && !kempty;
 #pragma unroll 1
-    for (int c = 0; c < BN; c += 32) {
+    for (int c = 0; c < ncols; c += 32) {
       uint32_t v[32];
       tmem_ld32(taddr + c, v);
       tmem_wait_ld();
@@ -355,7 +357,7 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
   } else if (p.epi == EPI_ACC_F32 || p.epi == EPI_STORE_F32) {
     float* out = reinterpret_cast<float*>(p.C) + static_cast<size_t>(row) * p.ldc + tn * BN;
 #pragma unroll 1
-    for (int c = 0; c < BN; c += 32) {
+    for (int c = 0; c < ncols; c += 32) {
       uint32_t v[32];
       tmem_ld32(taddr + c, v);
       tmem_wait_ld();
@@ -403,13 +405,13 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
       for (int i = 0; i < 4; ++i) r4n[i] = reinterpret_cast<const uint4*>(res)[i];
     }
 #pragma unroll 1
-    for (int c = 0; c < BN; c += 32) {
+    for (int c = 0; c < ncols; c += 32) {
       uint32_t v[32];
       tmem_ld32(taddr + c, v);
       if (gated) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) r4[i] = r4n[i];
-        if (c + 32 < BN) {
+        if (c + 32 < ncols) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) r4n[i] = reinterpret_cast<const uint4*>(res + c + 32)[i];
         }
@@ -447,7 +449,7 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
       gate = p.gate + static_cast<size_t>(row / p.rows_per_gate) * p.N + tn * BN;
     __nv_bfloat16* aux = p.aux ? p.aux + static_cast<size_t>(row) * p.ld_aux + tn * BN : nullptr;
 #pragma unroll 1
-    for (int c = 0; c < BN; c += 32) {
+    for (int c = 0; c < ncols; c += 32) {
       uint32_t v[32];
       tmem_ld32(taddr + c, v);
       tmem_wait_ld();

@@ -349,7 +349,7 @@ def block_backward(x: torch.Tensor, mod: torch.Tensor, dy: torch.Tensor, meta: B
     if dx is None:
         dx = torch.empty_like(x)
     mod = mod.contiguous()
-    ksplit_tok = 4
+    ksplit_tok = 0      # the kernel chooses
     for b in range(B):
         sh1, sc1, g1, sh2, sc2, g2 = [mod[b, i * D:(i + 1) * D] for i in range(6)]
         dsh1, dsc1, dg1, dsh2, dsc2, dg2 = [dmod[b, i * D:(i + 1) * D] for i in range(6)]

@@ -103,7 +103,7 @@ class EmbedFn(torch.autograd.Function):
             n = min(CHUNK_ROWS, T - r0)
             DF.embed_pack(x_img, c_img, cs, plan.geom, plan.ape_y, plan.ape_x, plan.seed, plan.sigma_data,
                           plan.noise, A[:n], row0=r0)
-            G.gemm(dout[r0:r0 + n], A[:n], a_t=True, b_t=True, out=Gw, epi=G.EPI_ACC_F32, k_splits=8)
+            G.gemm(dout[r0:r0 + n], A[:n], a_t=True, b_t=True, out=Gw, epi=G.EPI_ACC_F32, k_splits=0)
         dW = Gw[:, :Cin] + Gw[:, Cin:2 * Cin]
         db = Gw[:, 3 * Cin]
         sW, rW = _grad_slot(W)

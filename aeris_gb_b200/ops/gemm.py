@@ -7,7 +7,7 @@ import torch
 
 from . import lib as _l
 
-# The two-CTA (cta_group::2, 256 x 256 tile per SM pair) kernel is used for every product whose N is a multiple of 256
+# The two-CTA (cta_group::2, 256 x 256 tile per SM pair) kernel is used for every product that it takes (see gemm())
 # unless AERIS_GEMM_2CTA=0.
 TWO_CTA_DEFAULT = os.environ.get("AERIS_GEMM_2CTA", "1") != "0"
 
@@ -32,6 +32,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
     EPI_GATE_RESID ``resid + gate * acc`` (gate fp32 ``[M // rows_per_gate, N]``; ``aux`` optionally receives the
     raw product); EPI_ACC_F32 ``out += acc`` in fp32 (split-K allowed); EPI_STORE_F32 fp32 out;
     EPI_SWIGLU_BOTH = EPI_SWIGLU that also writes the raw ``[gate | up]`` product to ``aux [M, 2F]``;
+    ``k_splits``: slices of the reduction dimension (EPI_ACC_F32 only); 0 lets the kernel choose.
     EPI_SWIGLU_BWD: the product is d(act) ``[M, F]``, ``resid`` holds ``u = [gate | up]`` and ``out`` receives d(u).
     """
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
@@ -61,7 +62,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
     assert out.shape == (M, n_out) or epi == EPI_SWIGLU_BWD
     if two_cta is None:
         two_cta = TWO_CTA_DEFAULT and bn == 0
-    if two_cta and N % 256 == 0:
+    # a last tile with 128 valid columns costs as much as a full one: 6 % at 2048 columns, far less than the two-CTA kernel
+    # gains there (28800 x 13696 x 5120: 4.96 -> 3.38 ms), but 12150 x 1152 x 384 takes 43 us instead of 38; the SwiGLU
+    # forward pairs gate and up columns of whole tiles
+    if two_cta and (N % 256 == 0 or (N % 128 == 0 and N >= 2048 and epi not in (EPI_SWIGLU, EPI_SWIGLU_BOTH))):
         rc = _l.lib().aeris_gemm_bf16_2cta(
             _l.ptr(a), _l.ptr(b), _l.ptr(out), M, N, K, _ld(a), _ld(b), _ld(out), int(a_t), int(b_t), epi,
             _l.ptr(resid), _ld(resid) if resid is not None else 0, _l.ptr(gate), rows_per_gate,
@@ -71,6 +75,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
         return out
     if bn == 0:
         bn = 256 if N % 256 == 0 else 128
+    if k_splits == 0:        # this kernel's fixed choice: enough slices to fill the SMs on narrow weights
+        k_splits = 4
     rc = _l.lib().aeris_gemm_bf16(
         _l.ptr(a), _l.ptr(b), _l.ptr(out), M, N, K, _ld(a), _ld(b), _ld(out), int(a_t), int(b_t), epi,
         _l.ptr(resid), _ld(resid) if resid is not None else 0, _l.ptr(gate), rows_per_gate,

@@ -144,9 +144,9 @@ class TPMlpFn(torch.autograd.Function):
         gemm_allgather_a(tpx, x_buf, x_peers, w1, out=act, epi=G.EPI_SWIGLU_BOTH, aux=u)     # recompute; x gathered
         gemm_allgather_a(tpx, g_buf, g_peers, w2, out=u, b_t=True, epi=G.EPI_SWIGLU_BWD, resid=u)   # du; dy gathered
         s2, r2 = _grad_slot(w2)
-        G.gemm(g_buf, act, a_t=True, b_t=True, out=s2, epi=G.EPI_ACC_F32, k_splits=4)         # dW2_r = dY^T act_r
+        G.gemm(g_buf, act, a_t=True, b_t=True, out=s2, epi=G.EPI_ACC_F32, k_splits=0)         # dW2_r = dY^T act_r
         s1, r1 = _grad_slot(w1)
-        G.gemm(u, x_buf, a_t=True, b_t=True, out=s1, epi=G.EPI_ACC_F32, k_splits=4)           # dW1_r = dU_r^T X
+        G.gemm(u, x_buf, a_t=True, b_t=True, out=s1, epi=G.EPI_ACC_F32, k_splits=0)           # dW1_r = dU_r^T X
         dh = gemm_reduce_scatter(tpx, u, w1, b_t=True, name="rs_dx")                          # dX = RS(dU_r @ w1_r)
         return (dh, r1.to(w1.dtype) if r1 is not None else None, r2.to(w2.dtype) if r2 is not None else None, None)
 

@@ -151,6 +151,55 @@ def test_attention_bwd_rising_scores():
         assert rel_err(dqkv[:, i * HD:(i + 1) * HD], x.grad[:, i * HD:(i + 1) * HD]) < 2e-2
 
 
+@pytest.mark.parametrize("M,N,K", [(300, 2176, 192), (2100, 2944, 320), (5000, 2176, 64), (129, 2432, 128)])
+def test_gemm_half_empty_last_tile(M, N, K):
+    """N a multiple of 128 but not of 256 on the two-CTA kernel: the columns past N of the last tile are neither read nor
+    written (the output's neighbours keep their values), for every epilogue that takes such an N; more m-tiles than a
+    group of the tile order (2100, 5000 rows) and fewer."""
+    from aeris_gb_b200.ops import gemm as G
+    a, b = torch.randn(M, K, device=DEV).bfloat16(), torch.randn(N, K, device=DEV).bfloat16()
+    ref = a.float() @ b.float().t()
+    bt = b.t().contiguous()
+
+    def wide(dtype, cols=N):
+        buf = torch.full((M, cols + 128), 7.0, dtype=dtype, device=DEV)
+        return buf, buf[:, :cols]
+    for b_t in (False, True):
+        bb = bt if b_t else b
+        buf, out = wide(torch.bfloat16)
+        G.gemm(a, bb, b_t=b_t, out=out, two_cta=True)
+        assert rel_err(out, ref) < TOL and (buf[:, N:] == 7).all()
+        buf, out = wide(torch.float32)
+        G.gemm(a, bb, b_t=b_t, out=out, epi=G.EPI_STORE_F32, two_cta=True)
+        assert rel_err(out, ref) < 1e-5 and (buf[:, N:] == 7).all()
+        resid, gate = torch.randn(M, N, device=DEV).bfloat16(), torch.randn(1, N, device=DEV)
+        buf, out = wide(torch.bfloat16)
+        G.gemm(a, bb, b_t=b_t, out=out, epi=G.EPI_GATE_RESID, resid=resid, gate=gate, two_cta=True)
+        assert rel_err(out, resid.float() + gate * ref) < TOL and (buf[:, N:] == 7).all()
+        u = torch.randn(M, 2 * N, device=DEV).bfloat16()
+        g, up = u[:, :N].float(), u[:, N:].float()
+        s = torch.sigmoid(g)
+        buf, out = wide(torch.bfloat16, 2 * N)
+        buf2 = torch.empty(M, 2 * N, dtype=torch.bfloat16, device=DEV)
+        G.gemm(a, bb, b_t=b_t, out=buf2, epi=G.EPI_SWIGLU_BWD, resid=u, two_cta=True)
+        want = torch.cat([ref * up * s * (1 + g * (1 - s)), ref * g * s], dim=1)
+        assert rel_err(buf2, want) < TOL
+        G.gemm(a, bb, b_t=b_t, out=out, epi=G.EPI_SWIGLU_BWD, resid=u, two_cta=True)
+        assert torch.equal(out, buf2) and (buf[:, 2 * N:] == 7).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 256, 3600), (384, 640, 12150), (512, 1536, 200), (1536, 768, 28800), (256, 256, 40)])
+@pytest.mark.parametrize("k_splits", [0, 1, 3])
+def test_gemm_accumulate_splits(M, N, K, k_splits):
+    """Weight-gradient products with the kernel's own split of the token dimension, none, and a fixed one: fp32 sums in
+    another order. The tensor core adds 16 products at a time and may truncate: K / 16 additions of 2^-23 at most."""
+    from aeris_gb_b200.ops import gemm as G
+    a, b = torch.randn(K, M, device=DEV).bfloat16(), torch.randn(K, N, device=DEV).bfloat16()
+    out = torch.ones(M, N, device=DEV)
+    G.gemm(a, b, a_t=True, b_t=True, out=out, epi=G.EPI_ACC_F32, k_splits=k_splits)
+    assert rel_err(out, a.double().t() @ b.double() + 1) < K / 16 * 2.0 ** -23 + 1e-6
+
+
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("nw,N,H", [(2, 15, 2), (3, 64, 1), (40, 64, 8), (2, 65, 2), (1, 127, 2), (2, 129, 3), (5, 225, 30)])
 def test_attention_bwd_tile_edges(nw, N, H, d):
