@@ -102,8 +102,15 @@ int aeris_sampler_update(float* x_out, const float* x_base, const float* pa, con
 int aeris_noise_mix(float* x, float a, float b, unsigned long long seed, const TokGeom* g, int Cx, void* stream);
 int aeris_affine_channels(float* out, const float* in, const float* a, const float* b, const float* add, long long n,
                           int C, void* stream);
-int aeris_gemv_bias_act(const void* W, int w_f32, const float* bias, const float* x, float* y, int N, int K, int B,
-                        int act, int silu_in, void* stream);
+int aeris_gemv_bias_act(const void* W, int flags, const void* bias, const void* x, float* y, int N, int K, int B, int act,
+                        int silu_in, void* stream);
+// Gradients of the above without `act`; added to dW, db (may be null) and dx (may be null).
+int aeris_gemv_bwd(const void* W, int flags, const void* x, const float* dy, float* dW, float* db, float* dx, int N, int K,
+                   int B, int silu_in, void* stream);
+int aeris_noise_embedding(const float* t, void* out, int out_bf16, int B, int dim, double max_period, void* stream);
+int aeris_pack_embed_weights(const float* W, const float* b, void* out, int D, int Cin, int KP, void* stream);
+int aeris_fold_embed_grad(const float* G, float* dW, float* db, int D, int Cin, int KP, void* stream);
+int aeris_pack_head_weights(const float* W, void* hi, void* lo, int C, int rows, int D, void* stream);
 
 #ifdef __cplusplus
 }

@@ -10,7 +10,6 @@
 //   * sampler_update / noise_mix / affine_channels: Euler and Heun updates, churn and initial noise, and the
 //     (un)standardisation + residual add of the rollout, all on the device (src/aeris/pp_generate.py:228-241,
 //     298-333, which round-trips through host numpy)
-//   * gemv_bias_act: the M <= 8 modulation MLP layers (parallel_swin.py:321-325)
 // The noise of pixel (sample, Y, X), channel c depends only on the seed and on those global coordinates, so it does not
 // change with the window-parallel or sequence-parallel layout of the run.
 #include "common.cuh"
@@ -249,47 +248,6 @@ __global__ void affine_channels_kernel(float* __restrict__ out, const float* __r
   }
 }
 
-// y[b, n] = act(sum_k W[n, k] x[b, k] + bias[n]) for B <= 8 rows: one warp per output feature streams one weight
-// row. act: 0 none, 1 SiLU. W bf16 or fp32 (w_f32).
-template <typename WT>
-__global__ void gemv_bias_act_kernel(const WT* __restrict__ W, const float* __restrict__ bias,
-                                     const float* __restrict__ x, float* __restrict__ y, int N, int K, int B, int act,
-                                     int silu_in) {
-  extern __shared__ float xs[];  // [B, K]
-  for (int i = threadIdx.x; i < B * K; i += blockDim.x) {
-    const float t = x[i];
-    xs[i] = silu_in ? t / (1.f + __expf(-t)) : t;
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int n = blockIdx.x * nw + warp; n < N; n += gridDim.x * nw) {
-    float acc[8];
-#pragma unroll
-    for (int b = 0; b < 8; ++b) acc[b] = 0.f;
-    const WT* wr = W + static_cast<size_t>(n) * K;
-    for (int k = lane; k < K; k += 32) {
-      float w;
-      if constexpr (sizeof(WT) == 2) w = __bfloat162float(wr[k]); else w = wr[k];
-#pragma unroll
-      for (int b = 0; b < 8; ++b)
-        if (b < B) acc[b] = fmaf(w, xs[b * K + k], acc[b]);
-    }
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc[b] += __shfl_xor_sync(0xffffffffu, acc[b], o);
-    }
-    if (lane == 0) {
-      const float bv = bias ? bias[n] : 0.f;
-      for (int b = 0; b < B; ++b) {
-        float v = acc[b] + bv;
-        if (act == 1) v = v / (1.f + __expf(-v));
-        y[static_cast<size_t>(b) * N + n] = v;
-      }
-    }
-  }
-}
-
 }  // namespace aeris
 
 using namespace aeris;
@@ -361,24 +319,5 @@ extern "C" int aeris_affine_channels(float* out, const float* in, const float* a
   if (blocks > cap) blocks = cap;
   affine_channels_kernel<<<static_cast<int>(blocks), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(out, in, a, b,
                                                                                                        add, n, C);
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
-}
-
-extern "C" int aeris_gemv_bias_act(const void* W, int w_f32, const float* bias, const float* x, float* y, int N, int K,
-                                   int B, int act, int silu_in, void* stream) {
-  if (N <= 0 || K <= 0 || B <= 0 || B > 8) return -1;
-  const size_t smem = static_cast<size_t>(B) * K * sizeof(float);
-  if (smem > 48 * 1024) return -2;
-  const int warps = 8;
-  int grid = (N + warps - 1) / warps;
-  const int cap = aeris_num_sms() * 8;
-  if (grid > cap) grid = cap;
-  auto st = reinterpret_cast<cudaStream_t>(stream);
-  if (w_f32)
-    gemv_bias_act_kernel<float><<<grid, warps * 32, smem, st>>>(reinterpret_cast<const float*>(W), bias, x, y, N, K, B,
-                                                               act, silu_in);
-  else
-    gemv_bias_act_kernel<__nv_bfloat16><<<grid, warps * 32, smem, st>>>(reinterpret_cast<const __nv_bfloat16*>(W),
-                                                                       bias, x, y, N, K, B, act, silu_in);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }

@@ -292,7 +292,13 @@ class InputStage(nn.Module):
                 return self.interval_embed(t.reshape(-1, 1).to(cfg.data_dtype)).to(cfg.model_dtype)
             n = 1 if t is None else t.reshape(-1).shape[0]
             return torch.zeros((n, cfg.dim), dtype=cfg.model_dtype, device=self.proj.weight.device)
-        emb = O.timestep_embedding(t.to(cfg.data_dtype), cfg.dim, cfg.max_period)
+        if (use_fused(t) and not t.requires_grad and cfg.dim % 2 == 0 and cfg.data_dtype == torch.float32
+                and cfg.model_dtype in (torch.bfloat16, torch.float32)):
+            from ..ops import diffusion as DF
+            emb = DF.noise_embedding(t.float().contiguous(), cfg.dim, cfg.max_period,
+                                     cfg.model_dtype if cfg.layerwise_t_emb else torch.float32)
+        else:
+            emb = O.timestep_embedding(t.to(cfg.data_dtype), cfg.dim, cfg.max_period)
         if not cfg.layerwise_t_emb:
             emb = self.latent_embed(emb)
         return emb.to(cfg.model_dtype)
@@ -553,7 +559,8 @@ class AerisModel(nn.Module):
     @torch.no_grad()
     def predict_images(self, x_img, c_img, t, ctx: StreamContext, plan) -> torch.Tensor:
         """One network evaluation for the sampler: ``x_img`` is the noisy state; returns F in token order [T, 128]."""
-        cs = torch.tensor([[1.0, 0.0]], device=x_img.device).repeat(x_img.shape[0], 1)
+        cs = torch.zeros((x_img.shape[0], 2), device=x_img.device)
+        cs[:, 0] = 1.0
         x, dt = self.input_stage.forward_images(x_img, c_img, cs, t, plan)
         return self.output_stage.predict_tokens(self.trunk(x, dt, ctx), dt)
 

@@ -492,34 +492,36 @@ class FusedBlock(torch.autograd.Function):
 
 class GemvLinearFn(torch.autograd.Function):
     """``silu?(x) @ W^T + b`` for the handful of rows of a modulation MLP (one row per sample): the forward streams the
-    weight once through the GEMV kernel; weight gradients are rank-B updates added to the fp32 gradient buffers."""
+    weight once through the GEMV kernel; one backward kernel adds the rank-B weight gradient to the fp32 gradient buffers
+    and streams the weight once more for the gradient of ``x``."""
 
     @staticmethod
     def forward(ctx, x, W, b, silu_in: bool):
         from ..ops import diffusion as DF
-        x32 = x.float().contiguous()
-        y = DF.gemv_bias_act(W.detach(), b.detach().float() if b is not None else None, x32, act=0, silu_in=silu_in)
-        ctx.silu_in, ctx.x_dtype = silu_in, x.dtype
-        ctx.save_for_backward(x32, W, b)
-        return y
+        ctx.silu_in = silu_in
+        ctx.save_for_backward(x, W, b)
+        return DF.gemv_bias_act(W.detach(), b.detach() if b is not None else None, x.detach(), act=0, silu_in=silu_in)
 
     @staticmethod
     def backward(ctx, dy):
+        from ..ops import diffusion as DF
         from .fused_io import _grad_slot
-        x32, W, b = ctx.saved_tensors
-        dy = dy.float()
-        sig = torch.sigmoid(x32) if ctx.silu_in else None
-        h = x32 * sig if ctx.silu_in else x32
+        x, W, b = ctx.saved_tensors
         sW, rW = _grad_slot(W)
-        sW.addmm_(dy.t(), h)
-        rb = None
-        if b is not None:
-            sb, rb = _grad_slot(b)
-            sb += dy.sum(0)
-        dx = (dy.to(W.dtype) @ W).float()
-        if ctx.silu_in:
-            dx = dx * (sig * (1 + x32 * (1 - sig)))
-        return (dx.to(ctx.x_dtype), rW.to(W.dtype) if rW is not None else None,
+        sb, rb = _grad_slot(b) if b is not None else (None, None)
+        dx = torch.zeros(x.shape, dtype=torch.float32, device=x.device) if ctx.needs_input_grad[0] else None
+        if DF.gemv_bwd_ok(W, sW):
+            DF.gemv_bwd(W, x, dy, sW, sb, dx, ctx.silu_in)
+        else:
+            dy, x32 = dy.float(), x.float()
+            sig = torch.sigmoid(x32)
+            sW.addmm_(dy.t(), x32 * sig if ctx.silu_in else x32)
+            if sb is not None:
+                sb += dy.sum(0)
+            if dx is not None:
+                dx = dy @ W.float()
+                dx = dx * (sig * (1 + x32 * (1 - sig))) if ctx.silu_in else dx
+        return (dx.to(x.dtype) if dx is not None else None, rW.to(W.dtype) if rW is not None else None,
                 rb.to(b.dtype) if rb is not None else None, None)
 
 

@@ -45,6 +45,7 @@ def ape_tables(cfg, device) -> tuple[torch.Tensor, torch.Tensor]:
 
 
 def _split(t: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+    """bf16 value and bf16 remainder of an fp32 tensor (what the packing kernels write)."""
     hi = t.to(torch.bfloat16)
     return hi, (t - hi.float()).to(torch.bfloat16)
 
@@ -71,11 +72,7 @@ class EmbedFn(torch.autograd.Function):
         D, Cin = W.shape
         KP = _pack_dim(Cin)
         dev = x_img.device
-        Wp = torch.zeros((D, KP), dtype=torch.bfloat16, device=dev)
-        w_hi, w_lo = _split(W.detach().float())
-        b_hi, b_lo = _split(b.detach().float())
-        Wp[:, :Cin], Wp[:, Cin:2 * Cin], Wp[:, 2 * Cin:3 * Cin] = w_hi, w_hi, w_lo
-        Wp[:, 3 * Cin], Wp[:, 3 * Cin + 1] = b_hi, b_lo
+        Wp = DF.pack_embed_weights(W.detach().float().contiguous(), b.detach().float().contiguous(), KP)
         T = plan.geom.rows
         out = torch.empty((T, D), dtype=torch.bfloat16, device=dev)
         A = workspace().get("embed_a", (min(CHUNK_ROWS, T), KP), torch.bfloat16, dev)
@@ -104,23 +101,15 @@ class EmbedFn(torch.autograd.Function):
             DF.embed_pack(x_img, c_img, cs, plan.geom, plan.ape_y, plan.ape_x, plan.seed, plan.sigma_data,
                           plan.noise, A[:n], row0=r0)
             G.gemm(dout[r0:r0 + n], A[:n], a_t=True, b_t=True, out=Gw, epi=G.EPI_ACC_F32, k_splits=0)
-        dW = Gw[:, :Cin] + Gw[:, Cin:2 * Cin]
-        db = Gw[:, 3 * Cin]
         sW, rW = _grad_slot(W)
         sb, rb = _grad_slot(b)
-        sW += dW
-        sb += db
+        DF.fold_embed_grad(Gw, sW, sb)
         return (None, None, None, rW.to(W.dtype) if rW is not None else None,
                 rb.to(b.dtype) if rb is not None else None, None)
 
 
 def _head_weights(head_w: torch.Tensor):
-    C, D = head_w.shape
-    hi, lo = _split(head_w.detach().float())
-    w_hi = torch.zeros((PAD_N, D), dtype=torch.bfloat16, device=head_w.device)
-    w_lo = torch.zeros((PAD_N, D), dtype=torch.bfloat16, device=head_w.device)
-    w_hi[:C], w_lo[:C] = hi, lo
-    return w_hi, w_lo
+    return DF.pack_head_weights(head_w.detach().float().contiguous(), PAD_N)
 
 
 def _head_rows(x, scale_b, shift_b, norm_w, w_hi, w_lo, eps, pred, y_hi, y_lo):
@@ -200,9 +189,8 @@ class HeadLossFn(torch.autograd.Function):
         dy = ws.get("head_ylo", (cm, D), torch.bfloat16, dev)
         Gh = ws.get("head_g", (PAD_N, D), torch.float32, dev, zero=True)
         shift32, scale32 = shift.float().contiguous(), scale.float().contiguous()
-        dshift, dscale = torch.zeros_like(shift32), torch.zeros_like(scale32)
+        dshift, dscale = torch.zeros((2, *shift32.shape), dtype=torch.float32, device=dev).unbind(0)
         s_nw, r_nw = _grad_slot(norm_w)
-        dnw = torch.zeros(D, dtype=torch.float32, device=dev)
         dx = torch.empty_like(x)
         dpred = dpred * g.to(dpred.dtype)
         for b, r0, n in _sample_chunks(B, T // B):
@@ -212,8 +200,7 @@ class HeadLossFn(torch.autograd.Function):
             G.gemm(dp, y_hi[:n], a_t=True, b_t=True, out=Gh, epi=G.EPI_ACC_F32, k_splits=16, two_cta=False)
             G.gemm(dp, w_hi, b_t=True, out=dy[:n])
             E.modnorm_bwd(x[r0:r0 + n], dy[:n], None, scale32[b], shift32[b], norm_w, mode=E.MODE_NORM_THEN_MOD,
-                          eps=plan.eps, dx=dx[r0:r0 + n], dscale=dscale[b], dshift=dshift[b], dw=dnw)
-        s_nw += dnw
+                          eps=plan.eps, dx=dx[r0:r0 + n], dscale=dscale[b], dshift=dshift[b], dw=s_nw)
         s_hw, r_hw = _grad_slot(head_w)
         s_hw += Gh[:C]
         return (dx, dshift.to(shift.dtype), dscale.to(scale.dtype), r_nw.to(norm_w.dtype) if r_nw is not None else None,

@@ -90,13 +90,73 @@ def affine_channels(inp: torch.Tensor, a: torch.Tensor, b: torch.Tensor, add: to
     return out
 
 
+def _gemv_flags(W: torch.Tensor, bias: torch.Tensor | None, x: torch.Tensor) -> int:
+    return (int(W.dtype == torch.float32) | 2 * int(bias is not None and bias.dtype == torch.bfloat16)
+            | 4 * int(x.dtype == torch.bfloat16))
+
+
+def _f32_or_bf16(t: torch.Tensor | None) -> torch.Tensor | None:
+    return t if t is None or t.dtype in (torch.float32, torch.bfloat16) else t.float()
+
+
 def gemv_bias_act(W: torch.Tensor, bias: torch.Tensor | None, x: torch.Tensor, act: int = 0,
                   silu_in: bool = False) -> torch.Tensor:
-    """``act(silu?(x) @ W^T + bias)`` for at most 8 rows of fp32 ``x``; W bf16 or fp32 [N, K]; fp32 result."""
+    """``act(silu?(x) @ W^T + bias)`` for at most 8 rows of ``x``; W, bias and x bf16 or fp32, W [N, K]; fp32 result."""
     N, K = W.shape
+    x, bias = _f32_or_bf16(x).contiguous(), _f32_or_bf16(bias)
     B = x.shape[0]
     y = torch.empty((B, N), dtype=torch.float32, device=x.device)
-    rc = _l.lib().aeris_gemv_bias_act(_l.ptr(W), int(W.dtype == torch.float32), _l.ptr(bias), _l.ptr(x), _l.ptr(y), N,
+    rc = _l.lib().aeris_gemv_bias_act(_l.ptr(W), _gemv_flags(W, bias, x), _l.ptr(bias), _l.ptr(x), _l.ptr(y), N,
                                       K, B, act, int(silu_in), _l.stream_ptr())
     _l.check(rc, "aeris_gemv_bias_act")
     return y
+
+
+def gemv_bwd(W: torch.Tensor, x: torch.Tensor, dy: torch.Tensor, dW: torch.Tensor, db: torch.Tensor | None,
+             dx: torch.Tensor | None, silu_in: bool = False) -> None:
+    """Adds the gradients of ``silu?(x) @ W^T + b`` (at most 8 rows) to fp32 ``dW``, ``db`` and ``dx``."""
+    N, K = W.shape
+    x, dy = _f32_or_bf16(x).contiguous(), dy.float().contiguous()
+    rc = _l.lib().aeris_gemv_bwd(_l.ptr(W), _gemv_flags(W, None, x), _l.ptr(x), _l.ptr(dy), _l.ptr(dW), _l.ptr(db),
+                                 _l.ptr(dx), N, K, x.shape[0], int(silu_in), _l.stream_ptr())
+    _l.check(rc, "aeris_gemv_bwd")
+
+
+def gemv_bwd_ok(W: torch.Tensor, dW: torch.Tensor) -> bool:
+    """Whether :func:`gemv_bwd` takes these operands (whole vectors of four along K)."""
+    return (W.shape[1] % 4 == 0 and W.is_contiguous() and dW.is_contiguous() and dW.data_ptr() % 16 == 0
+            and W.data_ptr() % (4 * W.element_size()) == 0 and W.dtype in (torch.bfloat16, torch.float32))
+
+
+def noise_embedding(t: torch.Tensor, dim: int, max_period: float, dtype: torch.dtype) -> torch.Tensor:
+    """``[sin | cos]`` embedding [B, dim] of the noise levels ``t`` (fp32 [B]) in ``dtype`` (bf16 or fp32)."""
+    out = torch.empty((t.shape[0], dim), dtype=dtype, device=t.device)
+    rc = _l.lib().aeris_noise_embedding(_l.ptr(t), _l.ptr(out), int(dtype == torch.bfloat16), t.shape[0], dim,
+                                        ctypes.c_double(max_period), _l.stream_ptr())
+    _l.check(rc, "aeris_noise_embedding")
+    return out
+
+
+def pack_embed_weights(W: torch.Tensor, b: torch.Tensor, KP: int) -> torch.Tensor:
+    """``[hi(W) | hi(W) | lo(W) | hi(b) | lo(b) | 0..]`` (bf16 [D, KP]) of an fp32 weight [D, Cin] and bias."""
+    D, Cin = W.shape
+    out = torch.empty((D, KP), dtype=torch.bfloat16, device=W.device)
+    rc = _l.lib().aeris_pack_embed_weights(_l.ptr(W), _l.ptr(b), _l.ptr(out), D, Cin, KP, _l.stream_ptr())
+    _l.check(rc, "aeris_pack_embed_weights")
+    return out
+
+
+def fold_embed_grad(G: torch.Tensor, dW: torch.Tensor, db: torch.Tensor) -> None:
+    """Adds the gradient ``G`` (fp32 [D, KP]) of the packed operand to ``dW`` [D, Cin] and ``db`` [D]."""
+    D, Cin = dW.shape
+    rc = _l.lib().aeris_fold_embed_grad(_l.ptr(G), _l.ptr(dW), _l.ptr(db), D, Cin, G.shape[1], _l.stream_ptr())
+    _l.check(rc, "aeris_fold_embed_grad")
+
+
+def pack_head_weights(W: torch.Tensor, rows: int) -> tuple[torch.Tensor, torch.Tensor]:
+    """bf16 value and bf16 remainder of an fp32 weight [C, D], padded with zero rows to ``rows``."""
+    C, D = W.shape
+    hi, lo = torch.empty((2, rows, D), dtype=torch.bfloat16, device=W.device).unbind(0)
+    rc = _l.lib().aeris_pack_head_weights(_l.ptr(W), _l.ptr(hi), _l.ptr(lo), C, rows, D, _l.stream_ptr())
+    _l.check(rc, "aeris_pack_head_weights")
+    return hi, lo
