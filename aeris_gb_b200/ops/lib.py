@@ -38,7 +38,9 @@ def ptr(t: torch.Tensor | None) -> _c_void_p:
 
 
 def stream_ptr() -> _c_void_p:
-    return _c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current stream of the current device. Asked for on every launch: the raw handle costs 0.3 us, building the
+    ``torch.cuda.Stream`` object around it 5 us, a third of what issuing one kernel from Python takes."""
+    return _c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 _STATUS: dict[int, torch.Tensor] = {}
@@ -46,7 +48,7 @@ _STATUS: dict[int, torch.Tensor] = {}
 
 def status_word() -> torch.Tensor:
     """Per-device int32 word that kernels set when a bounded wait runs out or a bounds check fails."""
-    dev = torch.cuda.current_device()
+    dev = torch._C._cuda_getDevice()
     if dev not in _STATUS:
         _STATUS[dev] = torch.zeros(1, dtype=torch.int32, device=f"cuda:{dev}")
     return _STATUS[dev]
