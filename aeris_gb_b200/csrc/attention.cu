@@ -23,7 +23,7 @@ struct AttnFwdParams {
   int ldo;
   float* lse;  // [n_win * H * N], log2 domain: m + log2(l)
   int N, H, n_win;
-  int q_col0, k_col0, v_col0;
+  int d;         // head width, at most the kernel's HD (the tensor maps pad with zeros)
   float scale_log2;
   int* status;
   // Ulysses output push (all null / 0 when unused): row `grow` of window `win` belongs to rank grow / push_n_local and
@@ -230,7 +230,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       mbar_expect_tx(q_full, Q_BYTES);
 #pragma unroll
       for (int c = 0; c < DCH; ++c)
-        tma_load_3d(sQ + c * 16384, &tm_q, q_full, p.q_col0 + head * HD + c * 64, qt * TILE, win);
+        tma_load_4d(sQ + c * 16384, &tm_q, q_full, c * 64, head, qt * TILE, win);
       // K_i, then V_{i-1}: the order in which their slots come free (K_i after Q K^T of tile i - NSK, V_{i-1} after P V
       // of tile i - 1 - NSV, which completes later), so no wait holds up a load whose slot is already free
       for (int i = 0; i <= nkv; ++i) {
@@ -240,7 +240,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           mbar_expect_tx(&k_full[st], T_BYTES);
 #pragma unroll
           for (int c = 0; c < DCH; ++c)
-            tma_load_3d(sKr + st * T_BYTES + c * 8192, &tm_k, &k_full[st], p.k_col0 + head * HD + c * 64, i * KVT, win);
+            tma_load_4d(sKr + st * T_BYTES + c * 8192, &tm_k, &k_full[st], c * 64, head, i * KVT, win);
         }
         if (i >= 1) {
           const int j = i - 1, st = j % NSV;
@@ -248,7 +248,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           mbar_expect_tx(&v_full[st], T_BYTES);
 #pragma unroll
           for (int c = 0; c < DCH; ++c)
-            tma_load_3d(sVr + st * T_BYTES + c * 8192, &tm_v, &v_full[st], p.v_col0 + head * HD + c * 64, j * KVT, win);
+            tma_load_4d(sVr + st * T_BYTES + c * 8192, &tm_v, &v_full[st], c * 64, head, j * KVT, win);
         }
       }
     }
@@ -472,16 +472,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       {
         const float inv = 1.f / l;
         const size_t trow = static_cast<size_t>(win) * N + grow;
-        __nv_bfloat16* dst = (p.O && grow < N) ? p.O + trow * p.ldo + head * HD : nullptr;
+        __nv_bfloat16* dst = (p.O && grow < N) ? p.O + trow * p.ldo + head * p.d : nullptr;
         __nv_bfloat16* pdst = nullptr;
         if (p.push_n_local > 0 && grow < N) {
           const int owner = grow / p.push_n_local;
           pdst = reinterpret_cast<__nv_bfloat16*>(p.o_peers[owner]) +
                  (static_cast<size_t>(win) * p.push_n_local + (grow - owner * p.push_n_local)) * p.push_ld +
-                 p.push_col0 + head * HD;
+                 p.push_col0 + head * p.d;
         }
 #pragma unroll
         for (int c = 0; c < HD; c += 32) {
+          if (c >= p.d) break;
           uint32_t v[32];
           tmem_ld32(tO + lane_addr + c, v);
           tmem_wait_ld();
@@ -492,8 +493,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             u.y = pack_bf16x2(__uint_as_float(v[8 * g + 2]) * inv, __uint_as_float(v[8 * g + 3]) * inv);
             u.z = pack_bf16x2(__uint_as_float(v[8 * g + 4]) * inv, __uint_as_float(v[8 * g + 5]) * inv);
             u.w = pack_bf16x2(__uint_as_float(v[8 * g + 6]) * inv, __uint_as_float(v[8 * g + 7]) * inv);
-            if (dst) *reinterpret_cast<uint4*>(dst + c + 8 * g) = u;
-            if (pdst) *reinterpret_cast<uint4*>(pdst + c + 8 * g) = u;
+            const bool live = c + 8 * g < p.d;
+            if (dst && live) *reinterpret_cast<uint4*>(dst + c + 8 * g) = u;
+            if (pdst && live) *reinterpret_cast<uint4*>(pdst + c + 8 * g) = u;
           }
         }
         if (p.lse && grow < N) p.lse[(static_cast<size_t>(win) * p.H + head) * N + grow] = m_ref + log2f(l);
@@ -551,6 +553,7 @@ struct AttnBwdParams {
   __nv_bfloat16* dQKV;      // [T, ldg] gradient of the fused qkv tensor
   int ldg;
   int N, H, n_win;
+  int d;         // head width, at most the kernel's HD (the tensor maps pad with zeros)
   int q_col0, k_col0, v_col0;
   float scale_log2, scale;
   int* status;
@@ -561,16 +564,15 @@ struct AttnBwdParams {
 };
 constexpr int BT = 64;      // rows of a streamed tile
 
-template <int HD>
 __device__ __forceinline__ __nv_bfloat16* bwd_dst(const AttnBwdParams& p, int win, int grow, int head, int section,
                                                   int local_col0) {
   if (p.push_n_local > 0) {
     const int owner = grow / p.push_n_local;
     return reinterpret_cast<__nv_bfloat16*>(p.dq_peers[owner]) +
            (static_cast<size_t>(win) * p.push_n_local + (grow - owner * p.push_n_local)) * p.push_ld +
-           section * p.push_sec_w + p.push_col0 + head * HD;
+           section * p.push_sec_w + p.push_col0 + head * p.d;
   }
-  return p.dQKV + (static_cast<size_t>(win) * p.N + grow) * p.ldg + local_col0 + head * HD;
+  return p.dQKV + (static_cast<size_t>(win) * p.N + grow) * p.ldg + local_col0 + head * p.d;
 }
 
 // Chains, ring depth and copies of the item's own operands per head width; the shared memory of one CTA per SM (227 KB)
@@ -692,8 +694,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         uint8_t* d = sQ + b * R::ITEM_BYTES;
 #pragma unroll
         for (int c = 0; c < DCH; ++c) {
-          tma_load_3d(d + c * 16384, &tm_q, &q_full[b], p.q_col0 + w.head * HD + c * 64, w.tile * TILE, w.win);
-          tma_load_3d(d + QB + c * 16384, &tm_do, &q_full[b], w.head * HD + c * 64, w.tile * TILE, w.win);
+          tma_load_4d(d + c * 16384, &tm_q, &q_full[b], c * 64, w.head, w.tile * TILE, w.win);
+          tma_load_4d(d + QB + c * 16384, &tm_do, &q_full[b], c * 64, w.head, w.tile * TILE, w.win);
         }
         return true;
       };
@@ -712,8 +714,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           mbar_expect_tx(bar, R::STAGE);
 #pragma unroll
           for (int c = 0; c < DCH; ++c) {
-            tma_load_3d(d + c * 8192, &tm_k, bar, p.k_col0 + w.head * HD + c * 64, j * BT, w.win);
-            tma_load_3d(d + KB + c * 8192, &tm_v, bar, p.v_col0 + w.head * HD + c * 64, j * BT, w.win);
+            tma_load_4d(d + c * 8192, &tm_k, bar, c * 64, w.head, j * BT, w.win);
+            tma_load_4d(d + KB + c * 8192, &tm_v, bar, c * 64, w.head, j * BT, w.win);
           }
           if (++st == NST) { st = 0; ph ^= 1; }
           if (j == j_item) {
@@ -806,7 +808,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       const BwdItem w = bwd_item(it, row_tiles, p.H);
       float* st = s_stat + b * 2 * TILE;
       const size_t sbase = (static_cast<size_t>(w.win) * p.H + w.head) * N + w.tile * TILE;
-      const size_t obase = (static_cast<size_t>(w.win) * N + w.tile * TILE) * p.ldo + w.head * HD + sub * 8;
+      const size_t obase = (static_cast<size_t>(w.win) * N + w.tile * TILE) * p.ldo + w.head * p.d + sub * 8;
       const int live = N - w.tile * TILE;            // rows of this tile inside the window
       float lse[2];
 #pragma unroll
@@ -821,7 +823,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         for (int u = 0; u < UN; ++u) {
           const int row = r + u * RPW + r0;
           a[u] = g[u] = make_uint4(0u, 0u, 0u, 0u);
-          if (row < live) {
+          if (row < live && sub * 8 < p.d) {
             a[u] = *reinterpret_cast<const uint4*>(p.O + obase + static_cast<size_t>(row) * p.ldo);
             g[u] = *reinterpret_cast<const uint4*>(p.dO + obase + static_cast<size_t>(row) * p.ldo);
           }
@@ -869,10 +871,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       const BwdItem w = bwd_item(it, row_tiles, p.H);
       const int grow = w.tile * TILE + row;
       const bool row_ok = grow < N;
-      __nv_bfloat16* dst = bwd_dst<HD>(p, w.win, row_ok ? grow : 0, w.head, 0, p.q_col0);
+      __nv_bfloat16* dst = bwd_dst(p, w.win, row_ok ? grow : 0, w.head, 0, p.q_col0);
 #pragma unroll
       for (int c = 0; c < HD; c += 32) {
-        if ((c / 32) % NWG != wg) continue;
+        if ((c / 32) % NWG != wg || c >= p.d) continue;
         uint32_t v[32];
         tmem_ld32(tdQ + lane_addr + c, v);
         tmem_wait_ld();
@@ -883,7 +885,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 #pragma unroll
             for (int i = 0; i < 4; ++i)
               o[i] = pack_bf16x2(__uint_as_float(v[8 * gq + 2 * i]) * sc, __uint_as_float(v[8 * gq + 2 * i + 1]) * sc);
-            *reinterpret_cast<uint4*>(dst + c + gq * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+            if (c + gq * 8 < p.d) *reinterpret_cast<uint4*>(dst + c + gq * 8) = make_uint4(o[0], o[1], o[2], o[3]);
           }
         }
       }
@@ -1030,8 +1032,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         uint8_t* d = sKV + b * R::ITEM_BYTES;
 #pragma unroll
         for (int c = 0; c < DCH; ++c) {
-          tma_load_3d(d + c * 16384, &tm_k, &kv_full[b], p.k_col0 + w.head * HD + c * 64, w.tile * TILE, w.win);
-          tma_load_3d(d + KB + c * 16384, &tm_v, &kv_full[b], p.v_col0 + w.head * HD + c * 64, w.tile * TILE, w.win);
+          tma_load_4d(d + c * 16384, &tm_k, &kv_full[b], c * 64, w.head, w.tile * TILE, w.win);
+          tma_load_4d(d + KB + c * 16384, &tm_v, &kv_full[b], c * 64, w.head, w.tile * TILE, w.win);
         }
         return true;
       };
@@ -1050,8 +1052,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           mbar_expect_tx(bar, R::STAGE);
 #pragma unroll
           for (int c = 0; c < DCH; ++c) {
-            tma_load_3d(d + c * 8192, &tm_q, bar, p.q_col0 + w.head * HD + c * 64, j * BT, w.win);
-            tma_load_3d(d + QB + c * 8192, &tm_do, bar, w.head * HD + c * 64, j * BT, w.win);
+            tma_load_4d(d + c * 8192, &tm_q, bar, c * 64, w.head, j * BT, w.win);
+            tma_load_4d(d + QB + c * 8192, &tm_do, bar, c * 64, w.head, j * BT, w.win);
           }
           if (++st == NST) { st = 0; ph ^= 1; }
           if (j == j_item) {
@@ -1193,15 +1195,16 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       const BwdItem w = bwd_item(it, row_tiles, p.H);
       const int grow = w.tile * TILE + row;
       const bool row_ok = grow < N;
-      __nv_bfloat16* dk = bwd_dst<HD>(p, w.win, row_ok ? grow : 0, w.head, 1, p.k_col0);
-      __nv_bfloat16* dv = bwd_dst<HD>(p, w.win, row_ok ? grow : 0, w.head, 2, p.v_col0);
+      __nv_bfloat16* dk = bwd_dst(p, w.win, row_ok ? grow : 0, w.head, 1, p.k_col0);
+      __nv_bfloat16* dv = bwd_dst(p, w.win, row_ok ? grow : 0, w.head, 2, p.v_col0);
 #pragma unroll
       for (int c = 0; c < 2 * HD; c += 32) {
-        if ((c / 32) % NWG != wg) continue;
+        const int col = c < HD ? c : c - HD;            // column inside the head
+        if ((c / 32) % NWG != wg || col >= p.d) continue;
         uint32_t v[32];
         tmem_ld32(tdK + lane_addr + c, v);
         tmem_wait_ld();
-        __nv_bfloat16* dst = (c < HD) ? dk + c : dv + (c - HD);
+        __nv_bfloat16* dst = ((c < HD) ? dk : dv) + col;
         const float f = (c < HD) ? sc : 1.f;
         if (row_ok) {
 #pragma unroll
@@ -1210,7 +1213,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 #pragma unroll
             for (int i = 0; i < 4; ++i)
               o[i] = pack_bf16x2(__uint_as_float(v[8 * gq + 2 * i]) * f, __uint_as_float(v[8 * gq + 2 * i + 1]) * f);
-            *reinterpret_cast<uint4*>(dst + gq * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+            if (col + gq * 8 < p.d) *reinterpret_cast<uint4*>(dst + gq * 8) = make_uint4(o[0], o[1], o[2], o[3]);
           }
         }
       }
@@ -1358,21 +1361,22 @@ static int attn_fwd_impl(const void* q, int ldq, int q_col0, const void* k, int 
                          float scale, int* status, void* stream_, const void* const* o_peers, int sp,
                          int push_n_local, int push_ld, int push_col0) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
-  if (head_dim != 64 && head_dim != 128) return -1;
+  if (head_dim <= 0 || head_dim > 128 || head_dim % 8) return -1;
   if (n_win <= 0 || N <= 0 || H <= 0 || n_win > 65535 || H > 65535) return -2;
   if (sp < 0 || sp > 8 || (!o && !o_peers)) return -3;
   AttnFwdParams p{};
   for (int i = 0; i < sp; ++i) p.o_peers[i] = const_cast<void*>(o_peers[i]);
   p.push_n_local = o_peers ? push_n_local : 0; p.push_ld = push_ld; p.push_col0 = push_col0;
   p.O = reinterpret_cast<__nv_bfloat16*>(o); p.ldo = ldo; p.lse = lse; p.N = N; p.H = H; p.n_win = n_win;
-  p.q_col0 = q_col0; p.k_col0 = k_col0; p.v_col0 = v_col0;
+  p.d = head_dim;
   p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
   CUtensorMap tq, tk, tv;
   int r;
-  if ((r = make_tmap_3d_bf16(&tq, q, ldq, N, n_win, ldq, static_cast<uint64_t>(N) * ldq, 64, TILE))) return r;
-  if ((r = make_tmap_3d_bf16(&tk, k, ldk, N, n_win, ldk, static_cast<uint64_t>(N) * ldk, 64, KVT))) return r;
-  if ((r = make_tmap_3d_bf16(&tv, v, ldv, N, n_win, ldv, static_cast<uint64_t>(N) * ldv, 64, KVT))) return r;
-  if (head_dim == 128) {
+  auto at = [](const void* base, int col) { return static_cast<const void*>(reinterpret_cast<const __nv_bfloat16*>(base) + col); };
+  if ((r = make_tmap_heads_bf16(&tq, at(q, q_col0), head_dim, H, N, n_win, ldq, TILE))) return r;
+  if ((r = make_tmap_heads_bf16(&tk, at(k, k_col0), head_dim, H, N, n_win, ldk, KVT))) return r;
+  if ((r = make_tmap_heads_bf16(&tv, at(v, v_col0), head_dim, H, N, n_win, ldv, KVT))) return r;
+  if (head_dim > 64) {
     switch (g_fwd_mode) {
       case 1: return launch_attn_fwd<2, -1, 1>(tq, tk, tv, p, stream);
       default: return launch_attn_fwd<2, -1, 0>(tq, tk, tv, p, stream);
@@ -1417,7 +1421,7 @@ static int attn_bwd_impl(const void* qkv, int ldq, int q_col0, int k_col0, int v
                          int head_dim, float scale, int* status, void* stream_, const void* const* dq_peers, int sp,
                          int push_n_local, int push_ld, int push_sec_w, int push_col0) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
-  if (head_dim != 64 && head_dim != 128) return -1;
+  if (head_dim <= 0 || head_dim > 128 || head_dim % 8) return -1;
   if (n_win <= 0 || N <= 0 || H <= 0 || n_win > 65535 || H > 65535) return -2;
   if (sp < 0 || sp > 8 || (!dqkv && !dq_peers)) return -3;
   AttnBwdParams p{};
@@ -1425,17 +1429,18 @@ static int attn_bwd_impl(const void* qkv, int ldq, int q_col0, int k_col0, int v
   p.push_n_local = dq_peers ? push_n_local : 0; p.push_ld = push_ld; p.push_sec_w = push_sec_w; p.push_col0 = push_col0;
   p.O = reinterpret_cast<const __nv_bfloat16*>(o); p.dO = reinterpret_cast<const __nv_bfloat16*>(d_o); p.ldo = ldo;
   p.lse = lse; p.delta = delta; p.dQKV = reinterpret_cast<__nv_bfloat16*>(dqkv); p.ldg = ldg;
-  p.N = N; p.H = H; p.n_win = n_win; p.q_col0 = q_col0; p.k_col0 = k_col0; p.v_col0 = v_col0;
+  p.N = N; p.H = H; p.n_win = n_win; p.d = head_dim; p.q_col0 = q_col0; p.k_col0 = k_col0; p.v_col0 = v_col0;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
-  CUtensorMap t128, t64, d128, d64;
+  CUtensorMap q128, q64, k128, k64, v128, v64, d128, d64;
   int r;
-  const uint64_t wq = static_cast<uint64_t>(N) * ldq, wo = static_cast<uint64_t>(N) * ldo;
-  if ((r = make_tmap_3d_bf16(&t128, qkv, ldq, N, n_win, ldq, wq, 64, TILE))) return r;
-  if ((r = make_tmap_3d_bf16(&t64, qkv, ldq, N, n_win, ldq, wq, 64, BT))) return r;
-  if ((r = make_tmap_3d_bf16(&d128, d_o, ldo, N, n_win, ldo, wo, 64, TILE))) return r;
-  if ((r = make_tmap_3d_bf16(&d64, d_o, ldo, N, n_win, ldo, wo, 64, BT))) return r;
-  return head_dim == 64 ? launch_attn_bwd<1>(t128, t64, t64, d128, t64, t128, t128, d64, p, stream)
-                        : launch_attn_bwd<2>(t128, t64, t64, d128, t64, t128, t128, d64, p, stream);
+  const __nv_bfloat16* b = reinterpret_cast<const __nv_bfloat16*>(qkv);
+  const struct { CUtensorMap* m; const void* base; int ld; uint32_t rows; } maps[] = {
+      {&q128, b + q_col0, ldq, TILE}, {&q64, b + q_col0, ldq, BT}, {&k128, b + k_col0, ldq, TILE}, {&k64, b + k_col0, ldq, BT},
+      {&v128, b + v_col0, ldq, TILE}, {&v64, b + v_col0, ldq, BT}, {&d128, d_o, ldo, TILE},        {&d64, d_o, ldo, BT}};
+  for (const auto& m : maps)
+    if ((r = make_tmap_heads_bf16(m.m, m.base, head_dim, H, N, n_win, m.ld, m.rows))) return r;
+  return head_dim <= 64 ? launch_attn_bwd<1>(q128, k64, v64, d128, q64, k128, v128, d64, p, stream)
+                        : launch_attn_bwd<2>(q128, k64, v64, d128, q64, k128, v128, d64, p, stream);
 }
 
 // ------------------------------------------------------------------------------------------ allocation-free variant

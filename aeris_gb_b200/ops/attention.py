@@ -9,12 +9,11 @@ from . import lib as _l
 
 
 def _kernel_dim(d: int) -> int:
-    """The kernels are built for 64- and 128-wide heads; other widths (for example 32) run zero-padded to the next one:
-    zero columns change neither Q K^T nor the valid columns of P V."""
-    if d in (64, 128):
-        return d
-    assert 0 < d < 128, f"head_dim {d} is not supported"
-    return 64 if d < 64 else 128
+    """The kernels take heads of up to 128 channels in whole 16-byte vectors (narrower heads than the kernel's 64 or 128 are
+    padded by the tensor maps on the way into shared memory); other widths run zero-padded to the next multiple of
+    eight: zero columns change neither Q K^T nor the valid columns of P V."""
+    assert 0 < d <= 128, f"head_dim {d} is not supported"
+    return (d + 7) // 8 * 8
 
 
 def _pad_heads(t: torch.Tensor, parts: int, H: int, d: int, dp: int) -> torch.Tensor:

@@ -200,6 +200,26 @@ def test_gemm_accumulate_splits(M, N, K, k_splits):
     assert rel_err(out, a.double().t() @ b.double() + 1) < K / 16 * 2.0 ** -23 + 1e-6
 
 
+@pytest.mark.parametrize("d", [8, 20, 32, 72, 96])
+@pytest.mark.parametrize("nw,N,H", [(3, 64, 4), (2, 129, 3), (2, 225, 5)])
+def test_attention_narrow_heads(nw, N, H, d):
+    """Heads that do not fill the kernel's 64 or 128 channels: the tensor maps must not read the neighbouring head's
+    channels and the stores must not touch them (20: padded by the caller to whole vectors). Tolerance as below."""
+    from aeris_gb_b200.ops import attention as A
+    qkv = torch.randn(nw * N, 3 * H * d, device=DEV).bfloat16()
+    go = torch.randn(nw * N, H * d, device=DEV).bfloat16()
+    o, lse = A.attn_fwd(qkv, nw, N, H, d)
+    dqkv = torch.full_like(qkv, float("nan"))
+    A.attn_bwd(qkv, o, go, lse, nw, N, H, d, dqkv=dqkv)
+    x = qkv.float().requires_grad_(True)
+    ref = A.attn_reference(x, nw, N, H, d)
+    ref.backward(go.float())
+    assert rel_err(o, ref) < 6e-3
+    HD = H * d
+    for i in range(3):
+        assert rel_err(dqkv[:, i * HD:(i + 1) * HD], x.grad[:, i * HD:(i + 1) * HD]) < 6e-3
+
+
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("nw,N,H", [(2, 15, 2), (3, 64, 1), (40, 64, 8), (2, 65, 2), (1, 127, 2), (2, 129, 3), (5, 225, 30)])
 def test_attention_bwd_tile_edges(nw, N, H, d):
