@@ -47,6 +47,9 @@ int aeris_attn_bwd_push(const void* qkv, int ld, int H_local, const void* o, con
 int aeris_modnorm_fwd(const void* x, const void* gidx, const void* const* peer_ptrs, int n_peers, void* x_out,
                       const float* scale, const float* shift, const void* w, void* h, int rows, int D, int mode,
                       float eps, const float* w_f32, void* h_lo, void* stream);
+int aeris_modnorm_fwd_batch(const void* x, const void* gidx, const void* const* peer_ptrs, int n_peers, void* x_out,
+                            const float* scale, const float* shift, const void* w, void* h, int batch, int rows, int D,
+                            int mode, float eps, const float* w_f32, void* h_lo, void* stream);
 int aeris_modnorm_bwd(const void* x, const void* dh, const void* dres, const float* scale, const float* shift,
                       const void* w, void* dx, float* dscale, float* dshift, float* dw, int rows, int D, int mode,
                       float eps, const float* w_f32, void* stream);

@@ -253,6 +253,16 @@ modnorm_fwd_pair_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __r
                         const float* __restrict__ wf, __nv_bfloat16* __restrict__ h_lo) {
   static_assert(FWD_RPI == 4 && MAXT <= 256 * W8, "group_sum4 adds four values of at most 8 * W8 warps");
   __shared__ float red[2][32 * W8];
+  {  // grid.y = samples of `rows` rows each, with a modulation vector of their own
+    const size_t r0 = static_cast<size_t>(blockIdx.y) * rows;
+    if (x) x += r0 * D;
+    if (gidx) gidx += r0;
+    if (x_out) x_out += r0 * D;
+    h += r0 * D;
+    if (h_lo) h_lo += r0 * D;
+    if (scale) scale += static_cast<size_t>(blockIdx.y) * D;
+    if (shift) shift += static_cast<size_t>(blockIdx.y) * D;
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int i = threadIdx.x; i < 64 * W8; i += blockDim.x) (&red[0][0])[i] = 0.f;
   const int c0 = threadIdx.x * 8;
@@ -984,10 +994,10 @@ static int pick_rows_per_cta(int rows) {
   return rpc;
 }
 
-extern "C" int aeris_modnorm_fwd(const void* x, const void* gidx, const void* const* peer_ptrs, int n_peers,
+static int modnorm_fwd_impl(const void* x, const void* gidx, const void* const* peer_ptrs, int n_peers,
                                  void* x_out, const float* scale, const float* shift, const void* w, void* h,
                                  int rows, int D, int mode, float eps, const float* w_f32, void* h_lo,
-                                 void* stream) {
+                                 int batch, void* stream) {
   if (D % 8 || D > 8192 || rows <= 0 || (!w && !w_f32)) return -1;
   PeerPtrs pp{};
   for (int i = 0; i < n_peers && i < 16; ++i) pp.p[i] = reinterpret_cast<const __nv_bfloat16*>(peer_ptrs[i]);
@@ -998,10 +1008,11 @@ extern "C" int aeris_modnorm_fwd(const void* x, const void* gidx, const void* co
   if (D <= 5120) {
     // as many CTAs as the registers of an SM hold at once, each sweeping over the rows
     const int nt = row_threads(D), per_sm = nt > 320 ? 1 : nt > 192 ? 2 : 576 / nt;
-    if (grid > aeris_num_sms() * per_sm) grid = aeris_num_sms() * per_sm;
+    const int cap = (aeris_num_sms() * per_sm + batch - 1) / batch;
+    if (grid > cap) grid = cap;
     auto kern = nt <= 192 ? modnorm_fwd_pair_kernel<192, 3, 1>
               : nt <= 320 ? modnorm_fwd_pair_kernel<320, 2, 2> : modnorm_fwd_pair_kernel<640, 1, 3>;
-    kern<<<grid, nt, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+    kern<<<dim3(grid, batch), nt, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
         reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const uint32_t*>(gidx), pp,
         reinterpret_cast<__nv_bfloat16*>(x_out), scale, shift, reinterpret_cast<const __nv_bfloat16*>(w),
         reinterpret_cast<__nv_bfloat16*>(h), rows, D, mode, eps, w_f32, reinterpret_cast<__nv_bfloat16*>(h_lo));
@@ -1013,6 +1024,33 @@ extern "C" int aeris_modnorm_fwd(const void* x, const void* gidx, const void* co
       reinterpret_cast<__nv_bfloat16*>(x_out), scale, shift, reinterpret_cast<const __nv_bfloat16*>(w),
       reinterpret_cast<__nv_bfloat16*>(h), rows, D, mode, eps, rpc, w_f32, reinterpret_cast<__nv_bfloat16*>(h_lo));
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
+}
+
+extern "C" int aeris_modnorm_fwd(const void* x, const void* gidx, const void* const* peer_ptrs, int n_peers,
+                                 void* x_out, const float* scale, const float* shift, const void* w, void* h,
+                                 int rows, int D, int mode, float eps, const float* w_f32, void* h_lo,
+                                 void* stream) {
+  return modnorm_fwd_impl(x, gidx, peer_ptrs, n_peers, x_out, scale, shift, w, h, rows, D, mode, eps, w_f32, h_lo, 1, stream);
+}
+
+// The same for `batch` samples of `rows` consecutive rows each, scale and shift [batch, D]: one launch where D <= 5120.
+extern "C" int aeris_modnorm_fwd_batch(const void* x, const void* gidx, const void* const* peer_ptrs, int n_peers,
+                                       void* x_out, const float* scale, const float* shift, const void* w, void* h,
+                                       int batch, int rows, int D, int mode, float eps, const float* w_f32, void* h_lo,
+                                       void* stream) {
+  if (batch <= 0 || batch > 65535) return -1;
+  if (D <= 5120)
+    return modnorm_fwd_impl(x, gidx, peer_ptrs, n_peers, x_out, scale, shift, w, h, rows, D, mode, eps, w_f32, h_lo, batch, stream);
+  auto at = [](const void* p, size_t bytes) -> char* { return p ? reinterpret_cast<char*>(const_cast<void*>(p)) + bytes : nullptr; };
+  for (int b = 0; b < batch; ++b) {
+    const size_t r = static_cast<size_t>(b) * rows, e = r * D * 2;
+    const int rc = modnorm_fwd_impl(at(x, e), at(gidx, r * 4), peer_ptrs, n_peers, at(x_out, e),
+                                    scale ? scale + static_cast<size_t>(b) * D : nullptr,
+                                    shift ? shift + static_cast<size_t>(b) * D : nullptr, w, at(h, e), rows, D, mode, eps,
+                                    w_f32, at(h_lo, e), 1, stream);
+    if (rc) return rc;
+  }
+  return 0;
 }
 
 extern "C" int aeris_modnorm_bwd(const void* x, const void* dh, const void* dres, const float* scale,

@@ -174,6 +174,17 @@ def chunk_step(meta: BlockMeta, D: int, F: int) -> int:
     return min(max(meta.chunk_windows, floor), meta.n_win_per_sample)
 
 
+def _forward_spans(meta: BlockMeta, B: int, step: int, D: int, F: int, kept: bool) -> list[tuple[int, int, int, int]]:
+    """What one pass over the forward kernels covers: (first sample, first window, windows, samples). Samples that are one
+    chunk each run in one launch per kernel (their modulation vectors are picked by row), when their internals are kept
+    anyway or take less than the smallest chunk; the exchanges of the parallel paths work on one sample at a time."""
+    row = kept_bytes(1, D, meta.heads * meta.head_dim, meta.heads, F)
+    if (B > 1 and step == meta.n_win_per_sample and meta.sp is None and meta.tp is None
+            and (kept or B * step * meta.L * row <= MIN_CHUNK_BYTES) and B * step <= 65535):
+        return [(0, 0, B * step, B)]
+    return [(b, w0, nw, 1) for b in range(B) for w0, nw in _chunks(meta, step)]
+
+
 def _chunks(meta: BlockMeta, step: int):
     for w0 in range(0, meta.n_win_per_sample, step):
         yield w0, min(step, meta.n_win_per_sample - w0)
@@ -270,47 +281,47 @@ def block_forward(x: torch.Tensor, mod: torch.Tensor, meta: BlockMeta, wn1, wqkv
     y = out if out is not None else torch.empty_like(x)
     ws, dev, bf = _WS, x.device, torch.bfloat16
     step = chunk_step(meta, D, F)
+    spans = _forward_spans(meta, B, step, D, F, kept is not None)
     if kept is None:
-        cmax = step * meta.L
+        cmax = max(nw for _, _, nw, _ in spans) * meta.L
         h = ws.get("h", (cmax, D), bf, dev)
         tpn = meta.tp.tp if meta.tp is not None else 1   # gathered rows x local features: the same element count
         chunk_bufs = {"h1": h, "qkv": ws.get("qkv", (cmax, 3 * HD), bf, dev), "o": ws.get("o", (cmax, HD), bf, dev),
                       "lse": ws.get("lse", (cmax * meta.heads,), torch.float32, dev),
                       "x1": ws.get("x1", (cmax, D), bf, dev), "h2": h, "act": ws.get("act", (cmax * tpn, F), bf, dev)}
-    mod = mod.contiguous()
-    for b in range(B):
-        sh1, sc1, g1, sh2, sc2, g2 = [mod[b, i * D:(i + 1) * D] for i in range(6)]
-        for w0, nw in _chunks(meta, step):
-            r0 = b * rows_per_sample + w0 * meta.L
-            n = nw * meta.L
-            xc = x[r0:r0 + n]
-            h1, qkv, o, x1, h2, act, lse = _chunk_views(kept, r0, n, meta.heads) if kept is not None else \
-                _chunk_views(chunk_bufs, 0, n, meta.heads)
-            if gather is not None:
-                table, peers, src = gather
-                E.modnorm_fwd(None, sc1, sh1, wn1, mode=meta.mode, eps=meta.eps, out=h1,
-                              gather_idx=table[r0:r0 + n], peer_ptrs=peers, x_out=xc, rows=n,
-                              src_rows=src.shape[0])
-            else:
-                E.modnorm_fwd(xc, sc1, sh1, wn1, mode=meta.mode, eps=meta.eps, out=h1)
-            if meta.sp is None:
-                G.gemm(h1, wqkv, out=qkv)
-                if meta.rope is not None:
-                    _rope_qk_(qkv, meta, nw)
-                A.attn_fwd(qkv, nw, meta.L, meta.heads, meta.head_dim, out=o, lse=lse.view(nw, meta.heads, meta.L))
-                oc = o
-            else:
-                oc = _sp_attention_fwd(meta, h1, wqkv, nw, keep_local=False)[0]
-            G.gemm(oc, wo, out=x1, epi=G.EPI_GATE_RESID, resid=xc, gate=g1)
-            if meta.tp is not None:
-                _tp_mlp_fwd(meta.tp, x1, sc2, sh2, wn2, meta, w1, w2, g2, chunk_bufs["act"], y[r0:r0 + n])
-                continue
-            E.modnorm_fwd(x1, sc2, sh2, wn2, mode=meta.mode, eps=meta.eps, out=h2)
-            if kept is not None:
-                G.gemm(h2, w1, out=act, epi=G.EPI_SWIGLU_BOTH, aux=kept["u"][r0:r0 + n])
-            else:
-                G.gemm(h2, w1, out=act, epi=G.EPI_SWIGLU)
-            G.gemm(act, w2, out=y[r0:r0 + n], epi=G.EPI_GATE_RESID, resid=x1, gate=g2)
+    mods = mod.reshape(B, 6, D).transpose(0, 1).contiguous()           # [6, B, D]: every vector of all samples in a row
+    for b, w0, nw, nb in spans:
+        sh1, sc1, g1, sh2, sc2, g2 = (mods[:, b] if nb == 1 else mods[:, b:b + nb]).unbind(0)
+        r0 = b * rows_per_sample + w0 * meta.L
+        n = nw * meta.L
+        xc = x[r0:r0 + n]
+        h1, qkv, o, x1, h2, act, lse = _chunk_views(kept, r0, n, meta.heads) if kept is not None else \
+            _chunk_views(chunk_bufs, 0, n, meta.heads)
+        if gather is not None:
+            table, peers, src = gather
+            E.modnorm_fwd(None, sc1, sh1, wn1, mode=meta.mode, eps=meta.eps, batch=nb, out=h1,
+                          gather_idx=table[r0:r0 + n], peer_ptrs=peers, x_out=xc, rows=n,
+                          src_rows=src.shape[0])
+        else:
+            E.modnorm_fwd(xc, sc1, sh1, wn1, mode=meta.mode, eps=meta.eps, batch=nb, out=h1)
+        if meta.sp is None:
+            G.gemm(h1, wqkv, out=qkv)
+            if meta.rope is not None:
+                _rope_qk_(qkv, meta, nw)
+            A.attn_fwd(qkv, nw, meta.L, meta.heads, meta.head_dim, out=o, lse=lse.view(nw, meta.heads, meta.L))
+            oc = o
+        else:
+            oc = _sp_attention_fwd(meta, h1, wqkv, nw, keep_local=False)[0]
+        G.gemm(oc, wo, out=x1, epi=G.EPI_GATE_RESID, resid=xc, gate=g1, rows_per_gate=n // nb)
+        if meta.tp is not None:
+            _tp_mlp_fwd(meta.tp, x1, sc2, sh2, wn2, meta, w1, w2, g2, chunk_bufs["act"], y[r0:r0 + n])
+            continue
+        E.modnorm_fwd(x1, sc2, sh2, wn2, mode=meta.mode, eps=meta.eps, batch=nb, out=h2)
+        if kept is not None:
+            G.gemm(h2, w1, out=act, epi=G.EPI_SWIGLU_BOTH, aux=kept["u"][r0:r0 + n])
+        else:
+            G.gemm(h2, w1, out=act, epi=G.EPI_SWIGLU)
+        G.gemm(act, w2, out=y[r0:r0 + n], epi=G.EPI_GATE_RESID, resid=x1, gate=g2, rows_per_gate=n // nb)
     return y
 
 

@@ -112,20 +112,24 @@ def _head_weights(head_w: torch.Tensor):
     return DF.pack_head_weights(head_w.detach().float().contiguous(), PAD_N)
 
 
-def _head_rows(x, scale_b, shift_b, norm_w, w_hi, w_lo, eps, pred, y_hi, y_lo):
-    """pred[n, 128] (fp32) = (RMSNorm(x) * w * (1 + scale) + shift) @ head^T for ``n`` rows of one sample."""
+def _head_rows(x, scale, shift, norm_w, w_hi, w_lo, eps, pred, y_hi, y_lo):
+    """pred[n, 128] (fp32) = (RMSNorm(x) * w * (1 + scale) + shift) @ head^T for ``n`` rows of ``scale.shape[0]`` samples."""
     n = x.shape[0]
-    E.modnorm_fwd(x, scale_b, shift_b, norm_w, mode=E.MODE_NORM_THEN_MOD, eps=eps, out=y_hi[:n], out_lo=y_lo[:n])
+    E.modnorm_fwd(x, scale, shift, norm_w, mode=E.MODE_NORM_THEN_MOD, eps=eps, out=y_hi[:n], out_lo=y_lo[:n],
+                  batch=scale.shape[0])
     G.gemm(y_hi[:n], w_hi, out=pred[:n], epi=G.EPI_STORE_F32)
     G.gemm(y_lo[:n], w_hi, out=pred[:n], epi=G.EPI_ACC_F32)
     G.gemm(y_hi[:n], w_lo, out=pred[:n], epi=G.EPI_ACC_F32)
     return pred[:n]
 
 
-def _sample_chunks(B: int, rows_per_sample: int):
-    for b in range(B):
-        for r in range(0, rows_per_sample, CHUNK_ROWS):
-            yield b, b * rows_per_sample + r, min(CHUNK_ROWS, rows_per_sample - r)
+def _sample_chunks(B: int, rows_per_sample: int) -> list[tuple[int, int, int, int]]:
+    """(first sample, samples, first row, rows) of every pass over the head: all samples at once where they fit one
+    chunk, else chunks of one sample."""
+    if B * rows_per_sample <= CHUNK_ROWS:
+        return [(0, B, 0, B * rows_per_sample)]
+    return [(b, 1, b * rows_per_sample + r, min(CHUNK_ROWS, rows_per_sample - r))
+            for b in range(B) for r in range(0, rows_per_sample, CHUNK_ROWS)]
 
 
 def head_forward(x: torch.Tensor, shift: torch.Tensor, scale: torch.Tensor, norm_w: torch.Tensor,
@@ -136,13 +140,14 @@ def head_forward(x: torch.Tensor, shift: torch.Tensor, scale: torch.Tensor, norm
     dev = x.device
     w_hi, w_lo = _head_weights(head_w)
     ws = workspace()
-    cm = min(CHUNK_ROWS, T // B)
+    spans = _sample_chunks(B, T // B)
+    cm = max(n for *_, n in spans)
     y_hi = ws.get("head_yhi", (cm, D), torch.bfloat16, dev)
     y_lo = ws.get("head_ylo", (cm, D), torch.bfloat16, dev)
     pred = torch.empty((T, PAD_N), dtype=torch.float32, device=dev)
     shift, scale = shift.float().contiguous(), scale.float().contiguous()
-    for b, r0, n in _sample_chunks(B, T // B):
-        _head_rows(x[r0:r0 + n], scale[b], shift[b], norm_w, w_hi, w_lo, eps, pred[r0:r0 + n], y_hi, y_lo)
+    for b, nb, r0, n in spans:
+        _head_rows(x[r0:r0 + n], scale[b:b + nb], shift[b:b + nb], norm_w, w_hi, w_lo, eps, pred[r0:r0 + n], y_hi, y_lo)
     return pred
 
 
@@ -158,7 +163,8 @@ class HeadLossFn(torch.autograd.Function):
         dev = x.device
         w_hi, w_lo = _head_weights(head_w)
         ws = workspace()
-        cm = min(CHUNK_ROWS, T // B)
+        spans = _sample_chunks(B, T // B)
+        cm = max(n for *_, n in spans)
         y_hi = ws.get("head_yhi", (cm, D), torch.bfloat16, dev)
         y_lo = ws.get("head_ylo", (cm, D), torch.bfloat16, dev)
         pred = ws.get("head_pred", (cm, PAD_N), torch.float32, dev)
@@ -166,8 +172,8 @@ class HeadLossFn(torch.autograd.Function):
         loss = torch.zeros(1, dtype=torch.float64, device=dev)
         shift32, scale32 = shift.float().contiguous(), scale.float().contiguous()
         inv_rows = 1.0 / (T // B)
-        for b, r0, n in _sample_chunks(B, T // B):
-            _head_rows(x[r0:r0 + n], scale32[b], shift32[b], norm_w, w_hi, w_lo, plan.eps, pred, y_hi, y_lo)
+        for b, nb, r0, n in spans:
+            _head_rows(x[r0:r0 + n], scale32[b:b + nb], shift32[b:b + nb], norm_w, w_hi, w_lo, plan.eps, pred, y_hi, y_lo)
             DF.trigflow_loss(pred[:n], x_img, cs, plan.geom, plan.seed, plan.sigma_data, plan.w_var, plan.w_lat,
                              inv_rows, loss, dpred=dpred[r0:r0 + n], row0=r0)
         ctx.plan = plan
@@ -184,7 +190,8 @@ class HeadLossFn(torch.autograd.Function):
         dev = x.device
         w_hi, _ = _head_weights(head_w)
         ws = workspace()
-        cm = min(CHUNK_ROWS, T // B)
+        spans = _sample_chunks(B, T // B)
+        cm = max(n for *_, n in spans)
         y_hi = ws.get("head_yhi", (cm, D), torch.bfloat16, dev)
         dy = ws.get("head_ylo", (cm, D), torch.bfloat16, dev)
         Gh = ws.get("head_g", (PAD_N, D), torch.float32, dev, zero=True)
@@ -193,14 +200,18 @@ class HeadLossFn(torch.autograd.Function):
         s_nw, r_nw = _grad_slot(norm_w)
         dx = torch.empty_like(x)
         dpred = dpred * g.to(dpred.dtype)
-        for b, r0, n in _sample_chunks(B, T // B):
-            E.modnorm_fwd(x[r0:r0 + n], scale32[b], shift32[b], norm_w, mode=E.MODE_NORM_THEN_MOD, eps=plan.eps,
-                          out=y_hi[:n])
+        for b, nb, r0, n in spans:
+            E.modnorm_fwd(x[r0:r0 + n], scale32[b:b + nb], shift32[b:b + nb], norm_w, mode=E.MODE_NORM_THEN_MOD,
+                          eps=plan.eps, out=y_hi[:n], batch=nb)
             dp = dpred[r0:r0 + n]
             G.gemm(dp, y_hi[:n], a_t=True, b_t=True, out=Gh, epi=G.EPI_ACC_F32, k_splits=16, two_cta=False)
             G.gemm(dp, w_hi, b_t=True, out=dy[:n])
-            E.modnorm_bwd(x[r0:r0 + n], dy[:n], None, scale32[b], shift32[b], norm_w, mode=E.MODE_NORM_THEN_MOD,
-                          eps=plan.eps, dx=dx[r0:r0 + n], dscale=dscale[b], dshift=dshift[b], dw=s_nw)
+            m = n // nb
+            for i in range(nb):        # column sums per sample
+                sl = slice(r0 + i * m, r0 + (i + 1) * m)
+                E.modnorm_bwd(x[sl], dy[i * m:(i + 1) * m], None, scale32[b + i], shift32[b + i], norm_w,
+                              mode=E.MODE_NORM_THEN_MOD, eps=plan.eps, dx=dx[sl], dscale=dscale[b + i],
+                              dshift=dshift[b + i], dw=s_nw)
         s_hw, r_hw = _grad_slot(head_w)
         s_hw += Gh[:C]
         return (dx, dshift.to(shift.dtype), dscale.to(scale.dtype), r_nw.to(norm_w.dtype) if r_nw is not None else None,

@@ -21,8 +21,8 @@ def modnorm_fwd(x: torch.Tensor, scale: torch.Tensor | None, shift: torch.Tensor
                 mode: int, eps: float, out: torch.Tensor | None = None, gather_idx: torch.Tensor | None = None,
                 peer_ptrs: list[int] | None = None, x_out: torch.Tensor | None = None,
                 rows: int | None = None, out_lo: torch.Tensor | None = None,
-                src_rows: int | None = None) -> torch.Tensor:
-    """``w`` bf16, or fp32 (the output head's norm); ``out_lo`` optionally receives ``h - bf16(h)``. ``src_rows``:
+                src_rows: int | None = None, batch: int = 1) -> torch.Tensor:
+    """``batch`` > 1: the rows are that many samples of equal length, ``scale`` and ``shift`` are [batch, D]. ``w`` bf16, or fp32 (the output head's norm); ``out_lo`` optionally receives ``h - bf16(h)``. ``src_rows``:
     rows of every peer buffer the gather table points into (used by the checking build only)."""
     D = w.numel()
     rows = rows if rows is not None else (gather_idx.numel() if gather_idx is not None else x.shape[0])
@@ -32,9 +32,12 @@ def modnorm_fwd(x: torch.Tensor, scale: torch.Tensor | None, shift: torch.Tensor
         out = torch.empty((rows, D), dtype=torch.bfloat16, device=w.device)
     peers = _peer_array(peer_ptrs) if gather_idx is not None else None
     w32, w = (w, None) if w.dtype == torch.float32 else (None, w)
-    rc = _l.lib().aeris_modnorm_fwd(_l.ptr(x), _l.ptr(gather_idx), peers, len(peer_ptrs) if peer_ptrs else 0,
-                                    _l.ptr(x_out), _l.ptr(scale), _l.ptr(shift), _l.ptr(w), _l.ptr(out), rows, D,
-                                    mode, _l._c_float(eps), _l.ptr(w32), _l.ptr(out_lo), _l.stream_ptr())
+    assert batch == 1 or (rows % batch == 0 and all(v is None or (v.is_contiguous() and v.numel() == batch * D)
+                                                    for v in (scale, shift)))
+    rc = _l.lib().aeris_modnorm_fwd_batch(_l.ptr(x), _l.ptr(gather_idx), peers, len(peer_ptrs) if peer_ptrs else 0,
+                                          _l.ptr(x_out), _l.ptr(scale), _l.ptr(shift), _l.ptr(w), _l.ptr(out), batch,
+                                          rows // batch, D, mode, _l._c_float(eps), _l.ptr(w32), _l.ptr(out_lo),
+                                          _l.stream_ptr())
     _l.check(rc, "aeris_modnorm_fwd")
     return out
 

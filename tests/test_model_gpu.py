@@ -183,3 +183,35 @@ def test_kept_internals_give_the_gradients_of_the_recompute(mod_first, monkeypat
             for n, g in runs[0][1].items():
                 # bf16 gradients of bf16 weights: an atomic sum in another order may round to the neighbouring value
                 assert rel_err(got[n], g) < 2.0 ** -9, n
+
+
+@pytest.mark.parametrize("dim,heads", [(256, 4), (5376, 42)])
+def test_samples_in_one_launch_equal_samples_one_by_one(dim, heads):
+    """A batch whose samples are one chunk each runs every forward kernel once, with the modulation vectors picked by row:
+    the same values as each sample alone, bit for bit (windows of 225 tokens: tiles straddle the sample boundary). 5376
+    columns: no batched modulate + norm launch, one per sample."""
+    from aeris_gb_b200.models import fused
+    from aeris_gb_b200.ops import elementwise as E
+    torch.manual_seed(1)
+    L, n_win, B, F = 225, 3, 3, 512
+    if dim > 5120:
+        x = torch.randn(4, dim, device="cuda").bfloat16()
+        w, sc = torch.ones(dim, device="cuda").bfloat16(), torch.randn(2, dim, device="cuda")
+        try:
+            one = [E.modnorm_fwd(x[2 * b:2 * b + 2], sc[b], sc[b], w, mode=0, eps=1e-3) for b in range(2)]
+        except Exception:
+            pytest.skip("rows this wide are not taken")
+        assert torch.equal(E.modnorm_fwd(x, sc, sc, w, mode=0, eps=1e-3, batch=2), torch.cat(one))
+        return
+    meta = fused.BlockMeta(n_win, L, heads, dim // heads, E.MODE_MOD_THEN_NORM, 1e-3, 64)
+    T = B * n_win * L
+    x = torch.randn(T, dim, device="cuda").bfloat16()
+    mod = torch.randn(B, 6 * dim, device="cuda")
+    ws = [torch.ones(dim), torch.randn(3 * dim, dim) * 0.05, torch.randn(dim, dim) * 0.05, torch.ones(dim),
+          torch.randn(2 * F, dim) * 0.05, torch.randn(dim, F) * 0.05]
+    ws = [w.cuda().bfloat16() for w in ws]
+    assert len(fused._forward_spans(meta, B, n_win, dim, F, False)) == 1
+    y = fused.block_forward(x, mod, meta, *ws)
+    n = n_win * L
+    for b in range(B):
+        assert torch.equal(y[b * n:(b + 1) * n], fused.block_forward(x[b * n:(b + 1) * n], mod[b:b + 1], meta, *ws))
