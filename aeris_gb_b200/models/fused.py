@@ -157,7 +157,7 @@ def plan_kept_blocks(T: int, D: int, HD: int, heads: int, F: int, n_blocks: int,
     stats = torch.cuda.memory_stats_as_nested_dict(device)
     held = [stats.get(k, {}).get("all", {}).get("current", 0) for k in ("reserved_bytes", "allocated_bytes")]
     cached = max(0, held[0] - held[1])
-    if n_blocks * per_block + base <= cached:      # nothing new to ask the driver for (any step after the first)
+    if n_blocks * (per_block + T * D * 2) <= cached:      # an earlier step's buffers, ready to be handed out again
         return n_blocks
     free = cached + torch.cuda.mem_get_info(device)[0]
     return n_kept(n_blocks, per_block, base, free)

@@ -9,11 +9,17 @@ from . import lib as _l
 
 
 def _kernel_dim(d: int) -> int:
-    """The kernels take heads of up to 128 channels in whole 16-byte vectors (narrower heads than the kernel's 64 or 128 are
-    padded by the tensor maps on the way into shared memory); other widths run zero-padded to the next multiple of
-    eight: zero columns change neither Q K^T nor the valid columns of P V."""
-    assert 0 < d <= 128, f"head_dim {d} is not supported"
-    return (d + 7) // 8 * 8
+    """Width that the kernels compute a head of ``d`` channels at."""
+    if d in (64, 128):
+        return d
+    assert 0 < d < 128, f"head_dim {d} is not supported"
+    return 64 if d < 64 else 128
+
+
+def _padded_dim(d: int) -> int:
+    """Heads of whole 16-byte vectors are padded to the kernel's width by the tensor maps on the way into shared memory;
+    other widths run zero-padded: zero columns change neither Q K^T nor the valid columns of P V."""
+    return d if d % 8 == 0 and 0 < d <= 128 else _kernel_dim(d)
 
 
 def _pad_heads(t: torch.Tensor, parts: int, H: int, d: int, dp: int) -> torch.Tensor:
@@ -37,7 +43,7 @@ def attn_fwd(qkv: torch.Tensor, n_win: int, N: int, H: int, d: int, *, out: torc
     """
     T, C = qkv.shape
     assert T == n_win * N and C == 3 * H * d and qkv.dtype == torch.bfloat16 and qkv.stride(1) == 1
-    dp = _kernel_dim(d)
+    dp = _padded_dim(d)
     if dp != d:
         o_p, lse = attn_fwd(_pad_heads(qkv, 3, H, d, dp), n_win, N, H, dp, lse=lse,
                             scale=scale if scale is not None else 1.0 / math.sqrt(d))
@@ -83,7 +89,7 @@ def attn_bwd(qkv: torch.Tensor, o: torch.Tensor, d_o: torch.Tensor, lse: torch.T
     """Gradient of :func:`attn_fwd` with respect to the fused qkv tensor (same layout as ``qkv``)."""
     T, C = qkv.shape
     assert o.shape == (T, H * d) and d_o.shape == (T, H * d) and d_o.stride(1) == 1 and o.stride(0) == d_o.stride(0)
-    dp = _kernel_dim(d)
+    dp = _padded_dim(d)
     if dp != d:
         g_p = attn_bwd(_pad_heads(qkv, 3, H, d, dp), _pad_heads(o, 1, H, d, dp), _pad_heads(d_o, 1, H, d, dp), lse,
                        n_win, N, H, dp, delta=delta, scale=scale if scale is not None else 1.0 / math.sqrt(d))
