@@ -113,7 +113,8 @@ int aeris_gemv_bwd(const void* W, int flags, const void* x, const float* dy, flo
 int aeris_noise_embedding(const float* t, void* out, int out_bf16, int B, int dim, double max_period, void* stream);
 int aeris_pack_embed_weights(const float* W, const float* b, void* out, int D, int Cin, int KP, void* stream);
 int aeris_fold_embed_grad(const float* G, float* dW, float* db, int D, int Cin, int KP, void* stream);
-int aeris_pack_head_weights(const float* W, void* hi, void* lo, int C, int rows, int D, void* stream);
+int aeris_pack_head_weights(const float* W, void* out, int C, int rows, int D, void* stream);
+int aeris_gemm_split(const void* y, const void* w, float* C, int M, int D, int lo_row, int ldc, int* status, void* stream);
 
 #ifdef __cplusplus
 }

@@ -5,7 +5,7 @@
 //   * gemv_bias_act / gemv_bwd: the M <= 8 modulation MLP layers (parallel_swin.py:321-325) and their gradients
 //   * pack_embed_weights / fold_embed_grad: [hi(W) | hi(W) | lo(W) | hi(b) | lo(b)] operand of the input projection and
 //     the packed product's gradient back on W and b
-//   * pack_head_weights: hi and lo parts of the output head's weight, padded to a whole number of rows
+//   * pack_head_weights: [hi | lo | hi] parts of the output head's weight, padded to a whole number of rows
 #include "common.cuh"
 #include "api.h"
 
@@ -226,15 +226,17 @@ __global__ void fold_embed_grad_kernel(const float* __restrict__ G, float* __res
     else db[d] += g[3 * Cin];
   }
 }
-// hi and lo [rows, D] (bf16) of the fp32 head weight [C, D]; rows past C are zero.
-__global__ void pack_head_weights_kernel(const float* __restrict__ W, __nv_bfloat16* __restrict__ hi,
-                                         __nv_bfloat16* __restrict__ lo, int C, int rows, int D) {
+// Rows [hi(W) | lo(W) | hi(W)] (bf16, [rows, 3 D]) of the fp32 head weight [C, D]; rows past C are zero.
+__global__ void pack_head_weights_kernel(const float* __restrict__ W, __nv_bfloat16* __restrict__ out, int C, int rows, int D) {
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < static_cast<long long>(rows) * D;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const float v = i < static_cast<long long>(C) * D ? W[i] : 0.f;
+    const int r = static_cast<int>(i / D), c = static_cast<int>(i - static_cast<long long>(r) * D);
+    const float v = r < C ? W[i] : 0.f;
     const __nv_bfloat16 h = __float2bfloat16_rn(v);
-    hi[i] = h;
-    lo[i] = __float2bfloat16_rn(v - __bfloat162float(h));
+    __nv_bfloat16* o = out + static_cast<size_t>(r) * 3 * D + c;
+    o[0] = h;
+    o[D] = __float2bfloat16_rn(v - __bfloat162float(h));
+    o[2 * D] = h;
   }
 }
 
@@ -324,9 +326,9 @@ extern "C" int aeris_fold_embed_grad(const float* G, float* dW, float* db, int D
   return launched();
 }
 
-extern "C" int aeris_pack_head_weights(const float* W, void* hi, void* lo, int C, int rows, int D, void* stream) {
+extern "C" int aeris_pack_head_weights(const float* W, void* out, int C, int rows, int D, void* stream) {
   if (C <= 0 || rows < C || D <= 0) return -1;
   pack_head_weights_kernel<<<small_grid(static_cast<long long>(rows) * D), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      W, reinterpret_cast<__nv_bfloat16*>(hi), reinterpret_cast<__nv_bfloat16*>(lo), C, rows, D);
+      W, reinterpret_cast<__nv_bfloat16*>(out), C, rows, D);
   return launched();
 }

@@ -298,12 +298,13 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
 // tokens): the number of slices that minimises rounds x (k-blocks per slice + fixed cost of a slice), a round being one
 // slice per CTA pair. Constant four left the last round of many shapes nearly empty and small weights (dim 256: 4 slices
 // on 74 pairs) on a handful of SMs. The fixed cost, filling the ring and adding 256 x 256 fp32 values to memory, is
-// taken as 10 k-blocks of 64; slices of fewer than 8 are not made. Four slices
+// taken as 10 k-blocks of 64; slices of fewer than 8 are not made, and never fewer than four slices: the tensor core
+// truncates at every addition, so longer slices would be less accurate. Four slices
 // and now: 512 x 512 x 28800: 43.6 -> 22.6 us, 768 x 2048 x 28800: 83.6 -> 69.6 us, 1536 x 4096 x 64800: 716 -> 621 us.
 static int auto_k_splits(int mn_tiles, int kb_total, int pairs) {
-  int best = 1;
+  int best = 4;
   long long best_cost = 0x7fffffffffffll;
-  for (int s = 1; s <= 64 && (s == 1 || kb_total / s >= 8); ++s) {
+  for (int s = 4; s <= 64 && (s == 4 || kb_total / s >= 8); ++s) {
     const long long rounds = (static_cast<long long>(mn_tiles) * s + pairs - 1) / pairs;
     const long long cost = rounds * ((kb_total + s - 1) / s + 10);
     if (cost < best_cost) { best_cost = cost; best = s; }

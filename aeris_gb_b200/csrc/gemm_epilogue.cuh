@@ -47,6 +47,9 @@ struct GemmParams {
   int tm_rot;       // first m-tile (of 256 rows) visited by the two-CTA kernel; the others follow cyclically. The
                     // reduce-scatter GEMM starts at the rows of rank + 1 and ends with its own, so that at any moment
                     // every rank pushes to a different owner and no GPU's ingress carries all the traffic
+  // One-CTA kernel: the A operand is [lo | hi | hi] of a value split into two bf16 parts that are stored as two blocks of
+  // rows (lo at row `split_rows`) of `split_k` columns: K = 3 split_k (0: plain operand).
+  int split_k, split_rows;
   int group_m;      // two-CTA kernel: m-tiles per group of the tile order (<= 1: n fastest)
   int staged_out;   // bf16-output epilogues: move rows through the warp's shared-memory stage (coalesced global stores)
   int staged_red;   // split-K fp32 accumulation: stage 32 rows x 64 columns and issue the reductions row-contiguously

@@ -100,7 +100,7 @@ class EmbedFn(torch.autograd.Function):
             n = min(CHUNK_ROWS, T - r0)
             DF.embed_pack(x_img, c_img, cs, plan.geom, plan.ape_y, plan.ape_x, plan.seed, plan.sigma_data,
                           plan.noise, A[:n], row0=r0)
-            G.gemm(dout[r0:r0 + n], A[:n], a_t=True, b_t=True, out=Gw, epi=G.EPI_ACC_F32, k_splits=0)
+            G.gemm(dout[r0:r0 + n], A[:n], a_t=True, b_t=True, out=Gw, epi=G.EPI_ACC_F32, k_splits=8)
         sW, rW = _grad_slot(W)
         sb, rb = _grad_slot(b)
         DF.fold_embed_grad(Gw, sW, sb)
@@ -112,14 +112,13 @@ def _head_weights(head_w: torch.Tensor):
     return DF.pack_head_weights(head_w.detach().float().contiguous(), PAD_N)
 
 
-def _head_rows(x, scale, shift, norm_w, w_hi, w_lo, eps, pred, y_hi, y_lo):
-    """pred[n, 128] (fp32) = (RMSNorm(x) * w * (1 + scale) + shift) @ head^T for ``n`` rows of ``scale.shape[0]`` samples."""
+def _head_rows(x, scale, shift, norm_w, w3, eps, pred, y):
+    """pred[n, 128] (fp32) = (RMSNorm(x) * w * (1 + scale) + shift) @ head^T for ``n`` rows of ``scale.shape[0]`` samples;
+    ``y`` [2, rows, D]: workspace for the bf16 value and remainder of the normalised rows."""
     n = x.shape[0]
-    E.modnorm_fwd(x, scale, shift, norm_w, mode=E.MODE_NORM_THEN_MOD, eps=eps, out=y_hi[:n], out_lo=y_lo[:n],
+    E.modnorm_fwd(x, scale, shift, norm_w, mode=E.MODE_NORM_THEN_MOD, eps=eps, out=y[0, :n], out_lo=y[1, :n],
                   batch=scale.shape[0])
-    G.gemm(y_hi[:n], w_hi, out=pred[:n], epi=G.EPI_STORE_F32)
-    G.gemm(y_lo[:n], w_hi, out=pred[:n], epi=G.EPI_ACC_F32)
-    G.gemm(y_hi[:n], w_lo, out=pred[:n], epi=G.EPI_ACC_F32)
+    DF.head_gemm(y, n, w3, pred)
     return pred[:n]
 
 
@@ -138,16 +137,15 @@ def head_forward(x: torch.Tensor, shift: torch.Tensor, scale: torch.Tensor, norm
     T, D = x.shape
     B = shift.shape[0]
     dev = x.device
-    w_hi, w_lo = _head_weights(head_w)
+    w3 = _head_weights(head_w)
     ws = workspace()
     spans = _sample_chunks(B, T // B)
     cm = max(n for *_, n in spans)
-    y_hi = ws.get("head_yhi", (cm, D), torch.bfloat16, dev)
-    y_lo = ws.get("head_ylo", (cm, D), torch.bfloat16, dev)
+    y = ws.get("head_y", (2, cm, D), torch.bfloat16, dev)
     pred = torch.empty((T, PAD_N), dtype=torch.float32, device=dev)
     shift, scale = shift.float().contiguous(), scale.float().contiguous()
     for b, nb, r0, n in spans:
-        _head_rows(x[r0:r0 + n], scale[b:b + nb], shift[b:b + nb], norm_w, w_hi, w_lo, eps, pred[r0:r0 + n], y_hi, y_lo)
+        _head_rows(x[r0:r0 + n], scale[b:b + nb], shift[b:b + nb], norm_w, w3, eps, pred[r0:r0 + n], y)
     return pred
 
 
@@ -161,19 +159,18 @@ class HeadLossFn(torch.autograd.Function):
         T, D = x.shape
         B = shift.shape[0]
         dev = x.device
-        w_hi, w_lo = _head_weights(head_w)
+        w3 = _head_weights(head_w)
         ws = workspace()
         spans = _sample_chunks(B, T // B)
         cm = max(n for *_, n in spans)
-        y_hi = ws.get("head_yhi", (cm, D), torch.bfloat16, dev)
-        y_lo = ws.get("head_ylo", (cm, D), torch.bfloat16, dev)
+        y = ws.get("head_y", (2, cm, D), torch.bfloat16, dev)
         pred = ws.get("head_pred", (cm, PAD_N), torch.float32, dev)
         dpred = torch.empty((T, PAD_N), dtype=torch.bfloat16, device=dev)
         loss = torch.zeros(1, dtype=torch.float64, device=dev)
         shift32, scale32 = shift.float().contiguous(), scale.float().contiguous()
         inv_rows = 1.0 / (T // B)
         for b, nb, r0, n in spans:
-            _head_rows(x[r0:r0 + n], scale32[b:b + nb], shift32[b:b + nb], norm_w, w_hi, w_lo, plan.eps, pred, y_hi, y_lo)
+            _head_rows(x[r0:r0 + n], scale32[b:b + nb], shift32[b:b + nb], norm_w, w3, plan.eps, pred, y)
             DF.trigflow_loss(pred[:n], x_img, cs, plan.geom, plan.seed, plan.sigma_data, plan.w_var, plan.w_lat,
                              inv_rows, loss, dpred=dpred[r0:r0 + n], row0=r0)
         ctx.plan = plan
@@ -188,12 +185,11 @@ class HeadLossFn(torch.autograd.Function):
         B = shift.shape[0]
         C = head_w.shape[0]
         dev = x.device
-        w_hi, _ = _head_weights(head_w)
+        w_hi = _head_weights(head_w)[:, :D]
         ws = workspace()
         spans = _sample_chunks(B, T // B)
         cm = max(n for *_, n in spans)
-        y_hi = ws.get("head_yhi", (cm, D), torch.bfloat16, dev)
-        dy = ws.get("head_ylo", (cm, D), torch.bfloat16, dev)
+        y_hi, dy = ws.get("head_y", (2, cm, D), torch.bfloat16, dev).unbind(0)
         Gh = ws.get("head_g", (PAD_N, D), torch.float32, dev, zero=True)
         shift32, scale32 = shift.float().contiguous(), scale.float().contiguous()
         dshift, dscale = torch.zeros((2, *shift32.shape), dtype=torch.float32, device=dev).unbind(0)

@@ -153,10 +153,20 @@ def fold_embed_grad(G: torch.Tensor, dW: torch.Tensor, db: torch.Tensor) -> None
     _l.check(rc, "aeris_fold_embed_grad")
 
 
-def pack_head_weights(W: torch.Tensor, rows: int) -> tuple[torch.Tensor, torch.Tensor]:
-    """bf16 value and bf16 remainder of an fp32 weight [C, D], padded with zero rows to ``rows``."""
+def pack_head_weights(W: torch.Tensor, rows: int) -> torch.Tensor:
+    """``[hi | lo | hi]`` (bf16 [rows, 3 D]) of an fp32 weight [C, D], padded with zero rows."""
     C, D = W.shape
-    hi, lo = torch.empty((2, rows, D), dtype=torch.bfloat16, device=W.device).unbind(0)
-    rc = _l.lib().aeris_pack_head_weights(_l.ptr(W), _l.ptr(hi), _l.ptr(lo), C, rows, D, _l.stream_ptr())
+    out = torch.empty((rows, 3 * D), dtype=torch.bfloat16, device=W.device)
+    rc = _l.lib().aeris_pack_head_weights(_l.ptr(W), _l.ptr(out), C, rows, D, _l.stream_ptr())
     _l.check(rc, "aeris_pack_head_weights")
-    return hi, lo
+    return out
+
+
+def head_gemm(y: torch.Tensor, n: int, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+    """``out[:n]`` (fp32 [*, 128]) = the product of the values whose bf16 parts are ``y[0, :n]`` and ``y[1, :n]`` (``y``
+    [2, rows, D]) with the weight packed by :func:`pack_head_weights`, up to the dropped lo x lo term."""
+    assert y.is_contiguous() and y.dim() == 3 and w.shape == (128, 3 * y.shape[2])
+    rc = _l.lib().aeris_gemm_split(_l.ptr(y), _l.ptr(w), _l.ptr(out), n, y.shape[2], y.shape[1], out.stride(0),
+                                   _l.ptr(_l.status_word()), _l.stream_ptr())
+    _l.check(rc, "aeris_gemm_split")
+    return out

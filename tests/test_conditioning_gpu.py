@@ -68,5 +68,20 @@ def test_packed_weights_of_the_ends():
     G, dW, db = torch.randn(130, 128, device=DEV), torch.ones(130, 20, device=DEV), torch.ones(130, device=DEV)
     DF.fold_embed_grad(G, dW, db)
     assert torch.equal(dW, 1 + (G[:, :20] + G[:, 20:40])) and torch.equal(db, 1 + G[:, 60])
-    h, l = DF.pack_head_weights(W, 256)
-    assert torch.equal(h[:130], hi) and torch.equal(l[:130], lo) and not h[130:].any() and not l[130:].any()
+    w3 = DF.pack_head_weights(W, 256)
+    assert torch.equal(w3[:130], torch.cat([hi, lo, hi], 1)) and not w3[130:].any()
+
+
+@pytest.mark.parametrize("n,rows,D", [(1, 1, 64), (130, 200, 128), (1000, 1000, 384), (257, 300, 1536)])
+def test_head_product_of_split_operands(n, rows, D):
+    """hi and lo rows in two blocks (rows that are no multiple of a tile, a block longer than the rows in use), against
+    fp64: what is dropped is lo x lo, 2^-17 of a term at most, and the tensor core's fp32 sums."""
+    from aeris_gb_b200.ops import diffusion as DF
+    v, W = torch.randn(n, D, device=DEV), torch.randn(70, D, device=DEV)
+    y = torch.full((2, rows, D), float("nan"), dtype=torch.bfloat16, device=DEV)
+    y[0, :n] = v.bfloat16()
+    y[1, :n] = (v - y[0, :n].float()).bfloat16()
+    out = torch.full((n + 1, 128), 7.0, device=DEV)
+    DF.head_gemm(y, n, DF.pack_head_weights(W, 128), out)
+    assert rel_err(out[:n, :70], v.double() @ W.double().t()) < 2.0 ** -16 and not out[:n, 70:].any()
+    assert (out[n:] == 7).all()
