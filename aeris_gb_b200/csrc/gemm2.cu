@@ -24,13 +24,20 @@ namespace aeris {
 constexpr int G2_BM = 128;       // rows per CTA (256 per pair)
 constexpr int G2_BN = 256;
 constexpr int G2_BK = 64;
-constexpr int G2_THREADS = 192;
 constexpr int G2_STAGES = 6;
 constexpr int G2_A_BYTES = G2_BM * G2_BK * 2;         // 16 KB
 constexpr int G2_B_BYTES = (G2_BN / 2) * G2_BK * 2;   // 16 KB: this CTA's half of B
 constexpr int G2_STAGE_BYTES = G2_A_BYTES + G2_B_BYTES;
-constexpr int G2_PUSH_OFF = G2_STAGES * G2_STAGE_BYTES + 512;     // staging of the peer-push epilogues, 8 KB per warp
-constexpr int G2_SMEM = G2_PUSH_OFF + 4 * PUSH_STAGE_BYTES + 1024;
+// Epilogue warps and ring depth. With a short reduction the epilogue of a tile takes longer than its products, so the
+// heavier local epilogues then run on eight warps, two per 32 rows with half of the columns each, for the price of one ring
+// stage (their staging buffers; see aeris_gemm_bf16_2cta for the line). Everything else keeps four warps and six stages.
+template <int EW> struct G2Layout {
+  static constexpr int STAGES = EW == 8 ? G2_STAGES - 1 : G2_STAGES;
+  static constexpr int PUSH_OFF = STAGES * G2_STAGE_BYTES + 512;     // staging of the epilogues, 8 KB per warp
+  static constexpr int SMEM = PUSH_OFF + EW * PUSH_STAGE_BYTES + 1024;
+  static constexpr int THREADS = 64 + EW * 32;
+};
+static_assert(G2Layout<4>::SMEM <= 227 * 1024 && G2Layout<8>::SMEM <= 227 * 1024, "shared memory");
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -94,23 +101,25 @@ __device__ __forceinline__ void umma2_ss(uint32_t tmem_d, uint64_t adesc, uint64
 // starting with this rank's own row chunk while two extra warps (6, 7) of every CTA push that chunk into the peers'
 // buffers; the producer of each CTA waits for the chunks its 128 rows come from. The grid is then always the full
 // number of CTA pairs, so that every call adds the same amount to the arrival counters.
-template <int A_MN, int B_MN, bool AG = false>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(AG ? G2_THREADS + AG_COPY_THREADS : G2_THREADS, 1)
+template <int A_MN, int B_MN, int EW, bool AG = false>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G2Layout<EW>::THREADS + (AG ? AG_COPY_THREADS : 0), 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
              const GemmParams p) {
+  static_assert(!AG || EW == 4, "the copier warps follow four epilogue warps");
+  using LY = G2Layout<EW>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + G2_STAGES * G2_STAGE_BYTES);
-  uint64_t* empty_bar = full_bar + G2_STAGES;
-  uint64_t* tfull_bar = empty_bar + G2_STAGES;       // [2]
-  uint64_t* tempty_bar = tfull_bar + 2;              // [2], leader only: 8 arrivals (4 epilogue warps x 2 CTAs)
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + LY::STAGES * G2_STAGE_BYTES);
+  uint64_t* empty_bar = full_bar + LY::STAGES;
+  uint64_t* tfull_bar = empty_bar + LY::STAGES;       // [2]
+  uint64_t* tempty_bar = tfull_bar + 2;              // [2], leader only: one arrival per epilogue warp of both CTAs
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
 
   // AG: the last operand stage is the copier's ring (two 16 KB bulk-copy buffers), with its barriers behind tmem_slot
   // (the reduce-scatter epilogue gives up the same stage: its fourth warp stages its rows there)
-  const int STAGES = (AG || p.epi == EPI_RS_PUSH) ? G2_STAGES - 1 : G2_STAGES;
-  [[maybe_unused]] uint8_t* ag_ring = smem + (G2_STAGES - 1) * G2_STAGE_BYTES;
-  [[maybe_unused]] uint64_t* ag_bars = reinterpret_cast<uint64_t*>(smem + G2_STAGES * G2_STAGE_BYTES + 256);
+  const int STAGES = (EW == 4 && (AG || p.epi == EPI_RS_PUSH)) ? LY::STAGES - 1 : LY::STAGES;
+  [[maybe_unused]] uint8_t* ag_ring = smem + (LY::STAGES - 1) * G2_STAGE_BYTES;
+  [[maybe_unused]] uint64_t* ag_bars = reinterpret_cast<uint64_t*>(smem + LY::STAGES * G2_STAGE_BYTES + 256);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -145,13 +154,13 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   if (threadIdx.x == 0) {
     prefetch_tmap(&tmap_a);
     prefetch_tmap(&tmap_b);
-    for (int s = 0; s < G2_STAGES; ++s) {
+    for (int s = 0; s < LY::STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull_bar[a], 1);
-      mbar_init(&tempty_bar[a], 8);
+      mbar_init(&tempty_bar[a], 2 * EW);
       if constexpr (AG) mbar_init(&ag_bars[a], 1);
     }
     fence_barrier_init();
@@ -257,8 +266,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       if (elect_one_sync()) ag_push_chunk(p, ag_ring, ag_bars);
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..5 of both CTAs)
-    const int q = warp & 3;
+    // ------------------------------------------------------------ epilogue (warps 2 .. 1 + EW of both CTAs)
+    const int q = warp & 3, part = (warp - 2) >> 2;
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
@@ -273,10 +282,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       const int row = tm * 2 * G2_BM + crank * G2_BM + q * 32 + lane;
       const uint32_t taddr = tmem_base + acc * G2_BN + (static_cast<uint32_t>(q * 32) << 16);
       const bool kempty = (split * kb_per_split) >= kb_total;
-      uint8_t* stg = smem + G2_PUSH_OFF + q * PUSH_STAGE_BYTES;
+      uint8_t* stg = smem + LY::PUSH_OFF + (part * 4 + q) * PUSH_STAGE_BYTES;
       if (p.epi == EPI_RS_PUSH)     // 8704-byte linear stages: three in the push area, the fourth in the freed operand stage
-        stg = (q < 3) ? smem + G2_PUSH_OFF + q * RS_STAGE_BYTES : smem + (G2_STAGES - 1) * G2_STAGE_BYTES;
-      gemm_epilogue_row<G2_BN>(p, taddr, row, row < p.M, tn, kempty, stg);
+        stg = (q < 3) ? smem + LY::PUSH_OFF + q * RS_STAGE_BYTES : smem + (LY::STAGES - 1) * G2_STAGE_BYTES;
+      gemm_epilogue_row<G2_BN>(p, taddr, row, row < p.M, tn, kempty, stg, part, EW / 4);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(leader_tempty0 + acc * 8);
@@ -312,14 +321,14 @@ static int auto_k_splits(int mn_tiles, int kb_total, int pairs) {
   return best;
 }
 
-template <int A_MN, int B_MN, bool AG = false>
+template <int A_MN, int B_MN, int EW, bool AG = false>
 static int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p_in, cudaStream_t stream) {
   static bool configured = false;
   GemmParams p = p_in;
-  constexpr int THREADS = AG ? G2_THREADS + AG_COPY_THREADS : G2_THREADS;
-  auto kern = gemm2_kernel<A_MN, B_MN, AG>;
+  constexpr int THREADS = G2Layout<EW>::THREADS + (AG ? AG_COPY_THREADS : 0), SMEM = G2Layout<EW>::SMEM;
+  auto kern = gemm2_kernel<A_MN, B_MN, EW, AG>;
   if (!configured) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM) != cudaSuccess) return -20;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) return -20;
     configured = true;
   }
   const int m_tiles = (p.M + 2 * G2_BM - 1) / (2 * G2_BM);
@@ -330,7 +339,7 @@ static int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(num_sms(), 1, 1);
     cfg.blockDim = dim3(THREADS, 1, 1);
-    cfg.dynamicSmemBytes = G2_SMEM;
+    cfg.dynamicSmemBytes = SMEM;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
@@ -345,7 +354,7 @@ static int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
   const int tiles = mn_tiles * p.k_splits;
   if (tiles < clusters && !AG) clusters = tiles;
   if (AG) p.ag_expect *= static_cast<unsigned>(2 * clusters);   // came in as the call index
-  kern<<<2 * clusters, THREADS, G2_SMEM, stream>>>(ta, tb, p);
+  kern<<<2 * clusters, THREADS, SMEM, stream>>>(ta, tb, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
@@ -394,10 +403,16 @@ extern "C" int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M
     r = make_tmap_2d_bf16(&tb, B, N, K, ldb, 64, G2_BK);
   }
   if (r) return r - 100;
-  if (!a_mn && !b_mn) return launch_gemm2<0, 0>(ta, tb, p, stream);
-  if (!a_mn && b_mn) return launch_gemm2<0, 1>(ta, tb, p, stream);
-  if (a_mn && !b_mn) return launch_gemm2<1, 0>(ta, tb, p, stream);
-  return launch_gemm2<1, 1>(ta, tb, p, stream);
+  // Eight epilogue warps where the epilogue takes longer than the products of a tile. Four warps and six stages against
+  // eight and five, us: gated residual 28800 x 768 x 768 63 / 52, 64800 x 1536 x 1536 269 / 241; SwiGLU backward
+  // 64800 x 4096 x 1536 1306 / 1068, x 768 224 / 182; SwiGLU with the raw columns 28800 x 4096 x 768 190 / 167; plain
+  // store 28800 x 2304 x 768 89 / 84, but 64800 x 4608 x 1536 597 / 624 and its data gradient 220 / 258. Weight gradients
+  // (a_mn) lose a few per cent. Requesting the SwiGLU operands a step ahead spills at eight warps (1068 -> 1240).
+  const bool heavy = epi == EPI_SWIGLU_BOTH || epi == EPI_SWIGLU_BWD || epi == EPI_GATE_RESID;
+  const bool ew8 = (heavy && K <= 2048) || (epi == EPI_STORE && K <= 1024);
+  if (a_mn) return b_mn ? launch_gemm2<1, 1, 4>(ta, tb, p, stream) : launch_gemm2<1, 0, 4>(ta, tb, p, stream);
+  if (b_mn) return ew8 ? launch_gemm2<0, 1, 8>(ta, tb, p, stream) : launch_gemm2<0, 1, 4>(ta, tb, p, stream);
+  return ew8 ? launch_gemm2<0, 0, 8>(ta, tb, p, stream) : launch_gemm2<0, 0, 4>(ta, tb, p, stream);
 }
 
 // QKV (or dO) projection whose epilogue performs the Ulysses head<->sequence exchange: C is not written locally;
@@ -421,7 +436,7 @@ extern "C" int aeris_gemm_scatter_heads(const void* A, const void* B, int M, int
   if (r) return r;
   r = b_mn ? make_tmap_2d_bf16(&tb, B, N, K, ldb, 64, G2_BK) : make_tmap_2d_bf16(&tb, B, K, N, ldb, G2_BK, G2_BN / 2);
   if (r) return r - 100;
-  return b_mn ? launch_gemm2<0, 1>(ta, tb, p, stream) : launch_gemm2<0, 0>(ta, tb, p, stream);
+  return b_mn ? launch_gemm2<0, 1, 4>(ta, tb, p, stream) : launch_gemm2<0, 0, 4>(ta, tb, p, stream);
 }
 
 // GEMM -> reduce-scatter by rows in one kernel: rank `rank` computes its partial product for all `world *
@@ -446,7 +461,7 @@ extern "C" int aeris_gemm_rs_push(const void* A, const void* B, int M, int N, in
   if (r) return r;
   r = b_mn ? make_tmap_2d_bf16(&tb, B, N, K, ldb, 64, G2_BK) : make_tmap_2d_bf16(&tb, B, K, N, ldb, G2_BK, G2_BN / 2);
   if (r) return r - 100;
-  return b_mn ? launch_gemm2<0, 1>(ta, tb, p, stream) : launch_gemm2<0, 0>(ta, tb, p, stream);
+  return b_mn ? launch_gemm2<0, 1, 4>(ta, tb, p, stream) : launch_gemm2<0, 0, 4>(ta, tb, p, stream);
 }
 
 // All-gather -> GEMM in one kernel (two-CTA tiles). `A` is this rank's [world * rows_per_rank, K] buffer (row pitch K)
@@ -489,5 +504,5 @@ extern "C" int aeris_gemm_allgather_a(void* A, const void* const* peers, const v
     r = make_tmap_2d_bf16(&tb, B, N, K, ldb, 64, G2_BK);
   }
   if (r) return r - 100;
-  return b_mn ? launch_gemm2<0, 1, true>(ta, tb, p, stream) : launch_gemm2<0, 0, true>(ta, tb, p, stream);
+  return b_mn ? launch_gemm2<0, 1, 4, true>(ta, tb, p, stream) : launch_gemm2<0, 0, 4, true>(ta, tb, p, stream);
 }

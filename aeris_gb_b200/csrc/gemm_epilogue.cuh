@@ -160,9 +160,11 @@ __device__ __forceinline__ void push_stage_flush_red(uint8_t* stage, int lane, f
 // `stage`: this warp's PUSH_STAGE_BYTES of shared memory for the push epilogues, or null (direct stores).
 template <int BN>
 __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t taddr, int row, bool row_ok, int tn,
-                                                  bool kempty, uint8_t* stage = nullptr) {
+                                                  bool kempty, uint8_t* stage = nullptr, int part = 0, int parts = 1) {
   const int lane = threadIdx.x & 31;
-  const int ncols = min(BN, p.N - tn * BN);      // 128 in a half-empty last tile of the two-CTA kernel
+  // columns of this warp: all, or one of two halves where eight warps share a tile; p.N - tn * BN is 128 in a half-empty
+  // last tile of the two-CTA kernel
+  const int c_lo = part * (BN / parts), c_hi = min(c_lo + BN / parts, p.N - tn * BN);
 
   if (p.epi == EPI_SCATTER_HEADS) {
     const int w = row / p.scat_n_local;
@@ -233,7 +235,7 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
     const __nv_bfloat16* usrc = p.resid + static_cast<size_t>(row) * p.ldr + tn * BN;
     __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(row) * p.ldc + tn * BN;
 #pragma unroll 1
-    for (int c = 0; c < ncols; c += 32) {
+    for (int c = c_lo; c < c_hi; c += 32) {
       uint32_t v[32];
       tmem_ld32(taddr + c, v);
       tmem_wait_ld();
@@ -275,24 +277,27 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
     // and up columns follow as two more groups (second pass over the accumulator in TMEM)
     constexpr int H = BN / 2;
     __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(row) * p.ldc + tn * H;
+    // of two warps that share the rows the first writes the activation, the second the raw columns
+    if (part == 0) {
 #pragma unroll 1
-    for (int c = 0; c < H; c += 32) {
-      uint32_t g[32], u[32];
-      tmem_ld32(taddr + c, g);
-      tmem_ld32(taddr + H + c, u);
-      tmem_wait_ld();
-      uint32_t o[16];
+      for (int c = 0; c < H; c += 32) {
+        uint32_t g[32], u[32];
+        tmem_ld32(taddr + c, g);
+        tmem_ld32(taddr + H + c, u);
+        tmem_wait_ld();
+        uint32_t o[16];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const float g0 = __uint_as_float(g[2 * i]), g1 = __uint_as_float(g[2 * i + 1]);
-        const float u0 = __uint_as_float(u[2 * i]), u1 = __uint_as_float(u[2 * i + 1]);
-        const float s0 = g0 / (1.f + __expf(-g0)), s1 = g1 / (1.f + __expf(-g1));
-        o[i] = pack_bf16x2(s0 * u0, s1 * u1);
+        for (int i = 0; i < 16; ++i) {
+          const float g0 = __uint_as_float(g[2 * i]), g1 = __uint_as_float(g[2 * i + 1]);
+          const float u0 = __uint_as_float(u[2 * i]), u1 = __uint_as_float(u[2 * i + 1]);
+          const float s0 = g0 / (1.f + __expf(-g0)), s1 = g1 / (1.f + __expf(-g1));
+          o[i] = pack_bf16x2(s0 * u0, s1 * u1);
+        }
+        push_stage_put(stage, lane, c, o);
       }
-      push_stage_put(stage, lane, c, o);
+      push_stage_flush(stage, lane, row_ok ? out : nullptr);
     }
-    push_stage_flush(stage, lane, row_ok ? out : nullptr);
-    if (p.epi == EPI_SWIGLU_BOTH) {
+    if (p.epi == EPI_SWIGLU_BOTH && part == parts - 1) {
       __nv_bfloat16* raw = p.aux + static_cast<size_t>(row) * p.ld_aux + tn * H;
 #pragma unroll 1
       for (int half = 0; half < 2; ++half) {
@@ -313,7 +318,7 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
     __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(row) * p.ldc + tn * H;
     __nv_bfloat16* raw = (p.epi == EPI_SWIGLU_BOTH) ? p.aux + static_cast<size_t>(row) * p.ld_aux + tn * H : nullptr;
 #pragma unroll 1
-    for (int c = 0; c < H; c += 32) {
+    for (int c = part * (H / parts); c < (part + 1) * (H / parts); c += 32) {
       uint32_t g[32], u[32];
       tmem_ld32(taddr + c, g);
       tmem_ld32(taddr + H + c, u);
@@ -350,7 +355,7 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
     float* out = reinterpret_cast<float*>(p.C) + static_cast<size_t>(row) * p.ldc + tn * BN;
     const bool live = row_ok && !kempty;
 #pragma unroll 1
-    for (int c = 0; c < ncols; c += 32) {
+    for (int c = c_lo; c < c_hi; c += 32) {
       uint32_t v[32];
       tmem_ld32(taddr + c, v);
       tmem_wait_ld();
@@ -360,7 +365,7 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
   } else if (p.epi == EPI_ACC_F32 || p.epi == EPI_STORE_F32) {
     float* out = reinterpret_cast<float*>(p.C) + static_cast<size_t>(row) * p.ldc + tn * BN;
 #pragma unroll 1
-    for (int c = 0; c < ncols; c += 32) {
+    for (int c = c_lo; c < c_hi; c += 32) {
       uint32_t v[32];
       tmem_ld32(taddr + c, v);
       tmem_wait_ld();
@@ -403,18 +408,18 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
     const float* gate = nullptr;
     if (gated) gate = p.gate + static_cast<size_t>(row / p.rows_per_gate) * p.N + tn * BN;
     uint4 r4[4], r4n[4];       // residual of this and of the next 32 columns (requested one step ahead)
-    if (gated) {
+    if (gated && c_lo < c_hi) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) r4n[i] = reinterpret_cast<const uint4*>(res)[i];
+      for (int i = 0; i < 4; ++i) r4n[i] = reinterpret_cast<const uint4*>(res + c_lo)[i];
     }
 #pragma unroll 1
-    for (int c = 0; c < ncols; c += 32) {
+    for (int c = c_lo; c < c_hi; c += 32) {
       uint32_t v[32];
       tmem_ld32(taddr + c, v);
       if (gated) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) r4[i] = r4n[i];
-        if (c + 32 < ncols) {
+        if (c + 32 < c_hi) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) r4n[i] = reinterpret_cast<const uint4*>(res + c + 32)[i];
         }
@@ -452,7 +457,7 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
       gate = p.gate + static_cast<size_t>(row / p.rows_per_gate) * p.N + tn * BN;
     __nv_bfloat16* aux = p.aux ? p.aux + static_cast<size_t>(row) * p.ld_aux + tn * BN : nullptr;
 #pragma unroll 1
-    for (int c = 0; c < ncols; c += 32) {
+    for (int c = c_lo; c < c_hi; c += 32) {
       uint32_t v[32];
       tmem_ld32(taddr + c, v);
       tmem_wait_ld();

@@ -188,6 +188,35 @@ def test_gemm_half_empty_last_tile(M, N, K):
         assert torch.equal(out, buf2) and (buf[:, 2 * N:] == 7).all()
 
 
+@pytest.mark.parametrize("K", [64, 1024, 1088, 2048, 2112])
+def test_gemm_epilogue_warps(K):
+    """The epilogues on eight warps (short reductions) and on four, around the lines of the dispatch, with rows that end
+    inside a warp's 32 and inside the second CTA's half; both halves of the columns, in place where the caller may."""
+    from aeris_gb_b200.ops import gemm as G
+    M, N = 456, 512
+    a, b = torch.randn(M, K, device=DEV).bfloat16(), (torch.randn(N, K, device=DEV) / K ** 0.5).bfloat16()
+    ref = a.float() @ b.float().t()
+    assert rel_err(G.gemm(a, b), ref) < TOL
+    resid, gate = torch.randn(M, N, device=DEV).bfloat16(), torch.randn(3, N, device=DEV)
+    out = G.gemm(a, b, epi=G.EPI_GATE_RESID, resid=resid, gate=gate, rows_per_gate=M // 3)
+    assert rel_err(out, resid.float() + gate.repeat_interleave(M // 3, 0) * ref) < TOL
+    raw = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    act = G.gemm(a, b, epi=G.EPI_SWIGLU_BOTH, aux=raw)
+    g, up = ref[:, :N // 2], ref[:, N // 2:]
+    assert rel_err(raw, ref) < TOL and rel_err(act, torch.nn.functional.silu(g) * up) < TOL
+    u = torch.randn(M, 2 * N, device=DEV).bfloat16()
+    g, up = u[:, :N].float(), u[:, N:].float()
+    s = torch.sigmoid(g)
+    want = torch.cat([ref * up * s * (1 + g * (1 - s)), ref * g * s], dim=1)
+    for b_t in (False, True):
+        bb = b.t().contiguous() if b_t else b
+        apart = torch.empty_like(u)
+        G.gemm(a, bb, b_t=b_t, out=apart, epi=G.EPI_SWIGLU_BWD, resid=u)
+        in_place = u.clone()
+        G.gemm(a, bb, b_t=b_t, out=in_place, epi=G.EPI_SWIGLU_BWD, resid=in_place)
+        assert rel_err(apart, want) < TOL and torch.equal(apart, in_place)
+
+
 @pytest.mark.parametrize("M,N,K", [(256, 256, 3600), (384, 640, 12150), (512, 1536, 200), (1536, 768, 28800), (256, 256, 40)])
 @pytest.mark.parametrize("k_splits", [0, 1, 3])
 def test_gemm_accumulate_splits(M, N, K, k_splits):
