@@ -130,9 +130,10 @@ constexpr int GEMV_BWD_ROWS = 64;
 template <typename WT, int MB>
 __global__ void __launch_bounds__(256)
 gemv_bwd_kernel(const WT* __restrict__ W, const void* __restrict__ x, int x_bf16, const float* __restrict__ dy,
-                float* __restrict__ dW, float* __restrict__ db, float* __restrict__ dx, int N, int K, int B, int silu_in) {
+                float* __restrict__ dW, float* __restrict__ db, float* __restrict__ dx, int N, int K, int B, int silu_in,
+                int rows) {
   __shared__ float s_dy[GEMV_BWD_ROWS][MB];
-  const int n0 = blockIdx.y * GEMV_BWD_ROWS, nr = min(GEMV_BWD_ROWS, N - n0);
+  const int n0 = blockIdx.y * rows, nr = min(rows, N - n0);
   for (int i = threadIdx.x; i < nr * MB; i += blockDim.x) {
     const int r = i / MB, b = i - r * MB;
     s_dy[r][b] = b < B ? dy[static_cast<size_t>(b) * N + n0 + r] : 0.f;
@@ -163,7 +164,7 @@ gemv_bwd_kernel(const WT* __restrict__ W, const void* __restrict__ x, int x_bf16
         dh[b][i] = s * (1.f + v * (1.f - s));
       }
     }
-#pragma unroll 4
+#pragma unroll 8
   for (int r = 0; r < nr; ++r) {
     const size_t off = static_cast<size_t>(n0 + r) * K + k;
     float4 d = *reinterpret_cast<const float4*>(dW + off);
@@ -295,17 +296,21 @@ extern "C" int aeris_gemv_bias_act(const void* W, int flags, const void* bias, c
 // flags as above. K must be a multiple of 4; W, dW and dx aligned to four elements. dW, db and dx are added to.
 extern "C" int aeris_gemv_bwd(const void* W, int flags, const void* x, const float* dy, float* dW, float* db, float* dx,
                               int N, int K, int B, int silu_in, void* stream) {
-  if (N <= 0 || K <= 0 || K % 4 || B <= 0 || B > 8 || N > 65535 * GEMV_BWD_ROWS) return -1;
+  if (N <= 0 || K <= 0 || K % 4 || B <= 0 || B > 8 || N > 65535 * 16) return -1;
   if ((reinterpret_cast<uintptr_t>(W) & ((flags & 1) ? 15 : 7)) ||
       ((reinterpret_cast<uintptr_t>(dW) | reinterpret_cast<uintptr_t>(dx)) & 15))
     return -3;
   int nt = (K / 4 + 31) / 32 * 32;
   if (nt > 256) nt = 256;
-  const dim3 grid((K / 4 + nt - 1) / nt, (N + GEMV_BWD_ROWS - 1) / GEMV_BWD_ROWS);
+  // 64 rows per CTA where that still gives every SM four CTAs (fewer reductions into dx), else 16: the walk down the rows is
+  // a chain of loads, and a narrow layer spent 35 us in it (1536 x 256; 11 us with 16 rows)
+  const int kx = (K / 4 + nt - 1) / nt;
+  const int rows = static_cast<long long>(kx) * (N / GEMV_BWD_ROWS) >= 4ll * aeris_num_sms() ? GEMV_BWD_ROWS : 16;
+  const dim3 grid(kx, (N + rows - 1) / rows);
   const int mb = B <= 1 ? 1 : B <= 2 ? 2 : B <= 4 ? 4 : 8;
   const cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 #define AERIS_GEMV(WT, MB) \
-  gemv_bwd_kernel<WT, MB><<<grid, nt, 0, st>>>(reinterpret_cast<const WT*>(W), x, (flags >> 2) & 1, dy, dW, db, dx, N, K, B, silu_in)
+  gemv_bwd_kernel<WT, MB><<<grid, nt, 0, st>>>(reinterpret_cast<const WT*>(W), x, (flags >> 2) & 1, dy, dW, db, dx, N, K, B, silu_in, rows)
 #define AERIS_GEMV_MB(WT) \
   do { if (mb == 1) AERIS_GEMV(WT, 1); else if (mb == 2) AERIS_GEMV(WT, 2); else if (mb == 4) AERIS_GEMV(WT, 4); else AERIS_GEMV(WT, 8); } while (0)
   if (flags & 1) AERIS_GEMV_MB(float); else AERIS_GEMV_MB(__nv_bfloat16);

@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-@pytest.mark.parametrize("N,K", [(1, 4), (70, 100), (257, 256), (1536, 1536), (130, 2052), (64, 1001)])
+@pytest.mark.parametrize("N,K", [(1, 4), (70, 100), (257, 256), (1536, 1536), (130, 2052), (64, 1001), (20000, 1536)])
 @pytest.mark.parametrize("B", [1, 2, 3, 8])
 @pytest.mark.parametrize("silu_in", [False, True])
 def test_gemv_forward_and_gradients(N, K, B, silu_in):
