@@ -1333,6 +1333,12 @@ extern "C" int aeris_attn_set_fwd_smem_pad(int bytes) {
   return 0;
 }
 
+// The kernels read and write o, d_o and dqkv in 16-byte vectors: bases on 16-byte boundaries, pitches and column offsets
+// (`elems`: their bitwise or) in whole vectors of eight elements. q, k and v are checked where their tensor maps are made.
+static bool whole_vectors(const void* base, int elems) {
+  return (reinterpret_cast<uintptr_t>(base) & 15) == 0 && (elems & 7) == 0;
+}
+
 // q, k, v: base pointers of row-major [n_win * N, ld*] bf16 tensors; *_col0 = column of head 0.
 static int attn_fwd_impl(const void* q, int ldq, int q_col0, const void* k, int ldk, int k_col0, const void* v,
                          int ldv, int v_col0, void* o, int ldo, float* lse, int n_win, int N, int H, int head_dim,
@@ -1364,6 +1370,9 @@ static int attn_fwd_impl(const void* q, int ldq, int q_col0, const void* k, int 
   if (head_dim <= 0 || head_dim > 128 || head_dim % 8) return -1;
   if (n_win <= 0 || N <= 0 || H <= 0 || n_win > 65535 || H > 65535) return -2;
   if (sp < 0 || sp > 8 || (!o && !o_peers)) return -3;
+  if (!whole_vectors(o, ldo)) return -4;
+  for (int i = 0; i < sp; ++i)
+    if (!whole_vectors(o_peers[i], push_ld | push_col0)) return -4;
   AttnFwdParams p{};
   for (int i = 0; i < sp; ++i) p.o_peers[i] = const_cast<void*>(o_peers[i]);
   p.push_n_local = o_peers ? push_n_local : 0; p.push_ld = push_ld; p.push_col0 = push_col0;
@@ -1424,6 +1433,9 @@ static int attn_bwd_impl(const void* qkv, int ldq, int q_col0, int k_col0, int v
   if (head_dim <= 0 || head_dim > 128 || head_dim % 8) return -1;
   if (n_win <= 0 || N <= 0 || H <= 0 || n_win > 65535 || H > 65535) return -2;
   if (sp < 0 || sp > 8 || (!dqkv && !dq_peers)) return -3;
+  if (!whole_vectors(o, ldo) || !whole_vectors(d_o, ldo) || !whole_vectors(dqkv, ldg | q_col0 | k_col0 | v_col0)) return -4;
+  for (int i = 0; i < sp; ++i)
+    if (!whole_vectors(dq_peers[i], push_ld | push_sec_w | push_col0)) return -4;
   AttnBwdParams p{};
   for (int i = 0; i < sp; ++i) p.dq_peers[i] = const_cast<void*>(dq_peers[i]);
   p.push_n_local = dq_peers ? push_n_local : 0; p.push_ld = push_ld; p.push_sec_w = push_sec_w; p.push_col0 = push_col0;

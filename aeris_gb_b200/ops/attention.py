@@ -16,10 +16,18 @@ def _kernel_dim(d: int) -> int:
     return 64 if d < 64 else 128
 
 
-def _padded_dim(d: int) -> int:
-    """Heads of whole 16-byte vectors are padded to the kernel's width by the tensor maps on the way into shared memory;
-    other widths run zero-padded: zero columns change neither Q K^T nor the valid columns of P V."""
-    return d if d % 8 == 0 and 0 < d <= 128 else _kernel_dim(d)
+def _whole_vectors(t: torch.Tensor | None) -> bool:
+    """Rows that start on 16-byte boundaries and have no gaps: what the kernels' 16-byte accesses need."""
+    return t is None or (t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0)
+
+
+def _padded_dim(d: int, *tensors: torch.Tensor | None) -> int:
+    """Heads of whole 16-byte vectors are padded to the kernel's width by the tensor maps on the way into shared memory.
+    Other widths, and narrow heads in ``tensors`` that do not consist of whole vectors, run as zero-padded copies: zero
+    columns change neither Q K^T nor the valid columns of P V."""
+    if d in (64, 128) or (d % 8 == 0 and 0 < d < 128 and all(map(_whole_vectors, tensors))):
+        return d
+    return _kernel_dim(d)
 
 
 def _pad_heads(t: torch.Tensor, parts: int, H: int, d: int, dp: int) -> torch.Tensor:
@@ -43,7 +51,7 @@ def attn_fwd(qkv: torch.Tensor, n_win: int, N: int, H: int, d: int, *, out: torc
     """
     T, C = qkv.shape
     assert T == n_win * N and C == 3 * H * d and qkv.dtype == torch.bfloat16 and qkv.stride(1) == 1
-    dp = _padded_dim(d)
+    dp = _padded_dim(d, qkv, out)
     if dp != d:
         o_p, lse = attn_fwd(_pad_heads(qkv, 3, H, d, dp), n_win, N, H, dp, lse=lse,
                             scale=scale if scale is not None else 1.0 / math.sqrt(d))
@@ -89,7 +97,7 @@ def attn_bwd(qkv: torch.Tensor, o: torch.Tensor, d_o: torch.Tensor, lse: torch.T
     """Gradient of :func:`attn_fwd` with respect to the fused qkv tensor (same layout as ``qkv``)."""
     T, C = qkv.shape
     assert o.shape == (T, H * d) and d_o.shape == (T, H * d) and d_o.stride(1) == 1 and o.stride(0) == d_o.stride(0)
-    dp = _padded_dim(d)
+    dp = _padded_dim(d, qkv, o, d_o, dqkv)
     if dp != d:
         g_p = attn_bwd(_pad_heads(qkv, 3, H, d, dp), _pad_heads(o, 1, H, d, dp), _pad_heads(d_o, 1, H, d, dp), lse,
                        n_win, N, H, dp, delta=delta, scale=scale if scale is not None else 1.0 / math.sqrt(d))
