@@ -1353,10 +1353,11 @@ extern "C" int aeris_attn_fwd(const void* q, int ldq, int q_col0, const void* k,
 }
 
 // Forward whose output rows are (also) pushed to the ranks that own the tokens (Ulysses return exchange fused into the
-// attention epilogue). `o` may be null when only the pushed copy is wanted.
+// attention epilogue). `o` may be null when only the pushed copy is wanted. head_dim 64 or 128.
 extern "C" int aeris_attn_fwd_push(const void* qkv, int ld, int H_local, void* o, int ldo, float* lse, int n_win, int N,
                                    int head_dim, float scale, const void* const* o_peers, int sp, int n_local,
                                    int push_ld, int push_col0, int* status, void* stream_) {
+  if (head_dim != 64 && head_dim != 128) return -1;
   const int hd = H_local * head_dim;
   return attn_fwd_impl(qkv, ld, 0, qkv, ld, hd, qkv, ld, 2 * hd, o, ldo, lse, n_win, N, H_local, head_dim, scale,
                        status, stream_, o_peers, sp, n_local, push_ld, push_col0);
@@ -1416,10 +1417,12 @@ extern "C" int aeris_attn_bwd(const void* qkv, int ldq, int q_col0, int k_col0, 
 }
 
 // Backward whose dQ / dK / dV rows are pushed to the ranks that own the tokens (layout [tokens_local, 3 * heads * d]).
+// head_dim 64 or 128.
 extern "C" int aeris_attn_bwd_push(const void* qkv, int ld, int H_local, const void* o, const void* d_o, int ldo,
                                    const float* lse, float* delta, int n_win, int N, int head_dim, float scale,
                                    const void* const* dq_peers, int sp, int n_local, int push_ld, int push_sec_w,
                                    int push_col0, int* status, void* stream_) {
+  if (head_dim != 64 && head_dim != 128) return -1;
   const int hd = H_local * head_dim;
   return attn_bwd_impl(qkv, ld, 0, hd, 2 * hd, o, d_o, ldo, lse, delta, nullptr, 0, n_win, N, H_local, head_dim, scale,
                        status, stream_, dq_peers, sp, n_local, push_ld, push_sec_w, push_col0);

@@ -88,3 +88,15 @@ def test_narrow_heads_reach_the_kernels_in_whole_vectors_or_as_padded_copies(rec
     for width, ptrs, pitches in recorder.calls:
         assert width == (d if plain else (64 if d < 64 else 128))
         assert all(p % 16 == 0 for p in ptrs) and all(ld % 8 == 0 for ld in pitches)
+
+
+@pytest.mark.parametrize("d", [8, 32, 96, 120])
+def test_push_entries_take_the_kernels_own_head_widths_only(d):
+    peers = (V * 2)(BASE, BASE)
+    H, ld, hd = 2, 6 * d, 2 * d
+    rc = L.lib().aeris_attn_fwd_push(V(BASE), ld, H, V(BASE), hd, V(BASE), 2, 16, d, ctypes.c_float(1.0), peers, 2, 8, 2 * hd,
+                                     0, V(0), V(0))
+    assert rc == -1
+    rc = L.lib().aeris_attn_bwd_push(V(BASE), ld, H, V(BASE), V(BASE), hd, V(BASE), V(BASE), 2, 16, d, ctypes.c_float(1.0),
+                                     peers, 2, 8, 6 * hd, 2 * hd, 0, V(0), V(0))
+    assert rc == -1
