@@ -164,6 +164,7 @@ def plan_kept_blocks(T: int, D: int, HD: int, heads: int, F: int, n_blocks: int,
 
 
 MIN_CHUNK_BYTES = 512 << 20
+MAX_CHUNK_WINDOWS = 65535      # the attention kernels' grid has one layer per window
 
 
 def chunk_step(meta: BlockMeta, D: int, F: int) -> int:
@@ -171,7 +172,7 @@ def chunk_step(meta: BlockMeta, D: int, F: int) -> int:
     gigabyte saves no memory worth having and costs launches that the GPU finishes faster than they are issued (32
     windows of 64 tokens at dim 128 in chunks of 8: 1,582 launches per step for 7 ms of device time)."""
     floor = MIN_CHUNK_BYTES // (kept_bytes(1, D, meta.heads * meta.head_dim, meta.heads, F) * meta.L)
-    return min(max(meta.chunk_windows, floor), meta.n_win_per_sample)
+    return min(max(meta.chunk_windows, floor), meta.n_win_per_sample, MAX_CHUNK_WINDOWS)
 
 
 def _forward_spans(meta: BlockMeta, B: int, step: int, D: int, F: int, kept: bool) -> list[tuple[int, int, int, int]]:
@@ -180,7 +181,7 @@ def _forward_spans(meta: BlockMeta, B: int, step: int, D: int, F: int, kept: boo
     anyway or take less than the smallest chunk; the exchanges of the parallel paths work on one sample at a time."""
     row = kept_bytes(1, D, meta.heads * meta.head_dim, meta.heads, F)
     if (B > 1 and step == meta.n_win_per_sample and meta.sp is None and meta.tp is None
-            and (kept or B * step * meta.L * row <= MIN_CHUNK_BYTES) and B * step <= 65535):
+            and (kept or B * step * meta.L * row <= MIN_CHUNK_BYTES) and B * step <= MAX_CHUNK_WINDOWS):
         return [(0, 0, B * step, B)]
     return [(b, w0, nw, 1) for b in range(B) for w0, nw in _chunks(meta, step)]
 

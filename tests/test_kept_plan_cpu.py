@@ -29,3 +29,14 @@ def test_chunks_below_half_a_gigabyte_are_merged(dim, heads, mlp, L, chunk, n_wi
     assert step == want
     spans = list(fused._chunks(meta, step))
     assert sum(n for _, n in spans) == n_win and [w for w, _ in spans] == list(range(0, n_win, step))
+
+
+@pytest.mark.parametrize("win,dim,mlp", [((1, 1), 128, 256), ((1, 2), 128, 256), ((2, 2), 64, 64)])
+def test_merged_chunks_stay_within_the_attention_grid(win, dim, mlp):
+    """Windows of a few tokens on the full 720 x 1440 image: half a gigabyte of them is more than the grid's 65,535 layers."""
+    L = win[0] * win[1]
+    n_win = 720 * 1440 // L
+    meta = fused.BlockMeta(n_win, L, 2, dim // 2, E.MODE_MOD_THEN_NORM, 1e-6, 64)
+    step = fused.chunk_step(meta, dim, mlp)
+    assert fused.MIN_CHUNK_BYTES // (fused.kept_bytes(1, dim, dim, 2, mlp) * L) > 65535 and step == 65535
+    assert all(nw <= 65535 for b, _, nw, _ in fused._forward_spans(meta, 2, step, dim, mlp, True))
