@@ -172,6 +172,13 @@ def use_fused(t: torch.Tensor) -> bool:
     return t.is_cuda and os.environ.get("AERIS_FORCE_ORACLE") != "1"
 
 
+def plain_values(t: torch.Tensor) -> bool:
+    """Whether ``t`` is nothing but its values: a kernel launched on the data outside of an autograd function would drop a
+    recorded gradient, a forward-mode tangent or the dimension that a ``torch.func`` transform hides."""
+    return not (t.requires_grad or torch._C._functorch.is_functorch_wrapped_tensor(t)
+                or torch.autograd.forward_ad.unpack_dual(t).tangent is not None)
+
+
 # ---------------------------------------------------------------------------------------------------- sub-modules
 class LatentEmbedding(nn.Module):
     def __init__(self, dim):
@@ -292,7 +299,7 @@ class InputStage(nn.Module):
                 return self.interval_embed(t.reshape(-1, 1).to(cfg.data_dtype)).to(cfg.model_dtype)
             n = 1 if t is None else t.reshape(-1).shape[0]
             return torch.zeros((n, cfg.dim), dtype=cfg.model_dtype, device=self.proj.weight.device)
-        if (use_fused(t) and not t.requires_grad and cfg.dim % 2 == 0 and cfg.data_dtype == torch.float32
+        if (use_fused(t) and plain_values(t) and cfg.dim % 2 == 0 and cfg.data_dtype == torch.float32
                 and cfg.model_dtype in (torch.bfloat16, torch.float32)):
             from ..ops import diffusion as DF
             emb = DF.noise_embedding(t.float().contiguous(), cfg.dim, cfg.max_period,
