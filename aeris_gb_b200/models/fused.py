@@ -455,7 +455,7 @@ class FusedBlock(torch.autograd.Function):
         ctx.regroup = regroup
         out = out_alloc(x.shape[0], x.shape[1], x.dtype) if out_alloc is not None else None
         kept = None
-        if meta.keep:
+        if meta.keep and any(ctx.needs_input_grad):        # a frozen block has no backward pass to keep anything for
             shapes = _kept_shapes(regroup[0].numel() if regroup is not None else x.shape[0], x.shape[1],
                                   meta.heads * meta.head_dim, meta.heads, w2.shape[1])
             kept = {k: torch.empty(shape, dtype=dt, device=x.device) for k, (shape, dt) in shapes.items()}

@@ -1,5 +1,6 @@
 """How many blocks keep their internals for the backward pass, and how small a chunk may get."""
 import pytest
+import torch
 
 from aeris_gb_b200.models import fused
 from aeris_gb_b200.ops import elementwise as E
@@ -40,3 +41,25 @@ def test_merged_chunks_stay_within_the_attention_grid(win, dim, mlp):
     step = fused.chunk_step(meta, dim, mlp)
     assert fused.MIN_CHUNK_BYTES // (fused.kept_bytes(1, dim, dim, 2, mlp) * L) > 65535 and step == 65535
     assert all(nw <= 65535 for b, _, nw, _ in fused._forward_spans(meta, 2, step, dim, mlp, True))
+
+
+@pytest.mark.parametrize("trains", ["x", "mod", "weight", None])
+def test_internals_are_kept_only_for_a_backward_pass_that_can_come(trains, monkeypatch):
+    """A frozen block on inputs without gradients, called without no_grad: nothing is kept. Any differentiable input: all is."""
+    seen = []
+
+    def forward(x, mod, meta, *weights, out=None, gather=None, kept=None):
+        seen.append(kept)
+        return torch.zeros_like(x)
+
+    monkeypatch.setattr(fused, "block_forward", forward)
+    meta = fused.BlockMeta(2, 4, 2, 8, E.MODE_MOD_THEN_NORM, 1e-6, 64, keep=True)
+    bf = dict(dtype=torch.bfloat16)
+    x, mod = torch.zeros(8, 16, requires_grad=trains == "x", **bf), torch.zeros(1, 96, requires_grad=trains == "mod")
+    ws = [torch.zeros(16, **bf), torch.zeros(48, 16, **bf), torch.zeros(16, 16, **bf), torch.zeros(16, **bf),
+          torch.zeros(64, 16, **bf), torch.zeros(16, 32, requires_grad=trains == "weight", **bf)]
+    y = fused.FusedBlock.apply(x, mod, meta, *ws)
+    assert y.requires_grad == (trains is not None)
+    assert (seen[0] is not None) == (trains is not None)
+    if trains:
+        assert set(seen[0]) == set(fused.KEPT) and seen[0]["u"].shape == (8, 64)
