@@ -55,6 +55,9 @@ __device__ __forceinline__ float load_any(const void* p, size_t i, bool bf16) {
   return bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i]) : reinterpret_cast<const float*>(p)[i];
 }
 
+// Most shared memory that the rows of x (B rounded up to 1, 2, 4 or 8) may take: 8 rows of 6,400 columns, 4 of 12,800.
+constexpr int GEMV_X_BYTES = 200 * 1024;
+
 // y[b, n] = act(sum_k W[n, k] silu?(x[b, k]) + bias[n]) for B <= 8 rows: one warp per output feature streams one weight
 // row, eight weights (16 bytes of bf16) per lane and load where `vec` says that rows start on 16-byte boundaries. act: 0
 // none, 1 SiLU. Bound by the weight stream; MB is B rounded up to 1, 2, 4 or 8. 30720 x 5120 bf16 (B = 1): 281 ->
@@ -268,9 +271,9 @@ extern "C" int aeris_noise_embedding(const float* t, void* out, int out_bf16, in
 extern "C" int aeris_gemv_bias_act(const void* W, int flags, const void* bias, const void* x, float* y, int N, int K, int B,
                                    int act, int silu_in, void* stream) {
   if (N <= 0 || K <= 0 || B <= 0 || B > 8) return -1;
-  if (static_cast<size_t>(B) * K * sizeof(float) > 48 * 1024) return -2;
   const int mb = B <= 1 ? 1 : B <= 2 ? 2 : B <= 4 ? 4 : 8;
-  const size_t smem = static_cast<size_t>(mb) * ((K + 3) & ~3) * sizeof(float);     // at most 96 KB and a few bytes
+  const size_t smem = static_cast<size_t>(mb) * ((K + 3) & ~3) * sizeof(float);
+  if (smem > GEMV_X_BYTES) return -2;
   const int vec = K % 8 == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0;
   int grid = (N + 7) / 8;
   const int cap = aeris_num_sms() * 8;
@@ -280,7 +283,7 @@ extern "C" int aeris_gemv_bias_act(const void* W, int flags, const void* bias, c
   do {                                                                                                                  \
     auto kern = gemv_bias_act_kernel<WT, MB>;                                                                           \
     if (smem > 48 * 1024 &&                                                                                             \
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024) != cudaSuccess)             \
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMV_X_BYTES) != cudaSuccess)           \
       return -20;                                                                                                       \
     kern<<<grid, 256, smem, st>>>(reinterpret_cast<const WT*>(W), bias, (flags >> 1) & 1, x, (flags >> 2) & 1, y, N, K, \
                                   B, act, silu_in, vec);                                                                \

@@ -538,9 +538,10 @@ class GemvLinearFn(torch.autograd.Function):
 
 
 def modulation(seq: torch.nn.Sequential, emb: torch.Tensor) -> torch.Tensor:
-    """The AdaLN modulation MLP ``[Linear,] SiLU, Linear`` (src/aeris/models/parallel_swin.py:321-325) of at most 8
-    samples on the GEMV kernel; fp32 result ``[B, out]``."""
-    if emb.shape[0] > 8:
+    """The AdaLN modulation MLP ``[Linear,] SiLU, Linear`` (src/aeris/models/parallel_swin.py:321-325) on the GEMV kernel
+    where that takes all rows of every layer (at most 8 samples), else on stock operators; fp32 result ``[B, out]``."""
+    from ..ops import diffusion as DF
+    if not all(DF.gemv_ok(emb.shape[0], m.weight.shape[1]) for m in seq if isinstance(m, torch.nn.Linear)):
         return seq(emb.to(seq[-1].weight.dtype)).float()
     x = emb
     if len(seq) == 3:

@@ -99,9 +99,16 @@ def _f32_or_bf16(t: torch.Tensor | None) -> torch.Tensor | None:
     return t if t is None or t.dtype in (torch.float32, torch.bfloat16) else t.float()
 
 
+def gemv_ok(B: int, K: int) -> bool:
+    """Whether :func:`gemv_bias_act` takes ``B`` rows of ``K`` columns: at most 8, and what the kernel pads them to (1, 2, 4
+    or 8 rows of whole vectors, fp32) in 200 KB of shared memory."""
+    return B <= 8 and 4 * (1 << (B - 1).bit_length()) * ((K + 3) // 4 * 4) <= 200 * 1024
+
+
 def gemv_bias_act(W: torch.Tensor, bias: torch.Tensor | None, x: torch.Tensor, act: int = 0,
                   silu_in: bool = False) -> torch.Tensor:
-    """``act(silu?(x) @ W^T + bias)`` for at most 8 rows of ``x``; W, bias and x bf16 or fp32, W [N, K]; fp32 result."""
+    """``act(silu?(x) @ W^T + bias)`` for the few rows of ``x`` that :func:`gemv_ok` accepts; W [N, K], bias and x bf16 or
+    fp32; fp32 result."""
     N, K = W.shape
     x, bias = _f32_or_bf16(x).contiguous(), _f32_or_bf16(bias)
     B = x.shape[0]

@@ -14,9 +14,17 @@ DEV = "cuda"
 def test_gemv_forward_and_gradients(N, K, B, silu_in):
     """Row counts around the kernel's templates, widths that are no multiple of a vector (K = 1001: scalar loads, and no
     backward kernel) or of a CTA's columns, bf16 and fp32 operands; fp32 sums of K (or N) terms, fast exp in the SiLU."""
+    _gemv_case(N, K, B, silu_in)
+
+
+@pytest.mark.parametrize("B,K", [(1, 8192), (3, 3076), (3, 4096), (3, 5120), (5, 2456), (8, 1540), (8, 5120), (8, 6400)])
+def test_gemv_rows_beyond_the_default_shared_memory(B, K):
+    """Rows of x that need more than 48 KB, up to the kernel's limit of 200 KB."""
+    _gemv_case(300, K, B, True)
+
+
+def _gemv_case(N, K, B, silu_in):
     from aeris_gb_b200.ops import diffusion as DF
-    if B * K * 4 > 48 * 1024:
-        K = 1536               # the widest x that eight rows may have
     torch.manual_seed(N + K + B)
     for wt, xt in ((torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32), (torch.bfloat16, torch.float32)):
         W, b, x = torch.randn(N, K, device=DEV).to(wt), torch.randn(N, device=DEV).to(wt), torch.randn(B, K, device=DEV).to(xt)
@@ -34,6 +42,19 @@ def test_gemv_forward_and_gradients(N, K, B, silu_in):
         dW2 = torch.ones(N, K, device=DEV)
         DF.gemv_bwd(W, x, dy, dW2, None, None, silu_in)        # without the bias and without the gradient of x
         assert torch.equal(dW, dW2)
+
+
+def test_modulation_of_three_samples_at_dim_5120():
+    """The widest model with several samples per step: both layers on the kernel, against the stock operators."""
+    from aeris_gb_b200.models.aeris import ModulationLinear
+    from aeris_gb_b200.models.fused import modulation
+    from aeris_gb_b200.ops import diffusion as DF
+    assert DF.gemv_ok(3, 5120)
+    seq = ModulationLinear(5120, 640, True).cuda().modulation
+    for p in seq.parameters():
+        torch.nn.init.normal_(p, std=0.02)
+    emb = torch.randn(3, 5120, device=DEV)
+    assert rel_err(modulation(seq, emb), seq.double()(emb.double())) < 4e-6
 
 
 def test_modulation_gradients_without_the_kernel():
