@@ -517,13 +517,16 @@ class GemvLinearFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         from ..ops import diffusion as DF
-        from .fused_io import _grad_slot
+        from .fused_io import _grad_slot, _kernel_target, _settle
         x, W, b = ctx.saved_tensors
         sW, rW = _grad_slot(W)
         sb, rb = _grad_slot(b) if b is not None else (None, None)
         dx = torch.zeros(x.shape, dtype=torch.float32, device=x.device) if ctx.needs_input_grad[0] else None
         if DF.gemv_bwd_ok(W, sW):
-            DF.gemv_bwd(W, x, dy, sW, sb, dx, ctx.silu_in)
+            tb = _kernel_target(sb) if sb is not None else None
+            DF.gemv_bwd(W, x, dy, sW, tb, dx, ctx.silu_in)
+            if sb is not None:
+                _settle(sb, tb)
         else:
             dy, x32 = dy.float(), x.float()
             sig = torch.sigmoid(x32)

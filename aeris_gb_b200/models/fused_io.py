@@ -60,6 +60,19 @@ def _grad_slot(p: torch.Tensor):
     return z, z
 
 
+def _kernel_target(slot: torch.Tensor) -> torch.Tensor:
+    """Where a kernel may add fp32 gradients by address: the slot itself, or zeros for :func:`_settle` to add to it when
+    somebody's ``main_grad`` has another type or layout."""
+    if slot.dtype == torch.float32 and slot.is_contiguous():
+        return slot
+    return torch.zeros(slot.shape, dtype=torch.float32, device=slot.device)
+
+
+def _settle(slot: torch.Tensor, target: torch.Tensor) -> None:
+    if target is not slot:
+        slot += target
+
+
 def _pack_dim(c_in: int) -> int:
     return (3 * c_in + 2 + 127) // 128 * 128
 
@@ -103,7 +116,10 @@ class EmbedFn(torch.autograd.Function):
             G.gemm(dout[r0:r0 + n], A[:n], a_t=True, b_t=True, out=Gw, epi=G.EPI_ACC_F32, k_splits=8)
         sW, rW = _grad_slot(W)
         sb, rb = _grad_slot(b)
-        DF.fold_embed_grad(Gw, sW, sb)
+        tW, tb = _kernel_target(sW), _kernel_target(sb)
+        DF.fold_embed_grad(Gw, tW, tb)
+        _settle(sW, tW)
+        _settle(sb, tb)
         return (None, None, None, rW.to(W.dtype) if rW is not None else None,
                 rb.to(b.dtype) if rb is not None else None, None)
 
@@ -194,6 +210,7 @@ class HeadLossFn(torch.autograd.Function):
         shift32, scale32 = shift.float().contiguous(), scale.float().contiguous()
         dshift, dscale = torch.zeros((2, *shift32.shape), dtype=torch.float32, device=dev).unbind(0)
         s_nw, r_nw = _grad_slot(norm_w)
+        t_nw = _kernel_target(s_nw)
         dx = torch.empty_like(x)
         dpred = dpred * g.to(dpred.dtype)
         for b, nb, r0, n in spans:
@@ -207,7 +224,8 @@ class HeadLossFn(torch.autograd.Function):
                 sl = slice(r0 + i * m, r0 + (i + 1) * m)
                 E.modnorm_bwd(x[sl], dy[i * m:(i + 1) * m], None, scale32[b + i], shift32[b + i], norm_w,
                               mode=E.MODE_NORM_THEN_MOD, eps=plan.eps, dx=dx[sl], dscale=dscale[b + i],
-                              dshift=dshift[b + i], dw=s_nw)
+                              dshift=dshift[b + i], dw=t_nw)
+        _settle(s_nw, t_nw)
         s_hw, r_hw = _grad_slot(head_w)
         s_hw += Gh[:C]
         return (dx, dshift.to(shift.dtype), dscale.to(scale.dtype), r_nw.to(norm_w.dtype) if r_nw is not None else None,
