@@ -134,7 +134,14 @@ def _head_rows(x, scale, shift, norm_w, w3, eps, pred, y):
     n = x.shape[0]
     E.modnorm_fwd(x, scale, shift, norm_w, mode=E.MODE_NORM_THEN_MOD, eps=eps, out=y[0, :n], out_lo=y[1, :n],
                   batch=scale.shape[0])
-    DF.head_gemm(y, n, w3, pred)
+    D = x.shape[1]
+    if D % 64 == 0:
+        DF.head_gemm(y, n, w3, pred)
+    else:                                  # the packed product's three sections consist of whole k-blocks
+        w_hi, w_lo = w3[:, :D], w3[:, D:2 * D]
+        G.gemm(y[1, :n], w_hi, out=pred[:n], epi=G.EPI_STORE_F32)
+        G.gemm(y[0, :n], w_lo, out=pred[:n], epi=G.EPI_ACC_F32)
+        G.gemm(y[0, :n], w_hi, out=pred[:n], epi=G.EPI_ACC_F32)
     return pred[:n]
 
 

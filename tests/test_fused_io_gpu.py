@@ -216,3 +216,20 @@ def test_device_forecaster_matches_pytorch_sampler(heun, churn):
     z = _noise_image(grid, M, (4 << 32) + 1, C) * sampler.sigma_data
     ref = Forecaster(denoise, stats, sampler, C).step(state, forcing, x_init=z)
     assert rel_err(out - state, ref - state) < 3e-2
+
+
+@pytest.mark.parametrize("D", [8, 72, 96, 128, 200])
+def test_head_of_widths_that_are_no_multiple_of_a_k_block(D):
+    """Every width in whole vectors, against 64 bits. What is dropped is lo x lo, 2^-17 of a term at most; the norm's
+    reciprocal square root and the fp32 sums stay below that."""
+    from aeris_gb_b200.models import fused_io
+    torch.manual_seed(D)
+    B, T, C = 2, 300, 70
+    x = torch.randn(T, D, device="cuda").bfloat16()
+    shift, scale, w = torch.randn(B, D, device="cuda"), torch.randn(B, D, device="cuda"), torch.rand(D, device="cuda") + 0.5
+    head = torch.randn(C, D, device="cuda")
+    got = fused_io.head_forward(x, shift, scale, w, head, 1e-6)
+    xd = x.double()
+    y = (xd * torch.rsqrt((xd * xd).mean(1, keepdim=True) + 1e-6) * w.double()).view(B, -1, D)
+    ref = (y * (1 + scale.double()[:, None]) + shift.double()[:, None]).view(T, D) @ head.double().t()
+    assert rel_err(got[:, :C], ref) < 2.0 ** -16 and not got[:, C:].any()
