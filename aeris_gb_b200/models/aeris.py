@@ -55,7 +55,10 @@ class AerisConfig:
     tp_rank: int = 0
     chunk_windows: int = 64
     shift_layers: str = "odd"       # which layers use the half-window shift: "odd" | "none"
-    oracle_checkpoint: bool = False  # PyTorch (oracle) path only: recompute every block in backward
+    # recompute every block's internals in the backward pass: ``oracle_checkpoint`` on the PyTorch (oracle) path,
+    # ``recompute`` on the CUDA path (off: blocks whose internals fit the free memory keep them)
+    oracle_checkpoint: bool = False
+    recompute: bool = False
     use_rope: bool = False          # axial 2-D rotary embedding on q, k inside every window (the reference's is inert)
     rope_base: float = 10_000.0
     # model mode (parallel_swin.py:367-376, 394-397, 474-486): ``diffusion`` conditions every block on the noise level,
@@ -535,7 +538,7 @@ class AerisModel(nn.Module):
         The last blocks keep theirs: the backward pass gives that memory back first."""
         cfg = self.cfg
         n_blocks = len(self.layers) * cfg.sublayers
-        if not (torch.is_grad_enabled() and use_fused(x)) or ctx.grid.sp > 1 or cfg.tp > 1:
+        if cfg.recompute or not (torch.is_grad_enabled() and use_fused(x)) or ctx.grid.sp > 1 or cfg.tp > 1:
             return n_blocks
         from . import fused
         return n_blocks - fused.plan_kept_blocks(x.shape[0], cfg.dim, cfg.heads * cfg.head_dim, cfg.heads, cfg.mlp_dim,

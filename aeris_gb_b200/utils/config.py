@@ -255,9 +255,9 @@ def model_config(cfg: Config):
         shift_layers=m.get("shift_mode", "odd"), diffusion=bool(m.get("diffusion", True)),
         rit=bool(m.get("rit", False)), emb_norm=bool(m.get("emb_norm", False)) and bool(m.get("rit", False)),
         tp=int(m.get("TP", 1)),
-        # model.act_ckpt: per-block recompute on the PyTorch (CPU / oracle) path; the CUDA blocks always keep only
-        # their input
-        oracle_checkpoint=bool(m.get("act_ckpt", False)))
+        # model.act_ckpt: every block recomputes its internals in the backward pass. Without it the PyTorch path keeps
+        # them all, the CUDA path those that fit the free memory
+        oracle_checkpoint=bool(m.get("act_ckpt", False)), recompute=bool(m.get("act_ckpt", False)))
 
 
 def optim_config(cfg: Config):

@@ -63,3 +63,18 @@ def test_internals_are_kept_only_for_a_backward_pass_that_can_come(trains, monke
     assert (seen[0] is not None) == (trains is not None)
     if trains:
         assert set(seen[0]) == set(fused.KEPT) and seen[0]["u"].shape == (8, 64)
+
+
+@pytest.mark.parametrize("recompute,first", [(False, 1), (True, 4)])
+def test_an_explicit_request_to_recompute_is_followed(recompute, first, monkeypatch):
+    """``model.act_ckpt: true`` reaches the CUDA path: no block keeps anything and the memory is not even asked about."""
+    from aeris_gb_b200.models import aeris as M
+    from aeris_gb_b200.utils import config as C
+    run = C.compose("train", ["experiment=tiny_cpu", f"model.act_ckpt={str(recompute).lower()}"])
+    cfg = C.model_config(run)
+    assert cfg.recompute == recompute and cfg.oracle_checkpoint == recompute and cfg.n_blocks == 4
+    model = M.AerisModel(cfg)
+    ctx = M.StreamContext(cfg, 1)
+    monkeypatch.setattr(M, "use_fused", lambda x: True)
+    monkeypatch.setattr(fused, "plan_kept_blocks", lambda *a: pytest.fail("asked") if recompute else 3)
+    assert model._first_kept_block(torch.zeros(8, cfg.dim), ctx) == first
