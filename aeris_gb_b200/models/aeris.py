@@ -540,9 +540,11 @@ class AerisModel(nn.Module):
         n_blocks = len(self.layers) * cfg.sublayers
         if cfg.recompute or not (torch.is_grad_enabled() and use_fused(x)) or ctx.grid.sp > 1 or cfg.tp > 1:
             return n_blocks
+        from ..ops import elementwise as E
         from . import fused
-        return n_blocks - fused.plan_kept_blocks(x.shape[0], cfg.dim, cfg.heads * cfg.head_dim, cfg.heads, cfg.mlp_dim,
-                                                 n_blocks, cfg.chunk_windows * ctx.grid.n_local, x.device)
+        wins, L = ctx.grid.windows_per_rank, ctx.grid.n_local
+        meta = fused.BlockMeta(wins, L, cfg.heads, cfg.head_dim, E.MODE_MOD_THEN_NORM, cfg.eps(x.dtype), cfg.chunk_windows)
+        return n_blocks - fused.plan_kept_blocks(meta, x.shape[0] // (wins * L), cfg.dim, cfg.mlp_dim, n_blocks, x.device)
 
     def trunk(self, x: torch.Tensor, dt: torch.Tensor, ctx: StreamContext) -> torch.Tensor:
         cur = (0, 0)

@@ -56,6 +56,15 @@ class Workspace:
             v.zero_()
         return v
 
+    def missing(self, shapes: dict[str, tuple[tuple[int, ...], torch.dtype]], device) -> int:
+        """Bytes of the buffers that asking for ``shapes`` would allocate."""
+        total = 0
+        for name, (shape, dtype) in shapes.items():
+            b, n = self._buf.get(name), math.prod(shape)
+            if b is None or b.numel() < n or b.dtype != dtype or b.device != torch.device(device):
+                total += n * dtype.itemsize
+        return total
+
     def clear(self):
         self._buf.clear()
 
@@ -134,33 +143,60 @@ def kept_bytes(T: int, D: int, HD: int, heads: int, F: int) -> int:
     return sum(math.prod(shape) * dt.itemsize for shape, dt in _kept_shapes(T, D, HD, heads, F).values())
 
 
+def _chunk_shapes(rows: int, D: int, HD: int, heads: int, F: int, tpn: int = 1):
+    """Chunk workspaces of a forward pass that keeps nothing, and of the recompute (``h2`` in the forward pass is ``h``).
+    ``tpn``: ranks whose rows a tensor-parallel MLP gathers."""
+    bf = torch.bfloat16
+    return {"h": ((rows, D), bf), "qkv": ((rows, 3 * HD), bf), "o": ((rows, HD), bf),
+            "lse": ((rows * heads,), torch.float32), "x1": ((rows, D), bf), "h2": ((rows, D), bf), "act": ((rows * tpn, F), bf)}
+
+
+def _grad_shapes(rows: int, D: int, HD: int, heads: int, F: int, tpn: int = 1):
+    """Workspaces of every backward pass: a chunk's gradients, the gated weights, one sample's ungated weight gradients."""
+    bf, f32 = torch.bfloat16, torch.float32
+    return {"u": ((rows * tpn, 2 * F), bf), "dh": ((rows, D), bf), "dx1": ((rows, D), bf), "d_o": ((rows, HD), bf),
+            "dqkv": ((rows, 3 * HD), bf), "delta": ((rows * heads,), f32), "w2g": ((D, F), bf), "wog": ((D, HD), bf),
+            "G2": ((D, F), f32), "Go": ((D, HD), f32)}
+
+
 def n_kept(n_blocks: int, per_block: int, base: int, free: int) -> int:
     """How many of ``n_blocks`` blocks may keep their internals: these take at most half of what is left of ``free``
     after the ``base`` bytes that the step needs in any case."""
     return max(0, min(n_blocks, (free - base) // 2 // per_block))
 
 
-def plan_kept_blocks(T: int, D: int, HD: int, heads: int, F: int, n_blocks: int, chunk_rows: int, device) -> int:
+def plan_kept_blocks(meta: BlockMeta, batch: int, D: int, F: int, n_blocks: int, device) -> int:
     """How many blocks of a training forward keep their internals instead of recomputing them in the backward pass.
 
     The recompute is a quarter of a step's tensor-core work (one more QKV, wo and w1 product and attention forward per
     block) and under the power cap time follows work, so it is only worth its price where memory is short: a full-size
-    image (1 M tokens x 40 blocks) needs it, one with a few GB of internals on a 180 GB GPU does not. What counts is the
-    memory that is free now (unused allocator cache included), less the block inputs and the chunk workspaces that the
-    step will also allocate. The driver is asked only when the allocator's own cache does not cover the need (the question
-    costs up to milliseconds on a busy host), and not at all for needs below 1/256 of the device."""
-    per_block = kept_bytes(T, D, HD, heads, F)
-    if per_block * n_blocks <= torch.cuda.get_device_properties(device).total_memory // 256:
-        return n_blocks
-    # block inputs (a shifted layer holds its source too), stream gradients, two chunk working sets
-    base = (n_blocks + 4) * T * D * 2 + 2 * kept_bytes(min(T, chunk_rows), D, HD, heads, F)
+    image (1 M tokens x 40 blocks) needs it, one with a few GB of internals on a 180 GB GPU does not. The kept internals
+    take at most half of the memory that is free now (the allocator's unused cache included) and not needed by the step
+    in any case: block inputs, stream gradients, and the workspaces that are not there yet.
+
+    One exception saves a question to the driver (0.1 to 1.6 ms each, measured): where the allocator's cache by itself covers
+    the internals of all blocks and the rest of the step, as it does from the second step on, all blocks keep theirs.
+    Fragments (unused parts of blocks in use) count there only for needs below 1/256 of the device, whose tensors of a few
+    MB fit into them; elsewhere they do not count as free at all."""
+    HD = meta.heads * meta.head_dim
+    T = batch * meta.n_win_per_sample * meta.L
+    per_block = kept_bytes(T, D, HD, meta.heads, F)
+    step = chunk_step(meta, D, F)
+    rows = step * meta.L
+    fwd_rows = max(nw for _, _, nw, _ in _forward_spans(meta, batch, step, D, F, False)) * meta.L
+    # a shifted layer holds its source beside its input
+    streams = (n_blocks + 4) * T * D * 2
+    grads = _WS.missing(_grad_shapes(rows, D, HD, meta.heads, F), device)
     stats = torch.cuda.memory_stats_as_nested_dict(device)
-    held = [stats.get(k, {}).get("all", {}).get("current", 0) for k in ("reserved_bytes", "allocated_bytes")]
-    cached = max(0, held[0] - held[1])
-    if n_blocks * (per_block + T * D * 2) <= cached:      # an earlier step's buffers, ready to be handed out again
+    reserved, allocated, fragments = (stats.get(k, {}).get("all", {}).get("current", 0)
+                                      for k in ("reserved_bytes", "allocated_bytes", "inactive_split_bytes"))
+    cached, whole = max(0, reserved - allocated), max(0, reserved - allocated - fragments)
+    need = n_blocks * per_block
+    small = need <= torch.cuda.get_device_properties(device).total_memory // 256
+    if need + streams + grads <= (cached if small else whole):
         return n_blocks
-    free = cached + torch.cuda.mem_get_info(device)[0]
-    return n_kept(n_blocks, per_block, base, free)
+    base = streams + grads + _WS.missing(_chunk_shapes(fwd_rows, D, HD, meta.heads, F), device)
+    return n_kept(n_blocks, per_block, base, whole + torch.cuda.mem_get_info(device)[0])
 
 
 MIN_CHUNK_BYTES = 512 << 20
@@ -280,16 +316,15 @@ def block_forward(x: torch.Tensor, mod: torch.Tensor, meta: BlockMeta, wn1, wqkv
     rows_per_sample = meta.n_win_per_sample * meta.L
     assert T == B * rows_per_sample
     y = out if out is not None else torch.empty_like(x)
-    ws, dev, bf = _WS, x.device, torch.bfloat16
+    ws, dev = _WS, x.device
     step = chunk_step(meta, D, F)
     spans = _forward_spans(meta, B, step, D, F, kept is not None)
     if kept is None:
         cmax = max(nw for _, _, nw, _ in spans) * meta.L
-        h = ws.get("h", (cmax, D), bf, dev)
         tpn = meta.tp.tp if meta.tp is not None else 1   # gathered rows x local features: the same element count
-        chunk_bufs = {"h1": h, "qkv": ws.get("qkv", (cmax, 3 * HD), bf, dev), "o": ws.get("o", (cmax, HD), bf, dev),
-                      "lse": ws.get("lse", (cmax * meta.heads,), torch.float32, dev),
-                      "x1": ws.get("x1", (cmax, D), bf, dev), "h2": h, "act": ws.get("act", (cmax * tpn, F), bf, dev)}
+        shapes = _chunk_shapes(cmax, D, HD, meta.heads, F, tpn)
+        chunk_bufs = {k: ws.get(k, *sh, dev) for k, sh in shapes.items() if k != "h2"}
+        chunk_bufs["h1"] = chunk_bufs["h2"] = chunk_bufs["h"]
     mods = mod.reshape(B, 6, D).transpose(0, 1).contiguous()           # [6, B, D]: every vector of all samples in a row
     for b, w0, nw, nb in spans:
         sh1, sc1, g1, sh2, sc2, g2 = (mods[:, b] if nb == 1 else mods[:, b:b + nb]).unbind(0)
@@ -337,26 +372,18 @@ def block_backward(x: torch.Tensor, mod: torch.Tensor, dy: torch.Tensor, meta: B
     F = w2.shape[1]
     HD = meta.heads * meta.head_dim
     rows_per_sample = meta.n_win_per_sample * meta.L
-    ws, dev, bf, f32 = _WS, x.device, torch.bfloat16, torch.float32
+    ws, dev, f32 = _WS, x.device, torch.float32
     step = chunk_step(meta, D, F)
     cmax = step * meta.L
     tp = meta.tp
     tpn = tp.tp if tp is not None else 1
     if kept is None:
-        act_b = ws.get("act", (cmax * tpn, F), bf, dev)
-        chunk_bufs = {"h1": ws.get("h", (cmax, D), bf, dev), "qkv": ws.get("qkv", (cmax, 3 * HD), bf, dev),
-                      "o": ws.get("o", (cmax, HD), bf, dev), "lse": ws.get("lse", (cmax * meta.heads,), f32, dev),
-                      "x1": ws.get("x1", (cmax, D), bf, dev), "h2": ws.get("h2", (cmax, D), bf, dev), "act": act_b}
-    du_b = ws.get("u", (cmax * tpn, 2 * F), bf, dev)
-    dh = ws.get("dh", (cmax, D), bf, dev)
-    dx1 = ws.get("dx1", (cmax, D), bf, dev)
-    d_o = ws.get("d_o", (cmax, HD), bf, dev)
-    dqkv = ws.get("dqkv", (cmax, 3 * HD), bf, dev)
-    delta = ws.get("delta", (cmax * meta.heads,), f32, dev)
-    w2g = ws.get("w2g", tuple(w2.shape), bf, dev)
-    wog = ws.get("wog", tuple(wo.shape), bf, dev)
-    G2 = ws.get("G2", tuple(w2.shape), f32, dev, zero=True)   # dy^T act  (ungated w2 gradient of one sample)
-    Go = ws.get("Go", tuple(wo.shape), f32, dev, zero=True)   # dx1^T o
+        chunk_bufs = {k: ws.get(k, *sh, dev) for k, sh in _chunk_shapes(cmax, D, HD, meta.heads, F, tpn).items()}
+        chunk_bufs["h1"], act_b = chunk_bufs["h"], chunk_bufs["act"]
+    du_b, dh, dx1, d_o, dqkv, delta, w2g, wog, G2, Go = \
+        (ws.get(k, *sh, dev) for k, sh in _grad_shapes(cmax, D, HD, meta.heads, F, tpn).items())
+    G2.zero_()          # dy^T act (ungated w2 gradient of one sample)
+    Go.zero_()          # dx1^T o
     dmod = torch.zeros((B, 6 * D), dtype=f32, device=dev)
     if dx is None:
         dx = torch.empty_like(x)

@@ -1,4 +1,7 @@
 """How many blocks keep their internals for the backward pass, and how small a chunk may get."""
+import math
+from types import SimpleNamespace
+
 import pytest
 import torch
 
@@ -78,3 +81,113 @@ def test_an_explicit_request_to_recompute_is_followed(recompute, first, monkeypa
     monkeypatch.setattr(M, "use_fused", lambda x: True)
     monkeypatch.setattr(fused, "plan_kept_blocks", lambda *a: pytest.fail("asked") if recompute else 3)
     assert model._first_kept_block(torch.zeros(8, cfg.dim), ctx) == first
+
+
+GB, MB = 1 << 30, 1 << 20
+
+
+class _Memory:
+    """Stands in for the allocator and the driver."""
+
+    def __init__(self, monkeypatch, driver, cached=0, fragments=0):
+        self.asked = 0
+        stat = lambda n: {"all": {"current": n}}
+        monkeypatch.setattr(fused, "_WS", fused.Workspace())
+        monkeypatch.setattr(torch.cuda, "get_device_properties", lambda d: SimpleNamespace(total_memory=180 * GB))
+        monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict", lambda d: {
+            "reserved_bytes": stat(7 * GB + cached), "allocated_bytes": stat(7 * GB), "inactive_split_bytes": stat(fragments)})
+
+        def ask(device):
+            self.asked += 1
+            return driver, 180 * GB
+        monkeypatch.setattr(torch.cuda, "mem_get_info", ask)
+
+
+# the medium model: 2 samples of 32 windows x 900 tokens, 6 blocks
+META = fused.BlockMeta(32, 900, 12, 64, E.MODE_MOD_THEN_NORM, 1e-6, 64)
+D, FF, BLOCKS, ROWS = 768, 2048, 6, 2 * 32 * 900
+NEED = BLOCKS * fused.kept_bytes(ROWS, D, D, 12, FF)
+STREAMS = (BLOCKS + 4) * ROWS * D * 2
+# chunks of one sample: bytes per row of the gradient workspaces and of the recompute's, and the weight-sized ones
+GRADS = 32 * 900 * ((2 * FF + 2 * D + 4 * D) * 2 + 12 * 4) + D * (FF + D) * 6
+CHUNK = 32 * 900 * ((3 * D + 4 * D + FF) * 2 + 12 * 4)
+
+
+def _plan(meta=META, batch=2, d=D, f=FF, blocks=BLOCKS):
+    return fused.plan_kept_blocks(meta, batch, d, f, blocks, torch.device("cpu"))
+
+
+def test_a_cache_that_covers_the_whole_step_needs_no_question(monkeypatch):
+    mem = _Memory(monkeypatch, driver=0, cached=NEED + STREAMS + GRADS)
+    assert _plan() == BLOCKS and mem.asked == 0
+
+
+@pytest.mark.parametrize("short", [0, 1])
+def test_a_cache_that_covers_only_what_is_kept_leaves_room_for_the_step(short, monkeypatch):
+    """The internals alone fit the cache and the driver has nothing left: what the step needs besides comes first."""
+    cached = NEED if short else NEED + STREAMS + GRADS - 1
+    mem = _Memory(monkeypatch, driver=0, cached=cached)
+    want = (cached - STREAMS - GRADS - CHUNK) // 2 // (NEED // BLOCKS)
+    assert _plan() == want < BLOCKS and mem.asked == 1
+    assert want * (NEED // BLOCKS) + STREAMS + GRADS + CHUNK <= cached
+
+
+def test_workspaces_that_are_there_are_not_counted_again(monkeypatch):
+    mem = _Memory(monkeypatch, driver=0, cached=NEED + STREAMS)
+    assert _plan() < BLOCKS and mem.asked == 1
+    for name, (shape, dtype) in fused._grad_shapes(32 * 900, D, D, 12, FF).items():
+        fused._WS._buf[name] = torch.empty(shape, dtype=dtype, device="meta").flatten()
+    monkeypatch.setattr(fused._WS, "missing", lambda shapes, device: fused.Workspace.missing(fused._WS, shapes, "meta"))
+    assert _plan() == BLOCKS and mem.asked == 1
+
+
+def test_fragments_are_not_free_memory(monkeypatch):
+    mem = _Memory(monkeypatch, driver=0, cached=NEED + STREAMS + GRADS, fragments=NEED)
+    assert _plan() == 0 and mem.asked == 1
+
+
+def test_the_driver_s_memory_is_shared_half_and_half(monkeypatch):
+    free = STREAMS + GRADS + CHUNK + NEED                 # half of the rest: three of six blocks
+    mem = _Memory(monkeypatch, driver=free)
+    assert _plan() == BLOCKS // 2 and mem.asked == 1
+    _Memory(monkeypatch, driver=free + NEED)
+    assert _plan() == BLOCKS
+
+
+def test_a_small_model_on_a_full_device_recomputes(monkeypatch):
+    """Needs below 1/256 of the device are not exempt: with 100 MB left in all, a step that needs more keeps nothing. With
+    the fragments of an earlier step in the cache (its tensors of a few MB fit them) the driver is not asked."""
+    meta = fused.BlockMeta(8, 900, 4, 64, E.MODE_MOD_THEN_NORM, 1e-6, 4)
+    need = 2 * fused.kept_bytes(7200, 256, 256, 4, 512)
+    assert need < 180 * GB // 256
+    mem = _Memory(monkeypatch, driver=100 * MB)
+    assert _plan(meta, 1, 256, 512, 2) == 0 and mem.asked == 1
+    mem = _Memory(monkeypatch, driver=0, cached=need + 200 * MB, fragments=need)
+    assert _plan(meta, 1, 256, 512, 2) == 2 and mem.asked == 0
+
+
+def test_the_plan_counts_the_workspaces_that_the_passes_use(monkeypatch):
+    """The tables behind the plan are the ones that the passes allocate from, merged samples included."""
+    asked = {}
+
+    class Spy(fused.Workspace):
+        def get(self, name, shape, dtype, device, zero=False):
+            asked[name] = max(asked.get(name, 0), math.prod(shape) * dtype.itemsize)
+            return super().get(name, shape, dtype, device, zero)
+
+    monkeypatch.setattr(fused, "_WS", Spy())
+    for mod, names in ((fused.E, ("modnorm_fwd", "modnorm_bwd", "scale_rows", "gate_grad_finalize")),
+                       (fused.G, ("gemm",)), (fused.A, ("attn_fwd", "attn_bwd"))):
+        for n in names:
+            monkeypatch.setattr(mod, n, lambda *a, **k: None)
+    meta = fused.BlockMeta(4, 16, 2, 8, E.MODE_MOD_THEN_NORM, 1e-6, 64)
+    bf = torch.bfloat16
+    ws = [torch.zeros(s, dtype=bf) for s in ((16,), (48, 16), (16, 16), (16,), (64, 16), (16, 32))]
+    x, mod = torch.zeros(2 * 64, 16, dtype=bf), torch.zeros(2, 96)
+    fused.block_forward(x, mod, meta, *ws)
+    grads = {k: torch.zeros(w.shape) for k, w in zip(("n1", "to_qkv", "wo", "n2", "w1", "w2"), ws)}
+    fused.block_backward(x, mod, x.clone(), meta, *ws, grads)
+    shapes = {**fused._chunk_shapes(128, 16, 16, 2, 32), **fused._grad_shapes(64, 16, 16, 2, 32)}
+    assert asked["h"] == math.prod(shapes["h"][0]) * 2 and set(asked) == set(shapes)
+    empty = fused.Workspace()
+    assert sum(asked.values()) <= empty.missing(shapes, "cpu")
