@@ -571,12 +571,14 @@ def modulation(seq: torch.nn.Sequential, emb: torch.Tensor) -> torch.Tensor:
     """The AdaLN modulation MLP ``[Linear,] SiLU, Linear`` (src/aeris/models/parallel_swin.py:321-325) on the GEMV kernel
     where that takes all rows of every layer (at most 8 samples), else on stock operators; fp32 result ``[B, out]``."""
     from ..ops import diffusion as DF
-    if not all(DF.gemv_ok(emb.shape[0], m.weight.shape[1]) for m in seq if isinstance(m, torch.nn.Linear)):
-        return seq(emb.to(seq[-1].weight.dtype)).float()
+    last = seq[-1]
+    w = last.weight
+    if not DF.gemv_ok(emb.shape[0], max(emb.shape[1], w.shape[1])):
+        return seq(emb.to(w.dtype)).float()
     x = emb
     if len(seq) == 3:
         x = GemvLinearFn.apply(x, seq[0].weight, seq[0].bias, False)
-    return GemvLinearFn.apply(x, seq[-1].weight, seq[-1].bias, True)
+    return GemvLinearFn.apply(x, w, last.bias, True)
 
 
 class Regroup(torch.autograd.Function):
