@@ -114,6 +114,8 @@ int aeris_noise_embedding(const float* t, void* out, int out_bf16, int B, int di
 int aeris_pack_embed_weights(const float* W, const float* b, void* out, int D, int Cin, int KP, void* stream);
 int aeris_fold_embed_grad(const float* G, float* dW, float* db, int D, int Cin, int KP, void* stream);
 int aeris_pack_head_weights(const float* W, void* out, int C, int rows, int D, void* stream);
+// Slices that k_splits <= 0 stands for: `tiles` output tiles over `units` CTAs or CTA pairs (see gemm.cu).
+int aeris_choose_k_splits(int tiles, int kb_total, int units, int most, int want);
 int aeris_gemm_split(const void* y, const void* w, float* C, int M, int D, int lo_row, int ldc, int* status, void* stream);
 
 #ifdef __cplusplus

@@ -262,6 +262,37 @@ int num_sms() {
   return g_num_sms;
 }
 
+// Split of the reduction dimension of an accumulating product (weight gradients: few output tiles, a reduction over all
+// tokens): the number of slices, from four to `most`, that minimises rounds x (k-blocks per slice + fixed cost of a slice),
+// a round being one slice per unit (CTA or CTA pair). Constant four left the last round of many shapes nearly empty and small
+// weights (dim 256: 4 slices on 74 pairs) on a handful of SMs. The fixed cost, filling the ring and adding the tile's fp32
+// values to memory, is taken as 10 k-blocks of 64. More than four slices have at least eight k-blocks on average (the last
+// one holds what is left). The one-CTA kernel, whose products are narrow, stays at four.
+// Four slices and now: 512 x 512 x 28800: 43.6 -> 22.6 us, 768 x 2048 x 28800: 83.6 -> 69.6 us, 1536 x 4096 x 64800:
+// 716 -> 621 us.
+// Slices also bound the error: the tensor core truncates at every addition, so that of a sum grows with its slice (9e-10 of
+// the result per row: 1.4e-7 for slices of 128 rows, 8e-6 for 7,200). `want` slices are what the caller's sums had when they
+// came in more and shorter products; of the numbers from there down, the first that costs at most a quarter more than the
+// cheapest is taken. Error of the separate products, of one with the cheapest slices and of this rule: 512 x 128 x 2048 for
+// 4 x 512 rows 1.4e-7 / 4.7e-7 / 1.4e-7 (67, 18 and 18 us); 1024 x 4096 x 9000 for 16 windows of 225 at a time 8.2e-7 /
+// 2.3e-6 / 7.9e-7 (124, 66 and 101 us); 4096 x 512 x 27540 for 4 windows of 135 2.8e-7 / 3.2e-6 / 1.2e-6 (1028, 93, 119 us).
+int choose_k_splits(int tiles, int kb_total, int units, int most, int want) {
+  auto cost = [&](int s) {
+    const long long rounds = (static_cast<long long>(tiles) * s + units - 1) / units;
+    return rounds * ((kb_total + s - 1) / s + 10);
+  };
+  int best = kb_total < 4 ? kb_total : 4;
+  for (int s = 5; s <= most && kb_total / s >= 8; ++s)
+    if (cost(s) < cost(best)) best = s;
+  if (want > kb_total) want = kb_total;
+  for (int per = want > 0 ? (kb_total + want - 1) / want : kb_total; per < kb_total; ++per) {
+    const int s = (kb_total + per - 1) / per;
+    if (s <= best) break;
+    if (4 * cost(s) <= 5 * cost(best)) return s;
+  }
+  return best;
+}
+
 template <int BN, int A_MN, int B_MN>
 static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, cudaStream_t stream) {
   using S = GemmSmem<BN>;
@@ -285,6 +316,10 @@ using namespace aeris;
 
 int aeris_num_sms() { return aeris::num_sms(); }
 
+extern "C" int aeris_choose_k_splits(int tiles, int kb_total, int units, int most, int want) {
+  return tiles <= 0 || kb_total <= 0 || units <= 0 ? -1 : choose_k_splits(tiles, kb_total, units, most, want);
+}
+
 extern "C" int aeris_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb,
                                int ldc, int a_mn, int b_mn, int epi, const void* resid, int ldr,
                                const float* gate, int rows_per_gate, void* aux, int ld_aux, int swiglu_f,
@@ -295,7 +330,9 @@ extern "C" int aeris_gemm_bf16(const void* A, const void* B, void* C, int M, int
   if (N % bn != 0) return -2;
   const bool swiglu_fwd = (epi == EPI_SWIGLU || epi == EPI_SWIGLU_BOTH);
   if (swiglu_fwd && b_mn) return -3;
-  if (k_splits < 1) k_splits = 1;
+  if (k_splits < 1)
+    k_splits = epi != EPI_ACC_F32 ? 1
+             : choose_k_splits(((M + BM - 1) / BM) * (N / bn), (K + BK - 1) / BK, num_sms(), 4, -k_splits);
   if (k_splits > 1 && epi != EPI_ACC_F32) return -4;
   GemmParams p{};
   p.M = M; p.N = N; p.K = K; p.epi = epi; p.C = C; p.ldc = ldc;

@@ -303,24 +303,6 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   if (warp == 1) tmem_dealloc2(tmem_base, 2 * G2_BN);
 }
 
-// Split of the reduction dimension of an accumulating product (weight gradients: few output tiles, a reduction over all
-// tokens): the number of slices that minimises rounds x (k-blocks per slice + fixed cost of a slice), a round being one
-// slice per CTA pair. Constant four left the last round of many shapes nearly empty and small weights (dim 256: 4 slices
-// on 74 pairs) on a handful of SMs. The fixed cost, filling the ring and adding 256 x 256 fp32 values to memory, is
-// taken as 10 k-blocks of 64; slices of fewer than 8 are not made, and never fewer than four slices: the tensor core
-// truncates at every addition, so longer slices would be less accurate. Four slices
-// and now: 512 x 512 x 28800: 43.6 -> 22.6 us, 768 x 2048 x 28800: 83.6 -> 69.6 us, 1536 x 4096 x 64800: 716 -> 621 us.
-static int auto_k_splits(int mn_tiles, int kb_total, int pairs) {
-  int best = 4;
-  long long best_cost = 0x7fffffffffffll;
-  for (int s = 4; s <= 64 && (s == 4 || kb_total / s >= 8); ++s) {
-    const long long rounds = (static_cast<long long>(mn_tiles) * s + pairs - 1) / pairs;
-    const long long cost = rounds * ((kb_total + s - 1) / s + 10);
-    if (cost < best_cost) { best_cost = cost; best = s; }
-  }
-  return best;
-}
-
 template <int A_MN, int B_MN, int EW, bool AG = false>
 static int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p_in, cudaStream_t stream) {
   static bool configured = false;
@@ -350,7 +332,7 @@ static int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
     if (getenv("AERIS_DEBUG")) fprintf(stderr, "gemm2: max active clusters %d\n", n);
   }
   int clusters = max_clusters;
-  if (p.k_splits == 0) p.k_splits = auto_k_splits(mn_tiles, (p.K + G2_BK - 1) / G2_BK, clusters);
+  if (p.k_splits <= 0) p.k_splits = choose_k_splits(mn_tiles, (p.K + G2_BK - 1) / G2_BK, clusters, 64, -p.k_splits);
   const int tiles = mn_tiles * p.k_splits;
   if (tiles < clusters && !AG) clusters = tiles;
   if (AG) p.ag_expect *= static_cast<unsigned>(2 * clusters);   // came in as the call index
@@ -363,7 +345,7 @@ static int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
 using namespace aeris;
 
 // Same contract as aeris_gemm_bf16 (api.h); N must be a multiple of 128 (of 256 for the SwiGLU forward epilogues, whose
-// tiles pair gate and up columns). k_splits = 0 with EPI_ACC_F32: chosen by auto_k_splits.
+// tiles pair gate and up columns).
 extern "C" int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb,
                                     int ldc, int a_mn, int b_mn, int epi, const void* resid, int ldr,
                                     const float* gate, int rows_per_gate, void* aux, int ld_aux, int swiglu_f,
@@ -373,7 +355,7 @@ extern "C" int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M
   const bool swiglu_fwd = (epi == EPI_SWIGLU || epi == EPI_SWIGLU_BOTH);
   if (N % (swiglu_fwd ? G2_BN : G2_BN / 2) != 0) return -2;
   if (swiglu_fwd && b_mn) return -3;
-  if (k_splits < 0 || (k_splits == 0 && epi != EPI_ACC_F32)) k_splits = 1;
+  if (k_splits < 1 && epi != EPI_ACC_F32) k_splits = 1;
   if (k_splits > 1 && epi != EPI_ACC_F32) return -4;
   GemmParams p{};
   p.M = M; p.N = N; p.K = K; p.epi = epi; p.C = C; p.ldc = ldc;

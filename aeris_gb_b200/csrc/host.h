@@ -11,4 +11,6 @@ int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64
 int make_tmap_heads_bf16(CUtensorMap* out, const void* base, int d, int heads, int tokens, int windows, uint64_t ld,
                          uint32_t box_rows);
 int num_sms();
+// Slices of an accumulating product's reduction over `kb_total` blocks of 64: see gemm.cu.
+int choose_k_splits(int tiles, int kb_total, int units, int most, int want);
 }  // namespace aeris

@@ -388,7 +388,8 @@ def block_backward(x: torch.Tensor, mod: torch.Tensor, dy: torch.Tensor, meta: B
     if dx is None:
         dx = torch.empty_like(x)
     mod = mod.contiguous()
-    ksplit_tok = 0      # the kernel chooses
+    # four slices per chunk of `chunk_windows`: what a merged chunk's weight gradients should keep of the shorter sums
+    slices = lambda nw: -4 * -(-nw // min(meta.chunk_windows, meta.n_win_per_sample))
     for b in range(B):
         sh1, sc1, g1, sh2, sc2, g2 = [mod[b, i * D:(i + 1) * D] for i in range(6)]
         dsh1, dsc1, dg1, dsh2, dsc2, dg2 = [dmod[b, i * D:(i + 1) * D] for i in range(6)]
@@ -398,6 +399,7 @@ def block_backward(x: torch.Tensor, mod: torch.Tensor, dy: torch.Tensor, meta: B
             r0 = b * rows_per_sample + w0 * meta.L
             n = nw * meta.L
             xc, dyc = x[r0:r0 + n], dy[r0:r0 + n]
+            ksplit_tok = slices(nw)
             h1, qkv, o, x1, h2, act, lse = _chunk_views(kept, r0, n, meta.heads) if kept is not None else \
                 _chunk_views(chunk_bufs, 0, n, meta.heads)
             lse_c = lse.view(nw, meta.heads, meta.L)

@@ -224,7 +224,7 @@ class HeadLossFn(torch.autograd.Function):
             E.modnorm_fwd(x[r0:r0 + n], scale32[b:b + nb], shift32[b:b + nb], norm_w, mode=E.MODE_NORM_THEN_MOD,
                           eps=plan.eps, out=y_hi[:n], batch=nb)
             dp = dpred[r0:r0 + n]
-            G.gemm(dp, y_hi[:n], a_t=True, b_t=True, out=Gh, epi=G.EPI_ACC_F32, k_splits=16, two_cta=False)
+            G.gemm(dp, y_hi[:n], a_t=True, b_t=True, out=Gh, epi=G.EPI_ACC_F32, k_splits=16 * nb, two_cta=False)
             G.gemm(dp, w_hi, b_t=True, out=dy[:n])
             m = n // nb
             for i in range(nb):        # column sums per sample

@@ -32,7 +32,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
     EPI_GATE_RESID ``resid + gate * acc`` (gate fp32 ``[M // rows_per_gate, N]``; ``aux`` optionally receives the
     raw product); EPI_ACC_F32 ``out += acc`` in fp32 (split-K allowed); EPI_STORE_F32 fp32 out;
     EPI_SWIGLU_BOTH = EPI_SWIGLU that also writes the raw ``[gate | up]`` product to ``aux [M, 2F]``;
-    ``k_splits``: slices of the reduction dimension (EPI_ACC_F32 only); 0 lets the kernel choose.
+    ``k_splits``: slices of the reduction dimension (EPI_ACC_F32 only); 0 lets the kernel choose, -n as well but towards n
+    slices, for sums that should be no less accurate than those of n shorter products.
     EPI_SWIGLU_BWD: the product is d(act) ``[M, F]``, ``resid`` holds ``u = [gate | up]`` and ``out`` receives d(u).
     """
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
@@ -75,8 +76,6 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
         return out
     if bn == 0:
         bn = 256 if N % 256 == 0 else 128
-    if k_splits == 0:        # this kernel's fixed choice: enough slices to fill the SMs on narrow weights
-        k_splits = 4
     rc = _l.lib().aeris_gemm_bf16(
         _l.ptr(a), _l.ptr(b), _l.ptr(out), M, N, K, _ld(a), _ld(b), _ld(out), int(a_t), int(b_t), epi,
         _l.ptr(resid), _ld(resid) if resid is not None else 0, _l.ptr(gate), rows_per_gate,
