@@ -140,7 +140,9 @@ __device__ __forceinline__ void group_sum4(float (&s)[4], float* red, int lane, 
 // (plain RMSNorm). With `gidx`, source row r comes from peers.p[gidx[r] >> 28] at row (gidx[r] & 0x0fffffff), and
 // the gathered row is also written to x_out.
 constexpr int FWD_RPI = 4;  // rows per iteration of one CTA: one block-wide reduction serves four rows
-__global__ void modnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __restrict__ gidx,
+// Serves rows wider than 5120 columns (up to 1024 threads, register cap 64).
+__global__ void __launch_bounds__(1024, 1)
+modnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __restrict__ gidx,
                                    PeerPtrs peers, __nv_bfloat16* __restrict__ x_out,
                                    const float* __restrict__ scale, const float* __restrict__ shift,
                                    const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ h, int rows,

@@ -269,11 +269,11 @@ def test_attention_bwd_tile_edges(nw, N, H, d):
 
 
 @pytest.mark.parametrize("rows,D", [(1, 8), (5, 128), (3601, 256), (30, 264), (999, 768), (301, 1536), (7, 1544),
-                                    (300, 2048), (40, 2568), (151, 5120)])
+                                    (300, 2048), (40, 2568), (151, 5120), (151, 5128), (70, 8192)])
 @pytest.mark.parametrize("mode", [0, 1])
 def test_modnorm_row_widths(rows, D, mode):
     """One row group per CTA, several, one vector per thread and two, widths that leave threads idle, rows that leave
-    groups idle, and the edges of the variants (1536, 5120). fp32 sums over the rows and columns of bf16 inputs:
+    groups idle, and the edges of the variants (1536, 5120, 8192). fp32 sums over the rows and columns of bf16 inputs:
     2^-24 relative per addition; the outputs are rounded to bf16 (2^-9 at most). Targets of the column sums may start
     at any 4-byte address."""
     from aeris_gb_b200.ops import elementwise as E
