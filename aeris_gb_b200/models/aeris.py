@@ -54,6 +54,7 @@ class AerisConfig:
     tp: int = 1
     tp_rank: int = 0
     chunk_windows: int = 64
+    min_chunk_bytes: int | None = None  # None: chunks with less than half a gigabyte of internals are merged; 0: none is
     shift_layers: str = "odd"       # which layers use the half-window shift: "odd" | "none"
     # recompute every block's internals in the backward pass: ``oracle_checkpoint`` on the PyTorch (oracle) path,
     # ``recompute`` on the CUDA path (off: blocks whose internals fit the free memory keep them)
@@ -389,7 +390,8 @@ class SwinLayer(nn.Module):
                                        E.MODE_MOD_THEN_NORM if after_mod_norm else E.MODE_NORM_THEN_MOD,
                                        eps, cfg.chunk_windows, sp=ctx.sp_exchange if ctx.grid.sp > 1 else None,
                                        rope=ctx.rope(x.device), tp=ctx.tp_exchange if cfg.tp > 1 else None,
-                                       keep=keep_from is not None and j >= keep_from)
+                                       keep=keep_from is not None and j >= keep_from,
+                                       min_chunk_bytes=cfg.min_chunk_bytes)
                 if cfg.tp > 1 and ctx.tp_exchange is None:
                     raise RuntimeError("tensor parallelism on CUDA needs StreamContext.tp_exchange (tensor.TPExchange)")
                 rg = None
@@ -543,7 +545,8 @@ class AerisModel(nn.Module):
         from ..ops import elementwise as E
         from . import fused
         wins, L = ctx.grid.windows_per_rank, ctx.grid.n_local
-        meta = fused.BlockMeta(wins, L, cfg.heads, cfg.head_dim, E.MODE_MOD_THEN_NORM, cfg.eps(x.dtype), cfg.chunk_windows)
+        meta = fused.BlockMeta(wins, L, cfg.heads, cfg.head_dim, E.MODE_MOD_THEN_NORM, cfg.eps(x.dtype), cfg.chunk_windows,
+                               min_chunk_bytes=cfg.min_chunk_bytes)
         return n_blocks - fused.plan_kept_blocks(meta, x.shape[0] // (wins * L), cfg.dim, cfg.mlp_dim, n_blocks, x.device)
 
     def trunk(self, x: torch.Tensor, dt: torch.Tensor, ctx: StreamContext) -> torch.Tensor:

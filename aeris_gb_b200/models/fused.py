@@ -35,6 +35,11 @@ class BlockMeta:
     rope: tuple | None = None          # (cos, sin) [L, head_dim / 2]: optional 2-D rotary embedding of q and k
     tp: object | None = None           # parallel.tensor.TPExchange: w1 / w2 are this rank's shards of the MLP weights
     keep: bool = False                 # forward keeps its internals for the backward pass (see plan_kept_blocks)
+    min_chunk_bytes: int | None = None  # chunks with fewer bytes of internals are merged; None: MIN_CHUNK_BYTES
+
+    @property
+    def chunk_floor(self) -> int:
+        return MIN_CHUNK_BYTES if self.min_chunk_bytes is None else self.min_chunk_bytes
 
 
 class Workspace:
@@ -206,8 +211,9 @@ MAX_CHUNK_WINDOWS = 65535      # the attention kernels' grid has one layer per w
 def chunk_step(meta: BlockMeta, D: int, F: int) -> int:
     """Windows per chunk: ``meta.chunk_windows`` bounds the working set, but a chunk whose internals take less than half a
     gigabyte saves no memory worth having and costs launches that the GPU finishes faster than they are issued (32
-    windows of 64 tokens at dim 128 in chunks of 8: 1,582 launches per step for 7 ms of device time)."""
-    floor = MIN_CHUNK_BYTES // (kept_bytes(1, D, meta.heads * meta.head_dim, meta.heads, F) * meta.L)
+    windows of 64 tokens at dim 128 in chunks of 8: 1,582 launches per step for 7 ms of device time). With
+    ``min_chunk_bytes = 0`` the bound is ``chunk_windows`` itself."""
+    floor = meta.chunk_floor // (kept_bytes(1, D, meta.heads * meta.head_dim, meta.heads, F) * meta.L)
     return min(max(meta.chunk_windows, floor), meta.n_win_per_sample, MAX_CHUNK_WINDOWS)
 
 
@@ -217,7 +223,7 @@ def _forward_spans(meta: BlockMeta, B: int, step: int, D: int, F: int, kept: boo
     anyway or take less than the smallest chunk; the exchanges of the parallel paths work on one sample at a time."""
     row = kept_bytes(1, D, meta.heads * meta.head_dim, meta.heads, F)
     if (B > 1 and step == meta.n_win_per_sample and meta.sp is None and meta.tp is None
-            and (kept or B * step * meta.L * row <= MIN_CHUNK_BYTES) and B * step <= MAX_CHUNK_WINDOWS):
+            and (kept or B * step * meta.L * row <= meta.chunk_floor) and B * step <= MAX_CHUNK_WINDOWS):
         return [(0, 0, B * step, B)]
     return [(b, w0, nw, 1) for b in range(B) for w0, nw in _chunks(meta, step)]
 

@@ -251,7 +251,7 @@ def model_config(cfg: Config):
         layerwise_t_emb=bool(m.get("layerwise_t_emb", False)),
         after_mod_norm=bool(m.get("layerwise_t_emb_after_mod_norm", False)),
         max_period=float(m.get("sinusoidal_emb_max_period", 10000)), wp=(m.get("WP_Y", 1), m.get("WP_X", 1)),
-        chunk_windows=int(m.get("chunk_windows", 64)), norm_eps=m.get("norm_eps"),
+        chunk_windows=int(m.get("chunk_windows", 64)), min_chunk_bytes=m.get("min_chunk_bytes"), norm_eps=m.get("norm_eps"),
         shift_layers=m.get("shift_mode", "odd"), diffusion=bool(m.get("diffusion", True)),
         rit=bool(m.get("rit", False)), emb_norm=bool(m.get("emb_norm", False)) and bool(m.get("rit", False)),
         tp=int(m.get("TP", 1)),

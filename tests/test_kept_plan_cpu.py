@@ -222,3 +222,22 @@ def test_every_wanted_number_is_met_or_its_price_is_above_a_quarter():
                 per = -(-kb // min(want, kb))
                 finer = {-(-kb // p) for p in range(per, kb + 1)}
                 assert not [f for f in finer if s < f and 4 * cost(tiles, kb, f) <= 5 * cost(tiles, kb, best)]
+
+
+def test_chunk_windows_bounds_a_chunk_when_asked_to(monkeypatch):
+    """``model.min_chunk_bytes: 0``: small chunks are not merged, neither windows nor samples, whatever reads the bound."""
+    from aeris_gb_b200.models import aeris as M
+    from aeris_gb_b200.utils import config as C
+    cfg = C.model_config(C.compose("train", ["experiment=tiny_cpu", "+model.min_chunk_bytes=0", "model.chunk_windows=3"]))
+    assert cfg.min_chunk_bytes == 0
+    assert C.model_config(C.compose("train", ["experiment=tiny_cpu"])).min_chunk_bytes is None
+    meta = fused.BlockMeta(8, 16, 4, 32, E.MODE_MOD_THEN_NORM, 1e-6, 3, min_chunk_bytes=0)
+    step = fused.chunk_step(meta, 128, 256)
+    assert step == 3 and [n for _, n in fused._chunks(meta, step)] == [3, 3, 2]
+    whole = fused.BlockMeta(8, 16, 4, 32, E.MODE_MOD_THEN_NORM, 1e-6, 8, min_chunk_bytes=0)
+    assert len(fused._forward_spans(whole, 2, 8, 128, 256, False)) == 2
+    seen = {}
+    monkeypatch.setattr(M, "use_fused", lambda x: True)
+    monkeypatch.setattr(fused, "plan_kept_blocks", lambda meta, *a: seen.update(meta=meta) or 0)
+    M.AerisModel(cfg)._first_kept_block(torch.zeros(8, cfg.dim), M.StreamContext(cfg, 1))
+    assert seen["meta"].min_chunk_bytes == 0 and seen["meta"].chunk_windows == 3
