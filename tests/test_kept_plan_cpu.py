@@ -228,7 +228,8 @@ def test_chunk_windows_bounds_a_chunk_when_asked_to(monkeypatch):
     """``model.min_chunk_bytes: 0``: small chunks are not merged, neither windows nor samples, whatever reads the bound."""
     from aeris_gb_b200.models import aeris as M
     from aeris_gb_b200.utils import config as C
-    cfg = C.model_config(C.compose("train", ["experiment=tiny_cpu", "+model.min_chunk_bytes=0", "model.chunk_windows=3"]))
+    cfg = C.model_config(C.compose("train", ["experiment=tiny_cpu", "+model.min_chunk_bytes=0", "model.chunk_windows=3",
+                                               "model.act_ckpt=false"]))
     assert cfg.min_chunk_bytes == 0
     assert C.model_config(C.compose("train", ["experiment=tiny_cpu"])).min_chunk_bytes is None
     meta = fused.BlockMeta(8, 16, 4, 32, E.MODE_MOD_THEN_NORM, 1e-6, 3, min_chunk_bytes=0)
