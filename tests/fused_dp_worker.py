@@ -22,7 +22,7 @@ def main():
     dist.init_process_group("nccl", device_id=dev)
     wp = wp_grid_for(world)
     cfg = AerisConfig(img=(64, 128), window=(16, 16), in_channels=12, out_channels=6, dim=128, heads=2, head_dim=64,
-                      mlp_dim=256, n_layers=2, sublayers=1, norm_eps=1e-3, chunk_windows=3, wp=wp)
+                      mlp_dim=256, n_layers=2, sublayers=1, norm_eps=1e-3, chunk_windows=3, min_chunk_bytes=0, wp=wp)
     ocfg = OptimConfig(lr=1e-3, lr_rampup_img=0, grad_clip_max_norm=0.05, weight_decay=0.1, decay_policy="all",
                        ema_halflife_img=50, ema_rampup_ratio=None)
     dcfg = DiffusionConfig(cond_channels=6)

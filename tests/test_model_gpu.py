@@ -16,11 +16,19 @@ def _small_cfg(after_mod_norm=True, head_dim=64, window=(16, 16)):
                        norm_eps=1e-3, chunk_windows=3)
 
 
+def _recompute_in_chunks(cfg, recompute):
+    """Every block recomputes in chunks of three of its eight windows (two full ones and a remainder), or keeps its internals."""
+    if recompute:
+        cfg.recompute, cfg.min_chunk_bytes = True, 0
+    return cfg
+
+
+@pytest.mark.parametrize("recompute", [False, True])
 @pytest.mark.parametrize("after_mod_norm", [True, False])
-def test_fused_model_matches_oracle(after_mod_norm):
+def test_fused_model_matches_oracle(after_mod_norm, recompute):
     from aeris_gb_b200.models.aeris import AerisModel
     torch.manual_seed(1)
-    cfg = _small_cfg(after_mod_norm)
+    cfg = _recompute_in_chunks(_small_cfg(after_mod_norm), recompute)
     model = AerisModel(cfg).cuda()
     for n, p in model.named_parameters():
         if "modulation" in n and p.dim() == 2:
@@ -53,12 +61,13 @@ def test_fused_model_matches_oracle(after_mod_norm):
         assert rel_err(a, b) < 8e-2, (n, rel_err(a, b))
 
 
-def test_fused_model_with_rope_matches_oracle():
+@pytest.mark.parametrize("recompute", [False, True])
+def test_fused_model_with_rope_matches_oracle(recompute):
     """Optional 2-D rotary embedding: the CUDA path (rotation applied to the qkv chunks, inverse rotation of their
     gradients) against the PyTorch formulation."""
     from aeris_gb_b200.models.aeris import AerisModel
     torch.manual_seed(2)
-    cfg = _small_cfg()
+    cfg = _recompute_in_chunks(_small_cfg(), recompute)
     cfg.use_rope = True
     model = AerisModel(cfg).cuda()
     for n, p in model.named_parameters():
@@ -91,13 +100,15 @@ def test_fused_model_with_rope_matches_oracle():
         assert rel_err(a, b) < 8e-2
 
 
-def test_wide_block_dim5120_matches_oracle():
+@pytest.mark.parametrize("recompute", [False, True])
+def test_wide_block_dim5120_matches_oracle(recompute):
     """The block dimensions of the 13 B-class configuration (dim 5120, 40 heads x 128, 30 x 30 windows) on a small
     image: forward and input gradient of the CUDA path against the PyTorch formulation."""
     from aeris_gb_b200.models.aeris import AerisConfig, AerisModel
     torch.manual_seed(4)
     cfg = AerisConfig(img=(60, 120), window=(30, 30), in_channels=20, out_channels=8, dim=5120, heads=40, head_dim=128,
                       mlp_dim=13824, n_layers=2, sublayers=1, norm_eps=1e-3, chunk_windows=3)
+    _recompute_in_chunks(cfg, recompute)
     model = AerisModel(cfg).cuda()
     for n, p in model.named_parameters():
         if "modulation" in n and p.dim() == 2:
@@ -176,7 +187,8 @@ def test_kept_internals_give_the_gradients_of_the_recompute(mod_first, monkeypat
         first = {n: p.grad.float().clone() for n, p in model.named_parameters() if p.grad is not None}
         model.zero_grad(set_to_none=True)
         loss.backward()
-        runs[keep] = (y.detach(), first, {n: p.grad.float().clone() for n, p in model.named_parameters() if p.grad is not None})
+        second = {n: p.grad.float().clone() for n, p in model.named_parameters() if p.grad is not None}
+        runs[keep] = (y.detach(), first, second)
     for keep in (3, n_blocks):
         assert torch.equal(runs[keep][0], runs[0][0])
         for got in runs[keep][1:]:

@@ -36,7 +36,7 @@ def main():
         dist.init_process_group("gloo")
     par = dict(wp=(1, 1), sp=world) if mode == "sp" else dict(wp=(1, world), sp=1)
     base = dict(img=(32, 64 * world), window=(16, 16), in_channels=10, out_channels=4, dim=256, heads=4, head_dim=64,
-                mlp_dim=256 * world, n_layers=2, sublayers=1, norm_eps=1e-3, chunk_windows=3,
+                mlp_dim=256 * world, n_layers=2, sublayers=1, norm_eps=1e-3, chunk_windows=3, min_chunk_bytes=0,
                 model_dtype=torch.bfloat16 if cuda else torch.float32, **par)
     ocfg = OptimConfig(lr=1e-3, lr_rampup_img=0, grad_clip_max_norm=0.5)     # the clip is active: one shared norm
     dcfg = DiffusionConfig(cond_channels=6)
