@@ -146,7 +146,7 @@ modnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __restri
                                    PeerPtrs peers, __nv_bfloat16* __restrict__ x_out,
                                    const float* __restrict__ scale, const float* __restrict__ shift,
                                    const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ h, int rows,
-                                   int D, int mode, float eps, int rows_per_cta, const float* __restrict__ wf,
+                                   int D, int mode, float eps, const float* __restrict__ wf,
                                    __nv_bfloat16* __restrict__ h_lo) {
   __shared__ float red[2 * FWD_RPI * 32];
   const int c0 = threadIdx.x * 8;
@@ -162,7 +162,6 @@ modnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __restri
   // CTAs sweep the rows together (CTA b takes row groups b, b + grid, ...). The rows of the next group are requested
   // before the current group is reduced, so every thread keeps up to eight 16-byte loads in flight across the
   // block-wide reduction.
-  (void)rows_per_cta;
   const int r1 = rows;
   const int stride = gridDim.x * FWD_RPI;
   uint4 nxt[FWD_RPI];
@@ -1005,7 +1004,6 @@ static int modnorm_fwd_impl(const void* x, const void* gidx, const void* const* 
   for (int i = 0; i < n_peers && i < 16; ++i) pp.p[i] = reinterpret_cast<const __nv_bfloat16*>(peer_ptrs[i]);
   if (gidx && n_peers <= 0) return -2;
   AERIS_FILL_CHECK(pp, n_peers);
-  const int rpc = pick_rows_per_cta(rows);
   int grid = (rows + FWD_RPI - 1) / FWD_RPI;
   if (D <= 5120) {
     // as many CTAs as the registers of an SM hold at once, each sweeping over the rows
@@ -1024,7 +1022,7 @@ static int modnorm_fwd_impl(const void* x, const void* gidx, const void* const* 
   modnorm_fwd_kernel<<<grid, row_threads(D), 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const uint32_t*>(gidx), pp,
       reinterpret_cast<__nv_bfloat16*>(x_out), scale, shift, reinterpret_cast<const __nv_bfloat16*>(w),
-      reinterpret_cast<__nv_bfloat16*>(h), rows, D, mode, eps, rpc, w_f32, reinterpret_cast<__nv_bfloat16*>(h_lo));
+      reinterpret_cast<__nv_bfloat16*>(h), rows, D, mode, eps, w_f32, reinterpret_cast<__nv_bfloat16*>(h_lo));
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 

@@ -44,12 +44,6 @@ def ape_tables(cfg, device) -> tuple[torch.Tensor, torch.Tensor]:
     return ty[off:].contiguous().to(device), tx.contiguous().to(device)
 
 
-def _split(t: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
-    """bf16 value and bf16 remainder of an fp32 tensor (what the packing kernels write)."""
-    hi = t.to(torch.bfloat16)
-    return hi, (t - hi.float()).to(torch.bfloat16)
-
-
 def _grad_slot(p: torch.Tensor):
     """fp32 accumulation target of a parameter: the engine's ``main_grad`` view, or a fresh buffer handed back to
     autograd."""

