@@ -7,8 +7,10 @@
 // Data layout: tokens are window-major, rows [w*N, (w+1)*N) belong to window w; Q, K, V are column slices of a
 // row-major [T, ld] bf16 tensor (the fused qkv projection output, columns ordered (q|k|v, head, d)).
 //
-// Every kernel has the same skeleton (192 threads): warp 0 = TMA producer, warp 1 = MMA issuer and TMEM owner,
-// warps 2..5 = one thread per tile row doing the softmax-side math straight out of TMEM.
+// Roles are the same in every kernel: warp 0 = TMA producer, warp 1 = MMA issuer and TMEM owner, and warpgroups of math
+// warps, one thread per tile row, that work straight out of TMEM. The forward kernel has one such group (warps 2..5 of 192
+// threads). The backward kernels have two or three from warp 4 on (384 or 512 threads); warps 2 and 3 fetch the row
+// statistics there.
 #include "common.cuh"
 #include "api.h"
 #include "host.h"
@@ -542,8 +544,9 @@ static int launch_attn_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const C
 // back into the tensor memory columns they came from and are the A operand of the accumulating products from there:
 // no shared-memory round trip, and the B operand is all that those products read from shared memory.
 // Both kernels together, before (two 32-column halves in flight per CTA, P and dS through shared memory) and now:
-// 72 windows x 900 tokens, 24 heads x 64: 2.60 -> 1.76 ms; 12 heads x 128: 2.66 -> 1.50 ms; 16 windows x 3600 tokens,
-// 12 heads x 128: 8.65 -> 4.4 ms (730 TFLOP/s of the five products counted).
+// 72 windows x 900 tokens, 24 heads x 64: 2.61 -> 1.72 ms; 12 heads x 128: 2.67 -> 1.49 ms; 16 windows x 3600 tokens,
+// 12 heads x 128: 7.05 -> 3.80 ms (12 launches each from an idle clock; 1.91, 1.69 and 4.35 ms held for 0.6 s, at
+// 1740, 1725 and 1665 MHz under the power cap).
 struct AttnBwdParams {
   const __nv_bfloat16* O;   // forward output, [T, ldo]
   const __nv_bfloat16* dO;  // [T, ldo]
@@ -658,7 +661,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   const int nkv = nfull + (rem ? 1 : 0);
   const int n_last = rem ? ((rem + 15) & ~15) : BT;
   const int row_tiles = (N + TILE - 1) / TILE;
-  const int n_items = (n_items_total - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
+  const int n_ctas = static_cast<int>(gridDim.x);
+  const int n_items = (n_items_total - static_cast<int>(blockIdx.x) + n_ctas - 1) / n_ctas;
 
   if (threadIdx.x == 0) {
     int ab = (p.status && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
@@ -672,7 +676,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     for (int i = 0; i < 2; ++i) { mbar_init(&stat_full[i], 2); mbar_init(&stat_empty[i], 4 * NWG); }
     for (int i = 0; i < NB; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); }
     for (int i = 0; i < NST; ++i) mbar_init(&kv_empty[i], 1);
-    for (int i = 0; i < NWG; ++i) { mbar_init(&first_full[i], 1); mbar_init(&next_full[i], 4 + 1); mbar_init(&sp_full[i], 1); }
+    for (int i = 0; i < NWG; ++i) {
+      mbar_init(&first_full[i], 1);
+      mbar_init(&next_full[i], 4 + 1);
+      mbar_init(&sp_full[i], 1);
+    }
     mbar_init(acc_full, 1); mbar_init(acc_empty, 4 * NWG);
     fence_barrier_init();
   }
@@ -752,10 +760,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         const uint64_t d2 = make_smem_desc(aS + s_st * R::STAGE, 0, 1024), d3 = d2 + KB / 16;
 #pragma unroll
         for (int kk = 0; kk < 4 * DCH; ++kk)
-          umma_ss(tS, d0 + ((kk >> 2) * 16384 + (kk & 3) * 32) / 16, d2 + ((kk >> 2) * 8192 + (kk & 3) * 32) / 16, idesc, kk > 0);
+          umma_ss(tS, d0 + ((kk >> 2) * 16384 + (kk & 3) * 32) / 16, d2 + ((kk >> 2) * 8192 + (kk & 3) * 32) / 16, idesc,
+                  kk > 0);
 #pragma unroll
         for (int kk = 0; kk < 4 * DCH; ++kk)
-          umma_ss(tS + 64, d1 + ((kk >> 2) * 16384 + (kk & 3) * 32) / 16, d3 + ((kk >> 2) * 8192 + (kk & 3) * 32) / 16, idesc, kk > 0);
+          umma_ss(tS + 64, d1 + ((kk >> 2) * 16384 + (kk & 3) * 32) / 16, d3 + ((kk >> 2) * 8192 + (kk & 3) * 32) / 16, idesc,
+                  kk > 0);
         tc_commit(&sp_full[s_w]);
         if (last) tc_commit(&q_empty[b]);
         if (++s_w == NWG) s_w = 0;
@@ -933,8 +943,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             tmem_wait_ld();
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-              float d0 = mufu_exp2(fmaf(__uint_as_float(sv[2 * i]), p.scale_log2, nlse)) * (__uint_as_float(dv[2 * i]) + ndelta);
-              float d1 = mufu_exp2(fmaf(__uint_as_float(sv[2 * i + 1]), p.scale_log2, nlse)) * (__uint_as_float(dv[2 * i + 1]) + ndelta);
+              const float p0 = mufu_exp2(fmaf(__uint_as_float(sv[2 * i]), p.scale_log2, nlse));
+              const float p1 = mufu_exp2(fmaf(__uint_as_float(sv[2 * i + 1]), p.scale_log2, nlse));
+              float d0 = p0 * (__uint_as_float(dv[2 * i]) + ndelta);
+              float d1 = p1 * (__uint_as_float(dv[2 * i + 1]) + ndelta);
               if (c + 2 * i >= rem) d0 = 0.f;
               if (c + 2 * i + 1 >= rem) d1 = 0.f;
               pk[i] = pack_bf16x2(d0, d1);
@@ -996,7 +1008,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const int nq = nfull + (rem ? 1 : 0);
   const int n_last = rem ? ((rem + 15) & ~15) : BT;
   const int row_tiles = (N + TILE - 1) / TILE;
-  const int n_items = (n_items_total - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
+  const int n_ctas = static_cast<int>(gridDim.x);
+  const int n_items = (n_items_total - static_cast<int>(blockIdx.x) + n_ctas - 1) / n_ctas;
 
   if (threadIdx.x == 0) {
     int ab = (p.status && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
@@ -1010,7 +1023,11 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     for (int i = 0; i < NB; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1); }
     for (int i = 0; i < NST; ++i) mbar_init(&qd_empty[i], 1);
     // a tile's arrivals: the TMA loads and 32 lanes of row statistics (plus, from the second round on, four math warps)
-    for (int i = 0; i < NWG; ++i) { mbar_init(&first_full[i], 1 + 32); mbar_init(&next_full[i], 4 + 1 + 32); mbar_init(&sp_full[i], 1); }
+    for (int i = 0; i < NWG; ++i) {
+      mbar_init(&first_full[i], 1 + 32);
+      mbar_init(&next_full[i], 4 + 1 + 32);
+      mbar_init(&sp_full[i], 1);
+    }
     mbar_init(acc_full, 1); mbar_init(acc_empty, 4 * NWG);
     fence_barrier_init();
   }
@@ -1090,10 +1107,12 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const uint64_t d2 = make_smem_desc(aS + s_st * R::STAGE, 0, 1024), d3 = d2 + QB / 16;
 #pragma unroll
         for (int kk = 0; kk < 4 * DCH; ++kk)
-          umma_ss(tS, d0 + ((kk >> 2) * 16384 + (kk & 3) * 32) / 16, d2 + ((kk >> 2) * 8192 + (kk & 3) * 32) / 16, idesc, kk > 0);
+          umma_ss(tS, d0 + ((kk >> 2) * 16384 + (kk & 3) * 32) / 16, d2 + ((kk >> 2) * 8192 + (kk & 3) * 32) / 16, idesc,
+                  kk > 0);
 #pragma unroll
         for (int kk = 0; kk < 4 * DCH; ++kk)
-          umma_ss(tS + 64, d1 + ((kk >> 2) * 16384 + (kk & 3) * 32) / 16, d3 + ((kk >> 2) * 8192 + (kk & 3) * 32) / 16, idesc, kk > 0);
+          umma_ss(tS + 64, d1 + ((kk >> 2) * 16384 + (kk & 3) * 32) / 16, d3 + ((kk >> 2) * 8192 + (kk & 3) * 32) / 16, idesc,
+                  kk > 0);
         tc_commit(&sp_full[s_w]);
         if (last) tc_commit(&kv_empty[b]);
         if (++s_w == NWG) s_w = 0;
@@ -1181,7 +1200,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     bool ok = true;
     // Columns past the window's end have zero Q and dO rows and zero statistics (P = 1, dS = 0): they add nothing. Rows
     // past its end may hold anything: they are not stored.
-    auto pair = [&](uint32_t s0, uint32_t s1, uint32_t d0, uint32_t d1, uint64_t l, uint64_t de, uint32_t& pp, uint32_t& dd) {
+    auto pair = [&](uint32_t s0, uint32_t s1, uint32_t d0, uint32_t d1, uint64_t l, uint64_t de, uint32_t& pp,
+                    uint32_t& dd) {
       float t0, t1;
       f2_unpack(f2_fma(f2_pack(__uint_as_float(s0), __uint_as_float(s1)), nsl, l), t0, t1);     // -(log2 P)
       const uint64_t pr = f2_pack(mufu_exp2(-t0), mufu_exp2(-t1));
@@ -1382,7 +1402,7 @@ static int attn_fwd_impl(const void* q, int ldq, int q_col0, const void* k, int 
   p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
   CUtensorMap tq, tk, tv;
   int r;
-  auto at = [](const void* base, int col) { return static_cast<const void*>(reinterpret_cast<const __nv_bfloat16*>(base) + col); };
+  auto at = [](const void* base, int col) -> const void* { return reinterpret_cast<const __nv_bfloat16*>(base) + col; };
   if ((r = make_tmap_heads_bf16(&tq, at(q, q_col0), head_dim, H, N, n_win, ldq, TILE))) return r;
   if ((r = make_tmap_heads_bf16(&tk, at(k, k_col0), head_dim, H, N, n_win, ldk, KVT))) return r;
   if ((r = make_tmap_heads_bf16(&tv, at(v, v_col0), head_dim, H, N, n_win, ldv, KVT))) return r;
@@ -1450,8 +1470,10 @@ static int attn_bwd_impl(const void* qkv, int ldq, int q_col0, int k_col0, int v
   int r;
   const __nv_bfloat16* b = reinterpret_cast<const __nv_bfloat16*>(qkv);
   const struct { CUtensorMap* m; const void* base; int ld; uint32_t rows; } maps[] = {
-      {&q128, b + q_col0, ldq, TILE}, {&q64, b + q_col0, ldq, BT}, {&k128, b + k_col0, ldq, TILE}, {&k64, b + k_col0, ldq, BT},
-      {&v128, b + v_col0, ldq, TILE}, {&v64, b + v_col0, ldq, BT}, {&d128, d_o, ldo, TILE},        {&d64, d_o, ldo, BT}};
+      {&q128, b + q_col0, ldq, TILE}, {&q64, b + q_col0, ldq, BT},
+      {&k128, b + k_col0, ldq, TILE}, {&k64, b + k_col0, ldq, BT},
+      {&v128, b + v_col0, ldq, TILE}, {&v64, b + v_col0, ldq, BT},
+      {&d128, d_o, ldo, TILE},        {&d64, d_o, ldo, BT}};
   for (const auto& m : maps)
     if ((r = make_tmap_heads_bf16(m.m, m.base, head_dim, H, N, n_win, m.ld, m.rows))) return r;
   return head_dim <= 64 ? launch_attn_bwd<1>(q128, k64, v64, d128, q64, k128, v128, d64, p, stream)

@@ -14,7 +14,8 @@ namespace aeris {
 // out[b, :] = [sin(t f_i) | cos(t f_i)], f_i = exp(-ln(max_period) i / half). Double precision: a handful of values, and the
 // fast single-precision sine would cost accuracy at large angles.
 template <typename OT>
-__global__ void noise_embedding_kernel(const float* __restrict__ t, OT* __restrict__ out, int B, int dim, double log_period) {
+__global__ void noise_embedding_kernel(const float* __restrict__ t, OT* __restrict__ out, int B, int dim,
+                                       double log_period) {
   const int half = dim / 2;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < B * half; i += gridDim.x * blockDim.x) {
     const int b = i / half, k = i - b * half;
@@ -91,7 +92,8 @@ gemv_bias_act_kernel(const WT* __restrict__ W, const void* __restrict__ bias, in
         load_w8(wr + k, w);
 #pragma unroll
         for (int b = 0; b < MB; ++b) {
-          const float4 a = *reinterpret_cast<const float4*>(xs + b * Kp + k), c = *reinterpret_cast<const float4*>(xs + b * Kp + k + 4);
+          const float4* xv = reinterpret_cast<const float4*>(xs + b * Kp + k);
+          const float4 a = xv[0], c = xv[1];
           acc[b] = fmaf(w[0], a.x, acc[b]); acc[b] = fmaf(w[1], a.y, acc[b]);
           acc[b] = fmaf(w[2], a.z, acc[b]); acc[b] = fmaf(w[3], a.w, acc[b]);
           acc[b] = fmaf(w[4], c.x, acc[b]); acc[b] = fmaf(w[5], c.y, acc[b]);
@@ -224,7 +226,8 @@ __global__ void pack_embed_weights_kernel(const float* __restrict__ W, const flo
 // dW[d, c] += G[d, c] + G[d, Cin + c], db[d] += G[d, 3 Cin].
 __global__ void fold_embed_grad_kernel(const float* __restrict__ G, float* __restrict__ dW, float* __restrict__ db, int D,
                                        int Cin, int KP) {
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < static_cast<long long>(D) * (Cin + 1);
+  const long long n = static_cast<long long>(D) * (Cin + 1);
+  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const int d = static_cast<int>(i / (Cin + 1)), c = static_cast<int>(i - static_cast<long long>(d) * (Cin + 1));
     const float* g = G + static_cast<size_t>(d) * KP;
@@ -233,7 +236,8 @@ __global__ void fold_embed_grad_kernel(const float* __restrict__ G, float* __res
   }
 }
 // Rows [hi(W) | lo(W) | hi(W)] (bf16, [rows, 3 D]) of the fp32 head weight [C, D]; rows past C are zero.
-__global__ void pack_head_weights_kernel(const float* __restrict__ W, __nv_bfloat16* __restrict__ out, int C, int rows, int D) {
+__global__ void pack_head_weights_kernel(const float* __restrict__ W, __nv_bfloat16* __restrict__ out, int C, int rows,
+                                         int D) {
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < static_cast<long long>(rows) * D;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const int r = static_cast<int>(i / D), c = static_cast<int>(i - static_cast<long long>(r) * D);
@@ -257,7 +261,8 @@ static int small_grid(long long n) {
 }
 static int launched() { return cudaGetLastError() == cudaSuccess ? 0 : -21; }
 
-extern "C" int aeris_noise_embedding(const float* t, void* out, int out_bf16, int B, int dim, double max_period, void* stream) {
+extern "C" int aeris_noise_embedding(const float* t, void* out, int out_bf16, int B, int dim, double max_period,
+                                     void* stream) {
   if (B <= 0 || dim <= 0 || dim % 2 || !(max_period > 0)) return -1;
   const cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int grid = small_grid(static_cast<long long>(B) * (dim / 2));
@@ -289,7 +294,8 @@ extern "C" int aeris_gemv_bias_act(const void* W, int flags, const void* bias, c
                                   B, act, silu_in, vec);                                                                \
   } while (0)
 #define AERIS_GEMV_MB(WT) \
-  do { if (mb == 1) AERIS_GEMV(WT, 1); else if (mb == 2) AERIS_GEMV(WT, 2); else if (mb == 4) AERIS_GEMV(WT, 4); else AERIS_GEMV(WT, 8); } while (0)
+  do { if (mb == 1) AERIS_GEMV(WT, 1); else if (mb == 2) AERIS_GEMV(WT, 2); \
+       else if (mb == 4) AERIS_GEMV(WT, 4); else AERIS_GEMV(WT, 8); } while (0)
   if (flags & 1) AERIS_GEMV_MB(float); else AERIS_GEMV_MB(__nv_bfloat16);
 #undef AERIS_GEMV_MB
 #undef AERIS_GEMV
@@ -313,9 +319,11 @@ extern "C" int aeris_gemv_bwd(const void* W, int flags, const void* x, const flo
   const int mb = B <= 1 ? 1 : B <= 2 ? 2 : B <= 4 ? 4 : 8;
   const cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 #define AERIS_GEMV(WT, MB) \
-  gemv_bwd_kernel<WT, MB><<<grid, nt, 0, st>>>(reinterpret_cast<const WT*>(W), x, (flags >> 2) & 1, dy, dW, db, dx, N, K, B, silu_in, rows)
+  gemv_bwd_kernel<WT, MB><<<grid, nt, 0, st>>>(reinterpret_cast<const WT*>(W), x, (flags >> 2) & 1, dy, dW, db, dx, N, K, \
+                                               B, silu_in, rows)
 #define AERIS_GEMV_MB(WT) \
-  do { if (mb == 1) AERIS_GEMV(WT, 1); else if (mb == 2) AERIS_GEMV(WT, 2); else if (mb == 4) AERIS_GEMV(WT, 4); else AERIS_GEMV(WT, 8); } while (0)
+  do { if (mb == 1) AERIS_GEMV(WT, 1); else if (mb == 2) AERIS_GEMV(WT, 2); \
+       else if (mb == 4) AERIS_GEMV(WT, 4); else AERIS_GEMV(WT, 8); } while (0)
   if (flags & 1) AERIS_GEMV_MB(float); else AERIS_GEMV_MB(__nv_bfloat16);
 #undef AERIS_GEMV_MB
 #undef AERIS_GEMV
@@ -331,8 +339,8 @@ extern "C" int aeris_pack_embed_weights(const float* W, const float* b, void* ou
 
 extern "C" int aeris_fold_embed_grad(const float* G, float* dW, float* db, int D, int Cin, int KP, void* stream) {
   if (D <= 0 || Cin <= 0 || KP < 3 * Cin + 2) return -1;
-  fold_embed_grad_kernel<<<small_grid(static_cast<long long>(D) * (Cin + 1)), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      G, dW, db, D, Cin, KP);
+  const int grid = small_grid(static_cast<long long>(D) * (Cin + 1));
+  fold_embed_grad_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(G, dW, db, D, Cin, KP);
   return launched();
 }
 

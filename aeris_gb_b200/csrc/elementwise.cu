@@ -502,8 +502,8 @@ modnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 //     1,184 single-group CTAs, which took most of the time on narrow rows.
 //   * VPT = 2 (rows wider than 1536) halves the threads that a row's sum has to cross and reads scale, shift and weight
 //     from shared memory; one row per reduction is what the registers hold then (two spilled).
-// Before and now: 28800 x 512 columns 110 -> 26 us, 28800 x 768 117 -> 37 us, 64800 x 1536 203 -> 142 us (5.6 TB/s),
-// 28800 x 5120 500 -> 330 us.
+// Before and now (mode 0, held for 0.3 s at 1890-1965 MHz): 28800 x 512 columns 111 -> 26 us, 28800 x 768 115 -> 37 us,
+// 64800 x 1536 211 -> 144 us (5.5 TB/s), 28800 x 5120 459 -> 347 us (mode 1: 447 -> 314).
 template <int VPT, int RPI, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1)
 modnorm_bwd_group_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dh,
@@ -514,7 +514,8 @@ modnorm_bwd_group_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
                          int vec_atomics) {
   static_assert(RPI <= 2, "group_sum4 adds two values of two rows");
   constexpr bool PSMEM = VPT > 1;
-  extern __shared__ __align__(16) float sm[];    // [groups][3][D] column sums; with PSMEM first [3][D]: 1 + scale, shift, weight
+  // [groups][3][D] column sums; with PSMEM first [3][D]: 1 + scale, shift, weight
+  extern __shared__ __align__(16) float sm[];
   __shared__ float red[MAXT / 32][2][64];
   const int groups = blockDim.x / nt;
   const int grp = threadIdx.x / nt, tid = threadIdx.x - grp * nt;
@@ -706,7 +707,8 @@ modnorm_bwd_group_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
     if (!dst) continue;
     dst += c;
     if (vec_atomics) {
-      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                   : "memory");
     } else {
       atomicAdd(dst, v.x); atomicAdd(dst + 1, v.y); atomicAdd(dst + 2, v.z); atomicAdd(dst + 3, v.w);
     }
@@ -1030,7 +1032,8 @@ extern "C" int aeris_modnorm_fwd(const void* x, const void* gidx, const void* co
                                  void* x_out, const float* scale, const float* shift, const void* w, void* h,
                                  int rows, int D, int mode, float eps, const float* w_f32, void* h_lo,
                                  void* stream) {
-  return modnorm_fwd_impl(x, gidx, peer_ptrs, n_peers, x_out, scale, shift, w, h, rows, D, mode, eps, w_f32, h_lo, 1, stream);
+  return modnorm_fwd_impl(x, gidx, peer_ptrs, n_peers, x_out, scale, shift, w, h, rows, D, mode, eps, w_f32, h_lo, 1,
+                          stream);
 }
 
 // The same for `batch` samples of `rows` consecutive rows each, scale and shift [batch, D]: one launch where D <= 5120.
@@ -1040,8 +1043,11 @@ extern "C" int aeris_modnorm_fwd_batch(const void* x, const void* gidx, const vo
                                        void* stream) {
   if (batch <= 0 || batch > 65535) return -1;
   if (D <= 5120)
-    return modnorm_fwd_impl(x, gidx, peer_ptrs, n_peers, x_out, scale, shift, w, h, rows, D, mode, eps, w_f32, h_lo, batch, stream);
-  auto at = [](const void* p, size_t bytes) -> char* { return p ? reinterpret_cast<char*>(const_cast<void*>(p)) + bytes : nullptr; };
+    return modnorm_fwd_impl(x, gidx, peer_ptrs, n_peers, x_out, scale, shift, w, h, rows, D, mode, eps, w_f32, h_lo, batch,
+                            stream);
+  auto at = [](const void* p, size_t bytes) -> char* {
+    return p ? reinterpret_cast<char*>(const_cast<void*>(p)) + bytes : nullptr;
+  };
   for (int b = 0; b < batch; ++b) {
     const size_t r = static_cast<size_t>(b) * rows, e = r * D * 2;
     const int rc = modnorm_fwd_impl(at(x, e), at(gidx, r * 4), peer_ptrs, n_peers, at(x_out, e),
@@ -1065,9 +1071,12 @@ extern "C" int aeris_modnorm_bwd(const void* x, const void* dh, const void* dres
     const int smem = (groups + (vpt > 1 ? 1 : 0)) * 3 * D * 4;
     const int need = (rows + groups - 1) / groups;
     const int grid = need < aeris_num_sms() ? need : aeris_num_sms();
-    const int vec = ((reinterpret_cast<uintptr_t>(dscale) | reinterpret_cast<uintptr_t>(dshift) | reinterpret_cast<uintptr_t>(dw)) & 15) == 0;
+    const uintptr_t sums = reinterpret_cast<uintptr_t>(dscale) | reinterpret_cast<uintptr_t>(dshift) |
+                           reinterpret_cast<uintptr_t>(dw);
+    const int vec = (sums & 15) == 0;
     auto kern = vpt == 1 ? modnorm_bwd_group_kernel<1, 2, 384> : modnorm_bwd_group_kernel<2, 1, 320>;
-    if (smem > 32 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess)
+    if (smem > 32 * 1024 &&
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess)
       return -20;
     kern<<<grid, groups * nt, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
         reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(dh),

@@ -264,12 +264,12 @@ int num_sms() {
 
 // Split of the reduction dimension of an accumulating product (weight gradients: few output tiles, a reduction over all
 // tokens): the number of slices, from four to `most`, that minimises rounds x (k-blocks per slice + fixed cost of a slice),
-// a round being one slice per unit (CTA or CTA pair). Constant four left the last round of many shapes nearly empty and small
-// weights (dim 256: 4 slices on 74 pairs) on a handful of SMs. The fixed cost, filling the ring and adding the tile's fp32
-// values to memory, is taken as 10 k-blocks of 64. More than four slices have at least eight k-blocks on average (the last
+// a round being one slice per unit (CTA or CTA pair). Constant four left the last round of many shapes nearly empty and
+// small weights (dim 256: 4 slices on 74 pairs) on a handful of SMs. The fixed cost, filling the ring and adding the tile's
+// fp32 values to memory, is taken as 10 k-blocks of 64. More than four slices have at least eight k-blocks on average (the last
 // one holds what is left). The one-CTA kernel, whose products are narrow, stays at four.
-// Four slices and now: 512 x 512 x 28800: 43.6 -> 22.6 us, 768 x 2048 x 28800: 83.6 -> 69.6 us, 1536 x 4096 x 64800:
-// 716 -> 621 us.
+// Four slices and now, held for 0.6 s: 512 x 512 x 28800: 43.0 -> 22.1 us (1965 MHz); under the power cap 768 x 2048 x
+// 28800: 94.8 -> 87.0 us, 1536 x 4096 x 64800: 699 -> 662 us.
 // Slices also bound the error: the tensor core truncates at every addition, so that of a sum grows with its slice (9e-10 of
 // the result per row: 1.4e-7 for slices of 128 rows, 8e-6 for 7,200). `want` slices are what the caller's sums had when they
 // came in more and shorter products; of the numbers from there down, the first that costs at most a quarter more than the
@@ -370,12 +370,12 @@ extern "C" int aeris_gemm_bf16(const void* A, const void* B, void* C, int M, int
 }
 
 // C[M, 128] (fp32) = lo(y) W_hi^T + hi(y) W_lo^T + hi(y) W_hi^T in one pass: the output head at fp32-level accuracy. `y`
-// holds the hi parts in its first rows and the lo parts from row `lo_row` on ([*, D] bf16), `w` the rows [W_hi | W_lo | W_hi]
-// ([128, 3 D] bf16). D must be a multiple of 64. The small terms come first: the tensor core truncates at every addition, so
+// holds the hi parts in its first rows and the lo parts from row `lo_row` on ([*, D] bf16), `w` the rows
+// [W_hi | W_lo | W_hi] ([128, 3 D] bf16). D must be a multiple of 64. The small terms come first: the tensor core truncates at every addition, so
 // with the large sum already in the accumulator they would cost its last bits (error against 64 bits at D = 1536 8.8e-6
 // in the order hi, lo, hi; 4.7e-6 in this one and for three separate products). Three products wrote the 128 fp32 columns
 // once and added to them twice, a read and a write each, for little arithmetic (65536 rows of 1536, norm included:
-// 300 -> 229 us).
+// 312 -> 227 us, 12 launches).
 extern "C" int aeris_gemm_split(const void* y, const void* w, float* C, int M, int D, int lo_row, int ldc, int* status,
                                 void* stream_) {
   if (M <= 0 || D <= 0 || D % BK || lo_row < M || ldc < 128 || ldc % 4) return -1;

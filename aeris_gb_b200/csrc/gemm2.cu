@@ -386,10 +386,13 @@ extern "C" int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M
   }
   if (r) return r - 100;
   // Eight epilogue warps where the epilogue takes longer than the products of a tile. Four warps and six stages against
-  // eight and five, us: gated residual 28800 x 768 x 768 63 / 52, 64800 x 1536 x 1536 269 / 241; SwiGLU backward
-  // 64800 x 4096 x 1536 1306 / 1068, x 768 224 / 182; SwiGLU with the raw columns 28800 x 4096 x 768 190 / 167; plain
-  // store 28800 x 2304 x 768 89 / 84, but 64800 x 4608 x 1536 597 / 624 and its data gradient 220 / 258. Weight gradients
-  // (a_mn) lose a few per cent. Requesting the SwiGLU operands a step ahead spills at eight warps (1068 -> 1240).
+  // eight and five, us, held for 0.6 s (1.2-1.8 GHz under the power cap): gated residual 28800 x 768 x 768 62 / 53, 64800 x
+  // 1536 x 1536 311 / 284, 28800 x 2048 x 2048 217 / 210, x 2304 x 2304 255 / 256, x 3072 x 3072 424 / 436; SwiGLU backward
+  // 64800 x 4096 x 1536 1106 / 985, 28800 x 5376 x 2048 735 / 690, x 6144 x 2304 885 / 832, x 8192 x 3072 1334 / 1321;
+  // SwiGLU with the raw columns 28800 x 4096 x 768 220 / 191, x 8192 x 1536 615 / 611, x 10752 x 2048 999 / 1035, x 12288 x
+  // 2304 1270 / 1309. One line at 2048 for the three: the SwiGLU backward would gain above it, the raw columns lose below.
+  // Plain store 28800 x 2304 x 768 104 / 98, x 3072 x 1024 158 / 157, x 3840 x 1280 222 / 232. Weight gradients (a_mn) lose
+  // a few per cent. Requesting the SwiGLU operands a step ahead spills at eight warps (1068 -> 1240, 12 launches).
   const bool heavy = epi == EPI_SWIGLU_BOTH || epi == EPI_SWIGLU_BWD || epi == EPI_GATE_RESID;
   const bool ew8 = (heavy && K <= 2048) || (epi == EPI_STORE && K <= 1024);
   if (a_mn) return b_mn ? launch_gemm2<1, 1, 4>(ta, tb, p, stream) : launch_gemm2<1, 0, 4>(ta, tb, p, stream);

@@ -153,7 +153,8 @@ def _chunk_shapes(rows: int, D: int, HD: int, heads: int, F: int, tpn: int = 1):
     ``tpn``: ranks whose rows a tensor-parallel MLP gathers."""
     bf = torch.bfloat16
     return {"h": ((rows, D), bf), "qkv": ((rows, 3 * HD), bf), "o": ((rows, HD), bf),
-            "lse": ((rows * heads,), torch.float32), "x1": ((rows, D), bf), "h2": ((rows, D), bf), "act": ((rows * tpn, F), bf)}
+            "lse": ((rows * heads,), torch.float32), "x1": ((rows, D), bf), "h2": ((rows, D), bf),
+            "act": ((rows * tpn, F), bf)}
 
 
 def _grad_shapes(rows: int, D: int, HD: int, heads: int, F: int, tpn: int = 1):
@@ -477,8 +478,8 @@ def _pool_alloc(peer_fn, gradient: bool = False):
 
 
 class FusedBlock(torch.autograd.Function):
-    """Autograd wrapper: saves the block input and, with ``meta.keep``, the block's internals; weight gradients go to ``param.main_grad`` (fp32) when the
-    engine provides one, otherwise they are returned to autograd."""
+    """Autograd wrapper: saves the block input and, with ``meta.keep``, the block's internals; weight gradients go to
+    ``param.main_grad`` (fp32) when the engine provides one, otherwise they are returned to autograd."""
 
     @staticmethod
     def forward(ctx, x, mod, meta, wn1, wqkv, wo, wn2, w1, w2, regroup=None, out_alloc=None):

@@ -133,7 +133,8 @@ def gemv_bwd_ok(W: torch.Tensor, dW: torch.Tensor) -> bool:
     """Whether :func:`gemv_bwd` takes these operands: whole vectors of four along K, an fp32 gradient, and no more rows of
     W than the grid covers in its second dimension."""
     return (W.shape[1] % 4 == 0 and W.is_contiguous() and dW.is_contiguous() and dW.data_ptr() % 16 == 0
-            and dW.dtype == torch.float32 and W.shape[0] <= 65535 * 16 and W.data_ptr() % (4 * W.element_size()) == 0 and W.dtype in (torch.bfloat16, torch.float32))
+            and dW.dtype == torch.float32 and W.shape[0] <= 65535 * 16 and W.data_ptr() % (4 * W.element_size()) == 0
+            and W.dtype in (torch.bfloat16, torch.float32))
 
 
 def noise_embedding(t: torch.Tensor, dim: int, max_period: float, dtype: torch.dtype) -> torch.Tensor:

@@ -70,8 +70,8 @@ def _rows(T, C, ld=None, off=0, step=1):
 
 
 @pytest.mark.parametrize("d", [16, 32, 96])
-@pytest.mark.parametrize("qkv_kw,out_kw", [({}, {}), (dict(off=1), {}), ({}, dict(off=4)), (dict(pad=4), {}), ({}, dict(pad=2)),
-                                           ({}, dict(step=2))])
+@pytest.mark.parametrize("qkv_kw,out_kw", [({}, {}), (dict(off=1), {}), ({}, dict(off=4)), (dict(pad=4), {}),
+                                           ({}, dict(pad=2)), ({}, dict(step=2))])
 def test_narrow_heads_reach_the_kernels_in_whole_vectors_or_as_padded_copies(recorder, d, qkv_kw, out_kw):
     """Every form that the padded copies took is still taken, and only whole vectors go straight to the kernels."""
     n_win, N, H = 2, 5, 2
@@ -94,8 +94,8 @@ def test_narrow_heads_reach_the_kernels_in_whole_vectors_or_as_padded_copies(rec
 def test_push_entries_take_the_kernels_own_head_widths_only(d):
     peers = (V * 2)(BASE, BASE)
     H, ld, hd = 2, 6 * d, 2 * d
-    rc = L.lib().aeris_attn_fwd_push(V(BASE), ld, H, V(BASE), hd, V(BASE), 2, 16, d, ctypes.c_float(1.0), peers, 2, 8, 2 * hd,
-                                     0, V(0), V(0))
+    rc = L.lib().aeris_attn_fwd_push(V(BASE), ld, H, V(BASE), hd, V(BASE), 2, 16, d, ctypes.c_float(1.0), peers, 2, 8,
+                                     2 * hd, 0, V(0), V(0))
     assert rc == -1
     rc = L.lib().aeris_attn_bwd_push(V(BASE), ld, H, V(BASE), V(BASE), hd, V(BASE), V(BASE), 2, 16, d, ctypes.c_float(1.0),
                                      peers, 2, 8, 6 * hd, 2 * hd, 0, V(0), V(0))

@@ -27,7 +27,8 @@ def _gemv_case(N, K, B, silu_in):
     from aeris_gb_b200.ops import diffusion as DF
     torch.manual_seed(N + K + B)
     for wt, xt in ((torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32), (torch.bfloat16, torch.float32)):
-        W, b, x = torch.randn(N, K, device=DEV).to(wt), torch.randn(N, device=DEV).to(wt), torch.randn(B, K, device=DEV).to(xt)
+        W, b = torch.randn(N, K, device=DEV).to(wt), torch.randn(N, device=DEV).to(wt)
+        x = torch.randn(B, K, device=DEV).to(xt)
         dy = torch.randn(B, N, device=DEV)
         Wd, bd, xd = (v.double().requires_grad_(True) for v in (W, b, x))
         ref = (torch.nn.functional.silu(xd) if silu_in else xd) @ Wd.t() + bd

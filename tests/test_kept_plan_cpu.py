@@ -37,7 +37,8 @@ def test_chunks_below_half_a_gigabyte_are_merged(dim, heads, mlp, L, chunk, n_wi
 
 @pytest.mark.parametrize("win,dim,mlp", [((1, 1), 128, 256), ((1, 2), 128, 256), ((2, 2), 64, 64)])
 def test_merged_chunks_stay_within_the_attention_grid(win, dim, mlp):
-    """Windows of a few tokens on the full 720 x 1440 image: half a gigabyte of them is more than the grid's 65,535 layers."""
+    """Windows of a few tokens on the full 720 x 1440 image: half a gigabyte of them is more than the grid's 65,535
+    layers."""
     L = win[0] * win[1]
     n_win = 720 * 1440 // L
     meta = fused.BlockMeta(n_win, L, 2, dim // 2, E.MODE_MOD_THEN_NORM, 1e-6, 64)
@@ -48,7 +49,8 @@ def test_merged_chunks_stay_within_the_attention_grid(win, dim, mlp):
 
 @pytest.mark.parametrize("trains", ["x", "mod", "weight", None])
 def test_internals_are_kept_only_for_a_backward_pass_that_can_come(trains, monkeypatch):
-    """A frozen block on inputs without gradients, called without no_grad: nothing is kept. Any differentiable input: all is."""
+    """A frozen block on inputs without gradients, called without no_grad: nothing is kept. Any differentiable input: all
+    is."""
     seen = []
 
     def forward(x, mod, meta, *weights, out=None, gather=None, kept=None):
@@ -94,8 +96,9 @@ class _Memory:
         stat = lambda n: {"all": {"current": n}}
         monkeypatch.setattr(fused, "_WS", fused.Workspace())
         monkeypatch.setattr(torch.cuda, "get_device_properties", lambda d: SimpleNamespace(total_memory=180 * GB))
-        monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict", lambda d: {
-            "reserved_bytes": stat(7 * GB + cached), "allocated_bytes": stat(7 * GB), "inactive_split_bytes": stat(fragments)})
+        stats = {"reserved_bytes": stat(7 * GB + cached), "allocated_bytes": stat(7 * GB),
+                 "inactive_split_bytes": stat(fragments)}
+        monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict", lambda d: stats)
 
         def ask(device):
             self.asked += 1
@@ -206,7 +209,8 @@ def _slices(tiles, kb, units=74, most=64, want=0):
     (192, 1013, 74, 64, 4, 5), (108, 1013, 74, 64, 4, 4),   # nothing merged: the cheapest number
     (9, 1, 74, 64, 4, 1), (9, 3, 74, 64, 400, 3), (9, 4, 74, 64, 0, 4)])
 def test_slices_of_a_weight_gradient(tiles, kb, units, most, want, got):
-    """No empty slice, at least four where there are four k-blocks, and for merged chunks towards the slices of the shorter sums."""
+    """No empty slice, at least four where there are four k-blocks, and for merged chunks towards the slices of the shorter
+    sums."""
     assert _slices(tiles, kb, units, most, want) == got
     assert (got - 1) * -(-kb // got) < kb
 

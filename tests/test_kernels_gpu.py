@@ -217,7 +217,8 @@ def test_gemm_epilogue_warps(K):
         assert rel_err(apart, want) < TOL and torch.equal(apart, in_place)
 
 
-@pytest.mark.parametrize("M,N,K", [(256, 256, 3600), (384, 640, 12150), (512, 1536, 200), (1536, 768, 28800), (256, 256, 40)])
+@pytest.mark.parametrize("M,N,K", [(256, 256, 3600), (384, 640, 12150), (512, 1536, 200), (1536, 768, 28800),
+                                   (256, 256, 40)])
 @pytest.mark.parametrize("k_splits", [0, 1, 3])
 def test_gemm_accumulate_splits(M, N, K, k_splits):
     """Weight-gradient products with the kernel's own split of the token dimension, none, and a fixed one: fp32 sums in

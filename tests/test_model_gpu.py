@@ -17,7 +17,8 @@ def _small_cfg(after_mod_norm=True, head_dim=64, window=(16, 16)):
 
 
 def _recompute_in_chunks(cfg, recompute):
-    """Every block recomputes in chunks of three of its eight windows (two full ones and a remainder), or keeps its internals."""
+    """Every block recomputes in chunks of three of its eight windows (two full ones and a remainder), or keeps its
+    internals."""
     if recompute:
         cfg.recompute, cfg.min_chunk_bytes = True, 0
     return cfg

@@ -1,5 +1,5 @@
-"""Routes of the noise-level embedding: the kernel works on plain values only, everything that carries a derivative or a hidden
-dimension takes the formulas."""
+"""Routes of the noise-level embedding: the kernel works on plain values only, everything that carries a derivative or a
+hidden dimension takes the formulas."""
 import pytest
 import torch
 from torch.autograd import forward_ad
