@@ -272,10 +272,12 @@ int num_sms() {
 // 28800: 94.8 -> 87.0 us, 1536 x 4096 x 64800: 699 -> 662 us.
 // Slices also bound the error: the tensor core truncates at every addition, so that of a sum grows with its slice (9e-10 of
 // the result per row: 1.4e-7 for slices of 128 rows, 8e-6 for 7,200). `want` slices are what the caller's sums had when they
-// came in more and shorter products; of the numbers from there down, the first that costs at most a quarter more than the
-// cheapest is taken. Error of the separate products, of one with the cheapest slices and of this rule: 512 x 128 x 2048 for
-// 4 x 512 rows 1.4e-7 / 4.7e-7 / 1.4e-7 (67, 18 and 18 us); 1024 x 4096 x 9000 for 16 windows of 225 at a time 8.2e-7 /
-// 2.3e-6 / 7.9e-7 (124, 66 and 101 us); 4096 x 512 x 27540 for 4 windows of 135 2.8e-7 / 3.2e-6 / 1.2e-6 (1028, 93, 119 us).
+// came in more and shorter products; of the numbers from there down, the first that costs no more than the cheapest is
+// taken. Error of the separate products, of one with the cheapest slices and of this rule: 512 x 128 x 2048 for 4 x 512 rows
+// 1.4e-7 / 4.7e-7 / 1.4e-7 (67, 18 and 18 us); 256 x 256 x 18432 for 72 x 256 rows 3.1e-7 / 4.9e-7 / 2.8e-7 (872, 15 and 17).
+// Where finer slices have a price they are not taken: 1024 x 4096 x 9000 for 3 x 3600 rows stays at 2.3e-6 against 8.2e-7;
+// letting them cost a quarter more gave 7.9e-7 for 101 us instead of 66, and training steps with such chunks lost 3-9 %, for
+// an error that the bf16 operands (2^-9) hide.
 int choose_k_splits(int tiles, int kb_total, int units, int most, int want) {
   auto cost = [&](int s) {
     const long long rounds = (static_cast<long long>(tiles) * s + units - 1) / units;
@@ -288,7 +290,7 @@ int choose_k_splits(int tiles, int kb_total, int units, int most, int want) {
   for (int per = want > 0 ? (kb_total + want - 1) / want : kb_total; per < kb_total; ++per) {
     const int s = (kb_total + per - 1) / per;
     if (s <= best) break;
-    if (4 * cost(s) <= 5 * cost(best)) return s;
+    if (cost(s) <= cost(best)) return s;
   }
   return best;
 }

@@ -33,7 +33,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
     raw product); EPI_ACC_F32 ``out += acc`` in fp32 (split-K allowed); EPI_STORE_F32 fp32 out;
     EPI_SWIGLU_BOTH = EPI_SWIGLU that also writes the raw ``[gate | up]`` product to ``aux [M, 2F]``;
     ``k_splits``: slices of the reduction dimension (EPI_ACC_F32 only); 0 lets the kernel choose, -n as well but towards n
-    slices, for sums that should be no less accurate than those of n shorter products.
+    slices, as far as they cost nothing, for sums that used to come as n shorter ones.
     EPI_SWIGLU_BWD: the product is d(act) ``[M, F]``, ``resid`` holds ``u = [gate | up]`` and ``out`` receives d(u).
     """
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16

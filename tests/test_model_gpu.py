@@ -228,11 +228,12 @@ def test_samples_in_one_launch_equal_samples_one_by_one(dim, heads):
 
 
 @pytest.mark.parametrize("L,n_win,chunk,dims", [(64, 32, 8, (512, 128)), (64, 32, 8, (128, 256)), (900, 8, 4, (1024, 256)),
-                                                (225, 40, 16, (2304, 384)), (225, 40, 16, (1024, 1024))])
+                                                (64, 288, 4, (256, 256))])
 def test_weight_gradients_of_merged_chunks_are_as_accurate_as_those_of_the_chunks(L, n_win, chunk, dims):
-    """One product over all windows, with the slices that ``block_backward`` asks for, against one per ``chunk_windows``
-    with four slices each: the error against 64 bits may not grow by more than the price rule leaves, a slice of half as
-    many rows again (the tensor core's truncation is proportional to the rows of a slice; fp32 atomics add 2^-24 each)."""
+    """Small weights, where finer slices cost nothing: one product over all windows, with the slices that
+    ``block_backward`` asks for, against one per ``chunk_windows`` with four slices each. The error against 64 bits is the
+    tensor core's truncation, proportional to the rows of a slice, and may not grow beyond the rounding of the fp32
+    additions between slices (2^-24 each)."""
     from aeris_gb_b200.ops import gemm as G
     torch.manual_seed(L)
     a, b = (torch.randn(n_win * L, k, device="cuda").bfloat16() for k in dims)
@@ -246,4 +247,4 @@ def test_weight_gradients_of_merged_chunks_are_as_accurate_as_those_of_the_chunk
             G.gemm(a[sl], b[sl], a_t=True, b_t=True, out=out, epi=G.EPI_ACC_F32,
                    k_splits=4 if step == chunk else -4 * -(-n // chunk))
         err.append(((out.double() - ref).norm() / ref.norm()).item())
-    assert err[1] < 1.5 * err[0] + 2.0 ** -24, err
+    assert err[1] < err[0] + 2.0 ** -24, err
