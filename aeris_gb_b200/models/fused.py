@@ -180,29 +180,29 @@ def plan_kept_blocks(meta: BlockMeta, batch: int, D: int, F: int, n_blocks: int,
     take at most half of the memory that is free now (the allocator's unused cache included) and not needed by the step
     in any case: block inputs, stream gradients, and the workspaces that are not there yet.
 
-    One exception saves a question to the driver (0.1 to 1.6 ms each, measured): where the allocator's cache by itself covers
-    the internals of all blocks and the rest of the step, as it does from the second step on, all blocks keep theirs.
-    Fragments (unused parts of blocks in use) count there only for needs below 1/256 of the device, whose tensors of a few
-    MB fit into them; elsewhere they do not count as free at all."""
+    One exception saves a question to the driver (0.1 to 2 ms each, measured; a fifth of a small step): where the allocator's
+    cache by itself covers the internals of all blocks and the rest of the step, as it does from the second step on, all
+    blocks keep theirs. Fragments (unused parts of blocks in use) count there, because an earlier step's tensors lie in
+    them; where they turn out too small for a block's internals, :class:`FusedBlock` lets that block recompute. Elsewhere
+    they do not count as free."""
     HD = meta.heads * meta.head_dim
     T = batch * meta.n_win_per_sample * meta.L
     per_block = kept_bytes(T, D, HD, meta.heads, F)
     step = chunk_step(meta, D, F)
     rows = step * meta.L
     fwd_rows = max(nw for _, _, nw, _ in _forward_spans(meta, batch, step, D, F, False)) * meta.L
-    # a shifted layer holds its source beside its input
-    streams = (n_blocks + 4) * T * D * 2
+    # at the peak: every block's input, the gradient of the last one's output, and what a shifted layer hands back
+    stream = T * D * 2
     grads = _WS.missing(_grad_shapes(rows, D, HD, meta.heads, F), device)
     stats = torch.cuda.memory_stats_as_nested_dict(device)
     reserved, allocated, fragments = (stats.get(k, {}).get("all", {}).get("current", 0)
                                       for k in ("reserved_bytes", "allocated_bytes", "inactive_split_bytes"))
-    cached, whole = max(0, reserved - allocated), max(0, reserved - allocated - fragments)
-    need = n_blocks * per_block
-    small = need <= torch.cuda.get_device_properties(device).total_memory // 256
-    if need + streams + grads <= (cached if small else whole):
+    if n_blocks * per_block + (n_blocks + 2) * stream + grads <= reserved - allocated:
         return n_blocks
-    base = streams + grads + _WS.missing(_chunk_shapes(fwd_rows, D, HD, meta.heads, F), device)
-    return n_kept(n_blocks, per_block, base, whole + torch.cuda.mem_get_info(device)[0])
+    # a margin of two streams, and the workspaces of the blocks that recompute
+    base = (n_blocks + 4) * stream + grads + _WS.missing(_chunk_shapes(fwd_rows, D, HD, meta.heads, F), device)
+    free = max(0, reserved - allocated - fragments) + torch.cuda.mem_get_info(device)[0]
+    return n_kept(n_blocks, per_block, base, free)
 
 
 MIN_CHUNK_BYTES = 512 << 20
@@ -494,7 +494,10 @@ class FusedBlock(torch.autograd.Function):
         if meta.keep and any(ctx.needs_input_grad):        # a frozen block has no backward pass to keep anything for
             shapes = _kept_shapes(regroup[0].numel() if regroup is not None else x.shape[0], x.shape[1],
                                   meta.heads * meta.head_dim, meta.heads, w2.shape[1])
-            kept = {k: torch.empty(shape, dtype=dt, device=x.device) for k, (shape, dt) in shapes.items()}
+            try:
+                kept = {k: torch.empty(shape, dtype=dt, device=x.device) for k, (shape, dt) in shapes.items()}
+            except torch.OutOfMemoryError:
+                kept = None            # free in sum but not in pieces of this size: recompute instead
         if regroup is not None:
             table_fwd, _, peer_fn = regroup
             peers = peer_fn(x, "fwd") if peer_fn is not None else [x.data_ptr()]

@@ -1,6 +1,5 @@
 """How many blocks keep their internals for the backward pass, and how small a chunk may get."""
 import math
-from types import SimpleNamespace
 
 import pytest
 import torch
@@ -95,7 +94,6 @@ class _Memory:
         self.asked = 0
         stat = lambda n: {"all": {"current": n}}
         monkeypatch.setattr(fused, "_WS", fused.Workspace())
-        monkeypatch.setattr(torch.cuda, "get_device_properties", lambda d: SimpleNamespace(total_memory=180 * GB))
         stats = {"reserved_bytes": stat(7 * GB + cached), "allocated_bytes": stat(7 * GB),
                  "inactive_split_bytes": stat(fragments)}
         monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict", lambda d: stats)
@@ -110,7 +108,8 @@ class _Memory:
 META = fused.BlockMeta(32, 900, 12, 64, E.MODE_MOD_THEN_NORM, 1e-6, 64)
 D, FF, BLOCKS, ROWS = 768, 2048, 6, 2 * 32 * 900
 NEED = BLOCKS * fused.kept_bytes(ROWS, D, D, 12, FF)
-STREAMS = (BLOCKS + 4) * ROWS * D * 2
+STREAM = ROWS * D * 2
+PEAK = (BLOCKS + 2) * STREAM
 # chunks of one sample: bytes per row of the gradient workspaces and of the recompute's, and the weight-sized ones
 GRADS = 32 * 900 * ((2 * FF + 2 * D + 4 * D) * 2 + 12 * 4) + D * (FF + D) * 6
 CHUNK = 32 * 900 * ((3 * D + 4 * D + FF) * 2 + 12 * 4)
@@ -121,22 +120,25 @@ def _plan(meta=META, batch=2, d=D, f=FF, blocks=BLOCKS):
 
 
 def test_a_cache_that_covers_the_whole_step_needs_no_question(monkeypatch):
-    mem = _Memory(monkeypatch, driver=0, cached=NEED + STREAMS + GRADS)
-    assert _plan() == BLOCKS and mem.asked == 0
+    """Whole or in fragments, in which the earlier step's tensors lay."""
+    for fragments in (0, NEED):
+        mem = _Memory(monkeypatch, driver=0, cached=NEED + PEAK + GRADS, fragments=fragments)
+        assert _plan() == BLOCKS and mem.asked == 0
 
 
-@pytest.mark.parametrize("short", [0, 1])
-def test_a_cache_that_covers_only_what_is_kept_leaves_room_for_the_step(short, monkeypatch):
-    """The internals alone fit the cache and the driver has nothing left: what the step needs besides comes first."""
-    cached = NEED if short else NEED + STREAMS + GRADS - 1
+@pytest.mark.parametrize("cached", [NEED, NEED + BLOCKS * STREAM, NEED + PEAK + GRADS - 1])
+def test_a_cache_that_covers_only_what_is_kept_leaves_room_for_the_step(cached, monkeypatch):
+    """The internals alone, or with the block inputs, fit the cache and the driver has nothing left: what the step needs
+    besides comes first."""
     mem = _Memory(monkeypatch, driver=0, cached=cached)
-    want = (cached - STREAMS - GRADS - CHUNK) // 2 // (NEED // BLOCKS)
+    base = PEAK + 2 * STREAM + GRADS + CHUNK
+    want = max(0, (cached - base) // 2 // (NEED // BLOCKS))
     assert _plan() == want < BLOCKS and mem.asked == 1
-    assert want * (NEED // BLOCKS) + STREAMS + GRADS + CHUNK <= cached
+    assert want == 0 or want * (NEED // BLOCKS) + base <= cached
 
 
 def test_workspaces_that_are_there_are_not_counted_again(monkeypatch):
-    mem = _Memory(monkeypatch, driver=0, cached=NEED + STREAMS)
+    mem = _Memory(monkeypatch, driver=0, cached=NEED + PEAK)
     assert _plan() < BLOCKS and mem.asked == 1
     for name, (shape, dtype) in fused._grad_shapes(32 * 900, D, D, 12, FF).items():
         fused._WS._buf[name] = torch.empty(shape, dtype=dtype, device="meta").flatten()
@@ -144,13 +146,13 @@ def test_workspaces_that_are_there_are_not_counted_again(monkeypatch):
     assert _plan() == BLOCKS and mem.asked == 1
 
 
-def test_fragments_are_not_free_memory(monkeypatch):
-    mem = _Memory(monkeypatch, driver=0, cached=NEED + STREAMS + GRADS, fragments=NEED)
+def test_fragments_are_not_free_memory_where_the_driver_is_asked(monkeypatch):
+    mem = _Memory(monkeypatch, driver=0, cached=NEED + PEAK + GRADS - 1, fragments=NEED)
     assert _plan() == 0 and mem.asked == 1
 
 
 def test_the_driver_s_memory_is_shared_half_and_half(monkeypatch):
-    free = STREAMS + GRADS + CHUNK + NEED                 # half of the rest: three of six blocks
+    free = PEAK + 2 * STREAM + GRADS + CHUNK + NEED       # half of the rest: three of six blocks
     mem = _Memory(monkeypatch, driver=free)
     assert _plan() == BLOCKS // 2 and mem.asked == 1
     _Memory(monkeypatch, driver=free + NEED)
@@ -158,15 +160,29 @@ def test_the_driver_s_memory_is_shared_half_and_half(monkeypatch):
 
 
 def test_a_small_model_on_a_full_device_recomputes(monkeypatch):
-    """Needs below 1/256 of the device are not exempt: with 100 MB left in all, a step that needs more keeps nothing. With
-    the fragments of an earlier step in the cache (its tensors of a few MB fit them) the driver is not asked."""
+    """Needs below 1/256 of the device are not exempt: with 100 MB left in all, a step that needs more keeps nothing."""
     meta = fused.BlockMeta(8, 900, 4, 64, E.MODE_MOD_THEN_NORM, 1e-6, 4)
-    need = 2 * fused.kept_bytes(7200, 256, 256, 4, 512)
-    assert need < 180 * GB // 256
+    assert 2 * fused.kept_bytes(7200, 256, 256, 4, 512) < 180 * GB // 256
     mem = _Memory(monkeypatch, driver=100 * MB)
     assert _plan(meta, 1, 256, 512, 2) == 0 and mem.asked == 1
-    mem = _Memory(monkeypatch, driver=0, cached=need + 200 * MB, fragments=need)
-    assert _plan(meta, 1, 256, 512, 2) == 2 and mem.asked == 0
+
+
+def test_internals_that_find_no_room_are_recomputed(monkeypatch):
+    """The plan counts bytes; where the pieces are too small after all, the block runs without kept internals."""
+    seen = []
+    monkeypatch.setattr(fused, "block_forward", lambda x, *a, kept=None, **k: seen.append(kept) or torch.zeros_like(x))
+    monkeypatch.setattr(fused, "_kept_shapes", lambda *a: {k: ((1 << 60,), torch.uint8) for k in fused.KEPT})
+    real = torch.empty
+
+    def empty(shape, **kw):
+        if shape == (1 << 60,):
+            raise torch.OutOfMemoryError("no room")
+        return real(shape, **kw)
+    monkeypatch.setattr(torch, "empty", empty)
+    meta = fused.BlockMeta(2, 4, 2, 8, E.MODE_MOD_THEN_NORM, 1e-6, 64, keep=True)
+    ws = [torch.zeros(s, dtype=torch.bfloat16) for s in ((16,), (48, 16), (16, 16), (16,), (64, 16), (16, 32))]
+    y = fused.FusedBlock.apply(torch.zeros(8, 16, requires_grad=True), torch.zeros(1, 96), meta, *ws)
+    assert seen == [None] and len(y.grad_fn.saved_tensors) == 8
 
 
 def test_the_plan_counts_the_workspaces_that_the_passes_use(monkeypatch):
