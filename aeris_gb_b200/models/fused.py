@@ -218,6 +218,12 @@ def chunk_step(meta: BlockMeta, D: int, F: int) -> int:
     return min(max(meta.chunk_windows, floor), meta.n_win_per_sample, MAX_CHUNK_WINDOWS)
 
 
+def wanted_slices(meta: BlockMeta, nw: int) -> int:
+    """Slices that the weight gradients of a chunk of ``nw`` windows should keep of the shorter sums: four per chunk of
+    ``chunk_windows``, which may be 0 where the floor of :func:`chunk_step` alone sets the chunk."""
+    return 4 * -(-nw // max(1, min(meta.chunk_windows, meta.n_win_per_sample)))
+
+
 def _forward_spans(meta: BlockMeta, B: int, step: int, D: int, F: int, kept: bool) -> list[tuple[int, int, int, int]]:
     """What one pass over the forward kernels covers: (first sample, first window, windows, samples). Samples that are one
     chunk each run in one launch per kernel (their modulation vectors are picked by row), when their internals are kept
@@ -395,8 +401,6 @@ def block_backward(x: torch.Tensor, mod: torch.Tensor, dy: torch.Tensor, meta: B
     if dx is None:
         dx = torch.empty_like(x)
     mod = mod.contiguous()
-    # four slices per chunk of `chunk_windows`: what a merged chunk's weight gradients should keep of the shorter sums
-    slices = lambda nw: -4 * -(-nw // min(meta.chunk_windows, meta.n_win_per_sample))
     for b in range(B):
         sh1, sc1, g1, sh2, sc2, g2 = [mod[b, i * D:(i + 1) * D] for i in range(6)]
         dsh1, dsc1, dg1, dsh2, dsc2, dg2 = [dmod[b, i * D:(i + 1) * D] for i in range(6)]
@@ -406,7 +410,7 @@ def block_backward(x: torch.Tensor, mod: torch.Tensor, dy: torch.Tensor, meta: B
             r0 = b * rows_per_sample + w0 * meta.L
             n = nw * meta.L
             xc, dyc = x[r0:r0 + n], dy[r0:r0 + n]
-            ksplit_tok = slices(nw)
+            ksplit_tok = -wanted_slices(meta, nw)
             h1, qkv, o, x1, h2, act, lse = _chunk_views(kept, r0, n, meta.heads) if kept is not None else \
                 _chunk_views(chunk_bufs, 0, n, meta.heads)
             lse_c = lse.view(nw, meta.heads, meta.L)

@@ -231,6 +231,14 @@ def test_slices_of_a_weight_gradient(tiles, kb, units, most, want, got):
     assert (got - 1) * -(-kb // got) < kb
 
 
+@pytest.mark.parametrize("chunk,n_win,nw,want", [(8, 32, 32, 16), (64, 32, 32, 4), (5, 32, 32, 28), (0, 32, 32, 128)])
+def test_slices_that_a_merged_chunk_asks_for(chunk, n_win, nw, want):
+    """Four per chunk that ``chunk_windows`` names; 0 leaves the chunk to the floor in bytes and must not divide."""
+    meta = fused.BlockMeta(n_win, 64, 4, 32, E.MODE_MOD_THEN_NORM, 1e-6, chunk)
+    assert fused.chunk_step(meta, 128, 256) == nw
+    assert fused.wanted_slices(meta, nw) == want
+
+
 def test_every_wanted_number_is_met_or_has_a_price():
     cost = lambda t, kb, s: -(-t * s // 74) * (-(-kb // s) + 10)
     for tiles in (1, 7, 33, 74, 75, 500):
