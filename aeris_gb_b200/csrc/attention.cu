@@ -764,8 +764,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                   kk > 0);
 #pragma unroll
         for (int kk = 0; kk < 4 * DCH; ++kk)
-          umma_ss(tS + 64, d1 + ((kk >> 2) * 16384 + (kk & 3) * 32) / 16, d3 + ((kk >> 2) * 8192 + (kk & 3) * 32) / 16, idesc,
-                  kk > 0);
+          umma_ss(tS + 64, d1 + ((kk >> 2) * 16384 + (kk & 3) * 32) / 16, d3 + ((kk >> 2) * 8192 + (kk & 3) * 32) / 16,
+                  idesc, kk > 0);
         tc_commit(&sp_full[s_w]);
         if (last) tc_commit(&q_empty[b]);
         if (++s_w == NWG) s_w = 0;
@@ -1111,8 +1111,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                   kk > 0);
 #pragma unroll
         for (int kk = 0; kk < 4 * DCH; ++kk)
-          umma_ss(tS + 64, d1 + ((kk >> 2) * 16384 + (kk & 3) * 32) / 16, d3 + ((kk >> 2) * 8192 + (kk & 3) * 32) / 16, idesc,
-                  kk > 0);
+          umma_ss(tS + 64, d1 + ((kk >> 2) * 16384 + (kk & 3) * 32) / 16, d3 + ((kk >> 2) * 8192 + (kk & 3) * 32) / 16,
+                  idesc, kk > 0);
         tc_commit(&sp_full[s_w]);
         if (last) tc_commit(&kv_empty[b]);
         if (++s_w == NWG) s_w = 0;

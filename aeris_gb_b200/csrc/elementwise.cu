@@ -143,11 +143,11 @@ constexpr int FWD_RPI = 4;  // rows per iteration of one CTA: one block-wide red
 // Serves rows wider than 5120 columns (up to 1024 threads, register cap 64).
 __global__ void __launch_bounds__(1024, 1)
 modnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __restrict__ gidx,
-                                   PeerPtrs peers, __nv_bfloat16* __restrict__ x_out,
-                                   const float* __restrict__ scale, const float* __restrict__ shift,
-                                   const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ h, int rows,
-                                   int D, int mode, float eps, const float* __restrict__ wf,
-                                   __nv_bfloat16* __restrict__ h_lo) {
+                   PeerPtrs peers, __nv_bfloat16* __restrict__ x_out,
+                   const float* __restrict__ scale, const float* __restrict__ shift,
+                   const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ h, int rows,
+                   int D, int mode, float eps, const float* __restrict__ wf,
+                   __nv_bfloat16* __restrict__ h_lo) {
   __shared__ float red[2 * FWD_RPI * 32];
   const int c0 = threadIdx.x * 8;
   const bool active = c0 < D;

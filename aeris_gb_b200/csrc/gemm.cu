@@ -266,18 +266,18 @@ int num_sms() {
 // tokens): the number of slices, from four to `most`, that minimises rounds x (k-blocks per slice + fixed cost of a slice),
 // a round being one slice per unit (CTA or CTA pair). Constant four left the last round of many shapes nearly empty and
 // small weights (dim 256: 4 slices on 74 pairs) on a handful of SMs. The fixed cost, filling the ring and adding the tile's
-// fp32 values to memory, is taken as 10 k-blocks of 64. More than four slices have at least eight k-blocks on average (the last
-// one holds what is left). The one-CTA kernel, whose products are narrow, stays at four.
+// fp32 values to memory, is taken as 10 k-blocks of 64. More than four slices have at least eight k-blocks on average (the
+// last one holds what is left). The one-CTA kernel, whose products are narrow, stays at four.
 // Four slices and now, held for 0.6 s: 512 x 512 x 28800: 43.0 -> 22.1 us (1965 MHz); under the power cap 768 x 2048 x
 // 28800: 94.8 -> 87.0 us, 1536 x 4096 x 64800: 699 -> 662 us.
-// Slices also bound the error: the tensor core truncates at every addition, so that of a sum grows with its slice (9e-10 of
-// the result per row: 1.4e-7 for slices of 128 rows, 8e-6 for 7,200). `want` slices are what the caller's sums had when they
-// came in more and shorter products; of the numbers from there down, the first that costs no more than the cheapest is
-// taken. Error of the separate products, of one with the cheapest slices and of this rule: 512 x 128 x 2048 for 4 x 512 rows
-// 1.4e-7 / 4.7e-7 / 1.4e-7 (67, 18 and 18 us); 256 x 256 x 18432 for 72 x 256 rows 3.1e-7 / 4.9e-7 / 2.8e-7 (872, 15 and 17).
-// Where finer slices have a price they are not taken: 1024 x 4096 x 9000 for 3 x 3600 rows stays at 2.3e-6 against 8.2e-7;
-// letting them cost a quarter more gave 7.9e-7 for 101 us instead of 66, and training steps with such chunks lost 3-9 %, for
-// an error that the bf16 operands (2^-9) hide.
+// Slices also bound the error: the tensor core truncates at every addition, so that of a sum grows with its slice
+// (9e-10 of the result per row: 1.4e-7 for slices of 128 rows, 8e-6 for 7,200). `want` slices are what the caller's
+// sums had when they came in more and shorter products; of the numbers from there down, the first that costs no more
+// than the cheapest is taken. Error of the separate products, of one with the cheapest slices and of this rule: 512 x
+// 128 x 2048 for 4 x 512 rows 1.4e-7 / 4.7e-7 / 1.4e-7 (67, 18 and 18 us); 256 x 256 x 18432 for 72 x 256 rows 3.1e-7 /
+// 4.9e-7 / 2.8e-7 (872, 15 and 17). Where finer slices have a price they are not taken: 1024 x 4096 x 9000 for 3 x 3600
+// rows stays at 2.3e-6 against 8.2e-7; letting them cost a quarter more gave 7.9e-7 for 101 us instead of 66, and
+// training steps with such chunks lost 3-9 %, for an error that the bf16 operands (2^-9) hide.
 int choose_k_splits(int tiles, int kb_total, int units, int most, int want) {
   auto cost = [&](int s) {
     const long long rounds = (static_cast<long long>(tiles) * s + units - 1) / units;
@@ -371,13 +371,13 @@ extern "C" int aeris_gemm_bf16(const void* A, const void* B, void* C, int M, int
 #undef AERIS_DISPATCH
 }
 
-// C[M, 128] (fp32) = lo(y) W_hi^T + hi(y) W_lo^T + hi(y) W_hi^T in one pass: the output head at fp32-level accuracy. `y`
-// holds the hi parts in its first rows and the lo parts from row `lo_row` on ([*, D] bf16), `w` the rows
-// [W_hi | W_lo | W_hi] ([128, 3 D] bf16). D must be a multiple of 64. The small terms come first: the tensor core truncates at every addition, so
-// with the large sum already in the accumulator they would cost its last bits (error against 64 bits at D = 1536 8.8e-6
-// in the order hi, lo, hi; 4.7e-6 in this one and for three separate products). Three products wrote the 128 fp32 columns
-// once and added to them twice, a read and a write each, for little arithmetic (65536 rows of 1536, norm included:
-// 312 -> 227 us, 12 launches).
+// C[M, 128] (fp32) = lo(y) W_hi^T + hi(y) W_lo^T + hi(y) W_hi^T in one pass: the output head at fp32-level accuracy.
+// `y` holds the hi parts in its first rows and the lo parts from row `lo_row` on ([*, D] bf16), `w` the rows [W_hi |
+// W_lo | W_hi] ([128, 3 D] bf16). D must be a multiple of 64. The small terms come first: the tensor core truncates at
+// every addition, so with the large sum already in the accumulator they would cost its last bits (error against 64 bits
+// at D = 1536 8.8e-6 in the order hi, lo, hi; 4.7e-6 in this one and for three separate products). Three products wrote
+// the 128 fp32 columns once and added to them twice, a read and a write each, for little arithmetic (65536 rows of
+// 1536, norm included: 312 -> 227 us, 12 launches).
 extern "C" int aeris_gemm_split(const void* y, const void* w, float* C, int M, int D, int lo_row, int ldc, int* status,
                                 void* stream_) {
   if (M <= 0 || D <= 0 || D % BK || lo_row < M || ldc < 128 || ldc % 4) return -1;
