@@ -145,7 +145,8 @@ def _kept_shapes(T: int, D: int, HD: int, heads: int, F: int) -> dict[str, tuple
 
 
 def kept_bytes(T: int, D: int, HD: int, heads: int, F: int) -> int:
-    return sum(math.prod(shape) * dt.itemsize for shape, dt in _kept_shapes(T, D, HD, heads, F).values())
+    """Bytes of :func:`_kept_shapes`, in closed form: every pass over a block asks for them."""
+    return T * (2 * (3 * D + 4 * HD + 3 * F) + 4 * heads)
 
 
 def _chunk_shapes(rows: int, D: int, HD: int, heads: int, F: int, tpn: int = 1):
@@ -228,9 +229,9 @@ def _forward_spans(meta: BlockMeta, B: int, step: int, D: int, F: int, kept: boo
     """What one pass over the forward kernels covers: (first sample, first window, windows, samples). Samples that are one
     chunk each run in one launch per kernel (their modulation vectors are picked by row), when their internals are kept
     anyway or take less than the smallest chunk; the exchanges of the parallel paths work on one sample at a time."""
-    row = kept_bytes(1, D, meta.heads * meta.head_dim, meta.heads, F)
     if (B > 1 and step == meta.n_win_per_sample and meta.sp is None and meta.tp is None
-            and (kept or B * step * meta.L * row <= meta.chunk_floor) and B * step <= MAX_CHUNK_WINDOWS):
+            and (kept or kept_bytes(B * step * meta.L, D, meta.heads * meta.head_dim, meta.heads, F) <= meta.chunk_floor)
+            and B * step <= MAX_CHUNK_WINDOWS):
         return [(0, 0, B * step, B)]
     return [(b, w0, nw, 1) for b in range(B) for w0, nw in _chunks(meta, step)]
 

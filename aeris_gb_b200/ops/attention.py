@@ -18,7 +18,10 @@ def _kernel_dim(d: int) -> int:
 
 def _whole_vectors(t: torch.Tensor | None) -> bool:
     """Rows that start on 16-byte boundaries and have no gaps: what the kernels' 16-byte accesses need."""
-    return t is None or (t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0)
+    if t is None:
+        return True
+    stride = t.stride()
+    return stride[1] == 1 and stride[0] % 8 == 0 and t.data_ptr() % 16 == 0
 
 
 def _padded_dim(d: int, *tensors: torch.Tensor | None) -> int:

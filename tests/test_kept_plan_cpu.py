@@ -19,6 +19,8 @@ def test_a_block_keeps_every_recomputed_internal():
     per_row = 3 * 1536 * 2 + 4 * 1536 * 2 + 3 * 4096 * 2 + 24 * 4        # h1, x1, h2 | qkv, o | act, u | lse
     assert fused.kept_bytes(1000, 1536, 1536, 24, 4096) == 1000 * per_row
     assert set(fused._kept_shapes(8, 16, 16, 2, 32)) == set(fused.KEPT)
+    shapes = fused._kept_shapes(1000, 1536, 1280, 20, 4104).values()
+    assert fused.kept_bytes(1000, 1536, 1280, 20, 4104) == sum(math.prod(sh) * dt.itemsize for sh, dt in shapes)
 
 
 @pytest.mark.parametrize("dim,heads,mlp,L,chunk,n_win,want", [
