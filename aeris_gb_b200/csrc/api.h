@@ -17,6 +17,12 @@ int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M, int N, in
                          int rows_per_gate, void* aux, int ld_aux, int swiglu_f, int k_splits, int* status,
                          void* stream);
 
+// The one of the two that is the faster for the shape (see gemm2.cu). bn: tile width of the one-CTA kernel (0: from N);
+// allow_2cta = 0: never the other.
+int aeris_gemm_auto(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int a_mn,
+                    int b_mn, int epi, const void* resid, int ldr, const float* gate, int rows_per_gate, void* aux,
+                    int ld_aux, int swiglu_f, int k_splits, int bn, int allow_2cta, int* status, void* stream);
+
 int aeris_attn_fwd(const void* q, int ldq, int q_col0, const void* k, int ldk, int k_col0, const void* v, int ldv,
                    int v_col0, void* o, int ldo, float* lse, int n_win, int N, int H, int head_dim, float scale,
                    int* status, void* stream);
@@ -117,6 +123,35 @@ int aeris_pack_head_weights(const float* W, void* out, int C, int rows, int D, v
 // Slices that k_splits <= 0 stands for: `tiles` output tiles over `units` CTAs or CTA pairs (see gemm.cu).
 int aeris_choose_k_splits(int tiles, int kb_total, int units, int most, int want);
 int aeris_gemm_split(const void* y, const void* w, float* C, int M, int D, int lo_row, int ldc, int* status, void* stream);
+
+// One transformer block on one GPU (csrc/block.cu; mirrored in models/block.py). Every matrix is row-major without gaps.
+typedef struct AerisBlock {
+  int D, F, heads, head_dim, L, mode;
+  int n_win, batch;                 // windows of one sample, samples
+  int step, merged;                 // windows per chunk; merged: all samples are one chunk (forward)
+  int slice_windows;                // weight gradients: slices of a quarter of that many windows' rows at most, if free
+  int kept, two_cta, n_peers;       // kept: the internals are full-size buffers, not workspaces of one chunk
+  float eps, scale;
+  long long mod_vec, mod_sample;    // element strides of `mod`: between the six vectors, between samples
+  const float* mod;                 // shift1, scale1, gate1, shift2, scale2, gate2
+  const void *wn1, *wqkv, *wo, *wn2, *w1, *w2;
+  const float *rope_cos, *rope_sin; // null: no rotary embedding
+  void *x, *y;                      // block input (with `table`: receives the gathered rows) and output
+  const unsigned* table;            // null, or gather codes of the rows of x
+  const void* const* peers;
+  void *h1, *qkv, *o, *lse, *x1, *h2, *act, *u;
+  int* status;
+  void* stream;
+} AerisBlock;
+typedef struct AerisBlockGrad {
+  const void* dy;
+  void *dx, *du, *dh, *dx1, *d_o, *dqkv, *w2g, *wog;
+  float *delta, *G2, *Go, *dmod;    // dmod: [batch, 6 D], overwritten
+  float *n1, *to_qkv, *wo, *n2, *w1, *w2;   // weight gradients, added to
+} AerisBlockGrad;
+// Both return the number of kernels launched, or a negative code: that of the launch that failed less 1000 times its place.
+int aeris_block_forward(const AerisBlock* b);
+int aeris_block_backward(const AerisBlock* b, const AerisBlockGrad* g);
 
 #ifdef __cplusplus
 }

@@ -400,6 +400,21 @@ extern "C" int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M
   return ew8 ? launch_gemm2<0, 0, 8>(ta, tb, p, stream) : launch_gemm2<0, 0, 4>(ta, tb, p, stream);
 }
 
+// Which kernel takes a product. A last tile with 128 valid columns costs as much as a full one: 6 % at 2048 columns, far
+// less than the two-CTA kernel gains there (28800 x 13696 x 5120: 4.96 -> 3.38 ms), but 12150 x 1152 x 384 takes 43 us
+// instead of 38; the SwiGLU forward pairs gate and up columns of whole tiles.
+extern "C" int aeris_gemm_auto(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
+                               int a_mn, int b_mn, int epi, const void* resid, int ldr, const float* gate,
+                               int rows_per_gate, void* aux, int ld_aux, int swiglu_f, int k_splits, int bn,
+                               int allow_2cta, int* status, void* stream) {
+  const bool swiglu_fwd = (epi == EPI_SWIGLU || epi == EPI_SWIGLU_BOTH);
+  if (allow_2cta && (N % G2_BN == 0 || (N % (G2_BN / 2) == 0 && N >= 2048 && !swiglu_fwd)))
+    return aeris_gemm_bf16_2cta(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, resid, ldr, gate, rows_per_gate, aux,
+                                ld_aux, swiglu_f, k_splits, status, stream);
+  return aeris_gemm_bf16(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, resid, ldr, gate, rows_per_gate, aux, ld_aux,
+                         swiglu_f, k_splits, bn, status, stream);
+}
+
 // QKV (or dO) projection whose epilogue performs the Ulysses head<->sequence exchange: C is not written locally;
 // every head's tile goes straight into the symmetric buffer of the rank that owns the head (`peers[owner]`).
 // A: [M, K] row-major tokens (M = windows * n_local), B: [N, K] weights (or stored [K, N] with b_mn).

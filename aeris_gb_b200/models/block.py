@@ -1,0 +1,93 @@
+"""One native call per pass over a transformer block: the launches of :func:`.fused.block_forward` and
+:func:`.fused.block_backward` on one GPU, issued by ``csrc/block.cu`` instead of one by one from Python."""
+from __future__ import annotations
+
+import ctypes
+import math
+
+import torch
+
+from ..ops import elementwise as E
+from ..ops import gemm as G
+from ..ops import lib as _l
+
+_P, _I, _F, _LL = ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_longlong
+
+
+class BlockArgs(ctypes.Structure):
+    """Mirror of ``AerisBlock`` (csrc/api.h)."""
+    _fields_ = ([(n, _I) for n in ("D", "F", "heads", "head_dim", "L", "mode", "n_win", "batch", "step", "merged",
+                                   "slice_windows", "kept", "two_cta", "n_peers")]
+                + [("eps", _F), ("scale", _F), ("mod_vec", _LL), ("mod_sample", _LL)]
+                + [(n, _P) for n in ("mod", "wn1", "wqkv", "wo", "wn2", "w1", "w2", "rope_cos", "rope_sin", "x", "y", "table",
+                                     "peers", "h1", "qkv", "o", "lse", "x1", "h2", "act", "u", "status", "stream")])
+
+
+class BlockGradArgs(ctypes.Structure):
+    """Mirror of ``AerisBlockGrad`` (csrc/api.h)."""
+    _fields_ = [(n, _P) for n in ("dy", "dx", "du", "dh", "dx1", "d_o", "dqkv", "w2g", "wog", "delta", "G2", "Go", "dmod",
+                                  "n1", "to_qkv", "wo", "n2", "w1", "w2")]
+
+
+def _plain(t: torch.Tensor, dtype: torch.dtype) -> bool:
+    return t.dtype == dtype and t.is_cuda and t.is_contiguous()
+
+
+def takes(meta, x: torch.Tensor, mod: torch.Tensor, weights, grads=()) -> bool:
+    """Whether the native call takes this block: bf16 operands without gaps, fp32 modulation and gradients, heads of whole
+    16-byte vectors, none of the exchanges of the parallel paths. Everything else is issued (or refused) call by call."""
+    d = meta.head_dim
+    return (meta.sp is None and meta.tp is None and (d in (64, 128) or (d % 8 == 0 and 0 < d < 128))
+            and mod.dtype == torch.float32 and mod.is_cuda
+            and _plain(x, torch.bfloat16) and all(_plain(w, torch.bfloat16) for w in weights)
+            and all(_plain(g, torch.float32) for g in grads))
+
+
+def _args(meta, x, mod, B, D, F, step, weights, bufs: dict[str, int], kept: bool, stream: int) -> tuple[BlockArgs, tuple]:
+    """The arguments both directions share, and what has to live until the call returns. ``bufs``: addresses of internals."""
+    wn1, wqkv, wo, wn2, w1, w2 = weights
+    cos = sin = None
+    if meta.rope is not None:
+        cos, sin = (t.float().contiguous() for t in meta.rope)
+        assert cos.shape == (meta.L, meta.head_dim // 2)
+    a = BlockArgs(D=D, F=F, heads=meta.heads, head_dim=meta.head_dim, L=meta.L, mode=meta.mode, n_win=meta.n_win_per_sample,
+                  batch=B, step=step, slice_windows=max(1, min(meta.chunk_windows, meta.n_win_per_sample)), kept=kept,
+                  two_cta=G.TWO_CTA_DEFAULT, eps=meta.eps, scale=1.0 / math.sqrt(meta.head_dim), mod_vec=D, mod_sample=6 * D,
+                  mod=mod.data_ptr(), wn1=wn1.data_ptr(), wqkv=wqkv.data_ptr(), wo=wo.data_ptr(), wn2=wn2.data_ptr(),
+                  w1=w1.data_ptr(), w2=w2.data_ptr(), x=x.data_ptr(), status=_l.status_word().data_ptr(), stream=stream,
+                  **bufs)
+    if cos is not None:
+        a.rope_cos, a.rope_sin = cos.data_ptr(), sin.data_ptr()
+    return a, (mod, cos, sin)
+
+
+def _issued(rc: int, what: str) -> None:
+    _l.check(min(rc, 0), what, kernels=max(rc, 0))
+
+
+def forward(meta, x, mod, weights, y, step: int, merged: bool, bufs: dict[str, int], kept: bool, gather=None) -> None:
+    """``mod`` [B, 6 D] fp32. ``gather``: see :func:`.fused.block_forward`."""
+    B, D, F = mod.shape[0], x.shape[1], weights[5].shape[1]
+    if merged and B > 1:              # every vector of all samples in a row
+        mod, vec, sample = mod.view(B, 6, D).transpose(0, 1).contiguous(), B * D, D
+    else:
+        mod, vec, sample = mod.contiguous(), D, 6 * D
+    a, alive = _args(meta, x, mod, B, D, F, step, weights, bufs, kept, _l.raw_stream())
+    a.mod_vec, a.mod_sample, a.merged, a.y = vec, sample, merged, y.data_ptr()
+    if gather is not None:
+        table, peers, src = gather
+        if E._CHECKED:
+            E.set_gather_bounds(src.shape[0])
+        arr = E._peer_array(peers)
+        a.table, a.peers, a.n_peers = table.data_ptr(), ctypes.addressof(arr), len(peers)
+    _issued(_l.lib().aeris_block_forward(ctypes.byref(a)), "aeris_block_forward")
+
+
+def backward(meta, x, mod, dy, weights, step: int, bufs: dict[str, int], kept: bool, work: dict[str, int], dx, dmod,
+             grads: dict[str, torch.Tensor]) -> None:
+    """``work``: addresses of the gradient workspaces; ``dmod`` [B, 6 D] fp32 is overwritten."""
+    mod = mod.contiguous()
+    a, alive = _args(meta, x, mod, mod.shape[0], x.shape[1], weights[5].shape[1], step, weights, bufs, kept, _l.raw_stream())
+    g = BlockGradArgs(dy=dy.data_ptr(), dx=dx.data_ptr(), dmod=dmod.data_ptr(), **work,
+                      **{k: t.data_ptr() for k, t in grads.items()})
+    _issued(_l.lib().aeris_block_backward(ctypes.byref(a), ctypes.byref(g)), "aeris_block_backward")

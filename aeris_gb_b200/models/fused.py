@@ -20,6 +20,7 @@ import torch
 from ..ops import attention as A
 from ..ops import elementwise as E
 from ..ops import gemm as G
+from . import block as NB
 
 
 @dataclass
@@ -338,7 +339,12 @@ def block_forward(x: torch.Tensor, mod: torch.Tensor, meta: BlockMeta, wn1, wqkv
         tpn = meta.tp.tp if meta.tp is not None else 1   # gathered rows x local features: the same element count
         shapes = _chunk_shapes(cmax, D, HD, meta.heads, F, tpn)
         chunk_bufs = {k: ws.get(k, *sh, dev) for k, sh in shapes.items() if k != "h2"}
-        chunk_bufs["h1"] = chunk_bufs["h2"] = chunk_bufs["h"]
+        chunk_bufs["h1"] = chunk_bufs["h2"] = chunk_bufs.pop("h")
+    weights = (wn1, wqkv, wo, wn2, w1, w2)
+    if y.is_contiguous() and NB.takes(meta, x, mod, weights):
+        NB.forward(meta, x, mod, weights, y, step, spans[0][3] > 1,
+                   {k: t.data_ptr() for k, t in (kept or chunk_bufs).items()}, kept is not None, gather)
+        return y
     mods = mod.reshape(B, 6, D).transpose(0, 1).contiguous()           # [6, B, D]: every vector of all samples in a row
     for b, w0, nw, nb in spans:
         sh1, sc1, g1, sh2, sc2, g2 = (mods[:, b] if nb == 1 else mods[:, b:b + nb]).unbind(0)
@@ -393,9 +399,17 @@ def block_backward(x: torch.Tensor, mod: torch.Tensor, dy: torch.Tensor, meta: B
     tpn = tp.tp if tp is not None else 1
     if kept is None:
         chunk_bufs = {k: ws.get(k, *sh, dev) for k, sh in _chunk_shapes(cmax, D, HD, meta.heads, F, tpn).items()}
-        chunk_bufs["h1"], act_b = chunk_bufs["h"], chunk_bufs["act"]
-    du_b, dh, dx1, d_o, dqkv, delta, w2g, wog, G2, Go = \
-        (ws.get(k, *sh, dev) for k, sh in _grad_shapes(cmax, D, HD, meta.heads, F, tpn).items())
+        chunk_bufs["h1"], act_b = chunk_bufs.pop("h"), chunk_bufs["act"]
+    work = {k: ws.get(k, *sh, dev) for k, sh in _grad_shapes(cmax, D, HD, meta.heads, F, tpn).items()}
+    weights = (wn1, wqkv, wo, wn2, w1, w2)
+    if NB.takes(meta, x, mod, (*weights, dy, *(() if dx is None else (dx,))), grads.values()):
+        dx = torch.empty_like(x) if dx is None else dx
+        dmod = torch.empty((B, 6 * D), dtype=f32, device=dev)
+        addr = {"du" if k == "u" else k: t.data_ptr() for k, t in work.items()}
+        NB.backward(meta, x, mod, dy, weights, step, {k: t.data_ptr() for k, t in (kept or chunk_bufs).items()},
+                    kept is not None, addr, dx, dmod, grads)
+        return dx, dmod
+    du_b, dh, dx1, d_o, dqkv, delta, w2g, wog, G2, Go = work.values()
     G2.zero_()          # dy^T act (ungated w2 gradient of one sample)
     Go.zero_()          # dx1^T o
     dmod = torch.zeros((B, 6 * D), dtype=f32, device=dev)

@@ -7,8 +7,8 @@ import torch
 
 from . import lib as _l
 
-# The two-CTA (cta_group::2, 256 x 256 tile per SM pair) kernel is used for every product that it takes (see gemm())
-# unless AERIS_GEMM_2CTA=0.
+# The two-CTA (cta_group::2, 256 x 256 tile per SM pair) kernel is used where it is the faster (aeris_gemm_auto in
+# csrc/gemm2.cu) unless AERIS_GEMM_2CTA=0.
 TWO_CTA_DEFAULT = os.environ.get("AERIS_GEMM_2CTA", "1") != "0"
 
 EPI_STORE, EPI_SWIGLU, EPI_GATE_RESID, EPI_ACC_F32, EPI_STORE_F32, EPI_SWIGLU_BOTH, EPI_SWIGLU_BWD = range(7)
@@ -63,23 +63,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
     assert out.shape == (M, n_out) or epi == EPI_SWIGLU_BWD
     if two_cta is None:
         two_cta = TWO_CTA_DEFAULT and bn == 0
-    # a last tile with 128 valid columns costs as much as a full one: 6 % at 2048 columns, far less than the two-CTA kernel
-    # gains there (28800 x 13696 x 5120: 4.96 -> 3.38 ms), but 12150 x 1152 x 384 takes 43 us instead of 38; the SwiGLU
-    # forward pairs gate and up columns of whole tiles
-    if two_cta and (N % 256 == 0 or (N % 128 == 0 and N >= 2048 and epi not in (EPI_SWIGLU, EPI_SWIGLU_BOTH))):
-        rc = _l.lib().aeris_gemm_bf16_2cta(
-            _l.ptr(a), _l.ptr(b), _l.ptr(out), M, N, K, _ld(a), _ld(b), _ld(out), int(a_t), int(b_t), epi,
-            _l.ptr(resid), _ld(resid) if resid is not None else 0, _l.ptr(gate), rows_per_gate,
-            _l.ptr(aux), _ld(aux) if aux is not None else 0, swiglu_f, k_splits, _l.ptr(_l.status_word()),
-            _l.stream_ptr())
-        _l.check(rc, "aeris_gemm_bf16_2cta")
-        return out
-    if bn == 0:
-        bn = 256 if N % 256 == 0 else 128
-    rc = _l.lib().aeris_gemm_bf16(
+    rc = _l.lib().aeris_gemm_auto(
         _l.ptr(a), _l.ptr(b), _l.ptr(out), M, N, K, _ld(a), _ld(b), _ld(out), int(a_t), int(b_t), epi,
         _l.ptr(resid), _ld(resid) if resid is not None else 0, _l.ptr(gate), rows_per_gate,
-        _l.ptr(aux), _ld(aux) if aux is not None else 0, swiglu_f, k_splits, bn, _l.ptr(_l.status_word()),
+        _l.ptr(aux), _ld(aux) if aux is not None else 0, swiglu_f, k_splits, bn, int(two_cta), _l.ptr(_l.status_word()),
         _l.stream_ptr())
-    _l.check(rc, "aeris_gemm_bf16")
+    _l.check(rc, "aeris_gemm")
     return out
