@@ -530,6 +530,12 @@ static int launch_attn_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const C
 }
 
 
+}  // namespace aeris
+
+#include "attention_fwd_pair.cuh"
+
+namespace aeris {
+
 // -------------------------------------------------------------------------------------------------------- backward
 // Two kernels, neither needs atomics:
 //   attn_bwd_dq : items of one 128-row Q tile, K/V streamed in 64-row tiles.  S = Q K^T, dP = dO V^T,
@@ -1404,6 +1410,21 @@ static int attn_fwd_impl(const void* q, int ldq, int q_col0, const void* k, int 
   int r;
   auto at = [](const void* base, int col) -> const void* { return reinterpret_cast<const __nv_bfloat16*>(base) + col; };
   if ((r = make_tmap_heads_bf16(&tq, at(q, q_col0), head_dim, H, N, n_win, ldq, TILE))) return r;
+  // Two query tiles at a time where there are two; its masked columns need a positive scale. Three or five tiles of which the
+  // last is not full leave its second chain idle for a third or a fifth of the time: 64-wide heads are faster without then
+  // (one tile at a time / two, 24 x 64: 200 x 257 tokens 0.306 / 0.330 ms, 100 x 352 0.196 / 0.203, 64 x 520 0.264 / 0.275,
+  // 64 x 576 0.281 / 0.288; 100 x 384 0.208 / 0.198, 64 x 640 0.321 / 0.300, 32 x 1030 0.415 / 0.389), 128-wide ones are not
+  // (12 x 128: 200 x 257 0.256 / 0.237, 100 x 320 0.146 / 0.129, 64 x 576 0.218 / 0.201).
+  const int q_tiles = (N + TILE - 1) / TILE, tail = N % TILE;
+  const bool idle_chain = head_dim <= 64 && (q_tiles == 3 || q_tiles == 5) && tail > 0 && tail <= 96;
+  if (q_tiles > 1 && !idle_chain && scale > 0.f && g_fwd_mode == 0 && g_fwd_poly == -1) {
+    if ((r = make_tmap_heads_bf16(&tk, at(k, k_col0), head_dim, H, N, n_win, ldk, KVP))) return r;
+    if ((r = make_tmap_heads_bf16(&tv, at(v, v_col0), head_dim, H, N, n_win, ldv, KVP))) return r;
+    CUtensorMap to = tq;      // without a local output nothing is stored through it
+    if (o && (r = make_tmap_heads_bf16(&to, o, head_dim, H, N, n_win, ldo, TILE))) return r;
+    return head_dim > 64 ? launch_attn_fwd_pair<2>(tq, tk, tv, to, p, stream)
+                         : launch_attn_fwd_pair<1>(tq, tk, tv, to, p, stream);
+  }
   if ((r = make_tmap_heads_bf16(&tk, at(k, k_col0), head_dim, H, N, n_win, ldk, KVT))) return r;
   if ((r = make_tmap_heads_bf16(&tv, at(v, v_col0), head_dim, H, N, n_win, ldv, KVT))) return r;
   if (head_dim > 64) {
