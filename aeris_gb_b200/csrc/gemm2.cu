@@ -117,7 +117,12 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
 
   // AG: the last operand stage is the copier's ring (two 16 KB bulk-copy buffers), with its barriers behind tmem_slot
   // (the reduce-scatter epilogue gives up the same stage: its fourth warp stages its rows there)
-  const int STAGES = (EW == 4 && (AG || p.epi == EPI_RS_PUSH)) ? LY::STAGES - 1 : LY::STAGES;
+  // and so do the epilogues on eight warps that request a second operand ahead. The gated residual gains from that while its
+  // tile's products are short (us without / with: 28800 x 768 x 768 47.5 / 40.5, x 512 x 512 57.2 / 49.5; 64800 x 1536 x 1536
+  // 283 / 282, 28800 x 768 x 2048 84 / 88: the ring's fifth stage is worth more).
+  const bool ahead = EW == 8 && p.staged_out;
+  const bool u_ahead = ahead && p.epi == EPI_SWIGLU_BWD, r_ahead = ahead && p.epi == EPI_GATE_RESID && !p.aux && p.K <= 1024;
+  const int STAGES = (u_ahead || r_ahead || (EW == 4 && (AG || p.epi == EPI_RS_PUSH))) ? LY::STAGES - 1 : LY::STAGES;
   [[maybe_unused]] uint8_t* ag_ring = smem + (LY::STAGES - 1) * G2_STAGE_BYTES;
   [[maybe_unused]] uint64_t* ag_bars = reinterpret_cast<uint64_t*>(smem + LY::STAGES * G2_STAGE_BYTES + 256);
 
@@ -272,6 +277,24 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     uint32_t acc_phase = 0;
     bool ok = true;
     const uint32_t leader_tempty0 = map_to_cta(smem_u32(&tempty_bar[0]), 0);
+    [[maybe_unused]] uint8_t* ubuf = smem + (LY::STAGES - 1) * G2_STAGE_BYTES + (warp - 2) * SWIGLU_U_BYTES;
+    // first step of the next tile from `tile` on that has columns for this warp (the last tile of a row may be half empty)
+    [[maybe_unused]] auto request_tile = [&](int tile) {
+      for (; tile < total_tiles; tile += n_clusters) {
+        int tm, tn;
+        tile_mn(tile, tm, tn);
+        const int c = part * (G2_BN / 2);
+        if (tn * G2_BN + c >= p.N) continue;
+        if (u_ahead)
+          swiglu_u_request(ubuf, p, tm * 2 * G2_BM + crank * G2_BM + q * 32, tn * G2_BN + c, lane);
+        else
+          resid_request(ubuf, p, tm * 2 * G2_BM + crank * G2_BM + q * 32, tn * G2_BN + c, lane);
+        break;
+      }
+    };
+    if constexpr (EW == 8) {
+      if (u_ahead || r_ahead) request_tile(cluster_id);
+    }
     for (int tile = cluster_id; tile < total_tiles && ok; tile += n_clusters) {
       const int split = tile / (m_tiles * n_tiles);
       const int mn = tile - split * (m_tiles * n_tiles);
@@ -285,7 +308,78 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       uint8_t* stg = smem + LY::PUSH_OFF + (part * 4 + q) * PUSH_STAGE_BYTES;
       if (p.epi == EPI_RS_PUSH)     // 8704-byte linear stages: three in the push area, the fourth in the freed operand stage
         stg = (q < 3) ? smem + LY::PUSH_OFF + q * RS_STAGE_BYTES : smem + (LY::STAGES - 1) * G2_STAGE_BYTES;
-      gemm_epilogue_row<G2_BN>(p, taddr, row, row < p.M, tn, kempty, stg, part, EW / 4);
+      bool done = false;
+      if constexpr (EW == 8) {
+        if (u_ahead) {
+          const bool row_ok = row < p.M;
+          __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(row) * p.ldc + tn * G2_BN;
+          const int c_hi = min((part + 1) * (G2_BN / 2), p.N - tn * G2_BN);
+#pragma unroll 1
+          for (int c = part * (G2_BN / 2); c < c_hi; c += 32) {
+            uint4 g4[4], u4[4];
+            swiglu_u_take(ubuf, lane, g4, u4);
+            if (c + 32 < c_hi)
+              swiglu_u_request(ubuf, p, row - lane, tn * G2_BN + c + 32, lane);
+            else
+              request_tile(tile + n_clusters);
+            uint32_t v[32], og[16], ou[16];
+            tmem_ld32(taddr + c, v);
+            tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t gw[4] = {g4[i].x, g4[i].y, g4[i].z, g4[i].w}, uw[4] = {u4[i].x, u4[i].y, u4[i].z, u4[i].w};
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                swiglu_bwd_pair(__uint_as_float(v[8 * i + 2 * j]), __uint_as_float(v[8 * i + 2 * j + 1]), gw[j], uw[j],
+                                og[4 * i + j], ou[4 * i + j]);
+            }
+            // 64 d(gate) columns and the matching 64 d(up) columns share one stage group
+            push_stage_put(stg, lane, (c & 32), og);
+            push_stage_put(stg, lane, 64 + (c & 32), ou);
+            if (c & 32)
+              push_stage_flush2(stg, lane, row_ok ? dst + (c - 32) : nullptr,
+                                row_ok ? dst + p.swiglu_f + (c - 32) : nullptr);
+          }
+          done = true;
+        } else if (r_ahead) {
+          const bool row_ok = row < p.M;
+          __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(row) * p.ldc + tn * G2_BN;
+          const float* gate = p.gate + static_cast<size_t>((row_ok ? row : 0) / p.rows_per_gate) * p.N + tn * G2_BN;
+          const int c_hi = min((part + 1) * (G2_BN / 2), p.N - tn * G2_BN);
+#pragma unroll 1
+          for (int c = part * (G2_BN / 2); c < c_hi; c += 64) {
+            uint4 x[8];
+            resid_take(ubuf, lane, x);
+            if (c + 64 < c_hi)
+              resid_request(ubuf, p, row - lane, tn * G2_BN + c + 64, lane);
+            else
+              request_tile(tile + n_clusters);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              uint32_t v[32], o[16];
+              tmem_ld32(taddr + c + 32 * h, v);
+              tmem_wait_ld();
+              const float4* gsrc = reinterpret_cast<const float4*>(gate + c + 32 * h);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const uint32_t rr[4] = {x[4 * h + i].x, x[4 * h + i].y, x[4 * h + i].z, x[4 * h + i].w};
+                const float4 ga = gsrc[2 * i], gb = gsrc[2 * i + 1];
+                const float gg[8] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  const float2 r2 = unpack_bf16x2(rr[j]);
+                  o[4 * i + j] = pack_bf16x2(fmaf(gg[2 * j], __uint_as_float(v[8 * i + 2 * j]), r2.x),
+                                             fmaf(gg[2 * j + 1], __uint_as_float(v[8 * i + 2 * j + 1]), r2.y));
+                }
+              }
+              push_stage_put(stg, lane, (c & 64) + 32 * h, o);
+            }
+            if (c & 64) push_stage_flush(stg, lane, row_ok ? dst + (c - 64) : nullptr);
+          }
+          done = true;
+        }
+      }
+      if (!done) gemm_epilogue_row<G2_BN>(p, taddr, row, row < p.M, tn, kempty, stg, part, EW / 4);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(leader_tempty0 + acc * 8);
@@ -294,6 +388,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     // the bulk copies of the reduce-scatter push have been performed before this thread leaves (the owners read
     // their slots after a rank barrier that follows this kernel in the stream)
     if (p.epi == EPI_RS_PUSH) rs_stage_drain();
+    if constexpr (EW == 8) asm volatile("cp.async.wait_all;" ::: "memory");     // after a time-out: copies nobody took
   }
 
   tc_fence_before();
@@ -392,7 +487,8 @@ extern "C" int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M
   // SwiGLU with the raw columns 28800 x 4096 x 768 220 / 191, x 8192 x 1536 615 / 611, x 10752 x 2048 999 / 1035, x 12288 x
   // 2304 1270 / 1309. One line at 2048 for the three: the SwiGLU backward would gain above it, the raw columns lose below.
   // Plain store 28800 x 2304 x 768 104 / 98, x 3072 x 1024 158 / 157, x 3840 x 1280 222 / 232. Weight gradients (a_mn) lose
-  // a few per cent. Requesting the SwiGLU operands a step ahead spills at eight warps (1068 -> 1240, 12 launches).
+  // a few per cent. Since then the SwiGLU backward and the gated residual on eight warps request their second operand ahead
+  // (registers for that spilled; see swiglu_u_request).
   const bool heavy = epi == EPI_SWIGLU_BOTH || epi == EPI_SWIGLU_BWD || epi == EPI_GATE_RESID;
   const bool ew8 = (heavy && K <= 2048) || (epi == EPI_STORE && K <= 1024);
   if (a_mn) return b_mn ? launch_gemm2<1, 1, 4>(ta, tb, p, stream) : launch_gemm2<1, 0, 4>(ta, tb, p, stream);

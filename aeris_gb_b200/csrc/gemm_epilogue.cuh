@@ -155,6 +155,64 @@ __device__ __forceinline__ void push_stage_flush_red(uint8_t* stage, int lane, f
   __syncwarp();
 }
 
+// SwiGLU backward of a pair of columns: d(gate) = d(act) * up * dsilu(gate), d(up) = d(act) * silu(gate).
+__device__ __forceinline__ void swiglu_bwd_pair(float d0, float d1, uint32_t gw, uint32_t uw, uint32_t& og, uint32_t& ou) {
+  const float2 g2 = unpack_bf16x2(gw), u2 = unpack_bf16x2(uw);
+  const float s0 = 1.f / (1.f + __expf(-g2.x)), s1 = 1.f / (1.f + __expf(-g2.y));
+  const float si0 = g2.x * s0, si1 = g2.y * s1;
+  og = pack_bf16x2(d0 * u2.x * (s0 + si0 * (1.f - s0)), d1 * u2.y * (s1 + si1 * (1.f - s1)));
+  ou = pack_bf16x2(d0 * si0, d1 * si1);
+}
+
+// Operand u = [gate | up] of the SwiGLU backward epilogue, requested one step (32 rows x 32 gate and 32 up columns, 4 KB per
+// warp) ahead as 64-byte row segments with asynchronous copies, across tiles: it does not depend on the products. Read by
+// the lane that owns the row; 16-byte chunks XOR-swizzled by row. Read by every lane from its own row when its turn came, 32
+// rows per instruction, the operand's latency was paid four times per tile: 28800 x 2048 x 768 211 -> 168 us, 28800 x 1536 x
+// 512 158 -> 119, 64800 x 4096 x 1536 1088 -> 918. What is left is the arithmetic (two exponentials and two divisions per
+// element) and shared memory, which operands and staging fill to the brim: 15,000 cycles a tile against 6,100 of products.
+constexpr int SWIGLU_U_BYTES = 4096;
+__device__ __forceinline__ void swiglu_u_request(uint8_t* buf, const GemmParams& p, int row0, int col, int lane) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = i * 4 + (lane >> 3), ch = lane & 7;
+    if (row0 + r < p.M) {
+      const int c = col + (ch & 3) * 8 + (ch < 4 ? 0 : p.swiglu_f);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(buf + r * 128 + ((ch ^ (r & 7)) << 4))),
+                   "l"(p.resid + static_cast<size_t>(row0 + r) * p.ldr + c)
+                   : "memory");
+    }
+  }
+}
+__device__ __forceinline__ void swiglu_u_take(const uint8_t* buf, int lane, uint4 (&g)[4], uint4 (&u)[4]) {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    g[i] = *reinterpret_cast<const uint4*>(buf + lane * 128 + ((i ^ (lane & 7)) << 4));
+    u[i] = *reinterpret_cast<const uint4*>(buf + lane * 128 + (((i + 4) ^ (lane & 7)) << 4));
+  }
+  __syncwarp();       // the buffer may be filled again
+}
+
+// The same for the residual of the gated epilogue: 32 rows x 64 columns per step, 128-byte row segments.
+__device__ __forceinline__ void resid_request(uint8_t* buf, const GemmParams& p, int row0, int col, int lane) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = i * 4 + (lane >> 3), ch = lane & 7;
+    if (row0 + r < p.M)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(buf + r * 128 + ((ch ^ (r & 7)) << 4))),
+                   "l"(p.resid + static_cast<size_t>(row0 + r) * p.ldr + col + ch * 8)
+                   : "memory");
+  }
+}
+__device__ __forceinline__ void resid_take(const uint8_t* buf, int lane, uint4 (&x)[8]) {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) x[i] = *reinterpret_cast<const uint4*>(buf + lane * 128 + ((i ^ (lane & 7)) << 4));
+  __syncwarp();       // the buffer may be filled again
+}
+
 // One thread = one accumulator row (TMEM lane) of a BN-column tile whose first accumulator column is `taddr`.
 // `row` is the global output row, `tn` the tile's index along N, `kempty` marks a split-K slice without work.
 // `stage`: this warp's PUSH_STAGE_BYTES of shared memory for the push epilogues, or null (direct stores).
@@ -247,14 +305,9 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
           const uint4 u4 = *reinterpret_cast<const uint4*>(usrc + p.swiglu_f + c + 8 * i);
           const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w}, uw[4] = {u4.x, u4.y, u4.z, u4.w};
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float2 g2 = unpack_bf16x2(gw[j]), u2 = unpack_bf16x2(uw[j]);
-            const float d0 = __uint_as_float(v[8 * i + 2 * j]), d1 = __uint_as_float(v[8 * i + 2 * j + 1]);
-            const float s0 = 1.f / (1.f + __expf(-g2.x)), s1 = 1.f / (1.f + __expf(-g2.y));
-            const float si0 = g2.x * s0, si1 = g2.y * s1;
-            og[4 * i + j] = pack_bf16x2(d0 * u2.x * (s0 + si0 * (1.f - s0)), d1 * u2.y * (s1 + si1 * (1.f - s1)));
-            ou[4 * i + j] = pack_bf16x2(d0 * si0, d1 * si1);
-          }
+          for (int j = 0; j < 4; ++j)
+            swiglu_bwd_pair(__uint_as_float(v[8 * i + 2 * j]), __uint_as_float(v[8 * i + 2 * j + 1]), gw[j], uw[j],
+                            og[4 * i + j], ou[4 * i + j]);
         }
         if (stage != nullptr && p.staged_out) {
           // 64 d(gate) columns and the matching 64 d(up) columns share one stage group
