@@ -69,6 +69,10 @@ int aeris_rope_qk(void* qkv, const float* cos_t, const float* sin_t, long long r
                   void* stream);
 int aeris_gate_grad_finalize(float* G, const void* W, const float* g, float* dW, float* dg, int R, int C,
                              void* stream);
+int aeris_gate_prepare(const void* W2, const float* g2, void* W2g, float* G2, int C2, const void* Wo, const float* go,
+                       void* Wog, float* Go, int Co, int R, float* zero, int n_zero, void* stream);
+int aeris_gate_finalize_pair(float* G2, const void* W2, const float* g2, float* dW2, float* dg2, int C2, float* Go,
+                             const void* Wo, const float* go, float* dWo, float* dgo, int Co, int R, void* stream);
 int aeris_sumsq(const float* x, long long n, double* out, void* stream);
 int aeris_adamw(float* master, float* grad, float* m, float* v, void* wbf16, float* ema, const double* norm_sq,
                 long long n, float lr, float beta1, float beta2, float eps, float weight_decay, int step,
@@ -113,9 +117,14 @@ int aeris_affine_channels(float* out, const float* in, const float* a, const flo
                           int C, void* stream);
 int aeris_gemv_bias_act(const void* W, int flags, const void* bias, const void* x, float* y, int N, int K, int B, int act,
                         int silu_in, void* stream);
-// Gradients of the above without `act`; added to dW, db (may be null) and dx (may be null).
+int aeris_modulation_mlp(const void* W1, int flags1, const void* b1, const void* x, float* y1, int N1, int K, const void* W2,
+                         int flags2, const void* b2, float* y2, int N2, int B, void* stream);
+// Gradients of aeris_gemv_bias_act without `act`; added to dW, db (may be null) and dx (may be null).
 int aeris_gemv_bwd(const void* W, int flags, const void* x, const float* dy, float* dW, float* db, float* dx, int N, int K,
                    int B, int silu_in, void* stream);
+int aeris_modulation_mlp_bwd(const void* W1, int flags1, const void* x, float* dW1, float* db1, float* dx, int N1, int K,
+                             const void* W2, int flags2, const float* y1, const float* dy, float* dW2, float* db2,
+                             float* dy1, int N2, int B, void* stream);
 int aeris_noise_embedding(const float* t, void* out, int out_bf16, int B, int dim, double max_period, void* stream);
 int aeris_pack_embed_weights(const float* W, const float* b, void* out, int D, int Cin, int KP, void* stream);
 int aeris_fold_embed_grad(const float* G, float* dW, float* db, int D, int Cin, int KP, void* stream);

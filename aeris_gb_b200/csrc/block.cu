@@ -3,7 +3,6 @@
 // A block is 7 launches forward and about 20 backward per chunk and sample. Issued one by one from Python each costs the
 // host 10-20 us (argument objects, views, checks), which is longer than most of them run on small models; here a launch
 // costs what the driver takes for it.
-#include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "api.h"
@@ -47,8 +46,6 @@ struct Gemm {
   }
 };
 
-// First half of a chunk: h1 = modulated norm of x, q|k|v, attention, x1 = x + g1 * (o wo^T). `table`: x is gathered on the
-// way (see aeris_modnorm_fwd).
 struct Vectors {
   const float *shift1, *scale1, *gate1, *shift2, *scale2, *gate2;
 };
@@ -80,22 +77,25 @@ bool modnorm(const AerisBlock& b, Run& run, int where, const bf16* x, const uint
 }
 
 bool rope(const AerisBlock& b, Run& run, int where, bf16* qkv, int rows, int inverse) {
-  return !b.rope_cos || run(where, aeris_rope_qk(qkv, b.rope_cos, b.rope_sin, rows, b.L, b.heads, b.head_dim, inverse, b.stream));
+  return !b.rope_cos ||
+         run(where, aeris_rope_qk(qkv, b.rope_cos, b.rope_sin, rows, b.L, b.heads, b.head_dim, inverse, b.stream));
 }
 
-// x -> x1, and with `mlp` on to h2
+// First half of a chunk: h1 = modulated norm of x, q|k|v, attention, x1 = x + g1 * (o wo^T). `table`: x is gathered on the
+// way (see aeris_modnorm_fwd).
 bool attention_half(const AerisBlock& b, Run& run, const Chunk& c, const Vectors& v, bf16* x, const uint32_t* table, int nw,
                     int nb) {
   const Gemm gemm{b};
   const int n = nw * b.L, HD = b.heads * b.head_dim;
   return modnorm(b, run, 1, x, table, table ? x : nullptr, v.scale1, v.shift1, b.wn1, c.h1, nb, n) &&
-         run(2, gemm(c.h1, false, b.wqkv, false, c.qkv, n, 3 * HD, b.D, EPI_STORE, 3 * HD)) && rope(b, run, 3, c.qkv, n, 0) &&
+         run(2, gemm(c.h1, false, b.wqkv, false, c.qkv, n, 3 * HD, b.D, EPI_STORE, 3 * HD)) &&
+         rope(b, run, 3, c.qkv, n, 0) &&
          run(4, aeris_attn_fwd(c.qkv, 3 * HD, 0, c.qkv, 3 * HD, HD, c.qkv, 3 * HD, 2 * HD, c.o, HD, c.lse, nw, b.L, b.heads,
                                b.head_dim, b.scale, b.status, b.stream)) &&
          run(5, gemm(c.o, false, b.wo, false, c.x1, n, b.D, HD, EPI_GATE_RESID, b.D, x, b.D, v.gate1, n / nb));
 }
 
-// (shape of every chunk) windows [w0, w0 + step) of one sample
+// body(first row, windows) for every chunk of a sample, until one fails
 template <typename F>
 bool for_chunks(const AerisBlock& b, int sample, F&& body) {
   for (int w0 = 0; w0 < b.n_win; w0 += b.step) {
@@ -137,18 +137,12 @@ extern "C" int aeris_block_backward(const AerisBlock* pb, const AerisBlockGrad* 
   const AerisBlockGrad& g = *pg;
   const Gemm gemm{b};
   const int D = b.D, F = b.F, HD = b.heads * b.head_dim;
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(b.stream);
   Run run;
-  // dy^T act and dx1^T o, the ungated gradients of w2 and wo for one sample: the finalising kernel leaves zeros behind
-  if (cudaMemsetAsync(g.G2, 0, sizeof(float) * D * F, stream) != cudaSuccess ||
-      cudaMemsetAsync(g.Go, 0, sizeof(float) * D * HD, stream) != cudaSuccess ||
-      cudaMemsetAsync(g.dmod, 0, sizeof(float) * 6 * D * b.batch, stream) != cudaSuccess)
-    return -1;
   for (int s = 0; s < b.batch; ++s) {
     const Vectors v = vectors(b, s);
     float* dm = g.dmod + static_cast<long long>(s) * 6 * D;      // shift1, scale1, gate1, shift2, scale2, gate2
-    if (!run(10, aeris_scale_rows(b.w2, v.gate2, g.w2g, D, F, b.stream)) ||
-        !run(11, aeris_scale_rows(b.wo, v.gate1, g.wog, D, HD, b.stream)))
+    // G2 = dy^T act and Go = dx1^T o are the ungated gradients of w2 and wo for one sample
+    if (!run(10, aeris_gate_prepare(b.w2, v.gate2, g.w2g, g.G2, F, b.wo, v.gate1, g.wog, g.Go, HD, D, dm, 6 * D, b.stream)))
       break;
     const bool ok = for_chunks(b, s, [&](long long r0, int nw) {
       const Chunk c = chunk(b, r0);
@@ -159,10 +153,12 @@ extern "C" int aeris_block_backward(const AerisBlock* pb, const AerisBlockGrad* 
       if (!b.kept &&
           !(attention_half(b, run, c, v, x, nullptr, nw, 1) &&
             modnorm(b, run, 6, c.x1, nullptr, nullptr, v.scale2, v.shift2, b.wn2, c.h2, 1, n) &&
-            run(7, gemm(c.h2, false, b.w1, false, c.act, n, 2 * F, D, EPI_SWIGLU_BOTH, F, nullptr, 0, nullptr, 0, u, 2 * F))))
+            run(7, gemm(c.h2, false, b.w1, false, c.act, n, 2 * F, D, EPI_SWIGLU_BOTH, F, nullptr, 0, nullptr, 0, u,
+                        2 * F))))
         return false;
       auto wgrad = [&](int where, const void* dout, int M, const void* in, int N, float* G) {
-        return run(where, gemm(dout, true, in, true, G, M, N, n, EPI_ACC_F32, N, nullptr, 0, nullptr, 0, nullptr, 0, slices));
+        return run(where, gemm(dout, true, in, true, G, M, N, n, EPI_ACC_F32, N, nullptr, 0, nullptr, 0, nullptr, 0,
+                               slices));
       };
       // MLP half: y = x1 + g2 * (act w2^T). dact = (dy * g2) w2 never reaches memory: the epilogue turns it into du
       return wgrad(12, dy, D, c.act, F, g.G2) &&
@@ -182,9 +178,8 @@ extern "C" int aeris_block_backward(const AerisBlock* pb, const AerisBlockGrad* 
              run(23, aeris_modnorm_bwd(x, g.dh, g.dx1, v.scale1, v.shift1, b.wn1, dx, dm + D, dm, g.n1, n, D, b.mode, b.eps,
                                        nullptr, b.stream));
     });
-    // dW += g * G, dg = rowsum(W * G), G <- 0
-    if (!ok || !run(24, aeris_gate_grad_finalize(g.G2, b.w2, v.gate2, g.w2, dm + 5 * D, D, F, b.stream)) ||
-        !run(25, aeris_gate_grad_finalize(g.Go, b.wo, v.gate1, g.wo, dm + 2 * D, D, HD, b.stream)))
+    if (!ok || !run(24, aeris_gate_finalize_pair(g.G2, b.w2, v.gate2, g.w2, dm + 5 * D, F, g.Go, b.wo, v.gate1, g.wo,
+                                                 dm + 2 * D, HD, D, b.stream)))
       break;
   }
   return run.result();

@@ -302,6 +302,13 @@ extern "C" int aeris_gemv_bias_act(const void* W, int flags, const void* bias, c
   return launched();
 }
 
+// The modulation MLP: y1 = x W1^T + b1 [B, N1], y2 = silu(y1) W2^T + b2 [B, N2]. Flags as above, for each layer.
+extern "C" int aeris_modulation_mlp(const void* W1, int flags1, const void* b1, const void* x, float* y1, int N1, int K,
+                                    const void* W2, int flags2, const void* b2, float* y2, int N2, int B, void* stream) {
+  const int rc = aeris_gemv_bias_act(W1, flags1, b1, x, y1, N1, K, B, 0, 0, stream);
+  return rc ? rc : aeris_gemv_bias_act(W2, flags2, b2, y1, y2, N2, N1, B, 0, 1, stream);
+}
+
 // flags as above. K must be a multiple of 4; W, dW and dx aligned to four elements. dW, db and dx are added to.
 extern "C" int aeris_gemv_bwd(const void* W, int flags, const void* x, const float* dy, float* dW, float* db, float* dx,
                               int N, int K, int B, int silu_in, void* stream) {
@@ -328,6 +335,20 @@ extern "C" int aeris_gemv_bwd(const void* W, int flags, const void* x, const flo
 #undef AERIS_GEMV_MB
 #undef AERIS_GEMV
   return launched();
+}
+
+// Gradients of aeris_modulation_mlp, added to dW1, db1, dW2 and db2; dy1 [B, N1] (scratch) and dx [B, K] (may be null) are
+// overwritten.
+extern "C" int aeris_modulation_mlp_bwd(const void* W1, int flags1, const void* x, float* dW1, float* db1, float* dx, int N1,
+                                        int K, const void* W2, int flags2, const float* y1, const float* dy, float* dW2,
+                                        float* db2, float* dy1, int N2, int B, void* stream) {
+  if (N1 <= 0 || K <= 0 || B <= 0) return -1;
+  const cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (cudaMemsetAsync(dy1, 0, sizeof(float) * B * N1, st) != cudaSuccess ||
+      (dx && cudaMemsetAsync(dx, 0, sizeof(float) * B * K, st) != cudaSuccess))
+    return -20;
+  const int rc = aeris_gemv_bwd(W2, flags2, y1, dy, dW2, db2, dy1, N2, N1, B, 1, stream);
+  return rc ? rc : aeris_gemv_bwd(W1, flags1, x, dy1, dW1, db1, dx, N1, K, B, 0, stream);
 }
 
 extern "C" int aeris_pack_embed_weights(const float* W, const float* b, void* out, int D, int Cin, int KP, void* stream) {

@@ -853,6 +853,56 @@ __global__ void gate_grad_finalize_kernel(float* __restrict__ G, const __nv_bflo
   if (threadIdx.x == 0) dg[r] += acc[0];
 }
 
+// Both gated matrices of a block (w2 and wo, blockIdx.y) in one launch each: what a backward pass needs before a sample's
+// products, Wg = g * W with G and the sample's modulation gradients zeroed, and what it does with them afterwards. At the
+// sizes where launches count these four kernels and three memsets ran for 2-3 us each and were issued for 4-5.
+struct GatedMatrix {
+  const __nv_bfloat16* W;   // [R, C]
+  const float* g;           // [R]
+  __nv_bfloat16* Wg;        // prepare
+  float *G, *dW, *dg;       // dW, dg: finalize
+  int C;
+};
+__global__ void gate_prepare_kernel(const GatedMatrix m0, const GatedMatrix m1, int R, float* __restrict__ zero,
+                                    int n_zero) {
+  const GatedMatrix& m = blockIdx.y ? m1 : m0;
+  const int vec = m.C / 8;
+  const long long total = static_cast<long long>(R) * vec, step = static_cast<long long>(gridDim.x) * blockDim.x;
+  const long long first = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  for (long long i = first; i < total; i += step) {
+    const int r = static_cast<int>(i / vec);
+    float v[8];
+    load8(m.W + i * 8, v);
+    const float s = m.g[r];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] *= s;
+    store8(m.Wg + i * 8, v);
+    float4* G = reinterpret_cast<float4*>(m.G + i * 8);
+    G[0] = G[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  if (blockIdx.y == 0)
+    for (long long i = first; i < n_zero; i += step) zero[i] = 0.f;
+}
+__global__ void gate_finalize_pair_kernel(const GatedMatrix m0, const GatedMatrix m1) {
+  __shared__ float red[2 * 1 * 32];
+  const GatedMatrix& m = blockIdx.y ? m1 : m0;
+  const int r = blockIdx.x;
+  const float s = m.g[r];
+  float acc[1] = {0.f};
+  for (int c = threadIdx.x * 4; c < m.C; c += blockDim.x * 4) {
+    const size_t off = static_cast<size_t>(r) * m.C + c;
+    const float4 gv = *reinterpret_cast<const float4*>(m.G + off);
+    const uint2 wu = *reinterpret_cast<const uint2*>(m.W + off);
+    const float2 w01 = unpack_bf16x2(wu.x), w23 = unpack_bf16x2(wu.y);
+    acc[0] += gv.x * w01.x + gv.y * w01.y + gv.z * w23.x + gv.w * w23.y;
+    float4 d = *reinterpret_cast<float4*>(m.dW + off);
+    d.x = fmaf(s, gv.x, d.x); d.y = fmaf(s, gv.y, d.y); d.z = fmaf(s, gv.z, d.z); d.w = fmaf(s, gv.w, d.w);
+    *reinterpret_cast<float4*>(m.dW + off) = d;
+  }
+  block_sum<1>(acc, red, 0);
+  if (threadIdx.x == 0) m.dg[r] += acc[0];
+}
+
 // ------------------------------------------------------------------------------------------------ optimizer
 // Sum of squares of a flat fp32 buffer into out[0] (double), |x| finite check folded in by the caller.
 __global__ void sumsq_kernel(const float* __restrict__ x, long long n, double* __restrict__ out) {
@@ -1146,6 +1196,30 @@ extern "C" int aeris_gate_grad_finalize(float* G, const void* W, const float* g,
   if (C % 4) return -1;
   gate_grad_finalize_kernel<<<R, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       G, reinterpret_cast<const __nv_bfloat16*>(W), g, dW, dg, R, C);
+  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+}
+
+// W2 [R, C2] and Wo [R, Co] with their gates g2, go [R]: gated copies, zeroed G2 and Go, and `n_zero` zeroed floats.
+extern "C" int aeris_gate_prepare(const void* W2, const float* g2, void* W2g, float* G2, int C2, const void* Wo,
+                                  const float* go, void* Wog, float* Go, int Co, int R, float* zero, int n_zero,
+                                  void* stream) {
+  if (R <= 0 || C2 % 8 || Co % 8) return -1;
+  typedef __nv_bfloat16 bf;
+  const GatedMatrix a = {reinterpret_cast<const bf*>(W2), g2, reinterpret_cast<bf*>(W2g), G2, nullptr, nullptr, C2};
+  const GatedMatrix b = {reinterpret_cast<const bf*>(Wo), go, reinterpret_cast<bf*>(Wog), Go, nullptr, nullptr, Co};
+  const int grid = grid_for(static_cast<long long>(R) * ((C2 > Co ? C2 : Co) / 8), 256, aeris_num_sms() * 4);
+  gate_prepare_kernel<<<dim3(grid, 2), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(a, b, R, zero, n_zero);
+  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+}
+// dW += g * G and dg += rowsum(W * G) for both.
+extern "C" int aeris_gate_finalize_pair(float* G2, const void* W2, const float* g2, float* dW2, float* dg2, int C2,
+                                        float* Go, const void* Wo, const float* go, float* dWo, float* dgo, int Co, int R,
+                                        void* stream) {
+  if (R <= 0 || C2 % 4 || Co % 4) return -1;
+  typedef __nv_bfloat16 bf;
+  const GatedMatrix a = {reinterpret_cast<const bf*>(W2), g2, nullptr, G2, dW2, dg2, C2};
+  const GatedMatrix b = {reinterpret_cast<const bf*>(Wo), go, nullptr, Go, dWo, dgo, Co};
+  gate_finalize_pair_kernel<<<dim3(R, 2), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(a, b);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 

@@ -401,8 +401,8 @@ class SwinLayer(nn.Module):
                 alloc = None
                 if publish_out and j == len(blocks) - 1:
                     alloc = fused._pool_alloc(ctx.peer_fn)
-                x = fused.FusedBlock.apply(x, m, meta, n1w, attn.to_qkv.weight, attn.wo.weight, n2w,
-                                           ff.w1.weight, ff.w2.weight, rg, alloc)
+                x = fused.run_block(x, m, meta, n1w, attn.to_qkv.weight, attn.wo.weight, n2w,
+                                    ff.w1.weight, ff.w2.weight, rg, alloc)
             else:
                 m = mod(dt.to(mod.modulation[-1].weight.dtype)) if mod is not None else \
                     self._plain_modulation(ctx.batch, x.device, x.dtype)

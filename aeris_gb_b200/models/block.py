@@ -19,8 +19,8 @@ class BlockArgs(ctypes.Structure):
     _fields_ = ([(n, _I) for n in ("D", "F", "heads", "head_dim", "L", "mode", "n_win", "batch", "step", "merged",
                                    "slice_windows", "kept", "two_cta", "n_peers")]
                 + [("eps", _F), ("scale", _F), ("mod_vec", _LL), ("mod_sample", _LL)]
-                + [(n, _P) for n in ("mod", "wn1", "wqkv", "wo", "wn2", "w1", "w2", "rope_cos", "rope_sin", "x", "y", "table",
-                                     "peers", "h1", "qkv", "o", "lse", "x1", "h2", "act", "u", "status", "stream")])
+                + [(n, _P) for n in ("mod", "wn1", "wqkv", "wo", "wn2", "w1", "w2", "rope_cos", "rope_sin", "x", "y",
+                                     "table", "peers", "h1", "qkv", "o", "lse", "x1", "h2", "act", "u", "status", "stream")])
 
 
 class BlockGradArgs(ctypes.Structure):

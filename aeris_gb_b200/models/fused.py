@@ -16,6 +16,7 @@ import math
 from dataclasses import dataclass
 
 import torch
+from torch.autograd import forward_ad
 
 from ..ops import attention as A
 from ..ops import elementwise as E
@@ -496,6 +497,31 @@ def _pool_alloc(peer_fn, gradient: bool = False):
     return getattr(getattr(peer_fn, "__self__", None), "gradient_buffer" if gradient else "output_buffer", None)
 
 
+def recorded() -> bool:
+    """Whether anything would notice if an autograd function's forward ran as a plain call: a graph under construction, a
+    forward-mode level, a function transform, a trace. Sampling has none of them; the wrapper costs about 15 us."""
+    return (torch.is_grad_enabled() or forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active()
+            or torch._C._get_tracing_state() is not None)
+
+
+def run_block(x, mod, meta: BlockMeta, wn1, wqkv, wo, wn2, w1, w2, regroup=None, out_alloc=None) -> torch.Tensor:
+    """:class:`FusedBlock` where something is recorded, else its forward pass by itself."""
+    if recorded():
+        return FusedBlock.apply(x, mod, meta, wn1, wqkv, wo, wn2, w1, w2, regroup, out_alloc)
+    return _block_output(x, mod, meta, (wn1, wqkv, wo, wn2, w1, w2), regroup, out_alloc, None)[1]
+
+
+def _block_output(x, mod, meta: BlockMeta, weights, regroup, out_alloc, kept):
+    """(block input in the block's own window layout, output); see :meth:`FusedBlock.forward`."""
+    out = out_alloc(x.shape[0], x.shape[1], x.dtype) if out_alloc is not None else None
+    if regroup is None:
+        return x, block_forward(x, mod.float(), meta, *weights, out=out, kept=kept)
+    table_fwd, _, peer_fn = regroup
+    peers = peer_fn(x, "fwd") if peer_fn is not None else [x.data_ptr()]
+    xg = torch.empty((table_fwd.numel(), x.shape[1]), dtype=x.dtype, device=x.device)
+    return xg, block_forward(xg, mod.float(), meta, *weights, out=out, gather=(table_fwd, peers, x), kept=kept)
+
+
 class FusedBlock(torch.autograd.Function):
     """Autograd wrapper: saves the block input and, with ``meta.keep``, the block's internals; weight gradients go to
     ``param.main_grad`` (fp32) when the engine provides one, otherwise they are returned to autograd."""
@@ -508,7 +534,6 @@ class FusedBlock(torch.autograd.Function):
         output when the caller knows that it will be re-partitioned next (a peer-readable buffer: no publish copy)."""
         ctx.meta = meta
         ctx.regroup = regroup
-        out = out_alloc(x.shape[0], x.shape[1], x.dtype) if out_alloc is not None else None
         kept = None
         if meta.keep and any(ctx.needs_input_grad):        # a frozen block has no backward pass to keep anything for
             shapes = _kept_shapes(regroup[0].numel() if regroup is not None else x.shape[0], x.shape[1],
@@ -517,15 +542,7 @@ class FusedBlock(torch.autograd.Function):
                 kept = {k: torch.empty(shape, dtype=dt, device=x.device) for k, (shape, dt) in shapes.items()}
             except torch.OutOfMemoryError:
                 kept = None            # free in sum but not in pieces of this size: recompute instead
-        if regroup is not None:
-            table_fwd, _, peer_fn = regroup
-            peers = peer_fn(x, "fwd") if peer_fn is not None else [x.data_ptr()]
-            xg = torch.empty((table_fwd.numel(), x.shape[1]), dtype=x.dtype, device=x.device)
-            y = block_forward(xg, mod.float(), meta, wn1, wqkv, wo, wn2, w1, w2, out=out,
-                              gather=(table_fwd, peers, x), kept=kept)
-            x = xg
-        else:
-            y = block_forward(x, mod.float(), meta, wn1, wqkv, wo, wn2, w1, w2, out=out, kept=kept)
+        x, y = _block_output(x, mod, meta, (wn1, wqkv, wo, wn2, w1, w2), regroup, out_alloc, kept)
         ctx.save_for_backward(x, mod, wn1, wqkv, wo, wn2, w1, w2, *([kept[k] for k in KEPT] if kept is not None else ()))
         return y
 
@@ -574,28 +591,61 @@ class GemvLinearFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
+        dx, rW, rb = _gemv_backward(*ctx.saved_tensors, dy, ctx.silu_in, ctx.needs_input_grad[0])
+        return dx, rW, rb, None
+
+
+def _gemv_backward(x, W, b, dy, silu_in: bool, need_dx: bool):
+    """Gradients of ``silu?(x) @ W^T + b``: (dx or None, and dW and db where they do not go to a ``main_grad``)."""
+    from ..ops import diffusion as DF
+    from .fused_io import _grad_slot, _kernel_target, _settle
+    sW, rW = _grad_slot(W)
+    sb, rb = _grad_slot(b) if b is not None else (None, None)
+    dx = torch.zeros(x.shape, dtype=torch.float32, device=x.device) if need_dx else None
+    if DF.gemv_bwd_ok(W, sW):
+        tb = _kernel_target(sb) if sb is not None else None
+        DF.gemv_bwd(W, x, dy, sW, tb, dx, silu_in)
+        if sb is not None:
+            _settle(sb, tb)
+    else:
+        dy, x32 = dy.float(), x.float()
+        sig = torch.sigmoid(x32)
+        sW.addmm_(dy.t(), x32 * sig if silu_in else x32)
+        if sb is not None:
+            sb += dy.sum(0)
+        if dx is not None:
+            dx = dy @ W.float()
+            dx = dx * (sig * (1 + x32 * (1 - sig))) if silu_in else dx
+    return (dx.to(x.dtype) if dx is not None else None, rW.to(W.dtype) if rW is not None else None,
+            rb.to(b.dtype) if rb is not None else None)
+
+
+class ModulationFn(torch.autograd.Function):
+    """``silu(x @ W1^T + b1) @ W2^T + b2``: two :class:`GemvLinearFn` as one node, whose forward is one native call."""
+
+    @staticmethod
+    def forward(ctx, x, W1, b1, W2, b2):
+        from ..ops import diffusion as DF
+        y1, y2 = DF.modulation_mlp(W1.detach(), b1.detach(), x.detach(), W2.detach(), b2.detach())
+        ctx.save_for_backward(x, W1, b1, y1, W2, b2)
+        return y2
+
+    @staticmethod
+    def backward(ctx, dy):
         from ..ops import diffusion as DF
         from .fused_io import _grad_slot, _kernel_target, _settle
-        x, W, b = ctx.saved_tensors
-        sW, rW = _grad_slot(W)
-        sb, rb = _grad_slot(b) if b is not None else (None, None)
-        dx = torch.zeros(x.shape, dtype=torch.float32, device=x.device) if ctx.needs_input_grad[0] else None
-        if DF.gemv_bwd_ok(W, sW):
-            tb = _kernel_target(sb) if sb is not None else None
-            DF.gemv_bwd(W, x, dy, sW, tb, dx, ctx.silu_in)
-            if sb is not None:
-                _settle(sb, tb)
-        else:
-            dy, x32 = dy.float(), x.float()
-            sig = torch.sigmoid(x32)
-            sW.addmm_(dy.t(), x32 * sig if ctx.silu_in else x32)
-            if sb is not None:
-                sb += dy.sum(0)
-            if dx is not None:
-                dx = dy @ W.float()
-                dx = dx * (sig * (1 + x32 * (1 - sig))) if ctx.silu_in else dx
-        return (dx.to(x.dtype) if dx is not None else None, rW.to(W.dtype) if rW is not None else None,
-                rb.to(b.dtype) if rb is not None else None, None)
+        x, W1, b1, y1, W2, b2 = ctx.saved_tensors
+        (s1, r1), (sb1, rb1), (s2, r2), (sb2, rb2) = (_grad_slot(p) for p in (W1, b1, W2, b2))
+        if DF.gemv_bwd_ok(W1, s1) and DF.gemv_bwd_ok(W2, s2):
+            t1, t2 = _kernel_target(sb1), _kernel_target(sb2)
+            dx = DF.modulation_mlp_bwd(W1, x, W2, y1, dy, s1, t1, s2, t2, ctx.needs_input_grad[0])
+            _settle(sb1, t1)
+            _settle(sb2, t2)
+            grads = (r.to(p.dtype) if r is not None else None for p, r in zip((W1, b1, W2, b2), (r1, rb1, r2, rb2)))
+            return (dx.to(x.dtype) if dx is not None else None, *grads)
+        dy1, r2, rb2 = _gemv_backward(y1, W2, b2, dy, True, True)
+        dx, r1, rb1 = _gemv_backward(x, W1, b1, dy1, False, ctx.needs_input_grad[0])
+        return dx, r1, rb1, r2, rb2
 
 
 def modulation(seq: torch.nn.Sequential, emb: torch.Tensor) -> torch.Tensor:
@@ -606,6 +656,9 @@ def modulation(seq: torch.nn.Sequential, emb: torch.Tensor) -> torch.Tensor:
     w = last.weight
     if not DF.gemv_ok(emb.shape[0], max(emb.shape[1], w.shape[1])):
         return seq(emb.to(w.dtype)).float()
+    if len(seq) == 3 and seq[0].bias is not None and last.bias is not None:
+        args = (emb, seq[0].weight, seq[0].bias, w, last.bias)
+        return ModulationFn.apply(*args) if recorded() else DF.modulation_mlp(*args[1:3], emb, *args[3:])[1]
     x = emb
     if len(seq) == 3:
         x = GemvLinearFn.apply(x, seq[0].weight, seq[0].bias, False)

@@ -119,6 +119,21 @@ def gemv_bias_act(W: torch.Tensor, bias: torch.Tensor | None, x: torch.Tensor, a
     return y
 
 
+def modulation_mlp(W1: torch.Tensor, b1: torch.Tensor, x: torch.Tensor, W2: torch.Tensor,
+                   b2: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+    """``y1 = x @ W1^T + b1`` and ``silu(y1) @ W2^T + b2``, fp32: two :func:`gemv_bias_act` in one call."""
+    (N1, K), N2 = W1.shape, W2.shape[0]
+    assert W2.shape[1] == N1
+    x, b1, b2 = _f32_or_bf16(x).contiguous(), _f32_or_bf16(b1), _f32_or_bf16(b2)
+    B = x.shape[0]
+    y1 = torch.empty((B, N1), dtype=torch.float32, device=x.device)
+    y2 = torch.empty((B, N2), dtype=torch.float32, device=x.device)
+    rc = _l.lib().aeris_modulation_mlp(_l.ptr(W1), _gemv_flags(W1, b1, x), _l.ptr(b1), _l.ptr(x), _l.ptr(y1), N1, K,
+                                       _l.ptr(W2), _gemv_flags(W2, b2, y1), _l.ptr(b2), _l.ptr(y2), N2, B, _l.stream_ptr())
+    _l.check(rc, "aeris_modulation_mlp", kernels=2)
+    return y1, y2
+
+
 def gemv_bwd(W: torch.Tensor, x: torch.Tensor, dy: torch.Tensor, dW: torch.Tensor, db: torch.Tensor | None,
              dx: torch.Tensor | None, silu_in: bool = False) -> None:
     """Adds the gradients of ``silu?(x) @ W^T + b`` (at most 8 rows) to fp32 ``dW``, ``db`` and ``dx``."""
@@ -127,6 +142,22 @@ def gemv_bwd(W: torch.Tensor, x: torch.Tensor, dy: torch.Tensor, dW: torch.Tenso
     rc = _l.lib().aeris_gemv_bwd(_l.ptr(W), _gemv_flags(W, None, x), _l.ptr(x), _l.ptr(dy), _l.ptr(dW), _l.ptr(db),
                                  _l.ptr(dx), N, K, x.shape[0], int(silu_in), _l.stream_ptr())
     _l.check(rc, "aeris_gemv_bwd")
+
+
+def modulation_mlp_bwd(W1: torch.Tensor, x: torch.Tensor, W2: torch.Tensor, y1: torch.Tensor, dy: torch.Tensor,
+                       dW1: torch.Tensor, db1: torch.Tensor, dW2: torch.Tensor, db2: torch.Tensor,
+                       need_dx: bool) -> torch.Tensor | None:
+    """Adds the gradients of :func:`modulation_mlp` to fp32 ``dW1 .. db2``; returns that of ``x`` (fp32) if asked for."""
+    (N1, K), N2 = W1.shape, W2.shape[0]
+    x, dy = _f32_or_bf16(x).contiguous(), dy.float().contiguous()
+    B = x.shape[0]
+    dy1 = torch.empty((B, N1), dtype=torch.float32, device=x.device)
+    dx = torch.empty((B, K), dtype=torch.float32, device=x.device) if need_dx else None
+    rc = _l.lib().aeris_modulation_mlp_bwd(_l.ptr(W1), _gemv_flags(W1, None, x), _l.ptr(x), _l.ptr(dW1), _l.ptr(db1),
+                                           _l.ptr(dx), N1, K, _l.ptr(W2), _gemv_flags(W2, None, y1), _l.ptr(y1), _l.ptr(dy),
+                                           _l.ptr(dW2), _l.ptr(db2), _l.ptr(dy1), N2, B, _l.stream_ptr())
+    _l.check(rc, "aeris_modulation_mlp_bwd", kernels=2)
+    return dx
 
 
 def gemv_bwd_ok(W: torch.Tensor, dW: torch.Tensor) -> bool:

@@ -51,7 +51,8 @@ def test_what_the_native_call_does_not_take_goes_one_by_one():
                              (meta(36), T(), mod, ok, ()), (meta(136), T(), mod, ok, ()),
                              (meta(), T(torch.float32), mod, ok, ()), (meta(), T(cuda=False), mod, ok, ()),
                              (meta(), T(whole=False), mod, ok, ()), (meta(), T(), T(), ok, ()),
-                             (meta(), T(), mod, ok[:5] + [T(torch.float32)], ()), (meta(), T(), mod, ok[:5] + [T(whole=False)], ()),
+                             (meta(), T(), mod, ok[:5] + [T(torch.float32)], ()),
+                             (meta(), T(), mod, ok[:5] + [T(whole=False)], ()),
                              (meta(), T(), mod, ok, [T()]), (meta(), T(), mod, ok, [T(torch.float32, whole=False)])):
         assert not block.takes(m, x, md, ws, gs)
 
@@ -64,7 +65,8 @@ def test_what_the_native_call_does_not_take_goes_one_by_one():
     (3, 2, 30, 16, 40, 384, 64, None, 1, False)])    # narrow heads, widths for the one-CTA kernel
 @pytest.mark.parametrize("keep", [False, True])
 @pytest.mark.parametrize("gathered", [False, True])
-def test_block_in_one_call_equals_its_launches(B, n_win, L, heads, d, F, chunk, floor, mode, rope, keep, gathered, monkeypatch):
+def test_block_in_one_call_equals_its_launches(B, n_win, L, heads, d, F, chunk, floor, mode, rope, keep, gathered,
+                                               monkeypatch):
     from aeris_gb_b200.models import block, fused
     from aeris_gb_b200.ops import lib
     torch.manual_seed(B * L)
@@ -97,7 +99,9 @@ def test_block_in_one_call_equals_its_launches(B, n_win, L, heads, d, F, chunk, 
         out.append((y, dx, dmod, grads, (n1 - n0, lib.launch_count() - n1)))
     lib.check_status()
     (y0, dx0, dm0, g0, n0), (y1, dx1, dm1, g1, n1) = out
-    assert torch.equal(y0, y1) and torch.equal(dx0, dx1) and n0 == n1
+    assert torch.equal(y0, y1) and torch.equal(dx0, dx1)
+    # the two gated matrices share a launch before and after each sample's products
+    assert n0[0] == n1[0] and n0[1] == n1[1] - 2 * B
     # the column sums and split reductions are fp32 atomics in another order each time
     assert rel_err(dm0, dm1) < 1e-5
     for k in g0:
