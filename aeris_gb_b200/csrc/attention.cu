@@ -597,7 +597,9 @@ template <int DCH> struct BwdRing {
   static constexpr int NB = (DCH == 1) ? 2 : 1;         // buffers for the item's own 128-row operands
   static constexpr int ITEM_BYTES = 2 * DCH * 16384, STAGE = 2 * DCH * 8192;
   static constexpr int STAT = 4 * TILE > NST * 2 * BT ? 4 * TILE : NST * 2 * BT;
-  static constexpr int SMEM = NB * ITEM_BYTES + NST * STAGE + STAT * 4 + 512;
+  static constexpr bool STAGED = DCH == 2;              // gradient rows leave through shared memory, see BwdOut
+  static constexpr int OUT_BYTES = STAGED ? TILE * 64 : 0;      // 32 columns, per warpgroup
+  static constexpr int SMEM = NB * ITEM_BYTES + NST * STAGE + NWG * OUT_BYTES + STAT * 4 + 512;
   static constexpr int THREADS = 128 + 128 * NWG;
 };
 static_assert(BwdRing<1>::SMEM <= 227 * 1024 && BwdRing<2>::SMEM <= 227 * 1024, "shared memory");
@@ -609,6 +611,57 @@ __device__ __forceinline__ void cp_async4(float* smem_dst, const float* src, uin
 __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+
+// Gradient rows on their way out: a warpgroup turns 32 accumulator columns of its 128 rows into bf16 in shared memory, one
+// thread hands them to the TMA unit as one tiled store. The accumulator is free once it has been read; written by the threads
+// themselves (one row each, 32 rows with every 16-byte store instruction) it kept the next item's products waiting. Rows
+// past the window's end and columns past the head's width are clipped by the tensor map. Both kernels, ms, before and now,
+// 12 heads x 128: 400 x 128 tokens 0.550 -> 0.464, 200 x 225 0.625 -> 0.546, 72 x 900 1.69 -> 1.60, 16 x 3600 4.45 -> 4.34. At
+// 64, with a third of the columns per warpgroup, the hand-shakes cost more than they save (24 x 64, 200 x 225: 0.650 ->
+// 0.704, 72 x 900 1.91 -> 1.92): direct stores there.
+struct BwdOut {
+  uint8_t* stage;           // this warpgroup's
+  uint64_t *free_bar, *full_bar;
+  int* status;
+  int warp_in_group, lane, row, n = 0;
+
+  __device__ __forceinline__ bool leader() const { return warp_in_group == 0 && lane == 0; }
+  // `read`: called once the columns are out of tensor memory
+  template <typename F>
+  __device__ __forceinline__ bool put(uint32_t taddr, float f, const CUtensorMap* m, int col, int head, int grow, int win,
+                                      F&& read) {
+    uint32_t v[32];
+    tmem_ld32(taddr, v);
+    tmem_wait_ld();
+    read();
+    if (leader()) {
+      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+      mbar_arrive(free_bar);
+    }
+    if (!mbar_wait(free_bar, n & 1, status, ERR_TIMEOUT_ATTN)) return false;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      uint32_t o[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        o[i] = pack_bf16x2(__uint_as_float(v[8 * g + 2 * i]) * f, __uint_as_float(v[8 * g + 2 * i + 1]) * f);
+      *reinterpret_cast<uint4*>(stage + row * 64 + ((g ^ ((row >> 1) & 3)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(full_bar);
+    if (leader()) {
+      if (!mbar_wait(full_bar, n & 1, status, ERR_TIMEOUT_ATTN)) return false;
+      tma_store_4d(m, stage, col, head, grow, win);
+    }
+    ++n;
+    return true;
+  }
+  // before this thread leaves: its copies have been performed
+  __device__ __forceinline__ void drain() const {
+    if (leader()) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  }
+};
 
 // Position of a role in the CTA's stream of tiles: item `it` (of this CTA), tile `j` of the item, running number `g`.
 struct TileIter {
@@ -636,7 +689,7 @@ template <int DCH>
 __global__ void __launch_bounds__(128 + 128 * BwdRing<DCH>::NWG, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-                   const AttnBwdParams p, const int n_items_total) {
+                   const __grid_constant__ CUtensorMap tm_dq, const AttnBwdParams p, const int n_items_total) {
   using R = BwdRing<DCH>;
   constexpr int HD = 64 * DCH;
   constexpr int QB = DCH * 16384;       // Q tile, dO tile (128 rows)
@@ -646,7 +699,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sQ = smem;                   // [NB] items: Q | dO
   uint8_t* sKV = sQ + NB * R::ITEM_BYTES;                    // [NST] K | V
-  float* s_stat = reinterpret_cast<float*>(sKV + NST * R::STAGE);   // [2] items: lse [128] | delta [128]
+  uint8_t* sOut = sKV + NST * R::STAGE;                      // [NWG]
+  float* s_stat = reinterpret_cast<float*>(sOut + NWG * R::OUT_BYTES);   // [2] items: lse [128] | delta [128]
   uint64_t* bars = reinterpret_cast<uint64_t*>(s_stat + R::STAT);
   uint64_t* q_full = bars;              // [NB <= 2]
   uint64_t* q_empty = bars + 2;         // [NB]
@@ -658,7 +712,9 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   uint64_t* acc_empty = bars + 20;
   uint64_t* stat_full = bars + 21;      // [2]
   uint64_t* stat_empty = bars + 23;     // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 25);
+  uint64_t* out_free = bars + 25;       // [NWG]
+  uint64_t* out_full = bars + 28;       // [NWG]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 31);
   int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -685,7 +741,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     for (int i = 0; i < NWG; ++i) {
       mbar_init(&first_full[i], 1);
       mbar_init(&next_full[i], 4 + 1);
-      mbar_init(&sp_full[i], 1);
+      mbar_init(&sp_full[i], 1); mbar_init(&out_free[i], 1); mbar_init(&out_full[i], 4);
     }
     mbar_init(acc_full, 1); mbar_init(acc_empty, 4 * NWG);
     fence_barrier_init();
@@ -879,12 +935,27 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     uint32_t ph = 0;
     int j = wg;                       // first tile of this warpgroup in the item at hand
     bool ok = true;
+    BwdOut out{sOut + wg * R::OUT_BYTES, &out_free[wg], &out_full[wg], p.status, q, lane, row};
     // Gradient rows of item `it` from TMEM to memory. Runs after this warpgroup's first tile of the NEXT item, so that the
     // wait for the last products of `it` is spent on that tile.
     auto epilogue = [&](int it) -> bool {
       if (!mbar_wait(acc_full, it & 1, p.status, ERR_TIMEOUT_ATTN)) return false;
       tc_fence_after();
       const BwdItem w = bwd_item(it, row_tiles, p.H);
+      auto release = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty);
+      };
+      if (R::STAGED && p.push_n_local == 0) {
+        int mine = 0;                   // this warpgroup's groups of 32 columns
+        for (int c = wg * 32; c < p.d; c += 32 * NWG) ++mine;
+        if (mine == 0) release();
+        for (int c = wg * 32; c < p.d; c += 32 * NWG)
+          if (!out.put(tdQ + lane_addr + c, sc, &tm_dq, c, w.head, w.tile * TILE, w.win, [&] { if (--mine == 0) release(); }))
+            return false;
+        return true;
+      }
       const int grow = w.tile * TILE + row;
       const bool row_ok = grow < N;
       __nv_bfloat16* dst = bwd_dst(p, w.win, row_ok ? grow : 0, w.head, 0, p.q_col0);
@@ -974,6 +1045,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       j -= nkv;                        // the stream of tiles runs on into the next item
     }
     if (ok) epilogue(n_items - 1);
+    if (R::STAGED) out.drain();
   }
   tc_fence_before();
   __syncthreads();
@@ -985,6 +1057,7 @@ template <int DCH>
 __global__ void __launch_bounds__(128 + 128 * BwdRing<DCH>::NWG, 1)
 attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
+                    const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
                     const AttnBwdParams p, const int n_items_total) {
   using R = BwdRing<DCH>;
   constexpr int HD = 64 * DCH;
@@ -995,7 +1068,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sKV = smem;                   // [NB] items: K | V
   uint8_t* sQD = sKV + NB * R::ITEM_BYTES;                          // [NST] Q | dO
-  float* s_stat = reinterpret_cast<float*>(sQD + NST * R::STAGE);   // [NST] lse [64] | delta [64]
+  uint8_t* sOut = sQD + NST * R::STAGE;                             // [NWG]
+  float* s_stat = reinterpret_cast<float*>(sOut + NWG * R::OUT_BYTES);   // [NST] lse [64] | delta [64]
   uint64_t* bars = reinterpret_cast<uint64_t*>(s_stat + R::STAT);
   uint64_t* kv_full = bars;              // [NB <= 2]
   uint64_t* kv_empty = bars + 2;         // [NB]
@@ -1005,7 +1079,9 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   uint64_t* sp_full = bars + 16;         // [NWG]
   uint64_t* acc_full = bars + 19;
   uint64_t* acc_empty = bars + 20;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
+  uint64_t* out_free = bars + 21;        // [NWG]
+  uint64_t* out_full = bars + 24;        // [NWG]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 27);
   int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1032,7 +1108,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     for (int i = 0; i < NWG; ++i) {
       mbar_init(&first_full[i], 1 + 32);
       mbar_init(&next_full[i], 4 + 1 + 32);
-      mbar_init(&sp_full[i], 1);
+      mbar_init(&sp_full[i], 1); mbar_init(&out_free[i], 1); mbar_init(&out_full[i], 4);
     }
     mbar_init(acc_full, 1); mbar_init(acc_empty, 4 * NWG);
     fence_barrier_init();
@@ -1214,11 +1290,29 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       pp = f2_to_bf16x2(pr);
       dd = f2_to_bf16x2(f2_mul(pr, f2_sub(f2_pack(__uint_as_float(d0), __uint_as_float(d1)), de)));
     };
+    BwdOut out{sOut + wg * R::OUT_BYTES, &out_free[wg], &out_full[wg], p.status, q, lane, row};
     // see attn_bwd_dq_kernel: the epilogue of an item runs after this warpgroup's first tile of the next
     auto epilogue = [&](int it) -> bool {
       if (!mbar_wait(acc_full, it & 1, p.status, ERR_TIMEOUT_ATTN)) return false;
       tc_fence_after();
       const BwdItem w = bwd_item(it, row_tiles, p.H);
+      auto release = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty);
+      };
+      if (R::STAGED && p.push_n_local == 0) {
+        int mine = 0;                   // this warpgroup's groups of 32 columns of dK and dV
+        for (int c = wg * 32; c < 2 * HD; c += 32 * NWG) mine += (c < HD ? c : c - HD) < p.d;
+        if (mine == 0) release();
+        for (int c = wg * 32; c < 2 * HD; c += 32 * NWG) {
+          const int col = c < HD ? c : c - HD;          // column inside the head
+          if (col < p.d && !out.put(tdK + lane_addr + c, c < HD ? sc : 1.f, c < HD ? &tm_dk : &tm_dv, col, w.head,
+                                    w.tile * TILE, w.win, [&] { if (--mine == 0) release(); }))
+            return false;
+        }
+        return true;
+      }
       const int grow = w.tile * TILE + row;
       const bool row_ok = grow < N;
       __nv_bfloat16* dk = bwd_dst(p, w.win, row_ok ? grow : 0, w.head, 1, p.k_col0);
@@ -1303,6 +1397,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       j -= nq;                        // the stream of tiles runs on into the next item
     }
     if (ok) epilogue(n_items - 1);
+    if (R::STAGED) out.drain();
   }
   tc_fence_before();
   __syncthreads();
@@ -1313,8 +1408,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 template <int DCH>
 static int launch_attn_bwd(const CUtensorMap& tq128, const CUtensorMap& tk64, const CUtensorMap& tv64,
                            const CUtensorMap& tdo128, const CUtensorMap& tq64, const CUtensorMap& tk128,
-                           const CUtensorMap& tv128, const CUtensorMap& tdo64, const AttnBwdParams& p,
-                           cudaStream_t stream) {
+                           const CUtensorMap& tv128, const CUtensorMap& tdo64, const CUtensorMap (&out)[3],
+                           const AttnBwdParams& p, cudaStream_t stream) {
   using R = BwdRing<DCH>;
   auto k1 = attn_bwd_dq_kernel<DCH>;
   auto k2 = attn_bwd_dkv_kernel<DCH>;
@@ -1327,9 +1422,9 @@ static int launch_attn_bwd(const CUtensorMap& tq128, const CUtensorMap& tk64, co
   const long long items = static_cast<long long>((p.N + TILE - 1) / TILE) * p.H * p.n_win;
   if (items > 0x3fffffff) return -23;
   const int n = static_cast<int>(items), grid = n < num_sms() ? n : num_sms();
-  k1<<<grid, R::THREADS, R::SMEM, stream>>>(tq128, tk64, tv64, tdo128, p, n);
+  k1<<<grid, R::THREADS, R::SMEM, stream>>>(tq128, tk64, tv64, tdo128, out[0], p, n);
   if (cudaGetLastError() != cudaSuccess) return -21;
-  k2<<<grid, R::THREADS, R::SMEM, stream>>>(tq64, tk128, tv128, tdo64, p, n);
+  k2<<<grid, R::THREADS, R::SMEM, stream>>>(tq64, tk128, tv128, tdo64, out[1], out[2], p, n);
   return cudaGetLastError() == cudaSuccess ? 0 : -22;
 }
 
@@ -1497,8 +1592,15 @@ static int attn_bwd_impl(const void* qkv, int ldq, int q_col0, int k_col0, int v
       {&d128, d_o, ldo, TILE},        {&d64, d_o, ldo, BT}};
   for (const auto& m : maps)
     if ((r = make_tmap_heads_bf16(m.m, m.base, head_dim, H, N, n_win, m.ld, m.rows))) return r;
-  return head_dim <= 64 ? launch_attn_bwd<1>(q128, k64, v64, d128, q64, k128, v128, d64, p, stream)
-                        : launch_attn_bwd<2>(q128, k64, v64, d128, q64, k128, v128, d64, p, stream);
+  CUtensorMap out[3] = {q128, q128, q128};      // pushed gradients and those of narrow heads do not leave through them
+  if (head_dim > 64 && !dq_peers) {
+    const __nv_bfloat16* g = p.dQKV;
+    const int cols[3] = {q_col0, k_col0, v_col0};
+    for (int i = 0; i < 3; ++i)
+      if ((r = make_tmap_heads32_bf16(&out[i], g + cols[i], head_dim, H, N, n_win, ldg, TILE))) return r;
+  }
+  return head_dim <= 64 ? launch_attn_bwd<1>(q128, k64, v64, d128, q64, k128, v128, d64, out, p, stream)
+                        : launch_attn_bwd<2>(q128, k64, v64, d128, q64, k128, v128, d64, out, p, stream);
 }
 
 // ------------------------------------------------------------------------------------------ allocation-free variant

@@ -236,20 +236,30 @@ int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64
   return r == CUDA_SUCCESS ? 0 : -12;
 }
 
-int make_tmap_heads_bf16(CUtensorMap* out, const void* base, int d, int heads, int tokens, int windows, uint64_t ld,
-                         uint32_t box_rows) {
+static int make_tmap_heads(CUtensorMap* out, const void* base, int d, int heads, int tokens, int windows, uint64_t ld,
+                           uint32_t box_cols, uint32_t box_rows, CUtensorMapSwizzle swizzle) {
   PFN_encodeTiled enc = get_encode();
   if (!enc) return -10;
   if ((reinterpret_cast<uintptr_t>(base) & 15) || d % 8 || ((ld * 2) & 15)) return -11;
   cuuint64_t dims[4] = {static_cast<cuuint64_t>(d), static_cast<cuuint64_t>(heads), static_cast<cuuint64_t>(tokens),
                         static_cast<cuuint64_t>(windows)};
   cuuint64_t strides[3] = {static_cast<cuuint64_t>(d) * 2, ld * 2, static_cast<cuuint64_t>(tokens) * ld * 2};
-  cuuint32_t box[4] = {64, 1, box_rows, 1};
+  cuuint32_t box[4] = {box_cols, 1, box_rows, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -12;
+}
+
+int make_tmap_heads_bf16(CUtensorMap* out, const void* base, int d, int heads, int tokens, int windows, uint64_t ld,
+                         uint32_t box_rows) {
+  return make_tmap_heads(out, base, d, heads, tokens, windows, ld, 64, box_rows, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+int make_tmap_heads32_bf16(CUtensorMap* out, const void* base, int d, int heads, int tokens, int windows, uint64_t ld,
+                           uint32_t box_rows) {
+  return make_tmap_heads(out, base, d, heads, tokens, windows, ld, 32, box_rows, CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 static int g_num_sms = 0;

@@ -485,12 +485,13 @@ extern "C" int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M
   // 1536 x 1536 311 / 284, 28800 x 2048 x 2048 217 / 210, x 2304 x 2304 255 / 256, x 3072 x 3072 424 / 436; SwiGLU backward
   // 64800 x 4096 x 1536 1106 / 985, 28800 x 5376 x 2048 735 / 690, x 6144 x 2304 885 / 832, x 8192 x 3072 1334 / 1321;
   // SwiGLU with the raw columns 28800 x 4096 x 768 220 / 191, x 8192 x 1536 615 / 611, x 10752 x 2048 999 / 1035, x 12288 x
-  // 2304 1270 / 1309. One line at 2048 for the three: the SwiGLU backward would gain above it, the raw columns lose below.
+  // 2304 1270 / 1309. The raw columns lose below the line at 2048.
   // Plain store 28800 x 2304 x 768 104 / 98, x 3072 x 1024 158 / 157, x 3840 x 1280 222 / 232. Weight gradients (a_mn) lose
   // a few per cent. Since then the SwiGLU backward and the gated residual on eight warps request their second operand ahead
-  // (registers for that spilled; see swiglu_u_request).
+  // (registers for that spilled; see swiglu_u_request), and the SwiGLU backward's line moved up: 28800 x 6144 x 2304 832 / 740,
+  // x 8192 x 3072 1300 / 1310, x 13696 x 5120 3598 / 3619.
   const bool heavy = epi == EPI_SWIGLU_BOTH || epi == EPI_SWIGLU_BWD || epi == EPI_GATE_RESID;
-  const bool ew8 = (heavy && K <= 2048) || (epi == EPI_STORE && K <= 1024);
+  const bool ew8 = (heavy && K <= (epi == EPI_SWIGLU_BWD ? 2560 : 2048)) || (epi == EPI_STORE && K <= 1024);
   if (a_mn) return b_mn ? launch_gemm2<1, 1, 4>(ta, tb, p, stream) : launch_gemm2<1, 0, 4>(ta, tb, p, stream);
   if (b_mn) return ew8 ? launch_gemm2<0, 1, 8>(ta, tb, p, stream) : launch_gemm2<0, 1, 4>(ta, tb, p, stream);
   return ew8 ? launch_gemm2<0, 0, 8>(ta, tb, p, stream) : launch_gemm2<0, 0, 4>(ta, tb, p, stream);

@@ -10,6 +10,9 @@ int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64
 // whose first head starts at `base`; box {64, 1, box_rows, 1}. Channels past d, tokens past the window's end: zeros.
 int make_tmap_heads_bf16(CUtensorMap* out, const void* base, int d, int heads, int tokens, int windows, uint64_t ld,
                          uint32_t box_rows);
+// The same dims with box {32, 1, box_rows, 1} and the 64-byte swizzle: for tiled stores of 32 columns.
+int make_tmap_heads32_bf16(CUtensorMap* out, const void* base, int d, int heads, int tokens, int windows, uint64_t ld,
+                           uint32_t box_rows);
 int num_sms();
 // Slices of an accumulating product's reduction over `kb_total` blocks of 64: see gemm.cu.
 int choose_k_splits(int tiles, int kb_total, int units, int most, int want);
