@@ -59,6 +59,11 @@ int aeris_modnorm_fwd_batch(const void* x, const void* gidx, const void* const* 
 int aeris_modnorm_bwd(const void* x, const void* dh, const void* dres, const float* scale, const float* shift,
                       const void* w, void* dx, float* dscale, float* dshift, float* dw, int rows, int D, int mode,
                       float eps, const float* w_f32, void* stream);
+int aeris_modnorm_fwd_f32(const void* x, const float* scale, const float* shift, const float* w_f32, float* h, int batch,
+                          int rows, int D, int mode, float eps, void* stream);
+int aeris_modnorm_bwd_f32(const void* x, const float* dh, const float* scale, const float* shift, const float* w_f32,
+                          void* dx, float* dscale, float* dshift, float* dw, float* sums, int sum_rows, int rows, int D,
+                          int mode, float eps, void* stream);
 int aeris_gather_rows(const void* gidx, const void* const* peer_ptrs, int n_peers, void* out, long long rows, int D,
                       void* stream);
 int aeris_swiglu_fwd(const void* u, void* act, long long rows, int F, void* stream);

@@ -9,6 +9,8 @@
 #include "common.cuh"
 #include "api.h"
 
+#include <type_traits>
+
 namespace aeris {
 
 struct PeerPtrs {
@@ -245,13 +247,14 @@ modnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __restri
 // and the four rows' sums go through group_sum4. Rows of up to 1536 columns: three CTAs of at most six warps per SM
 // at their widest; up to 2560 two CTAs of at most ten; wider ones: one
 // CTA of up to twenty warps (28800 x 5120: 165 -> 98 us, 6.0 TB/s).
-template <int MAXT, int MINB, int W8>
+// F32: `h` is fp32 (the stock fp32 output head reads it).
+template <int MAXT, int MINB, int W8, bool F32 = false>
 __global__ void __launch_bounds__(MAXT, MINB)
 modnorm_fwd_pair_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __restrict__ gidx, PeerPtrs peers,
                         __nv_bfloat16* __restrict__ x_out, const float* __restrict__ scale,
                         const float* __restrict__ shift, const __nv_bfloat16* __restrict__ w,
-                        __nv_bfloat16* __restrict__ h, int rows, int D, int mode, float eps,
-                        const float* __restrict__ wf, __nv_bfloat16* __restrict__ h_lo) {
+                        std::conditional_t<F32, float, __nv_bfloat16>* __restrict__ h, int rows, int D, int mode,
+                        float eps, const float* __restrict__ wf, __nv_bfloat16* __restrict__ h_lo) {
   static_assert(FWD_RPI == 4 && MAXT <= 256 * W8, "group_sum4 adds four values of at most 8 * W8 warps");
   __shared__ float red[2][32 * W8];
   {  // grid.y = samples of `rows` rows each, with a modulation vector of their own
@@ -349,15 +352,21 @@ modnorm_fwd_pair_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __r
         const uint64_t n = f2_mul(f2_mul(y[k][i], rinv2), wv[i]);
         o[i] = (mode == 0) ? n : f2_fma(n, sc1[i], sh[i]);
       }
-      uint32_t hw[4];
+      if constexpr (F32) {
+        ulonglong2* dst = reinterpret_cast<ulonglong2*>(h + static_cast<size_t>(rr) * D + c0);
+        dst[0] = make_ulonglong2(o[0], o[1]);
+        dst[1] = make_ulonglong2(o[2], o[3]);
+      } else {
+        uint32_t hw[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) hw[i] = f2_to_bf16x2(o[i]);
-      *reinterpret_cast<uint4*>(h + static_cast<size_t>(rr) * D + c0) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-      if (h_lo) {          // the part of the fp32 value that the bf16 value above does not hold
-        uint32_t lw[4];
+        for (int i = 0; i < 4; ++i) hw[i] = f2_to_bf16x2(o[i]);
+        *reinterpret_cast<uint4*>(h + static_cast<size_t>(rr) * D + c0) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+        if (h_lo) {          // the part of the fp32 value that the bf16 value above does not hold
+          uint32_t lw[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) lw[i] = f2_to_bf16x2(f2_sub(o[i], f2_from_bf16x2(hw[i])));
-        *reinterpret_cast<uint4*>(h_lo + static_cast<size_t>(rr) * D + c0) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+          for (int i = 0; i < 4; ++i) lw[i] = f2_to_bf16x2(f2_sub(o[i], f2_from_bf16x2(hw[i])));
+          *reinterpret_cast<uint4*>(h_lo + static_cast<size_t>(rr) * D + c0) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+        }
       }
     }
   }
@@ -504,9 +513,15 @@ modnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 //     from shared memory; one row per reduction is what the registers hold then (two spilled).
 // Before and now (mode 0, held for 0.3 s at 1890-1965 MHz): 28800 x 512 columns 111 -> 26 us, 28800 x 768 115 -> 37 us,
 // 64800 x 1536 211 -> 144 us (5.5 TB/s), 28800 x 5120 459 -> 347 us (mode 1: 447 -> 314).
-template <int VPT, int RPI, int MAXT>
+// F32: `dh` is fp32 (from the stock fp32 output head). The column sums are the gradients of a fp32 stage then and may not be
+// less accurate than PyTorch's own: a thread adds up SUM_ROWS rows at a time, and every CTA stores its sums as a row of
+// `dscale` [CTAs, 3, D], which column_sums_kernel adds up in double. Relative error against 64 bits, 65536 rows of 1536
+// columns: 4.0e-7 with one chain of additions and atomics, 2.5e-7 from PyTorch, 2.1e-7 here.
+constexpr int SUM_ROWS = 16;
+template <int VPT, int RPI, int MAXT, bool F32 = false>
 __global__ void __launch_bounds__(MAXT, 1)
-modnorm_bwd_group_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dh,
+modnorm_bwd_group_kernel(const __nv_bfloat16* __restrict__ x,
+                         const std::conditional_t<F32, float, __nv_bfloat16>* __restrict__ dh,
                          const __nv_bfloat16* __restrict__ dres, const float* __restrict__ scale,
                          const float* __restrict__ shift, const __nv_bfloat16* __restrict__ w,
                          __nv_bfloat16* __restrict__ dx, float* __restrict__ dscale, float* __restrict__ dshift,
@@ -576,11 +591,52 @@ modnorm_bwd_group_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
   const int stride = gstep * RPI;
   const float inv_d = 1.f / D;
   int parity = 0;
-  uint4 nx[RPI][VPT], ng[RPI][VPT], nr[RPI][VPT];
+  // [group][3][D] column sums in shared memory: each thread's columns are its own until the CTA adds them up
+  auto put_sums = [&](auto add) {
+    float* part = sm + (PSMEM ? 3 * D : 0);
+#pragma unroll
+    for (int q = 0; q < VPT; ++q) {
+      if (!act[q]) continue;
+      float* t = part + static_cast<size_t>(grp) * 3 * D + col[q];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        auto put = [&](float* at, uint64_t& a, uint64_t& b) {
+          ulonglong2 v = make_ulonglong2(a, b);
+          if constexpr (decltype(add)::value) {
+            const ulonglong2 o = *reinterpret_cast<const ulonglong2*>(at);
+            v = make_ulonglong2(f2_add(a, o.x), f2_add(b, o.y));
+            a = b = 0ull;
+          }
+          *reinterpret_cast<ulonglong2*>(at) = v;
+        };
+        put(t + 4 * h, a_sc[q][2 * h], a_sc[q][2 * h + 1]);
+        put(t + D + 4 * h, a_sh[q][2 * h], a_sh[q][2 * h + 1]);
+        put(t + 2 * D + 4 * h, a_w[q][2 * h], a_w[q][2 * h + 1]);
+      }
+    }
+  };
+  if constexpr (F32) put_sums(std::false_type{});    // zeros
+  [[maybe_unused]] int rows_in_sum = 0;
+  constexpr int GV = F32 ? 2 : 1;                  // 16-byte vectors of eight gradient columns
+  uint4 nx[RPI][VPT], ng[RPI][VPT][GV], nr[RPI][VPT];
 #pragma unroll
   for (int k = 0; k < RPI; ++k)
 #pragma unroll
-    for (int q = 0; q < VPT; ++q) nx[k][q] = ng[k][q] = nr[k][q] = make_uint4(0u, 0u, 0u, 0u);
+    for (int q = 0; q < VPT; ++q) {
+      nx[k][q] = nr[k][q] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+      for (int e = 0; e < GV; ++e) ng[k][q][e] = make_uint4(0u, 0u, 0u, 0u);
+    }
+  // gradient columns 2 i and 2 i + 1 of a vector
+  auto grad_pair = [](const uint4 (&g)[GV], int i) -> uint64_t {
+    if constexpr (F32) {
+      const uint4& h = g[i >> 1];
+      return (i & 1) ? f2_pack(__uint_as_float(h.z), __uint_as_float(h.w))
+                     : f2_pack(__uint_as_float(h.x), __uint_as_float(h.y));
+    } else {
+      return f2_from_bf16x2(i == 0 ? g[0].x : i == 1 ? g[0].y : i == 2 ? g[0].z : g[0].w);
+    }
+  };
   auto fetch = [&](int base) {
 #pragma unroll
     for (int k = 0; k < RPI; ++k) {
@@ -590,7 +646,8 @@ modnorm_bwd_group_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
         if (act[q] && r < rows) {
           const size_t off = static_cast<size_t>(r) * D + col[q];
           nx[k][q] = *reinterpret_cast<const uint4*>(x + off);
-          ng[k][q] = *reinterpret_cast<const uint4*>(dh + off);
+#pragma unroll
+          for (int e = 0; e < GV; ++e) ng[k][q][e] = reinterpret_cast<const uint4*>(dh + off)[e];
           if (dres) nr[k][q] = *reinterpret_cast<const uint4*>(dres + off);
         }
       }
@@ -599,11 +656,16 @@ modnorm_bwd_group_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
   const int first = blockIdx.x * groups + grp;
   if (first < rows) fetch(first);
   for (int base = first; base < rows; base += stride, parity ^= 1) {
-    uint4 cx[RPI][VPT], cg[RPI][VPT], cr[RPI][VPT];
+    uint4 cx[RPI][VPT], cg[RPI][VPT][GV], cr[RPI][VPT];
 #pragma unroll
     for (int k = 0; k < RPI; ++k)
 #pragma unroll
-      for (int q = 0; q < VPT; ++q) { cx[k][q] = nx[k][q]; cg[k][q] = ng[k][q]; cr[k][q] = nr[k][q]; }
+      for (int q = 0; q < VPT; ++q) {
+        cx[k][q] = nx[k][q];
+        cr[k][q] = nr[k][q];
+#pragma unroll
+        for (int e = 0; e < GV; ++e) cg[k][q][e] = ng[k][q][e];
+      }
     if (base + stride < rows) fetch(base + stride);
     // ---- the two row sums of each row: mode 0  sum y^2, sum y (g w);  mode 1  sum x^2, sum x (g (1 + sc) w)
     uint64_t p0[RPI], p1[RPI];
@@ -615,12 +677,11 @@ modnorm_bwd_group_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
 #pragma unroll
       for (int k = 0; k < RPI; ++k) {
         const uint32_t xw[4] = {cx[k][q].x, cx[k][q].y, cx[k][q].z, cx[k][q].w};
-        const uint32_t gw[4] = {cg[k][q].x, cg[k][q].y, cg[k][q].z, cg[k][q].w};
         const bool live = act[q] && base + k * gstep < rows;
         uint64_t s0 = 0ull, s1 = 0ull;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const uint64_t v = f2_from_bf16x2(xw[i]), g = f2_from_bf16x2(gw[i]);
+          const uint64_t v = f2_from_bf16x2(xw[i]), g = grad_pair(cg[k][q], i);
           if (mode == 0) {
             const uint64_t y = f2_fma(v, p_sc[q][i], p_sh[q][i]);
             s0 = f2_fma(y, y, s0);
@@ -655,12 +716,11 @@ modnorm_bwd_group_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
         const float ncoef = -rinv * rinv * rinv * (s[2 * k + 1] * inv_d);
         const uint64_t rinv2 = f2_pack(rinv, rinv), ncoef2 = f2_pack(ncoef, ncoef);
         const uint32_t xw[4] = {cx[k][q].x, cx[k][q].y, cx[k][q].z, cx[k][q].w};
-        const uint32_t gw[4] = {cg[k][q].x, cg[k][q].y, cg[k][q].z, cg[k][q].w};
         const uint32_t dw4[4] = {cr[k][q].x, cr[k][q].y, cr[k][q].z, cr[k][q].w};
         uint32_t ow[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const uint64_t v = f2_from_bf16x2(xw[i]), g = f2_from_bf16x2(gw[i]);
+          const uint64_t v = f2_from_bf16x2(xw[i]), g = grad_pair(cg[k][q], i);
           if (mode == 0) {
             const uint64_t y = f2_fma(v, p_sc[q][i], p_sh[q][i]);
             const uint64_t dy = f2_fma(ncoef2, y, f2_mul(rinv2, f2_mul(g, p_w[q][i])));
@@ -681,26 +741,26 @@ modnorm_bwd_group_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
         *reinterpret_cast<uint4*>(dx + static_cast<size_t>(r) * D + col[q]) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
       }
     }
-  }
-  // ---- column sums: [group][3][D] in shared memory, added up and handed to memory by the whole CTA
-  float* part = sm + (PSMEM ? 3 * D : 0);
-#pragma unroll
-  for (int q = 0; q < VPT; ++q) {
-    if (!act[q]) continue;
-    float* t = part + static_cast<size_t>(grp) * 3 * D + col[q];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      *reinterpret_cast<ulonglong2*>(t + 4 * h) = make_ulonglong2(a_sc[q][2 * h], a_sc[q][2 * h + 1]);
-      *reinterpret_cast<ulonglong2*>(t + D + 4 * h) = make_ulonglong2(a_sh[q][2 * h], a_sh[q][2 * h + 1]);
-      *reinterpret_cast<ulonglong2*>(t + 2 * D + 4 * h) = make_ulonglong2(a_w[q][2 * h], a_w[q][2 * h + 1]);
+    if constexpr (F32) {
+      if ((rows_in_sum += RPI) == SUM_ROWS) {
+        put_sums(std::true_type{});
+        rows_in_sum = 0;
+      }
     }
   }
+  // ---- column sums, added up and handed to memory by the whole CTA
+  put_sums(std::bool_constant<F32>{});
+  const float* part = sm + (PSMEM ? 3 * D : 0);
   __syncthreads();
   for (int i = threadIdx.x * 4; i < 3 * D; i += blockDim.x * 4) {
     float4 v = *reinterpret_cast<const float4*>(part + i);
     for (int g = 1; g < groups; ++g) {
       const float4 u = *reinterpret_cast<const float4*>(part + static_cast<size_t>(g) * 3 * D + i);
       v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+    }
+    if constexpr (F32) {
+      *reinterpret_cast<float4*>(dscale + static_cast<size_t>(blockIdx.x) * 3 * D + i) = v;
+      continue;
     }
     const int which = i / D, c = i - which * D;          // D is a multiple of 8: the four columns share one target
     float* dst = which == 0 ? dscale : which == 1 ? dshift : dw;
@@ -713,6 +773,25 @@ modnorm_bwd_group_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
       atomicAdd(dst, v.x); atomicAdd(dst + 1, v.y); atomicAdd(dst + 2, v.z); atomicAdd(dst + 3, v.w);
     }
   }
+}
+
+// Adds the rows of `sums` [n, 3, D] up in double and adds the result to dscale, dshift and dw: 32 columns a block, every
+// warp takes each eighth row.
+__global__ void __launch_bounds__(256) column_sums_kernel(const float* __restrict__ sums, int n, int D,
+                                                          float* __restrict__ dscale, float* __restrict__ dshift,
+                                                          float* __restrict__ dw) {
+  __shared__ double part[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+  double v = 0.;
+  if (i < 3 * D)
+    for (int r = warp; r < n; r += 8) v += sums[static_cast<size_t>(r) * 3 * D + i];
+  part[warp][lane] = v;
+  __syncthreads();
+  if (warp || i >= 3 * D) return;
+  for (int k = 1; k < 8; ++k) v += part[k][lane];
+  const int which = i / D;
+  float* dst = (which == 0 ? dscale : which == 1 ? dshift : dw) + (i - which * D);
+  *dst = static_cast<float>(*dst + v);
 }
 
 // ------------------------------------------------------------------------------------------------ row gather
@@ -1109,31 +1188,71 @@ extern "C" int aeris_modnorm_fwd_batch(const void* x, const void* gidx, const vo
   return 0;
 }
 
+// h (fp32) = (RMSNorm(x) * w) * (1 + scale) + shift (or the other order) for `batch` samples of `rows` rows: what the fp32
+// output head of the objectives without a fused loss multiplies. Rows of at most 5120 columns.
+extern "C" int aeris_modnorm_fwd_f32(const void* x, const float* scale, const float* shift, const float* w_f32, float* h,
+                                     int batch, int rows, int D, int mode, float eps, void* stream) {
+  if (D % 8 || D > 5120 || rows <= 0 || batch <= 0 || batch > 65535 || !w_f32) return -1;
+  const int nt = row_threads(D), per_sm = nt > 320 ? 1 : nt > 192 ? 2 : 576 / nt;
+  int grid = (rows + FWD_RPI - 1) / FWD_RPI;
+  const int cap = (aeris_num_sms() * per_sm + batch - 1) / batch;
+  if (grid > cap) grid = cap;
+  auto kern = nt <= 192 ? modnorm_fwd_pair_kernel<192, 3, 1, true>
+            : nt <= 320 ? modnorm_fwd_pair_kernel<320, 2, 2, true> : modnorm_fwd_pair_kernel<640, 1, 3, true>;
+  kern<<<dim3(grid, batch), nt, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+      reinterpret_cast<const __nv_bfloat16*>(x), nullptr, PeerPtrs{}, nullptr, scale, shift, nullptr, h, rows, D, mode, eps,
+      w_f32, nullptr);
+  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+}
+
+template <bool F32>
+static int launch_modnorm_bwd_group(const void* x, const void* dh, const void* dres, const float* scale, const float* shift,
+                                    const void* w, void* dx, float* dscale, float* dshift, float* dw, int rows, int D,
+                                    int mode, float eps, const float* w_f32, void* stream, float* sums = nullptr,
+                                    int sum_rows = 0) {
+  // one group of nt threads per row; CTAs of at most 384 (320) threads, one per SM
+  const int vpt = D <= 1536 ? 1 : 2, maxt = vpt == 1 ? 384 : 320;
+  const int nt = (D / 8 + vpt * 32 - 1) / (vpt * 32) * 32;
+  const int groups = maxt / nt;
+  const int smem = (groups + (vpt > 1 ? 1 : 0)) * 3 * D * 4;
+  const int need = (rows + groups - 1) / groups;
+  const int most = F32 && sum_rows < aeris_num_sms() ? sum_rows : aeris_num_sms();
+  const int grid = need < most ? need : most;
+  const uintptr_t sums_at = reinterpret_cast<uintptr_t>(dscale) | reinterpret_cast<uintptr_t>(dshift) |
+                         reinterpret_cast<uintptr_t>(dw);
+  const int vec = (sums_at & 15) == 0;
+  auto kern = vpt == 1 ? modnorm_bwd_group_kernel<1, 2, 384, F32> : modnorm_bwd_group_kernel<2, 1, 320, F32>;
+  if (smem > 32 * 1024 &&
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess)
+    return -20;
+  kern<<<grid, groups * nt, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
+      reinterpret_cast<const __nv_bfloat16*>(x),
+      reinterpret_cast<const std::conditional_t<F32, float, __nv_bfloat16>*>(dh),
+      reinterpret_cast<const __nv_bfloat16*>(dres), scale, shift, reinterpret_cast<const __nv_bfloat16*>(w),
+      reinterpret_cast<__nv_bfloat16*>(dx), F32 ? sums : dscale, dshift, dw, rows, D, mode, eps, w_f32, nt, vec);
+  if constexpr (F32)
+    column_sums_kernel<<<(3 * D + 31) / 32, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(sums, grid, D, dscale, dshift,
+                                                                                              dw);
+  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+}
+
+// Backward of aeris_modnorm_fwd_f32 for one sample, dh fp32: dx (bf16) written, dscale, dshift and dw added to. `sums`:
+// scratch of sum_rows * 3 * D values, 16-byte aligned; at most sum_rows CTAs run.
+extern "C" int aeris_modnorm_bwd_f32(const void* x, const float* dh, const float* scale, const float* shift,
+                                     const float* w_f32, void* dx, float* dscale, float* dshift, float* dw, float* sums,
+                                     int sum_rows, int rows, int D, int mode, float eps, void* stream) {
+  if (D % 8 || D > 5120 || rows <= 0 || sum_rows <= 0 || !w_f32 || !dscale || !dshift || !dw || !sums) return -1;
+  return launch_modnorm_bwd_group<true>(x, dh, nullptr, scale, shift, nullptr, dx, dscale, dshift, dw, rows, D, mode, eps,
+                                        w_f32, stream, sums, sum_rows);
+}
+
 extern "C" int aeris_modnorm_bwd(const void* x, const void* dh, const void* dres, const float* scale,
                                  const float* shift, const void* w, void* dx, float* dscale, float* dshift,
                                  float* dw, int rows, int D, int mode, float eps, const float* w_f32, void* stream) {
   if (D % 8 || D > 8192 || rows <= 0 || (!w && !w_f32)) return -1;
-  if (D <= 5120) {
-    // one group of nt threads per row; CTAs of at most 384 (320) threads, one per SM
-    const int vpt = D <= 1536 ? 1 : 2, maxt = vpt == 1 ? 384 : 320;
-    const int nt = (D / 8 + vpt * 32 - 1) / (vpt * 32) * 32;
-    const int groups = maxt / nt;
-    const int smem = (groups + (vpt > 1 ? 1 : 0)) * 3 * D * 4;
-    const int need = (rows + groups - 1) / groups;
-    const int grid = need < aeris_num_sms() ? need : aeris_num_sms();
-    const uintptr_t sums = reinterpret_cast<uintptr_t>(dscale) | reinterpret_cast<uintptr_t>(dshift) |
-                           reinterpret_cast<uintptr_t>(dw);
-    const int vec = (sums & 15) == 0;
-    auto kern = vpt == 1 ? modnorm_bwd_group_kernel<1, 2, 384> : modnorm_bwd_group_kernel<2, 1, 320>;
-    if (smem > 32 * 1024 &&
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess)
-      return -20;
-    kern<<<grid, groups * nt, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
-        reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(dh),
-        reinterpret_cast<const __nv_bfloat16*>(dres), scale, shift, reinterpret_cast<const __nv_bfloat16*>(w),
-        reinterpret_cast<__nv_bfloat16*>(dx), dscale, dshift, dw, rows, D, mode, eps, w_f32, nt, vec);
-    return cudaGetLastError() == cudaSuccess ? 0 : -21;
-  }
+  if (D <= 5120)
+    return launch_modnorm_bwd_group<false>(x, dh, dres, scale, shift, w, dx, dscale, dshift, dw, rows, D, mode, eps, w_f32,
+                                           stream);
   int rpc = pick_rows_per_cta(rows);
   if (rpc < 16) rpc = rows < 16 ? rows : 16;  // amortise the atomic flush of the column sums
   const int grid = (rows + rpc - 1) / rpc;    // every CTA takes about rpc rows, interleaved with the others

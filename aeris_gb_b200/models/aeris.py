@@ -484,10 +484,46 @@ class _HeadFn(torch.autograd.Function):
     STEP = 1 << 16
 
     @staticmethod
+    def _kernels(x, shift, scale, norm_w, head_w) -> bool:
+        """Whether the norm runs on the fp32 modulate + norm kernels, which read the bf16 stream once per pass: a stream of
+        whole 16-byte vectors, rows of at most 5120 columns (what the backward kernel takes) and fp32 parameters. The
+        products with the head are fp32 matrix products either way. Forward and backward of 28,800 rows of 512 columns
+        0.49 ms, against 1.50 ms on PyTorch's elementwise kernels; of 1536 columns 0.96 / 3.68, of 5120 2.94 / 11.0."""
+        D = x.shape[1]
+        return (use_fused(x) and x.dtype == torch.bfloat16 and x.numel() > 0 and D % 8 == 0 and D <= 5120
+                and x.is_contiguous() and x.data_ptr() % 16 == 0 and norm_w.is_contiguous() and norm_w.data_ptr() % 16 == 0
+                and shift.shape == scale.shape
+                and all(t.dtype == torch.float32 and t.device == x.device for t in (shift, scale, norm_w, head_w)))
+
+    @staticmethod
+    def _rows_of(t: torch.Tensor) -> torch.Tensor:
+        """``t`` [B, D] as the kernels read it: without gaps (``shift`` and ``scale`` are halves of one tensor), aligned."""
+        t = t.contiguous()
+        return t if t.data_ptr() % 16 == 0 else t.clone()
+
+    @staticmethod
+    def _pieces(B: int, rows: int) -> list[tuple[int, slice]]:
+        """(sample, its rows of the stream) of every piece."""
+        return [(b, slice(b * rows + r, b * rows + min(rows, r + _HeadFn.STEP)))
+                for b in range(B) for r in range(0, rows, _HeadFn.STEP)]
+
+    @staticmethod
     def forward(ctx, x, shift, scale, norm_w, head_w, stage):
         B = shift.shape[0]
         rows = x.shape[0] // B
         out = torch.empty((x.shape[0], head_w.shape[0]), dtype=head_w.dtype, device=x.device)
+        ctx.kernels = _HeadFn._kernels(x, shift, scale, norm_w, head_w)
+        if ctx.kernels:
+            from ..ops import elementwise as E
+            sc, sh = _HeadFn._rows_of(scale), _HeadFn._rows_of(shift)
+            for b, sl in _HeadFn._pieces(B, rows):
+                y = torch.empty(x[sl].shape, dtype=torch.float32, device=x.device)
+                E.modnorm_fwd_f32(x[sl], sc[b:b + 1], sh[b:b + 1], norm_w, mode=E.MODE_NORM_THEN_MOD,
+                                  eps=stage.cfg.eps(stage.cfg.data_dtype), out=y)
+                torch.mm(y, head_w.t(), out=out[sl])
+            ctx.stage = stage
+            ctx.save_for_backward(x, shift, scale, norm_w, head_w)
+            return out
         with torch.no_grad():
             for b in range(B):
                 for r in range(0, rows, _HeadFn.STEP):
@@ -503,9 +539,25 @@ class _HeadFn(torch.autograd.Function):
         stage = ctx.stage
         B = shift.shape[0]
         rows = x.shape[0] // B
+        dnw, dhw = torch.zeros_like(norm_w), torch.zeros_like(head_w)
+        if ctx.kernels:
+            from ..ops import elementwise as E
+            kw = dict(mode=E.MODE_NORM_THEN_MOD, eps=stage.cfg.eps(stage.cfg.data_dtype))
+            # a saved-tensor hook may hand back other strides
+            xs, nw, sc, sh = (_HeadFn._rows_of(t) for t in (x, norm_w, scale, shift))
+            dx = torch.empty_like(xs)
+            dshift, dscale = x.new_zeros(shift.shape, dtype=shift.dtype), x.new_zeros(scale.shape, dtype=scale.dtype)
+            with torch.no_grad():
+                for b, sl in _HeadFn._pieces(B, rows):
+                    y = torch.empty(x[sl].shape, dtype=torch.float32, device=x.device)
+                    E.modnorm_fwd_f32(xs[sl], sc[b:b + 1], sh[b:b + 1], nw, out=y, **kw)
+                    dhw.addmm_(dout[sl].t(), y)
+                    dy = torch.mm(dout[sl], head_w, out=y)
+                    E.modnorm_bwd_f32(xs[sl], dy, sc[b], sh[b], nw, dx=dx[sl], dscale=dscale[b], dshift=dshift[b], dw=dnw,
+                                      **kw)
+            return dx, dshift, dscale, dnw, dhw, None
         dx = torch.empty_like(x)
         dshift, dscale = torch.zeros_like(shift), torch.zeros_like(scale)
-        dnw, dhw = torch.zeros_like(norm_w), torch.zeros_like(head_w)
         for b in range(B):
             for r in range(0, rows, _HeadFn.STEP):
                 sl = slice(b * rows + r, b * rows + min(rows, r + _HeadFn.STEP))

@@ -56,6 +56,28 @@ def modnorm_bwd(x: torch.Tensor, dh: torch.Tensor, dres: torch.Tensor | None, sc
     return dx
 
 
+def modnorm_fwd_f32(x: torch.Tensor, scale: torch.Tensor, shift: torch.Tensor, w: torch.Tensor, *, mode: int, eps: float,
+                    out: torch.Tensor) -> torch.Tensor:
+    """:func:`modnorm_fwd` with an fp32 result ``out`` [rows, D]; ``w`` fp32, ``scale`` and ``shift`` [batch, D]."""
+    B, D = scale.shape
+    rc = _l.lib().aeris_modnorm_fwd_f32(_l.ptr(x), _l.ptr(scale), _l.ptr(shift), _l.ptr(w), _l.ptr(out), B,
+                                        x.shape[0] // B, D, mode, _l._c_float(eps), _l.stream_ptr())
+    _l.check(rc, "aeris_modnorm_fwd_f32")
+    return out
+
+
+def modnorm_bwd_f32(x: torch.Tensor, dh: torch.Tensor, scale: torch.Tensor, shift: torch.Tensor, w: torch.Tensor, *,
+                    mode: int, eps: float, dx: torch.Tensor, dscale: torch.Tensor, dshift: torch.Tensor,
+                    dw: torch.Tensor) -> None:
+    """Backward of :func:`modnorm_fwd_f32` for one sample, ``dh`` fp32; ``dscale``, ``dshift`` and ``dw`` are added to."""
+    rows, D = x.shape
+    sums = torch.empty((148, 3, D), dtype=torch.float32, device=x.device)      # one row per CTA, one CTA per SM
+    rc = _l.lib().aeris_modnorm_bwd_f32(_l.ptr(x), _l.ptr(dh), _l.ptr(scale), _l.ptr(shift), _l.ptr(w), _l.ptr(dx),
+                                        _l.ptr(dscale), _l.ptr(dshift), _l.ptr(dw), _l.ptr(sums), sums.shape[0], rows, D,
+                                        mode, _l._c_float(eps), _l.stream_ptr())
+    _l.check(rc, "aeris_modnorm_bwd_f32")
+
+
 def set_gather_bounds(src_rows: int) -> bool:
     """Checking build (AERIS_BOUNDS_CHECK=1) only: rows of the source buffers of the gathers launched next, so that
     every table entry is validated on the device. Returns whether the loaded library checks at all."""
