@@ -142,7 +142,8 @@ class StreamContext:
         fwd, bwd = self.table(src, dst, x.device), self.table(dst, src, x.device)
         if use_fused(x):
             from . import fused
-            return fused.Regroup.apply(x, fwd, bwd, self.peer_fn)
+            return (fused.Regroup.apply(x, fwd, bwd, self.peer_fn) if fused.recorded() else
+                    fused.Regroup.gather(x, fwd, self.peer_fn))
         if self.grid.n_ranks == 1:
             _, row = LY.decode_table(fwd)
             return x[row.to(x.device)]
@@ -318,8 +319,9 @@ class InputStage(nn.Module):
         """CUDA path from image-layout fields: x_img [B, hb, wb, C_out] (clean target when ``plan.noise``, else the
         noisy state), c_img [B, hb, wb, C_cond], cs [B, 2] = (cos t, sin t) (or (1, 0) when sampling). Noising,
         position encoding, window partition and the projection run in :mod:`.fused_io`."""
-        from . import fused_io
-        out = fused_io.EmbedFn.apply(x_img, c_img, cs, self.proj.weight, self.proj.bias, plan)
+        from . import fused, fused_io
+        args = (x_img, c_img, cs, self.proj.weight, self.proj.bias, plan)
+        out = fused_io.EmbedFn.apply(*args) if fused.recorded() else fused_io.embed(*args)
         return out, self.noise_embedding(t)
 
 
@@ -378,10 +380,12 @@ class SwinLayer(nn.Module):
         blocks = self.blocks()
         # plain blocks normalise first (there is nothing to modulate before the norm)
         after_mod_norm = cfg.after_mod_norm and cfg.conditioned
+        on_kernels = use_fused(x)
+        if on_kernels:
+            from . import fused
+            from ..ops import elementwise as E
         for j, (n1w, attn, n2w, ff, mod) in enumerate(blocks):
-            if use_fused(x):
-                from . import fused
-                from ..ops import elementwise as E
+            if on_kernels:
                 if ctx.grid.sp > 1 and ctx.sp_exchange is None:
                     raise RuntimeError("sequence parallelism on CUDA needs StreamContext.sp_exchange (fused.SPExchange)")
                 m = fused.modulation(mod.modulation, dt) if mod is not None else \

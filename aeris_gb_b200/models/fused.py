@@ -50,15 +50,18 @@ class Workspace:
     def __init__(self):
         self._buf: dict[str, torch.Tensor] = {}
 
-    def get(self, name: str, shape: tuple[int, ...], dtype: torch.dtype, device, zero: bool = False) -> torch.Tensor:
-        n = 1
-        for s in shape:
-            n *= s
+    def whole(self, name: str, shape: tuple[int, ...], dtype: torch.dtype, device) -> torch.Tensor:
+        """The buffer behind :meth:`get`, without the view of ``shape``: for callers that only pass its address on.
+        0.6 us of host time against 3.8, and a block asks for seven buffers forward and ten backward."""
+        n = math.prod(shape)
         b = self._buf.get(name)
         if b is None or b.numel() < n or b.dtype != dtype or b.device != torch.device(device):
             b = torch.empty(n, dtype=dtype, device=device)
             self._buf[name] = b
-        v = b[:n].view(*shape)
+        return b
+
+    def get(self, name: str, shape: tuple[int, ...], dtype: torch.dtype, device, zero: bool = False) -> torch.Tensor:
+        v = self.whole(name, shape, dtype, device)[:math.prod(shape)].view(*shape)
         if zero:
             v.zero_()
         return v
@@ -335,14 +338,16 @@ def block_forward(x: torch.Tensor, mod: torch.Tensor, meta: BlockMeta, wn1, wqkv
     ws, dev = _WS, x.device
     step = chunk_step(meta, D, F)
     spans = _forward_spans(meta, B, step, D, F, kept is not None)
+    weights = (wn1, wqkv, wo, wn2, w1, w2)
+    native = y.is_contiguous() and NB.takes(meta, x, mod, weights)
     if kept is None:
         cmax = max(nw for _, _, nw, _ in spans) * meta.L
         tpn = meta.tp.tp if meta.tp is not None else 1   # gathered rows x local features: the same element count
         shapes = _chunk_shapes(cmax, D, HD, meta.heads, F, tpn)
-        chunk_bufs = {k: ws.get(k, *sh, dev) for k, sh in shapes.items() if k != "h2"}
+        get = ws.whole if native else ws.get
+        chunk_bufs = {k: get(k, *sh, dev) for k, sh in shapes.items() if k != "h2"}
         chunk_bufs["h1"] = chunk_bufs["h2"] = chunk_bufs.pop("h")
-    weights = (wn1, wqkv, wo, wn2, w1, w2)
-    if y.is_contiguous() and NB.takes(meta, x, mod, weights):
+    if native:
         NB.forward(meta, x, mod, weights, y, step, spans[0][3] > 1,
                    {k: t.data_ptr() for k, t in (kept or chunk_bufs).items()}, kept is not None, gather)
         return y
@@ -398,12 +403,14 @@ def block_backward(x: torch.Tensor, mod: torch.Tensor, dy: torch.Tensor, meta: B
     cmax = step * meta.L
     tp = meta.tp
     tpn = tp.tp if tp is not None else 1
-    if kept is None:
-        chunk_bufs = {k: ws.get(k, *sh, dev) for k, sh in _chunk_shapes(cmax, D, HD, meta.heads, F, tpn).items()}
-        chunk_bufs["h1"], act_b = chunk_bufs.pop("h"), chunk_bufs["act"]
-    work = {k: ws.get(k, *sh, dev) for k, sh in _grad_shapes(cmax, D, HD, meta.heads, F, tpn).items()}
     weights = (wn1, wqkv, wo, wn2, w1, w2)
-    if NB.takes(meta, x, mod, (*weights, dy, *(() if dx is None else (dx,))), grads.values()):
+    native = NB.takes(meta, x, mod, (*weights, dy, *(() if dx is None else (dx,))), grads.values())
+    get = ws.whole if native else ws.get
+    if kept is None:
+        chunk_bufs = {k: get(k, *sh, dev) for k, sh in _chunk_shapes(cmax, D, HD, meta.heads, F, tpn).items()}
+        chunk_bufs["h1"], act_b = chunk_bufs.pop("h"), chunk_bufs["act"]
+    work = {k: get(k, *sh, dev) for k, sh in _grad_shapes(cmax, D, HD, meta.heads, F, tpn).items()}
+    if native:
         dx = torch.empty_like(x) if dx is None else dx
         dmod = torch.empty((B, 6 * D), dtype=f32, device=dev)
         addr = {"du" if k == "u" else k: t.data_ptr() for k, t in work.items()}
@@ -652,16 +659,16 @@ def modulation(seq: torch.nn.Sequential, emb: torch.Tensor) -> torch.Tensor:
     """The AdaLN modulation MLP ``[Linear,] SiLU, Linear`` (src/aeris/models/parallel_swin.py:321-325) on the GEMV kernel
     where that takes all rows of every layer (at most 8 samples), else on stock operators; fp32 result ``[B, out]``."""
     from ..ops import diffusion as DF
-    last = seq[-1]
+    first, *_, last = parts = list(seq)
     w = last.weight
     if not DF.gemv_ok(emb.shape[0], max(emb.shape[1], w.shape[1])):
         return seq(emb.to(w.dtype)).float()
-    if len(seq) == 3 and seq[0].bias is not None and last.bias is not None:
-        args = (emb, seq[0].weight, seq[0].bias, w, last.bias)
+    if len(parts) == 3 and first.bias is not None and last.bias is not None:
+        args = (emb, first.weight, first.bias, w, last.bias)
         return ModulationFn.apply(*args) if recorded() else DF.modulation_mlp(*args[1:3], emb, *args[3:])[1]
     x = emb
-    if len(seq) == 3:
-        x = GemvLinearFn.apply(x, seq[0].weight, seq[0].bias, False)
+    if len(parts) == 3:
+        x = GemvLinearFn.apply(x, first.weight, first.bias, False)
     return GemvLinearFn.apply(x, w, last.bias, True)
 
 
@@ -672,6 +679,10 @@ class Regroup(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, table_fwd, table_bwd, peer_fn):
         ctx.table_bwd, ctx.peer_fn = table_bwd, peer_fn
+        return Regroup.gather(x, table_fwd, peer_fn)
+
+    @staticmethod
+    def gather(x, table_fwd, peer_fn):
         out = torch.empty((table_fwd.numel(), x.shape[1]), dtype=x.dtype, device=x.device)
         peers = peer_fn(x, "fwd") if peer_fn is not None else [x.data_ptr()]
         E.gather_rows(table_fwd, peers, out, src_rows=x.shape[0])

@@ -71,26 +71,31 @@ def _pack_dim(c_in: int) -> int:
     return (3 * c_in + 2 + 127) // 128 * 128
 
 
-class EmbedFn(torch.autograd.Function):
+def embed(x_img, c_img, cs, W, b, plan: IoPlan) -> torch.Tensor:
     """``(cat[(cos t x + sin t z) / sigma_d, cond] + ape) W^T + b`` -> bf16 token stream in the unshifted window layout."""
+    D, Cin = W.shape
+    KP = _pack_dim(Cin)
+    dev = x_img.device
+    Wp = DF.pack_embed_weights(W.detach().float().contiguous(), b.detach().float().contiguous(), KP)
+    T = plan.geom.rows
+    out = torch.empty((T, D), dtype=torch.bfloat16, device=dev)
+    A = workspace().get("embed_a", (min(CHUNK_ROWS, T), KP), torch.bfloat16, dev)
+    for r0 in range(0, T, CHUNK_ROWS):
+        n = min(CHUNK_ROWS, T - r0)
+        DF.embed_pack(x_img, c_img, cs, plan.geom, plan.ape_y, plan.ape_x, plan.seed, plan.sigma_data,
+                      plan.noise, A[:n], row0=r0)
+        G.gemm(A[:n], Wp, out=out[r0:r0 + n])
+    return out
+
+
+class EmbedFn(torch.autograd.Function):
+    """:func:`embed` with the gradients of the weight and the bias."""
 
     @staticmethod
     def forward(ctx, x_img, c_img, cs, W, b, plan: IoPlan):
-        D, Cin = W.shape
-        KP = _pack_dim(Cin)
-        dev = x_img.device
-        Wp = DF.pack_embed_weights(W.detach().float().contiguous(), b.detach().float().contiguous(), KP)
-        T = plan.geom.rows
-        out = torch.empty((T, D), dtype=torch.bfloat16, device=dev)
-        A = workspace().get("embed_a", (min(CHUNK_ROWS, T), KP), torch.bfloat16, dev)
-        for r0 in range(0, T, CHUNK_ROWS):
-            n = min(CHUNK_ROWS, T - r0)
-            DF.embed_pack(x_img, c_img, cs, plan.geom, plan.ape_y, plan.ape_x, plan.seed, plan.sigma_data,
-                          plan.noise, A[:n], row0=r0)
-            G.gemm(A[:n], Wp, out=out[r0:r0 + n])
         ctx.plan = plan
         ctx.save_for_backward(x_img, c_img, cs, W, b)
-        return out
+        return embed(x_img, c_img, cs, W, b, plan)
 
     @staticmethod
     def backward(ctx, dout):
