@@ -7,10 +7,11 @@
 // Data layout: tokens are window-major, rows [w*N, (w+1)*N) belong to window w; Q, K, V are column slices of a
 // row-major [T, ld] bf16 tensor (the fused qkv projection output, columns ordered (q|k|v, head, d)).
 //
-// Roles are the same in every kernel: warp 0 = TMA producer, warp 1 = MMA issuer and TMEM owner, and warpgroups of math
+// Roles in the kernels of this file: warp 0 = TMA producer, warp 1 = MMA issuer and TMEM owner, and warpgroups of math
 // warps, one thread per tile row, that work straight out of TMEM. The forward kernel has one such group (warps 2..5 of 192
 // threads). The backward kernels have two or three from warp 4 on (384 or 512 threads); warps 2 and 3 fetch the row
-// statistics there.
+// statistics there. The forward kernel for windows of several query tiles (attention_fwd_pair.cuh) has its two softmax
+// groups first, then a producer warp and one issuer warp per group.
 #include "common.cuh"
 #include "api.h"
 #include "host.h"
@@ -613,12 +614,12 @@ __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
 }
 
 // Gradient rows on their way out: a warpgroup turns 32 accumulator columns of its 128 rows into bf16 in shared memory, one
-// thread hands them to the TMA unit as one tiled store. The accumulator is free once it has been read; written by the threads
-// themselves (one row each, 32 rows with every 16-byte store instruction) it kept the next item's products waiting. Rows
-// past the window's end and columns past the head's width are clipped by the tensor map. Both kernels, ms, before and now,
-// 12 heads x 128: 400 x 128 tokens 0.550 -> 0.464, 200 x 225 0.625 -> 0.546, 72 x 900 1.69 -> 1.60, 16 x 3600 4.45 -> 4.34. At
-// 64, with a third of the columns per warpgroup, the hand-shakes cost more than they save (24 x 64, 200 x 225: 0.650 ->
-// 0.704, 72 x 900 1.91 -> 1.92): direct stores there.
+// thread hands them to the TMA unit as one tiled store. The accumulator is free once it has been read; written by the
+// threads themselves (one row each, 32 rows with every 16-byte store instruction) it kept the next item's products waiting.
+// Rows past the window's end and columns past the head's width are clipped by the tensor map. Both kernels, ms, before and
+// now, 12 heads x 128: 400 x 128 tokens 0.550 -> 0.464, 200 x 225 0.625 -> 0.546, 72 x 900 1.69 -> 1.60, 16 x 3600 4.45 ->
+// 4.34. At 64, with a third of the columns per warpgroup, the hand-shakes cost more than they save (24 x 64, 200 x 225:
+// 0.650 -> 0.704, 72 x 900 1.91 -> 1.92): direct stores there.
 struct BwdOut {
   uint8_t* stage;           // this warpgroup's
   uint64_t *free_bar, *full_bar;
@@ -952,7 +953,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         for (int c = wg * 32; c < p.d; c += 32 * NWG) ++mine;
         if (mine == 0) release();
         for (int c = wg * 32; c < p.d; c += 32 * NWG)
-          if (!out.put(tdQ + lane_addr + c, sc, &tm_dq, c, w.head, w.tile * TILE, w.win, [&] { if (--mine == 0) release(); }))
+          if (!out.put(tdQ + lane_addr + c, sc, &tm_dq, c, w.head, w.tile * TILE, w.win,
+                       [&] { if (--mine == 0) release(); }))
             return false;
         return true;
       }
@@ -1505,10 +1507,10 @@ static int attn_fwd_impl(const void* q, int ldq, int q_col0, const void* k, int 
   int r;
   auto at = [](const void* base, int col) -> const void* { return reinterpret_cast<const __nv_bfloat16*>(base) + col; };
   if ((r = make_tmap_heads_bf16(&tq, at(q, q_col0), head_dim, H, N, n_win, ldq, TILE))) return r;
-  // Two query tiles at a time where there are two; its masked columns need a positive scale. Three or five tiles of which the
-  // last is not full leave its second chain idle for a third or a fifth of the time: 64-wide heads are faster without then
-  // (one tile at a time / two, 24 x 64: 200 x 257 tokens 0.306 / 0.330 ms, 100 x 352 0.196 / 0.203, 64 x 520 0.264 / 0.275,
-  // 64 x 576 0.281 / 0.288; 100 x 384 0.208 / 0.198, 64 x 640 0.321 / 0.300, 32 x 1030 0.415 / 0.389), 128-wide ones are not
+  // Two query tiles at a time where there are two; its masked columns need a positive scale. Three or five tiles of which
+  // the last is not full leave its second chain idle for a third or a fifth of the time: 64-wide heads are faster without
+  // then (one tile at a time / two, 24 x 64: 200 x 257 tokens 0.306 / 0.330 ms, 100 x 352 0.196 / 0.203, 64 x 520 0.264 /
+  // 0.275, 64 x 576 0.281 / 0.288; 100 x 384 0.208 / 0.198, 64 x 640 0.321 / 0.300, 32 x 1030 0.415 / 0.389), 128-wide ones are not
   // (12 x 128: 200 x 257 0.256 / 0.237, 100 x 320 0.146 / 0.129, 64 x 576 0.218 / 0.201).
   const int q_tiles = (N + TILE - 1) / TILE, tail = N % TILE;
   const bool idle_chain = head_dim <= 64 && (q_tiles == 3 || q_tiles == 5) && tail > 0 && tail <= 96;

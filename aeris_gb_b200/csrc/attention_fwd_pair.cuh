@@ -8,9 +8,10 @@
 // of a tile (711 cycles by themselves) take 1,100-1,700, and waits, maximum and hand-over another 1,000.
 // Tensor memory: per chain 128 score columns, O, and P. At head_dim 64 P has columns of its own, so that the next scores are
 // computed under the softmax; at 128 it lies over the scores, whose successors then wait for P V, and the chains take turns.
-// Before and now (launches held for 0.15 s, ms, one B200), windows x tokens, heads x width: 72 x 900, 24 x 64: 0.695 -> 0.620;
-// 72 x 900, 12 x 128: 0.539 -> 0.484; 16 x 3600, 24 x 64: 2.00 -> 1.80; 16 x 3600, 12 x 128: 1.38 -> 1.26; 200 x 225, 24 x 64:
-// 0.210 -> 0.168; 200 x 225, 12 x 128: 0.188 -> 0.124; 400 x 135, 12 x 64: 0.150 -> 0.134; 8 x 900, 4 x 64: 0.0225 -> 0.0186.
+// Before and now (launches held for 0.15 s, ms, one B200), windows x tokens, heads x width: 72 x 900, 24 x 64: 0.695 ->
+// 0.620; 72 x 900, 12 x 128: 0.539 -> 0.484; 16 x 3600, 24 x 64: 2.00 -> 1.80; 16 x 3600, 12 x 128: 1.38 -> 1.26; 200 x 225,
+// 24 x 64: 0.210 -> 0.168; 200 x 225, 12 x 128: 0.188 -> 0.124; 400 x 135, 12 x 64: 0.150 -> 0.134; 8 x 900, 4 x 64: 0.0225
+// -> 0.0186.
 // Tried: one piece of straight code per full tile and a rolled loop for the last one (no gain at 900 tokens, 225: 0.168 ->
 // 0.190); strict turns of the two chains at the exponentials (0.620 -> 0.677); one warp for the products of both chains is
 // not needed: issuing a tile's twelve products and their commits takes 400 cycles of 3,000.

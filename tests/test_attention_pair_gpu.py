@@ -64,7 +64,8 @@ def test_forward_pushes_the_rows_to_their_owners(N, d, keep):
     lse = torch.empty_like(lref)
     arr = (ctypes.c_void_p * sp)(*[b.data_ptr() for b in bufs])
     rc = L.lib().aeris_attn_fwd_push(L.ptr(qkv), 3 * HD, H, L.ptr(o), HD, L.ptr(lse), nw, N, d,
-                                     ctypes.c_float(1 / math.sqrt(d)), arr, sp, n_loc, 2 * HD, HD, L.ptr(L.status_word()), L.stream_ptr())
+                                     ctypes.c_float(1 / math.sqrt(d)), arr, sp, n_loc, 2 * HD, HD, L.ptr(L.status_word()),
+                                     L.stream_ptr())
     assert rc == 0
     got = torch.stack([b.view(nw, n_loc, 2 * HD) for b in bufs], 1).reshape(nw * N, 2 * HD)
     assert torch.equal(got[:, HD:], ref) and float(got[:, :HD].abs().max()) == 0
