@@ -18,10 +18,11 @@ int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M, int N, in
                          void* stream);
 
 // The one of the two that is the faster for the shape (see gemm2.cu). bn: tile width of the one-CTA kernel (0: from N);
-// allow_2cta = 0: never the other.
+// allow_2cta = 0: never the other. ld_gate: elements from one gate row to the next (a multiple of 4; N where they lie
+// without gaps).
 int aeris_gemm_auto(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int a_mn,
-                    int b_mn, int epi, const void* resid, int ldr, const float* gate, int rows_per_gate, void* aux,
-                    int ld_aux, int swiglu_f, int k_splits, int bn, int allow_2cta, int* status, void* stream);
+                    int b_mn, int epi, const void* resid, int ldr, const float* gate, int rows_per_gate, int ld_gate,
+                    void* aux, int ld_aux, int swiglu_f, int k_splits, int bn, int allow_2cta, int* status, void* stream);
 
 int aeris_attn_fwd(const void* q, int ldq, int q_col0, const void* k, int ldk, int k_col0, const void* v, int ldv,
                    int v_col0, void* o, int ldo, float* lse, int n_win, int N, int H, int head_dim, float scale,
@@ -53,9 +54,10 @@ int aeris_attn_bwd_push(const void* qkv, int ld, int H_local, const void* o, con
 int aeris_modnorm_fwd(const void* x, const void* gidx, const void* const* peer_ptrs, int n_peers, void* x_out,
                       const float* scale, const float* shift, const void* w, void* h, int rows, int D, int mode,
                       float eps, const float* w_f32, void* h_lo, void* stream);
+// mod_stride: elements from one sample's scale (shift) to the next, a multiple of 4
 int aeris_modnorm_fwd_batch(const void* x, const void* gidx, const void* const* peer_ptrs, int n_peers, void* x_out,
-                            const float* scale, const float* shift, const void* w, void* h, int batch, int rows, int D,
-                            int mode, float eps, const float* w_f32, void* h_lo, void* stream);
+                            const float* scale, const float* shift, int mod_stride, const void* w, void* h, int batch,
+                            int rows, int D, int mode, float eps, const float* w_f32, void* h_lo, void* stream);
 int aeris_modnorm_bwd(const void* x, const void* dh, const void* dres, const float* scale, const float* shift,
                       const void* w, void* dx, float* dscale, float* dshift, float* dw, int rows, int D, int mode,
                       float eps, const float* w_f32, void* stream);

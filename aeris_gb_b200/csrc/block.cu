@@ -42,7 +42,7 @@ struct Gemm {
                  void* aux = nullptr, int ld_aux = 0, int k_splits = 1) const {
     const int f = epi == EPI_SWIGLU || epi == EPI_SWIGLU_BOTH ? N / 2 : epi == EPI_SWIGLU_BWD ? N : 0;
     return aeris_gemm_auto(A, B, C, M, N, K, a_t ? M : K, b_t ? N : K, ldc, a_t, b_t, epi, resid, ldr, gate, rows_per_gate,
-                           aux, ld_aux, f, k_splits, 0, b.two_cta, b.status, b.stream);
+                           static_cast<int>(b.mod_sample), aux, ld_aux, f, k_splits, 0, b.two_cta, b.status, b.stream);
   }
 };
 
@@ -72,8 +72,9 @@ bool modnorm(const AerisBlock& b, Run& run, int where, const bf16* x, const uint
   if (nb == 1)
     return run(where, aeris_modnorm_fwd(gx, table, b.peers, b.n_peers, x_out, scale, shift, w, h, rows, b.D, b.mode, b.eps,
                                         nullptr, nullptr, b.stream));
-  return run(where, aeris_modnorm_fwd_batch(gx, table, b.peers, b.n_peers, x_out, scale, shift, w, h, nb, rows / nb, b.D,
-                                            b.mode, b.eps, nullptr, nullptr, b.stream));
+  return run(where, aeris_modnorm_fwd_batch(gx, table, b.peers, b.n_peers, x_out, scale, shift,
+                                            static_cast<int>(b.mod_sample), w, h, nb, rows / nb, b.D, b.mode, b.eps, nullptr,
+                                            nullptr, b.stream));
 }
 
 bool rope(const AerisBlock& b, Run& run, int where, bf16* qkv, int rows, int inverse) {

@@ -335,7 +335,14 @@ extern "C" int aeris_choose_k_splits(int tiles, int kb_total, int units, int mos
 extern "C" int aeris_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb,
                                int ldc, int a_mn, int b_mn, int epi, const void* resid, int ldr,
                                const float* gate, int rows_per_gate, void* aux, int ld_aux, int swiglu_f,
-                               int k_splits, int bn, int* status, void* stream_) {
+                               int k_splits, int bn, int* status, void* stream) {
+  return gemm_one_cta(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, resid, ldr, gate, rows_per_gate, N, aux, ld_aux,
+                      swiglu_f, k_splits, bn, status, stream);
+}
+
+int aeris::gemm_one_cta(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int a_mn,
+                        int b_mn, int epi, const void* resid, int ldr, const float* gate, int rows_per_gate, int ld_gate,
+                        void* aux, int ld_aux, int swiglu_f, int k_splits, int bn, int* status, void* stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   if (M <= 0 || N <= 0 || K <= 0) return -1;
   if (bn != 128 && bn != 256) bn = (N % 256 == 0) ? 256 : 128;
@@ -349,7 +356,7 @@ extern "C" int aeris_gemm_bf16(const void* A, const void* B, void* C, int M, int
   GemmParams p{};
   p.M = M; p.N = N; p.K = K; p.epi = epi; p.C = C; p.ldc = ldc;
   p.resid = reinterpret_cast<const __nv_bfloat16*>(resid); p.ldr = ldr;
-  p.gate = gate; p.rows_per_gate = rows_per_gate > 0 ? rows_per_gate : M;
+  p.gate = gate; p.rows_per_gate = rows_per_gate > 0 ? rows_per_gate : M; p.ld_gate = ld_gate;
   p.aux = reinterpret_cast<__nv_bfloat16*>(aux); p.ld_aux = ld_aux;
   p.k_splits = k_splits; p.status = status; p.swiglu_f = swiglu_f;
   if (swiglu_fwd) {

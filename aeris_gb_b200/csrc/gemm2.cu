@@ -344,7 +344,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         } else if (r_ahead) {
           const bool row_ok = row < p.M;
           __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(row) * p.ldc + tn * G2_BN;
-          const float* gate = p.gate + static_cast<size_t>((row_ok ? row : 0) / p.rows_per_gate) * p.N + tn * G2_BN;
+          const float* gate = p.gate + static_cast<size_t>(min(row, p.M - 1) / p.rows_per_gate) * p.ld_gate + tn * G2_BN;
           const int c_hi = min((part + 1) * (G2_BN / 2), p.N - tn * G2_BN);
 #pragma unroll 1
           for (int c = part * (G2_BN / 2); c < c_hi; c += 64) {
@@ -441,10 +441,9 @@ using namespace aeris;
 
 // Same contract as aeris_gemm_bf16 (api.h); N must be a multiple of 128 (of 256 for the SwiGLU forward epilogues, whose
 // tiles pair gate and up columns).
-extern "C" int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb,
-                                    int ldc, int a_mn, int b_mn, int epi, const void* resid, int ldr,
-                                    const float* gate, int rows_per_gate, void* aux, int ld_aux, int swiglu_f,
-                                    int k_splits, int* status, void* stream_) {
+static int gemm_two_cta(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int a_mn,
+                        int b_mn, int epi, const void* resid, int ldr, const float* gate, int rows_per_gate, int ld_gate,
+                        void* aux, int ld_aux, int swiglu_f, int k_splits, int* status, void* stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   if (M <= 0 || N <= 0 || K <= 0) return -1;
   const bool swiglu_fwd = (epi == EPI_SWIGLU || epi == EPI_SWIGLU_BOTH);
@@ -455,7 +454,7 @@ extern "C" int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M
   GemmParams p{};
   p.M = M; p.N = N; p.K = K; p.epi = epi; p.C = C; p.ldc = ldc;
   p.resid = reinterpret_cast<const __nv_bfloat16*>(resid); p.ldr = ldr;
-  p.gate = gate; p.rows_per_gate = rows_per_gate > 0 ? rows_per_gate : M;
+  p.gate = gate; p.rows_per_gate = rows_per_gate > 0 ? rows_per_gate : M; p.ld_gate = ld_gate;
   p.aux = reinterpret_cast<__nv_bfloat16*>(aux); p.ld_aux = ld_aux;
   p.k_splits = k_splits; p.status = status; p.swiglu_f = swiglu_f; p.group_m = 8;
   {
@@ -497,19 +496,27 @@ extern "C" int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M
   return ew8 ? launch_gemm2<0, 0, 8>(ta, tb, p, stream) : launch_gemm2<0, 0, 4>(ta, tb, p, stream);
 }
 
+extern "C" int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb,
+                                    int ldc, int a_mn, int b_mn, int epi, const void* resid, int ldr,
+                                    const float* gate, int rows_per_gate, void* aux, int ld_aux, int swiglu_f,
+                                    int k_splits, int* status, void* stream) {
+  return gemm_two_cta(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, resid, ldr, gate, rows_per_gate, N, aux, ld_aux,
+                      swiglu_f, k_splits, status, stream);
+}
+
 // Which kernel takes a product. A last tile with 128 valid columns costs as much as a full one: 6 % at 2048 columns, far
 // less than the two-CTA kernel gains there (28800 x 13696 x 5120: 4.96 -> 3.38 ms), but 12150 x 1152 x 384 takes 43 us
 // instead of 38; the SwiGLU forward pairs gate and up columns of whole tiles.
 extern "C" int aeris_gemm_auto(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
                                int a_mn, int b_mn, int epi, const void* resid, int ldr, const float* gate,
-                               int rows_per_gate, void* aux, int ld_aux, int swiglu_f, int k_splits, int bn,
-                               int allow_2cta, int* status, void* stream) {
+                               int rows_per_gate, int ld_gate, void* aux, int ld_aux, int swiglu_f, int k_splits,
+                               int bn, int allow_2cta, int* status, void* stream) {
   const bool swiglu_fwd = (epi == EPI_SWIGLU || epi == EPI_SWIGLU_BOTH);
   if (allow_2cta && (N % G2_BN == 0 || (N % (G2_BN / 2) == 0 && N >= 2048 && !swiglu_fwd)))
-    return aeris_gemm_bf16_2cta(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, resid, ldr, gate, rows_per_gate, aux,
-                                ld_aux, swiglu_f, k_splits, status, stream);
-  return aeris_gemm_bf16(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, resid, ldr, gate, rows_per_gate, aux, ld_aux,
-                         swiglu_f, k_splits, bn, status, stream);
+    return gemm_two_cta(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, resid, ldr, gate, rows_per_gate, ld_gate, aux,
+                        ld_aux, swiglu_f, k_splits, status, stream);
+  return gemm_one_cta(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, resid, ldr, gate, rows_per_gate, ld_gate, aux,
+                      ld_aux, swiglu_f, k_splits, bn, status, stream);
 }
 
 // QKV (or dO) projection whose epilogue performs the Ulysses head<->sequence exchange: C is not written locally;

@@ -19,7 +19,7 @@ struct GemmParams {
   int ldc;
   const __nv_bfloat16* resid;  // EPI_GATE_RESID: out = resid + gate[col] * acc
   int ldr;
-  const float* gate;           // [M / rows_per_gate][N]
+  const float* gate;           // [M / rows_per_gate][N], rows of pitch ld_gate
   int rows_per_gate;
   __nv_bfloat16* aux;          // optional raw copy of acc (bf16) in EPI_GATE_RESID
   int ld_aux;
@@ -53,6 +53,7 @@ struct GemmParams {
   int group_m;      // two-CTA kernel: m-tiles per group of the tile order (<= 1: n fastest)
   int staged_out;   // bf16-output epilogues: move rows through the warp's shared-memory stage (coalesced global stores)
   int staged_red;   // split-K fp32 accumulation: stage 32 rows x 64 columns and issue the reductions row-contiguously
+  int ld_gate;
   int* status;
 };
 
@@ -459,7 +460,7 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
     const bool gated = (p.epi == EPI_GATE_RESID) && row_ok;
     const __nv_bfloat16* res = p.resid ? p.resid + static_cast<size_t>(row) * p.ldr + tn * BN : nullptr;
     const float* gate = nullptr;
-    if (gated) gate = p.gate + static_cast<size_t>(row / p.rows_per_gate) * p.N + tn * BN;
+    if (gated) gate = p.gate + static_cast<size_t>(row / p.rows_per_gate) * p.ld_gate + tn * BN;
     uint4 r4[4], r4n[4];       // residual of this and of the next 32 columns (requested one step ahead)
     if (gated && c_lo < c_hi) {
 #pragma unroll
@@ -507,7 +508,7 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
         p.resid ? p.resid + static_cast<size_t>(row) * p.ldr + tn * BN : nullptr;
     const float* gate = nullptr;
     if (p.epi == EPI_GATE_RESID && row_ok)
-      gate = p.gate + static_cast<size_t>(row / p.rows_per_gate) * p.N + tn * BN;
+      gate = p.gate + static_cast<size_t>(row / p.rows_per_gate) * p.ld_gate + tn * BN;
     __nv_bfloat16* aux = p.aux ? p.aux + static_cast<size_t>(row) * p.ld_aux + tn * BN : nullptr;
 #pragma unroll 1
     for (int c = c_lo; c < c_hi; c += 32) {

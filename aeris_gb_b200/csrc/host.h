@@ -16,4 +16,8 @@ int make_tmap_heads32_bf16(CUtensorMap* out, const void* base, int d, int heads,
 int num_sms();
 // Slices of an accumulating product's reduction over `kb_total` blocks of 64: see gemm.cu.
 int choose_k_splits(int tiles, int kb_total, int units, int most, int want);
+// aeris_gemm_bf16 (api.h) with gate rows of pitch `ld_gate`.
+int gemm_one_cta(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int a_mn, int b_mn,
+                 int epi, const void* resid, int ldr, const float* gate, int rows_per_gate, int ld_gate, void* aux,
+                 int ld_aux, int swiglu_f, int k_splits, int bn, int* status, void* stream);
 }  // namespace aeris

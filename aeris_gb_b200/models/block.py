@@ -66,14 +66,13 @@ def _issued(rc: int, what: str) -> None:
 
 
 def forward(meta, x, mod, weights, y, step: int, merged: bool, bufs: dict[str, int], kept: bool, gather=None) -> None:
-    """``mod`` [B, 6 D] fp32. ``gather``: see :func:`.fused.block_forward`."""
+    """``mod`` [B, 6 D] fp32, read in place: samples that run in one launch find their vectors 6 D apart. ``gather``: see :func:`.fused.block_forward`."""
     B, D, F = mod.shape[0], x.shape[1], weights[5].shape[1]
-    if merged and B > 1:              # every vector of all samples in a row
-        mod, vec, sample = mod.view(B, 6, D).transpose(0, 1).contiguous(), B * D, D
-    else:
-        mod, vec, sample = mod.contiguous(), D, 6 * D
+    mod = mod.contiguous()
+    if mod.data_ptr() % 16:               # the kernels read vectors of four
+        mod = mod.clone()
     a, alive = _args(meta, x, mod, B, D, F, step, weights, bufs, kept, _l.raw_stream())
-    a.mod_vec, a.mod_sample, a.merged, a.y = vec, sample, merged, y.data_ptr()
+    a.merged, a.y = merged, y.data_ptr()
     if gather is not None:
         table, peers, src = gather
         if E._CHECKED:

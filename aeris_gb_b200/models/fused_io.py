@@ -144,6 +144,16 @@ def _head_rows(x, scale, shift, norm_w, w3, eps, pred, y):
     return pred[:n]
 
 
+def _mod_rows(shift: torch.Tensor, scale: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+    """fp32 ``shift`` and ``scale`` [B, D] as the kernels read them: where they are (halves of one tensor) if their rows are
+    whole 16-byte vectors at the same pitch."""
+    shift, scale = shift.float(), scale.float()
+    if (shift.stride() == scale.stride() and shift.stride(1) == 1 and shift.stride(0) % 4 == 0
+            and shift.data_ptr() % 16 == 0 and scale.data_ptr() % 16 == 0):
+        return shift, scale
+    return shift.contiguous(), scale.contiguous()
+
+
 def _sample_chunks(B: int, rows_per_sample: int) -> list[tuple[int, int, int, int]]:
     """(first sample, samples, first row, rows) of every pass over the head: all samples at once where they fit one
     chunk, else chunks of one sample."""
@@ -165,7 +175,7 @@ def head_forward(x: torch.Tensor, shift: torch.Tensor, scale: torch.Tensor, norm
     cm = max(n for *_, n in spans)
     y = ws.get("head_y", (2, cm, D), torch.bfloat16, dev)
     pred = torch.empty((T, PAD_N), dtype=torch.float32, device=dev)
-    shift, scale = shift.float().contiguous(), scale.float().contiguous()
+    shift, scale = _mod_rows(shift, scale)
     for b, nb, r0, n in spans:
         _head_rows(x[r0:r0 + n], scale[b:b + nb], shift[b:b + nb], norm_w, w3, eps, pred[r0:r0 + n], y)
     return pred
@@ -189,7 +199,7 @@ class HeadLossFn(torch.autograd.Function):
         pred = ws.get("head_pred", (cm, PAD_N), torch.float32, dev)
         dpred = torch.empty((T, PAD_N), dtype=torch.bfloat16, device=dev)
         loss = torch.zeros(1, dtype=torch.float64, device=dev)
-        shift32, scale32 = shift.float().contiguous(), scale.float().contiguous()
+        shift32, scale32 = _mod_rows(shift, scale)
         inv_rows = 1.0 / (T // B)
         for b, nb, r0, n in spans:
             _head_rows(x[r0:r0 + n], scale32[b:b + nb], shift32[b:b + nb], norm_w, w3, plan.eps, pred, y)
@@ -213,7 +223,7 @@ class HeadLossFn(torch.autograd.Function):
         cm = max(n for *_, n in spans)
         y_hi, dy = ws.get("head_y", (2, cm, D), torch.bfloat16, dev).unbind(0)
         Gh = ws.get("head_g", (PAD_N, D), torch.float32, dev, zero=True)
-        shift32, scale32 = shift.float().contiguous(), scale.float().contiguous()
+        shift32, scale32 = _mod_rows(shift, scale)
         dshift, dscale = torch.zeros((2, *shift32.shape), dtype=torch.float32, device=dev).unbind(0)
         s_nw, r_nw = _grad_slot(norm_w)
         t_nw = _kernel_target(s_nw)

@@ -17,6 +17,13 @@ def _peer_array(ptrs: list[int]):
     return arr
 
 
+def _pitch(v: torch.Tensor, batch: int, D: int) -> int | None:
+    """Elements between the rows of ``v`` [batch, D], or None where the kernels cannot read it in place."""
+    if v.is_contiguous() and v.numel() == batch * D:
+        return D
+    return v.stride(0) if v.shape == (batch, D) and v.stride(1) == 1 and v.stride(0) % 4 == 0 else None
+
+
 def modnorm_fwd(x: torch.Tensor, scale: torch.Tensor | None, shift: torch.Tensor | None, w: torch.Tensor, *,
                 mode: int, eps: float, out: torch.Tensor | None = None, gather_idx: torch.Tensor | None = None,
                 peer_ptrs: list[int] | None = None, x_out: torch.Tensor | None = None,
@@ -24,7 +31,7 @@ def modnorm_fwd(x: torch.Tensor, scale: torch.Tensor | None, shift: torch.Tensor
                 src_rows: int | None = None, batch: int = 1) -> torch.Tensor:
     """``w`` bf16, or fp32 (the output head's norm); ``out_lo`` optionally receives ``h - bf16(h)``. ``src_rows``: rows of
     every peer buffer the gather table points into (used by the checking build only). ``batch`` > 1: the rows are that
-    many samples of equal length, ``scale`` and ``shift`` are [batch, D]."""
+    many samples of equal length, ``scale`` and ``shift`` are [batch, D], without gaps inside a row."""
     D = w.numel()
     rows = rows if rows is not None else (gather_idx.numel() if gather_idx is not None else x.shape[0])
     if _CHECKED and gather_idx is not None:
@@ -33,13 +40,16 @@ def modnorm_fwd(x: torch.Tensor, scale: torch.Tensor | None, shift: torch.Tensor
         out = torch.empty((rows, D), dtype=torch.bfloat16, device=w.device)
     peers = _peer_array(peer_ptrs) if gather_idx is not None else None
     w32, w = (w, None) if w.dtype == torch.float32 else (None, w)
-    assert batch == 1 or (rows % batch == 0 and all(v is None or (v.is_contiguous() and v.numel() == batch * D)
-                                                    for v in (scale, shift)))
+    stride = D
+    if batch > 1:
+        pitches = {_pitch(v, batch, D) for v in (scale, shift) if v is not None} or {D}
+        stride = pitches.pop()
+        assert rows % batch == 0 and stride is not None and not pitches
     head = (_l.ptr(x), _l.ptr(gather_idx), peers, len(peer_ptrs) if peer_ptrs else 0, _l.ptr(x_out), _l.ptr(scale),
-            _l.ptr(shift), _l.ptr(w), _l.ptr(out))
+            _l.ptr(shift))
     tail = (D, mode, _l._c_float(eps), _l.ptr(w32), _l.ptr(out_lo), _l.stream_ptr())
-    rc = (_l.lib().aeris_modnorm_fwd(*head, rows, *tail) if batch == 1 else
-          _l.lib().aeris_modnorm_fwd_batch(*head, batch, rows // batch, *tail))
+    rc = (_l.lib().aeris_modnorm_fwd(*head, _l.ptr(w), _l.ptr(out), rows, *tail) if batch == 1 else
+          _l.lib().aeris_modnorm_fwd_batch(*head, stride, _l.ptr(w), _l.ptr(out), batch, rows // batch, *tail))
     _l.check(rc, "aeris_modnorm_fwd")
     return out
 

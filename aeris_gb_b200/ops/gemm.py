@@ -65,7 +65,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
         two_cta = TWO_CTA_DEFAULT and bn == 0
     rc = _l.lib().aeris_gemm_auto(
         _l.ptr(a), _l.ptr(b), _l.ptr(out), M, N, K, _ld(a), _ld(b), _ld(out), int(a_t), int(b_t), epi,
-        _l.ptr(resid), _ld(resid) if resid is not None else 0, _l.ptr(gate), rows_per_gate,
+        _l.ptr(resid), _ld(resid) if resid is not None else 0, _l.ptr(gate), rows_per_gate, N,
         _l.ptr(aux), _ld(aux) if aux is not None else 0, swiglu_f, k_splits, bn, int(two_cta), _l.ptr(_l.status_word()),
         _l.stream_ptr())
     _l.check(rc, "aeris_gemm")
