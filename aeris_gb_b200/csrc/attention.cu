@@ -1507,20 +1507,28 @@ static int attn_fwd_impl(const void* q, int ldq, int q_col0, const void* k, int 
   int r;
   auto at = [](const void* base, int col) -> const void* { return reinterpret_cast<const __nv_bfloat16*>(base) + col; };
   if ((r = make_tmap_heads_bf16(&tq, at(q, q_col0), head_dim, H, N, n_win, ldq, TILE))) return r;
-  // Two query tiles at a time where there are two; its masked columns need a positive scale. Three or five tiles of which
-  // the last is not full leave its second chain idle for a third or a fifth of the time: 64-wide heads are faster without
-  // then (one tile at a time / two, 24 x 64: 200 x 257 tokens 0.306 / 0.330 ms, 100 x 352 0.196 / 0.203, 64 x 520 0.264 /
-  // 0.275, 64 x 576 0.281 / 0.288; 100 x 384 0.208 / 0.198, 64 x 640 0.321 / 0.300, 32 x 1030 0.415 / 0.389), 128-wide ones are not
-  // (12 x 128: 200 x 257 0.256 / 0.237, 100 x 320 0.146 / 0.129, 64 x 576 0.218 / 0.201).
-  const int q_tiles = (N + TILE - 1) / TILE, tail = N % TILE;
-  const bool idle_chain = head_dim <= 64 && (q_tiles == 3 || q_tiles == 5) && tail > 0 && tail <= 96;
-  if (q_tiles > 1 && !idle_chain && scale > 0.f && g_fwd_mode == 0 && g_fwd_poly == -1) {
+  // Two query tiles at a time where there are two; its masked columns need a positive scale. ms, windows x tokens, one tile
+  // at a time / two, 24 heads x 64 and 12 x 128:
+  // - Three or five tiles of which the last is not full leave the second chain idle for a third or a fifth of the time.
+  //   64-wide heads are faster without then (249 x 260 tokens 0.377 / 0.417, 202 x 320 0.347 / 0.364, 221 x 513 0.866 /
+  //   0.927, 175 x 576 0.743 / 0.813; full ones 168 x 384 0.348 / 0.332, 142 x 640 0.694 / 0.681; seven tiles 84 x 832 0.681
+  //   / 0.665, 97 x 772 0.734 / 0.750), 128-wide ones are not (249 x 260 0.306 / 0.295, 175 x 576 0.590 / 0.577).
+  // - A last half tile that is cut off (CUT) costs every tile: short windows only. 64: 240 tokens 0.302 / 0.246, 500 0.449 /
+  //   0.383, 740 0.728 / 0.685, 970 0.654 / 0.674, 1500 0.588 / 0.605, 3600 0.496 / 0.538. 128: 740 0.572 / 0.461, 1250
+  //   0.477 / 0.422, 1500 0.442 / 0.431, 2000 0.407 / 0.425, 3600 0.350 / 0.374.
+  const int q_tiles = (N + TILE - 1) / TILE;
+  const bool idle_chain = head_dim <= 64 && (q_tiles == 3 || q_tiles == 5) && N % TILE != 0;
+  const bool cut = N % KVT > 4, long_cut = cut && q_tiles > (head_dim > 64 ? 12 : 6);
+  if (q_tiles > 1 && !idle_chain && !long_cut && scale > 0.f && g_fwd_mode == 0 && g_fwd_poly == -1) {
     if ((r = make_tmap_heads_bf16(&tk, at(k, k_col0), head_dim, H, N, n_win, ldk, KVP))) return r;
     if ((r = make_tmap_heads_bf16(&tv, at(v, v_col0), head_dim, H, N, n_win, ldv, KVP))) return r;
     CUtensorMap to = tq;      // without a local output nothing is stored through it
     if (o && (r = make_tmap_heads_bf16(&to, o, head_dim, H, N, n_win, ldo, TILE))) return r;
-    return head_dim > 64 ? launch_attn_fwd_pair<2>(tq, tk, tv, to, p, stream)
-                         : launch_attn_fwd_pair<1>(tq, tk, tv, to, p, stream);
+    if (cut)
+      return head_dim > 64 ? launch_attn_fwd_pair<2, true>(tq, tk, tv, to, p, stream)
+                           : launch_attn_fwd_pair<1, true>(tq, tk, tv, to, p, stream);
+    return head_dim > 64 ? launch_attn_fwd_pair<2, false>(tq, tk, tv, to, p, stream)
+                         : launch_attn_fwd_pair<1, false>(tq, tk, tv, to, p, stream);
   }
   if ((r = make_tmap_heads_bf16(&tk, at(k, k_col0), head_dim, H, N, n_win, ldk, KVT))) return r;
   if ((r = make_tmap_heads_bf16(&tv, at(v, v_col0), head_dim, H, N, n_win, ldv, KVT))) return r;

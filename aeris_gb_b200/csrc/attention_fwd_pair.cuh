@@ -8,10 +8,11 @@
 // of a tile (711 cycles by themselves) take 1,100-1,700, and waits, maximum and hand-over another 1,000.
 // Tensor memory: per chain 128 score columns, O, and P. At head_dim 64 P has columns of its own, so that the next scores are
 // computed under the softmax; at 128 it lies over the scores, whose successors then wait for P V, and the chains take turns.
-// Before and now (launches held for 0.15 s, ms, one B200), windows x tokens, heads x width: 72 x 900, 24 x 64: 0.695 ->
-// 0.620; 72 x 900, 12 x 128: 0.539 -> 0.484; 16 x 3600, 24 x 64: 2.00 -> 1.80; 16 x 3600, 12 x 128: 1.38 -> 1.26; 200 x 225,
-// 24 x 64: 0.210 -> 0.168; 200 x 225, 12 x 128: 0.188 -> 0.124; 400 x 135, 12 x 64: 0.150 -> 0.134; 8 x 900, 4 x 64: 0.0225
-// -> 0.0186.
+// The output is that of attn_fwd_kernel in every bit (reference maximum and sums go by 64 columns as there) unless the
+// second half of a tile raises the reference maximum. Against one tile at a time, in turn under the power cap, ms, windows
+// x tokens, 24 heads x 64 / 12 x 128: 72 x 900 0.726 -> 0.667 / 0.548 -> 0.491; 253 x 256 0.298 -> 0.215 / 0.266 -> 0.161;
+// 288 x 225 0.309 -> 0.259 / 0.281 -> 0.180; 502 x 129 0.367 -> 0.327 / 0.301 -> 0.221; 55 x 1024 0.644 -> 0.549 / 0.483 ->
+// 0.399; 8 x 900, 4 x 64: 0.0226 -> 0.0202. Maximum and sum over whole tiles would save 1-2 %, and 5-10 % where CUT.
 // Tried: one piece of straight code per full tile and a rolled loop for the last one (no gain at 900 tokens, 225: 0.168 ->
 // 0.190); strict turns of the two chains at the exponentials (0.620 -> 0.677); one warp for the products of both chains is
 // not needed: issuing a tile's twelve products and their commits takes 400 cycles of 3,000.
@@ -49,22 +50,43 @@ __device__ __forceinline__ PairItem pair_item(int it, int n_pairs, int H) {
   return b;
 }
 
-// Probabilities of 32 scores of a row against the reference maximum: bf16 pairs into tensor memory, sums into acc.
-__device__ __forceinline__ void softmax_chunk(const uint32_t (&v)[32], uint64_t sl, uint64_t nm, uint64_t (&acc)[2],
-                                              uint32_t tP) {
+// Sum of 64 probabilities of a row in the order in which attn_fwd_kernel adds them up: four sums by column, or pair after
+// pair in a half tile that the window's end cuts off.
+struct HalfSum {
+  uint64_t by_col[2] = {0ull, 0ull};       // bit pattern of (0.f, 0.f)
+  float in_row = 0.f;
+
+  __device__ __forceinline__ float total(bool cut) const {
+    float s0, s1, s2, s3;
+    f2_unpack(by_col[0], s0, s1);
+    f2_unpack(by_col[1], s2, s3);
+    return cut ? in_row : (s0 + s1) + (s2 + s3);
+  }
+};
+
+// Probabilities of 32 scores of a row against the reference maximum: bf16 pairs into tensor memory, added to `sum`.
+template <bool IN_ROW>
+__device__ __forceinline__ void softmax_chunk(const uint32_t (&v)[32], uint64_t sl, uint64_t nm, HalfSum& sum, uint32_t tP) {
   uint32_t pk[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     float t0, t1;
     f2_unpack(f2_fma(f2_pack(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), sl, nm), t0, t1);
-        const uint64_t pr = f2_pack(fast_exp2(t0), fast_exp2(t1));
-    acc[i & 1] = f2_add(acc[i & 1], pr);
+    const float p0 = fast_exp2(t0), p1 = fast_exp2(t1);
+    const uint64_t pr = f2_pack(p0, p1);
+    if (IN_ROW)
+      sum.in_row += p0 + p1;
+    else
+      sum.by_col[i & 1] = f2_add(sum.by_col[i & 1], pr);
     pk[i] = f2_to_bf16x2(pr);
   }
   tmem_st16(tP, pk);
 }
 
-template <int DCH>
+// CUT: the window's last half tile has more than four but not all of its 64 columns (up to four come out the same in either
+// order of adding up). A kernel of its own: the code by its mere presence costs full tiles 8 % (72 x 900, 24 x 64: 0.635 ->
+// 0.701 ms; as a rolled loop over the cut columns or as a call it costs more).
+template <int DCH, bool CUT>
 __global__ void __launch_bounds__(AttnPair<DCH>::THREADS, 1)
 attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
@@ -411,23 +433,36 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 #pragma unroll
       for (int h = 0; h < 4; ++h) tmem_ld32(tS + 32 * h, v[h]);      // what lies past `cols` is not looked at
       tmem_wait_ld();
-      if constexpr (!P_OVER_S) arrive(&s_free[c]);
-      float mx[4];
+      if (!P_OVER_S) arrive(&s_free[c]);
+      // The reference maximum is raised as attn_fwd_kernel raises it, which sees 64 columns at a time: by the first half
+      // alone, unless the second exceeds that by 2^8 (then both halves take the second's). One vote serves a tile that does
+      // not raise it, the usual one.
+      auto row_max = [&](const uint32_t (&x)[32], const uint32_t (&y)[32], bool both) {
+        float mx[4];
 #pragma unroll
-      for (int h = 0; h < 4; ++h) {
-        if (h > 0 && cols <= 32 * h) break;
+        for (int k = 0; k < 4; ++k) mx[k] = fmaxf(__uint_as_float(x[k]), __uint_as_float(x[k + 4]));
 #pragma unroll
-        for (int i = 0; i < 32; i += 8) {
+        for (int i = 8; i < 32; i += 8) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const float x = __uint_as_float(v[h][i + k]), y = __uint_as_float(v[h][i + k + 4]);
-            mx[k] = h == 0 && i == 0 ? fmaxf(x, y) : max3(mx[k], x, y);
+          for (int k = 0; k < 4; ++k) mx[k] = max3(mx[k], __uint_as_float(x[i + k]), __uint_as_float(x[i + k + 4]));
+        }
+        if (both) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 8) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) mx[k] = max3(mx[k], __uint_as_float(y[i + k]), __uint_as_float(y[i + k + 4]));
           }
         }
-      }
-      const float m_new = fmaxf(m_ref, fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]) * sl2);
+        return fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]) * sl2;
+      };
+      const float max_1 = row_max(v[0], v[1], cols > 32);
+      float max_2 = -INFINITY;
+      if (cols > 64) max_2 = row_max(v[2], v[3], true);
       bool waited = P_OVER_S || j == 0;     // P_OVER_S: these scores were issued behind the P V of the tile before
-      if (__any_sync(0xffffffffu, m_new - m_ref > RESCALE_LOG2)) {
+      if (__any_sync(0xffffffffu, max3(m_ref, max_1, max_2) - m_ref > RESCALE_LOG2)) {
+        float m_new = fmaxf(m_ref, max_1);
+        if (!__any_sync(0xffffffffu, m_new - m_ref > RESCALE_LOG2)) m_new = m_ref;
+        if (__any_sync(0xffffffffu, max_2 - m_new > RESCALE_LOG2)) m_new = fmaxf(m_new, max_2);
         if (j > 0) {
           if (!waited && !wait_pv()) return false;
           waited = true;
@@ -440,21 +475,26 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const uint64_t nm = f2_pack(-m_ref, -m_ref);
       if (!waited && !wait_pv()) return false;
       if (!P_OVER_S && !their_half()) return false;
-      uint64_t acc[2] = {0ull, 0ull};       // bit pattern of (0.f, 0.f)
-      softmax_chunk(v[0], sl, nm, acc, tP);
-      if (cols > 32) softmax_chunk(v[1], sl, nm, acc, tP + 16);
+      const bool cut_1 = CUT && fill < 64, cut_2 = CUT && fill < KVP;
+      HalfSum sum_1, sum_2;
+      auto half = [&](const uint32_t (&x)[32], const uint32_t (&y)[32], bool both, bool cut, HalfSum& sum, uint32_t to) {
+        if (cut) {
+          softmax_chunk<true>(x, sl, nm, sum, to);
+          if (both) softmax_chunk<true>(y, sl, nm, sum, to + 16);
+        } else {
+          softmax_chunk<false>(x, sl, nm, sum, to);
+          if (both) softmax_chunk<false>(y, sl, nm, sum, to + 16);
+        }
+      };
+      half(v[0], v[1], cols > 32, cut_1, sum_1, tP);
       if (!P_OVER_S) my_half();
       if constexpr (P_OVER_S) {
         tmem_wait_st();
         arrive(&p_full[c]);
       }
-      if (cols > 64) {
-        softmax_chunk(v[2], sl, nm, acc, tP + 32);
-        softmax_chunk(v[3], sl, nm, acc, tP + 48);
-      }
-      float s0, s1;
-      f2_unpack(f2_add(acc[0], acc[1]), s0, s1);
-      l += s0 + s1;
+      if (cols > 64) half(v[2], v[3], true, cut_2, sum_2, tP + 32);
+      l += sum_1.total(cut_1);
+      l += sum_2.total(cut_2);
       tmem_wait_st();
       arrive(P_OVER_S ? &p_full2[c] : &p_full[c]);
       ++t;
@@ -491,11 +531,11 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   if (warp == 8) tmem_dealloc(tmem_base, 512);
 }
 
-template <int DCH>
+template <int DCH, bool CUT>
 static int launch_attn_fwd_pair(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                                 const CUtensorMap& to, const AttnFwdParams& p, cudaStream_t stream) {
   using R = AttnPair<DCH>;
-  auto kern = attn_fwd_pair_kernel<DCH>;
+  auto kern = attn_fwd_pair_kernel<DCH, CUT>;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, R::SMEM) != cudaSuccess) return -20;

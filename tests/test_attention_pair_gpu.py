@@ -39,6 +39,25 @@ def test_forward_at_the_edges_of_its_tiles(nw, N, H, d):
     assert float((wide[:, :8] - 7).abs().max()) == 0 and float((wide[:, 8 + H * d:] - 7).abs().max()) == 0
 
 
+@pytest.mark.parametrize("d", [64, 128, 40])
+@pytest.mark.parametrize("N", [129, 132, 133, 160, 225, 255, 256, 320, 384, 448, 700, 900, 1025])
+def test_forward_equals_the_kernel_that_sees_64_columns(N, d):
+    """Two query tiles at a time over 128 columns give what the kernel of one query tile over 64 columns gives, bit for bit,
+    as long as no row's maximum is raised in the second half of a tile (scores of N(0, 1) stay far below 2^8)."""
+    from aeris_gb_b200.ops import attention as A, lib as L
+    torch.manual_seed(N)
+    nw, H = 3, 60
+    qkv = torch.randn(nw * N, 3 * H * d, device=DEV).bfloat16()
+    o, lse = A.attn_fwd(qkv, nw, N, H, d)
+    assert L.lib().aeris_attn_set_fwd_variant(-1, 1) == 0        # the same arithmetic, one query tile at a time
+    try:
+        ref, lref = A.attn_fwd(qkv, nw, N, H, d)
+        torch.cuda.synchronize()
+    finally:
+        L.lib().aeris_attn_set_fwd_variant(-1, 0)
+    assert torch.equal(o, ref) and torch.equal(lse, lref)
+
+
 @pytest.mark.parametrize("N", [100, 300])
 @pytest.mark.parametrize("scale", [0.0, -0.1])
 def test_forward_with_a_scale_that_is_not_positive(N, scale):
