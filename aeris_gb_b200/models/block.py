@@ -43,6 +43,39 @@ def takes(meta, x: torch.Tensor, mod: torch.Tensor, weights, grads=()) -> bool:
             and all(_plain(g, torch.float32) for g in grads))
 
 
+WEIGHTS = ("n1", "to_qkv", "wo", "n2", "w1", "w2")
+
+
+def fits(meta, x: torch.Tensor, mod: torch.Tensor, weights, rows=(), grads=None, table=None) -> bool:
+    """Whether every operand has the extents that the native call derives from ``x``, ``w2`` and ``meta``: it has no other
+    check. ``rows``: tensors shaped like ``x``; ``grads``: as :func:`.fused.block_backward` takes them. What does not fit goes
+    launch by launch, where each is checked by itself."""
+    (T, D), F, HD, B = x.shape, weights[5].shape[1], meta.heads * meta.head_dim, mod.shape[0]
+    want = ((D,), (3 * HD, D), (D, HD), (D,), (2 * F, D), (D, F))
+    return (T == B * meta.n_win_per_sample * meta.L and mod.shape == (B, 6 * D)
+            and all(w.shape == s for w, s in zip(weights, want)) and all(r.shape == x.shape for r in rows)
+            and (grads is None or all(grads[k].shape == s for k, s in zip(WEIGHTS, want)))
+            and (table is None or table.numel() == T))
+
+
+def refuse_misfits(meta, x: torch.Tensor, mod: torch.Tensor, weights, dx=None, grads=None, table=None) -> None:
+    """Raises for the extents that no launch checks by itself, where kernels would read or write out of range."""
+    (T, D), need = x.shape, mod.shape[0] * meta.n_win_per_sample * meta.L
+    wrong = [k for k, w in zip(WEIGHTS, weights) if k in ("n1", "n2") and w.numel() != D]
+    if T < need:
+        wrong.append("x")
+    if mod.numel() < mod.shape[0] * 6 * D or (grads is not None and (mod.dim() != 2 or mod.shape[1] < 6 * D)):
+        wrong.append("mod")
+    if dx is not None and (dx.shape[0] < need or dx.shape[1] != D):
+        wrong.append("dx")
+    if grads is not None:
+        wrong += [f"grads[{k}]" for k, w in zip(WEIGHTS, weights) if grads[k].numel() != w.numel()]
+    if table is not None and table.numel() < T:
+        wrong.append("gather table")
+    if wrong:
+        raise ValueError(f"operands that do not fit a block of {T} rows of {D}: {', '.join(wrong)}")
+
+
 def _args(meta, x, mod, B, D, F, step, weights, bufs: dict[str, int], kept: bool, stream: int) -> tuple[BlockArgs, tuple]:
     """The arguments both directions share, and what has to live until the call returns. ``bufs``: addresses of internals."""
     wn1, wqkv, wo, wn2, w1, w2 = weights
@@ -66,7 +99,8 @@ def _issued(rc: int, what: str) -> None:
 
 
 def forward(meta, x, mod, weights, y, step: int, merged: bool, bufs: dict[str, int], kept: bool, gather=None) -> None:
-    """``mod`` [B, 6 D] fp32, read in place: samples that run in one launch find their vectors 6 D apart. ``gather``: see :func:`.fused.block_forward`."""
+    """``mod`` [B, 6 D] fp32, read in place: samples that run in one launch find their vectors 6 D apart. ``gather``: see
+    :func:`.fused.block_forward`."""
     B, D, F = mod.shape[0], x.shape[1], weights[5].shape[1]
     mod = mod.contiguous()
     if mod.data_ptr() % 16:               # the kernels read vectors of four

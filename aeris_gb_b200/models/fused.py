@@ -339,7 +339,10 @@ def block_forward(x: torch.Tensor, mod: torch.Tensor, meta: BlockMeta, wn1, wqkv
     step = chunk_step(meta, D, F)
     spans = _forward_spans(meta, B, step, D, F, kept is not None)
     weights = (wn1, wqkv, wo, wn2, w1, w2)
-    native = y.is_contiguous() and NB.takes(meta, x, mod, weights)
+    table = gather[0] if gather is not None else None
+    native = NB.takes(meta, x, mod, (*weights, y)) and NB.fits(meta, x, mod, weights, (y,), table=table)
+    if not native:
+        NB.refuse_misfits(meta, x, mod, weights, table=table)
     if kept is None:
         cmax = max(nw for _, _, nw, _ in spans) * meta.L
         tpn = meta.tp.tp if meta.tp is not None else 1   # gathered rows x local features: the same element count
@@ -404,7 +407,10 @@ def block_backward(x: torch.Tensor, mod: torch.Tensor, dy: torch.Tensor, meta: B
     tp = meta.tp
     tpn = tp.tp if tp is not None else 1
     weights = (wn1, wqkv, wo, wn2, w1, w2)
-    native = NB.takes(meta, x, mod, (*weights, dy, *(() if dx is None else (dx,))), grads.values())
+    rows = (dy,) if dx is None else (dy, dx)
+    native = NB.takes(meta, x, mod, (*weights, *rows), grads.values()) and NB.fits(meta, x, mod, weights, rows, grads)
+    if not native:
+        NB.refuse_misfits(meta, x, mod, weights, dx, grads)
     get = ws.whole if native else ws.get
     if kept is None:
         chunk_bufs = {k: get(k, *sh, dev) for k, sh in _chunk_shapes(cmax, D, HD, meta.heads, F, tpn).items()}

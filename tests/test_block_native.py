@@ -57,6 +57,64 @@ def test_what_the_native_call_does_not_take_goes_one_by_one():
         assert not block.takes(m, x, md, ws, gs)
 
 
+def _operands():
+    """A block of two samples of two windows of 16 tokens, on the CPU: (meta, operands by name)."""
+    from aeris_gb_b200.models import fused
+    from aeris_gb_b200.ops import elementwise as E
+    meta, T, D, HD, F = fused.BlockMeta(2, 16, 2, 64, E.MODE_MOD_THEN_NORM, 1e-6, 64), 64, 32, 128, 48
+    z = lambda *s, dt=torch.bfloat16: torch.zeros(s, dtype=dt)
+    f = lambda *s: z(*s, dt=torch.float32)
+    shapes = {"n1": (D,), "to_qkv": (3 * HD, D), "wo": (D, HD), "n2": (D,), "w1": (2 * F, D), "w2": (D, F)}
+    ops = {"x": z(T, D), "mod": f(2, 6 * D), "dy": z(T, D), "dx": z(T, D), "out": z(T, D), "table": torch.arange(T).int()}
+    return meta, {**ops, **{k: z(*s) for k, s in shapes.items()}, **{"g_" + k: f(*s) for k, s in shapes.items()}}
+
+
+MISFITS = {                         # operand -> one of another extent; which directions take it
+    "n1": ((16,), "fb"), "n2": ((16,), "fb"), "to_qkv": ((320, 32), "fb"), "wo": ((32, 64), "fb"), "w1": ((64, 32), "fb"),
+    "w2": ((16, 48), "fb"), "mod": ((2, 160), "fb"), "x": ((32, 32), "fb"), "out": ((32, 32), "f"), "table": ((32,), "f"),
+    "dy": ((32, 32), "b"), "dx": ((32, 32), "b"), "g_n1": ((16,), "b"), "g_n2": ((16,), "b"), "g_wo": ((32, 64), "b"),
+    "g_to_qkv": ((320, 32), "b"), "g_w1": ((64, 32), "b"), "g_w2": ((16, 48), "b")}
+
+
+@pytest.mark.parametrize("name,way", [(n, w) for n, (_, ways) in MISFITS.items() for w in ways] + [(None, "f"), (None, "b")])
+def test_operands_of_other_extents_are_refused(name, way, monkeypatch):
+    """The native call derives every extent; what does not fit goes launch by launch and is refused there. The library is a
+    stand-in that accepts every launch."""
+    from aeris_gb_b200.models import block, fused
+    from aeris_gb_b200.ops import lib
+
+    class Library:
+        def __getattr__(self, entry):
+            return lambda *a: 0
+
+    meta, ops = _operands()
+    if name is not None:
+        ops[name] = torch.zeros(MISFITS[name][0], dtype=ops[name].dtype)
+    native = []
+    monkeypatch.setattr(lib, "lib", Library)
+    monkeypatch.setattr(lib, "raw_stream", lambda: 0)
+    monkeypatch.setattr(lib, "status_word", lambda: torch.zeros(1, dtype=torch.int32))
+    monkeypatch.setattr(fused, "_WS", fused.Workspace())
+    monkeypatch.setattr(block, "takes", lambda *a: True)          # all but the extents is right
+    monkeypatch.setattr(block, "forward", lambda *a: native.append("f"))
+    monkeypatch.setattr(block, "backward", lambda *a: native.append("b"))
+    ws = [ops[k] for k in block.WEIGHTS]
+
+    def run():
+        if way == "f":
+            fused.block_forward(ops["x"], ops["mod"], meta, *ws, out=ops["out"], gather=(ops["table"], [0], ops["x"]))
+        else:
+            grads = {k: ops["g_" + k] for k in block.WEIGHTS}
+            fused.block_backward(ops["x"], ops["mod"], ops["dy"], meta, *ws, grads, dx=ops["dx"])
+    if name is None:
+        run()
+        assert native == [way]
+    else:
+        with pytest.raises((AssertionError, RuntimeError, ValueError)):
+            run()
+        assert not native
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("B,n_win,L,heads,d,F,chunk,floor,mode,rope", [
     (1, 3, 225, 4, 64, 512, 2, 0, 0, False),        # two chunks, the second one short
