@@ -165,7 +165,8 @@ typedef struct AerisBlockGrad {
   float *delta, *G2, *Go, *dmod;    // dmod: [batch, 6 D], overwritten
   float *n1, *to_qkv, *wo, *n2, *w1, *w2;   // weight gradients, added to
 } AerisBlockGrad;
-// Both return the number of kernels launched, or a negative code: that of the launch that failed less 1000 times its place.
+// Both return the number of kernels launched, or a negative code: -1 where `step` is not positive, else that of the launch
+// that failed less 1000 times its place.
 int aeris_block_forward(const AerisBlock* b);
 int aeris_block_backward(const AerisBlock* b, const AerisBlockGrad* g);
 

@@ -110,6 +110,7 @@ bool for_chunks(const AerisBlock& b, int sample, F&& body) {
 
 extern "C" int aeris_block_forward(const AerisBlock* pb) {
   const AerisBlock& b = *pb;
+  if (b.step <= 0) return -1;        // chunks of no windows never end
   const Gemm gemm{b};
   Run run;
   auto body = [&](int sample, int nb, long long r0, int nw) {
@@ -136,6 +137,7 @@ extern "C" int aeris_block_forward(const AerisBlock* pb) {
 extern "C" int aeris_block_backward(const AerisBlock* pb, const AerisBlockGrad* pg) {
   const AerisBlock& b = *pb;
   const AerisBlockGrad& g = *pg;
+  if (b.step <= 0) return -1;
   const Gemm gemm{b};
   const int D = b.D, F = b.F, HD = b.heads * b.head_dim;
   Run run;

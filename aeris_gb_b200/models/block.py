@@ -48,8 +48,8 @@ WEIGHTS = ("n1", "to_qkv", "wo", "n2", "w1", "w2")
 
 def fits(meta, x: torch.Tensor, mod: torch.Tensor, weights, rows=(), grads=None, table=None) -> bool:
     """Whether every operand has the extents that the native call derives from ``x``, ``w2`` and ``meta``: it has no other
-    check. ``rows``: tensors shaped like ``x``; ``grads``: as :func:`.fused.block_backward` takes them. What does not fit goes
-    launch by launch, where each is checked by itself."""
+    check. ``rows``: tensors shaped like ``x``; ``grads``: as :func:`.fused.block_backward` takes them. What does not fit
+    goes launch by launch, where each is checked by itself."""
     (T, D), F, HD, B = x.shape, weights[5].shape[1], meta.heads * meta.head_dim, mod.shape[0]
     want = ((D,), (3 * HD, D), (D, HD), (D,), (2 * F, D), (D, F))
     return (T == B * meta.n_win_per_sample * meta.L and mod.shape == (B, 6 * D)

@@ -221,7 +221,11 @@ def chunk_step(meta: BlockMeta, D: int, F: int) -> int:
     windows of 64 tokens at dim 128 in chunks of 8: 1,582 launches per step for 7 ms of device time). With
     ``min_chunk_bytes = 0`` the bound is ``chunk_windows`` itself."""
     floor = meta.chunk_floor // (kept_bytes(1, D, meta.heads * meta.head_dim, meta.heads, F) * meta.L)
-    return min(max(meta.chunk_windows, floor), meta.n_win_per_sample, MAX_CHUNK_WINDOWS)
+    step = min(max(meta.chunk_windows, floor), meta.n_win_per_sample, MAX_CHUNK_WINDOWS)
+    if step < 1:
+        raise ValueError(f"chunks of {step} windows: chunk_windows {meta.chunk_windows} with min_chunk_bytes "
+                         f"{meta.chunk_floor}, {meta.n_win_per_sample} windows per sample")
+    return step
 
 
 def wanted_slices(meta: BlockMeta, nw: int) -> int:

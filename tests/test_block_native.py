@@ -115,6 +115,24 @@ def test_operands_of_other_extents_are_refused(name, way, monkeypatch):
         assert not native
 
 
+@pytest.mark.parametrize("step", [0, -1])
+def test_chunks_of_no_windows_are_refused(step):
+    """Before anything is launched: by the entry points, whose loop over chunks would not end, and by both directions."""
+    import ctypes
+    from aeris_gb_b200.models import block, fused
+    from aeris_gb_b200.ops import lib
+    a, g = block.BlockArgs(step=step, batch=1, n_win=2, L=16, D=32, F=48, heads=2, head_dim=64), block.BlockGradArgs()
+    assert lib.lib().aeris_block_forward(ctypes.byref(a)) == -1
+    assert lib.lib().aeris_block_backward(ctypes.byref(a), ctypes.byref(g)) == -1
+    meta, ops = _operands()
+    meta = fused.BlockMeta(2, 16, 2, 64, meta.mode, 1e-6, step, min_chunk_bytes=0)
+    ws = [ops[k] for k in block.WEIGHTS]
+    with pytest.raises(ValueError):
+        fused.block_forward(ops["x"], ops["mod"], meta, *ws)
+    with pytest.raises(ValueError):
+        fused.block_backward(ops["x"], ops["mod"], ops["dy"], meta, *ws, {k: ops["g_" + k] for k in block.WEIGHTS})
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("B,n_win,L,heads,d,F,chunk,floor,mode,rope", [
     (1, 3, 225, 4, 64, 512, 2, 0, 0, False),        # two chunks, the second one short
