@@ -76,6 +76,12 @@ def refuse_misfits(meta, x: torch.Tensor, mod: torch.Tensor, weights, dx=None, g
         raise ValueError(f"operands that do not fit a block of {T} rows of {D}: {', '.join(wrong)}")
 
 
+def vectors(mod: torch.Tensor) -> torch.Tensor:
+    """``mod`` as the kernels of both directions read it: without gaps, from a 16-byte boundary on (vectors of four)."""
+    mod = mod.contiguous()
+    return mod if mod.data_ptr() % 16 == 0 else mod.clone()
+
+
 def _args(meta, x, mod, B, D, F, step, weights, bufs: dict[str, int], kept: bool, stream: int) -> tuple[BlockArgs, tuple]:
     """The arguments both directions share, and what has to live until the call returns. ``bufs``: addresses of internals."""
     wn1, wqkv, wo, wn2, w1, w2 = weights
@@ -102,9 +108,7 @@ def forward(meta, x, mod, weights, y, step: int, merged: bool, bufs: dict[str, i
     """``mod`` [B, 6 D] fp32, read in place: samples that run in one launch find their vectors 6 D apart. ``gather``: see
     :func:`.fused.block_forward`."""
     B, D, F = mod.shape[0], x.shape[1], weights[5].shape[1]
-    mod = mod.contiguous()
-    if mod.data_ptr() % 16:               # the kernels read vectors of four
-        mod = mod.clone()
+    mod = vectors(mod)
     a, alive = _args(meta, x, mod, B, D, F, step, weights, bufs, kept, _l.raw_stream())
     a.merged, a.y = merged, y.data_ptr()
     if gather is not None:
@@ -119,7 +123,7 @@ def forward(meta, x, mod, weights, y, step: int, merged: bool, bufs: dict[str, i
 def backward(meta, x, mod, dy, weights, step: int, bufs: dict[str, int], kept: bool, work: dict[str, int], dx, dmod,
              grads: dict[str, torch.Tensor]) -> None:
     """``work``: addresses of the gradient workspaces; ``dmod`` [B, 6 D] fp32 is overwritten."""
-    mod = mod.contiguous()
+    mod = vectors(mod)
     a, alive = _args(meta, x, mod, mod.shape[0], x.shape[1], weights[5].shape[1], step, weights, bufs, kept, _l.raw_stream())
     g = BlockGradArgs(dy=dy.data_ptr(), dx=dx.data_ptr(), dmod=dmod.data_ptr(), **work,
                       **{k: t.data_ptr() for k, t in grads.items()})

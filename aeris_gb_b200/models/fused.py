@@ -433,7 +433,7 @@ def block_backward(x: torch.Tensor, mod: torch.Tensor, dy: torch.Tensor, meta: B
     dmod = torch.zeros((B, 6 * D), dtype=f32, device=dev)
     if dx is None:
         dx = torch.empty_like(x)
-    mod = mod.contiguous()
+    mod = NB.vectors(mod)
     for b in range(B):
         sh1, sc1, g1, sh2, sc2, g2 = [mod[b, i * D:(i + 1) * D] for i in range(6)]
         dsh1, dsc1, dg1, dsh2, dsc2, dg2 = [dmod[b, i * D:(i + 1) * D] for i in range(6)]
