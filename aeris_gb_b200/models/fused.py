@@ -149,6 +149,24 @@ def _kept_shapes(T: int, D: int, HD: int, heads: int, F: int) -> dict[str, tuple
             "x1": ((T, D), bf), "h2": ((T, D), bf), "act": ((T, F), bf), "u": ((T, 2 * F), bf)}
 
 
+def _is_whole(t: torch.Tensor, shape: tuple[int, ...], dtype: torch.dtype, device) -> bool:
+    return t.shape == shape and t.dtype == dtype and t.device == device and t.is_contiguous() and t.data_ptr() % 16 == 0
+
+
+def _whole_kept(kept: dict[str, torch.Tensor], shapes, device) -> dict[str, torch.Tensor]:
+    """``kept`` as the kernels read it, by address: a saved-tensor hook may have handed back other strides or an odd start
+    (copied) or something else altogether (refused). ``shapes``: see :func:`_kept_shapes`."""
+    out = {}
+    for k, (shape, dt) in shapes.items():
+        t = kept[k]
+        if not _is_whole(t, shape, dt, device):
+            if t.shape != shape or t.dtype != dt or t.device != device:
+                raise ValueError(f"kept {k}: {tuple(t.shape)} {t.dtype} on {t.device}, not {shape} {dt} on {device}")
+            t = t.clone(memory_format=torch.contiguous_format)
+        out[k] = t
+    return out
+
+
 def kept_bytes(T: int, D: int, HD: int, heads: int, F: int) -> int:
     """Bytes of :func:`_kept_shapes`, in closed form: every pass over a block asks for them."""
     return T * (2 * (3 * D + 4 * HD + 3 * F) + 4 * heads)
@@ -344,7 +362,9 @@ def block_forward(x: torch.Tensor, mod: torch.Tensor, meta: BlockMeta, wn1, wqkv
     spans = _forward_spans(meta, B, step, D, F, kept is not None)
     weights = (wn1, wqkv, wo, wn2, w1, w2)
     table = gather[0] if gather is not None else None
-    native = NB.takes(meta, x, mod, (*weights, y)) and NB.fits(meta, x, mod, weights, (y,), table=table)
+    native = (NB.takes(meta, x, mod, (*weights, y)) and NB.fits(meta, x, mod, weights, (y,), table=table)
+              and (kept is None or all(_is_whole(kept[k], *sh, dev)
+                                       for k, sh in _kept_shapes(T, D, HD, meta.heads, F).items())))
     if not native:
         NB.refuse_misfits(meta, x, mod, weights, table=table)
     if kept is None:
@@ -416,7 +436,9 @@ def block_backward(x: torch.Tensor, mod: torch.Tensor, dy: torch.Tensor, meta: B
     if not native:
         NB.refuse_misfits(meta, x, mod, weights, dx, grads)
     get = ws.whole if native else ws.get
-    if kept is None:
+    if kept is not None:
+        kept = _whole_kept(kept, _kept_shapes(T, D, HD, meta.heads, F), dev)
+    else:
         chunk_bufs = {k: get(k, *sh, dev) for k, sh in _chunk_shapes(cmax, D, HD, meta.heads, F, tpn).items()}
         chunk_bufs["h1"], act_b = chunk_bufs.pop("h"), chunk_bufs["act"]
     work = {k: get(k, *sh, dev) for k, sh in _grad_shapes(cmax, D, HD, meta.heads, F, tpn).items()}
@@ -577,7 +599,7 @@ class FusedBlock(torch.autograd.Function):
             else:
                 grads[k] = torch.zeros(p.shape, dtype=torch.float32, device=p.device)
                 ret[k] = grads[k]
-        dy = dy.contiguous()
+        x, dy = x.contiguous(), dy.contiguous()        # a saved-tensor hook may hand back other strides
         dx, dmod = block_backward(x, mod.float(), dy, ctx.meta, wn1, wqkv, wo, wn2, w1, w2, grads, dx=dy, kept=kept)
         if ctx.regroup is not None:
             _, table_bwd, peer_fn = ctx.regroup
