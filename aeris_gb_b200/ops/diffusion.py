@@ -147,10 +147,12 @@ def gemv_bwd(W: torch.Tensor, x: torch.Tensor, dy: torch.Tensor, dW: torch.Tenso
 def modulation_mlp_bwd(W1: torch.Tensor, x: torch.Tensor, W2: torch.Tensor, y1: torch.Tensor, dy: torch.Tensor,
                        dW1: torch.Tensor, db1: torch.Tensor, dW2: torch.Tensor, db2: torch.Tensor,
                        need_dx: bool) -> torch.Tensor | None:
-    """Adds the gradients of :func:`modulation_mlp` to fp32 ``dW1 .. db2``; returns that of ``x`` (fp32) if asked for."""
+    """Adds the gradients of :func:`modulation_mlp` to fp32 ``dW1 .. db2``; returns that of ``x`` (fp32) if asked for. ``x``
+    and ``y1`` may have any strides: they are what autograd saved."""
     (N1, K), N2 = W1.shape, W2.shape[0]
-    x, dy = _f32_or_bf16(x).contiguous(), dy.float().contiguous()
+    x, y1, dy = _f32_or_bf16(x).contiguous(), _f32_or_bf16(y1).contiguous(), dy.float().contiguous()
     B = x.shape[0]
+    assert y1.shape == (B, N1) and dy.shape == (B, N2)
     dy1 = torch.empty((B, N1), dtype=torch.float32, device=x.device)
     dx = torch.empty((B, K), dtype=torch.float32, device=x.device) if need_dx else None
     rc = _l.lib().aeris_modulation_mlp_bwd(_l.ptr(W1), _gemv_flags(W1, None, x), _l.ptr(x), _l.ptr(dW1), _l.ptr(db1),

@@ -87,3 +87,48 @@ def test_block_with_kept_internals(B, L):
     assert torch.equal(got[0], want[0])
     for a, b in zip(got[1:], want[1:]):                # fp32 sums by atomics, rounded to the parameters' bf16
         assert rel_err(a, b) < 1e-3
+
+
+def test_modulation_mlp_reads_the_first_layer_in_order(monkeypatch):
+    """The address handed on is that of dense rows, whatever strides a hook gave the first layer's result."""
+    import ctypes
+    from aeris_gb_b200.ops import diffusion as DF
+    from aeris_gb_b200.ops import lib
+    B, K, N1, N2 = 3, 8, 12, 16
+    seen = []
+
+    class Library:
+        def aeris_modulation_mlp_bwd(self, *a):
+            seen.append(list((ctypes.c_float * (B * N1)).from_address(a[10].value)))
+            return 0
+
+    monkeypatch.setattr(lib, "lib", Library)
+    monkeypatch.setattr(lib, "raw_stream", lambda: 0)
+    x, y1, dy = torch.randn(B, K), torch.randn(B, N1), torch.randn(B, N2)
+    z = torch.zeros
+    for t in (y1, _other_strides(y1), y1.double()):
+        DF.modulation_mlp_bwd(z(N1, K), x, z(N2, N1), t, dy, z(N1, K), z(N1), z(N2, N1), z(N2), True)
+    assert seen == [y1.flatten().tolist()] * 3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B", [1, 2, 5])
+@pytest.mark.parametrize("K,N1,N2", [(64, 128, 96), (128, 64, 6 * 128)])
+def test_modulation_mlp(B, K, N1, N2):
+    x, W1, b1, W2, b2 = (torch.randn(*s, device=DEV) for s in ((B, K), (N1, K), (N1,), (N2, N1), (N2,)))
+    dy = torch.randn(B, N2, device=DEV)
+
+    def grads():
+        leaves = [t.clone().requires_grad_(True) for t in (x, W1, b1, W2, b2)]
+        return torch.autograd.grad(fused.ModulationFn.apply(*leaves), leaves, dy)
+
+    want = grads()
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, _other_strides):
+        got = grads()
+    for a, b in zip(got, want):          # other strides of a weight take the PyTorch formulas: 2e-7, and fast exponentials
+        assert rel_err(a, b) < 4e-6
+    keep = lambda t: t if t.shape in (W1.shape, W2.shape) and t.shape != (B, N1) else _other_strides(t)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, keep):       # y1 with other strides on the kernels
+        got = grads()
+    for a, b in zip(got, want):
+        assert rel_err(a, b) < 1e-6
