@@ -599,7 +599,7 @@ template <int DCH> struct BwdRing {
   static constexpr int ITEM_BYTES = 2 * DCH * 16384, STAGE = 2 * DCH * 8192;
   static constexpr int STAT = 4 * TILE > NST * 2 * BT ? 4 * TILE : NST * 2 * BT;
   static constexpr bool STAGED = DCH == 2;              // gradient rows leave through shared memory, see BwdOut
-  static constexpr int OUT_BYTES = STAGED ? TILE * 64 : 0;      // 32 columns, per warpgroup
+  static constexpr int OUT_BYTES = STAGED ? 2 * TILE * 64 : 0;  // two buffers of 32 columns, per warpgroup
   static constexpr int SMEM = NB * ITEM_BYTES + NST * STAGE + NWG * OUT_BYTES + STAT * 4 + 512;
   static constexpr int THREADS = 128 + 128 * NWG;
 };
@@ -613,54 +613,51 @@ __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// Gradient rows on their way out: a warpgroup turns 32 accumulator columns of its 128 rows into bf16 in shared memory, one
-// thread hands them to the TMA unit as one tiled store. The accumulator is free once it has been read; written by the
-// threads themselves (one row each, 32 rows with every 16-byte store instruction) it kept the next item's products waiting.
-// Rows past the window's end and columns past the head's width are clipped by the tensor map. Both kernels, ms, before and
-// now, 12 heads x 128: 400 x 128 tokens 0.550 -> 0.464, 200 x 225 0.625 -> 0.546, 72 x 900 1.69 -> 1.60, 16 x 3600 4.45 ->
-// 4.34. At 64, with a third of the columns per warpgroup, the hand-shakes cost more than they save (24 x 64, 200 x 225:
-// 0.650 -> 0.704, 72 x 900 1.91 -> 1.92): direct stores there.
+// Gradient rows on their way out: a warp turns 32 accumulator columns of its 32 rows into bf16 in shared memory, one lane
+// hands them to the TMA unit as a tiled store. The accumulator is free once it has been read; written by the threads
+// themselves (one row each, 32 rows with every 16-byte store instruction) it kept the next item's products waiting. Rows
+// past the window's end and columns past the head's width are clipped by the tensor map. No warp waits for another one's
+// rows. Both kernels, ms, direct stores / now, in turn, 12 heads x 128: 400 x 128 tokens 0.548 / 0.456, 200 x 225 0.631 /
+// 0.535, 72 x 900 1.73 / 1.61, 16 x 3600 4.50 / 4.31; with one buffer a warp 0.527, 0.602, 1.59 and 4.35. At 64, with a
+// third of the columns per warpgroup, staging (of a warpgroup's 128 rows at a time) cost more than it saved (24 x 64, 200 x
+// 225: 0.650 -> 0.704, 72 x 900 1.91 -> 1.92): direct stores there.
 struct BwdOut {
-  uint8_t* stage;           // this warpgroup's
-  uint64_t *free_bar, *full_bar;
-  int* status;
-  int warp_in_group, lane, row, n = 0;
+  uint8_t* stage;           // this warp's two: 32 rows of 64 bytes, the vectors of 16 swizzled as the tensor map has it
+  int lane, first_row;      // of this warp inside the tile
+  int n = 0;                // groups of columns so far
 
-  __device__ __forceinline__ bool leader() const { return warp_in_group == 0 && lane == 0; }
   // `read`: called once the columns are out of tensor memory
   template <typename F>
-  __device__ __forceinline__ bool put(uint32_t taddr, float f, const CUtensorMap* m, int col, int head, int grow, int win,
-                                      F&& read) {
+  __device__ __forceinline__ void put(uint32_t taddr, float f, const CUtensorMap* m, int col, int head, int tile_row,
+                                      int win, int N, F&& read) {
     uint32_t v[32];
     tmem_ld32(taddr, v);
     tmem_wait_ld();
     read();
-    if (leader()) {
-      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-      mbar_arrive(free_bar);
-    }
-    if (!mbar_wait(free_bar, n & 1, status, ERR_TIMEOUT_ATTN)) return false;
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+    __syncwarp();
+    uint8_t* buf = stage + (n++ & 1) * 2048;
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
       uint32_t o[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         o[i] = pack_bf16x2(__uint_as_float(v[8 * g + 2 * i]) * f, __uint_as_float(v[8 * g + 2 * i + 1]) * f);
-      *reinterpret_cast<uint4*>(stage + row * 64 + ((g ^ ((row >> 1) & 3)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+      *reinterpret_cast<uint4*>(buf + lane * 64 + ((g ^ ((lane >> 1) & 3)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
     }
     fence_proxy_async_smem();
     __syncwarp();
-    if (lane == 0) mbar_arrive(full_bar);
-    if (leader()) {
-      if (!mbar_wait(full_bar, n & 1, status, ERR_TIMEOUT_ATTN)) return false;
-      tma_store_4d(m, stage, col, head, grow, win);
+    if (lane == 0) {
+      if (tile_row + first_row < N)
+        tma_store_4d(m, buf, col, head, tile_row + first_row, win);
+      else                  // no rows: an empty group, so that the buffers still come free in turn
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     }
-    ++n;
-    return true;
+    __syncwarp();           // the warp goes on as one: the next step reads tensor memory
   }
-  // before this thread leaves: its copies have been performed
+  // before this warp leaves: its copies have been performed
   __device__ __forceinline__ void drain() const {
-    if (leader()) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
 };
 
@@ -713,9 +710,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   uint64_t* acc_empty = bars + 20;
   uint64_t* stat_full = bars + 21;      // [2]
   uint64_t* stat_empty = bars + 23;     // [2]
-  uint64_t* out_free = bars + 25;       // [NWG]
-  uint64_t* out_full = bars + 28;       // [NWG]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 31);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 25);
   int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -742,7 +737,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     for (int i = 0; i < NWG; ++i) {
       mbar_init(&first_full[i], 1);
       mbar_init(&next_full[i], 4 + 1);
-      mbar_init(&sp_full[i], 1); mbar_init(&out_free[i], 1); mbar_init(&out_full[i], 4);
+      mbar_init(&sp_full[i], 1);
     }
     mbar_init(acc_full, 1); mbar_init(acc_empty, 4 * NWG);
     fence_barrier_init();
@@ -936,7 +931,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     uint32_t ph = 0;
     int j = wg;                       // first tile of this warpgroup in the item at hand
     bool ok = true;
-    BwdOut out{sOut + wg * R::OUT_BYTES, &out_free[wg], &out_full[wg], p.status, q, lane, row};
+    BwdOut out{sOut + wg * R::OUT_BYTES + q * 4096, lane, q * 32};
     // Gradient rows of item `it` from TMEM to memory. Runs after this warpgroup's first tile of the NEXT item, so that the
     // wait for the last products of `it` is spent on that tile.
     auto epilogue = [&](int it) -> bool {
@@ -953,9 +948,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         for (int c = wg * 32; c < p.d; c += 32 * NWG) ++mine;
         if (mine == 0) release();
         for (int c = wg * 32; c < p.d; c += 32 * NWG)
-          if (!out.put(tdQ + lane_addr + c, sc, &tm_dq, c, w.head, w.tile * TILE, w.win,
-                       [&] { if (--mine == 0) release(); }))
-            return false;
+          out.put(tdQ + lane_addr + c, sc, &tm_dq, c, w.head, w.tile * TILE, w.win, N,
+                  [&] { if (--mine == 0) release(); });
         return true;
       }
       const int grow = w.tile * TILE + row;
@@ -1081,9 +1075,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   uint64_t* sp_full = bars + 16;         // [NWG]
   uint64_t* acc_full = bars + 19;
   uint64_t* acc_empty = bars + 20;
-  uint64_t* out_free = bars + 21;        // [NWG]
-  uint64_t* out_full = bars + 24;        // [NWG]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 27);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
   int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1110,7 +1102,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     for (int i = 0; i < NWG; ++i) {
       mbar_init(&first_full[i], 1 + 32);
       mbar_init(&next_full[i], 4 + 1 + 32);
-      mbar_init(&sp_full[i], 1); mbar_init(&out_free[i], 1); mbar_init(&out_full[i], 4);
+      mbar_init(&sp_full[i], 1);
     }
     mbar_init(acc_full, 1); mbar_init(acc_empty, 4 * NWG);
     fence_barrier_init();
@@ -1292,7 +1284,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       pp = f2_to_bf16x2(pr);
       dd = f2_to_bf16x2(f2_mul(pr, f2_sub(f2_pack(__uint_as_float(d0), __uint_as_float(d1)), de)));
     };
-    BwdOut out{sOut + wg * R::OUT_BYTES, &out_free[wg], &out_full[wg], p.status, q, lane, row};
+    BwdOut out{sOut + wg * R::OUT_BYTES + q * 4096, lane, q * 32};
     // see attn_bwd_dq_kernel: the epilogue of an item runs after this warpgroup's first tile of the next
     auto epilogue = [&](int it) -> bool {
       if (!mbar_wait(acc_full, it & 1, p.status, ERR_TIMEOUT_ATTN)) return false;
@@ -1309,9 +1301,9 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         if (mine == 0) release();
         for (int c = wg * 32; c < 2 * HD; c += 32 * NWG) {
           const int col = c < HD ? c : c - HD;          // column inside the head
-          if (col < p.d && !out.put(tdK + lane_addr + c, c < HD ? sc : 1.f, c < HD ? &tm_dk : &tm_dv, col, w.head,
-                                    w.tile * TILE, w.win, [&] { if (--mine == 0) release(); }))
-            return false;
+          if (col < p.d)
+            out.put(tdK + lane_addr + c, c < HD ? sc : 1.f, c < HD ? &tm_dk : &tm_dv, col, w.head, w.tile * TILE, w.win, N,
+                    [&] { if (--mine == 0) release(); });
         }
         return true;
       }
@@ -1523,7 +1515,7 @@ static int attn_fwd_impl(const void* q, int ldq, int q_col0, const void* k, int 
     if ((r = make_tmap_heads_bf16(&tk, at(k, k_col0), head_dim, H, N, n_win, ldk, KVP))) return r;
     if ((r = make_tmap_heads_bf16(&tv, at(v, v_col0), head_dim, H, N, n_win, ldv, KVP))) return r;
     CUtensorMap to = tq;      // without a local output nothing is stored through it
-    if (o && (r = make_tmap_heads_bf16(&to, o, head_dim, H, N, n_win, ldo, TILE))) return r;
+    if (o && (r = make_tmap_heads_bf16(&to, o, head_dim, H, N, n_win, ldo, 32))) return r;
     if (cut)
       return head_dim > 64 ? launch_attn_fwd_pair<2, true>(tq, tk, tv, to, p, stream)
                            : launch_attn_fwd_pair<1, true>(tq, tk, tv, to, p, stream);
@@ -1607,7 +1599,7 @@ static int attn_bwd_impl(const void* qkv, int ldq, int q_col0, int k_col0, int v
     const __nv_bfloat16* g = p.dQKV;
     const int cols[3] = {q_col0, k_col0, v_col0};
     for (int i = 0; i < 3; ++i)
-      if ((r = make_tmap_heads32_bf16(&out[i], g + cols[i], head_dim, H, N, n_win, ldg, TILE))) return r;
+      if ((r = make_tmap_heads32_bf16(&out[i], g + cols[i], head_dim, H, N, n_win, ldg, 32))) return r;
   }
   return head_dim <= 64 ? launch_attn_bwd<1>(q128, k64, v64, d128, q64, k128, v128, d64, out, p, stream)
                         : launch_attn_bwd<2>(q128, k64, v64, d128, q64, k128, v128, d64, out, p, stream);

@@ -26,7 +26,7 @@ template <int DCH> struct AttnPair {
   static constexpr int Q_BYTES = DCH * 16384, T_BYTES = DCH * 16384;      // a query tile; a K or V tile
   static constexpr int NBQ = DCH == 1 ? 2 : 1;                            // buffers per chain for its query tile
   static constexpr int NS = DCH == 1 ? 3 : 2;                             // depth of the K ring and of the V ring
-  static constexpr int OUT_BYTES = 16384;                                 // staging of 64 output columns of a chain
+  static constexpr int OUT_BYTES = 16384;                                 // staging of 64 output columns, 4 KB a warp
   static constexpr int SMEM = 2 * NBQ * Q_BYTES + 2 * NS * T_BYTES + 2 * OUT_BYTES + 512;
   static constexpr int THREADS = 384;
   // tensor memory columns of a chain (256 each): scores at 0, then
@@ -113,9 +113,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   uint64_t* pv_done = bars + 32;        // [2] P V has completed: P may be overwritten, the accumulator is up to date
   uint64_t* turn = bars + 34;           // [2] P_OVER_S: whose products are next
   uint64_t* half = bars + 36;           // [2][4] a warp is half way through its exponentials
-  uint64_t* o_free = bars + 44;         // [2] the chain's staging buffer has been read out
-  uint64_t* o_full = bars + 46;         // [2] and filled again
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 48);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 44);
   int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -144,7 +142,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s_full[i], 1); mbar_init(&s_free[i], 4); mbar_init(&p_full[i], 4); mbar_init(&p_full2[i], 4);
-      mbar_init(&pv_done[i], 1); mbar_init(&turn[i], 1); mbar_init(&o_free[i], 1); mbar_init(&o_full[i], 4);
+      mbar_init(&pv_done[i], 1); mbar_init(&turn[i], 1);
     }
     for (int i = 0; i < 8; ++i) mbar_init(&half[i], 1);
     fence_barrier_init();
@@ -317,12 +315,11 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       tc_fence_after();
       return true;
     };
-    // Output rows and row statistics of an item, whose last P V has completed. The rows leave as one tile through shared
-    // memory (one thread a row, 16 bytes a store, would touch 32 rows with every instruction).
-    uint8_t* stage = sO + c * R::OUT_BYTES;
-    const bool leader = q == 0 && lane == 0;
-    int n_staged = 0;
-    auto epilogue = [&](const PairItem& w, bool rows) -> bool {
+    // Output rows and row statistics of an item, whose last P V has completed. A warp's rows leave as tiles of 32 through
+    // shared memory (one thread a row, 16 bytes a store, would touch 32 rows with every instruction). Every lane-0 block is
+    // followed by a warp barrier: the next step reads tensor memory, which takes the whole warp.
+    uint8_t* stage = sO + c * R::OUT_BYTES + q * 4096;
+    auto epilogue = [&](const PairItem& w) {
       const int grow = (2 * w.pair + c) * TILE + row;
       const float inv = 1.f / l;
       __nv_bfloat16* pdst = nullptr;
@@ -334,42 +331,32 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       }
 #pragma unroll 1
       for (int col = 0; col < HD && col < p.d; col += 64) {
-        if (leader) {
-          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-          mbar_arrive(&o_free[c]);
-        }
-        if (!mbar_wait(&o_free[c], n_staged & 1, p.status, ERR_TIMEOUT_ATTN)) return false;
-        if (rows) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            uint32_t v[32];
-            tmem_ld32(tO + col + 32 * h, v);
-            tmem_wait_ld();
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              uint32_t o[4];
-#pragma unroll
-              for (int i = 0; i < 4; ++i)
-                o[i] = pack_bf16x2(__uint_as_float(v[8 * g + 2 * i]) * inv, __uint_as_float(v[8 * g + 2 * i + 1]) * inv);
-              const uint4 u = make_uint4(o[0], o[1], o[2], o[3]);
-              *reinterpret_cast<uint4*>(stage + swz128(row, 4 * h + g)) = u;
-              if (pdst && col + 32 * h + 8 * g < p.d) *reinterpret_cast<uint4*>(pdst + col + 32 * h + 8 * g) = u;
-            }
-          }
-          fence_proxy_async_smem();
-        }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         __syncwarp();
-        if (lane == 0) mbar_arrive(&o_full[c]);
-        // columns past the head's width and rows past the window's end are clipped
-        if (leader) {
-          if (!mbar_wait(&o_full[c], n_staged & 1, p.status, ERR_TIMEOUT_ATTN)) return false;
-          if (p.O) tma_store_4d(&tm_o, stage, col, w.head, (2 * w.pair + c) * TILE, w.win);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t v[32];
+          tmem_ld32(tO + col + 32 * h, v);
+          tmem_wait_ld();
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            uint32_t o[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              o[i] = pack_bf16x2(__uint_as_float(v[8 * g + 2 * i]) * inv, __uint_as_float(v[8 * g + 2 * i + 1]) * inv);
+            const uint4 u = make_uint4(o[0], o[1], o[2], o[3]);
+            *reinterpret_cast<uint4*>(stage + swz128(lane, 4 * h + g)) = u;
+            if (pdst && col + 32 * h + 8 * g < p.d) *reinterpret_cast<uint4*>(pdst + col + 32 * h + 8 * g) = u;
+          }
         }
-        ++n_staged;
+        fence_proxy_async_smem();
+        __syncwarp();
+        // columns past the head's width and rows past the window's end are clipped
+        if (lane == 0 && p.O) tma_store_4d(&tm_o, stage, col, w.head, (2 * w.pair + c) * TILE + q * 32, w.win);
+        __syncwarp();
       }
       if (p.lse && grow < N)
         p.lse[(static_cast<size_t>(w.win) * p.H + w.head) * N + grow] = m_ref + log2f(l);
-      return true;
     };
     auto arrive = [&](uint64_t* bar) {
       tc_fence_before();
@@ -520,10 +507,10 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         for (int j = 0; j < nkv && ok; ++j) ok = idle_tile(j);
       }
       if (!ok || !wait_pv()) break;
-      if (!epilogue(w, rows)) break;
+      if (rows) epilogue(w);
     }
     // the copies have been performed before their shared memory goes
-    if (leader) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
