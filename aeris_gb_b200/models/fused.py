@@ -538,9 +538,11 @@ def _pool_alloc(peer_fn, gradient: bool = False):
 
 def recorded() -> bool:
     """Whether anything would notice if an autograd function's forward ran as a plain call: a graph under construction, a
-    forward-mode level, a function transform, a trace. Sampling has none of them; the wrapper costs about 15 us."""
-    return (torch.is_grad_enabled() or forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active()
-            or torch._C._get_tracing_state() is not None)
+    forward-mode level, a function transform, a trace. Sampling has none of them; the wrapper costs about 15 us. PyTorch has
+    no public names for the last three: where a private one is gone, everything counts as recorded."""
+    return (torch.is_grad_enabled() or getattr(forward_ad, "_current_level", 0) >= 0
+            or getattr(torch._C, "_are_functorch_transforms_active", lambda: True)()
+            or getattr(torch._C, "_get_tracing_state", lambda: True)() is not None)
 
 
 def run_block(x, mod, meta: BlockMeta, wn1, wqkv, wo, wn2, w1, w2, regroup=None, out_alloc=None) -> torch.Tensor:
