@@ -406,7 +406,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             if (j > 0 && !waited && !mbar_wait(pv_done, (j - 1) & 1, p.status, ERR_TIMEOUT_ATTN)) { ok = false; break; }
 #pragma unroll
             for (int g = 0; g < 8; ++g)
-              *reinterpret_cast<uint4*>(sP + swz128(row, g)) = make_uint4(pk[4 * g], pk[4 * g + 1], pk[4 * g + 2], pk[4 * g + 3]);
+              *reinterpret_cast<uint4*>(sP + swz128(row, g)) =
+                  make_uint4(pk[4 * g], pk[4 * g + 1], pk[4 * g + 2], pk[4 * g + 3]);
           }
         }
       } else {

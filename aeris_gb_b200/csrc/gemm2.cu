@@ -118,8 +118,9 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   // AG: the last operand stage is the copier's ring (two 16 KB bulk-copy buffers), with its barriers behind tmem_slot
   // (the reduce-scatter epilogue gives up the same stage: its fourth warp stages its rows there)
   // and so do the epilogues on eight warps that request a second operand ahead. The gated residual gains from that while
-  // its tile's products are short (us without / with: 28800 x 768 x 768 47.5 / 40.5, x 512 x 512 57.2 / 49.5; 64800 x 1536 x
-  // 1536 283 / 282, 28800 x 768 x 2048 84 / 88: the ring's fifth stage is worth more).
+  // its tile's products are short (us without / with, in turn: 28800 x 512 x 512 36.8 / 31.0, x 768 x 768 57.0 / 48.3, x
+  // 1024 x 1024 86.0 / 73.2, 64800 x 512 x 512 71.5 / 61.1; a few per cent at 28800 x 768 x 1536 79.8 / 76.2 and 64800 x 1536 x
+  // 1536 321 / 308; 28800 x 768 x 2048 94.3 / 97.7: the ring's fifth stage is worth more).
   const bool ahead = EW == 8 && p.staged_out;
   const bool u_ahead = ahead && p.epi == EPI_SWIGLU_BWD, r_ahead = ahead && p.epi == EPI_GATE_RESID && !p.aux && p.K <= 1024;
   const int STAGES = (u_ahead || r_ahead || (EW == 4 && (AG || p.epi == EPI_RS_PUSH))) ? LY::STAGES - 1 : LY::STAGES;
@@ -487,8 +488,9 @@ static int gemm_two_cta(const void* A, const void* B, void* C, int M, int N, int
   // 2304 1270 / 1309. The raw columns lose below the line at 2048.
   // Plain store 28800 x 2304 x 768 104 / 98, x 3072 x 1024 158 / 157, x 3840 x 1280 222 / 232. Weight gradients (a_mn) lose
   // a few per cent. Since then the SwiGLU backward and the gated residual on eight warps request their second operand ahead
-  // (registers for that spilled; see swiglu_u_request), and the SwiGLU backward's line moved up: 28800 x 6144 x 2304 832 /
-  // 740, x 8192 x 3072 1300 / 1310, x 13696 x 5120 3598 / 3619.
+  // (registers for that spilled; see swiglu_u_request), and the SwiGLU backward's line moved up. In turn, 1.2-1.5 GHz:
+  // 28800 x 5376 x 2048 712 / 684, x 6144 x 2304 1017 / 810, x 6400 x 2432 1094 / 897, x 6912 x 2560 1167 / 1031; it would
+  // gain further up (x 7680 x 2816 1376 / 1255), but no more at x 8192 x 3072 1469 / 1478.
   const bool heavy = epi == EPI_SWIGLU_BOTH || epi == EPI_SWIGLU_BWD || epi == EPI_GATE_RESID;
   const bool ew8 = (heavy && K <= (epi == EPI_SWIGLU_BWD ? 2560 : 2048)) || (epi == EPI_STORE && K <= 1024);
   if (a_mn) return b_mn ? launch_gemm2<1, 1, 4>(ta, tb, p, stream) : launch_gemm2<1, 0, 4>(ta, tb, p, stream);

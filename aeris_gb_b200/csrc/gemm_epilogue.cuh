@@ -170,7 +170,8 @@ __device__ __forceinline__ void swiglu_bwd_pair(float d0, float d1, uint32_t gw,
 // the lane that owns the row; 16-byte chunks XOR-swizzled by row. Read by every lane from its own row when its turn came, 32
 // rows per instruction, the operand's latency was paid four times per tile: 28800 x 2048 x 768 211 -> 168 us, 28800 x 1536 x
 // 512 158 -> 119, 64800 x 4096 x 1536 1088 -> 918. What is left is the arithmetic (two exponentials and two divisions per
-// element) and shared memory, which operands and staging fill to the brim: 15,000 cycles a tile against 6,100 of products.
+// element) and shared memory, which operands and staging fill to the brim: at 28800 x 2048 x 768 each of the 13 rounds of
+// tiles takes 12.9 us, of which the products alone would take 4.6 at the rate of a large GEMM (1.6 PFLOP/s).
 constexpr int SWIGLU_U_BYTES = 4096;
 __device__ __forceinline__ void swiglu_u_request(uint8_t* buf, const GemmParams& p, int row0, int col, int lane) {
 #pragma unroll

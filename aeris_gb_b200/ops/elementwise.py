@@ -81,7 +81,8 @@ def modnorm_bwd_f32(x: torch.Tensor, dh: torch.Tensor, scale: torch.Tensor, shif
                     dw: torch.Tensor) -> None:
     """Backward of :func:`modnorm_fwd_f32` for one sample, ``dh`` fp32; ``dscale``, ``dshift`` and ``dw`` are added to."""
     rows, D = x.shape
-    sums = torch.empty((148, 3, D), dtype=torch.float32, device=x.device)      # one row per CTA, one CTA per SM
+    ctas = torch.cuda.get_device_properties(x.device).multi_processor_count      # one per SM at most, one row of sums each
+    sums = torch.empty((ctas, 3, D), dtype=torch.float32, device=x.device)
     rc = _l.lib().aeris_modnorm_bwd_f32(_l.ptr(x), _l.ptr(dh), _l.ptr(scale), _l.ptr(shift), _l.ptr(w), _l.ptr(dx),
                                         _l.ptr(dscale), _l.ptr(dshift), _l.ptr(dw), _l.ptr(sums), sums.shape[0], rows, D,
                                         mode, _l._c_float(eps), _l.stream_ptr())

@@ -1,5 +1,6 @@
-"""Attention backward, heads wider than 64: gradient rows leave warp by warp as tiled stores from two buffers in turn. Windows
-whose last tile has rows for one to three of its four warps, several items a CTA, so that copies and empty groups alternate."""
+"""Attention backward, heads wider than 64: gradient rows leave warp by warp as tiled stores from two buffers in turn.
+Windows whose last tile has rows for one to three of its four warps, several items a CTA: copies and empty groups
+alternate."""
 import math
 
 import pytest

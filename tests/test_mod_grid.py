@@ -12,7 +12,7 @@ DEV = "cuda"
 @pytest.mark.parametrize("native", [True, False])
 @pytest.mark.parametrize("way", ["forward", "backward"])
 def test_vectors_off_the_grid_are_moved_before_a_kernel_reads_them(way, native, monkeypatch):
-    """Both directions, in one native call and launch by launch: the addresses handed on, with a library that runs nothing."""
+    """Both directions, in one native call and launch by launch: the addresses handed on to a library that runs nothing."""
     from aeris_gb_b200.ops import lib
     seen = []
 
