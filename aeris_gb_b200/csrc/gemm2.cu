@@ -119,8 +119,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   // (the reduce-scatter epilogue gives up the same stage: its fourth warp stages its rows there)
   // and so do the epilogues on eight warps that request a second operand ahead. The gated residual gains from that while
   // its tile's products are short (us without / with, in turn: 28800 x 512 x 512 36.8 / 31.0, x 768 x 768 57.0 / 48.3, x
-  // 1024 x 1024 86.0 / 73.2, 64800 x 512 x 512 71.5 / 61.1; a few per cent at 28800 x 768 x 1536 79.8 / 76.2 and 64800 x 1536 x
-  // 1536 321 / 308; 28800 x 768 x 2048 94.3 / 97.7: the ring's fifth stage is worth more).
+  // 1024 x 1024 86.0 / 73.2, 64800 x 512 x 512 71.5 / 61.1; a few per cent at 28800 x 768 x 1536 79.8 / 76.2 and 64800 x
+  // 1536 x 1536 321 / 308; 28800 x 768 x 2048 94.3 / 97.7: the ring's fifth stage is worth more).
   const bool ahead = EW == 8 && p.staged_out;
   const bool u_ahead = ahead && p.epi == EPI_SWIGLU_BWD, r_ahead = ahead && p.epi == EPI_GATE_RESID && !p.aux && p.K <= 1024;
   const int STAGES = (u_ahead || r_ahead || (EW == 4 && (AG || p.epi == EPI_RS_PUSH))) ? LY::STAGES - 1 : LY::STAGES;

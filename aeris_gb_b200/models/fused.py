@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import math
 from dataclasses import dataclass
+from types import SimpleNamespace
 
 import torch
 from torch.autograd import forward_ad
@@ -149,21 +150,32 @@ def _kept_shapes(T: int, D: int, HD: int, heads: int, F: int) -> dict[str, tuple
             "x1": ((T, D), bf), "h2": ((T, D), bf), "act": ((T, F), bf), "u": ((T, 2 * F), bf)}
 
 
-def _is_whole(t: torch.Tensor, shape: tuple[int, ...], dtype: torch.dtype, device) -> bool:
-    return t.shape == shape and t.dtype == dtype and t.device == device and t.is_contiguous() and t.data_ptr() % 16 == 0
+class FreshKept(dict):
+    """Internals' buffers as :class:`FusedBlock` allocates them for one forward pass: nothing about them needs a check."""
+
+
+def _all_whole(kept: dict[str, torch.Tensor], T: int, D: int, HD: int, heads: int, F: int, device: int) -> bool:
+    """Whether kernels may take all of ``kept`` (:func:`_kept_shapes`) by address. Every backward pass asks."""
+    td, th, tf = T * D, T * HD, T * F
+    for k, n in (("h1", td), ("qkv", 3 * th), ("o", th), ("x1", td), ("h2", td), ("act", tf), ("u", 2 * tf),
+                 ("lse", T * heads)):
+        t = kept[k]
+        if not (t.is_contiguous() and t.numel() == n and t.dtype is (torch.float32 if k == "lse" else torch.bfloat16)
+                and t.get_device() == device and t.data_ptr() % 16 == 0):
+            return False
+    return True
 
 
 def _whole_kept(kept: dict[str, torch.Tensor], shapes, device) -> dict[str, torch.Tensor]:
-    """``kept`` as the kernels read it, by address: a saved-tensor hook may have handed back other strides or an odd start
-    (copied) or something else altogether (refused). ``shapes``: see :func:`_kept_shapes`."""
+    """``kept`` for kernels where :func:`_all_whole` says no: a saved-tensor hook may have handed back other strides or an
+    odd start (copied) or something else altogether (refused). ``shapes``: see :func:`_kept_shapes`."""
     out = {}
     for k, (shape, dt) in shapes.items():
         t = kept[k]
-        if not _is_whole(t, shape, dt, device):
-            if t.shape != shape or t.dtype != dt or t.device != device:
-                raise ValueError(f"kept {k}: {tuple(t.shape)} {t.dtype} on {t.device}, not {shape} {dt} on {device}")
-            t = t.clone(memory_format=torch.contiguous_format)
-        out[k] = t
+        if t.shape != shape or t.dtype != dt or t.device != device:
+            raise ValueError(f"kept {k}: {tuple(t.shape)} {t.dtype} on {t.device}, not {shape} {dt} on {device}")
+        whole = t.is_contiguous() and t.data_ptr() % 16 == 0
+        out[k] = t if whole else t.clone(memory_format=torch.contiguous_format)
     return out
 
 
@@ -363,8 +375,7 @@ def block_forward(x: torch.Tensor, mod: torch.Tensor, meta: BlockMeta, wn1, wqkv
     weights = (wn1, wqkv, wo, wn2, w1, w2)
     table = gather[0] if gather is not None else None
     native = (NB.takes(meta, x, mod, (*weights, y)) and NB.fits(meta, x, mod, weights, (y,), table=table)
-              and (kept is None or all(_is_whole(kept[k], *sh, dev)
-                                       for k, sh in _kept_shapes(T, D, HD, meta.heads, F).items())))
+              and (kept is None or type(kept) is FreshKept or _all_whole(kept, T, D, HD, meta.heads, F, x.get_device())))
     if not native:
         NB.refuse_misfits(meta, x, mod, weights, table=table)
     if kept is None:
@@ -437,7 +448,8 @@ def block_backward(x: torch.Tensor, mod: torch.Tensor, dy: torch.Tensor, meta: B
         NB.refuse_misfits(meta, x, mod, weights, dx, grads)
     get = ws.whole if native else ws.get
     if kept is not None:
-        kept = _whole_kept(kept, _kept_shapes(T, D, HD, meta.heads, F), dev)
+        if not _all_whole(kept, T, D, HD, meta.heads, F, x.get_device()):
+            kept = _whole_kept(kept, _kept_shapes(T, D, HD, meta.heads, F), dev)
     else:
         chunk_bufs = {k: get(k, *sh, dev) for k, sh in _chunk_shapes(cmax, D, HD, meta.heads, F, tpn).items()}
         chunk_bufs["h1"], act_b = chunk_bufs.pop("h"), chunk_bufs["act"]
@@ -536,13 +548,17 @@ def _pool_alloc(peer_fn, gradient: bool = False):
     return getattr(getattr(peer_fn, "__self__", None), "gradient_buffer" if gradient else "output_buffer", None)
 
 
+# Names that PyTorch does not publish, looked up once: where a version lacks one, everything counts as recorded.
+_forward_level = forward_ad if hasattr(forward_ad, "_current_level") else SimpleNamespace(_current_level=0)
+_transforms_active = getattr(torch._C, "_are_functorch_transforms_active", lambda: True)
+_tracing_state = getattr(torch._C, "_get_tracing_state", lambda: True)
+
+
 def recorded() -> bool:
     """Whether anything would notice if an autograd function's forward ran as a plain call: a graph under construction, a
-    forward-mode level, a function transform, a trace. Sampling has none of them; the wrapper costs about 15 us. PyTorch has
-    no public names for the last three: where a private one is gone, everything counts as recorded."""
-    return (torch.is_grad_enabled() or getattr(forward_ad, "_current_level", 0) >= 0
-            or getattr(torch._C, "_are_functorch_transforms_active", lambda: True)()
-            or getattr(torch._C, "_get_tracing_state", lambda: True)() is not None)
+    forward-mode level, a function transform, a trace. Sampling has none of them; the wrapper costs about 15 us."""
+    return (torch.is_grad_enabled() or _forward_level._current_level >= 0 or _transforms_active()
+            or _tracing_state() is not None)
 
 
 def run_block(x, mod, meta: BlockMeta, wn1, wqkv, wo, wn2, w1, w2, regroup=None, out_alloc=None) -> torch.Tensor:
@@ -580,7 +596,7 @@ class FusedBlock(torch.autograd.Function):
             shapes = _kept_shapes(regroup[0].numel() if regroup is not None else x.shape[0], x.shape[1],
                                   meta.heads * meta.head_dim, meta.heads, w2.shape[1])
             try:
-                kept = {k: torch.empty(shape, dtype=dt, device=x.device) for k, (shape, dt) in shapes.items()}
+                kept = FreshKept({k: torch.empty(shape, dtype=dt, device=x.device) for k, (shape, dt) in shapes.items()})
             except torch.OutOfMemoryError:
                 kept = None            # free in sum but not in pieces of this size: recompute instead
         x, y = _block_output(x, mod, meta, (wn1, wqkv, wo, wn2, w1, w2), regroup, out_alloc, kept)
