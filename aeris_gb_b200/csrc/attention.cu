@@ -1501,14 +1501,14 @@ static int attn_fwd_impl(const void* q, int ldq, int q_col0, const void* k, int 
   auto at = [](const void* base, int col) -> const void* { return reinterpret_cast<const __nv_bfloat16*>(base) + col; };
   if ((r = make_tmap_heads_bf16(&tq, at(q, q_col0), head_dim, H, N, n_win, ldq, TILE))) return r;
   // Two query tiles at a time where there are two; its masked columns need a positive scale. ms, windows x tokens, one tile
-  // at a time / two, 24 heads x 64 and 12 x 128:
+  // at a time / two in turn, 24 heads x 64 and 12 x 128:
   // - Three or five tiles of which the last is not full leave the second chain idle for a third or a fifth of the time.
-  //   64-wide heads are faster without then (249 x 260 tokens 0.377 / 0.417, 202 x 320 0.347 / 0.364, 221 x 513 0.866 /
-  //   0.927, 175 x 576 0.743 / 0.813; full ones 168 x 384 0.348 / 0.332, 142 x 640 0.694 / 0.681; seven tiles 84 x 832 0.681
-  //   / 0.665, 97 x 772 0.734 / 0.750), 128-wide ones are not (249 x 260 0.306 / 0.295, 175 x 576 0.590 / 0.577).
-  // - A last half tile that is cut off (CUT) costs every tile: short windows only. 64: 240 tokens 0.302 / 0.246, 500 0.449 /
-  //   0.383, 740 0.728 / 0.685, 970 0.654 / 0.674, 1500 0.588 / 0.605, 3600 0.496 / 0.538. 128: 740 0.572 / 0.461, 1250
-  //   0.477 / 0.422, 1500 0.442 / 0.431, 2000 0.407 / 0.425, 3600 0.350 / 0.374.
+  //   64-wide heads are faster without then (249 x 260 tokens 0.387 / 0.416, 202 x 320 0.348 / 0.352, 221 x 513 0.857 /
+  //   0.925, 175 x 576 0.732 / 0.772; full ones 168 x 384 0.363 / 0.337, 142 x 640 0.689 / 0.664; seven tiles 84 x 832 0.692
+  //   / 0.667, 97 x 772 0.758 / 0.754), 128-wide ones are not (249 x 260 0.325 / 0.295, 175 x 576 0.621 / 0.550).
+  // - A last half tile that is cut off (CUT) costs every tile: short windows only. 64: 240 tokens 0.295 / 0.243, 500 0.458 /
+  //   0.393, 740 0.726 / 0.689, 970 0.661 / 0.680, 1250 0.635 / 0.624, 1500 0.588 / 0.605, 3600 0.498 / 0.538. 128: 740
+  //   0.577 / 0.458, 1250 0.481 / 0.423, 1500 0.441 / 0.421, 2000 0.417 / 0.423, 3600 0.360 / 0.372.
   const int q_tiles = (N + TILE - 1) / TILE;
   const bool idle_chain = head_dim <= 64 && (q_tiles == 3 || q_tiles == 5) && N % TILE != 0;
   const bool cut = N % KVT > 4, long_cut = cut && q_tiles > (head_dim > 64 ? 12 : 6);

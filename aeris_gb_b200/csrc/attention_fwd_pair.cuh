@@ -10,9 +10,9 @@
 // computed under the softmax; at 128 it lies over the scores, whose successors then wait for P V, and the chains take turns.
 // The output is that of attn_fwd_kernel in every bit (reference maximum and sums go by 64 columns as there) unless the
 // second half of a tile raises the reference maximum. Against one tile at a time, in turn under the power cap, ms, windows
-// x tokens, 24 heads x 64 / 12 x 128: 72 x 900 0.726 -> 0.667 / 0.548 -> 0.491; 253 x 256 0.298 -> 0.215 / 0.266 -> 0.161;
-// 288 x 225 0.309 -> 0.259 / 0.281 -> 0.180; 502 x 129 0.367 -> 0.327 / 0.301 -> 0.221; 55 x 1024 0.644 -> 0.549 / 0.483 ->
-// 0.399; 8 x 900, 4 x 64: 0.0226 -> 0.0202. Maximum and sum over whole tiles would save 1-2 %, and 5-10 % where CUT.
+// x tokens, 24 heads x 64 / 12 x 128: 72 x 900 0.734 -> 0.662 / 0.565 -> 0.487; 253 x 256 0.308 -> 0.216 / 0.275 -> 0.166;
+// 288 x 225 0.303 -> 0.258 / 0.284 -> 0.182; 502 x 129 0.367 -> 0.318 / 0.307 -> 0.216; 55 x 1024 0.646 -> 0.543 / 0.489 ->
+// 0.396; 8 x 900, 4 x 64: 0.0247 -> 0.0218. Maximum and sum over whole tiles would save 1-2 %, and 5-10 % where CUT.
 // Tried: one piece of straight code per full tile and a rolled loop for the last one (no gain at 900 tokens, 225: 0.168 ->
 // 0.190); strict turns of the two chains at the exponentials (0.620 -> 0.677); one warp for the products of both chains is
 // not needed: issuing a tile's twelve products and their commits takes 400 cycles of 3,000.
