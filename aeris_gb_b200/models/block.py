@@ -37,10 +37,16 @@ def takes(meta, x: torch.Tensor, mod: torch.Tensor, weights, grads=()) -> bool:
     """Whether the native call takes this block: bf16 operands without gaps, fp32 modulation and gradients, heads of whole
     16-byte vectors, none of the exchanges of the parallel paths. Everything else is issued (or refused) call by call."""
     d = meta.head_dim
-    return (meta.sp is None and meta.tp is None and (d in (64, 128) or (d % 8 == 0 and 0 < d < 128))
-            and mod.dtype == torch.float32 and mod.is_cuda
-            and _plain(x, torch.bfloat16) and all(_plain(w, torch.bfloat16) for w in weights)
-            and all(_plain(g, torch.float32) for g in grads))
+    if not (meta.sp is None and meta.tp is None and (d in (64, 128) or (d % 8 == 0 and 0 < d < 128))
+            and mod.dtype == torch.float32 and mod.is_cuda and _plain(x, torch.bfloat16)):
+        return False
+    for w in weights:
+        if not _plain(w, torch.bfloat16):
+            return False
+    for g in grads:
+        if not _plain(g, torch.float32):
+            return False
+    return True
 
 
 WEIGHTS = ("n1", "to_qkv", "wo", "n2", "w1", "w2")
@@ -49,19 +55,19 @@ WEIGHTS = ("n1", "to_qkv", "wo", "n2", "w1", "w2")
 def fits(meta, x: torch.Tensor, mod: torch.Tensor, weights, rows=(), grads=None, table=None) -> bool:
     """Whether every operand has the extents that the native call derives from ``x``, ``w2`` and ``meta``: it has no other
     check. ``rows``: tensors shaped like ``x``; ``grads``: as :func:`.fused.block_backward` takes them. What does not fit
-    goes launch by launch, where each is checked by itself. Written out: 2 us of host time forward, 3.5 backward."""
+    goes launch by launch, where each is checked by itself. Every pass over a block asks: what :func:`takes` has found to be
+    whole is compared by its number of elements where another shape of as many reads the same."""
     n1, to_qkv, wo, n2, w1, w2 = weights
-    xs = x.shape
-    (T, D), F, HD, B = xs, w2.shape[1], meta.heads * meta.head_dim, mod.shape[0]
+    xs, ms, w2_shape, HD = x.shape, mod.shape, w2.shape, meta.heads * meta.head_dim
+    (T, D), F = xs, w2_shape[1]
     qkv_shape, w1_shape = (3 * HD, D), (2 * F, D)
-    if (T != B * meta.n_win_per_sample * meta.L or mod.shape != (B, 6 * D) or to_qkv.shape != qkv_shape
-            or wo.shape != (D, HD) or w1.shape != w1_shape or w2.shape[0] != D or n1.shape != (D,) or n2.shape != (D,)
+    if (T != ms[0] * meta.n_win_per_sample * meta.L or ms != (ms[0], 6 * D) or to_qkv.shape != qkv_shape
+            or wo.shape != (D, HD) or w1.shape != w1_shape or w2_shape != (D, F) or n1.numel() != D or n2.numel() != D
             or (table is not None and table.numel() != T)):
         return False
     for r in rows:
         if r.shape != xs:
             return False
-    # the other gradients are added to element by element, whatever their shape
     return grads is None or (grads["to_qkv"].shape == qkv_shape and grads["w1"].shape == w1_shape
                              and grads["wo"].numel() == D * HD and grads["w2"].numel() == D * F
                              and grads["n1"].numel() == D and grads["n2"].numel() == D)

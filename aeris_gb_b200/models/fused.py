@@ -374,7 +374,8 @@ def block_forward(x: torch.Tensor, mod: torch.Tensor, meta: BlockMeta, wn1, wqkv
     spans = _forward_spans(meta, B, step, D, F, kept is not None)
     weights = (wn1, wqkv, wo, wn2, w1, w2)
     table = gather[0] if gather is not None else None
-    native = (NB.takes(meta, x, mod, (*weights, y)) and NB.fits(meta, x, mod, weights, (y,), table=table)
+    rows = () if out is None else (out,)
+    native = (NB.takes(meta, x, mod, (*weights, *rows)) and NB.fits(meta, x, mod, weights, rows, table=table)
               and (kept is None or type(kept) is FreshKept or _all_whole(kept, T, D, HD, meta.heads, F, x.get_device())))
     if not native:
         NB.refuse_misfits(meta, x, mod, weights, table=table)
