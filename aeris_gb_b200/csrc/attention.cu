@@ -7,11 +7,9 @@
 // Data layout: tokens are window-major, rows [w*N, (w+1)*N) belong to window w; Q, K, V are column slices of a
 // row-major [T, ld] bf16 tensor (the fused qkv projection output, columns ordered (q|k|v, head, d)).
 //
-// Roles in the kernels of this file: warp 0 = TMA producer, warp 1 = MMA issuer and TMEM owner, and warpgroups of math
-// warps, one thread per tile row, that work straight out of TMEM. The forward kernel has one such group (warps 2..5 of 192
-// threads). The backward kernels have two or three from warp 4 on (384 or 512 threads); warps 2 and 3 fetch the row
-// statistics there. The forward kernel for windows of several query tiles (attention_fwd_pair.cuh) has its two softmax
-// groups first, then a producer warp and one issuer warp per group.
+// Roles in the kernel of this file: warp 0 = TMA producer, warp 1 = MMA issuer and TMEM owner, warps 2..5 = softmax, one
+// thread per tile row, working straight out of TMEM. The forward kernel for windows of several query tiles
+// (attention_fwd_pair.cuh) and the backward kernels (attention_bwd.cuh) are described there.
 #include "common.cuh"
 #include "api.h"
 #include "host.h"
@@ -535,895 +533,7 @@ static int launch_attn_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const C
 }  // namespace aeris
 
 #include "attention_fwd_pair.cuh"
-
-namespace aeris {
-
-// -------------------------------------------------------------------------------------------------------- backward
-// Two kernels, neither needs atomics:
-//   attn_bwd_dq : items of one 128-row Q tile, K/V streamed in 64-row tiles.  S = Q K^T, dP = dO V^T,
-//                 dS = P * (dP - delta), dQ = scale * sum dS K.   Also writes delta = rowsum(dO * O).
-//   attn_bwd_dkv: items of one 128-row K/V tile, Q/dO streamed in 64-row tiles. S^T = K Q^T, dP^T = V dO^T,
-//                 dV += P^T dO, dK = scale * sum dS^T Q.
-// What bounds them is the chain MMA -> commit -> TMEM load -> exponentials -> hand-over -> MMA: every link costs 200-300
-// cycles of latency, so one tile in flight leaves the tensor core idle most of the time. Both kernels therefore run
-// one persistent CTA per SM with NWG warpgroups of math warps, each with score buffers of its own in tensor memory and
-// every NWG-th tile of the stream, so NWG chains are always in flight; the chains run on across work items (operands of
-// the next item are prefetched, its first scores are computed under the epilogue of the current one). P and dS go
-// back into the tensor memory columns they came from and are the A operand of the accumulating products from there:
-// no shared-memory round trip, and the B operand is all that those products read from shared memory.
-// Both kernels together, before (two 32-column halves in flight per CTA, P and dS through shared memory) and now:
-// 72 windows x 900 tokens, 24 heads x 64: 2.61 -> 1.72 ms; 12 heads x 128: 2.67 -> 1.49 ms; 16 windows x 3600 tokens,
-// 12 heads x 128: 7.05 -> 3.80 ms (12 launches each from an idle clock; 1.91, 1.69 and 4.35 ms held for 0.6 s, at
-// 1740, 1725 and 1665 MHz under the power cap).
-struct AttnBwdParams {
-  const __nv_bfloat16* O;   // forward output, [T, ldo]
-  const __nv_bfloat16* dO;  // [T, ldo]
-  int ldo;
-  const float* lse;         // [n_win*H*N] log2 domain
-  float* delta;             // [n_win*H*N]
-  __nv_bfloat16* dQKV;      // [T, ldg] gradient of the fused qkv tensor
-  int ldg;
-  int N, H, n_win;
-  int d;         // head width, at most the kernel's HD (the tensor maps pad with zeros)
-  int q_col0, k_col0, v_col0;
-  float scale_log2, scale;
-  int* status;
-  // Ulysses gradient push (null / 0 when unused): the gradient row of token `grow` goes to rank grow / push_n_local,
-  // row win * push_n_local + grow % push_n_local, column section * push_sec_w + push_col0 + head * d.
-  void* dq_peers[8];
-  int push_n_local, push_ld, push_sec_w, push_col0;
-};
-constexpr int BT = 64;      // rows of a streamed tile
-
-__device__ __forceinline__ __nv_bfloat16* bwd_dst(const AttnBwdParams& p, int win, int grow, int head, int section,
-                                                  int local_col0) {
-  if (p.push_n_local > 0) {
-    const int owner = grow / p.push_n_local;
-    return reinterpret_cast<__nv_bfloat16*>(p.dq_peers[owner]) +
-           (static_cast<size_t>(win) * p.push_n_local + (grow - owner * p.push_n_local)) * p.push_ld +
-           section * p.push_sec_w + p.push_col0 + head * p.d;
-  }
-  return p.dQKV + (static_cast<size_t>(win) * p.N + grow) * p.ldg + local_col0 + head * p.d;
-}
-
-// Chains, ring depth and copies of the item's own operands per head width; the shared memory of one CTA per SM (227 KB)
-// and its 512 TMEM columns set them: NWG * 128 score columns + the accumulators (dQ: HD, dK and dV: 2 HD).
-// The ring holds 2 * NWG tiles. That is also what makes `next_full` sound, the one barrier per chain and round that the
-// MMA thread waits on: it completes when the four math warps have handed over tile t AND the loads of tile t + NWG have
-// landed. The producer may arm it for tile t + NWG only when the previous round is complete, which the slot it waits
-// for (freed by the products of tile t - NWG) implies. One wait, one fence and two commits per tile matter because each
-// costs the MMA thread 60-200 cycles: with separate barriers for the operands that thread was the bottleneck.
-template <int DCH> struct BwdRing {
-  static constexpr int NWG = (DCH == 1) ? 3 : 2;
-  static constexpr int NST = 2 * NWG;
-  static constexpr int NB = (DCH == 1) ? 2 : 1;         // buffers for the item's own 128-row operands
-  static constexpr int ITEM_BYTES = 2 * DCH * 16384, STAGE = 2 * DCH * 8192;
-  static constexpr int STAT = 4 * TILE > NST * 2 * BT ? 4 * TILE : NST * 2 * BT;
-  static constexpr bool STAGED = DCH == 2;              // gradient rows leave through shared memory, see BwdOut
-  static constexpr int OUT_BYTES = STAGED ? 2 * TILE * 64 : 0;  // two buffers of 32 columns, per warpgroup
-  static constexpr int SMEM = NB * ITEM_BYTES + NST * STAGE + NWG * OUT_BYTES + STAT * 4 + 512;
-  static constexpr int THREADS = 128 + 128 * NWG;
-};
-static_assert(BwdRing<1>::SMEM <= 227 * 1024 && BwdRing<2>::SMEM <= 227 * 1024, "shared memory");
-
-// Asynchronous 4-byte copy (`bytes` = 0: zero fill), and this lane's arrival on a barrier once its copies have landed.
-__device__ __forceinline__ void cp_async4(float* smem_dst, const float* src, uint32_t bytes) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(smem_dst)), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-// Gradient rows on their way out: a warp turns 32 accumulator columns of its 32 rows into bf16 in shared memory, one lane
-// hands them to the TMA unit as a tiled store. The accumulator is free once it has been read; written by the threads
-// themselves (one row each, 32 rows with every 16-byte store instruction) it kept the next item's products waiting. Rows
-// past the window's end and columns past the head's width are clipped by the tensor map. No warp waits for another one's
-// rows. Both kernels, ms, direct stores / now, in turn, 12 heads x 128: 400 x 128 tokens 0.548 / 0.456, 200 x 225 0.631 /
-// 0.535, 72 x 900 1.73 / 1.61, 16 x 3600 4.50 / 4.31; with one buffer a warp 0.527, 0.602, 1.59 and 4.35. At 64, with a
-// third of the columns per warpgroup, staging (of a warpgroup's 128 rows at a time) cost more than it saved (24 x 64, 200 x
-// 225: 0.650 -> 0.704, 72 x 900 1.91 -> 1.92): direct stores there.
-struct BwdOut {
-  uint8_t* stage;           // this warp's two: 32 rows of 64 bytes, the vectors of 16 swizzled as the tensor map has it
-  int lane, first_row;      // of this warp inside the tile
-  int n = 0;                // groups of columns so far
-
-  // `read`: called once the columns are out of tensor memory
-  template <typename F>
-  __device__ __forceinline__ void put(uint32_t taddr, float f, const CUtensorMap* m, int col, int head, int tile_row,
-                                      int win, int N, F&& read) {
-    uint32_t v[32];
-    tmem_ld32(taddr, v);
-    tmem_wait_ld();
-    read();
-    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-    __syncwarp();
-    uint8_t* buf = stage + (n++ & 1) * 2048;
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-      uint32_t o[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        o[i] = pack_bf16x2(__uint_as_float(v[8 * g + 2 * i]) * f, __uint_as_float(v[8 * g + 2 * i + 1]) * f);
-      *reinterpret_cast<uint4*>(buf + lane * 64 + ((g ^ ((lane >> 1) & 3)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-    }
-    fence_proxy_async_smem();
-    __syncwarp();
-    if (lane == 0) {
-      if (tile_row + first_row < N)
-        tma_store_4d(m, buf, col, head, tile_row + first_row, win);
-      else                  // no rows: an empty group, so that the buffers still come free in turn
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-    }
-    __syncwarp();           // the warp goes on as one: the next step reads tensor memory
-  }
-  // before this warp leaves: its copies have been performed
-  __device__ __forceinline__ void drain() const {
-    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-  }
-};
-
-// Position of a role in the CTA's stream of tiles: item `it` (of this CTA), tile `j` of the item, running number `g`.
-struct TileIter {
-  int it = 0, j = 0, g = 0;
-  __device__ __forceinline__ void next(int n_tiles) {
-    ++g;
-    if (++j == n_tiles) { j = 0; ++it; }
-  }
-};
-struct BwdItem {
-  int tile, head, win;
-};
-// Items of one (window, head) are neighbours, so the CTAs at work share their streamed operands in L2.
-__device__ __forceinline__ BwdItem bwd_item(int it, int n_row_tiles, int H) {
-  const int idx = blockIdx.x + it * gridDim.x;
-  const int wh = idx / n_row_tiles;
-  BwdItem b;
-  b.tile = idx - wh * n_row_tiles;
-  b.win = wh / H;
-  b.head = wh - b.win * H;
-  return b;
-}
-
-template <int DCH>
-__global__ void __launch_bounds__(128 + 128 * BwdRing<DCH>::NWG, 1)
-attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-                   const __grid_constant__ CUtensorMap tm_dq, const AttnBwdParams p, const int n_items_total) {
-  using R = BwdRing<DCH>;
-  constexpr int HD = 64 * DCH;
-  constexpr int QB = DCH * 16384;       // Q tile, dO tile (128 rows)
-  constexpr int KB = DCH * 8192;        // K tile, V tile (64 rows)
-  constexpr int NWG = R::NWG, NST = R::NST, NB = R::NB;
-  static_assert(NWG * 128 + HD <= 512, "TMEM columns");
-  extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t* sQ = smem;                   // [NB] items: Q | dO
-  uint8_t* sKV = sQ + NB * R::ITEM_BYTES;                    // [NST] K | V
-  uint8_t* sOut = sKV + NST * R::STAGE;                      // [NWG]
-  float* s_stat = reinterpret_cast<float*>(sOut + NWG * R::OUT_BYTES);   // [2] items: lse [128] | delta [128]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_stat + R::STAT);
-  uint64_t* q_full = bars;              // [NB <= 2]
-  uint64_t* q_empty = bars + 2;         // [NB]
-  uint64_t* first_full = bars + 4;      // [NWG <= 3] K and V of the first tile of each chain
-  uint64_t* next_full = bars + 7;       // [NWG] dS of the chain's tile is in TMEM, K and V of its next tile have landed
-  uint64_t* kv_empty = bars + 10;       // [NST <= 6]
-  uint64_t* sp_full = bars + 16;        // [NWG] scores and dP of a tile are in the chain's TMEM columns
-  uint64_t* acc_full = bars + 19;
-  uint64_t* acc_empty = bars + 20;
-  uint64_t* stat_full = bars + 21;      // [2]
-  uint64_t* stat_empty = bars + 23;     // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 25);
-  int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int N = p.N;
-  const int nfull = N / BT, rem = N - nfull * BT;
-  const int nkv = nfull + (rem ? 1 : 0);
-  const int n_last = rem ? ((rem + 15) & ~15) : BT;
-  const int row_tiles = (N + TILE - 1) / TILE;
-  const int n_ctas = static_cast<int>(gridDim.x);
-  const int n_items = (n_items_total - static_cast<int>(blockIdx.x) + n_ctas - 1) / n_ctas;
-
-  if (threadIdx.x == 0) {
-    int ab = (p.status && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
-    if ((smem_u32(smem) & 1023u) != 0) { ab = 1; if (p.status) atomicCAS(p.status, 0, ERR_BOUNDS); }
-    *s_abort = ab;
-  }
-  __syncthreads();
-  if (*s_abort) return;
-  if (threadIdx.x == 0) {
-    prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v); prefetch_tmap(&tm_do);
-    for (int i = 0; i < 2; ++i) { mbar_init(&stat_full[i], 2); mbar_init(&stat_empty[i], 4 * NWG); }
-    for (int i = 0; i < NB; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); }
-    for (int i = 0; i < NST; ++i) mbar_init(&kv_empty[i], 1);
-    for (int i = 0; i < NWG; ++i) {
-      mbar_init(&first_full[i], 1);
-      mbar_init(&next_full[i], 4 + 1);
-      mbar_init(&sp_full[i], 1);
-    }
-    mbar_init(acc_full, 1); mbar_init(acc_empty, 4 * NWG);
-    fence_barrier_init();
-  }
-  if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tdQ = tmem_base + NWG * 128;      // chain w: S at w * 128, dP at w * 128 + 64
-
-  if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer
-    if (elect_one_sync()) {
-      auto load_item = [&](int it) -> bool {
-        const int b = it % NB;
-        if (!mbar_wait(&q_empty[b], ((it / NB) & 1) ^ 1, p.status, ERR_TIMEOUT_ATTN)) return false;
-        const BwdItem w = bwd_item(it, row_tiles, p.H);
-        mbar_expect_tx(&q_full[b], R::ITEM_BYTES);
-        uint8_t* d = sQ + b * R::ITEM_BYTES;
-#pragma unroll
-        for (int c = 0; c < DCH; ++c) {
-          tma_load_4d(d + c * 16384, &tm_q, &q_full[b], c * 64, w.head, w.tile * TILE, w.win);
-          tma_load_4d(d + QB + c * 16384, &tm_do, &q_full[b], c * 64, w.head, w.tile * TILE, w.win);
-        }
-        return true;
-      };
-      bool ok = load_item(0);
-      int st = 0, t = 0;
-      uint32_t ph = 1;
-      // where an item's own operands are requested: with two buffers those of the next item early in this one, with one
-      // buffer those of this item behind its first tiles (they have to wait for the last scores of the item before)
-      const int j_item = min(NB == 2 ? 2 : NWG - 1, nkv - 1);
-      for (int it = 0; it < n_items && ok; ++it) {
-        const BwdItem w = bwd_item(it, row_tiles, p.H);
-        for (int j = 0; j < nkv; ++j, ++t) {
-          if (!mbar_wait(&kv_empty[st], ph, p.status, ERR_TIMEOUT_ATTN)) { ok = false; break; }
-          uint64_t* bar = t < NWG ? &first_full[t] : &next_full[t % NWG];
-          uint8_t* d = sKV + st * R::STAGE;
-          mbar_expect_tx(bar, R::STAGE);
-#pragma unroll
-          for (int c = 0; c < DCH; ++c) {
-            tma_load_4d(d + c * 8192, &tm_k, bar, c * 64, w.head, j * BT, w.win);
-            tma_load_4d(d + KB + c * 8192, &tm_v, bar, c * 64, w.head, j * BT, w.win);
-          }
-          if (++st == NST) { st = 0; ph ^= 1; }
-          if (j == j_item) {
-            if (NB == 2 && it + 1 < n_items && !load_item(it + 1)) { ok = false; break; }
-            if (NB == 1 && it > 0 && !load_item(it)) { ok = false; break; }
-          }
-        }
-      }
-      // the last tile of each chain has no successor: its round completes without loads
-      for (int e = t + NWG; t < e && ok; ++t) {
-        if (!mbar_wait(&kv_empty[st], ph, p.status, ERR_TIMEOUT_ATTN)) break;
-        if (t >= NWG) mbar_arrive(&next_full[t % NWG]);
-        if (++st == NST) { st = 0; ph ^= 1; }
-      }
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    if (elect_one_sync()) {
-      const uint32_t aI = smem_u32(sQ), aS = smem_u32(sKV);
-      const int total = n_items * nkv;
-      TileIter s;                       // next tile whose scores are issued
-      int s_w = 0, s_st = 0;
-      // S = Q K_j^T and dP = dO V_j^T of tile s
-      auto issue_sp = [&]() -> bool {
-        const int b = s.it % NB;
-        if (s.j == 0) {
-          if (!mbar_wait(&q_full[b], (s.it / NB) & 1, p.status, ERR_TIMEOUT_ATTN)) return false;
-          tc_fence_after();
-        }
-        const bool last = s.j == nkv - 1;
-        const uint32_t idesc = make_idesc_bf16(TILE, last ? n_last : BT, 0, 0);
-        const uint32_t tS = tmem_base + s_w * 128;
-        const uint64_t d0 = make_smem_desc(aI + b * R::ITEM_BYTES, 0, 1024), d1 = d0 + QB / 16;
-        const uint64_t d2 = make_smem_desc(aS + s_st * R::STAGE, 0, 1024), d3 = d2 + KB / 16;
-#pragma unroll
-        for (int kk = 0; kk < 4 * DCH; ++kk)
-          umma_ss(tS, d0 + ((kk >> 2) * 16384 + (kk & 3) * 32) / 16, d2 + ((kk >> 2) * 8192 + (kk & 3) * 32) / 16, idesc,
-                  kk > 0);
-#pragma unroll
-        for (int kk = 0; kk < 4 * DCH; ++kk)
-          umma_ss(tS + 64, d1 + ((kk >> 2) * 16384 + (kk & 3) * 32) / 16, d3 + ((kk >> 2) * 8192 + (kk & 3) * 32) / 16,
-                  idesc, kk > 0);
-        tc_commit(&sp_full[s_w]);
-        if (last) tc_commit(&q_empty[b]);
-        if (++s_w == NWG) s_w = 0;
-        if (++s_st == NST) s_st = 0;
-        s.next(nkv);
-        return true;
-      };
-      bool ok = true;
-      for (int i = 0; i < NWG && i < total && ok; ++i) {
-        ok = mbar_wait(&first_full[i], 0, p.status, ERR_TIMEOUT_ATTN);
-        tc_fence_after();
-        if (ok) ok = issue_sp();
-      }
-      int w = 0, st = 0;
-      uint32_t ph = 0;
-      TileIter a;
-      constexpr uint32_t idesc_acc = make_idesc_bf16(TILE, HD, 0, 1);
-      while (ok && a.g < total) {
-        if (!mbar_wait(&next_full[w], ph, p.status, ERR_TIMEOUT_ATTN)) break;
-        if (a.j == 0 && a.it > 0 && !mbar_wait(acc_empty, (a.it - 1) & 1, p.status, ERR_TIMEOUT_ATTN)) break;
-        tc_fence_after();
-        const bool last = a.j == nkv - 1;
-        const uint32_t acc0 = a.j > 0 ? 1u : 0u;
-        const uint32_t tA = tmem_base + w * 128;
-        // dQ += dS_j K_j : A = dS (TMEM, 16 kv columns = 8 words per K step), B = K MN-major (d contiguous)
-        const uint64_t dk = make_smem_desc(aS + st * R::STAGE, 8192, 1024);
-        if (!last || rem == 0) {
-#pragma unroll
-          for (int kk = 0; kk < BT / 16; ++kk) umma_ts(tdQ, tA + kk * 8, dk + kk * 128, idesc_acc, kk ? 1u : acc0);
-        } else {
-          for (int kk = 0; kk < n_last / 16; ++kk) umma_ts(tdQ, tA + kk * 8, dk + kk * 128, idesc_acc, kk ? 1u : acc0);
-        }
-        tc_commit(&kv_empty[st]);
-        if (last) tc_commit(acc_full);
-        // the tensor core executes in issue order: these scores overwrite the A operand above only after it was read
-        if (s.g < total && !issue_sp()) break;
-        if (++w == NWG) { w = 0; ph ^= 1; }
-        if (++st == NST) st = 0;
-        a.next(nkv);
-      }
-    }
-  } else if (warp < 4) {
-    // ------------------------------------------------------------ lse and delta of the rows of the coming items (two warps)
-    constexpr int LPR = HD / 8, RPW = 32 / LPR;      // lanes per row, rows per warp and load
-    constexpr int UN = 8;                            // loads in flight: an item must not wait for its statistics
-    const int sub = lane % LPR, r0 = lane / LPR, half = (warp - 2) * (TILE / 2);
-    for (int it = 0; it < n_items; ++it) {
-      const int b = it & 1;
-      if (!mbar_wait(&stat_empty[b], ((it >> 1) & 1) ^ 1, p.status, ERR_TIMEOUT_ATTN)) break;
-      const BwdItem w = bwd_item(it, row_tiles, p.H);
-      float* st = s_stat + b * 2 * TILE;
-      const size_t sbase = (static_cast<size_t>(w.win) * p.H + w.head) * N + w.tile * TILE;
-      const size_t obase = (static_cast<size_t>(w.win) * N + w.tile * TILE) * p.ldo + w.head * p.d + sub * 8;
-      const int live = N - w.tile * TILE;            // rows of this tile inside the window
-      float lse[2];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int row = half + u * 32 + lane;
-        lse[u] = (row < live) ? p.lse[sbase + row] : 0.f;
-      }
-#pragma unroll 1
-      for (int r = half; r < half + TILE / 2; r += RPW * UN) {
-        uint4 a[UN], g[UN];
-#pragma unroll
-        for (int u = 0; u < UN; ++u) {
-          const int row = r + u * RPW + r0;
-          a[u] = g[u] = make_uint4(0u, 0u, 0u, 0u);
-          if (row < live && sub * 8 < p.d) {
-            a[u] = *reinterpret_cast<const uint4*>(p.O + obase + static_cast<size_t>(row) * p.ldo);
-            g[u] = *reinterpret_cast<const uint4*>(p.dO + obase + static_cast<size_t>(row) * p.ldo);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < UN; ++u) {
-          const uint32_t aw[4] = {a[u].x, a[u].y, a[u].z, a[u].w}, gw[4] = {g[u].x, g[u].y, g[u].z, g[u].w};
-          float d = 0.f;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float2 x = unpack_bf16x2(aw[i]), y = unpack_bf16x2(gw[i]);
-            d = fmaf(x.x, y.x, d);
-            d = fmaf(x.y, y.y, d);
-          }
-#pragma unroll
-          for (int o = LPR / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-          const int row = r + u * RPW + r0;
-          if (sub == 0) {
-            st[TILE + row] = d;
-            if (row < live) p.delta[sbase + row] = d;
-          }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u) st[half + u * 32 + lane] = lse[u];
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&stat_full[b]);
-    }
-  } else if (warp >= 4) {
-    // ------------------------------------------------------------ math: one thread = one Q row, every NWG-th tile
-    const int wg = (warp >> 2) - 1, q = warp & 3;
-    const int row = q * 32 + lane;
-    const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
-    const uint32_t tS = tmem_base + lane_addr + wg * 128, tdP = tS + 64;
-    const uint64_t sl = f2_pack(p.scale_log2, p.scale_log2);
-    const float sc = p.scale;
-    uint32_t ph = 0;
-    int j = wg;                       // first tile of this warpgroup in the item at hand
-    bool ok = true;
-    BwdOut out{sOut + wg * R::OUT_BYTES + q * 4096, lane, q * 32};
-    // Gradient rows of item `it` from TMEM to memory. Runs after this warpgroup's first tile of the NEXT item, so that the
-    // wait for the last products of `it` is spent on that tile.
-    auto epilogue = [&](int it) -> bool {
-      if (!mbar_wait(acc_full, it & 1, p.status, ERR_TIMEOUT_ATTN)) return false;
-      tc_fence_after();
-      const BwdItem w = bwd_item(it, row_tiles, p.H);
-      auto release = [&]() {
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(acc_empty);
-      };
-      if (R::STAGED && p.push_n_local == 0) {
-        int mine = 0;                   // this warpgroup's groups of 32 columns
-        for (int c = wg * 32; c < p.d; c += 32 * NWG) ++mine;
-        if (mine == 0) release();
-        for (int c = wg * 32; c < p.d; c += 32 * NWG)
-          out.put(tdQ + lane_addr + c, sc, &tm_dq, c, w.head, w.tile * TILE, w.win, N,
-                  [&] { if (--mine == 0) release(); });
-        return true;
-      }
-      const int grow = w.tile * TILE + row;
-      const bool row_ok = grow < N;
-      __nv_bfloat16* dst = bwd_dst(p, w.win, row_ok ? grow : 0, w.head, 0, p.q_col0);
-#pragma unroll
-      for (int c = 0; c < HD; c += 32) {
-        if ((c / 32) % NWG != wg || c >= p.d) continue;
-        uint32_t v[32];
-        tmem_ld32(tdQ + lane_addr + c, v);
-        tmem_wait_ld();
-        if (row_ok) {
-#pragma unroll
-          for (int gq = 0; gq < 4; ++gq) {
-            uint32_t o[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              o[i] = pack_bf16x2(__uint_as_float(v[8 * gq + 2 * i]) * sc, __uint_as_float(v[8 * gq + 2 * i + 1]) * sc);
-            if (c + gq * 8 < p.d) *reinterpret_cast<uint4*>(dst + c + gq * 8) = make_uint4(o[0], o[1], o[2], o[3]);
-          }
-        }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(acc_empty);
-      return true;
-    };
-    for (int it = 0; it < n_items && ok; ++it) {
-      bool pending = it > 0;
-      const int b = it & 1;
-      if (!mbar_wait(&stat_full[b], (it >> 1) & 1, p.status, ERR_TIMEOUT_ATTN)) { ok = false; break; }
-      const float nlse = -s_stat[b * 2 * TILE + row], ndelta = -s_stat[b * 2 * TILE + TILE + row];
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&stat_empty[b]);
-      const uint64_t nl = f2_pack(nlse, nlse), nd = f2_pack(ndelta, ndelta);
-      for (; j < nkv; j += NWG, ph ^= 1) {
-        if (!mbar_wait(&sp_full[wg], ph, p.status, ERR_TIMEOUT_ATTN)) { ok = false; break; }
-        tc_fence_after();
-        if (j < nfull) {
-#pragma unroll
-          for (int c = 0; c < 64; c += 32) {
-            uint32_t sv[32], dv[32], pk[16];
-            tmem_ld32(tS + c, sv);
-            tmem_ld32(tdP + c, dv);
-            tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              float t0, t1;
-              f2_unpack(f2_fma(f2_pack(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), sl, nl), t0, t1);
-              const uint64_t pr = f2_pack(mufu_exp2(t0), mufu_exp2(t1));
-              const uint64_t df = f2_add(f2_pack(__uint_as_float(dv[2 * i]), __uint_as_float(dv[2 * i + 1])), nd);
-              pk[i] = f2_to_bf16x2(f2_mul(pr, df));
-            }
-            // 32 scores become 16 words at column c / 2 <= c: only scores that were read are overwritten
-            tmem_st16(tS + (c >> 1), pk);
-          }
-        } else {
-          // columns past the window's end: their K rows are zeros, but an exponential may be infinite there
-#pragma unroll 1
-          for (int c = 0; c < n_last; c += 16) {
-            uint32_t sv[16], dv[16], pk[8];
-            tmem_ld16(tS + c, sv);
-            tmem_ld16(tdP + c, dv);
-            tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const float p0 = mufu_exp2(fmaf(__uint_as_float(sv[2 * i]), p.scale_log2, nlse));
-              const float p1 = mufu_exp2(fmaf(__uint_as_float(sv[2 * i + 1]), p.scale_log2, nlse));
-              float d0 = p0 * (__uint_as_float(dv[2 * i]) + ndelta);
-              float d1 = p1 * (__uint_as_float(dv[2 * i + 1]) + ndelta);
-              if (c + 2 * i >= rem) d0 = 0.f;
-              if (c + 2 * i + 1 >= rem) d1 = 0.f;
-              pk[i] = pack_bf16x2(d0, d1);
-            }
-            tmem_st8(tS + (c >> 1), pk);
-          }
-        }
-        tmem_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&next_full[wg]);
-        if (pending) {
-          pending = false;
-          if (!epilogue(it - 1)) { ok = false; break; }
-        }
-      }
-      if (!ok) break;
-      if (pending && !epilogue(it - 1)) { ok = false; break; }
-      j -= nkv;                        // the stream of tiles runs on into the next item
-    }
-    if (ok) epilogue(n_items - 1);
-    if (R::STAGED) out.drain();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  if (warp == 1) tmem_dealloc(tmem_base, 512);
-}
-
-template <int DCH>
-__global__ void __launch_bounds__(128 + 128 * BwdRing<DCH>::NWG, 1)
-attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-                    const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
-                    const AttnBwdParams p, const int n_items_total) {
-  using R = BwdRing<DCH>;
-  constexpr int HD = 64 * DCH;
-  constexpr int KB = DCH * 16384;  // K tile, V tile (128 rows)
-  constexpr int QB = DCH * 8192;   // Q tile, dO tile (64 rows)
-  constexpr int NWG = R::NWG, NST = R::NST, NB = R::NB;
-  static_assert(NWG * 128 + 2 * HD <= 512, "TMEM columns");
-  extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t* sKV = smem;                   // [NB] items: K | V
-  uint8_t* sQD = sKV + NB * R::ITEM_BYTES;                          // [NST] Q | dO
-  uint8_t* sOut = sQD + NST * R::STAGE;                             // [NWG]
-  float* s_stat = reinterpret_cast<float*>(sOut + NWG * R::OUT_BYTES);   // [NST] lse [64] | delta [64]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_stat + R::STAT);
-  uint64_t* kv_full = bars;              // [NB <= 2]
-  uint64_t* kv_empty = bars + 2;         // [NB]
-  uint64_t* first_full = bars + 4;       // [NWG <= 3] Q, dO and their row statistics for the first tile of each chain
-  uint64_t* next_full = bars + 7;        // [NWG] P and dS of the chain's tile are in TMEM, its next tile has landed
-  uint64_t* qd_empty = bars + 10;        // [NST <= 6]
-  uint64_t* sp_full = bars + 16;         // [NWG]
-  uint64_t* acc_full = bars + 19;
-  uint64_t* acc_empty = bars + 20;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
-  int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int N = p.N;
-  const int nfull = N / BT, rem = N - nfull * BT;
-  const int nq = nfull + (rem ? 1 : 0);
-  const int n_last = rem ? ((rem + 15) & ~15) : BT;
-  const int row_tiles = (N + TILE - 1) / TILE;
-  const int n_ctas = static_cast<int>(gridDim.x);
-  const int n_items = (n_items_total - static_cast<int>(blockIdx.x) + n_ctas - 1) / n_ctas;
-
-  if (threadIdx.x == 0) {
-    int ab = (p.status && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
-    if ((smem_u32(smem) & 1023u) != 0) { ab = 1; if (p.status) atomicCAS(p.status, 0, ERR_BOUNDS); }
-    *s_abort = ab;
-  }
-  __syncthreads();
-  if (*s_abort) return;
-  if (threadIdx.x == 0) {
-    prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v); prefetch_tmap(&tm_do);
-    for (int i = 0; i < NB; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1); }
-    for (int i = 0; i < NST; ++i) mbar_init(&qd_empty[i], 1);
-    // a tile's arrivals: the TMA loads and 32 lanes of row statistics (plus, from the second round on, four math warps)
-    for (int i = 0; i < NWG; ++i) {
-      mbar_init(&first_full[i], 1 + 32);
-      mbar_init(&next_full[i], 4 + 1 + 32);
-      mbar_init(&sp_full[i], 1);
-    }
-    mbar_init(acc_full, 1); mbar_init(acc_empty, 4 * NWG);
-    fence_barrier_init();
-  }
-  if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tdK = tmem_base + NWG * 128, tdV = tdK + HD;     // chain w: S^T at w * 128, dP^T at w * 128 + 64
-
-  if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer
-    if (elect_one_sync()) {
-      auto load_item = [&](int it) -> bool {
-        const int b = it % NB;
-        if (!mbar_wait(&kv_empty[b], ((it / NB) & 1) ^ 1, p.status, ERR_TIMEOUT_ATTN)) return false;
-        const BwdItem w = bwd_item(it, row_tiles, p.H);
-        mbar_expect_tx(&kv_full[b], R::ITEM_BYTES);
-        uint8_t* d = sKV + b * R::ITEM_BYTES;
-#pragma unroll
-        for (int c = 0; c < DCH; ++c) {
-          tma_load_4d(d + c * 16384, &tm_k, &kv_full[b], c * 64, w.head, w.tile * TILE, w.win);
-          tma_load_4d(d + KB + c * 16384, &tm_v, &kv_full[b], c * 64, w.head, w.tile * TILE, w.win);
-        }
-        return true;
-      };
-      bool ok = load_item(0);
-      int st = 0, t = 0;
-      uint32_t ph = 1;
-      // where an item's own operands are requested: with two buffers those of the next item early in this one, with one
-      // buffer those of this item behind its first tiles (they have to wait for the last scores of the item before)
-      const int j_item = min(NB == 2 ? 2 : NWG - 1, nq - 1);
-      for (int it = 0; it < n_items && ok; ++it) {
-        const BwdItem w = bwd_item(it, row_tiles, p.H);
-        for (int j = 0; j < nq; ++j, ++t) {
-          if (!mbar_wait(&qd_empty[st], ph, p.status, ERR_TIMEOUT_ATTN)) { ok = false; break; }
-          uint64_t* bar = t < NWG ? &first_full[t] : &next_full[t % NWG];
-          uint8_t* d = sQD + st * R::STAGE;
-          mbar_expect_tx(bar, R::STAGE);
-#pragma unroll
-          for (int c = 0; c < DCH; ++c) {
-            tma_load_4d(d + c * 8192, &tm_q, bar, c * 64, w.head, j * BT, w.win);
-            tma_load_4d(d + QB + c * 8192, &tm_do, bar, c * 64, w.head, j * BT, w.win);
-          }
-          if (++st == NST) { st = 0; ph ^= 1; }
-          if (j == j_item) {
-            if (NB == 2 && it + 1 < n_items && !load_item(it + 1)) { ok = false; break; }
-            if (NB == 1 && it > 0 && !load_item(it)) { ok = false; break; }
-          }
-        }
-      }
-      // the last tile of each chain has no successor: its round completes without loads
-      for (int e = t + NWG; t < e && ok; ++t) {
-        if (!mbar_wait(&qd_empty[st], ph, p.status, ERR_TIMEOUT_ATTN)) break;
-        if (t >= NWG) mbar_arrive(&next_full[t % NWG]);
-        if (++st == NST) { st = 0; ph ^= 1; }
-      }
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    if (elect_one_sync()) {
-      const uint32_t aI = smem_u32(sKV), aS = smem_u32(sQD);
-      const int total = n_items * nq;
-      TileIter s;                       // next tile whose scores are issued
-      int s_w = 0, s_st = 0;
-      // S^T = K Q_j^T and dP^T = V dO_j^T of tile s
-      auto issue_sp = [&]() -> bool {
-        const int b = s.it % NB;
-        if (s.j == 0) {
-          if (!mbar_wait(&kv_full[b], (s.it / NB) & 1, p.status, ERR_TIMEOUT_ATTN)) return false;
-          tc_fence_after();
-        }
-        const bool last = s.j == nq - 1;
-        const uint32_t idesc = make_idesc_bf16(TILE, last ? n_last : BT, 0, 0);
-        const uint32_t tS = tmem_base + s_w * 128;
-        const uint64_t d0 = make_smem_desc(aI + b * R::ITEM_BYTES, 0, 1024), d1 = d0 + KB / 16;
-        const uint64_t d2 = make_smem_desc(aS + s_st * R::STAGE, 0, 1024), d3 = d2 + QB / 16;
-#pragma unroll
-        for (int kk = 0; kk < 4 * DCH; ++kk)
-          umma_ss(tS, d0 + ((kk >> 2) * 16384 + (kk & 3) * 32) / 16, d2 + ((kk >> 2) * 8192 + (kk & 3) * 32) / 16, idesc,
-                  kk > 0);
-#pragma unroll
-        for (int kk = 0; kk < 4 * DCH; ++kk)
-          umma_ss(tS + 64, d1 + ((kk >> 2) * 16384 + (kk & 3) * 32) / 16, d3 + ((kk >> 2) * 8192 + (kk & 3) * 32) / 16,
-                  idesc, kk > 0);
-        tc_commit(&sp_full[s_w]);
-        if (last) tc_commit(&kv_empty[b]);
-        if (++s_w == NWG) s_w = 0;
-        if (++s_st == NST) s_st = 0;
-        s.next(nq);
-        return true;
-      };
-      bool ok = true;
-      for (int i = 0; i < NWG && i < total && ok; ++i) {
-        ok = mbar_wait(&first_full[i], 0, p.status, ERR_TIMEOUT_ATTN);
-        tc_fence_after();
-        if (ok) ok = issue_sp();
-      }
-      int w = 0, st = 0;
-      uint32_t ph = 0;
-      TileIter a;
-      constexpr uint32_t idesc_acc = make_idesc_bf16(TILE, HD, 0, 1);
-      while (ok && a.g < total) {
-        if (!mbar_wait(&next_full[w], ph, p.status, ERR_TIMEOUT_ATTN)) break;
-        if (a.j == 0 && a.it > 0 && !mbar_wait(acc_empty, (a.it - 1) & 1, p.status, ERR_TIMEOUT_ATTN)) break;
-        tc_fence_after();
-        const bool last = a.j == nq - 1;
-        const uint32_t acc0 = a.j > 0 ? 1u : 0u;
-        const uint32_t tA = tmem_base + w * 128;
-        // dV += P^T dO_j, dK += dS^T Q_j : A from TMEM (16 q columns = 8 words per K step), B MN-major (d contiguous)
-        const uint64_t dq = make_smem_desc(aS + st * R::STAGE, 8192, 1024), dg = dq + QB / 16;
-        if (!last || rem == 0) {
-#pragma unroll
-          for (int kk = 0; kk < BT / 16; ++kk) umma_ts(tdV, tA + kk * 8, dg + kk * 128, idesc_acc, kk ? 1u : acc0);
-#pragma unroll
-          for (int kk = 0; kk < BT / 16; ++kk) umma_ts(tdK, tA + 64 + kk * 8, dq + kk * 128, idesc_acc, kk ? 1u : acc0);
-        } else {
-          for (int kk = 0; kk < n_last / 16; ++kk) umma_ts(tdV, tA + kk * 8, dg + kk * 128, idesc_acc, kk ? 1u : acc0);
-          for (int kk = 0; kk < n_last / 16; ++kk) umma_ts(tdK, tA + 64 + kk * 8, dq + kk * 128, idesc_acc, kk ? 1u : acc0);
-        }
-        tc_commit(&qd_empty[st]);
-        if (last) tc_commit(acc_full);
-        // the tensor core executes in issue order: these scores overwrite the A operand above only after it was read
-        if (s.g < total && !issue_sp()) break;
-        if (++w == NWG) { w = 0; ph ^= 1; }
-        if (++st == NST) st = 0;
-        a.next(nq);
-      }
-    }
-  } else if (warp == 2) {
-    // ------------------------------------------------------------ lse and delta of the rows of every streamed tile
-    // (asynchronous 4-byte copies: a window's first row need not be 16-byte aligned; rows past its end become zeros)
-    int st = 0, t = 0;
-    uint32_t ph = 1;
-    bool ok = true;
-    for (int it = 0; it < n_items && ok; ++it) {
-      const BwdItem w = bwd_item(it, row_tiles, p.H);
-      const size_t sbase = (static_cast<size_t>(w.win) * p.H + w.head) * N;
-      for (int j = 0; j < nq; ++j, ++t) {
-        if (!mbar_wait(&qd_empty[st], ph, p.status, ERR_TIMEOUT_ATTN)) { ok = false; break; }
-        float* d = s_stat + st * 2 * BT + lane;
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int r = j * BT + u * 32 + lane;
-          const uint32_t bytes = (r < N) ? 4u : 0u;
-          const size_t src = sbase + (r < N ? r : 0);
-          cp_async4(d + u * 32, p.lse + src, bytes);
-          cp_async4(d + BT + u * 32, p.delta + src, bytes);
-        }
-        cp_async_arrive(t < NWG ? &first_full[t] : &next_full[t % NWG]);
-        if (++st == NST) { st = 0; ph ^= 1; }
-      }
-    }
-    for (int e = t + NWG; t < e && ok; ++t) {
-      if (!mbar_wait(&qd_empty[st], ph, p.status, ERR_TIMEOUT_ATTN)) break;
-      if (t >= NWG) mbar_arrive(&next_full[t % NWG]);
-      if (++st == NST) { st = 0; ph ^= 1; }
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-  } else if (warp >= 4) {
-    // ------------------------------------------------------------ math: one thread = one K/V row, every NWG-th tile
-    const int wg = (warp >> 2) - 1, q = warp & 3;
-    const int row = q * 32 + lane;  // kv row within the tile
-    const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
-    const uint32_t tS = tmem_base + lane_addr + wg * 128, tdP = tS + 64;
-    const uint64_t nsl = f2_pack(-p.scale_log2, -p.scale_log2);
-    const float sc = p.scale;
-    uint32_t ph = 0;
-    int j = wg, g = wg;
-    bool ok = true;
-    // Columns past the window's end have zero Q and dO rows and zero statistics (P = 1, dS = 0): they add nothing. Rows
-    // past its end may hold anything: they are not stored.
-    auto pair = [&](uint32_t s0, uint32_t s1, uint32_t d0, uint32_t d1, uint64_t l, uint64_t de, uint32_t& pp,
-                    uint32_t& dd) {
-      float t0, t1;
-      f2_unpack(f2_fma(f2_pack(__uint_as_float(s0), __uint_as_float(s1)), nsl, l), t0, t1);     // -(log2 P)
-      const uint64_t pr = f2_pack(mufu_exp2(-t0), mufu_exp2(-t1));
-      pp = f2_to_bf16x2(pr);
-      dd = f2_to_bf16x2(f2_mul(pr, f2_sub(f2_pack(__uint_as_float(d0), __uint_as_float(d1)), de)));
-    };
-    BwdOut out{sOut + wg * R::OUT_BYTES + q * 4096, lane, q * 32};
-    // see attn_bwd_dq_kernel: the epilogue of an item runs after this warpgroup's first tile of the next
-    auto epilogue = [&](int it) -> bool {
-      if (!mbar_wait(acc_full, it & 1, p.status, ERR_TIMEOUT_ATTN)) return false;
-      tc_fence_after();
-      const BwdItem w = bwd_item(it, row_tiles, p.H);
-      auto release = [&]() {
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(acc_empty);
-      };
-      if (R::STAGED && p.push_n_local == 0) {
-        int mine = 0;                   // this warpgroup's groups of 32 columns of dK and dV
-        for (int c = wg * 32; c < 2 * HD; c += 32 * NWG) mine += (c < HD ? c : c - HD) < p.d;
-        if (mine == 0) release();
-        for (int c = wg * 32; c < 2 * HD; c += 32 * NWG) {
-          const int col = c < HD ? c : c - HD;          // column inside the head
-          if (col < p.d)
-            out.put(tdK + lane_addr + c, c < HD ? sc : 1.f, c < HD ? &tm_dk : &tm_dv, col, w.head, w.tile * TILE, w.win, N,
-                    [&] { if (--mine == 0) release(); });
-        }
-        return true;
-      }
-      const int grow = w.tile * TILE + row;
-      const bool row_ok = grow < N;
-      __nv_bfloat16* dk = bwd_dst(p, w.win, row_ok ? grow : 0, w.head, 1, p.k_col0);
-      __nv_bfloat16* dv = bwd_dst(p, w.win, row_ok ? grow : 0, w.head, 2, p.v_col0);
-#pragma unroll
-      for (int c = 0; c < 2 * HD; c += 32) {
-        const int col = c < HD ? c : c - HD;            // column inside the head
-        if ((c / 32) % NWG != wg || col >= p.d) continue;
-        uint32_t v[32];
-        tmem_ld32(tdK + lane_addr + c, v);
-        tmem_wait_ld();
-        __nv_bfloat16* dst = ((c < HD) ? dk : dv) + col;
-        const float f = (c < HD) ? sc : 1.f;
-        if (row_ok) {
-#pragma unroll
-          for (int gq = 0; gq < 4; ++gq) {
-            uint32_t o[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              o[i] = pack_bf16x2(__uint_as_float(v[8 * gq + 2 * i]) * f, __uint_as_float(v[8 * gq + 2 * i + 1]) * f);
-            if (col + gq * 8 < p.d) *reinterpret_cast<uint4*>(dst + gq * 8) = make_uint4(o[0], o[1], o[2], o[3]);
-          }
-        }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(acc_empty);
-      return true;
-    };
-    for (int it = 0; it < n_items && ok; ++it) {
-      bool pending = it > 0;
-      for (; j < nq; j += NWG, g += NWG, ph ^= 1) {
-        const int st = g % NST;
-        if (!mbar_wait(&sp_full[wg], ph, p.status, ERR_TIMEOUT_ATTN)) { ok = false; break; }
-        tc_fence_after();
-        const ulonglong2* ls = reinterpret_cast<const ulonglong2*>(s_stat + st * 2 * BT);
-        const ulonglong2* ds = ls + BT / 4;
-        if (j < nfull) {
-#pragma unroll
-          for (int c = 0; c < 64; c += 32) {
-            uint32_t sv[32], dv[32], pp[16], dd[16];
-            tmem_ld32(tS + c, sv);
-            tmem_ld32(tdP + c, dv);
-            tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const ulonglong2 l = ls[c / 4 + i], de = ds[c / 4 + i];
-              pair(sv[4 * i], sv[4 * i + 1], dv[4 * i], dv[4 * i + 1], l.x, de.x, pp[2 * i], dd[2 * i]);
-              pair(sv[4 * i + 2], sv[4 * i + 3], dv[4 * i + 2], dv[4 * i + 3], l.y, de.y, pp[2 * i + 1], dd[2 * i + 1]);
-            }
-            tmem_st16(tS + (c >> 1), pp);
-            tmem_st16(tdP + (c >> 1), dd);
-          }
-        } else {
-#pragma unroll 1
-          for (int c = 0; c < n_last; c += 16) {
-            uint32_t sv[16], dv[16], pp[8], dd[8];
-            tmem_ld16(tS + c, sv);
-            tmem_ld16(tdP + c, dv);
-            tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const ulonglong2 l = ls[c / 4 + i], de = ds[c / 4 + i];
-              pair(sv[4 * i], sv[4 * i + 1], dv[4 * i], dv[4 * i + 1], l.x, de.x, pp[2 * i], dd[2 * i]);
-              pair(sv[4 * i + 2], sv[4 * i + 3], dv[4 * i + 2], dv[4 * i + 3], l.y, de.y, pp[2 * i + 1], dd[2 * i + 1]);
-            }
-            tmem_st8(tS + (c >> 1), pp);
-            tmem_st8(tdP + (c >> 1), dd);
-          }
-        }
-        tmem_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&next_full[wg]);
-        if (pending) {
-          pending = false;
-          if (!epilogue(it - 1)) { ok = false; break; }
-        }
-      }
-      if (!ok) break;
-      if (pending && !epilogue(it - 1)) { ok = false; break; }
-      j -= nq;                        // the stream of tiles runs on into the next item
-    }
-    if (ok) epilogue(n_items - 1);
-    if (R::STAGED) out.drain();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  if (warp == 1) tmem_dealloc(tmem_base, 512);
-}
-
-template <int DCH>
-static int launch_attn_bwd(const CUtensorMap& tq128, const CUtensorMap& tk64, const CUtensorMap& tv64,
-                           const CUtensorMap& tdo128, const CUtensorMap& tq64, const CUtensorMap& tk128,
-                           const CUtensorMap& tv128, const CUtensorMap& tdo64, const CUtensorMap (&out)[3],
-                           const AttnBwdParams& p, cudaStream_t stream) {
-  using R = BwdRing<DCH>;
-  auto k1 = attn_bwd_dq_kernel<DCH>;
-  auto k2 = attn_bwd_dkv_kernel<DCH>;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, R::SMEM) != cudaSuccess) return -20;
-    if (cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, R::SMEM) != cudaSuccess) return -20;
-    configured = true;
-  }
-  const long long items = static_cast<long long>((p.N + TILE - 1) / TILE) * p.H * p.n_win;
-  if (items > 0x3fffffff) return -23;
-  const int n = static_cast<int>(items), grid = n < num_sms() ? n : num_sms();
-  k1<<<grid, R::THREADS, R::SMEM, stream>>>(tq128, tk64, tv64, tdo128, out[0], p, n);
-  if (cudaGetLastError() != cudaSuccess) return -21;
-  k2<<<grid, R::THREADS, R::SMEM, stream>>>(tq64, tk128, tv128, tdo64, out[1], out[2], p, n);
-  return cudaGetLastError() == cudaSuccess ? 0 : -22;
-}
-
-}  // namespace aeris
+#include "attention_bwd.cuh"
 
 using namespace aeris;
 
@@ -1586,17 +696,18 @@ static int attn_bwd_impl(const void* qkv, int ldq, int q_col0, int k_col0, int v
   p.N = N; p.H = H; p.n_win = n_win; p.d = head_dim; p.q_col0 = q_col0; p.k_col0 = k_col0; p.v_col0 = v_col0;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
   CUtensorMap q128, q64, k128, k64, v128, v64, d128, d64;
+  const uint32_t bt = head_dim <= 64 ? BwdCfg<1, false>::BT : BwdCfg<2, false>::BT;
   int r;
   const __nv_bfloat16* b = reinterpret_cast<const __nv_bfloat16*>(qkv);
   const struct { CUtensorMap* m; const void* base; int ld; uint32_t rows; } maps[] = {
-      {&q128, b + q_col0, ldq, TILE}, {&q64, b + q_col0, ldq, BT},
-      {&k128, b + k_col0, ldq, TILE}, {&k64, b + k_col0, ldq, BT},
-      {&v128, b + v_col0, ldq, TILE}, {&v64, b + v_col0, ldq, BT},
-      {&d128, d_o, ldo, TILE},        {&d64, d_o, ldo, BT}};
+      {&q128, b + q_col0, ldq, TILE}, {&q64, b + q_col0, ldq, bt},
+      {&k128, b + k_col0, ldq, TILE}, {&k64, b + k_col0, ldq, bt},
+      {&v128, b + v_col0, ldq, TILE}, {&v64, b + v_col0, ldq, bt},
+      {&d128, d_o, ldo, TILE},        {&d64, d_o, ldo, bt}};
   for (const auto& m : maps)
     if ((r = make_tmap_heads_bf16(m.m, m.base, head_dim, H, N, n_win, m.ld, m.rows))) return r;
-  CUtensorMap out[3] = {q128, q128, q128};      // pushed gradients and those of narrow heads do not leave through them
-  if (head_dim > 64 && !dq_peers) {
+  CUtensorMap out[3] = {q128, q128, q128};      // pushed gradients do not leave through them
+  if (!dq_peers) {
     const __nv_bfloat16* g = p.dQKV;
     const int cols[3] = {q_col0, k_col0, v_col0};
     for (int i = 0; i < 3; ++i)

@@ -98,6 +98,55 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
   if (mbar_try_wait(bar, parity)) return true;
   return mbar_wait_slow(bar, parity, status, code);
 }
+// Waits of a warp that stays together: every lane asks, the votes keep it one, and the loop is in line. Against mbar_wait, whose
+// second try is behind a call, a hand-over that has to be waited for takes 103 instead of 287 cycles (two warps handing one
+// back and forth), and a kernel without calls can split its registers between warpgroups. A try that fails suspends the
+// warp for 1.3 us (measured), so the limit is about as long as the other waits' 2 s.
+constexpr int MBAR_TRIES = 1500000;
+__device__ __forceinline__ bool mbar_try_wait_at(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t"
+      "}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int* status, int code) {
+#pragma unroll 1
+  for (int i = 0; i < MBAR_TRIES; ++i)
+    if (__all_sync(0xffffffffu, mbar_try_wait_at(bar, parity))) return true;
+  if (status) atomicCAS(status, 0, code);
+  return false;
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* status, int code) {
+  return mbar_wait_warp(smem_u32(bar), parity, status, code);
+}
+// Two barriers, both tries under way at once: a wait that is over costs 110-200 cycles of latency.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, int* status, int code) {
+#pragma unroll 1
+  for (int i = 0; i < MBAR_TRIES; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
+        "and.pred p, p, q;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(ok)
+        : "r"(b0), "r"(p0), "r"(b1), "r"(p1)
+        : "memory");
+    if (__all_sync(0xffffffffu, ok != 0)) return true;
+  }
+  if (status) atomicCAS(status, 0, code);
+  return false;
+}
 // Non-suspending poll (mbarrier.test_wait) with the same time limit: the waiting thread never yields its issue slot,
 // which suits single elected threads that wait on barriers signalled from another CTA of the cluster.
 __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
@@ -209,6 +258,50 @@ __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64
       : "memory");
 }
 
+// Products and commits of a warp that stays together: the lane with `lead` set issues them, and what they are made of can live
+// in uniform registers. A loop of two waits, eight products and two commits: 251 cycles, by a single thread 304.
+__device__ __forceinline__ void umma_ss_warp(uint32_t lead, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+                                             uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, e;\n\t"
+      "setp.ne.b32 e, %5, 0;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "}\n" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void umma_ts_warp(uint32_t lead, uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc,
+                                             uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, e;\n\t"
+      "setp.ne.b32 e, %5, 0;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void tc_commit_warp(uint32_t lead, uint32_t bar) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred e;\n\t"
+      "setp.ne.b32 e, %1, 0;\n\t"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+      "}\n" ::"r"(bar),
+      "r"(lead)
+      : "memory");
+}
+// Registers per thread of the warpgroup that executes this; a kernel's shares may add up to what it was launched with.
+template <int N> __device__ __forceinline__ void regs_dec() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
+template <int N> __device__ __forceinline__ void regs_inc() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
+
 // 32 lanes x 32 columns of fp32: thread i of the warp gets row (lane base + i), 32 consecutive columns.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
@@ -277,6 +370,16 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t 
   d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFF) << 32;
   d |= static_cast<uint64_t>(1) << 46;  // descriptor version for sm_100
   d |= static_cast<uint64_t>(2) << 61;  // SWIZZLE_128B
+  return d;
+}
+// The same in two halves. The low word (address, leading offset) advances by bytes / 16; the high one is that of every
+// 128-byte swizzled tile whose groups of eight rows are 1024 bytes apart.
+__device__ __forceinline__ uint32_t smem_desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) {
+  return ((smem_addr & 0x3FFFF) >> 4) | ((lbo_bytes >> 4) << 16);
+}
+__device__ __forceinline__ uint64_t smem_desc(uint32_t lo) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"((1024u >> 4) | (1u << 14) | (2u << 29)));
   return d;
 }
 // Instruction descriptor for kind::f16 with bf16 inputs and fp32 accumulation.
