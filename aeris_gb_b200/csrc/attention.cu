@@ -97,6 +97,15 @@ __device__ __forceinline__ float softmax_row64(const uint32_t (&v0)[32], const u
   return s0 + s1;
 }
 
+// A slot that comes round after `n` uses, and the parity of the round it is in.
+struct Slot {
+  int i = 0;
+  uint32_t ph = 0;
+  __device__ __forceinline__ void next(int n) {
+    if (++i == n) { i = 0; ph ^= 1; }
+  }
+};
+
 // -------------------------------------------------------------------------------------------------------- forward
 // grid = (q_tiles, H, n_win). One CTA owns a 128-row Q tile and streams the window's K/V in 64-row tiles through a
 // two-stage TMA ring. Per tile: S = Q K^T lands in TMEM, the four softmax warps (one thread per query row) read its 64
@@ -533,6 +542,7 @@ static int launch_attn_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const C
 }  // namespace aeris
 
 #include "attention_fwd_pair.cuh"
+#include "attention_fwd_quad.cuh"
 #include "attention_bwd.cuh"
 
 using namespace aeris;
@@ -612,7 +622,7 @@ static int attn_fwd_impl(const void* q, int ldq, int q_col0, const void* k, int 
   if ((r = make_tmap_heads_bf16(&tq, at(q, q_col0), head_dim, H, N, n_win, ldq, TILE))) return r;
   // Two query tiles at a time where there are two; its masked columns need a positive scale. ms, windows x tokens, one tile
   // at a time / two in turn, 24 heads x 64 and 12 x 128:
-  // - Three or five tiles of which the last is not full leave the second chain idle for a third or a fifth of the time.
+  // - Three tiles (of few windows) or five of which the last is not full leave the second chain idle for part of the time.
   //   64-wide heads are faster without then (249 x 260 tokens 0.387 / 0.416, 202 x 320 0.348 / 0.352, 221 x 513 0.857 /
   //   0.925, 175 x 576 0.732 / 0.772; full ones 168 x 384 0.363 / 0.337, 142 x 640 0.689 / 0.664; seven tiles 84 x 832 0.692
   //   / 0.667, 97 x 772 0.758 / 0.754), 128-wide ones are not (249 x 260 0.325 / 0.295, 175 x 576 0.621 / 0.550).
@@ -620,9 +630,28 @@ static int attn_fwd_impl(const void* q, int ldq, int q_col0, const void* k, int 
   //   0.393, 740 0.726 / 0.689, 970 0.661 / 0.680, 1250 0.635 / 0.624, 1500 0.588 / 0.605, 3600 0.498 / 0.538. 128: 740
   //   0.577 / 0.458, 1250 0.481 / 0.423, 1500 0.441 / 0.421, 2000 0.417 / 0.423, 3600 0.360 / 0.372.
   const int q_tiles = (N + TILE - 1) / TILE;
+  // Four query tiles at a time (heads up to 64) where a window has three, or fills all groups of four but for one tile, and
+  // where rounds of whole items do not cost more than they save: a group of four takes 1.74 times as long as a pair (72 x
+  // 900, 12 x 64: 12 rounds in 0.280 ms, 24 in 0.323). ms, windows x tokens, 12 x 64, before / now: 252 x 257 0.196 / 0.156,
+  // 202 x 320 0.171 / 0.134, 168 x 384 0.163 / 0.133, 126 x 512 0.165 / 0.155, 77 x 832 0.288 / 0.258, 72 x 900 0.320 /
+  // 0.277, 64 x 1000 0.348 / 0.286, 63 x 1024 0.294 / 0.282, 43 x 1500 0.479 / 0.410. By rounds, where it was taken for all
+  // counts: 3 x 900 (one round each) 0.0190 / 0.0301, 6 x 900 0.0329 / 0.0309, 8 x 900 0.0458 / 0.0532, 12 x 900 0.0596 /
+  // 0.0540. Groups left half empty: 101 x 640 0.230 / 0.242, 58 x 1100 0.377 / 0.410, 253 x 256 0.102 / 0.122.
+  const long long wh = static_cast<long long>(H) * n_win;
+  const int groups = (q_tiles + 3) / 4, pairs = (q_tiles + 1) / 2;
+  auto rounds = [](long long items) { return (items + num_sms() - 1) / num_sms(); };
+  const bool plain = scale > 0.f && g_fwd_mode == 0 && g_fwd_poly == -1;
+  if (head_dim <= 64 && plain && q_tiles >= 3 && 4 * groups - q_tiles <= 1 &&
+      7 * rounds(groups * wh) <= 4 * rounds(pairs * wh)) {
+    if ((r = make_tmap_heads_bf16(&tk, at(k, k_col0), head_dim, H, N, n_win, ldk, KVT))) return r;
+    if ((r = make_tmap_heads_bf16(&tv, at(v, v_col0), head_dim, H, N, n_win, ldv, KVT))) return r;
+    CUtensorMap to = tq;      // without a local output nothing is stored through it
+    if (o && (r = make_tmap_heads32_bf16(&to, o, head_dim, H, N, n_win, ldo, 32))) return r;
+    return launch_attn_fwd_quad(tq, tk, tv, to, p, stream);
+  }
   const bool idle_chain = head_dim <= 64 && (q_tiles == 3 || q_tiles == 5) && N % TILE != 0;
   const bool cut = N % KVT > 4, long_cut = cut && q_tiles > (head_dim > 64 ? 12 : 6);
-  if (q_tiles > 1 && !idle_chain && !long_cut && scale > 0.f && g_fwd_mode == 0 && g_fwd_poly == -1) {
+  if (q_tiles > 1 && !idle_chain && !long_cut && plain) {
     if ((r = make_tmap_heads_bf16(&tk, at(k, k_col0), head_dim, H, N, n_win, ldk, KVP))) return r;
     if ((r = make_tmap_heads_bf16(&tv, at(v, v_col0), head_dim, H, N, n_win, ldv, KVP))) return r;
     CUtensorMap to = tq;      // without a local output nothing is stored through it

@@ -155,14 +155,6 @@ struct BwdOut {
   }
 };
 
-// A slot that comes round after `n` uses, and the parity of the round it is in.
-struct Slot {
-  int i = 0;
-  uint32_t ph = 0;
-  __device__ __forceinline__ void next(int n) {
-    if (++i == n) { i = 0; ph ^= 1; }
-  }
-};
 struct BwdItem {
   int tile, head, win;
 };

@@ -98,10 +98,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
   if (mbar_try_wait(bar, parity)) return true;
   return mbar_wait_slow(bar, parity, status, code);
 }
-// Waits of a warp that stays together: every lane asks, the votes keep it one, and the loop is in line. Against mbar_wait, whose
-// second try is behind a call, a hand-over that has to be waited for takes 103 instead of 287 cycles (two warps handing one
-// back and forth), and a kernel without calls can split its registers between warpgroups. A try that fails suspends the
-// warp for 1.3 us (measured), so the limit is about as long as the other waits' 2 s.
+// Waits of a warp that stays together: every lane asks, the votes keep it one, and the loop is in line. Against mbar_wait,
+// whose second try is behind a call, a hand-over that has to be waited for takes 103 instead of 287 cycles (two warps that
+// hand one back and forth), and a kernel without calls can split its registers between warpgroups. A try that fails suspends
+// the warp for 1.3 us (measured), so the limit is about as long as the other waits' 2 s.
 constexpr int MBAR_TRIES = 1500000;
 __device__ __forceinline__ bool mbar_try_wait_at(uint32_t bar, uint32_t parity) {
   uint32_t ok;
@@ -258,8 +258,8 @@ __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64
       : "memory");
 }
 
-// Products and commits of a warp that stays together: the lane with `lead` set issues them, and what they are made of can live
-// in uniform registers. A loop of two waits, eight products and two commits: 251 cycles, by a single thread 304.
+// Products and commits of a warp that stays together: the lane with `lead` set issues them, and what they are made of can
+// live in uniform registers. A loop of two waits, eight products and two commits: 251 cycles, by a single thread 304.
 __device__ __forceinline__ void umma_ss_warp(uint32_t lead, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
                                              uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -282,6 +282,70 @@ __device__ __forceinline__ void umma_ts_warp(uint32_t lead, uint32_t tmem_d, uin
       "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
       "}\n" ::"r"(tmem_d),
       "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead)
+      : "memory");
+}
+// Four steps of 16 at a time: the operands' low words advance by A_STEP and B_STEP (tensor memory: words), `acc` is the
+// first step's. Fewer instructions than four calls.
+template <int A_STEP, int B_STEP>
+__device__ __forceinline__ void umma_ss4_warp(uint32_t lead, uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
+                                              uint32_t acc) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, e;\n\t"
+      ".reg .b32 a, b;\n\t"
+      ".reg .b64 x, y;\n\t"
+      "setp.ne.b32 e, %5, 0;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "mov.b64 x, {%1, %6};\n\t"
+      "mov.b64 y, {%2, %6};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %3, p;\n\t"
+      "add.u32 a, %1, %7;\n\t"
+      "add.u32 b, %2, %8;\n\t"
+      "mov.b64 x, {a, %6};\n\t"
+      "mov.b64 y, {b, %6};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %3, 1;\n\t"
+      "add.u32 a, a, %7;\n\t"
+      "add.u32 b, b, %8;\n\t"
+      "mov.b64 x, {a, %6};\n\t"
+      "mov.b64 y, {b, %6};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %3, 1;\n\t"
+      "add.u32 a, a, %7;\n\t"
+      "add.u32 b, b, %8;\n\t"
+      "mov.b64 x, {a, %6};\n\t"
+      "mov.b64 y, {b, %6};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %3, 1;\n\t"
+      "}\n" ::"r"(tmem_d),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(acc), "r"(lead), "r"((1024u >> 4) | (1u << 14) | (2u << 29)), "n"(A_STEP),
+      "n"(B_STEP)
+      : "memory");
+}
+template <int A_STEP, int B_STEP>
+__device__ __forceinline__ void umma_ts4_warp(uint32_t lead, uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc,
+                                              uint32_t acc) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, e;\n\t"
+      ".reg .b32 a, b;\n\t"
+      ".reg .b64 y;\n\t"
+      "setp.ne.b32 e, %5, 0;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "mov.b64 y, {%2, %6};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], y, %3, p;\n\t"
+      "add.u32 a, %1, %7;\n\t"
+      "add.u32 b, %2, %8;\n\t"
+      "mov.b64 y, {b, %6};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a], y, %3, 1;\n\t"
+      "add.u32 a, a, %7;\n\t"
+      "add.u32 b, b, %8;\n\t"
+      "mov.b64 y, {b, %6};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a], y, %3, 1;\n\t"
+      "add.u32 a, a, %7;\n\t"
+      "add.u32 b, b, %8;\n\t"
+      "mov.b64 y, {b, %6};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a], y, %3, 1;\n\t"
+      "}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "r"(b_lo), "r"(idesc), "r"(acc), "r"(lead), "r"((1024u >> 4) | (1u << 14) | (2u << 29)), "n"(A_STEP),
+      "n"(B_STEP)
       : "memory");
 }
 __device__ __forceinline__ void tc_commit_warp(uint32_t lead, uint32_t bar) {
