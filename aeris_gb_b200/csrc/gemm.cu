@@ -221,8 +221,8 @@ static PFN_encodeTiled get_encode() {
 }
 
 // 2-D bf16 tensor map: `inner` contiguous elements per row, `rows` rows, row pitch `ld` elements.
-int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t rows, uint64_t ld,
-                      uint32_t box_inner, uint32_t box_rows) {
+static int make_tmap_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t rows, uint64_t ld, uint32_t box_inner,
+                        uint32_t box_rows, CUtensorMapSwizzle swizzle) {
   PFN_encodeTiled enc = get_encode();
   if (!enc) return -10;
   if ((reinterpret_cast<uintptr_t>(base) & 15) || ((ld * 2) & 15)) return -11;
@@ -231,9 +231,18 @@ int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64
   cuuint32_t box[2] = {box_inner, box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -12;
+}
+
+int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t rows, uint64_t ld,
+                      uint32_t box_inner, uint32_t box_rows) {
+  return make_tmap_2d(out, base, inner, rows, ld, box_inner, box_rows, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+int make_tmap_2d_sw64_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t rows, uint64_t ld,
+                           uint32_t box_inner, uint32_t box_rows) {
+  return make_tmap_2d(out, base, inner, rows, ld, box_inner, box_rows, CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 static int make_tmap_heads(CUtensorMap* out, const void* base, int d, int heads, int tokens, int windows, uint64_t ld,

@@ -33,7 +33,7 @@ constexpr int G2_STAGE_BYTES = G2_A_BYTES + G2_B_BYTES;
 // stage (their staging buffers; see aeris_gemm_bf16_2cta for the line). Everything else keeps four warps and six stages.
 template <int EW> struct G2Layout {
   static constexpr int STAGES = EW == 8 ? G2_STAGES - 1 : G2_STAGES;
-  static constexpr int PUSH_OFF = STAGES * G2_STAGE_BYTES + 512;     // staging of the epilogues, 8 KB per warp
+  static constexpr int PUSH_OFF = STAGES * G2_STAGE_BYTES + 1024;     // staging of the epilogues, 8 KB per warp
   static constexpr int SMEM = PUSH_OFF + EW * PUSH_STAGE_BYTES + 1024;
   static constexpr int THREADS = 64 + EW * 32;
 };
@@ -104,7 +104,7 @@ __device__ __forceinline__ void umma2_ss(uint32_t tmem_d, uint64_t adesc, uint64
 template <int A_MN, int B_MN, int EW, bool AG = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G2Layout<EW>::THREADS + (AG ? AG_COPY_THREADS : 0), 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-             const GemmParams p) {
+             const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_x, const GemmParams p) {
   static_assert(!AG || EW == 4, "the copier warps follow four epilogue warps");
   using LY = G2Layout<EW>;
   extern __shared__ uint8_t smem_raw[];
@@ -117,15 +117,16 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
 
   // AG: the last operand stage is the copier's ring (two 16 KB bulk-copy buffers), with its barriers behind tmem_slot
   // (the reduce-scatter epilogue gives up the same stage: its fourth warp stages its rows there)
-  // and so do the epilogues on eight warps that request a second operand ahead. The gated residual gains from that while
-  // its tile's products are short (us without / with, in turn: 28800 x 512 x 512 36.8 / 31.0, x 768 x 768 57.0 / 48.3, x
+  // and so does the gated residual on eight warps where it requests its second operand ahead, which it gains from while its
+  // tile's products are short (us without / with, in turn: 28800 x 512 x 512 36.8 / 31.0, x 768 x 768 57.0 / 48.3, x
   // 1024 x 1024 86.0 / 73.2, 64800 x 512 x 512 71.5 / 61.1; a few per cent at 28800 x 768 x 1536 79.8 / 76.2 and 64800 x
   // 1536 x 1536 321 / 308; 28800 x 768 x 2048 94.3 / 97.7: the ring's fifth stage is worth more).
   const bool ahead = EW == 8 && p.staged_out;
   const bool u_ahead = ahead && p.epi == EPI_SWIGLU_BWD, r_ahead = ahead && p.epi == EPI_GATE_RESID && !p.aux && p.K <= 1024;
-  const int STAGES = (u_ahead || r_ahead || (EW == 4 && (AG || p.epi == EPI_RS_PUSH))) ? LY::STAGES - 1 : LY::STAGES;
+  const int STAGES = (r_ahead || (EW == 4 && (AG || p.epi == EPI_RS_PUSH))) ? LY::STAGES - 1 : LY::STAGES;
   [[maybe_unused]] uint8_t* ag_ring = smem + (LY::STAGES - 1) * G2_STAGE_BYTES;
   [[maybe_unused]] uint64_t* ag_bars = reinterpret_cast<uint64_t*>(smem + LY::STAGES * G2_STAGE_BYTES + 256);
+  uint64_t* u_bars = reinterpret_cast<uint64_t*>(smem + LY::STAGES * G2_STAGE_BYTES + 320);     // [EW][2]
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -164,6 +165,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
+    for (int i = 0; i < 2 * EW; ++i) mbar_init(&u_bars[i], 1);
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull_bar[a], 1);
       mbar_init(&tempty_bar[a], 2 * EW);
@@ -279,6 +281,21 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     bool ok = true;
     const uint32_t leader_tempty0 = map_to_cta(smem_u32(&tempty_bar[0]), 0);
     [[maybe_unused]] uint8_t* ubuf = smem + (LY::STAGES - 1) * G2_STAGE_BYTES + (warp - 2) * SWIGLU_U_BYTES;
+    // two buffers per warp in turn: gate and up columns of a step come in, their gradients leave from the same place
+    [[maybe_unused]] uint64_t* u_bar = &u_bars[2 * (warp - 2)];
+    [[maybe_unused]] uint8_t* ustage = smem + LY::PUSH_OFF + (part * 4 + q) * PUSH_STAGE_BYTES;
+    [[maybe_unused]] int u_n = 0, u_m = 0;         // steps requested, taken
+    [[maybe_unused]] auto u_request = [&](int row0, int col) {
+      if (lane == 0) {
+        uint8_t* dst = ustage + (u_n & 1) * SWIGLU_U_BYTES;
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // the gradients before have left it
+        mbar_expect_tx(u_bar + (u_n & 1), SWIGLU_U_BYTES);
+        tma_load_2d(dst, &tmap_x, u_bar + (u_n & 1), col, row0);
+        tma_load_2d(dst + SWIGLU_U_BYTES / 2, &tmap_x, u_bar + (u_n & 1), p.swiglu_f + col, row0);
+      }
+      ++u_n;
+      __syncwarp();
+    };
     // first step of the next tile from `tile` on that has columns for this warp (the last tile of a row may be half empty)
     [[maybe_unused]] auto request_tile = [&](int tile) {
       for (; tile < total_tiles; tile += n_clusters) {
@@ -287,7 +304,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         const int c = part * (G2_BN / 2);
         if (tn * G2_BN + c >= p.N) continue;
         if (u_ahead)
-          swiglu_u_request(ubuf, p, tm * 2 * G2_BM + crank * G2_BM + q * 32, tn * G2_BN + c, lane);
+          u_request(tm * 2 * G2_BM + crank * G2_BM + q * 32, tn * G2_BN + c);
         else
           resid_request(ubuf, p, tm * 2 * G2_BM + crank * G2_BM + q * 32, tn * G2_BN + c, lane);
         break;
@@ -312,15 +329,24 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       bool done = false;
       if constexpr (EW == 8) {
         if (u_ahead) {
-          const bool row_ok = row < p.M;
-          __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(row) * p.ldc + tn * G2_BN;
           const int c_hi = min((part + 1) * (G2_BN / 2), p.N - tn * G2_BN);
+          const int row0 = row - lane;
 #pragma unroll 1
           for (int c = part * (G2_BN / 2); c < c_hi; c += 32) {
             uint4 g4[4], u4[4];
-            swiglu_u_take(ubuf, lane, g4, u4);
+            ok = mbar_wait_warp(u_bar + (u_m & 1), (u_m >> 1) & 1, p.status, ERR_TIMEOUT_FULL);
+            if (!ok) break;
+            uint8_t* buf = ustage + (u_m & 1) * SWIGLU_U_BYTES;
+            uint8_t* mine = buf + lane * 64;
+            ++u_m;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint8_t* src = mine + ((i ^ ((lane >> 1) & 3)) << 4);
+              g4[i] = *reinterpret_cast<const uint4*>(src);
+              u4[i] = *reinterpret_cast<const uint4*>(src + SWIGLU_U_BYTES / 2);
+            }
             if (c + 32 < c_hi)
-              swiglu_u_request(ubuf, p, row - lane, tn * G2_BN + c + 32, lane);
+              u_request(row0, tn * G2_BN + c + 32);
             else
               request_tile(tile + n_clusters);
             uint32_t v[32], og[16], ou[16];
@@ -331,20 +357,30 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
               const uint32_t gw[4] = {g4[i].x, g4[i].y, g4[i].z, g4[i].w}, uw[4] = {u4[i].x, u4[i].y, u4[i].z, u4[i].w};
 #pragma unroll
               for (int j = 0; j < 4; ++j)
-                swiglu_bwd_pair(__uint_as_float(v[8 * i + 2 * j]), __uint_as_float(v[8 * i + 2 * j + 1]), gw[j], uw[j],
-                                og[4 * i + j], ou[4 * i + j]);
+                swiglu_bwd_pair(v[8 * i + 2 * j], v[8 * i + 2 * j + 1], gw[j], uw[j], og[4 * i + j], ou[4 * i + j]);
             }
-            // 64 d(gate) columns and the matching 64 d(up) columns share one stage group
-            push_stage_put(stg, lane, (c & 32), og);
-            push_stage_put(stg, lane, 64 + (c & 32), ou);
-            if (c & 32)
-              push_stage_flush2(stg, lane, row_ok ? dst + (c - 32) : nullptr,
-                                row_ok ? dst + p.swiglu_f + (c - 32) : nullptr);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              uint8_t* dst = mine + ((i ^ ((lane >> 1) & 3)) << 4);
+              *reinterpret_cast<uint4*>(dst) = make_uint4(og[4 * i], og[4 * i + 1], og[4 * i + 2], og[4 * i + 3]);
+              *reinterpret_cast<uint4*>(dst + SWIGLU_U_BYTES / 2) =
+                  make_uint4(ou[4 * i], ou[4 * i + 1], ou[4 * i + 2], ou[4 * i + 3]);
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              if (row0 < p.M) {
+                tma_store_2d(&tmap_c, buf, tn * G2_BN + c, row0);
+                tma_store_2d(&tmap_c, buf + SWIGLU_U_BYTES / 2, p.swiglu_f + tn * G2_BN + c, row0);
+              }
+              asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            }
+            __syncwarp();
           }
+          if (!ok) break;
           done = true;
         } else if (r_ahead) {
-          const bool row_ok = row < p.M;
-          __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(row) * p.ldc + tn * G2_BN;
+          const TileOut to{stg, lane};
           const float* gate = p.gate + static_cast<size_t>(min(row, p.M - 1) / p.rows_per_gate) * p.ld_gate + tn * G2_BN;
           const int c_hi = min((part + 1) * (G2_BN / 2), p.N - tn * G2_BN);
 #pragma unroll 1
@@ -373,14 +409,16 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
                                              fmaf(gg[2 * j + 1], __uint_as_float(v[8 * i + 2 * j + 1]), r2.y));
                 }
               }
-              push_stage_put(stg, lane, (c & 64) + 32 * h, o);
+              if (h == 0) to.wait_one();
+              to.put((c >> 6) & 1, h, o);
+              if (h == 1) to.send((c >> 6) & 1, &tmap_c, tn * G2_BN + c, row - lane, p.M);
             }
-            if (c & 64) push_stage_flush(stg, lane, row_ok ? dst + (c - 64) : nullptr);
           }
           done = true;
         }
       }
-      if (!done) gemm_epilogue_row<G2_BN>(p, taddr, row, row < p.M, tn, kempty, stg, part, EW / 4);
+      if (!done) gemm_epilogue_row<G2_BN>(p, taddr, row, row < p.M, tn, kempty, stg, part, EW / 4,
+                                          p.staged_out ? &tmap_c : nullptr, &tmap_x);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(leader_tempty0 + acc * 8);
@@ -389,6 +427,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     // the bulk copies of the reduce-scatter push have been performed before this thread leaves (the owners read
     // their slots after a rank barrier that follows this kernel in the stream)
     if (p.epi == EPI_RS_PUSH) rs_stage_drain();
+    if (p.staged_out) TileOut{nullptr, lane}.drain();
     if constexpr (EW == 8) asm volatile("cp.async.wait_all;" ::: "memory");     // after a time-out: copies nobody took
   }
 
@@ -400,7 +439,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
 }
 
 template <int A_MN, int B_MN, int EW, bool AG = false>
-static int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p_in, cudaStream_t stream) {
+static int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p_in, cudaStream_t stream,
+                        const CUtensorMap* tc = nullptr, const CUtensorMap* tx = nullptr) {
   static bool configured = false;
   GemmParams p = p_in;
   constexpr int THREADS = G2Layout<EW>::THREADS + (AG ? AG_COPY_THREADS : 0), SMEM = G2Layout<EW>::SMEM;
@@ -432,7 +472,7 @@ static int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
   const int tiles = mn_tiles * p.k_splits;
   if (tiles < clusters && !AG) clusters = tiles;
   if (AG) p.ag_expect *= static_cast<unsigned>(2 * clusters);   // came in as the call index
-  kern<<<2 * clusters, THREADS, SMEM, stream>>>(ta, tb, p);
+  kern<<<2 * clusters, THREADS, SMEM, stream>>>(ta, tb, tc ? *tc : ta, tx ? *tx : ta, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
@@ -459,10 +499,6 @@ static int gemm_two_cta(const void* A, const void* B, void* C, int M, int N, int
   p.aux = reinterpret_cast<__nv_bfloat16*>(aux); p.ld_aux = ld_aux;
   p.k_splits = k_splits; p.status = status; p.swiglu_f = swiglu_f; p.group_m = 8;
   {
-    // bf16-output epilogues write through the shared-memory stage as 256-byte row segments (measured 1-13 % faster
-    // than one 16-byte piece per row and instruction); AERIS_GEMM_STAGED_OUT=0 selects the direct stores
-    static const int staged = [] { const char* e = getenv("AERIS_GEMM_STAGED_OUT"); return e ? atoi(e) : 1; }();
-    p.staged_out = staged;
     static const int staged_red = [] { const char* e = getenv("AERIS_GEMM_STAGED_RED"); return e ? atoi(e) : 0; }();
     p.staged_red = staged_red;
   }
@@ -480,6 +516,24 @@ static int gemm_two_cta(const void* A, const void* B, void* C, int M, int N, int
     r = make_tmap_2d_bf16(&tb, B, N, K, ldb, 64, G2_BK);
   }
   if (r) return r - 100;
+  // bf16 outputs leave as tiles of 32 rows (TileOut; on eight warps the SwiGLU backward has narrower ones, see
+  // SWIGLU_U_BYTES). AERIS_GEMM_STAGED_OUT=0 selects direct stores, one 16-byte piece per row and instruction.
+  const bool heavy = epi == EPI_SWIGLU_BOTH || epi == EPI_SWIGLU_BWD || epi == EPI_GATE_RESID;
+  const bool ew8 = (heavy && K <= (epi == EPI_SWIGLU_BWD ? 2560 : 2048)) || (epi == EPI_STORE && K <= 1024);
+  CUtensorMap tc = ta, tx = ta;
+  static const int staged = [] { const char* e = getenv("AERIS_GEMM_STAGED_OUT"); return e ? atoi(e) : 1; }();
+  p.staged_out = staged && !a_mn && (heavy || epi == EPI_STORE || epi == EPI_SWIGLU) && !(epi == EPI_GATE_RESID && aux);
+  if (p.staged_out) {
+    const uint64_t two_f = 2 * static_cast<uint64_t>(swiglu_f);
+    if (epi == EPI_SWIGLU_BWD && ew8) {
+      if ((r = make_tmap_2d_sw64_bf16(&tc, C, two_f, M, ldc, 32, 32))) return r - 200;
+      if ((r = make_tmap_2d_sw64_bf16(&tx, resid, two_f, M, ldr, 32, 32))) return r - 300;
+    } else {
+      const uint64_t cols = epi == EPI_SWIGLU_BWD ? two_f : swiglu_fwd ? swiglu_f : N;
+      if ((r = make_tmap_2d_bf16(&tc, C, cols, M, ldc, 64, 32))) return r - 200;
+      if (epi == EPI_SWIGLU_BOTH && (r = make_tmap_2d_bf16(&tx, aux, two_f, M, ld_aux, 64, 32))) return r - 300;
+    }
+  }
   // Eight epilogue warps where the epilogue takes longer than the products of a tile. Four warps and six stages against
   // eight and five, us, held for 0.6 s (1.2-1.8 GHz under the power cap): gated residual 28800 x 768 x 768 62 / 53, 64800 x
   // 1536 x 1536 311 / 284, 28800 x 2048 x 2048 217 / 210, x 2304 x 2304 255 / 256, x 3072 x 3072 424 / 436; SwiGLU backward
@@ -488,14 +542,13 @@ static int gemm_two_cta(const void* A, const void* B, void* C, int M, int N, int
   // 2304 1270 / 1309. The raw columns lose below the line at 2048.
   // Plain store 28800 x 2304 x 768 104 / 98, x 3072 x 1024 158 / 157, x 3840 x 1280 222 / 232. Weight gradients (a_mn) lose
   // a few per cent. Since then the SwiGLU backward and the gated residual on eight warps request their second operand ahead
-  // (registers for that spilled; see swiglu_u_request), and the SwiGLU backward's line moved up. In turn, 1.2-1.5 GHz:
+  // (registers for that spilled; see SWIGLU_U_BYTES), and the SwiGLU backward's line moved up. In turn, 1.2-1.5 GHz:
   // 28800 x 5376 x 2048 712 / 684, x 6144 x 2304 1017 / 810, x 6400 x 2432 1094 / 897, x 6912 x 2560 1167 / 1031; it would
   // gain further up (x 7680 x 2816 1376 / 1255), but no more at x 8192 x 3072 1469 / 1478.
-  const bool heavy = epi == EPI_SWIGLU_BOTH || epi == EPI_SWIGLU_BWD || epi == EPI_GATE_RESID;
-  const bool ew8 = (heavy && K <= (epi == EPI_SWIGLU_BWD ? 2560 : 2048)) || (epi == EPI_STORE && K <= 1024);
   if (a_mn) return b_mn ? launch_gemm2<1, 1, 4>(ta, tb, p, stream) : launch_gemm2<1, 0, 4>(ta, tb, p, stream);
-  if (b_mn) return ew8 ? launch_gemm2<0, 1, 8>(ta, tb, p, stream) : launch_gemm2<0, 1, 4>(ta, tb, p, stream);
-  return ew8 ? launch_gemm2<0, 0, 8>(ta, tb, p, stream) : launch_gemm2<0, 0, 4>(ta, tb, p, stream);
+  if (b_mn)
+    return ew8 ? launch_gemm2<0, 1, 8>(ta, tb, p, stream, &tc, &tx) : launch_gemm2<0, 1, 4>(ta, tb, p, stream, &tc, &tx);
+  return ew8 ? launch_gemm2<0, 0, 8>(ta, tb, p, stream, &tc, &tx) : launch_gemm2<0, 0, 4>(ta, tb, p, stream, &tc, &tx);
 }
 
 extern "C" int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb,

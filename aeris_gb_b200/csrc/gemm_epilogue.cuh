@@ -51,7 +51,7 @@ struct GemmParams {
   // rows (lo at row `split_rows`) of `split_k` columns: K = 3 split_k (0: plain operand).
   int split_k, split_rows;
   int group_m;      // two-CTA kernel: m-tiles per group of the tile order (<= 1: n fastest)
-  int staged_out;   // bf16-output epilogues: move rows through the warp's shared-memory stage (coalesced global stores)
+  int staged_out;   // two-CTA kernel, bf16 outputs: rows leave through shared memory as tiled stores (TileOut)
   int staged_red;   // split-K fp32 accumulation: stage 32 rows x 64 columns and issue the reductions row-contiguously
   int ld_gate;
   int* status;
@@ -80,23 +80,6 @@ __device__ __forceinline__ void push_stage_flush(uint8_t* stage, int lane, __nv_
     const unsigned long long d = __shfl_sync(0xffffffffu, mine, r);
     const uint4 v = *reinterpret_cast<const uint4*>(stage + r * 256 + ((ch ^ (r & 15)) << 4));
     if (d) *reinterpret_cast<uint4*>(d + ch * 16) = v;
-  }
-  __syncwarp();
-}
-
-// Same, but the staged 128 columns are two 64-column halves with different destinations (two 128-byte segments per row).
-__device__ __forceinline__ void push_stage_flush2(uint8_t* stage, int lane, __nv_bfloat16* dst_a, __nv_bfloat16* dst_b) {
-  __syncwarp();
-  const unsigned long long ma = reinterpret_cast<unsigned long long>(dst_a);
-  const unsigned long long mb = reinterpret_cast<unsigned long long>(dst_b);
-  const int ch = lane & 15;
-#pragma unroll 4
-  for (int i = 0; i < 16; ++i) {
-    const int r = 2 * i + (lane >> 4);
-    const unsigned long long da = __shfl_sync(0xffffffffu, ma, r), db = __shfl_sync(0xffffffffu, mb, r);
-    const uint4 v = *reinterpret_cast<const uint4*>(stage + r * 256 + ((ch ^ (r & 15)) << 4));
-    const unsigned long long d = (ch < 8) ? da + ch * 16 : db + (ch - 8) * 16;
-    if (da) *reinterpret_cast<uint4*>(d) = v;
   }
   __syncwarp();
 }
@@ -156,47 +139,75 @@ __device__ __forceinline__ void push_stage_flush_red(uint8_t* stage, int lane, f
   __syncwarp();
 }
 
-// SwiGLU backward of a pair of columns: d(gate) = d(act) * up * dsilu(gate), d(up) = d(act) * silu(gate).
-__device__ __forceinline__ void swiglu_bwd_pair(float d0, float d1, uint32_t gw, uint32_t uw, uint32_t& og, uint32_t& ou) {
-  const float2 g2 = unpack_bf16x2(gw), u2 = unpack_bf16x2(uw);
-  const float s0 = 1.f / (1.f + __expf(-g2.x)), s1 = 1.f / (1.f + __expf(-g2.y));
-  const float si0 = g2.x * s0, si1 = g2.y * s1;
-  og = pack_bf16x2(d0 * u2.x * (s0 + si0 * (1.f - s0)), d1 * u2.y * (s1 + si1 * (1.f - s1)));
-  ou = pack_bf16x2(d0 * si0, d1 * si1);
-}
-
-// Operand u = [gate | up] of the SwiGLU backward epilogue, requested one step (32 rows x 32 gate and 32 up columns, 4 KB per
-// warp) ahead as 64-byte row segments with asynchronous copies, across tiles: it does not depend on the products. Read by
-// the lane that owns the row; 16-byte chunks XOR-swizzled by row. Read by every lane from its own row when its turn came, 32
-// rows per instruction, the operand's latency was paid four times per tile: 28800 x 2048 x 768 211 -> 168 us, 28800 x 1536 x
-// 512 158 -> 119, 64800 x 4096 x 1536 1088 -> 918. What is left is the arithmetic (two exponentials and two divisions per
-// element) and shared memory, which operands and staging fill to the brim: at 28800 x 2048 x 768 each of the 13 rounds of
-// tiles takes 12.9 us, of which the products alone would take 4.6 at the rate of a large GEMM (1.6 PFLOP/s).
-constexpr int SWIGLU_U_BYTES = 4096;
-__device__ __forceinline__ void swiglu_u_request(uint8_t* buf, const GemmParams& p, int row0, int col, int lane) {
+// bf16 output columns of a warp's 32 rows on their way out: two tiles of 64 columns in shared memory, which one lane hands
+// to the TMA unit when they are complete; rows past the matrix are clipped. Written by the warp itself, two 256-byte row
+// segments an instruction behind two shuffles and a read, the stores took longer than the products of short reductions.
+// us, bursts, before / now: 28800 x 1536 x 512 53.3 / 48.1, gated residual 28800 x 512 x 512 30.6 / 26.9, SwiGLU with the raw
+// columns 28800 x 3072 x 512 110.5 / 98.2, 57600 x 4096 x 768 331 / 308, plain 57600 x 2304 x 768 166 / 161, gated 64800 x
+// 1536 x 1536 234 / 228.
+struct TileOut {
+  uint8_t* stage;        // 8 KB
+  int lane;
+  // both tiles may be written again
+  __device__ __forceinline__ void wait_all() const {
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    __syncwarp();
+  }
+  // the tile before the last one may
+  __device__ __forceinline__ void wait_one() const {
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+    __syncwarp();
+  }
+  // 32 columns of this lane's row: first or second half of tile `t`
+  __device__ __forceinline__ void put(int t, int half, const uint32_t (&o)[16]) const {
+    uint8_t* b = stage + t * 4096 + lane * 128;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int r = i * 4 + (lane >> 3), ch = lane & 7;
-    if (row0 + r < p.M) {
-      const int c = col + (ch & 3) * 8 + (ch < 4 ? 0 : p.swiglu_f);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(buf + r * 128 + ((ch ^ (r & 7)) << 4))),
-                   "l"(p.resid + static_cast<size_t>(row0 + r) * p.ldr + c)
-                   : "memory");
+    for (int i = 0; i < 4; ++i)
+      *reinterpret_cast<uint4*>(b + (((4 * half + i) ^ (lane & 7)) << 4)) =
+          make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+  }
+  // tile `t`, complete, to columns `col`.. of the 32 rows from `row`: a group of its own
+  __device__ __forceinline__ void send(int t, const CUtensorMap* m, int col, int row, int n_rows) const {
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      if (row < n_rows) tma_store_2d(m, stage + t * 4096, col, row);
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     }
+    __syncwarp();
   }
-}
-__device__ __forceinline__ void swiglu_u_take(const uint8_t* buf, int lane, uint4 (&g)[4], uint4 (&u)[4]) {
-  asm volatile("cp.async.wait_all;" ::: "memory");
-  __syncwarp();
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    g[i] = *reinterpret_cast<const uint4*>(buf + lane * 128 + ((i ^ (lane & 7)) << 4));
-    u[i] = *reinterpret_cast<const uint4*>(buf + lane * 128 + (((i + 4) ^ (lane & 7)) << 4));
+  // before the warp leaves: its copies have been performed
+  __device__ __forceinline__ void drain() const {
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
-  __syncwarp();       // the buffer may be filled again
+};
+
+// SwiGLU backward of a pair of columns, in packed arithmetic: d(gate) = d(act) * up * dsilu(gate), d(up) = d(act) *
+// silu(gate).
+__device__ __forceinline__ void swiglu_bwd_pair(uint32_t d0, uint32_t d1, uint32_t gw, uint32_t uw, uint32_t& og,
+                                                uint32_t& ou) {
+  const uint64_t g = f2_from_bf16x2(gw), u = f2_from_bf16x2(uw), d = f2_pack(__uint_as_float(d0), __uint_as_float(d1));
+  float g0, g1;
+  f2_unpack(g, g0, g1);
+  const uint64_t one = f2_pack(1.f, 1.f);
+  const uint64_t s = f2_pack(1.f / (1.f + __expf(-g0)), 1.f / (1.f + __expf(-g1))), si = f2_mul(g, s);
+  og = f2_to_bf16x2(f2_mul(f2_mul(d, u), f2_fma(si, f2_sub(one, s), s)));
+  ou = f2_to_bf16x2(f2_mul(d, si));
 }
 
-// The same for the residual of the gated epilogue: 32 rows x 64 columns per step, 128-byte row segments.
+// Operand u = [gate | up] of the SwiGLU backward epilogue on eight warps, 32 rows x 32 gate and 32 up columns a step: tiled
+// loads one step ahead, across tiles (it does not depend on the products), into one of two buffers of the warp; the
+// gradients of a step take the place of its operand and leave from there as tiled stores. That is all the shared memory
+// the epilogue needs, so the ring of operands keeps its five stages. us, bursts, asynchronous 16-byte copies and stores by
+// the warp / now: 28800 x 1536 x 512 101 / 98, 57600 x 2048 x 768 262 / 241, 64800 x 4096 x 1536 787 / 763, 7200 x 512 x 256
+// 16.2 / 14.4. Without the operand ahead its latency is paid four times a tile (28800 x 2048 x 768: 211 us for 168 then). With
+// gradients in tiles of their own, 64 columns wide, and four stages 97, 242 and 792. What is left are the arithmetic (two
+// exponentials and two divisions per element; none of it: 10 % less) and the products' own loads beside 2.3 GB of
+// operand and gradients (no loads and stores: 64800 x 4096 x 1536 595 us, the products alone 519).
+constexpr int SWIGLU_U_BYTES = 4096;
+
+// Residual of the gated epilogue, requested one step (32 rows x 64 columns, 4 KB per warp) ahead as 128-byte row segments
+// with asynchronous copies. Read by the lane that owns the row; 16-byte chunks XOR-swizzled by row.
 __device__ __forceinline__ void resid_request(uint8_t* buf, const GemmParams& p, int row0, int col, int lane) {
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
@@ -217,10 +228,12 @@ __device__ __forceinline__ void resid_take(const uint8_t* buf, int lane, uint4 (
 
 // One thread = one accumulator row (TMEM lane) of a BN-column tile whose first accumulator column is `taddr`.
 // `row` is the global output row, `tn` the tile's index along N, `kempty` marks a split-K slice without work.
-// `stage`: this warp's PUSH_STAGE_BYTES of shared memory for the push epilogues, or null (direct stores).
+// `stage`: this warp's PUSH_STAGE_BYTES of shared memory. `mc`, `mx`: tensor maps of the bf16 output and of the raw columns,
+// boxes of 64 columns x 32 rows, or null (direct stores).
 template <int BN>
 __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t taddr, int row, bool row_ok, int tn,
-                                                  bool kempty, uint8_t* stage = nullptr, int part = 0, int parts = 1) {
+                                                  bool kempty, uint8_t* stage = nullptr, int part = 0, int parts = 1,
+                                                  const CUtensorMap* mc = nullptr, const CUtensorMap* mx = nullptr) {
   const int lane = threadIdx.x & 31;
   // columns of this warp: all, or one of two halves where eight warps share a tile; p.N - tn * BN is 128 in a half-empty
   // last tile of the two-CTA kernel
@@ -291,49 +304,51 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
       }
     }
   } else if (p.epi == EPI_SWIGLU_BWD) {
-    // d(gate) = d(act) * up * dsilu(gate), d(up) = d(act) * silu(gate); u is read and d(u) written in place
-    const __nv_bfloat16* usrc = p.resid + static_cast<size_t>(row) * p.ldr + tn * BN;
+    // u is read and d(u) written in place
+    const __nv_bfloat16* usrc = p.resid + static_cast<size_t>(min(row, p.M - 1)) * p.ldr + tn * BN;
     __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(row) * p.ldc + tn * BN;
+    const TileOut to{stage, lane};
 #pragma unroll 1
     for (int c = c_lo; c < c_hi; c += 32) {
-      uint32_t v[32];
+      uint32_t v[32], og[16], ou[16];
       tmem_ld32(taddr + c, v);
       tmem_wait_ld();
-      if (row_ok) {
-        uint32_t og[16], ou[16];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint4 g4 = *reinterpret_cast<const uint4*>(usrc + c + 8 * i);
+        const uint4 u4 = *reinterpret_cast<const uint4*>(usrc + p.swiglu_f + c + 8 * i);
+        const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w}, uw[4] = {u4.x, u4.y, u4.z, u4.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          swiglu_bwd_pair(v[8 * i + 2 * j], v[8 * i + 2 * j + 1], gw[j], uw[j], og[4 * i + j], ou[4 * i + j]);
+      }
+      if (mc) {
+        // 64 d(gate) columns and the matching 64 d(up) columns are a tile each
+        if (!(c & 32)) to.wait_all();
+        to.put(0, (c >> 5) & 1, og);
+        to.put(1, (c >> 5) & 1, ou);
+        if (c & 32) {
+          to.send(0, mc, tn * BN + c - 32, row - lane, p.M);
+          to.send(1, mc, p.swiglu_f + tn * BN + c - 32, row - lane, p.M);
+        }
+      } else if (row_ok) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const uint4 g4 = *reinterpret_cast<const uint4*>(usrc + c + 8 * i);
-          const uint4 u4 = *reinterpret_cast<const uint4*>(usrc + p.swiglu_f + c + 8 * i);
-          const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w}, uw[4] = {u4.x, u4.y, u4.z, u4.w};
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            swiglu_bwd_pair(__uint_as_float(v[8 * i + 2 * j]), __uint_as_float(v[8 * i + 2 * j + 1]), gw[j], uw[j],
-                            og[4 * i + j], ou[4 * i + j]);
-        }
-        if (stage != nullptr && p.staged_out) {
-          // 64 d(gate) columns and the matching 64 d(up) columns share one stage group
-          push_stage_put(stage, lane, (c & 32), og);
-          push_stage_put(stage, lane, 64 + (c & 32), ou);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            *reinterpret_cast<uint4*>(dst + c + 8 * i) = make_uint4(og[4 * i], og[4 * i + 1], og[4 * i + 2], og[4 * i + 3]);
-            *reinterpret_cast<uint4*>(dst + p.swiglu_f + c + 8 * i) =
-                make_uint4(ou[4 * i], ou[4 * i + 1], ou[4 * i + 2], ou[4 * i + 3]);
-          }
+          *reinterpret_cast<uint4*>(dst + c + 8 * i) = make_uint4(og[4 * i], og[4 * i + 1], og[4 * i + 2], og[4 * i + 3]);
+          *reinterpret_cast<uint4*>(dst + p.swiglu_f + c + 8 * i) =
+              make_uint4(ou[4 * i], ou[4 * i + 1], ou[4 * i + 2], ou[4 * i + 3]);
         }
       }
-      if (stage != nullptr && p.staged_out && (c & 32))
-        push_stage_flush2(stage, lane, row_ok ? dst + (c - 32) : nullptr, row_ok ? dst + p.swiglu_f + (c - 32) : nullptr);
     }
-  } else if ((p.epi == EPI_SWIGLU || p.epi == EPI_SWIGLU_BOTH) && stage != nullptr && p.staged_out && BN == 256) {
-    // staged stores: the 128 activation columns of the tile are one stage group; with EPI_SWIGLU_BOTH the raw gate
-    // and up columns follow as two more groups (second pass over the accumulator in TMEM)
+  } else if ((p.epi == EPI_SWIGLU || p.epi == EPI_SWIGLU_BOTH) && mc != nullptr && BN == 256) {
+    // the 128 activation columns of the tile are two tiled stores; with EPI_SWIGLU_BOTH the raw gate and up columns follow
+    // as two each (second pass over the accumulator in TMEM)
     constexpr int H = BN / 2;
-    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(row) * p.ldc + tn * H;
     // of two warps that share the rows the first writes the activation, the second the raw columns
+    const TileOut to{stage, lane};
+    const int row0 = row - lane;
     if (part == 0) {
+      to.wait_all();
 #pragma unroll 1
       for (int c = 0; c < H; c += 32) {
         uint32_t g[32], u[32];
@@ -348,14 +363,14 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
           const float s0 = g0 / (1.f + __expf(-g0)), s1 = g1 / (1.f + __expf(-g1));
           o[i] = pack_bf16x2(s0 * u0, s1 * u1);
         }
-        push_stage_put(stage, lane, c, o);
+        to.put(c >> 6, (c >> 5) & 1, o);
+        if (c & 32) to.send(c >> 6, mc, tn * H + c - 32, row0, p.M);
       }
-      push_stage_flush(stage, lane, row_ok ? out : nullptr);
     }
     if (p.epi == EPI_SWIGLU_BOTH && part == parts - 1) {
-      __nv_bfloat16* raw = p.aux + static_cast<size_t>(row) * p.ld_aux + tn * H;
 #pragma unroll 1
       for (int half = 0; half < 2; ++half) {
+        to.wait_all();
 #pragma unroll 1
         for (int c = 0; c < H; c += 32) {
           uint32_t v[32], o[16];
@@ -363,9 +378,9 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
           tmem_wait_ld();
 #pragma unroll
           for (int i = 0; i < 16; ++i) o[i] = pack_bf16x2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
-          push_stage_put(stage, lane, c, o);
+          to.put(c >> 6, (c >> 5) & 1, o);
+          if (c & 32) to.send(c >> 6, mx, half * p.swiglu_f + tn * H + c - 32, row0, p.M);
         }
-        push_stage_flush(stage, lane, row_ok ? raw + half * p.swiglu_f : nullptr);
       }
     }
   } else if (p.epi == EPI_SWIGLU || p.epi == EPI_SWIGLU_BOTH) {
@@ -453,11 +468,10 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
         }
       }
     }
-  } else if (stage != nullptr && p.staged_out && p.aux == nullptr) {
-    // EPI_STORE / EPI_GATE_RESID with coalesced stores: every lane combines its own row (the residual is read
-    // directly: staging it too was measured slower), the packed results of a 128-column group go through the warp's
-    // stage and leave as 256-byte row segments.
-    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(row) * p.ldc + tn * BN;
+  } else if (mc != nullptr && p.aux == nullptr) {
+    // EPI_STORE / EPI_GATE_RESID: every lane combines its own row (the residual is read directly: staging it too was
+    // measured slower), 64 columns leave at a time.
+    const TileOut to{stage, lane};
     const bool gated = (p.epi == EPI_GATE_RESID) && row_ok;
     const __nv_bfloat16* res = p.resid ? p.resid + static_cast<size_t>(row) * p.ldr + tn * BN : nullptr;
     const float* gate = nullptr;
@@ -499,8 +513,9 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
 #pragma unroll
         for (int i = 0; i < 16; ++i) o[i] = pack_bf16x2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
       }
-      push_stage_put(stage, lane, c & 127, o);
-      if ((c & 127) == 96) push_stage_flush(stage, lane, row_ok ? out + (c - 96) : nullptr);
+      if (!(c & 32)) to.wait_one();
+      to.put((c >> 6) & 1, (c >> 5) & 1, o);
+      if (c & 32) to.send((c >> 6) & 1, mc, tn * BN + c - 32, row - lane, p.M);
     }
   } else {
     // EPI_STORE / EPI_GATE_RESID : bf16 output

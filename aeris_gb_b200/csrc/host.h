@@ -6,6 +6,9 @@ namespace aeris {
 // 2-D bf16 map with 128-byte swizzle: `inner` contiguous elements, `rows` rows of pitch `ld` elements.
 int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t rows, uint64_t ld,
                       uint32_t box_inner, uint32_t box_rows);
+// The same with the 64-byte swizzle, for boxes of 32 columns.
+int make_tmap_2d_sw64_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t rows, uint64_t ld,
+                           uint32_t box_inner, uint32_t box_rows);
 // Heads of window-major token rows, 128-byte swizzle: dims {d, heads, tokens, windows} of a [windows * tokens, ld] tensor
 // whose first head starts at `base`; box {64, 1, box_rows, 1}. Channels past d, tokens past the window's end: zeros.
 int make_tmap_heads_bf16(CUtensorMap* out, const void* base, int d, int heads, int tokens, int windows, uint64_t ld,
