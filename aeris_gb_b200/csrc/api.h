@@ -133,6 +133,8 @@ int aeris_modulation_mlp_bwd(const void* W1, int flags1, const void* x, float* d
                              const void* W2, int flags2, const float* y1, const float* dy, float* dW2, float* db2,
                              float* dy1, int N2, int B, void* stream);
 int aeris_noise_embedding(const float* t, void* out, int out_bf16, int B, int dim, double max_period, void* stream);
+// The same of 1 to 64 levels that the host knows (no copy: they travel as kernel arguments).
+int aeris_noise_embedding_of(const float* levels, void* out, int out_bf16, int n, int dim, double max_period, void* stream);
 int aeris_pack_embed_weights(const float* W, const float* b, void* out, int D, int Cin, int KP, void* stream);
 int aeris_fold_embed_grad(const float* G, float* dW, float* db, int D, int Cin, int KP, void* stream);
 int aeris_pack_head_weights(const float* W, void* out, int C, int rows, int D, void* stream);
@@ -169,6 +171,8 @@ typedef struct AerisBlockGrad {
 // that failed less 1000 times its place.
 int aeris_block_forward(const AerisBlock* b);
 int aeris_block_backward(const AerisBlock* b, const AerisBlockGrad* g);
+// aeris_block_forward of `n` records in a row, each with `mod + mod_offset` and on `stream`; same result codes.
+int aeris_blocks_forward(const AerisBlock* blocks, int n, long long mod_offset, void* stream);
 
 #ifdef __cplusplus
 }

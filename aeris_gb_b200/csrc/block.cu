@@ -134,6 +134,21 @@ extern "C" int aeris_block_forward(const AerisBlock* pb) {
   return run.result();
 }
 
+// The whole trunk of a network evaluation. A sampler's evaluations differ in the modulation vectors only: `mod_offset`
+// elements further on in every block's.
+extern "C" int aeris_blocks_forward(const AerisBlock* blocks, int n, long long mod_offset, void* stream) {
+  int launches = 0;
+  for (int i = 0; i < n; ++i) {
+    AerisBlock b = blocks[i];
+    b.mod += mod_offset;
+    b.stream = stream;
+    const int rc = aeris_block_forward(&b);
+    if (rc < 0) return rc;
+    launches += rc;
+  }
+  return launches;
+}
+
 extern "C" int aeris_block_backward(const AerisBlock* pb, const AerisBlockGrad* pg) {
   const AerisBlock& b = *pb;
   const AerisBlockGrad& g = *pg;

@@ -13,9 +13,18 @@ namespace aeris {
 
 // out[b, :] = [sin(t f_i) | cos(t f_i)], f_i = exp(-ln(max_period) i / half). Double precision: a handful of values, and the
 // fast single-precision sine would cost accuracy at large angles.
-template <typename OT>
-__global__ void noise_embedding_kernel(const float* __restrict__ t, OT* __restrict__ out, int B, int dim,
-                                       double log_period) {
+// `Levels`: where t comes from, an array in memory or one that travels with the launch.
+constexpr int MAX_LEVELS = 64;
+struct DeviceLevels {
+  const float* t;
+  __device__ float operator[](int b) const { return t[b]; }
+};
+struct HostLevels {
+  float t[MAX_LEVELS];
+  __device__ float operator[](int b) const { return t[b]; }
+};
+template <typename OT, typename Levels>
+__global__ void noise_embedding_kernel(const Levels t, OT* __restrict__ out, int B, int dim, double log_period) {
   const int half = dim / 2;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < B * half; i += gridDim.x * blockDim.x) {
     const int b = i / half, k = i - b * half;
@@ -261,8 +270,8 @@ static int small_grid(long long n) {
 }
 static int launched() { return cudaGetLastError() == cudaSuccess ? 0 : -21; }
 
-extern "C" int aeris_noise_embedding(const float* t, void* out, int out_bf16, int B, int dim, double max_period,
-                                     void* stream) {
+template <typename Levels>
+static int noise_embedding(const Levels& t, void* out, int out_bf16, int B, int dim, double max_period, void* stream) {
   if (B <= 0 || dim <= 0 || dim % 2 || !(max_period > 0)) return -1;
   const cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int grid = small_grid(static_cast<long long>(B) * (dim / 2));
@@ -270,6 +279,17 @@ extern "C" int aeris_noise_embedding(const float* t, void* out, int out_bf16, in
   if (out_bf16) noise_embedding_kernel<<<grid, 256, 0, st>>>(t, reinterpret_cast<__nv_bfloat16*>(out), B, dim, lp);
   else          noise_embedding_kernel<<<grid, 256, 0, st>>>(t, reinterpret_cast<float*>(out), B, dim, lp);
   return launched();
+}
+extern "C" int aeris_noise_embedding(const float* t, void* out, int out_bf16, int B, int dim, double max_period,
+                                     void* stream) {
+  return noise_embedding(DeviceLevels{t}, out, out_bf16, B, dim, max_period, stream);
+}
+extern "C" int aeris_noise_embedding_of(const float* levels, void* out, int out_bf16, int n, int dim, double max_period,
+                                        void* stream) {
+  if (n <= 0 || n > MAX_LEVELS) return -1;
+  HostLevels t = {};
+  for (int i = 0; i < n; ++i) t.t[i] = levels[i];
+  return noise_embedding(t, out, out_bf16, n, dim, max_period, stream);
 }
 
 // flags: 1 = W fp32 (else bf16), 2 = bias bf16 (else fp32), 4 = x bf16 (else fp32)

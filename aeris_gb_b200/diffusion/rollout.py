@@ -102,6 +102,7 @@ class DeviceForecaster(Forecaster):
     def step(self, state: torch.Tensor, forcing: torch.Tensor | None, generator=None, x_init=None) -> torch.Tensor:
         import math
         from ..models import fused_io
+        from ..models.sampling import Evaluations
         from ..ops import diffusion as DF
         s = self.s
         M = state.shape[0]
@@ -116,20 +117,37 @@ class DeviceForecaster(Forecaster):
         else:
             x = DF.noise_mix(torch.empty_like(state), 0.0, s.sigma_data, self._next_seed(), geom)
         x_e = torch.empty_like(x)
-        level = lambda v: torch.full((M,), v, device=state.device)
+        # per step: from which level, how much fresh noise before it, to which level
+        moves, levels = [], []
         for i in range(s.n_steps):
-            cur, nxt = ts[i], ts[i + 1]
+            cur, nxt, churn = ts[i], ts[i + 1], None
             if s.s_churn > 0 and s.s_min <= math.tan(cur) * s.sigma_data <= s.s_max:
                 gamma = min(s.s_churn / s.n_steps, math.sqrt(2) - 1)
                 hat = math.atan(math.tan(cur) * (1 + gamma))
-                rot = math.atan(max(math.tan(hat) - math.tan(cur), 0.0))
-                DF.noise_mix(x, math.cos(rot), math.sin(rot) * s.sigma_data * s.s_noise, self._next_seed(), geom)
+                churn = math.atan(max(math.tan(hat) - math.tan(cur), 0.0))
                 cur = hat
+            second = s.heun and i < s.n_steps - 1
+            moves.append((cur, nxt, churn, second))
+            levels += [cur, nxt] if second else [cur]
+        together = Evaluations.prepare(self.model, c_img, levels, self.ctx, plan, 2 if s.heun else 1, x)
+        n_evals = 0
+
+        def network(x, slot):
+            nonlocal n_evals
+            n_evals += 1
+            if together is not None:
+                return together.run(n_evals - 1, x, slot)
+            return self.model.predict_images(x, c_img, torch.full((M,), levels[n_evals - 1], device=state.device), self.ctx,
+                                             plan)
+
+        for cur, nxt, churn, second in moves:
+            if churn is not None:
+                DF.noise_mix(x, math.cos(churn), math.sin(churn) * s.sigma_data * s.s_noise, self._next_seed(), geom)
             d = (nxt - cur) * s.sigma_data
-            f_s = self.model.predict_images(x, c_img, level(cur), self.ctx, plan)
+            f_s = network(x, 0)
             DF.sampler_update(x_e, x, f_s, None, d, 0.0, geom)
-            if s.heun and i < s.n_steps - 1:
-                f_t = self.model.predict_images(x_e, c_img, level(nxt), self.ctx, plan)
+            if second:
+                f_t = network(x_e, 1)
                 DF.sampler_update(x, x, f_s, f_t, 0.5 * d, 0.5 * d, geom)
             else:
                 x, x_e = x_e, x

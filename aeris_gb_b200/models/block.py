@@ -135,6 +135,12 @@ def forward(meta, x, mod, weights, y, step: int, merged: bool, bufs: dict[str, i
     _issued(_l.lib().aeris_block_forward(ctypes.byref(a)), "aeris_block_forward")
 
 
+def issue_forward(records: ctypes.Array, mod_offset: int) -> None:
+    """The forward passes over consecutive blocks in one call, on the current stream: ``records`` as :func:`_args` lays them
+    out, with ``mod_offset`` elements added to each one's modulation vectors."""
+    _issued(_l.lib().aeris_blocks_forward(records, len(records), _LL(mod_offset), _l.stream_ptr()), "aeris_blocks_forward")
+
+
 def backward(meta, x, mod, dy, weights, step: int, bufs: dict[str, int], kept: bool, work: dict[str, int], dx, dmod,
              grads: dict[str, torch.Tensor]) -> None:
     """``work``: addresses of the gradient workspaces; ``dmod`` [B, 6 D] fp32 is overwritten."""

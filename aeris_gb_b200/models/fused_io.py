@@ -71,15 +71,28 @@ def _pack_dim(c_in: int) -> int:
     return (3 * c_in + 2 + 127) // 128 * 128
 
 
-def embed(x_img, c_img, cs, W, b, plan: IoPlan) -> torch.Tensor:
-    """``(cat[(cos t x + sin t z) / sigma_d, cond] + ape) W^T + b`` -> bf16 token stream in the unshifted window layout."""
+def embed_workspace(c_in: int, T: int, dev) -> torch.Tensor:
+    return workspace().get("embed_a", (min(CHUNK_ROWS, T), _pack_dim(c_in)), torch.bfloat16, dev)
+
+
+def head_workspace(T: int, B: int, D: int, dev) -> torch.Tensor:
+    """The bf16 value and remainder of the normalised rows of one pass over the head."""
+    rows = max(n for *_, n in _sample_chunks(B, T // B))
+    return workspace().get("head_y", (2, rows, D), torch.bfloat16, dev)
+
+
+def embed(x_img, c_img, cs, W, b, plan: IoPlan, packed: torch.Tensor | None = None,
+          out: torch.Tensor | None = None) -> torch.Tensor:
+    """``(cat[(cos t x + sin t z) / sigma_d, cond] + ape) W^T + b`` -> bf16 token stream in the unshifted window layout.
+    ``packed``: :func:`.diffusion.pack_embed_weights` of W and b, from callers with several evaluations to run."""
     D, Cin = W.shape
     KP = _pack_dim(Cin)
     dev = x_img.device
-    Wp = DF.pack_embed_weights(W.detach().float().contiguous(), b.detach().float().contiguous(), KP)
+    Wp = packed if packed is not None else \
+        DF.pack_embed_weights(W.detach().float().contiguous(), b.detach().float().contiguous(), KP)
     T = plan.geom.rows
-    out = torch.empty((T, D), dtype=torch.bfloat16, device=dev)
-    A = workspace().get("embed_a", (min(CHUNK_ROWS, T), KP), torch.bfloat16, dev)
+    out = out if out is not None else torch.empty((T, D), dtype=torch.bfloat16, device=dev)
+    A = embed_workspace(Cin, T, dev)
     for r0 in range(0, T, CHUNK_ROWS):
         n = min(CHUNK_ROWS, T - r0)
         DF.embed_pack(x_img, c_img, cs, plan.geom, plan.ape_y, plan.ape_x, plan.seed, plan.sigma_data,
@@ -164,17 +177,17 @@ def _sample_chunks(B: int, rows_per_sample: int) -> list[tuple[int, int, int, in
 
 
 def head_forward(x: torch.Tensor, shift: torch.Tensor, scale: torch.Tensor, norm_w: torch.Tensor,
-                 head_w: torch.Tensor, eps: float) -> torch.Tensor:
-    """Network output ``F`` in token order, fp32 ``[T, 128]`` (columns past the channel count are zero)."""
+                 head_w: torch.Tensor, eps: float, packed: torch.Tensor | None = None,
+                 pred: torch.Tensor | None = None) -> torch.Tensor:
+    """Network output ``F`` in token order, fp32 ``[T, 128]`` (columns past the channel count are zero). ``packed``:
+    :func:`_head_weights` of ``head_w``."""
     T, D = x.shape
     B = shift.shape[0]
     dev = x.device
-    w3 = _head_weights(head_w)
-    ws = workspace()
+    w3 = packed if packed is not None else _head_weights(head_w)
     spans = _sample_chunks(B, T // B)
-    cm = max(n for *_, n in spans)
-    y = ws.get("head_y", (2, cm, D), torch.bfloat16, dev)
-    pred = torch.empty((T, PAD_N), dtype=torch.float32, device=dev)
+    y = head_workspace(T, B, D, dev)
+    pred = pred if pred is not None else torch.empty((T, PAD_N), dtype=torch.float32, device=dev)
     shift, scale = _mod_rows(shift, scale)
     for b, nb, r0, n in spans:
         _head_rows(x[r0:r0 + n], scale[b:b + nb], shift[b:b + nb], norm_w, w3, eps, pred[r0:r0 + n], y)

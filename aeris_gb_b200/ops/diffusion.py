@@ -179,6 +179,21 @@ def noise_embedding(t: torch.Tensor, dim: int, max_period: float, dtype: torch.d
     return out
 
 
+MAX_LEVELS = 64
+
+
+def noise_embedding_of(levels: list[float], dim: int, max_period: float, dtype: torch.dtype, device) -> torch.Tensor:
+    """:func:`noise_embedding` of levels that the host knows, without a copy to the device (which would wait)."""
+    out = torch.empty((len(levels), dim), dtype=dtype, device=device)
+    for i in range(0, len(levels), MAX_LEVELS):
+        part = levels[i:i + MAX_LEVELS]
+        rc = _l.lib().aeris_noise_embedding_of((ctypes.c_float * len(part))(*part), _l.ptr(out[i:]),
+                                               int(dtype == torch.bfloat16), len(part), dim, ctypes.c_double(max_period),
+                                               _l.stream_ptr())
+        _l.check(rc, "aeris_noise_embedding_of")
+    return out
+
+
 def pack_embed_weights(W: torch.Tensor, b: torch.Tensor, KP: int) -> torch.Tensor:
     """``[hi(W) | hi(W) | lo(W) | hi(b) | lo(b) | 0..]`` (bf16 [D, KP]) of an fp32 weight [D, Cin] and bias."""
     D, Cin = W.shape
