@@ -214,7 +214,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     *s_abort = ab;
   }
   __syncthreads();
-  if (*s_abort) return;
+  if (*s_abort) { chain_point(); return; }
 
   if (threadIdx.x == 0) {
     prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v);
@@ -232,6 +232,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_point();
   const uint32_t tS = tmem_base;          // S : 64 columns
   const uint32_t tO = tmem_base + 64;     // O : HD columns, accumulated over all tiles
 
@@ -534,8 +535,7 @@ static int launch_attn_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const C
     configured = smem;
   }
   dim3 grid((p.N + TILE - 1) / TILE, p.H, p.n_win);
-  kern<<<grid, ATT_THREADS, smem, stream>>>(tq, tk, tv, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  return launch_chained(kern, grid, ATT_THREADS, smem, stream, tq, tk, tv, p);
 }
 
 

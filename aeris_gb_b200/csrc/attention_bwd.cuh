@@ -204,7 +204,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_i0, const __grid_constant
     *s_abort = ab;
   }
   __syncthreads();
-  if (*s_abort) return;
+  if (*s_abort) { chain_point(); return; }
   if (threadIdx.x == 0) {
     prefetch_tmap(&tm_i0); prefetch_tmap(&tm_i1); prefetch_tmap(&tm_r0); prefetch_tmap(&tm_r1);
     for (int i = 0; i < NB; ++i) {
@@ -228,6 +228,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_i0, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_point();
 
   if ((warp & ~3) == R::W_LOAD) {
     regs_dec<R::REGS_REST>();
@@ -781,10 +782,8 @@ static int launch_attn_bwd(const CUtensorMap& tq128, const CUtensorMap& tk64, co
   const long long items = static_cast<long long>((p.N + TILE - 1) / TILE) * p.H * p.n_win;
   if (items > 0x3fffffff) return -23;
   const int n = static_cast<int>(items), grid = n < num_sms() ? n : num_sms();
-  k1<<<grid, R1::THREADS, R1::SMEM, stream>>>(tq128, tdo128, tk64, tv64, out[0], out[0], p, n);
-  if (cudaGetLastError() != cudaSuccess) return -21;
-  k2<<<grid, R2::THREADS, R2::SMEM, stream>>>(tk128, tv128, tq64, tdo64, out[1], out[2], p, n);
-  return cudaGetLastError() == cudaSuccess ? 0 : -22;
+  if (launch_chained(k1, grid, R1::THREADS, R1::SMEM, stream, tq128, tdo128, tk64, tv64, out[0], out[0], p, n)) return -21;
+  return launch_chained(k2, grid, R2::THREADS, R2::SMEM, stream, tk128, tv128, tq64, tdo64, out[1], out[2], p, n) ? -22 : 0;
 }
 
 }  // namespace aeris

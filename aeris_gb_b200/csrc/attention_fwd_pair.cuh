@@ -132,7 +132,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     *s_abort = ab;
   }
   __syncthreads();
-  if (*s_abort) return;
+  if (*s_abort) { chain_point(); return; }
   if (threadIdx.x == 0) {
     prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v);
     for (int i = 0; i < 4; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); }
@@ -152,6 +152,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_point();
 
   if (warp == 8) {
     // ------------------------------------------------------------ TMA producer
@@ -533,8 +534,7 @@ static int launch_attn_fwd_pair(const CUtensorMap& tq, const CUtensorMap& tk, co
   const int nkv = (p.N + KVP - 1) / KVP;
   if (items > 0x3fffffff || items * nkv > 0x3fffffffll * num_sms()) return -23;
   const int n = static_cast<int>(items), grid = n < num_sms() ? n : num_sms();
-  kern<<<grid, R::THREADS, R::SMEM, stream>>>(tq, tk, tv, to, p, n);
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  return launch_chained(kern, grid, R::THREADS, R::SMEM, stream, tq, tk, tv, to, p, n);
 }
 
 }  // namespace aeris

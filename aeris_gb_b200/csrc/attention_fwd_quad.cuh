@@ -74,7 +74,7 @@ attn_fwd_quad_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     *s_abort = ab;
   }
   __syncthreads();
-  if (*s_abort) return;
+  if (*s_abort) { chain_point(); return; }
   if (threadIdx.x == 0) {
     prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v);
     for (int c = 0; c < NC; ++c) {
@@ -89,6 +89,7 @@ attn_fwd_quad_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_point();
 
   if (warp >= R::W_LOAD) {
     regs_dec<R::REGS_REST>();
@@ -375,8 +376,7 @@ static int launch_attn_fwd_quad(const CUtensorMap& tq, const CUtensorMap& tk, co
   const int nkv = (p.N + KVT - 1) / KVT;
   if (items > 0x3fffffff || items * nkv > 0x3fffffffll * num_sms()) return -23;
   const int n = static_cast<int>(items), grid = n < num_sms() ? n : num_sms();
-  attn_fwd_quad_kernel<<<grid, R::THREADS, R::SMEM, stream>>>(tq, tk, tv, to, p, n);
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  return launch_chained(attn_fwd_quad_kernel, grid, R::THREADS, R::SMEM, stream, tq, tk, tv, to, p, n);
 }
 
 }  // namespace aeris

@@ -79,6 +79,7 @@ embed_pack_kernel(const float* __restrict__ x_img, const float* __restrict__ c_i
                   TokGeom g, int Cx, int Cc, const float* __restrict__ ape_y, const float* __restrict__ ape_x,
                   int ape_ch, unsigned long long seed, float sd, int noise, __nv_bfloat16* __restrict__ out, int KP,
                   long long row0, long long rows) {
+  chain_point();
   __shared__ float vbuf[EMBED_WARPS][EMBED_MAX_C];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float* v = vbuf[warp];
@@ -194,6 +195,7 @@ trigflow_loss_kernel(const float* __restrict__ pred, int ldp, const float* __res
 __global__ void sampler_update_kernel(float* __restrict__ x_out, const float* __restrict__ x_base,
                                       const float* __restrict__ pa, const float* __restrict__ pb, int ldp, float ca,
                                       float cb, TokGeom g, int Cx, long long rows) {
+  chain_point();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (long long i = static_cast<long long>(blockIdx.x) * nw + warp; i < rows;
        i += static_cast<long long>(gridDim.x) * nw) {
@@ -271,10 +273,9 @@ extern "C" int aeris_embed_pack(const float* x_img, const float* c_img, const fl
   if (!geom_ok(g) || Cx <= 0 || Cc < 0 || Cx + Cc > EMBED_MAX_C || KP % 8 || KP < 3 * (Cx + Cc) + 2 || rows <= 0)
     return -1;
   if (row0 < 0 || row0 + rows > static_cast<long long>(g->B) * g->nwy_loc * g->nwx_loc * g->n_local) return -2;
-  embed_pack_kernel<<<warp_grid(rows, EMBED_WARPS), EMBED_WARPS * 32, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      x_img, c_img, cs, *g, Cx, Cc, ape_y, ape_x, ape_ch, seed, sd, noise, reinterpret_cast<__nv_bfloat16*>(out), KP,
-      row0, rows);
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  return launch_chained(embed_pack_kernel, warp_grid(rows, EMBED_WARPS), EMBED_WARPS * 32, 0,
+                        reinterpret_cast<cudaStream_t>(stream), x_img, c_img, cs, *g, Cx, Cc, ape_y, ape_x, ape_ch, seed, sd,
+                        noise, reinterpret_cast<__nv_bfloat16*>(out), KP, row0, rows);
 }
 
 extern "C" int aeris_trigflow_loss(const float* pred, int ldp, const float* x_img, const float* cs, const TokGeom* g,
@@ -293,9 +294,8 @@ extern "C" int aeris_sampler_update(float* x_out, const float* x_base, const flo
                                     float ca, float cb, const TokGeom* g, int Cx, void* stream) {
   if (!geom_ok(g) || Cx <= 0 || Cx > ldp) return -1;
   const long long rows = static_cast<long long>(g->B) * g->nwy_loc * g->nwx_loc * g->n_local;
-  sampler_update_kernel<<<warp_grid(rows, 8), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      x_out, x_base, pa, pb, ldp, ca, cb, *g, Cx, rows);
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  return launch_chained(sampler_update_kernel, warp_grid(rows, 8), 256, 0, reinterpret_cast<cudaStream_t>(stream), x_out,
+                        x_base, pa, pb, ldp, ca, cb, *g, Cx, rows);
 }
 
 extern "C" int aeris_noise_mix(float* x, float a, float b, unsigned long long seed, const TokGeom* g, int Cx,

@@ -255,6 +255,7 @@ modnorm_fwd_pair_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __r
                         const float* __restrict__ shift, const __nv_bfloat16* __restrict__ w,
                         std::conditional_t<F32, float, __nv_bfloat16>* __restrict__ h, int rows, int D, int mode,
                         float eps, const float* __restrict__ wf, __nv_bfloat16* __restrict__ h_lo, int mod_stride) {
+  chain_point();
   static_assert(FWD_RPI == 4 && MAXT <= 256 * W8, "group_sum4 adds four values of at most 8 * W8 warps");
   __shared__ float red[2][32 * W8];
   {  // grid.y = samples of `rows` rows each, with a modulation vector of their own
@@ -527,6 +528,7 @@ modnorm_bwd_group_kernel(const __nv_bfloat16* __restrict__ x,
                          __nv_bfloat16* __restrict__ dx, float* __restrict__ dscale, float* __restrict__ dshift,
                          float* __restrict__ dw, int rows, int D, int mode, float eps, const float* __restrict__ wf, int nt,
                          int vec_atomics) {
+  chain_point();
   static_assert(RPI <= 2, "group_sum4 adds two values of two rows");
   constexpr bool PSMEM = VPT > 1;
   // [groups][3][D] column sums; with PSMEM first [3][D]: 1 + scale, shift, weight
@@ -797,6 +799,7 @@ __global__ void __launch_bounds__(256) column_sums_kernel(const float* __restric
 // ------------------------------------------------------------------------------------------------ row gather
 __global__ void gather_rows_kernel(const uint32_t* __restrict__ gidx, PeerPtrs peers,
                                    __nv_bfloat16* __restrict__ out, long long rows, int D) {
+  chain_point();
   const int vec_per_row = D / 8;
   const long long total = rows * vec_per_row;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -864,6 +867,7 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ u, const __n
 // pass applies to the gradients of the rotated q and k). One thread: eight channels = four pairs.
 __global__ void rope_qk_kernel(__nv_bfloat16* __restrict__ qkv, const float* __restrict__ cs, const float* __restrict__ sn,
                                long long rows, int L, int heads, int d, int inverse) {
+  chain_point();
   const int HD = heads * d;
   const int vec_per_row = 2 * HD / 8;              // q and k sections only
   const long long total = rows * vec_per_row;
@@ -944,6 +948,7 @@ struct GatedMatrix {
 };
 __global__ void gate_prepare_kernel(const GatedMatrix m0, const GatedMatrix m1, int R, float* __restrict__ zero,
                                     int n_zero) {
+  chain_point();
   const GatedMatrix& m = blockIdx.y ? m1 : m0;
   const int vec = m.C / 8;
   const long long total = static_cast<long long>(R) * vec, step = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -963,6 +968,7 @@ __global__ void gate_prepare_kernel(const GatedMatrix m0, const GatedMatrix m1, 
     for (long long i = first; i < n_zero; i += step) zero[i] = 0.f;
 }
 __global__ void gate_finalize_pair_kernel(const GatedMatrix m0, const GatedMatrix m1) {
+  chain_point();
   __shared__ float red[2 * 1 * 32];
   const GatedMatrix& m = blockIdx.y ? m1 : m0;
   const int r = blockIdx.x;
@@ -1143,11 +1149,11 @@ static int modnorm_fwd_impl(const void* x, const void* gidx, const void* const* 
     if (grid > cap) grid = cap;
     auto kern = nt <= 192 ? modnorm_fwd_pair_kernel<192, 3, 1>
               : nt <= 320 ? modnorm_fwd_pair_kernel<320, 2, 2> : modnorm_fwd_pair_kernel<640, 1, 3>;
-    kern<<<dim3(grid, batch), nt, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const uint32_t*>(gidx), pp,
-        reinterpret_cast<__nv_bfloat16*>(x_out), scale, shift, reinterpret_cast<const __nv_bfloat16*>(w),
-        reinterpret_cast<__nv_bfloat16*>(h), rows, D, mode, eps, w_f32, reinterpret_cast<__nv_bfloat16*>(h_lo), mod_stride);
-    return cudaGetLastError() == cudaSuccess ? 0 : -21;
+    return launch_chained(kern, dim3(grid, batch), nt, 0, reinterpret_cast<cudaStream_t>(stream),
+                          reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const uint32_t*>(gidx), pp,
+                          reinterpret_cast<__nv_bfloat16*>(x_out), scale, shift, reinterpret_cast<const __nv_bfloat16*>(w),
+                          reinterpret_cast<__nv_bfloat16*>(h), rows, D, mode, eps, w_f32,
+                          reinterpret_cast<__nv_bfloat16*>(h_lo), mod_stride);
   }
   if (grid > aeris_num_sms() * 8) grid = aeris_num_sms() * 8;
   modnorm_fwd_kernel<<<grid, row_threads(D), 0, reinterpret_cast<cudaStream_t>(stream)>>>(
@@ -1201,10 +1207,9 @@ extern "C" int aeris_modnorm_fwd_f32(const void* x, const float* scale, const fl
   if (grid > cap) grid = cap;
   auto kern = nt <= 192 ? modnorm_fwd_pair_kernel<192, 3, 1, true>
             : nt <= 320 ? modnorm_fwd_pair_kernel<320, 2, 2, true> : modnorm_fwd_pair_kernel<640, 1, 3, true>;
-  kern<<<dim3(grid, batch), nt, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const __nv_bfloat16*>(x), nullptr, PeerPtrs{}, nullptr, scale, shift, nullptr, h, rows, D, mode, eps,
-      w_f32, nullptr, D);
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  return launch_chained(kern, dim3(grid, batch), nt, 0, reinterpret_cast<cudaStream_t>(stream),
+                        reinterpret_cast<const __nv_bfloat16*>(x), nullptr, PeerPtrs{}, nullptr, scale, shift, nullptr, h,
+                        rows, D, mode, eps, w_f32, nullptr, D);
 }
 
 template <bool F32>
@@ -1227,11 +1232,11 @@ static int launch_modnorm_bwd_group(const void* x, const void* dh, const void* d
   if (smem > 32 * 1024 &&
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess)
     return -20;
-  kern<<<grid, groups * nt, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const __nv_bfloat16*>(x),
-      reinterpret_cast<const std::conditional_t<F32, float, __nv_bfloat16>*>(dh),
-      reinterpret_cast<const __nv_bfloat16*>(dres), scale, shift, reinterpret_cast<const __nv_bfloat16*>(w),
-      reinterpret_cast<__nv_bfloat16*>(dx), F32 ? sums : dscale, dshift, dw, rows, D, mode, eps, w_f32, nt, vec);
+  launch_chained(kern, grid, groups * nt, smem, reinterpret_cast<cudaStream_t>(stream),
+                 reinterpret_cast<const __nv_bfloat16*>(x),
+                 reinterpret_cast<const std::conditional_t<F32, float, __nv_bfloat16>*>(dh),
+                 reinterpret_cast<const __nv_bfloat16*>(dres), scale, shift, reinterpret_cast<const __nv_bfloat16*>(w),
+                 reinterpret_cast<__nv_bfloat16*>(dx), F32 ? sums : dscale, dshift, dw, rows, D, mode, eps, w_f32, nt, vec);
   if constexpr (F32)
     column_sums_kernel<<<(3 * D + 31) / 32, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(sums, grid, D, dscale, dshift,
                                                                                               dw);
@@ -1272,9 +1277,8 @@ extern "C" int aeris_gather_rows(const void* gidx, const void* const* peer_ptrs,
   for (int i = 0; i < n_peers && i < 16; ++i) pp.p[i] = reinterpret_cast<const __nv_bfloat16*>(peer_ptrs[i]);
   AERIS_FILL_CHECK(pp, n_peers);
   const int grid = grid_for(rows * (D / 8), 256, aeris_num_sms() * 16);
-  gather_rows_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const uint32_t*>(gidx), pp, reinterpret_cast<__nv_bfloat16*>(out), rows, D);
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  return launch_chained(gather_rows_kernel, grid, 256, 0, reinterpret_cast<cudaStream_t>(stream),
+                        reinterpret_cast<const uint32_t*>(gidx), pp, reinterpret_cast<__nv_bfloat16*>(out), rows, D);
 }
 
 extern "C" int aeris_swiglu_fwd(const void* u, void* act, long long rows, int F, void* stream) {
@@ -1307,9 +1311,8 @@ extern "C" int aeris_rope_qk(void* qkv, const float* cos_t, const float* sin_t, 
   if (rows <= 0 || L <= 0 || d % 8 != 0 || heads <= 0) return -1;
   if ((reinterpret_cast<uintptr_t>(cos_t) | reinterpret_cast<uintptr_t>(sin_t)) & 15) return -3;
   const int grid = grid_for(rows * (2 * heads * d / 8), 256, aeris_num_sms() * 16);
-  rope_qk_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<__nv_bfloat16*>(qkv), cos_t, sin_t, rows, L, heads, d, inverse);
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  return launch_chained(rope_qk_kernel, grid, 256, 0, reinterpret_cast<cudaStream_t>(stream),
+                        reinterpret_cast<__nv_bfloat16*>(qkv), cos_t, sin_t, rows, L, heads, d, inverse);
 }
 
 extern "C" int aeris_gate_grad_finalize(float* G, const void* W, const float* g, float* dW, float* dg, int R,
@@ -1329,8 +1332,8 @@ extern "C" int aeris_gate_prepare(const void* W2, const float* g2, void* W2g, fl
   const GatedMatrix a = {reinterpret_cast<const bf*>(W2), g2, reinterpret_cast<bf*>(W2g), G2, nullptr, nullptr, C2};
   const GatedMatrix b = {reinterpret_cast<const bf*>(Wo), go, reinterpret_cast<bf*>(Wog), Go, nullptr, nullptr, Co};
   const int grid = grid_for(static_cast<long long>(R) * ((C2 > Co ? C2 : Co) / 8), 256, aeris_num_sms() * 4);
-  gate_prepare_kernel<<<dim3(grid, 2), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(a, b, R, zero, n_zero);
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  return launch_chained(gate_prepare_kernel, dim3(grid, 2), 256, 0, reinterpret_cast<cudaStream_t>(stream), a, b, R, zero,
+                        n_zero);
 }
 // dW += g * G and dg += rowsum(W * G) for both.
 extern "C" int aeris_gate_finalize_pair(float* G2, const void* W2, const float* g2, float* dW2, float* dg2, int C2,
@@ -1340,8 +1343,7 @@ extern "C" int aeris_gate_finalize_pair(float* G2, const void* W2, const float* 
   typedef __nv_bfloat16 bf;
   const GatedMatrix a = {reinterpret_cast<const bf*>(W2), g2, nullptr, G2, dW2, dg2, C2};
   const GatedMatrix b = {reinterpret_cast<const bf*>(Wo), go, nullptr, Go, dWo, dgo, Co};
-  gate_finalize_pair_kernel<<<dim3(R, 2), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(a, b);
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  return launch_chained(gate_finalize_pair_kernel, dim3(R, 2), 256, 0, reinterpret_cast<cudaStream_t>(stream), a, b);
 }
 
 extern "C" int aeris_sumsq(const float* x, long long n, double* out, void* stream) {

@@ -55,7 +55,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     __shared__ int s_abort;
     if (threadIdx.x == 0) s_abort = (p.status && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
     __syncthreads();
-    if (s_abort) return;
+    if (s_abort) { chain_point(); return; }
   }
 
   const int m_tiles = (p.M + BM - 1) / BM;
@@ -85,6 +85,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_point();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -327,8 +328,7 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmP
   const int m_tiles = (p.M + BM - 1) / BM;
   const int tiles = m_tiles * (p.N / BN) * p.k_splits;
   const int grid = tiles < num_sms() ? tiles : num_sms();
-  kern<<<grid, GEMM_THREADS, S::TOTAL, stream>>>(ta, tb, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  return launch_chained(kern, grid, GEMM_THREADS, S::TOTAL, stream, ta, tb, p);
 }
 
 }  // namespace aeris

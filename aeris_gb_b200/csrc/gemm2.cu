@@ -182,6 +182,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   cluster_sync_all();       // both CTAs' barriers are initialised and TMEM is allocated before anyone signals
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_point();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (each CTA loads its own operands)
@@ -472,8 +473,11 @@ static int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
   const int tiles = mn_tiles * p.k_splits;
   if (tiles < clusters && !AG) clusters = tiles;
   if (AG) p.ag_expect *= static_cast<unsigned>(2 * clusters);   // came in as the call index
-  kern<<<2 * clusters, THREADS, SMEM, stream>>>(ta, tb, tc ? *tc : ta, tx ? *tx : ta, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  if constexpr (AG) {          // waits for its peers: nothing of it starts before its turn
+    kern<<<2 * clusters, THREADS, SMEM, stream>>>(ta, tb, tc ? *tc : ta, tx ? *tx : ta, p);
+    return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  }
+  return launch_chained(kern, 2 * clusters, THREADS, SMEM, stream, ta, tb, tc ? *tc : ta, tx ? *tx : ta, p);
 }
 
 }  // namespace aeris
