@@ -224,8 +224,8 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, const void* s
 // this sound: every thread passes it before it touches global memory, early exits included (the kernel after next waits for
 // this one alone), and a kernel passes it after its TMEM allocation (a waiting CTA may hold what an older one would need).
 // Kernels that wait for other GPUs are launched without it. us per launch, back to back, plain / chained: two-CTA product
-// 256 x 256 x 256 10.3 / 7.6, 14400 x 768 x 768 21.1 / 18.5; a sampler step of seven evaluations of two blocks of width 256 on
-// 14,400 tokens (155 launches) 2.24 / 1.95 ms. Chained products and attention alone: 2.06.
+// 256 x 256 x 256 10.3 / 7.6, 14400 x 768 x 768 21.1 / 18.5; a sampler step of seven evaluations of two blocks of width 256
+// on 14,400 tokens (155 launches) 2.24 / 1.95 ms. Chained products and attention alone: 2.06.
 __device__ __forceinline__ void chain_point() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

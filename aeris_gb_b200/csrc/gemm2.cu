@@ -563,17 +563,39 @@ extern "C" int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M
                       swiglu_f, k_splits, status, stream);
 }
 
-// Which kernel takes a product. A last tile with 128 valid columns costs as much as a full one: 6 % at 2048 columns, far
-// less than the two-CTA kernel gains there (28800 x 13696 x 5120: 4.96 -> 3.38 ms), but 12150 x 1152 x 384 takes 43 us
-// instead of 38; the SwiGLU forward pairs gate and up columns of whole tiles.
+// Which kernel takes a product of N = n * 128 columns: CTA pairs on tiles of 256 x 256, whose last one may be half empty,
+// or single CTAs on tiles of 128 x 128 (256 wide where `bn` is 0 and N allows it). us, bursts, one CTA / pairs:
+//   * plain and gated stores: a wave of pairs takes 1.2 to 1.4 times as long as one of single CTAs, so the numbers of waves
+//     decide. 12150 x 384 x 1152 13.1 / 16.7 (2 and 2 waves), 4096 x 1152 x 3456 28.6 / 39.1 (2, 2), 28800 x 384 x 384
+//     26.2 / 21.8 (5, 4), 12150 x 1152 x 1152 51.0 / 50.5 (6, 4), 12150 x 640 x 640 22.6 / 16.4 (4, 2), 4096 x 1664 x 4992 60.9 /
+//     63.0 (3, 2), 28800 x 896 x 896 87.5 / 59.0 (11, 7); one wave of either: 3600 x 512 x 512 5.6 / 8.8.
+//   * SwiGLU backward: only the pairs' kernel requests its second operand ahead. 4096 x 384 x 128 9.8 / 9.8, 12150 x 896 x
+//     384 44.1 / 28.3, 64800 x 3456 x 1664 1179 / 669.
+//   * SwiGLU forward without the raw columns: its tiles halve on the way out, and short sums leave the epilogue as the
+//     bound, which every CTA of its own overlaps better. 14400 x 1024 x 256 13.8 / 17.2, 64800 x 1024 x 384 59 / 67,
+//     28800 x 3072 x 384 76.6 / 83.6; held for 0.25 s 64800 x 2048 x 384 120 / 126, x 2048 x 512 146 / 144.
+//   * weight gradients (sums over tokens, split where tiles are few): with a half-empty last tile the pairs win by their
+//     longer sums. 1152 x 384 x 12150 14.5 / 18.5, x 28800 31.8 / 32.0, x 64800 69.7 / 63.0; 384 x 384 x 28800 25.2 / 21.6;
+//     1664 x 1664 x 12150 88.0 / 79.1, x 4096 39.0 / 43.9.
+static bool pairs_pay(int M, int N, int K, int epi) {
+  if (epi == EPI_SWIGLU) return K > 384;
+  if (epi == EPI_SWIGLU_BOTH || epi == EPI_SWIGLU_BWD) return true;
+  if (epi == EPI_ACC_F32) return N % G2_BN == 0 || N >= 2048 || K >= 20000 || static_cast<double>(M) * N * K >= 2e10;
+  const long long one = static_cast<long long>((M + 127) / 128) * (N / 128);
+  const long long two = static_cast<long long>((M + 255) / 256) * ((N + 255) / 256);
+  const int sms = num_sms(), pairs = sms > 1 ? sms / 2 : 1;
+  return 5 * ((two + pairs - 1) / pairs) <= 4 * ((one + sms - 1) / sms);
+}
 extern "C" int aeris_gemm_auto(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
                                int a_mn, int b_mn, int epi, const void* resid, int ldr, const float* gate,
                                int rows_per_gate, int ld_gate, void* aux, int ld_aux, int swiglu_f, int k_splits,
                                int bn, int allow_2cta, int* status, void* stream) {
-  const bool swiglu_fwd = (epi == EPI_SWIGLU || epi == EPI_SWIGLU_BOTH);
-  if (allow_2cta && (N % G2_BN == 0 || (N % (G2_BN / 2) == 0 && N >= 2048 && !swiglu_fwd)))
+  const bool taken = N % (epi == EPI_SWIGLU || epi == EPI_SWIGLU_BOTH ? G2_BN : G2_BN / 2) == 0;
+  if (taken && (allow_2cta == 2 || (allow_2cta && pairs_pay(M, N, K, epi))))
     return gemm_two_cta(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, resid, ldr, gate, rows_per_gate, ld_gate, aux,
                         ld_aux, swiglu_f, k_splits, status, stream);
+  // few tiles: the smaller ones (wide tiles are for SwiGLU, whose columns come in pairs)
+  if (allow_2cta && bn == 0 && (epi == EPI_STORE || epi == EPI_GATE_RESID || epi == EPI_STORE_F32)) bn = 128;
   return gemm_one_cta(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, resid, ldr, gate, rows_per_gate, ld_gate, aux,
                       ld_aux, swiglu_f, k_splits, bn, status, stream);
 }

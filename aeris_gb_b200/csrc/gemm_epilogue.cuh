@@ -139,12 +139,12 @@ __device__ __forceinline__ void push_stage_flush_red(uint8_t* stage, int lane, f
   __syncwarp();
 }
 
-// bf16 output columns of a warp's 32 rows on their way out: two tiles of 64 columns in shared memory, which one lane hands
-// to the TMA unit when they are complete; rows past the matrix are clipped. Written by the warp itself, two 256-byte row
-// segments an instruction behind two shuffles and a read, the stores took longer than the products of short reductions.
-// us, bursts, before / now: 28800 x 1536 x 512 53.3 / 48.1, gated residual 28800 x 512 x 512 30.6 / 26.9, SwiGLU with the raw
-// columns 28800 x 3072 x 512 110.5 / 98.2, 57600 x 4096 x 768 331 / 308, plain 57600 x 2304 x 768 166 / 161, gated 64800 x
-// 1536 x 1536 234 / 228.
+// bf16 output columns of a warp's 32 rows on their way out: two tiles of 64 columns in shared memory, which one lane
+// hands to the TMA unit when they are complete; rows past the matrix are clipped. Written by the warp itself, two
+// 256-byte row segments an instruction behind two shuffles and a read, the stores took longer than the products of short
+// reductions. us, bursts, before / now: 28800 x 1536 x 512 53.3 / 48.1, gated residual 28800 x 512 x 512 30.6 / 26.9,
+// SwiGLU with the raw columns 28800 x 3072 x 512 110.5 / 98.2, 57600 x 4096 x 768 331 / 308, plain 57600 x 2304 x 768 166
+// / 161, gated 64800 x 1536 x 1536 234 / 228.
 struct TileOut {
   uint8_t* stage;        // 8 KB
   int lane;
@@ -195,15 +195,15 @@ __device__ __forceinline__ void swiglu_bwd_pair(uint32_t d0, uint32_t d1, uint32
   ou = f2_to_bf16x2(f2_mul(d, si));
 }
 
-// Operand u = [gate | up] of the SwiGLU backward epilogue on eight warps, 32 rows x 32 gate and 32 up columns a step: tiled
-// loads one step ahead, across tiles (it does not depend on the products), into one of two buffers of the warp; the
+// Operand u = [gate | up] of the SwiGLU backward epilogue on eight warps, 32 rows x 32 gate and 32 up columns a step:
+// tiled loads one step ahead, across tiles (it does not depend on the products), into one of two buffers of the warp; the
 // gradients of a step take the place of its operand and leave from there as tiled stores. That is all the shared memory
-// the epilogue needs, so the ring of operands keeps its five stages. us, bursts, asynchronous 16-byte copies and stores by
-// the warp / now: 28800 x 1536 x 512 101 / 98, 57600 x 2048 x 768 262 / 241, 64800 x 4096 x 1536 787 / 763, 7200 x 512 x 256
-// 16.2 / 14.4. Without the operand ahead its latency is paid four times a tile (28800 x 2048 x 768: 211 us for 168 then). With
-// gradients in tiles of their own, 64 columns wide, and four stages 97, 242 and 792. What is left are the arithmetic (two
-// exponentials and two divisions per element; none of it: 10 % less) and the products' own loads beside 2.3 GB of
-// operand and gradients (no loads and stores: 64800 x 4096 x 1536 595 us, the products alone 519).
+// the epilogue needs, so the ring of operands keeps its five stages. us, bursts, asynchronous 16-byte copies and stores
+// by the warp / now: 28800 x 1536 x 512 101 / 98, 57600 x 2048 x 768 262 / 241, 64800 x 4096 x 1536 787 / 763, 7200 x 512
+// x 256 16.2 / 14.4. Without the operand ahead its latency is paid four times a tile (28800 x 2048 x 768: 211 us for 168
+// then). With gradients in tiles of their own, 64 columns wide, and four stages 97, 242 and 792. What is left are the
+// arithmetic (two exponentials and two divisions per element; none of it: 10 % less) and the products' own loads beside
+// 2.3 GB of operand and gradients (no loads and stores: 64800 x 4096 x 1536 595 us, the products alone 519).
 constexpr int SWIGLU_U_BYTES = 4096;
 
 // Residual of the gated epilogue, requested one step (32 rows x 64 columns, 4 KB per warp) ahead as 128-byte row segments

@@ -34,6 +34,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
     EPI_SWIGLU_BOTH = EPI_SWIGLU that also writes the raw ``[gate | up]`` product to ``aux [M, 2F]``;
     ``k_splits``: slices of the reduction dimension (EPI_ACC_F32 only); 0 lets the kernel choose, -n as well but towards n
     slices, as far as they cost nothing, for sums that used to come as n shorter ones.
+    ``two_cta``: False never, True wherever the two-CTA kernel takes the product, None where it is the faster.
     EPI_SWIGLU_BWD: the product is d(act) ``[M, F]``, ``resid`` holds ``u = [gate | up]`` and ``out`` receives d(u).
     """
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
@@ -61,8 +62,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
         dt = torch.float32 if epi in (EPI_ACC_F32, EPI_STORE_F32) else torch.bfloat16
         out = (torch.zeros if epi == EPI_ACC_F32 else torch.empty)((M, n_out), dtype=dt, device=a.device)
     assert out.shape == (M, n_out) or epi == EPI_SWIGLU_BWD
-    if two_cta is None:
-        two_cta = TWO_CTA_DEFAULT and bn == 0
+    two_cta = (TWO_CTA_DEFAULT and bn == 0) if two_cta is None else 2 if two_cta else 0
     rc = _l.lib().aeris_gemm_auto(
         _l.ptr(a), _l.ptr(b), _l.ptr(out), M, N, K, _ld(a), _ld(b), _ld(out), int(a_t), int(b_t), epi,
         _l.ptr(resid), _ld(resid) if resid is not None else 0, _l.ptr(gate), rows_per_gate, N,

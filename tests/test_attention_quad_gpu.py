@@ -1,6 +1,6 @@
-"""Attention forward, four query tiles at a time: windows of three, four, seven and eight tiles whose last tile, last 64 columns
-and last step of 16 are full, nearly full or nearly empty, groups with an idle chain, one and several items a CTA. The
-output is that of the kernel of one query tile, bit for bit."""
+"""Attention forward, four query tiles at a time: windows of three, four, seven and eight tiles whose last tile, last 64
+columns and last step of 16 are full, nearly full or nearly empty, groups with an idle chain, one and several items a CTA.
+The output is that of the kernel of one query tile, bit for bit."""
 import math
 
 import pytest
@@ -22,8 +22,9 @@ def _quad_ran(fn):
 
 # 96 (window, head) pairs of 3 or 4 tiles and 74 of 7 or 8 are one item a CTA, 296 and 222 several
 @pytest.mark.parametrize("d", [64, 40])
-@pytest.mark.parametrize("nw,N,H", [(3, 257, 32), (3, 272, 32), (3, 320, 32), (3, 321, 32), (3, 383, 32), (3, 384, 32), (3, 385, 32),
-                                    (8, 450, 37), (3, 512, 32), (2, 769, 37), (6, 831, 37), (2, 895, 37), (2, 896, 37),
+@pytest.mark.parametrize("nw,N,H", [(3, 257, 32), (3, 272, 32), (3, 320, 32), (3, 321, 32), (3, 383, 32), (3, 384, 32),
+                                    (3, 385, 32), (8, 450, 37), (3, 512, 32), (2, 769, 37), (6, 831, 37), (2, 895, 37),
+                                    (2, 896, 37),
                                     (6, 900, 37), (2, 1024, 37)])
 @pytest.mark.parametrize("sharp", [False, True])
 def test_equals_the_kernel_of_one_query_tile(nw, N, H, d, sharp):

@@ -1,6 +1,6 @@
-"""Two-CTA GEMM: bf16 outputs leave as tiled stores of 32 rows. Rows that end inside a tile of 32, inside a CTA's and a pair's
-rows, a last column tile that is half empty, outputs that are slices of wider tensors (nothing beside them is written), short
-and long reductions (eight and four epilogue warps), the SwiGLU backward in place."""
+"""Two-CTA GEMM: bf16 outputs leave as tiled stores of 32 rows. Rows that end inside a tile of 32, inside a CTA's and a
+pair's rows, a last column tile that is half empty, outputs that are slices of wider tensors (nothing beside them is written),
+short and long reductions (eight and four epilogue warps), the SwiGLU backward in place."""
 import pytest
 import torch
 
@@ -33,10 +33,10 @@ def test_outputs(M, N, F, K):
     a, b, x, g = r(M, K), r(N, K), r(M, N), torch.randn(1, N, device=DEV)
     c, ok = _wide(M, N)
     ref = a.double() @ b.double().t()
-    G.gemm(a, b, out=c)
+    G.gemm(a, b, out=c, two_cta=True)
     assert rel_err(c, ref) < TOL and ok()
     c, ok = _wide(M, N)
-    G.gemm(a, b, out=c, epi=G.EPI_GATE_RESID, resid=x, gate=g)
+    G.gemm(a, b, out=c, epi=G.EPI_GATE_RESID, resid=x, gate=g, two_cta=True)
     assert rel_err(c, x.double() + g.double() * ref) < TOL and ok()
     # SwiGLU: gate and up rows of the weights, activation and raw columns
     f = F if F % 256 == 0 else 256
@@ -44,16 +44,16 @@ def test_outputs(M, N, F, K):
     u = a.double() @ w.double().t()
     act, ok = _wide(M, f)
     raw, ok2 = _wide(M, 2 * f)
-    G.gemm(a, w, out=act, epi=G.EPI_SWIGLU_BOTH, aux=raw)
+    G.gemm(a, w, out=act, epi=G.EPI_SWIGLU_BOTH, aux=raw, two_cta=True)
     assert rel_err(act, torch.nn.functional.silu(u[:, :f]) * u[:, f:]) < TOL and rel_err(raw, u) < TOL and ok() and ok2()
     act2, ok = _wide(M, f)
-    G.gemm(a, w, out=act2, epi=G.EPI_SWIGLU)
+    G.gemm(a, w, out=act2, epi=G.EPI_SWIGLU, two_cta=True)
     assert torch.equal(act2, act) and ok()
     # its backward: d(act) = a b^T over N columns, operand u and gradient in place
     du, ok = _wide(M, 2 * N)
     uu = r(M, 2 * N)
     du.copy_(uu)
-    G.gemm(a, b.t().contiguous(), b_t=True, out=du, epi=G.EPI_SWIGLU_BWD, resid=du)
+    G.gemm(a, b.t().contiguous(), b_t=True, out=du, epi=G.EPI_SWIGLU_BWD, resid=du, two_cta=True)
     ud = uu.double().requires_grad_(True)
     (torch.nn.functional.silu(ud[:, :N]) * ud[:, N:]).backward(ref)
     assert rel_err(du, ud.grad) < TOL and ok()
