@@ -472,13 +472,14 @@ class OutputStage(nn.Module):
         shift, scale = fused.modulation(self.modulation, dt).chunk(2, dim=1)
         return fused_io.HeadLossFn.apply(x, shift, scale, self.norm.weight, self.head.weight, x_img, cs, plan)
 
-    def predict_tokens(self, x, dt):
-        """Network output in token order, fp32 ``[T, 128]`` (channels past ``out_channels`` are zero); no autograd."""
+    def predict_tokens(self, x, dt, table=None):
+        """Network output in token order, fp32 ``[T, 128]`` (channels past ``out_channels`` are zero); no autograd.
+        ``table``: where the row of each token is in ``x`` (see :func:`.fused_io.head_forward`)."""
         from . import fused, fused_io
         with torch.no_grad():
             shift, scale = fused.modulation(self.modulation, dt).chunk(2, dim=1)
             return fused_io.head_forward(x, shift, scale, self.norm.weight, self.head.weight,
-                                         self.cfg.eps(self.cfg.data_dtype))
+                                         self.cfg.eps(self.cfg.data_dtype), table=table)
 
 
 class _HeadFn(torch.autograd.Function):
@@ -606,6 +607,11 @@ class AerisModel(nn.Module):
         return n_blocks - fused.plan_kept_blocks(meta, x.shape[0] // (wins * L), cfg.dim, cfg.mlp_dim, n_blocks, x.device)
 
     def trunk(self, x: torch.Tensor, dt: torch.Tensor, ctx: StreamContext) -> torch.Tensor:
+        x, layout = self._shifted_trunk(x, dt, ctx)
+        return ctx.regroup_unfused(x, layout, (0, 0))
+
+    def _shifted_trunk(self, x: torch.Tensor, dt: torch.Tensor, ctx: StreamContext) -> tuple[torch.Tensor, tuple[int, int]]:
+        """All layers; the stream is left in the window layout of the last one, which is returned as well."""
         cur = (0, 0)
         n = len(self.layers)
         first_kept = self._first_kept_block(x, ctx)
@@ -615,7 +621,7 @@ class AerisModel(nn.Module):
             x = layer(x, dt, ctx, regroup=(cur, nxt), publish_out=(after != nxt),
                       keep_from=max(0, first_kept - i * self.cfg.sublayers))
             cur = nxt
-        return ctx.regroup_unfused(x, cur, (0, 0))
+        return x, cur
 
     def forward_tokens(self, x_tok: torch.Tensor, t: torch.Tensor, ctx: StreamContext) -> torch.Tensor:
         x, dt = self.input_stage(x_tok, t, ctx)
@@ -632,8 +638,13 @@ class AerisModel(nn.Module):
         """One network evaluation for the sampler: ``x_img`` is the noisy state; returns F in token order [T, 128]."""
         cs = torch.zeros((x_img.shape[0], 2), device=x_img.device)
         cs[:, 0] = 1.0
+        from . import fused
         x, dt = self.input_stage.forward_images(x_img, c_img, cs, t, plan)
-        return self.output_stage.predict_tokens(self.trunk(x, dt, ctx), dt)
+        if ctx.grid.n_ranks > 1 or ctx.peer_fn is not None or fused.recorded() or "trunk" in vars(self):
+            return self.output_stage.predict_tokens(self.trunk(x, dt, ctx), dt)
+        x, layout = self._shifted_trunk(x, dt, ctx)       # the head's norm reads the rows from where they are
+        table = ctx.table(layout, (0, 0), x.device) if layout != (0, 0) else None
+        return self.output_stage.predict_tokens(x, dt, table)
 
     def forward(self, x_img: torch.Tensor, t: torch.Tensor) -> torch.Tensor:
         """x_img: [B, H, W, in_channels] fp32; t: [B]. Returns [B, H, W, out_channels] fp32 (single rank)."""

@@ -123,9 +123,8 @@ class Evaluations:
                 cur = y
             layout = shift
         self.records = (NB.BlockArgs * len(records))(*records)
-        self.last, self.back = self.streams[cur], None
-        if layout != (0, 0):
-            self.back = (ctx.table(layout, (0, 0), dev), self.streams[(cur + 1) % 3])
+        self.last = self.streams[cur]
+        self.back = ctx.table(layout, (0, 0), dev) if layout != (0, 0) else None
 
     def run(self, e: int, x_img: torch.Tensor, slot: int) -> torch.Tensor:
         proj, out, cfg = self.model.input_stage.proj, self.model.output_stage, self.cfg
@@ -135,10 +134,6 @@ class Evaluations:
         if E._CHECKED:
             E.set_gather_bounds(self.last.shape[0])
         NB.issue_forward(self.records, e * 6 * D)
-        x = self.last
-        if self.back is not None:
-            table, x = self.back
-            E.gather_rows(table, [self.last.data_ptr()], x, src_rows=x.shape[0])
         shift, scale = self.head_mod[e].view(2, 1, D).expand(2, M, D).unbind(0)
-        return fused_io.head_forward(x, shift, scale, out.norm.weight, out.head.weight, cfg.eps(cfg.data_dtype),
-                                     packed=self.head_w, pred=self.pred[slot])
+        return fused_io.head_forward(self.last, shift, scale, out.norm.weight, out.head.weight, cfg.eps(cfg.data_dtype),
+                                     packed=self.head_w, pred=self.pred[slot], table=self.back)
