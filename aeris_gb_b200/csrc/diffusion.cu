@@ -51,7 +51,8 @@ __device__ __forceinline__ int geom_rows_per_sample(const TokGeom& g) { return g
 __device__ __forceinline__ Pixel row_to_pixel(const TokGeom& g, long long row) {
   const int rps = geom_rows_per_sample(g);
   Pixel p;
-  p.b = static_cast<int>(row / rps);
+  // a 64-bit quotient takes as long as the rest of the row's addresses
+  p.b = row >> 32 ? static_cast<int>(row / rps) : static_cast<int>(static_cast<uint32_t>(row) / static_cast<uint32_t>(rps));
   const int r = static_cast<int>(row - static_cast<long long>(p.b) * rps);
   const int w = r / g.n_local, tok = r - w * g.n_local;
   const int seq = g.sp_rank * g.n_local + tok;
@@ -70,68 +71,120 @@ __device__ __forceinline__ size_t block_pixel(const TokGeom& g, const Pixel& p) 
 
 constexpr int EMBED_MAX_C = 256;
 constexpr int EMBED_WARPS = 8;
+constexpr int EMBED_LINE = (3 * EMBED_MAX_C + 2 + 7) / 8 * 8;      // columns of a packed row that can be other than zero
 
-// One warp per token row. Output row: [hi(v) | lo(v) | hi(v) | 1 | 1 | 0...] of width KP (bf16), v the fp32 model
-// input cat[x_t / sigma_d, cond] + ape. Multiplied by [hi(W) | hi(W) | lo(W) | hi(b) | lo(b) | 0...] this gives
-// v W^T + b up to the dropped lo*lo term.
-__global__ void __launch_bounds__(EMBED_WARPS * 32)
+// Output row of a token: [hi(v) | lo(v) | hi(v) | 1 | 1 | 0...] of width KP (bf16), v the fp32 model input
+// cat[x_t / sigma_d, cond] + ape. Multiplied by [hi(W) | hi(W) | lo(W) | hi(b) | lo(b) | 0...] this gives v W^T + b up to the
+// dropped lo*lo term. Bound by instructions and their latency, not by its bytes, so:
+//   * A warp takes `chunk` consecutive rows: a lane's addresses move by one pixel, and what has to be divided or multiplied
+//     out is done once per row of a window.
+//   * A lane takes W = 2 channels at a time where all counts are even and all tables start on 8 bytes, else one.
+//   * The row is put together in shared memory, where its constant end stays from row to row, and leaves in 16-byte vectors
+//     (`vec`; two-column words where `out` starts elsewhere): the parts of a channel are computed once.
+// us, 70 + 74 channels, a row at a time with divisions per column / now (40 warps per SM, 48 registers): 64,800 rows 86 / 32,
+// 14,400 22.6 / 9.6, 64,800 with noise 92 / 44; 259,200 rows of 69 + 71 channels 334 / 157. Its bytes take 16, 3.5, 16, 63.
+template <int W, bool NOISE>
+__global__ void __launch_bounds__(EMBED_WARPS * 32, 5)
 embed_pack_kernel(const float* __restrict__ x_img, const float* __restrict__ c_img, const float* __restrict__ cs,
                   TokGeom g, int Cx, int Cc, const float* __restrict__ ape_y, const float* __restrict__ ape_x,
-                  int ape_ch, unsigned long long seed, float sd, int noise, __nv_bfloat16* __restrict__ out, int KP,
-                  long long row0, long long rows) {
+                  int ape_ch, unsigned long long seed, float sd, __nv_bfloat16* __restrict__ out, int KP,
+                  long long row0, long long rows, int chunk, int vec) {
   chain_point();
-  __shared__ float vbuf[EMBED_WARPS][EMBED_MAX_C];
+  constexpr int STEPS = EMBED_MAX_C / (32 * W);
+  __shared__ __align__(16) __nv_bfloat16 lines[EMBED_WARPS][EMBED_LINE];
+  __shared__ __align__(16) float zs[EMBED_WARPS][NOISE ? EMBED_MAX_C : 4];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float* v = vbuf[warp];
+  __nv_bfloat16* line = lines[warp];
+  float* z = zs[warp];
   const int Cin = Cx + Cc;
   const float inv_sd = 1.0f / sd;
-  for (long long i = static_cast<long long>(blockIdx.x) * EMBED_WARPS + warp; i < rows;
-       i += static_cast<long long>(gridDim.x) * EMBED_WARPS) {
-    const Pixel p = row_to_pixel(g, row0 + i);
-    const size_t bp = block_pixel(g, p);
-    const unsigned long long gp = global_pixel(g, p);
-    const float ct = cs[2 * p.b], st = cs[2 * p.b + 1];
-    for (int grp = lane; grp * 4 < Cx; grp += 32) {
-      float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (noise) z = normal4(seed, gp, grp);
-      const float zz[4] = {z.x, z.y, z.z, z.w};
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int c = grp * 4 + k;
-        if (c < Cx) v[c] = (ct * x_img[bp * Cx + c] + st * sd * zz[k]) * inv_sd;
-      }
+  for (int j = lane; j < EMBED_LINE; j += 32) line[j] = __float2bfloat16_rn(j >= 3 * Cin && j < 3 * Cin + 2 ? 1.f : 0.f);
+  const long long first = (static_cast<long long>(blockIdx.x) * EMBED_WARPS + warp) * chunk;
+  const int n = static_cast<int>(rows - first < chunk ? rows - first : chunk);
+  Pixel p{};
+  int tok = g.n_local, ix = 0;          // the first row is looked up
+  float ct = 0.f, st = 0.f;
+  // of the pixel, for channel 0 plus this lane's first: state, conditioning, position encoding of its row and column
+  const float *xp = nullptr, *cp = nullptr, *ay = nullptr, *ax = nullptr;
+  const int ape_c = ape_y ? 2 * ape_ch : 0;
+  for (int k = 0; k < n; ++k) {
+    const bool look_up = tok == g.n_local;
+    if (look_up) {
+      p = row_to_pixel(g, row0 + first + k);
+      tok = static_cast<int>((row0 + first + k) % g.n_local);
+      ix = (g.sp_rank * g.n_local + tok) % g.ws_x;
+      ct = cs[2 * p.b];
+      st = cs[2 * p.b + 1];
     }
-    for (int c = lane; c < Cc; c += 32) v[Cx + c] = c_img[bp * Cc + c];
-    __syncwarp();
-    if (ape_y) {
-      const float* ay = ape_y + static_cast<size_t>(g.y0 + p.y) * ape_ch;
-      const float* ax = ape_x + static_cast<size_t>(g.x0 + p.x) * ape_ch;
-      for (int c = lane; c < Cin; c += 32) {
-        if (c < ape_ch) v[c] += ay[c];
-        else if (c < 2 * ape_ch) v[c] += ax[c - ape_ch];
-      }
-      __syncwarp();
+    if (look_up || ix == 0) {
+      const size_t bp = block_pixel(g, p);
+      xp = x_img + bp * Cx + lane * W;
+      cp = c_img + bp * Cc + lane * W - Cx;
+      ay = ape_y + static_cast<size_t>(g.y0 + p.y) * ape_ch + lane * W;
+      ax = ape_x + static_cast<size_t>(g.x0 + p.x) * ape_ch + lane * W - ape_ch;
     }
-    uint32_t* orow = reinterpret_cast<uint32_t*>(out + static_cast<size_t>(i) * KP);
-    for (int j2 = lane; j2 < KP / 2; j2 += 32) {
-      float o[2];
+    if constexpr (NOISE) {
+      const unsigned long long gp = global_pixel(g, p);
+      for (int grp = lane; grp * 4 < Cx; grp += 32) *reinterpret_cast<float4*>(z + grp * 4) = normal4(seed, gp, grp);
+    }
+    __syncwarp();                       // the row before has left, this one's noise is there
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int j = 2 * j2 + h;
-        float val = 0.f;
-        if (j < 3 * Cin) {
-          const int sec = j / Cin, c = j - sec * Cin;
-          const float f = v[c];
-          const float hi = __bfloat162float(__float2bfloat16_rn(f));
-          val = (sec == 1) ? (f - hi) : hi;
-        } else if (j < 3 * Cin + 2) {
-          val = 1.0f;
+    for (int i = 0; i < STEPS; ++i) {
+      const int c = (lane + 32 * i) * W;
+      if (c >= Cin) break;
+      float f[W], a[W];
+      auto load = [&](const float* at, float (&t)[W]) {
+        if constexpr (W == 2) {
+          const float2 u = *reinterpret_cast<const float2*>(at + 64 * i);
+          t[0] = u.x;
+          t[1] = u.y;
+        } else {
+          t[0] = at[32 * i];
         }
-        o[h] = val;
+      };
+      load(c < Cx ? xp : cp, f);
+      if (c < ape_c) load(c < ape_ch ? ay : ax, a);
+      if (c < Cx) {
+#pragma unroll
+        for (int h = 0; h < W; ++h) f[h] = NOISE ? (ct * f[h] + st * sd * z[c + h]) * inv_sd : ct * f[h] * inv_sd;
       }
-      orow[j2] = pack_bf16x2(o[0], o[1]);
+      if (c < ape_c) {
+#pragma unroll
+        for (int h = 0; h < W; ++h) f[h] = __fadd_rn(f[h], a[h]);     // never one rounding with the product before it
+      }
+      if constexpr (W == 2) {
+        const uint32_t hi = pack_bf16x2(f[0], f[1]);
+        const float2 h = unpack_bf16x2(hi);
+        *reinterpret_cast<uint32_t*>(line + c) = hi;
+        *reinterpret_cast<uint32_t*>(line + Cin + c) = pack_bf16x2(f[0] - h.x, f[1] - h.y);
+        *reinterpret_cast<uint32_t*>(line + 2 * Cin + c) = hi;
+      } else {
+        const __nv_bfloat16 hi = __float2bfloat16_rn(f[0]);
+        line[c] = hi;
+        line[Cin + c] = __float2bfloat16_rn(f[0] - __bfloat162float(hi));
+        line[2 * Cin + c] = hi;
+      }
     }
     __syncwarp();
+    __nv_bfloat16* orow = out + static_cast<size_t>(first + k) * KP;
+    if (vec) {
+      for (int j = lane; j < KP / 8; j += 32)
+        reinterpret_cast<uint4*>(orow)[j] =
+            j < EMBED_LINE / 8 ? reinterpret_cast<const uint4*>(line)[j] : make_uint4(0u, 0u, 0u, 0u);
+    } else {
+      for (int j = lane; j < KP / 2; j += 32)
+        reinterpret_cast<uint32_t*>(orow)[j] = j < EMBED_LINE / 2 ? reinterpret_cast<const uint32_t*>(line)[j] : 0u;
+    }
+    ++tok;
+    ++p.x;
+    xp += Cx;
+    cp += Cc;
+    ax += ape_ch;
+    if (++ix == g.ws_x) {
+      ix = 0;
+      p.x -= g.ws_x;
+      ++p.y;
+    }
   }
 }
 
@@ -273,9 +326,18 @@ extern "C" int aeris_embed_pack(const float* x_img, const float* c_img, const fl
   if (!geom_ok(g) || Cx <= 0 || Cc < 0 || Cx + Cc > EMBED_MAX_C || KP % 8 || KP < 3 * (Cx + Cc) + 2 || rows <= 0)
     return -1;
   if (row0 < 0 || row0 + rows > static_cast<long long>(g->B) * g->nwy_loc * g->nwx_loc * g->n_local) return -2;
-  return launch_chained(embed_pack_kernel, warp_grid(rows, EMBED_WARPS), EMBED_WARPS * 32, 0,
-                        reinterpret_cast<cudaStream_t>(stream), x_img, c_img, cs, *g, Cx, Cc, ape_y, ape_x, ape_ch, seed, sd,
-                        noise, reinterpret_cast<__nv_bfloat16*>(out), KP, row0, rows);
+  // 40 warps per SM, of consecutive rows each; two channels a lane where pairs of them are whole 8-byte words
+  const long long warps = static_cast<long long>(aeris_num_sms()) * 40;
+  const long long chunk = (rows + warps - 1) / warps, ctas = ((rows + chunk - 1) / chunk + EMBED_WARPS - 1) / EMBED_WARPS;
+  if (chunk > 0x7fffffff) return -1;
+  const uintptr_t at = reinterpret_cast<uintptr_t>(x_img) | reinterpret_cast<uintptr_t>(c_img) |
+                       reinterpret_cast<uintptr_t>(ape_y) | reinterpret_cast<uintptr_t>(ape_x);
+  const bool two = (Cx | Cc | ape_ch) % 2 == 0 && at % 8 == 0;
+  auto kern = noise ? (two ? embed_pack_kernel<2, true> : embed_pack_kernel<1, true>)
+                    : (two ? embed_pack_kernel<2, false> : embed_pack_kernel<1, false>);
+  return launch_chained(kern, static_cast<unsigned>(ctas), EMBED_WARPS * 32, 0, reinterpret_cast<cudaStream_t>(stream), x_img,
+                        c_img, cs, *g, Cx, Cc, ape_y, ape_x, ape_ch, seed, sd, reinterpret_cast<__nv_bfloat16*>(out), KP,
+                        row0, rows, static_cast<int>(chunk), (reinterpret_cast<uintptr_t>(out) & 15) == 0);
 }
 
 extern "C" int aeris_trigflow_loss(const float* pred, int ldp, const float* x_img, const float* cs, const TokGeom* g,
