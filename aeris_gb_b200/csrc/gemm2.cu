@@ -586,12 +586,16 @@ static bool pairs_pay(int M, int N, int K, int epi) {
   const int sms = num_sms(), pairs = sms > 1 ? sms / 2 : 1;
   return 5 * ((two + pairs - 1) / pairs) <= 4 * ((one + sms - 1) / sms);
 }
+extern "C" int aeris_gemm_takes_pairs(int M, int N, int K, int epi, int allow_2cta) {
+  const bool taken = N % (epi == EPI_SWIGLU || epi == EPI_SWIGLU_BOTH ? G2_BN : G2_BN / 2) == 0;
+  return taken && (allow_2cta == 2 || (allow_2cta && pairs_pay(M, N, K, epi)));
+}
+
 extern "C" int aeris_gemm_auto(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
                                int a_mn, int b_mn, int epi, const void* resid, int ldr, const float* gate,
                                int rows_per_gate, int ld_gate, void* aux, int ld_aux, int swiglu_f, int k_splits,
                                int bn, int allow_2cta, int* status, void* stream) {
-  const bool taken = N % (epi == EPI_SWIGLU || epi == EPI_SWIGLU_BOTH ? G2_BN : G2_BN / 2) == 0;
-  if (taken && (allow_2cta == 2 || (allow_2cta && pairs_pay(M, N, K, epi))))
+  if (allow_2cta && aeris_gemm_takes_pairs(M, N, K, epi, allow_2cta))
     return gemm_two_cta(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, resid, ldr, gate, rows_per_gate, ld_gate, aux,
                         ld_aux, swiglu_f, k_splits, status, stream);
   // few tiles: the smaller ones (wide tiles are for SwiGLU, whose columns come in pairs)
