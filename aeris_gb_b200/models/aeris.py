@@ -640,7 +640,8 @@ class AerisModel(nn.Module):
         cs[:, 0] = 1.0
         from . import fused
         x, dt = self.input_stage.forward_images(x_img, c_img, cs, t, plan)
-        if ctx.grid.n_ranks > 1 or ctx.peer_fn is not None or fused.recorded() or "trunk" in vars(self):
+        stock = getattr(self.trunk, "__func__", None) is AerisModel.trunk and type(self.output_stage) is OutputStage
+        if not stock or ctx.grid.n_ranks > 1 or ctx.peer_fn is not None or fused.recorded():
             return self.output_stage.predict_tokens(self.trunk(x, dt, ctx), dt)
         x, layout = self._shifted_trunk(x, dt, ctx)       # the head's norm reads the rows from where they are
         table = ctx.table(layout, (0, 0), x.device) if layout != (0, 0) else None
