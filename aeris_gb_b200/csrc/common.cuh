@@ -226,6 +226,7 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, const void* s
 // Kernels that wait for other GPUs are launched without it. us per launch, back to back, plain / chained: two-CTA product
 // 256 x 256 x 256 10.3 / 7.6, 14400 x 768 x 768 21.1 / 18.5; a sampler step of seven evaluations of two blocks of width 256
 // on 14,400 tokens (155 launches) 2.24 / 1.95 ms. Chained products and attention alone: 2.06.
+// The modulation vectors' small products and the loss too: training steps of 209 and 217 launches 3.85 / 3.82, 2.90 / 2.89.
 __device__ __forceinline__ void chain_point() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -76,6 +76,7 @@ template <typename WT, int MB>
 __global__ void __launch_bounds__(256)
 gemv_bias_act_kernel(const WT* __restrict__ W, const void* __restrict__ bias, int bias_bf16, const void* __restrict__ x,
                      int x_bf16, float* __restrict__ y, int N, int K, int B, int act, int silu_in, int vec) {
+  chain_point();
   extern __shared__ __align__(16) float xs[];  // [MB, Kp], rows padded to a multiple of four floats
   const int Kp = (K + 3) & ~3;
   for (int b = 0; b < MB; ++b)
@@ -146,6 +147,7 @@ __global__ void __launch_bounds__(256)
 gemv_bwd_kernel(const WT* __restrict__ W, const void* __restrict__ x, int x_bf16, const float* __restrict__ dy,
                 float* __restrict__ dW, float* __restrict__ db, float* __restrict__ dx, int N, int K, int B, int silu_in,
                 int rows) {
+  chain_point();
   __shared__ float s_dy[GEMV_BWD_ROWS][MB];
   const int n0 = blockIdx.y * rows, nr = min(rows, N - n0);
   for (int i = threadIdx.x; i < nr * MB; i += blockDim.x) {
@@ -310,8 +312,8 @@ extern "C" int aeris_gemv_bias_act(const void* W, int flags, const void* bias, c
     if (smem > 48 * 1024 &&                                                                                             \
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMV_X_BYTES) != cudaSuccess)           \
       return -20;                                                                                                       \
-    kern<<<grid, 256, smem, st>>>(reinterpret_cast<const WT*>(W), bias, (flags >> 1) & 1, x, (flags >> 2) & 1, y, N, K, \
-                                  B, act, silu_in, vec);                                                                \
+    return launch_chained(kern, grid, 256, smem, st, reinterpret_cast<const WT*>(W), bias, (flags >> 1) & 1, x,         \
+                          (flags >> 2) & 1, y, N, K, B, act, silu_in, vec);                                             \
   } while (0)
 #define AERIS_GEMV_MB(WT) \
   do { if (mb == 1) AERIS_GEMV(WT, 1); else if (mb == 2) AERIS_GEMV(WT, 2); \
@@ -319,7 +321,6 @@ extern "C" int aeris_gemv_bias_act(const void* W, int flags, const void* bias, c
   if (flags & 1) AERIS_GEMV_MB(float); else AERIS_GEMV_MB(__nv_bfloat16);
 #undef AERIS_GEMV_MB
 #undef AERIS_GEMV
-  return launched();
 }
 
 // The modulation MLP: y1 = x W1^T + b1 [B, N1], y2 = silu(y1) W2^T + b2 [B, N2]. Flags as above, for each layer.
@@ -346,15 +347,14 @@ extern "C" int aeris_gemv_bwd(const void* W, int flags, const void* x, const flo
   const int mb = B <= 1 ? 1 : B <= 2 ? 2 : B <= 4 ? 4 : 8;
   const cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 #define AERIS_GEMV(WT, MB) \
-  gemv_bwd_kernel<WT, MB><<<grid, nt, 0, st>>>(reinterpret_cast<const WT*>(W), x, (flags >> 2) & 1, dy, dW, db, dx, N, K, \
-                                               B, silu_in, rows)
+  return launch_chained(gemv_bwd_kernel<WT, MB>, grid, nt, 0, st, reinterpret_cast<const WT*>(W), x, (flags >> 2) & 1, dy, dW, \
+                        db, dx, N, K, B, silu_in, rows)
 #define AERIS_GEMV_MB(WT) \
   do { if (mb == 1) AERIS_GEMV(WT, 1); else if (mb == 2) AERIS_GEMV(WT, 2); \
        else if (mb == 4) AERIS_GEMV(WT, 4); else AERIS_GEMV(WT, 8); } while (0)
   if (flags & 1) AERIS_GEMV_MB(float); else AERIS_GEMV_MB(__nv_bfloat16);
 #undef AERIS_GEMV_MB
 #undef AERIS_GEMV
-  return launched();
 }
 
 // Gradients of aeris_modulation_mlp, added to dW1, db1, dW2 and db2; dy1 [B, N1] (scratch) and dx [B, K] (may be null) are

@@ -197,6 +197,7 @@ trigflow_loss_kernel(const float* __restrict__ pred, int ldp, const float* __res
                      const float* __restrict__ w_var, const float* __restrict__ w_lat, float inv_rows, float gscale,
                      __nv_bfloat16* __restrict__ dpred, int ldd, double* __restrict__ loss, long long row0,
                      long long rows) {
+  chain_point();
   __shared__ float part[EMBED_WARPS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float acc = 0.f;
@@ -346,10 +347,9 @@ extern "C" int aeris_trigflow_loss(const float* pred, int ldp, const float* x_im
                                    long long rows, void* stream) {
   if (!geom_ok(g) || Cx <= 0 || Cx > ldp || ldd % 4 || (dpred && Cx > ldd) || rows <= 0) return -1;
   if (row0 < 0 || row0 + rows > static_cast<long long>(g->B) * g->nwy_loc * g->nwx_loc * g->n_local) return -2;
-  trigflow_loss_kernel<<<warp_grid(rows, EMBED_WARPS), EMBED_WARPS * 32, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      pred, ldp, x_img, cs, *g, Cx, seed, sd, w_var, w_lat, inv_rows, gscale, reinterpret_cast<__nv_bfloat16*>(dpred),
-      ldd, loss, row0, rows);
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  return launch_chained(trigflow_loss_kernel, warp_grid(rows, EMBED_WARPS), EMBED_WARPS * 32, 0,
+                        reinterpret_cast<cudaStream_t>(stream), pred, ldp, x_img, cs, *g, Cx, seed, sd, w_var, w_lat, inv_rows,
+                        gscale, reinterpret_cast<__nv_bfloat16*>(dpred), ldd, loss, row0, rows);
 }
 
 extern "C" int aeris_sampler_update(float* x_out, const float* x_base, const float* pa, const float* pb, int ldp,
