@@ -18,8 +18,8 @@ int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M, int N, in
                          void* stream);
 
 // The one of the two that is the faster for the shape (see gemm2.cu). bn: tile width of the one-CTA kernel (0: from N);
-// allow_2cta = 0: never the other, 2: the other wherever it takes the product. ld_gate: elements from one gate row to the next (a multiple of 4; N where they lie
-// without gaps).
+// allow_2cta = 0: never the other, 2: the other wherever it takes the product. ld_gate: elements from one gate row to the
+// next (a multiple of 4; N where they lie without gaps).
 int aeris_gemm_auto(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int a_mn,
                     int b_mn, int epi, const void* resid, int ldr, const float* gate, int rows_per_gate, int ld_gate,
                     void* aux, int ld_aux, int swiglu_f, int k_splits, int bn, int allow_2cta, int* status, void* stream);

@@ -347,8 +347,8 @@ extern "C" int aeris_gemv_bwd(const void* W, int flags, const void* x, const flo
   const int mb = B <= 1 ? 1 : B <= 2 ? 2 : B <= 4 ? 4 : 8;
   const cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 #define AERIS_GEMV(WT, MB) \
-  return launch_chained(gemv_bwd_kernel<WT, MB>, grid, nt, 0, st, reinterpret_cast<const WT*>(W), x, (flags >> 2) & 1, dy, dW, \
-                        db, dx, N, K, B, silu_in, rows)
+  return launch_chained(gemv_bwd_kernel<WT, MB>, grid, nt, 0, st, reinterpret_cast<const WT*>(W), x, (flags >> 2) & 1, \
+                        dy, dW, db, dx, N, K, B, silu_in, rows)
 #define AERIS_GEMV_MB(WT) \
   do { if (mb == 1) AERIS_GEMV(WT, 1); else if (mb == 2) AERIS_GEMV(WT, 2); \
        else if (mb == 4) AERIS_GEMV(WT, 4); else AERIS_GEMV(WT, 8); } while (0)

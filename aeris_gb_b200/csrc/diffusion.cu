@@ -74,15 +74,16 @@ constexpr int EMBED_WARPS = 8;
 constexpr int EMBED_LINE = (3 * EMBED_MAX_C + 2 + 7) / 8 * 8;      // columns of a packed row that can be other than zero
 
 // Output row of a token: [hi(v) | lo(v) | hi(v) | 1 | 1 | 0...] of width KP (bf16), v the fp32 model input
-// cat[x_t / sigma_d, cond] + ape. Multiplied by [hi(W) | hi(W) | lo(W) | hi(b) | lo(b) | 0...] this gives v W^T + b up to the
-// dropped lo*lo term. Bound by instructions and their latency, not by its bytes, so:
+// cat[x_t / sigma_d, cond] + ape. Multiplied by [hi(W) | hi(W) | lo(W) | hi(b) | lo(b) | 0...] this gives v W^T + b up to
+// the dropped lo*lo term. Bound by instructions and their latency, not by its bytes, so:
 //   * A warp takes `chunk` consecutive rows: a lane's addresses move by one pixel, and what has to be divided or multiplied
 //     out is done once per row of a window.
 //   * A lane takes W = 2 channels at a time where all counts are even and all tables start on 8 bytes, else one.
 //   * The row is put together in shared memory, where its constant end stays from row to row, and leaves in 16-byte vectors
 //     (`vec`; two-column words where `out` starts elsewhere): the parts of a channel are computed once.
-// us, 70 + 74 channels, a row at a time with divisions per column / now (40 warps per SM, 48 registers): 64,800 rows 86 / 32,
-// 14,400 22.6 / 9.6, 64,800 with noise 92 / 44; 259,200 rows of 69 + 71 channels 334 / 157. Its bytes take 16, 3.5, 16, 63.
+// us, 70 + 74 channels, a row at a time with divisions per column / now (40 warps per SM, 48 registers): 64,800 rows
+// 86 / 32, 14,400 22.6 / 9.6, 64,800 with noise 92 / 44; 259,200 rows of 69 + 71 channels 334 / 157.
+// Its bytes take 16, 3.5, 16 and 63.
 template <int W, bool NOISE>
 __global__ void __launch_bounds__(EMBED_WARPS * 32, 5)
 embed_pack_kernel(const float* __restrict__ x_img, const float* __restrict__ c_img, const float* __restrict__ cs,
@@ -336,9 +337,9 @@ extern "C" int aeris_embed_pack(const float* x_img, const float* c_img, const fl
   const bool two = (Cx | Cc | ape_ch) % 2 == 0 && at % 8 == 0;
   auto kern = noise ? (two ? embed_pack_kernel<2, true> : embed_pack_kernel<1, true>)
                     : (two ? embed_pack_kernel<2, false> : embed_pack_kernel<1, false>);
-  return launch_chained(kern, static_cast<unsigned>(ctas), EMBED_WARPS * 32, 0, reinterpret_cast<cudaStream_t>(stream), x_img,
-                        c_img, cs, *g, Cx, Cc, ape_y, ape_x, ape_ch, seed, sd, reinterpret_cast<__nv_bfloat16*>(out), KP,
-                        row0, rows, static_cast<int>(chunk), (reinterpret_cast<uintptr_t>(out) & 15) == 0);
+  return launch_chained(kern, static_cast<unsigned>(ctas), EMBED_WARPS * 32, 0, reinterpret_cast<cudaStream_t>(stream),
+                        x_img, c_img, cs, *g, Cx, Cc, ape_y, ape_x, ape_ch, seed, sd, reinterpret_cast<__nv_bfloat16*>(out),
+                        KP, row0, rows, static_cast<int>(chunk), (reinterpret_cast<uintptr_t>(out) & 15) == 0);
 }
 
 extern "C" int aeris_trigflow_loss(const float* pred, int ldp, const float* x_img, const float* cs, const TokGeom* g,
@@ -348,8 +349,8 @@ extern "C" int aeris_trigflow_loss(const float* pred, int ldp, const float* x_im
   if (!geom_ok(g) || Cx <= 0 || Cx > ldp || ldd % 4 || (dpred && Cx > ldd) || rows <= 0) return -1;
   if (row0 < 0 || row0 + rows > static_cast<long long>(g->B) * g->nwy_loc * g->nwx_loc * g->n_local) return -2;
   return launch_chained(trigflow_loss_kernel, warp_grid(rows, EMBED_WARPS), EMBED_WARPS * 32, 0,
-                        reinterpret_cast<cudaStream_t>(stream), pred, ldp, x_img, cs, *g, Cx, seed, sd, w_var, w_lat, inv_rows,
-                        gscale, reinterpret_cast<__nv_bfloat16*>(dpred), ldd, loss, row0, rows);
+                        reinterpret_cast<cudaStream_t>(stream), pred, ldp, x_img, cs, *g, Cx, seed, sd, w_var, w_lat,
+                        inv_rows, gscale, reinterpret_cast<__nv_bfloat16*>(dpred), ldd, loss, row0, rows);
 }
 
 extern "C" int aeris_sampler_update(float* x_out, const float* x_base, const float* pa, const float* pb, int ldp,

@@ -567,8 +567,8 @@ extern "C" int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M
 // or single CTAs on tiles of 128 x 128 (256 wide where `bn` is 0 and N allows it). us, bursts, one CTA / pairs:
 //   * plain and gated stores: a wave of pairs takes 1.2 to 1.4 times as long as one of single CTAs, so the numbers of waves
 //     decide. 12150 x 384 x 1152 13.1 / 16.7 (2 and 2 waves), 4096 x 1152 x 3456 28.6 / 39.1 (2, 2), 28800 x 384 x 384
-//     26.2 / 21.8 (5, 4), 12150 x 1152 x 1152 51.0 / 50.5 (6, 4), 12150 x 640 x 640 22.6 / 16.4 (4, 2), 4096 x 1664 x 4992 60.9 /
-//     63.0 (3, 2), 28800 x 896 x 896 87.5 / 59.0 (11, 7); one wave of either: 3600 x 512 x 512 5.6 / 8.8.
+//     26.2 / 21.8 (5, 4), 12150 x 1152 x 1152 51.0 / 50.5 (6, 4), 12150 x 640 x 640 22.6 / 16.4 (4, 2), 4096 x 1664 x 4992
+//     60.9 / 63.0 (3, 2), 28800 x 896 x 896 87.5 / 59.0 (11, 7); one wave of either: 3600 x 512 x 512 5.6 / 8.8.
 //   * SwiGLU backward: only the pairs' kernel requests its second operand ahead. 4096 x 384 x 128 9.8 / 9.8, 12150 x 896 x
 //     384 44.1 / 28.3, 64800 x 3456 x 1664 1179 / 669.
 //   * SwiGLU forward without the raw columns: its tiles halve on the way out, and short sums leave the epilogue as the
