@@ -26,8 +26,8 @@ def test_products(M, N, K, plain, swiglu, bwd, wgrad):
     r = lambda *s: torch.randn(*s, device=DEV).bfloat16()
     a, b, x, g = r(M, K), r(N, K), r(M, N), torch.randn(1, N, device=DEV)
     bt = b.t().contiguous()
-    for epi, path in ((G.EPI_STORE, plain), (G.EPI_GATE_RESID, plain), (G.EPI_SWIGLU, swiglu), (G.EPI_SWIGLU_BWD, bwd),
-                      (G.EPI_ACC_F32, wgrad)):
+    for epi, path in ((G.EPI_STORE, plain), (G.EPI_STORE_F32, plain), (G.EPI_GATE_RESID, plain), (G.EPI_SWIGLU, swiglu),
+                      (G.EPI_SWIGLU_BWD, bwd), (G.EPI_ACC_F32, wgrad)):
         if path:
             assert lib().aeris_gemm_takes_pairs(M, N, K, epi, 1) == (path == "pairs")
             assert lib().aeris_gemm_takes_pairs(M, N, K, epi, 2) and not lib().aeris_gemm_takes_pairs(M, N, K, epi, 0)
@@ -40,6 +40,8 @@ def test_products(M, N, K, plain, swiglu, bwd, wgrad):
             assert rel_err(out, want) < tol
         check(G.gemm(a, b, out=c, **kw), ref)
         check(G.gemm(a, bt, b_t=True, out=c, **kw), ref)
+        # fp32 sums of K products of bf16 values, exact each
+        check(G.gemm(a, b, epi=G.EPI_STORE_F32, **kw), ref, 2.0 ** -23 * K ** 0.5 * 4)
         check(G.gemm(a, b, out=c, epi=G.EPI_GATE_RESID, resid=x, gate=g, **kw), x.double() + g.double() * ref)
         u, du = r(M, 2 * N), torch.empty(M, 2 * N, device=DEV, dtype=torch.bfloat16)
         ud = u.double().requires_grad_(True)
@@ -48,7 +50,7 @@ def test_products(M, N, K, plain, swiglu, bwd, wgrad):
         if swiglu:
             act = torch.empty(M, N // 2, device=DEV, dtype=torch.bfloat16)
             check(G.gemm(a, b, out=act, epi=G.EPI_SWIGLU, **kw), torch.nn.functional.silu(ref[:, :N // 2]) * ref[:, N // 2:])
-        # [M, N] += [K, M]^T [K, N]: fp32 sums of K products of bf16 values, exact each
+        # [M, N] += [K, M]^T [K, N]
         at, w = a.t().contiguous() if M % 8 == 0 else None, torch.zeros(M, N, device=DEV)
         if at is not None:
             check(G.gemm(at, bt, a_t=True, b_t=True, out=w, epi=G.EPI_ACC_F32, k_splits=0, **kw), ref,
