@@ -571,6 +571,8 @@ extern "C" int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M
 //     60.9 / 63.0 (3, 2), 28800 x 896 x 896 87.5 / 59.0 (11, 7); one wave of either: 3600 x 512 x 512 5.6 / 8.8.
 //   * SwiGLU backward: only the pairs' kernel requests its second operand ahead. 4096 x 384 x 128 9.8 / 9.8, 12150 x 896 x
 //     384 44.1 / 28.3, 64800 x 3456 x 1664 1179 / 669.
+//   * SwiGLU forward that also stores the raw columns: the pairs' tiled stores. 4096 x 1024 x 256 7.9 / 8.2, 12150 x 1792 x
+//     384 38.6 / 26.0, 57600 x 4096 x 768 469 / 321; only at the very smallest one CTA, 4096 x 512 x 128 5.4 / 7.3.
 //   * SwiGLU forward without the raw columns: its tiles halve on the way out, and short sums leave the epilogue as the
 //     bound, which every CTA of its own overlaps better. 14400 x 1024 x 256 13.8 / 17.2, 64800 x 1024 x 384 59 / 67,
 //     28800 x 3072 x 384 76.6 / 83.6; held for 0.25 s 64800 x 2048 x 384 120 / 126, x 2048 x 512 146 / 144.
