@@ -231,8 +231,10 @@ __device__ __forceinline__ void chain_point() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// The result is the launch's only trace: it has taken the error from the runtime.
 template <typename... P, typename... A>
-static inline int launch_chained(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, A&&... args) {
+[[nodiscard]] static inline int launch_chained(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream,
+                                               A&&... args) {
   cudaLaunchAttribute attr = {};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;

@@ -1232,14 +1232,13 @@ static int launch_modnorm_bwd_group(const void* x, const void* dh, const void* d
   if (smem > 32 * 1024 &&
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess)
     return -20;
-  launch_chained(kern, grid, groups * nt, smem, reinterpret_cast<cudaStream_t>(stream),
-                 reinterpret_cast<const __nv_bfloat16*>(x),
-                 reinterpret_cast<const std::conditional_t<F32, float, __nv_bfloat16>*>(dh),
-                 reinterpret_cast<const __nv_bfloat16*>(dres), scale, shift, reinterpret_cast<const __nv_bfloat16*>(w),
-                 reinterpret_cast<__nv_bfloat16*>(dx), F32 ? sums : dscale, dshift, dw, rows, D, mode, eps, w_f32, nt, vec);
-  if constexpr (F32)
-    column_sums_kernel<<<(3 * D + 31) / 32, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(sums, grid, D, dscale, dshift,
-                                                                                              dw);
+  const int rc = launch_chained(
+      kern, grid, groups * nt, smem, reinterpret_cast<cudaStream_t>(stream), reinterpret_cast<const __nv_bfloat16*>(x),
+      reinterpret_cast<const std::conditional_t<F32, float, __nv_bfloat16>*>(dh),
+      reinterpret_cast<const __nv_bfloat16*>(dres), scale, shift, reinterpret_cast<const __nv_bfloat16*>(w),
+      reinterpret_cast<__nv_bfloat16*>(dx), F32 ? sums : dscale, dshift, dw, rows, D, mode, eps, w_f32, nt, vec);
+  if (rc || !F32) return rc;       // the sums of a kernel that did not start are not added
+  column_sums_kernel<<<(3 * D + 31) / 32, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(sums, grid, D, dscale, dshift, dw);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
