@@ -15,6 +15,7 @@ hand-written sm_100a kernels (:mod:`.fused`); on CPU they run the PyTorch oracle
 """
 from __future__ import annotations
 
+import inspect
 import math
 import os
 from dataclasses import dataclass, field
@@ -640,8 +641,9 @@ class AerisModel(nn.Module):
         cs[:, 0] = 1.0
         from . import fused
         x, dt = self.input_stage.forward_images(x_img, c_img, cs, t, plan)
-        stock = getattr(self.trunk, "__func__", None) is AerisModel.trunk and type(self.output_stage) is OutputStage
-        if not stock or ctx.grid.n_ranks > 1 or ctx.peer_fn is not None or fused.recorded():
+        if (replaced(self, AerisModel, "trunk", "_shifted_trunk") or replaced(self.output_stage, OutputStage, "predict_tokens")
+                or replaced(ctx, StreamContext, "regroup_unfused", "table")
+                or ctx.grid.n_ranks > 1 or ctx.peer_fn is not None or fused.recorded()):
             return self.output_stage.predict_tokens(self.trunk(x, dt, ctx), dt)
         x, layout = self._shifted_trunk(x, dt, ctx)       # the head's norm reads the rows from where they are
         table = ctx.table(layout, (0, 0), x.device) if layout != (0, 0) else None
@@ -654,6 +656,22 @@ class AerisModel(nn.Module):
         tok = LY.image_to_tokens(x_img, ctx.grid, (0, 0), 0)
         out = self.forward_tokens(tok, t, ctx)
         return LY.tokens_to_image([out], ctx.grid, (0, 0), B)
+
+
+# methods as they are defined here
+_STOCK = {kind: {k: f for k, f in vars(kind).items() if inspect.isfunction(f)}
+          for kind in (AerisModel, InputStage, OutputStage, SwinLayer, StreamContext)}
+
+
+def replaced(part, kind, *names: str) -> bool:
+    """Whether ``part`` does not have ``kind``'s own methods ``names``, whoever put others in their place (the instance, a
+    subclass, a patched class); without names: is of another class or has one method that is not ``kind``'s. A shortcut past
+    a part's methods is for parts that have them."""
+    def own(k: str) -> bool:
+        m = getattr(part, k, None)
+        return getattr(m, "__func__", None) is stock[k] and m.__self__ is part
+    stock = _STOCK[kind]
+    return (not names and type(part) is not kind) or not all(own(k) for k in names or stock)
 
 
 # ---------------------------------------------------------------------------------------------------- stage factory

@@ -26,11 +26,6 @@ class _Refused(Exception):
     """A block that the native call does not take."""
 
 
-def _replaced(module, kind) -> bool:
-    """Whether ``module`` is another class than ``kind`` or carries a method of its own in place of one of ``kind``'s."""
-    return type(module) is not kind or any(k in kind.__dict__ for k in vars(module))
-
-
 def _hooked(modules) -> bool:
     """Whether a forward hook would miss a call of one of ``modules`` (where PyTorch does not say: yes)."""
     return bool(getattr(_module, "_global_forward_hooks", True) or getattr(_module, "_global_forward_pre_hooks", True)
@@ -48,8 +43,9 @@ class Evaluations:
         where all buffers at once do not fit."""
         from . import aeris as A
         cfg, grid, M, D = model.cfg, ctx.grid, plan.geom.B, model.cfg.dim
-        if (not levels or not len(model.layers) or _replaced(model, A.AerisModel) or _replaced(model.input_stage, A.InputStage)
-                or _replaced(model.output_stage, A.OutputStage) or any(_replaced(l, A.SwinLayer) for l in model.layers)
+        if (not levels or not len(model.layers) or A.replaced(model, A.AerisModel)
+                or A.replaced(model.input_stage, A.InputStage) or A.replaced(model.output_stage, A.OutputStage)
+                or any(A.replaced(l, A.SwinLayer) for l in model.layers) or A.replaced(ctx, A.StreamContext)
                 or _hooked(model.layers)
                 or grid.n_ranks != 1 or ctx.peer_fn is not None or cfg.tp != 1 or ctx.batch != M
                 or not (cfg.diffusion and cfg.conditioned and cfg.layerwise_t_emb) or cfg.model_dtype != torch.bfloat16
