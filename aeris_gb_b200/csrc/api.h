@@ -24,8 +24,10 @@ int aeris_gemm_auto(const void* A, const void* B, void* C, int M, int N, int K, 
                     int b_mn, int epi, const void* resid, int ldr, const float* gate, int rows_per_gate, int ld_gate,
                     void* aux, int ld_aux, int swiglu_f, int k_splits, int bn, int allow_2cta, int* status, void* stream);
 
-// 1 where aeris_gemm_auto takes the two-CTA kernel, else 0.
+// 1 where aeris_gemm_auto takes the two-CTA kernel, else 0; the second for weight gradients that ask for slices
+// (k_splits < 0) on a device of `sms` multiprocessors.
 int aeris_gemm_takes_pairs(int M, int N, int K, int epi, int allow_2cta);
+int aeris_wgrad_takes_pairs(int M, int N, int K, int k_splits, int sms);
 
 int aeris_attn_fwd(const void* q, int ldq, int q_col0, const void* k, int ldk, int k_col0, const void* v, int ldv,
                    int v_col0, void* o, int ldo, float* lse, int n_win, int N, int H, int head_dim, float scale,

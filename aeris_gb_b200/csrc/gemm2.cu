@@ -588,6 +588,24 @@ static bool pairs_pay(int M, int N, int K, int epi) {
   const int sms = num_sms(), pairs = sms > 1 ? sms / 2 : 1;
   return 5 * ((two + pairs - 1) / pairs) <= 4 * ((one + sms - 1) / sms);
 }
+// A weight gradient that asks for slices (k_splits < 0) gets them from either kernel only as far as they are free, and a
+// quarter of the tiles leaves less room for free ones: of 60 asked for at 1152 x 384 x 53550 single CTAs make 27 of 1,984
+// rows, pairs 7 of 7,680; of 240 at 384 x 384 210 of 256 and 18 of 3,008. The error of a sum grows with its slice's rows, so
+// between the lines above pairs take it only where their slices are no longer. (k_splits = 0: four slices on single CTAs, at
+// least as many on pairs.) Error against 64 bits and us, single CTAs /
+// pairs: the first 2.0e-6 / 8.5e-6 and 57 / 54, the second 3.5e-7 / 3.2e-6 and 70 / 29, 1792 x 384 x 28800 with 240 7.3e-7 /
+// 6.3e-6 and 58 / 43, 1152 x 384 x 20250 with 16 1.3e-6 / 3.1e-6 and 25 / 28.
+static bool slices_stay(int M, int N, int K, int k_splits, int sms) {
+  if (k_splits >= 0 || N % G2_BN == 0 || N >= 2048) return true;
+  const int kb = (K + G2_BK - 1) / G2_BK, pairs = sms > 1 ? sms / 2 : 1;
+  const int one = choose_k_splits(((M + 127) / 128) * (N / 128), kb, sms, 4, -k_splits);
+  const int two = choose_k_splits(((M + 255) / 256) * ((N + G2_BN - 1) / G2_BN), kb, pairs, 64, -k_splits);
+  return (kb + two - 1) / two <= (kb + one - 1) / one;
+}
+// The rule for weight gradients with k_splits as aeris_gemm_auto takes it, on a device of `sms` multiprocessors.
+extern "C" int aeris_wgrad_takes_pairs(int M, int N, int K, int k_splits, int sms) {
+  return N % (G2_BN / 2) == 0 && pairs_pay(M, N, K, EPI_ACC_F32) && slices_stay(M, N, K, k_splits, sms);
+}
 extern "C" int aeris_gemm_takes_pairs(int M, int N, int K, int epi, int allow_2cta) {
   const bool taken = N % (epi == EPI_SWIGLU || epi == EPI_SWIGLU_BOTH ? G2_BN : G2_BN / 2) == 0;
   return taken && (allow_2cta == 2 || (allow_2cta && pairs_pay(M, N, K, epi)));
@@ -597,7 +615,8 @@ extern "C" int aeris_gemm_auto(const void* A, const void* B, void* C, int M, int
                                int a_mn, int b_mn, int epi, const void* resid, int ldr, const float* gate,
                                int rows_per_gate, int ld_gate, void* aux, int ld_aux, int swiglu_f, int k_splits,
                                int bn, int allow_2cta, int* status, void* stream) {
-  if (allow_2cta && aeris_gemm_takes_pairs(M, N, K, epi, allow_2cta))
+  if (allow_2cta == 1 && epi == EPI_ACC_F32 ? aeris_wgrad_takes_pairs(M, N, K, k_splits, num_sms())
+                                            : aeris_gemm_takes_pairs(M, N, K, epi, allow_2cta))
     return gemm_two_cta(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, resid, ldr, gate, rows_per_gate, ld_gate, aux,
                         ld_aux, swiglu_f, k_splits, status, stream);
   // few tiles: the smaller ones (wide tiles are for SwiGLU, whose columns come in pairs)
