@@ -196,7 +196,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   uint64_t* pv_done = bars + 20;   // P V of tile j has completed (P buffer reusable, accumulator up to date)
   static_assert(NSK <= 4 && NSV <= 4, "barrier slots");
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
-  int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int qt = blockIdx.x, head = blockIdx.y, win = blockIdx.z;
@@ -204,17 +203,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const int nfull = N / KVT, rem = N - nfull * KVT;
   const int nkv = nfull + (rem ? 1 : 0);
   const int n_last = rem ? ((rem + 15) & ~15) : KVT;  // MMA N of the last K/V tile
-
-  if (threadIdx.x == 0) {
-    int ab = (p.status && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
-    if ((smem_u32(smem) & 1023u) != 0) {
-      ab = 1;
-      if (p.status) atomicCAS(p.status, 0, ERR_BOUNDS);
-    }
-    *s_abort = ab;
-  }
-  __syncthreads();
-  if (*s_abort) { chain_point(); return; }
 
   if (threadIdx.x == 0) {
     prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v);
@@ -236,7 +224,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const uint32_t tS = tmem_base;          // S : 64 columns
   const uint32_t tO = tmem_base + 64;     // O : HD columns, accumulated over all tiles
 
-  if (warp == 0) {
+  if (given_up(p.status, (smem_u32(smem) & 1023u) != 0)) {
+  } else if (warp == 0) {
     if (elect_one_sync()) {
       mbar_expect_tx(q_full, Q_BYTES);
 #pragma unroll

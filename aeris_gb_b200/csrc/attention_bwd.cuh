@@ -186,7 +186,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_i0, const __grid_constant
   float* s_stat = reinterpret_cast<float*>(s_out + R::OUT_BYTES);
   BwdBars* bar = reinterpret_cast<BwdBars*>(s_stat + R::STAT);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 1);
-  int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int N = p.N;
@@ -198,13 +197,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_i0, const __grid_constant
   const int n_items = (n_items_total - static_cast<int>(blockIdx.x) + n_ctas - 1) / n_ctas;
   const int total = n_items * n_str;
 
-  if (threadIdx.x == 0) {
-    int ab = (p.status && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
-    if ((smem_u32(smem) & 1023u) != 0) { ab = 1; if (p.status) atomicCAS(p.status, 0, ERR_BOUNDS); }
-    *s_abort = ab;
-  }
-  __syncthreads();
-  if (*s_abort) { chain_point(); return; }
   if (threadIdx.x == 0) {
     prefetch_tmap(&tm_i0); prefetch_tmap(&tm_i1); prefetch_tmap(&tm_r0); prefetch_tmap(&tm_r1);
     for (int i = 0; i < NB; ++i) {
@@ -230,7 +222,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_i0, const __grid_constant
   const uint32_t tmem_base = *tmem_slot;
   chain_point();
 
-  if ((warp & ~3) == R::W_LOAD) {
+  if (given_up(p.status, (smem_u32(smem) & 1023u) != 0)) {
+  } else if ((warp & ~3) == R::W_LOAD) {
     regs_dec<R::REGS_REST>();
     if (warp == R::W_LOAD) {
       // ---------------------------------------------------------- TMA producer, one lane; dK/dV: all lanes copy statistics

@@ -114,7 +114,6 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   uint64_t* turn = bars + 34;           // [2] P_OVER_S: whose products are next
   uint64_t* half = bars + 36;           // [2][4] a warp is half way through its exponentials
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 44);
-  int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int N = p.N;
@@ -126,13 +125,6 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const int n_items = (n_items_total - static_cast<int>(blockIdx.x) + n_ctas - 1) / n_ctas;
   const int total = n_items * nkv;
 
-  if (threadIdx.x == 0) {
-    int ab = (p.status && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
-    if ((smem_u32(smem) & 1023u) != 0) { ab = 1; if (p.status) atomicCAS(p.status, 0, ERR_BOUNDS); }
-    *s_abort = ab;
-  }
-  __syncthreads();
-  if (*s_abort) { chain_point(); return; }
   if (threadIdx.x == 0) {
     prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v);
     for (int i = 0; i < 4; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); }
@@ -154,7 +146,8 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const uint32_t tmem_base = *tmem_slot;
   chain_point();
 
-  if (warp == 8) {
+  if (given_up(p.status, (smem_u32(smem) & 1023u) != 0)) {
+  } else if (warp == 8) {
     // ------------------------------------------------------------ TMA producer
     if (elect_one_sync()) {
       int vi[2] = {0, 0};               // query tiles requested so far, per chain

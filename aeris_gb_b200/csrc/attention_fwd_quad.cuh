@@ -55,7 +55,6 @@ attn_fwd_quad_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   uint8_t* sO = sT + NST * R::STAGE;                // [softmax warps]
   QuadBars* bar = reinterpret_cast<QuadBars*>(sO + 4 * NC * R::OUT_BYTES);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 1);
-  int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int N = p.N;
@@ -68,13 +67,6 @@ attn_fwd_quad_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const int n_items = (n_items_total - static_cast<int>(blockIdx.x) + n_ctas - 1) / n_ctas;
   const int total = n_items * nkv;
 
-  if (threadIdx.x == 0) {
-    int ab = (p.status && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
-    if ((smem_u32(smem) & 1023u) != 0) { ab = 1; if (p.status) atomicCAS(p.status, 0, ERR_BOUNDS); }
-    *s_abort = ab;
-  }
-  __syncthreads();
-  if (*s_abort) { chain_point(); return; }
   if (threadIdx.x == 0) {
     prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v);
     for (int c = 0; c < NC; ++c) {
@@ -91,7 +83,8 @@ attn_fwd_quad_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const uint32_t tmem_base = *tmem_slot;
   chain_point();
 
-  if (warp >= R::W_LOAD) {
+  if (given_up(p.status, (smem_u32(smem) & 1023u) != 0)) {
+  } else if (warp >= R::W_LOAD) {
     regs_dec<R::REGS_REST>();
     if (warp == R::W_LOAD) {
       // ---------------------------------------------------------- TMA producer

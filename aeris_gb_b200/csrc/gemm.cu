@@ -51,12 +51,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  {  // an earlier kernel already failed: leave before touching TMEM (decision made once per CTA)
-    __shared__ int s_abort;
-    if (threadIdx.x == 0) s_abort = (p.status && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
-    __syncthreads();
-    if (s_abort) { chain_point(); return; }
-  }
 
   const int m_tiles = (p.M + BM - 1) / BM;
   const int n_tiles = p.N / BN;
@@ -87,7 +81,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   const uint32_t tmem_base = *tmem_slot;
   chain_point();
 
-  if (warp == 0) {
+  if (given_up(p.status)) {
+  } else if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     if (elect_one_sync()) {
       int stage = 0;
