@@ -9,7 +9,8 @@
 //   * stage free   : one `tcgen05.commit` arrives on the same barrier in both CTAs (commit with a CTA mask);
 //   * accumulator ready: same two-CTA commit; accumulator drained: both CTAs' epilogue warps arrive on the leader.
 // Every wait is bounded and every role falls through to one final cluster barrier, so a time-out in one CTA can not
-// leave its peer waiting forever.
+// leave its peer waiting forever. Nothing is under way any more when a CTA gets there: each role waits for what it started
+// and nobody took (operand tiles, requests ahead, products), whatever it was that ended its loop.
 #include "common.cuh"
 #include "api.h"
 #include "host.h"
@@ -229,6 +230,12 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
+      // the tiles that the issuer did not take, of both CTAs: their bytes are on the leader's barriers (a stage never filled
+      // counts as there)
+      for (int s = 0; s < STAGES && !ok && crank == 0; ++s) {
+        if (--stage < 0) { stage = STAGES - 1; phase ^= 1; }
+        if (!mbar_wait_poll(&full_bar[stage], phase, nullptr, 0)) break;
+      }
     }
   } else if (warp == 1) {
     if (elect_one_sync()) {
@@ -267,6 +274,9 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
           tc_commit2_mc(&tfull_bar[acc], 0x3);         // accumulator ready in both CTAs
           if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         }
+        // the last products have completed: an epilogue that gave up has not waited for them
+        if (--stage < 0) { stage = STAGES - 1; phase ^= 1; }
+        mbar_wait_poll(&empty_bar[stage], phase, nullptr, 0);
       }
     }
   } else if (AG && warp >= 6) {
@@ -319,7 +329,9 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       const int mn = tile - split * (m_tiles * n_tiles);
       int tm, tn;
       tile_mn(mn, tm, tn);
-      if (!mbar_wait_poll(&tfull_bar[acc], acc_phase, p.status, ERR_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      // the warp decides as one: what it does after giving up takes all lanes
+      ok = __all_sync(0xffffffffu, mbar_wait_poll(&tfull_bar[acc], acc_phase, p.status, ERR_TIMEOUT_TMEM_FULL));
+      if (!ok) break;
       tc_fence_after();
       const int row = tm * 2 * G2_BM + crank * G2_BM + q * 32 + lane;
       const uint32_t taddr = tmem_base + acc * G2_BN + (static_cast<uint32_t>(q * 32) << 16);
@@ -429,7 +441,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     // their slots after a rank barrier that follows this kernel in the stream)
     if (p.epi == EPI_RS_PUSH) rs_stage_drain();
     if (p.staged_out) TileOut{nullptr, lane}.drain();
-    if constexpr (EW == 8) asm volatile("cp.async.wait_all;" ::: "memory");     // after a time-out: copies nobody took
+    if constexpr (EW == 8) {       // after a time-out: what was requested ahead and nobody took
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      for (; u_m < u_n; ++u_m) mbar_wait_warp(u_bar + (u_m & 1), (u_m >> 1) & 1, p.status, ERR_TIMEOUT_FULL);
+    }
   }
 
   tc_fence_before();
