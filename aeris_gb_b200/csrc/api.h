@@ -36,6 +36,8 @@ int aeris_attn_fwd(const void* q, int ldq, int q_col0, const void* k, int ldk, i
 int aeris_attn_bwd(const void* qkv, int ldq, int q_col0, int k_col0, int v_col0, const void* o, const void* d_o,
                    int ldo, const float* lse, float* delta, void* dqkv, int ldg, int n_win, int N, int H,
                    int head_dim, float scale, int* status, void* stream);
+// 1 where aeris_attn_bwd takes these extents on a device of `sms` multiprocessors, 0 where it returns -23.
+int aeris_attn_bwd_countable(int n_win, int N, int H, int head_dim, int sms);
 
 int aeris_gemm_scatter_heads(const void* A, const void* B, int M, int N, int K, int lda, int ldb, int b_mn,
                              const void* const* peers, int sp, int sp_rank, int n_local, int L, int sec_w, int* status,

@@ -669,6 +669,13 @@ static int attn_fwd_impl(const void* q, int ldq, int q_col0, const void* k, int 
   return poly ? launch_attn_fwd<1, 2, 0>(tq, tk, tv, p, stream) : launch_attn_fwd<1, -1, 0>(tq, tk, tv, p, stream);
 }
 
+// Whether the backward kernels can count their items, and a CTA the tiles it streams past them, in 32 bits.
+extern "C" int aeris_attn_bwd_countable(int n_win, int N, int H, int head_dim, int sms) {
+  const int bt = head_dim <= 64 ? BwdCfg<1, false>::BT : BwdCfg<2, false>::BT;
+  const long long items = (static_cast<long long>(N) + TILE - 1) / TILE * H * n_win;
+  return items <= 0x3fffffff && items * ((static_cast<long long>(N) + bt - 1) / bt) <= 0x3fffffffll * sms;
+}
+
 // Backward. qkv: fused [T, ldq] tensor (q/k/v column blocks at *_col0); o, d_o: [T, ldo]; dqkv: [T, ldg] (same
 // column layout as qkv); lse from the forward; delta: scratch [n_win*H*N] fp32 written by the first kernel.
 static int attn_bwd_impl(const void* qkv, int ldq, int q_col0, int k_col0, int v_col0, const void* o, const void* d_o,
@@ -706,6 +713,7 @@ static int attn_bwd_impl(const void* qkv, int ldq, int q_col0, int k_col0, int v
   if (!whole_vectors(o, ldo) || !whole_vectors(d_o, ldo) || !whole_vectors(dqkv, ldg | q_col0 | k_col0 | v_col0)) return -4;
   for (int i = 0; i < sp; ++i)
     if (!whole_vectors(dq_peers[i], push_ld | push_sec_w | push_col0)) return -4;
+  if (!aeris_attn_bwd_countable(n_win, N, H, head_dim, num_sms())) return -23;
   AttnBwdParams p{};
   for (int i = 0; i < sp; ++i) p.dq_peers[i] = const_cast<void*>(dq_peers[i]);
   p.push_n_local = dq_peers ? push_n_local : 0; p.push_ld = push_ld; p.push_sec_w = push_sec_w; p.push_col0 = push_col0;

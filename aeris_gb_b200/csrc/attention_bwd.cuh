@@ -772,9 +772,7 @@ static int launch_attn_bwd(const CUtensorMap& tq128, const CUtensorMap& tk64, co
     if (f1.numRegs * R1::THREADS < R1::REGS || f2.numRegs * R2::THREADS < R2::REGS) return -24;
     configured = true;
   }
-  const long long items = static_cast<long long>((p.N + TILE - 1) / TILE) * p.H * p.n_win;
-  if (items > 0x3fffffff) return -23;
-  const int n = static_cast<int>(items), grid = n < num_sms() ? n : num_sms();
+  const int n = (p.N + TILE - 1) / TILE * p.H * p.n_win, grid = n < num_sms() ? n : num_sms();
   if (launch_chained(k1, grid, R1::THREADS, R1::SMEM, stream, tq128, tdo128, tk64, tv64, out[0], out[0], p, n)) return -21;
   return launch_chained(k2, grid, R2::THREADS, R2::SMEM, stream, tk128, tv128, tq64, tdo64, out[1], out[2], p, n) ? -22 : 0;
 }
