@@ -126,10 +126,11 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, in
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* status, int code) {
   return mbar_wait_warp(smem_u32(bar), parity, status, code);
 }
-// Two barriers, both tries under way at once: a wait that is over costs 110-200 cycles of latency.
+// Two barriers in one step: a wait that is over costs 110-200 cycles of latency once for both. Each of the two tries may
+// suspend the warp, hence half the steps.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, int* status, int code) {
 #pragma unroll 1
-  for (int i = 0; i < MBAR_TRIES; ++i) {
+  for (int i = 0; i < MBAR_TRIES / 2; ++i) {
     uint32_t ok;
     asm volatile(
         "{\n\t"
