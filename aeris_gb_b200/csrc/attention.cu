@@ -216,16 +216,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     fence_barrier_init();
   }
   if (warp == 1) { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
+  chain_point();
   tc_fence_before();
-  __syncthreads();
+  const bool stop = given_up(p.status, reinterpret_cast<int*>(tmem_slot + 1), (smem_u32(smem) & 1023u) != 0);
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  chain_point();
   const uint32_t tS = tmem_base;          // S : 64 columns
   const uint32_t tO = tmem_base + 64;     // O : HD columns, accumulated over all tiles
 
-  if (given_up(p.status, (smem_u32(smem) & 1023u) != 0)) {
-  } else if (warp == 0) {
+  if (stop) {
+    if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
+    return;
+  }
+  if (warp == 0) {
     if (elect_one_sync()) {
       mbar_expect_tx(q_full, Q_BYTES);
 #pragma unroll

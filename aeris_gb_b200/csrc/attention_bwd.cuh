@@ -221,9 +221,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_i0, const __grid_constant
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   chain_point();
+  const bool stop = given_up(p.status, reinterpret_cast<int*>(tmem_slot + 1), (smem_u32(smem) & 1023u) != 0);
 
-  if (given_up(p.status, (smem_u32(smem) & 1023u) != 0)) {
-  } else if ((warp & ~3) == R::W_LOAD) {
+  if (stop) {
+    if (warp == R::W_A) tmem_dealloc(tmem_base, 512);
+    return;
+  }
+  if ((warp & ~3) == R::W_LOAD) {
     regs_dec<R::REGS_REST>();
     if (warp == R::W_LOAD) {
       // ---------------------------------------------------------- TMA producer, one lane; dK/dV: all lanes copy statistics

@@ -140,14 +140,17 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     fence_barrier_init();
   }
   if (warp == 8) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  chain_point();
   tc_fence_before();
-  __syncthreads();
+  const bool stop = given_up(p.status, reinterpret_cast<int*>(tmem_slot + 1), (smem_u32(smem) & 1023u) != 0);
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  chain_point();
 
-  if (given_up(p.status, (smem_u32(smem) & 1023u) != 0)) {
-  } else if (warp == 8) {
+  if (stop) {
+    if (warp == 8) tmem_dealloc(tmem_base, 512);
+    return;
+  }
+  if (warp == 8) {
     // ------------------------------------------------------------ TMA producer
     if (elect_one_sync()) {
       int vi[2] = {0, 0};               // query tiles requested so far, per chain

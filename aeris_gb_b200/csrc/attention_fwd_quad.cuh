@@ -77,14 +77,17 @@ attn_fwd_quad_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     fence_barrier_init();
   }
   if (warp == R::W_LOAD) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  chain_point();
   tc_fence_before();
-  __syncthreads();
+  const bool stop = given_up(p.status, reinterpret_cast<int*>(tmem_slot + 1), (smem_u32(smem) & 1023u) != 0);
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  chain_point();
 
-  if (given_up(p.status, (smem_u32(smem) & 1023u) != 0)) {
-  } else if (warp >= R::W_LOAD) {
+  if (stop) {
+    if (warp == R::W_LOAD) tmem_dealloc(tmem_base, 512);
+    return;
+  }
+  if (warp >= R::W_LOAD) {
     regs_dec<R::REGS_REST>();
     if (warp == R::W_LOAD) {
       // ---------------------------------------------------------- TMA producer
@@ -199,7 +202,6 @@ attn_fwd_quad_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     // ------------------------------------------------------------ softmax: one thread = one query row of its chain
     regs_inc<R::REGS_SOFTMAX>();
     const int c = warp >> 2, q = warp & 3;
-    const int row = q * 32 + lane;
     const uint32_t tS = tmem_base + c * R::COLS + (static_cast<uint32_t>(q * 32) << 16), tO = tS + R::COL_O;
     const float sl2 = p.scale_log2;
     const uint64_t sl = f2_pack(sl2, sl2);

@@ -234,12 +234,17 @@ __device__ __forceinline__ void chain_point() {
 }
 // Whether a kernel before this one gave up (what it wrote is incomplete, so this one leaves as well), or this CTA's shared
 // memory is `misplaced`. All threads call it behind chain_point: before that the kernel in front may still be running, and
-// its time-out would be seen one launch late. The CTA decides as one. The read behind the wait costs a sampler step of seven
-// evaluations of two blocks of width 256 on 14,400 tokens 1,740 -> 1,750 us; wider models nothing that can be measured.
-// (The two-CTA products do not ask.)
-__device__ __forceinline__ bool given_up(int* status, bool misplaced = false) {
-  if (threadIdx.x == 0 && misplaced && status) atomicCAS(status, 0, ERR_BOUNDS);
-  return __syncthreads_or(misplaced || (threadIdx.x == 0 && status && *reinterpret_cast<volatile int*>(status) != 0));
+// its time-out would be seen one launch late. The CTA decides as one, through `shared`; the barrier serves the TMEM address
+// too, except in the backward kernel, where that way spills registers (200 windows x 225 tokens, 24 heads x 64: 0.484 ms
+// before, 0.505 with one barrier, 0.483 with one more). The read behind the wait takes 0.3 us: a sampler step of seven
+// evaluations of two blocks of width 256 on 14,400 tokens 1,737 -> 1,755 us. (The two-CTA products do not ask.)
+__device__ __forceinline__ bool given_up(int* status, int* shared, bool misplaced = false) {
+  if (threadIdx.x == 0) {
+    if (misplaced && status) atomicCAS(status, 0, ERR_BOUNDS);
+    *shared = misplaced || (status && *reinterpret_cast<volatile int*>(status) != 0);
+  }
+  __syncthreads();
+  return *shared != 0;
 }
 // The result is the launch's only trace: it has taken the error from the runtime.
 template <typename... P, typename... A>

@@ -75,14 +75,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     tmem_alloc(tmem_slot, 2 * BN);  // 2 accumulators of BN fp32 columns (256 or 512 columns)
     tmem_relinquish();
   }
+  chain_point();
   tc_fence_before();
-  __syncthreads();
+  const bool stop = given_up(p.status, reinterpret_cast<int*>(tmem_slot + 1));
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  chain_point();
 
-  if (given_up(p.status)) {
-  } else if (warp == 0) {
+  if (stop) {
+    if (warp == 1) tmem_dealloc(tmem_base, 2 * BN);
+    return;
+  }
+  if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     if (elect_one_sync()) {
       int stage = 0;
