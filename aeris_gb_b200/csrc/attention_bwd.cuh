@@ -12,16 +12,17 @@
 // scores and dV, B dP and dQ or dK. Two warpgroups share a chain's tile, half of the columns each, because what bounds the
 // math warps is the latency of their own steps, not a unit; another warpgroup takes the gradients to memory, so that no
 // math warp waits for an item's last products. A chain's round of 2,300 cycles at head_dim 64 (96 columns) is 1,070 of
-// exponentials (768 by themselves), 440 of dS and 500-800 of waits; tensor core and exponential unit are at 55-65 %.
+// exponentials (768 by themselves), 440 of dS and 500-800 of waits; ncu, 36 windows of 900 tokens, dQ and dK/dV: tensor core
+// at 48 and 56 %, exponential unit at 65 and 56.
 // At 128 the products bound it: 64-column tiles (a wider one has no room in shared memory) take 48 cycles per step of 16
 // where 32 would be the rate, because both operands come from shared memory.
 //
 // Both kernels, ms, one call, bursts of 6 ms, with one issuer and 64 columns per chain and warpgroup / now: 72 windows x 900
-// tokens, 24 heads x 64 1.728 / 1.432; 12 x 128 1.418 / 1.260; 16 x 3600, 12 x 128 3.80 / 3.43; 200 x 225, 24 x 64
-// 0.645 / 0.490, 12 x 128 0.534 / 0.465; 400 x 64, 24 x 64 0.436 / 0.352; 8 x 900, 4 x 64 0.0522 / 0.0457.
+// tokens, 24 heads x 64 1.73 / 1.41; 12 x 128 1.42 / 1.24; 16 x 3600, 12 x 128 3.80 / 3.40; 200 x 225, 24 x 64
+// 0.645 / 0.488, 12 x 128 0.534 / 0.465; 400 x 64, 24 x 64 0.436 / 0.349; 8 x 900, 4 x 64 0.0522 / 0.0457.
 // On the way: three chains of 64 columns and one warpgroup each 1.57, with 32-column halves in a rolled loop 1.62; the
-// issuers' loops unrolled over the ring 2.45 (instruction cache); single threads as issuers 1.446 (128: 1.333 for 1.260);
-// waits with a call behind the first try 1.65; turns at the exponentials 1.83 for 1.57.
+// issuers' loops unrolled over the ring 2.45 (instruction cache); single threads as issuers 1.446 for 1.432 (128: 1.333
+// for 1.260); waits with a call behind the first try 1.65; turns at the exponentials 1.83 for 1.57.
 #pragma once
 #include <stddef.h>
 

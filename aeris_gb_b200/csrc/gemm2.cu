@@ -579,7 +579,8 @@ extern "C" int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M
 }
 
 // Which kernel takes a product of N = n * 128 columns: CTA pairs on tiles of 256 x 256, whose last one may be half empty,
-// or single CTAs on tiles of 128 x 128 (256 wide where `bn` is 0 and N allows it). us, bursts, one CTA / pairs:
+// or single CTAs, on tiles of 128 x 128 for stores, 256 wide where N allows it for SwiGLU and accumulating products. us,
+// bursts, one CTA / pairs:
 //   * plain and gated stores: a wave of pairs takes 1.2 to 1.4 times as long as one of single CTAs, so the numbers of waves
 //     decide. 12150 x 384 x 1152 13.1 / 16.7 (2 and 2 waves), 4096 x 1152 x 3456 28.6 / 39.1 (2, 2), 28800 x 384 x 384
 //     26.2 / 21.8 (5, 4), 12150 x 1152 x 1152 51.0 / 50.5 (6, 4), 12150 x 640 x 640 22.6 / 16.4 (4, 2), 4096 x 1664 x 4992
@@ -587,7 +588,8 @@ extern "C" int aeris_gemm_bf16_2cta(const void* A, const void* B, void* C, int M
 //   * SwiGLU backward: only the pairs' kernel requests its second operand ahead. 4096 x 384 x 128 9.8 / 9.8, 12150 x 896 x
 //     384 44.1 / 28.3, 64800 x 3456 x 1664 1179 / 669.
 //   * SwiGLU forward that also stores the raw columns: the pairs' tiled stores. 4096 x 1024 x 256 7.9 / 8.2, 12150 x 1792 x
-//     384 38.6 / 26.0, 57600 x 4096 x 768 469 / 321; only at the very smallest one CTA, 4096 x 512 x 128 5.4 / 7.3.
+//     384 38.6 / 26.0, 57600 x 4096 x 768 469 / 321; only at the very smallest one CTA, 4096 x 512 x 128 5.4 / 7.3
+//     (pairs take that one too: where the line would lie has not been measured).
 //   * SwiGLU forward without the raw columns: its tiles halve on the way out, and short sums leave the epilogue as the
 //     bound, which every CTA of its own overlaps better. 14400 x 1024 x 256 13.8 / 17.2, 64800 x 1024 x 384 59 / 67,
 //     28800 x 3072 x 384 76.6 / 83.6; held for 0.25 s 64800 x 2048 x 384 120 / 126, x 2048 x 512 146 / 144.
@@ -607,9 +609,9 @@ static bool pairs_pay(int M, int N, int K, int epi) {
 // quarter of the tiles leaves less room for free ones: of 60 asked for at 1152 x 384 x 53550 single CTAs make 27 of 1,984
 // rows, pairs 7 of 7,680; of 240 at 384 x 384 210 of 256 and 18 of 3,008. The error of a sum grows with its slice's rows, so
 // between the lines above pairs take it only where their slices are no longer. (k_splits = 0: four slices on single CTAs, at
-// least as many on pairs.) Error against 64 bits and us, single CTAs /
-// pairs: the first 2.0e-6 / 8.5e-6 and 57 / 54, the second 3.5e-7 / 3.2e-6 and 70 / 29, 1792 x 384 x 28800 with 240 7.3e-7 /
-// 6.3e-6 and 58 / 43, 1152 x 384 x 20250 with 16 1.3e-6 / 3.1e-6 and 25 / 28.
+// least as many on pairs.) Error against 64 bits and us, single CTAs / pairs: the first 2.0e-6 / 8.5e-6 and 57 / 54, the
+// second 3.5e-7 / 3.2e-6 and 70 / 29, 1792 x 384 x 28800 with 240 7.3e-7 / 6.3e-6 and 58 / 43, 1152 x 384 x 20250 with 16
+// 1.3e-6 / 3.1e-6 and 25 / 28.
 static bool slices_stay(int M, int N, int K, int k_splits, int sms) {
   if (k_splits >= 0 || N % G2_BN == 0 || N >= 2048) return true;
   const int kb = (K + G2_BK - 1) / G2_BK, pairs = sms > 1 ? sms / 2 : 1;

@@ -10,8 +10,8 @@ pytestmark = pytest.mark.gpu
 
 def _config(**kw):
     from aeris_gb_b200.models.aeris import AerisConfig
-    return AerisConfig(img=(60, 120), window=(30, 30), in_channels=20, out_channels=9, dim=256, heads=4, head_dim=64, mlp_dim=512,
-                       n_layers=2, sublayers=1, chunk_windows=4, **kw)
+    return AerisConfig(img=(60, 120), window=(30, 30), in_channels=20, out_channels=9, dim=256, heads=4, head_dim=64,
+                       mlp_dim=512, n_layers=2, sublayers=1, chunk_windows=4, **kw)
 
 
 def _wait_after_each_launch(monkeypatch):

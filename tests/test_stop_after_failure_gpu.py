@@ -61,7 +61,8 @@ def _attention(n_win, N, H, d):
 
 
 # one query tile, two in turn, four at a time
-@pytest.mark.parametrize("n_win,N,H,d", [(8, 100, 2, 64), (8, 100, 2, 128), (8, 250, 2, 64), (8, 200, 2, 128), (50, 300, 2, 64)])
+@pytest.mark.parametrize("n_win,N,H,d", [(8, 100, 2, 64), (8, 100, 2, 128), (8, 250, 2, 64), (8, 200, 2, 128),
+                                         (50, 300, 2, 64)])
 def test_attention_forward(n_win, N, H, d):
     qkv, o, lse = _attention(n_win, N, H, d)
     ld, p = 3 * H * d, L.ptr
