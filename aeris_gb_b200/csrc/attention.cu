@@ -196,6 +196,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   uint64_t* pv_done = bars + 20;   // P V of tile j has completed (P buffer reusable, accumulator up to date)
   static_assert(NSK <= 4 && NSV <= 4, "barrier slots");
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
+  int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
+  int* s_failed = s_abort + 1;      // [4] see note_failure
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int qt = blockIdx.x, head = blockIdx.y, win = blockIdx.z;
@@ -203,6 +205,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const int nfull = N / KVT, rem = N - nfull * KVT;
   const int nkv = nfull + (rem ? 1 : 0);
   const int n_last = rem ? ((rem + 15) & ~15) : KVT;  // MMA N of the last K/V tile
+
+  if (threadIdx.x == 0) {
+    int ab = (p.status && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
+    if ((smem_u32(smem) & 1023u) != 0) { ab = 1; if (p.status) atomicCAS(p.status, 0, ERR_BOUNDS); }
+    *s_abort = ab;
+  }
+  __syncthreads();
+  if (*s_abort) { chain_point(); return; }
 
   if (threadIdx.x == 0) {
     prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v);
@@ -216,18 +226,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     fence_barrier_init();
   }
   if (warp == 1) { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
-  chain_point();
   tc_fence_before();
-  const bool stop = given_up(p.status, reinterpret_cast<int*>(tmem_slot + 1), (smem_u32(smem) & 1023u) != 0);
+  __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_point();
   const uint32_t tS = tmem_base;          // S : 64 columns
   const uint32_t tO = tmem_base + 64;     // O : HD columns, accumulated over all tiles
 
-  if (stop) {
-    if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
-    return;
-  }
   if (warp == 0) {
     if (elect_one_sync()) {
       mbar_expect_tx(q_full, Q_BYTES);
@@ -313,6 +319,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const int q = warp & 3;
     const int row = q * 32 + lane;            // row inside the Q tile == TMEM lane
     const int grow = qt * TILE + row;         // row inside the window
+    note_failure(p.status, &s_failed[q]);
     const bool warp_valid = (qt * TILE + q * 32) < N;
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     const float sl2 = p.scale_log2;
@@ -471,7 +478,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (lane == 0) mbar_arrive(p_full);
       ATTN_STAMP(6);
     }
-    if (ok && warp_valid && mbar_wait(pv_done, (nkv - 1) & 1, p.status, ERR_TIMEOUT_ATTN)) {
+    if (ok && warp_valid && mbar_wait(pv_done, (nkv - 1) & 1, p.status, ERR_TIMEOUT_ATTN) &&
+        !noted(&s_failed[q])) {
       tc_fence_after();
       {
         const float inv = 1.f / l;

@@ -103,7 +103,7 @@ struct BwdBars {
   uint64_t b_full[2], b_empty[2];
   uint64_t stat_full[4], stat_empty[4];
 };
-static_assert(sizeof(BwdBars) + 8 <= 512, "barriers");
+static_assert(sizeof(BwdBars) + 8 + 4 * 4 <= 512, "barriers");
 
 // Asynchronous 4-byte copy (`bytes` = 0: zero fill), and this lane's arrival on a barrier once its copies have landed.
 __device__ __forceinline__ void cp_async4(float* smem_dst, const float* src, uint32_t bytes) {
@@ -187,6 +187,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_i0, const __grid_constant
   float* s_stat = reinterpret_cast<float*>(s_out + R::OUT_BYTES);
   BwdBars* bar = reinterpret_cast<BwdBars*>(s_stat + R::STAT);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 1);
+  int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
+  int* s_failed = s_abort + 1;      // [4] see note_failure
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int N = p.N;
@@ -198,6 +200,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_i0, const __grid_constant
   const int n_items = (n_items_total - static_cast<int>(blockIdx.x) + n_ctas - 1) / n_ctas;
   const int total = n_items * n_str;
 
+  if (threadIdx.x == 0) {
+    int ab = (p.status && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
+    if ((smem_u32(smem) & 1023u) != 0) { ab = 1; if (p.status) atomicCAS(p.status, 0, ERR_BOUNDS); }
+    *s_abort = ab;
+  }
+  __syncthreads();
+  if (*s_abort) { chain_point(); return; }
   if (threadIdx.x == 0) {
     prefetch_tmap(&tm_i0); prefetch_tmap(&tm_i1); prefetch_tmap(&tm_r0); prefetch_tmap(&tm_r1);
     for (int i = 0; i < NB; ++i) {
@@ -222,12 +231,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_i0, const __grid_constant
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   chain_point();
-  const bool stop = given_up(p.status, reinterpret_cast<int*>(tmem_slot + 1), (smem_u32(smem) & 1023u) != 0);
 
-  if (stop) {
-    if (warp == R::W_A) tmem_dealloc(tmem_base, 512);
-    return;
-  }
   if ((warp & ~3) == R::W_LOAD) {
     regs_dec<R::REGS_REST>();
     if (warp == R::W_LOAD) {
@@ -442,6 +446,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_i0, const __grid_constant
     // ------------------------------------------------------------ epilogue; dQ: also lse and delta of the coming items
     const int q = warp & 3;
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
+    note_failure(p.status, &s_failed[q]);
+    __syncwarp();
     BwdOut out{s_out + q * 4096, lane, q * 32};
     Slot sb, si;
     auto statistics = [&](int it) -> bool {
@@ -514,14 +520,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_i0, const __grid_constant
         __syncwarp();
         if (lane == 0) mbar_arrive(empty);
       };
-      const int n = (p.d + 31) / 32;
+      const int n = (p.d + 31) / 32, N_out = noted(&s_failed[q]) ? 0 : N;      // rows that leave
       if (p.push_n_local == 0) {
         for (int c = 0; c < n; ++c)
-          out.put(t + lane_addr + c * 32, f, m, c * 32, w.head, w.tile * TILE, w.win, N, [&] { if (c == n - 1) release(); });
+          out.put(t + lane_addr + c * 32, f, m, c * 32, w.head, w.tile * TILE, w.win, N_out,
+                  [&] { if (c == n - 1) release(); });
         return;
       }
       const int grow = w.tile * TILE + q * 32 + lane;
-      const bool row_ok = grow < N;
+      const bool row_ok = grow < N_out;
       __nv_bfloat16* dst = bwd_dst(p, w.win, row_ok ? grow : 0, w.head, section, col0);
       for (int c = 0; c < n; ++c) {
         uint32_t v[32];

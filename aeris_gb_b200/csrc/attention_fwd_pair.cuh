@@ -114,6 +114,8 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   uint64_t* turn = bars + 34;           // [2] P_OVER_S: whose products are next
   uint64_t* half = bars + 36;           // [2][4] a warp is half way through its exponentials
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 44);
+  int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
+  int* s_failed = s_abort + 1;      // [8] see note_failure
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int N = p.N;
@@ -125,6 +127,13 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const int n_items = (n_items_total - static_cast<int>(blockIdx.x) + n_ctas - 1) / n_ctas;
   const int total = n_items * nkv;
 
+  if (threadIdx.x == 0) {
+    int ab = (p.status && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
+    if ((smem_u32(smem) & 1023u) != 0) { ab = 1; if (p.status) atomicCAS(p.status, 0, ERR_BOUNDS); }
+    *s_abort = ab;
+  }
+  __syncthreads();
+  if (*s_abort) { chain_point(); return; }
   if (threadIdx.x == 0) {
     prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v);
     for (int i = 0; i < 4; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); }
@@ -140,16 +149,12 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     fence_barrier_init();
   }
   if (warp == 8) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
-  chain_point();
   tc_fence_before();
-  const bool stop = given_up(p.status, reinterpret_cast<int*>(tmem_slot + 1), (smem_u32(smem) & 1023u) != 0);
+  __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_point();
 
-  if (stop) {
-    if (warp == 8) tmem_dealloc(tmem_base, 512);
-    return;
-  }
   if (warp == 8) {
     // ------------------------------------------------------------ TMA producer
     if (elect_one_sync()) {
@@ -300,6 +305,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     // ------------------------------------------------------------ softmax: one thread = one query row of its chain
     const int c = warp >> 2, q = warp & 3;
     const int row = q * 32 + lane;
+    note_failure(p.status, &s_failed[warp]);
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     const uint32_t tS = tmem_base + c * 256 + lane_addr, tP = tS + R::COL_P, tO = tS + R::COL_O;
     const float sl2 = p.scale_log2;
@@ -504,7 +510,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         for (int j = 0; j < nkv && ok; ++j) ok = idle_tile(j);
       }
       if (!ok || !wait_pv()) break;
-      if (rows) epilogue(w);
+      if (rows && !noted(&s_failed[warp])) epilogue(w);
     }
     // the copies have been performed before their shared memory goes
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");

@@ -41,7 +41,7 @@ struct QuadBars {
   uint64_t p_full[4];                   // its probabilities have taken their place
   uint64_t o_full[4];                   // the last P V of an item has completed
 };
-static_assert(sizeof(QuadBars) + 8 <= 512, "barriers");
+static_assert(sizeof(QuadBars) + 8 + 4 * 16 <= 512, "barriers");
 
 __global__ void __launch_bounds__(AttnQuad::THREADS, 1)
 attn_fwd_quad_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -55,6 +55,8 @@ attn_fwd_quad_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   uint8_t* sO = sT + NST * R::STAGE;                // [softmax warps]
   QuadBars* bar = reinterpret_cast<QuadBars*>(sO + 4 * NC * R::OUT_BYTES);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 1);
+  int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
+  int* s_failed = s_abort + 1;      // [16] see note_failure
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int N = p.N;
@@ -68,6 +70,13 @@ attn_fwd_quad_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const int total = n_items * nkv;
 
   if (threadIdx.x == 0) {
+    int ab = (p.status && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
+    if ((smem_u32(smem) & 1023u) != 0) { ab = 1; if (p.status) atomicCAS(p.status, 0, ERR_BOUNDS); }
+    *s_abort = ab;
+  }
+  __syncthreads();
+  if (*s_abort) { chain_point(); return; }
+  if (threadIdx.x == 0) {
     prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v);
     for (int c = 0; c < NC; ++c) {
       for (int b = 0; b < NBQ; ++b) { mbar_init(&bar->q_full[c][b], 1); mbar_init(&bar->q_empty[c][b], 1); }
@@ -77,16 +86,12 @@ attn_fwd_quad_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     fence_barrier_init();
   }
   if (warp == R::W_LOAD) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
-  chain_point();
   tc_fence_before();
-  const bool stop = given_up(p.status, reinterpret_cast<int*>(tmem_slot + 1), (smem_u32(smem) & 1023u) != 0);
+  __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_point();
 
-  if (stop) {
-    if (warp == R::W_LOAD) tmem_dealloc(tmem_base, 512);
-    return;
-  }
   if (warp >= R::W_LOAD) {
     regs_dec<R::REGS_REST>();
     if (warp == R::W_LOAD) {
@@ -202,6 +207,7 @@ attn_fwd_quad_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     // ------------------------------------------------------------ softmax: one thread = one query row of its chain
     regs_inc<R::REGS_SOFTMAX>();
     const int c = warp >> 2, q = warp & 3;
+    note_failure(p.status, &s_failed[warp]);
     const uint32_t tS = tmem_base + c * R::COLS + (static_cast<uint32_t>(q * 32) << 16), tO = tS + R::COL_O;
     const float sl2 = p.scale_log2;
     const uint64_t sl = f2_pack(sl2, sl2);
@@ -274,7 +280,7 @@ attn_fwd_quad_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         tc_fence_after();
         if (j == 0) {
           // these scores were issued behind the last P V of the item before: its rows leave now
-          if (pending) epilogue(prev);
+          if (pending && !noted(&s_failed[warp])) epilogue(prev);
           pending = rows;
           prev = w;
           m_ref = -INFINITY;
@@ -340,7 +346,7 @@ attn_fwd_quad_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       }
       o_ph ^= 1;
     }
-    if (ok && pending && mbar_wait_warp(&bar->o_full[c], o_ph ^ 1, p.status, ERR_TIMEOUT_ATTN)) {
+    if (ok && pending && mbar_wait_warp(&bar->o_full[c], o_ph ^ 1, p.status, ERR_TIMEOUT_ATTN) && !noted(&s_failed[warp])) {
       tc_fence_after();
       epilogue(prev);
     }

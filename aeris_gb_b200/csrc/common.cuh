@@ -232,20 +232,23 @@ __device__ __forceinline__ void chain_point() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-// Whether a kernel before this one gave up (what it wrote is incomplete, so this one leaves as well), or this CTA's shared
-// memory is `misplaced`. All threads call it behind chain_point: before that the kernel in front may still be running, and
-// its time-out would be seen one launch late. The CTA decides as one, through `shared`; the barrier serves the TMEM address
-// too, except in the backward kernel, where that way spills registers (200 windows x 225 tokens, 24 heads x 64: 0.484 ms
-// before, 0.505 with one barrier, 0.483 with one more). The read behind the wait takes 0.3 us: a sampler step of seven
-// evaluations of two blocks of width 256 on 14,400 tokens 1,737 -> 1,755 us. (The two-CTA products do not ask.)
-__device__ __forceinline__ bool given_up(int* status, int* shared, bool misplaced = false) {
-  if (threadIdx.x == 0) {
-    if (misplaced && status) atomicCAS(status, 0, ERR_BOUNDS);
-    *shared = misplaced || (status && *reinterpret_cast<volatile int*>(status) != 0);
-  }
-  __syncthreads();
-  return *shared != 0;
+// Whether a kernel gave up.
+__device__ __forceinline__ bool failed(const int* status) {
+  return status && *reinterpret_cast<const volatile int*>(status) != 0;
 }
+// A kernel may look at the status word before its chain_point (or set it, where its shared memory is misplaced) and leave at
+// once: the one exception to the first rule. What it sees there are kernels that have ended, not the one in front, which may
+// still be running. Behind chain_point every warp that writes results asks again, and keeps them to itself where the kernel
+// in front has given up (what it read of that one is incomplete; scratch for a kernel behind, which asks as well, is
+// written). `slot` is the warp's own word of shared memory: nothing is held in registers, and the read's 0.3 us pass while the
+// first operands are on their way. A sampler step of seven evaluations of two blocks of width 256 on 14,400 tokens 1,733 ->
+// 1,738 us; one decision for the whole CTA behind chain_point is on the way of every kernel (1,755) and spilled registers of
+// the attention kernels, a look at `slot` for every row of delta took 3 % of the backward pass. (The two-CTA products do not
+// ask.)
+__device__ __forceinline__ void note_failure(const int* status, int* slot) {
+  if ((threadIdx.x & 31) == 0) *reinterpret_cast<volatile int*>(slot) = failed(status);
+}
+__device__ __forceinline__ bool noted(const int* slot) { return *reinterpret_cast<const volatile int*>(slot) != 0; }
 // The result is the launch's only trace: it has taken the error from the runtime.
 template <typename... P, typename... A>
 [[nodiscard]] static inline int launch_chained(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream,

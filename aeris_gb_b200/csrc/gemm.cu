@@ -52,6 +52,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
+  {  // an earlier kernel already failed: leave before touching TMEM (decision made once per CTA)
+    __shared__ int s_abort;
+    if (threadIdx.x == 0) s_abort = (p.status && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
+    __syncthreads();
+    if (s_abort) { chain_point(); return; }
+  }
+
   const int m_tiles = (p.M + BM - 1) / BM;
   const int n_tiles = p.N / BN;
   const int kb_total = (p.K + BK - 1) / BK;
@@ -75,16 +82,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     tmem_alloc(tmem_slot, 2 * BN);  // 2 accumulators of BN fp32 columns (256 or 512 columns)
     tmem_relinquish();
   }
-  chain_point();
   tc_fence_before();
-  const bool stop = given_up(p.status, reinterpret_cast<int*>(tmem_slot + 1));
+  __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_point();
 
-  if (stop) {
-    if (warp == 1) tmem_dealloc(tmem_base, 2 * BN);
-    return;
-  }
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     if (elect_one_sync()) {
@@ -178,6 +181,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
+    const bool keep = !failed(p.status);       // see note_failure
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
       const int split = tile / (m_tiles * n_tiles);
       const int mn = tile - split * (m_tiles * n_tiles);
@@ -187,7 +191,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const int row = tm * BM + q * 32 + lane;
       const uint32_t taddr = tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16);
       const bool kempty = (split * kb_per_split) >= kb_total;  // split with no k-blocks: accumulator undefined
-      gemm_epilogue_row<BN>(p, taddr, row, row < p.M, tn, kempty);
+      gemm_epilogue_row<BN>(p, taddr, row, keep && row < p.M, tn, kempty);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty_bar[acc]);

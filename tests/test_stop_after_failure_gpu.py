@@ -1,5 +1,5 @@
-"""A kernel behind one that gave up leaves its outputs alone, also where it started while that one was still running. Here the
-word that tells it is part of what a long product of one tile writes: zero while the kernel behind it starts on the other
+"""A kernel behind one that gave up keeps its results to itself, also where it started while that one was still running. Here
+the word that tells it is part of what a long product of one tile writes: zero while the kernel behind it starts on the other
 multiprocessors, not zero when its turn comes."""
 import ctypes
 
@@ -79,4 +79,4 @@ def test_attention_backward(n_win, N, H, d):
     ld, p = 3 * H * d, L.ptr
     _behind_a_failure(lambda status: (lambda: L.lib().aeris_attn_bwd(
         p(qkv), ld, 0, H * d, 2 * H * d, p(o), p(d_o), H * d, p(lse), p(delta), p(g), ld, n_win, N, H, d, ctypes.c_float(0.125),
-        status, L.stream_ptr()), [delta, g]))
+        status, L.stream_ptr()), [g]))         # delta is scratch
